@@ -760,10 +760,9 @@ static int sz_ffn(cudaStream_t st, int type, const SzPlan* plan, int groups, u64
 }
 
 
-struct SzXWindows { int n = 1; long long x = 0, gu = 0, d = 0; };   // plans in a row, one block row each: elements between the windows' inputs and sums
 template <int K, int NTC>
 static int sz_x3_launch_k(cudaStream_t st, const sz_moe_layer* L, int m, const SzPlan* plan, const float* x, long long* acc_gu, long long* acc_d,
-                          u32* ctrl, bool sh, bool only_xw = false, SzXWindows win = SzXWindows()) {
+                          u32* ctrl, bool sh) {
     static bool set = false;
     if (!set) {
         SZ_CUDA(cudaFuncSetAttribute(sz_x3_gateup_kernel<K, NTC>, cudaFuncAttributeMaxDynamicSharedMemorySize, SzX3<K, NTC>::SMEM_BYTES));
@@ -773,7 +772,7 @@ static int sz_x3_launch_k(cudaStream_t st, const sz_moe_layer* L, int m, const S
     // SZ_X3_CLASSIC=1: the block-synchronous kernels of sz_moe_exl3.cuh (the second implementation; same bits) instead of the
     // warp-specialised ones
     const char* cl = getenv("SZ_X3_CLASSIC");   // (read at every call: a test switches it inside one process)
-    const bool classic = !only_xw && cl && atoi(cl) != 0;
+    const bool classic = cl && atoi(cl) != 0;
     if (!classic) {
         // Shape of the launch: OCC blocks a multiprocessor (2 or 3), a unit 8 TW tile columns a consumer warp wide (TW = 4, 2 or 1: 24, 12
         // or 6 KB of trellis at 3 bits).  Narrower units and a third block spread the units evenly: gate / up of 40 experts of the
@@ -790,7 +789,7 @@ static int sz_x3_launch_k(cudaStream_t st, const sz_moe_layer* L, int m, const S
         if (!(tw == 1 || tw == 2 || tw == 4) || tw > NTC || NTC % tw) tw = NTC < 4 ? NTC : 4;
         if (tw == 3) tw = 1;
         if (!(twd == 1 || twd == 2 || twd == 4)) twd = 4;
-        const dim3 grid(occ * sz_sm_count(), win.n);
+        const dim3 grid(occ * sz_sm_count());
         int rc = SZ_E_TYPE;
 #define SZ_XW_GU(TT, OO)                                                                                                                    \
     if (tw == TT && occ == OO) {                                                                                                            \
@@ -798,7 +797,7 @@ static int sz_x3_launch_k(cudaStream_t st, const sz_moe_layer* L, int m, const S
         if (!setv) { SZ_CUDA(cudaFuncSetAttribute(sz_xw_gateup_kernel<K, NTC, TT, OO>, cudaFuncAttributeMaxDynamicSharedMemorySize, SzXW<K, TT, OO>::SMEM_BYTES)); setv = true; } \
         SZ_CUDA(sz_launch("gateup_exl3s", sz_xw_gateup_kernel<K, NTC, TT, OO>, grid, block, SzXW<K, TT, OO>::SMEM_BYTES, st, true, plan, (const u8*)L->gate, \
                           (u64)L->gate_stride, (const u8*)L->up, (u64)L->up_stride, (const u8*)(sh ? L->sh_gate : 0), (const u8*)(sh ? L->sh_up : 0), x, m, \
-                          (int)L->hidden, (int)L->top_k, acc_gu, ctrl, win.x, win.gu));                                                     \
+                          (int)L->hidden, (int)L->top_k, acc_gu, ctrl));                                                                    \
         rc = SZ_OK;                                                                                                                         \
     }
 #define SZ_XW_DN(TT, OO)                                                                                                                    \
@@ -808,7 +807,7 @@ static int sz_x3_launch_k(cudaStream_t st, const sz_moe_layer* L, int m, const S
         SZ_CUDA(sz_launch("down_exl3s", sz_xw_down_kernel<K, TT, OO>, grid, block, SzXW<K, TT, OO>::SMEM_BYTES, st, true, plan, (const u8*)L->gate, (u64)L->gate_stride, \
                           (const u8*)L->up, (u64)L->up_stride, (const u8*)L->down, (u64)L->down_stride, (const u8*)(sh ? L->sh_gate : 0),   \
                           (const u8*)(sh ? L->sh_up : 0), (const u8*)(sh ? L->sh_down : 0), m, (int)L->hidden, (int)L->expert_ff, (int)L->top_k, \
-                          (const long long*)acc_gu, acc_d, ctrl, win.gu, win.d));                                                           \
+                          (const long long*)acc_gu, acc_d, ctrl));                                                                          \
         rc = SZ_OK;                                                                                                                         \
     }
         if constexpr (NTC % 4 == 0) { SZ_XW_GU(4, 2) SZ_XW_GU(4, 3) }
@@ -835,9 +834,9 @@ static int sz_x3_launch_k(cudaStream_t st, const sz_moe_layer* L, int m, const S
 }
 
 static int sz_x3_launch(cudaStream_t st, const sz_moe_layer* L, int m, const SzPlan* plan, const float* x, long long* acc_gu, long long* acc_d,
-                        u32* ctrl, bool sh, bool only_xw = false, SzXWindows win = SzXWindows()) {
+                        u32* ctrl, bool sh) {
     const int K = L->expert_type - 1020, NTC = L->expert_ff / 128;
-#define SZ_X3_CASE(KK, NN) if (K == KK && NTC == NN) return sz_x3_launch_k<KK, NN>(st, L, m, plan, x, acc_gu, acc_d, ctrl, sh, only_xw, win);
+#define SZ_X3_CASE(KK, NN) if (K == KK && NTC == NN) return sz_x3_launch_k<KK, NN>(st, L, m, plan, x, acc_gu, acc_d, ctrl, sh);
     SZ_X3_CASE(2, 1) SZ_X3_CASE(2, 2) SZ_X3_CASE(2, 4) SZ_X3_CASE(3, 1) SZ_X3_CASE(3, 2) SZ_X3_CASE(3, 4) SZ_X3_CASE(4, 1) SZ_X3_CASE(4, 2) SZ_X3_CASE(4, 4)
 #undef SZ_X3_CASE
     return sz_fail(SZ_E_TYPE, "no streaming EXL3 kernel for K = %d, FF = %d", K, L->expert_ff);
@@ -997,17 +996,18 @@ extern "C" int sz_moe_verify(const sz_moe_layer* L, uint64_t x, int m, uint64_t 
 
 // ---- many rows at once (sz_moe_rows.cuh) ---------------------------------------------------------------------------------------------
 struct SzRowsScratch {
-    int64_t ctrl, logits, ridx, rw, cplan, cplan_sh, plan, xg, acc_gu, acc_d, total;
-    int64_t gu_row, d_row;   // i64 elements a slot
+    int64_t ctrl, logits, ridx, rw, cplan, cplan_sh, plan, frags, gu, dn, parts, total;
 };
-// One layout whatever the rows of a call (sized for SZ_ROWS_MAX): a scratch serves calls of any row count, and the tickets and the
-// error word stay where they were cleared - a layout that moved with the row count would put one call's tickets on another's data.
-static SzRowsScratch sz_rows_layout(const sz_moe_layer* L) {
+static int sz_rows_grid() { return sz_sm_count() < SZ_ROWS_MAXB ? sz_sm_count() : SZ_ROWS_MAXB; }
+// One layout whatever the rows of a call (sized for `cap`): a scratch serves calls of any row count, and what has to be found as the
+// call before left it - tickets, error word, sums at zero - stays where it was.
+static SzRowsScratch sz_rows_layout(const sz_moe_layer* L, int cap) {
     SzRowsScratch s;
     int64_t o = 0;
-    const int R = SZ_ROWS_MAX;
-    const int chunks = R / 8, W = SZ_ROWS_WIN + SZ_ROWS_SHWIN;
+    const int R = cap, chunks = R / 8;
+    const int64_t slots = (int64_t)R * (L->top_k + 1), pairs = (int64_t)R * L->top_k;
     const int64_t ffm = L->expert_ff > L->shared_ff ? L->expert_ff : L->shared_ff;
+    const int64_t groups = (L->n_expert < pairs ? L->n_expert : pairs) + pairs / SZ_ROWS_G + (R + SZ_ROWS_G - 1) / SZ_ROWS_G;
     s.ctrl = o; o = sz_up256(o + 64 * (int64_t)(chunks + 1));            // one block of 16 words a chunk (the router's ticket), then the expert kernels'
     s.logits = o; o = sz_up256(o + 4 * (int64_t)R * (L->n_expert + 1));
     s.ridx = o; o = sz_up256(o + 4 * (int64_t)R * L->top_k);
@@ -1015,60 +1015,61 @@ static SzRowsScratch sz_rows_layout(const sz_moe_layer* L) {
     s.cplan = o; o = sz_up256(o + (int64_t)sizeof(SzPlan) * chunks);
     s.cplan_sh = o; o = sz_up256(o + (int64_t)sizeof(SzPlan) * chunks);
     s.plan = o; o = sz_up256(o + (int64_t)sizeof(SzRowsPlan));
-    s.xg = o; o = sz_up256(o + 4 * (int64_t)W * SZ_ROWS_SLOTS * L->hidden);
-    s.gu_row = 2 * ffm; s.d_row = L->hidden;
-    s.acc_gu = o; o = sz_up256(o + 8 * (int64_t)W * SZ_ROWS_SLOTS * s.gu_row);
-    s.acc_d = o; o = sz_up256(o + 8 * (int64_t)W * SZ_ROWS_SLOTS * s.d_row);
+    s.frags = o; o = sz_up256(o + groups * (ffm / 128) * 8192);
+    s.gu = o; o = sz_up256(o + 4 * slots * 2 * ffm);
+    s.dn = o; o = sz_up256(o + 4 * slots * L->hidden);
+    s.parts = o; o = sz_up256(o + 8 * (int64_t)sz_rows_grid() * 2 * SZ_ROWS_G * 512);
     s.total = o;
     return s;
 }
 
-// zeroes the accumulators of the slots a window uses (grid (slots, windows), block 256)
-static __global__ void __launch_bounds__(256)
-sz_rows_zero_kernel(const SzRowsPlan* __restrict__ P, long long* __restrict__ acc_gu, long long gu_row, long long* __restrict__ acc_d, long long d_row) {
-    sz_pdl_wait();
-    sz_pdl_trigger();
-    const int s = blockIdx.x, w = blockIdx.y;
-    if (P->src[w][s] < 0) return;
-    uint4* a = (uint4*)(acc_gu + ((size_t)w * SZ_ROWS_SLOTS + s) * gu_row);
-    uint4* b = (uint4*)(acc_d + ((size_t)w * SZ_ROWS_SLOTS + s) * d_row);
-    for (long long i = threadIdx.x; i < gu_row / 2; i += 256) a[i] = make_uint4(0, 0, 0, 0);
-    for (long long i = threadIdx.x; i < d_row / 2; i += 256) b[i] = make_uint4(0, 0, 0, 0);
-}
-
-extern "C" int sz_moe_rows_scratch_bytes(const sz_moe_layer* L, int rows, int64_t* bytes) {
-    if (!L || !bytes) return sz_fail(SZ_E_ARG, "sz_moe_rows_scratch_bytes: null argument");
-    if (rows < 8 || rows > SZ_ROWS_MAX || rows % 8) return sz_fail(SZ_E_ARG, "sz_moe_rows: rows = %d (a multiple of 8 up to %d)", rows, SZ_ROWS_MAX);
-    *bytes = sz_rows_layout(L).total;
+template <int K, int TW>
+static int sz_rows_experts(cudaStream_t st, const sz_moe_layer* L, int slots, const SzRowsPlan* P, const float* x, u8* base, const SzRowsScratch& S, u32* err) {
+    using X = SzRowsX<K, TW>;
+    using XD = SzRowsX<K, 2>;
+    static bool set = false;
+    if (!set) {
+        SZ_CUDA(cudaFuncSetAttribute(sz_rows_gateup_kernel<K, TW>, cudaFuncAttributeMaxDynamicSharedMemorySize, X::GU_SMEM));
+        SZ_CUDA(cudaFuncSetAttribute(sz_rows_down_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, XD::DN_SMEM));
+        set = true;
+    }
+    const int H = L->hidden, FF = L->expert_ff, KB = FF / 128;
+    const dim3 grid(sz_rows_grid());
+    float *gu = (float*)(base + S.gu), *dn = (float*)(base + S.dn);
+    long long* parts = (long long*)(base + S.parts);    // (the gate / up kernel's are read by act before the down kernel writes its own)
+    SZ_CUDA(sz_launch("rows_gateup", sz_rows_gateup_kernel<K, TW>, grid, dim3(32 * (SZ_ROWS_CW + SZ_ROWS_PW)), X::GU_SMEM, st, true, P, (const u8*)L->gate,
+                      (u64)L->gate_stride, (const u8*)L->up, (u64)L->up_stride, (const u8*)L->sh_gate, (const u8*)L->sh_up, x, H, FF, gu, parts, err));
+    SZ_CUDA(sz_launch("rows_act", sz_rows_act_kernel, dim3((slots * KB + 7) / 8), dim3(256), 0, st, true, P, (const u8*)L->gate, (u64)L->gate_stride,
+                      (const u8*)L->up, (u64)L->up_stride, (const u8*)L->down, (u64)L->down_stride, (const u8*)L->sh_gate, (const u8*)L->sh_up, (const u8*)L->sh_down,
+                      H, FF, slots, (const float*)gu, (const long long*)parts, (uint4*)(base + S.frags)));
+    SZ_CUDA(sz_launch("rows_down", sz_rows_down_kernel<K>, grid, dim3(32 * (SZ_ROWS_CW + 1)), XD::DN_SMEM, st, true, P, (const u8*)L->down, (u64)L->down_stride,
+                      (const u8*)L->sh_down, H, FF, (const uint4*)(base + S.frags), dn, parts, err));
     return SZ_OK;
 }
 
-// y[j] = moe(x[j]) for j < rows; x, y: f32 [rows][hidden].  EXL3 experts (routed and shared); every distinct expert is decoded once.
-// route_idx / route_w: as sz_moe_verify's, [rows][top_k], or 0.
-extern "C" int sz_moe_rows(const sz_moe_layer* L, uint64_t x, int rows, uint64_t y, uint64_t route_idx, uint64_t route_w, uint64_t scratch,
-                           int64_t scratch_bytes, uint64_t stream) {
+// The rows of one call (cap: what the scratch was laid out for).
+static int sz_rows_run(const sz_moe_layer* L, uint64_t x, int rows, uint64_t y, uint64_t route_idx, uint64_t route_w, uint64_t scratch, int64_t scratch_bytes, int cap,
+                       uint64_t stream) {
     int rc = sz_moe_check(L, 8);
     if (rc) return rc;
-    if (rows < 8 || rows > SZ_ROWS_MAX || rows % 8) return sz_fail(SZ_E_ARG, "sz_moe_rows: rows = %d (a multiple of 8 up to %d)", rows, SZ_ROWS_MAX);
+    if (rows < 8 || rows > cap || rows % 8) return sz_fail(SZ_E_ARG, "sz_moe_rows: rows = %d (a multiple of 8 up to %d)", rows, cap);
     const SzFast fast = sz_fast_path(L);
     if (!fast.exl3 || L->ep_count > 0 || (L->shared_ff > 0 && !fast.shared_fused))
         return sz_fail(SZ_E_TYPE, "sz_moe_rows: EXL3 experts of the streaming kernels' shapes, a shared expert of the same width and type, no expert sharding");
     if (!x || !y || !sz_aligned16(x) || !sz_aligned16(y)) return sz_fail(SZ_E_ARG, "sz_moe_rows: x and y must be non-null and 16-byte aligned");
-    const SzRowsScratch S = sz_rows_layout(L);
+    const SzRowsScratch S = sz_rows_layout(L, cap);
     if (!scratch || (scratch & 255)) return sz_fail(SZ_E_ARG, "scratch must be 256-byte aligned");
     if (scratch_bytes < S.total) return sz_fail(SZ_E_SCRATCH, "scratch of %lld bytes, %lld needed", (long long)scratch_bytes, (long long)S.total);
     cudaStream_t st = (cudaStream_t)stream;
     u8* base = (u8*)scratch;
-    const int H = L->hidden, chunks = rows / 8, W = SZ_ROWS_WIN + SZ_ROWS_SHWIN;
+    const int H = L->hidden, chunks = rows / 8;
     const bool shared = L->shared_ff > 0;
     u32* ctrl = (u32*)(base + S.ctrl);
-    u32* ctrl_x = ctrl + 16 * (SZ_ROWS_MAX / 8);   // the expert kernels' error word lives in word 1 of the block after the chunks'
+    u32* err = ctrl + 16 * (cap / 8) + 1;
     float* logits = (float*)(base + S.logits);
     int32_t* ridx = (int32_t*)(base + S.ridx);
     double* rw = (double*)(base + S.rw);
     SzRowsPlan* P = (SzRowsPlan*)(base + S.plan);
-    float* xg = (float*)(base + S.xg);
-    long long *acc_gu = (long long*)(base + S.acc_gu), *acc_d = (long long*)(base + S.acc_d);
     {   // routing: 8 rows a block row of the verify pass's router kernel (the chunks' own plans are written and not used)
         const int route_rows = L->n_expert + (shared ? 1 : 0);
         const dim3 grid((route_rows + SZ_ROUTE_RB - 1) / SZ_ROUTE_RB, chunks), block(SZ_ROUTE_THREADS);
@@ -1082,50 +1083,44 @@ extern "C" int sz_moe_rows(const sz_moe_layer* L, uint64_t x, int rows, uint64_t
 #undef SZ_ROWS_ROUTE
         SZ_CUDA(e);
     }
-    SZ_CUDA(sz_launch("rows_plan", sz_rows_plan_kernel, dim3(1), dim3(1024), 0, st, true, (const int32_t*)ridx, rows, (int)L->top_k, (int)L->n_expert,
-                      shared ? 1 : 0, P));
-    SZ_CUDA(sz_launch("rows_zero", sz_rows_zero_kernel, dim3(SZ_ROWS_SLOTS, W), dim3(256), 0, st, true, (const SzRowsPlan*)P, acc_gu, (long long)S.gu_row, acc_d,
-                      (long long)S.d_row));
-    SZ_CUDA(sz_launch("rows_gather", sz_rows_gather_kernel, dim3(SZ_ROWS_SLOTS, W), dim3(256), 0, st, true, (const float*)x, H, (const SzRowsPlan*)P, xg));
-    // the experts: every window a block row of one gate/up and one down launch (how many windows the routing needs is known on the
-    // device only: the blocks of a window without groups return at once).  SZ_ROWS_SERIAL=1: a launch pair a window, one after the
-    // other (the second form; same bits).
-    const size_t win_plan = offsetof(SzRowsPlan, win);
-    const char* ser = getenv("SZ_ROWS_SERIAL");   // (read at every call: a test switches it inside one process)
-    if (ser && atoi(ser) != 0) {
-        for (int w = 0; w < SZ_ROWS_WIN; w++) {
-            const SzPlan* pw = (const SzPlan*)((u8*)P + win_plan + (size_t)w * sizeof(SzPlan));
-            if ((rc = sz_x3_launch(st, L, 8, pw, xg + (size_t)w * SZ_ROWS_SLOTS * H, acc_gu + (size_t)w * SZ_ROWS_SLOTS * S.gu_row,
-                                   acc_d + (size_t)w * SZ_ROWS_SLOTS * S.d_row, ctrl_x, false, true)))
-                return rc;
-        }
-    } else {
-        SzXWindows win;
-        win.n = SZ_ROWS_WIN; win.x = (long long)SZ_ROWS_SLOTS * H; win.gu = (long long)SZ_ROWS_SLOTS * S.gu_row; win.d = (long long)SZ_ROWS_SLOTS * S.d_row;
-        if ((rc = sz_x3_launch(st, L, 8, (const SzPlan*)((u8*)P + win_plan), xg, acc_gu, acc_d, ctrl_x, false, true, win))) return rc;
-    }
-    if (shared) {   // the shared expert as expert 0 of a layer of one
-        sz_moe_layer Ls = *L;
-        Ls.gate = L->sh_gate; Ls.up = L->sh_up; Ls.down = L->sh_down;
-        Ls.gate_stride = Ls.up_stride = Ls.down_stride = 0;
-        Ls.expert_ff = L->shared_ff; Ls.expert_type = L->shared_type;
-        const int w = SZ_ROWS_WIN;
-        const SzPlan* pw = (const SzPlan*)((u8*)P + win_plan + (size_t)w * sizeof(SzPlan));
-        if ((rc = sz_x3_launch(st, &Ls, 8, pw, xg + (size_t)w * SZ_ROWS_SLOTS * H, acc_gu + (size_t)w * SZ_ROWS_SLOTS * S.gu_row,
-                               acc_d + (size_t)w * SZ_ROWS_SLOTS * S.d_row, ctrl_x, false, true)))
-            return rc;
-    }
-    SZ_CUDA(sz_launch("rows_combine", sz_rows_combine_kernel, dim3(rows * (H / 128)), dim3((L->top_k + 1) * 32), 0, st, true, (const long long*)acc_d,
-                      (const SzRowsPlan*)P, (const int32_t*)ridx, (const double*)rw, (const u8*)L->down, (u64)L->down_stride, (const u8*)L->sh_down,
-                      (const float*)logits, (int)L->n_expert, (int)L->top_k, H, (int)L->expert_ff, (int)L->shared_ff, shared ? 1 : 0, (float*)y));
+    const size_t pmem = (size_t)L->n_expert * (SZ_ROWS_CAP / 32) * 4;
+    static bool set = false;
+    if (!set) { SZ_CUDA(cudaFuncSetAttribute(sz_rows_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SZ_MAX_EXPERTS * (SZ_ROWS_CAP / 32) * 4)); set = true; }
+    SZ_CUDA(sz_launch("rows_plan", sz_rows_plan_kernel, dim3(1), dim3(1024), pmem, st, true, (const int32_t*)ridx, rows, (int)L->top_k, (int)L->n_expert,
+                      shared ? 1 : 0, 2 * (H / 128), H / 128, H / 512 * (L->expert_ff / 128), (int)L->expert_ff / 128, sz_rows_grid(), P));
+    const int slots = rows * (L->top_k + (shared ? 1 : 0));
+    rc = SZ_E_TYPE;
+#define SZ_ROWS_K(KK)                                                                                                                              \
+    if (L->expert_type == 1020 + KK) rc = L->expert_ff % 256 == 0 ? sz_rows_experts<KK, 2>(st, L, slots, P, (const float*)x, base, S, err)      \
+                                                                  : sz_rows_experts<KK, 1>(st, L, slots, P, (const float*)x, base, S, err);
+    SZ_ROWS_K(2) SZ_ROWS_K(3) SZ_ROWS_K(4)
+#undef SZ_ROWS_K
+    if (rc) return rc;
+    SZ_CUDA(sz_launch("rows_combine", sz_rows_combine_kernel, dim3(rows * (H / 128)), dim3((L->top_k + 1) * 32), 0, st, true, (const float*)(base + S.dn),
+                      (const long long*)(base + S.parts), (const SzRowsPlan*)P, (const int32_t*)ridx, (const double*)rw, (const u8*)L->down, (u64)L->down_stride, (const u8*)L->sh_down,
+                      (const float*)logits, (int)L->n_expert, (int)L->top_k, rows, H, (int)L->expert_ff, (int)L->shared_ff, shared ? 1 : 0, (float*)y));
     return SZ_OK;
 }
 
-// Clears the scratch's counters (once after allocation, and after a failed call); code != null: reads the expert kernels' error
-// word and the plan's overflow flag instead (synchronises).
+extern "C" int sz_moe_rows_scratch_bytes(const sz_moe_layer* L, int rows, int64_t* bytes) {
+    if (!L || !bytes) return sz_fail(SZ_E_ARG, "sz_moe_rows_scratch_bytes: null argument");
+    if (rows < 8 || rows > SZ_ROWS_MAX || rows % 8) return sz_fail(SZ_E_ARG, "sz_moe_rows: rows = %d (a multiple of 8 up to %d)", rows, SZ_ROWS_MAX);
+    *bytes = sz_rows_layout(L, SZ_ROWS_MAX).total;
+    return SZ_OK;
+}
+
+// y[j] = moe(x[j]) for j < rows; x, y: f32 [rows][hidden].  EXL3 experts (routed and shared); every distinct expert is decoded once.
+// route_idx / route_w: as sz_moe_verify's, [rows][top_k], or 0.
+extern "C" int sz_moe_rows(const sz_moe_layer* L, uint64_t x, int rows, uint64_t y, uint64_t route_idx, uint64_t route_w, uint64_t scratch,
+                           int64_t scratch_bytes, uint64_t stream) {
+    return sz_rows_run(L, x, rows, y, route_idx, route_w, scratch, scratch_bytes, SZ_ROWS_MAX, stream);
+}
+
+// Clears the scratch's counters (once after allocation, and after a failed call); code != null: reads the expert kernels'
+// error word and the plan's overflow flag instead (synchronises).
 extern "C" int sz_moe_rows_status(const sz_moe_layer* L, int rows, uint64_t scratch, int* code, uint64_t stream) {
     if (!L || !scratch || rows < 8 || rows > SZ_ROWS_MAX || rows % 8) return sz_fail(SZ_E_ARG, "sz_moe_rows_status: bad argument");
-    const SzRowsScratch S = sz_rows_layout(L);
+    const SzRowsScratch S = sz_rows_layout(L, SZ_ROWS_MAX);
     cudaStream_t st = (cudaStream_t)stream;
     u8* base = (u8*)scratch;
     if (!code) { SZ_CUDA(cudaMemsetAsync(base + S.ctrl, 0, (size_t)(S.logits - S.ctrl), st)); return SZ_OK; }
@@ -1134,7 +1129,7 @@ extern "C" int sz_moe_rows_status(const sz_moe_layer* L, int rows, uint64_t scra
     SZ_CUDA(cudaMemcpyAsync(&err, base + S.ctrl + 64 * (SZ_ROWS_MAX / 8) + 4, 4, cudaMemcpyDeviceToHost, st));
     SZ_CUDA(cudaMemcpyAsync(&over, base + S.plan + offsetof(SzRowsPlan, overflow), 4, cudaMemcpyDeviceToHost, st));
     SZ_CUDA(cudaStreamSynchronize(st));
-    *code = (int)(err ? 1 : 0) | (over & 1 ? 2 : 0) | (over & 4);
+    *code = (int)(err ? 1 : 0) | (over & 4);
     return SZ_OK;
 }
 

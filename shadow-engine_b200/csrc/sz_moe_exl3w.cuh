@@ -6,8 +6,7 @@
 // two sides meet only at mbarriers - a `full` barrier a stage (the copy's bytes have landed and the fragments are written) and an
 // `empty` barrier a stage (all eight consumer warps are done with it) - so the consumers never stop at a block-wide barrier and
 // never wait for the one thread that issues copies.  The decode itself is leaner: a lane's 8 windows of a tile span two 32-bit
-// words at every bit rate this kernel takes (2, 3, 4 bits), so it loads two words instead of four, and the integer byte-sum MMA
-// takes its 0x6400 start value from registers that are set once instead of being re-initialised for every tile.
+// words at every bit rate this kernel takes (2, 3, 4 bits), so it loads two words instead of four.
 #pragma once
 
 #include "sz_moe_exl3.cuh"
@@ -54,37 +53,24 @@ struct SzExl3Two {
         for (int j = 0; j < 8; j++) {
             const int pos = j * K;
             if (pos == 0) st[j] = a0 >> 16;
-            else if (pos <= 16) st[j] = (a0 >> (16 - pos)) & 0xffffu;
+            else if (pos <= 16) { u32 p; asm("mul.lo.u32 %0, %1, %2;" : "=r"(p) : "r"(a0), "r"(1u << pos)); st[j] = p >> 16; }
             else st[j] = __funnelshift_l(a1, a0, pos) >> 16;
         }
     }
 };
 
-// Byte sums of four products on the integer tensor pipe (see sz_bytesum4), the 0x6400 start value read from `base` (four registers
-// that hold it): the accumulator input is a separate operand, so nothing has to be re-initialised per call.
-__device__ __forceinline__ void sz_bytesum4c(const u32* x, u32 sel0, u32 sel1, const u32* base, u32* c) {
-    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
-                 : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
-                 : "r"(x[0]), "r"(x[2]), "r"(x[1]), "r"(x[3]), "r"(sel0), "r"(sel1), "r"(base[0]), "r"(base[1]), "r"(base[2]), "r"(base[3]));
-}
-
-// What a consumer lane keeps for the whole kernel.
+// The decode's instructions are spread over the pipes.  Measured from shared memory alone, 16 warps a multiprocessor, in cycles a tile
+// and scheduler: windows by shift and mask with the byte sums on the integer tensor pipe 63.1 (the ALU pipe, at two cycles an
+// instruction, has 21 of the tile's 48); byte sums by dp4a 60.9; windows of the first word by a multiplication that puts them on top
+// and one shift, too, 59.8, in 52 registers instead of 83.  In the many-row gate / up kernel 400 -> 369 us.
 template <int K>
 struct SzXWLane {
     typename SzExl3Two<K>::Lane L;
-    u32 sel0, sel1;
-    u32 base[4];
 };
 template <int K>
 __device__ __forceinline__ SzXWLane<K> sz_xw_lane(int lane) {
     SzXWLane<K> s;
     s.L = SzExl3Two<K>::lane_setup(lane);
-    const int n = lane >> 2, q = lane & 3;
-    s.sel0 = ((n & 1) == 0 && (n >> 1) == q) ? 0x01010101u : 0u;
-    s.sel1 = ((n & 1) == 1 && (n >> 1) == q) ? 0x01010101u : 0u;
-    // (an opaque move: the compiler must keep four registers for the accumulator operand rather than re-materialise the constant)
-#pragma unroll
-    for (int i = 0; i < 4; i++) asm volatile("mov.u32 %0, 0x6400;" : "=r"(s.base[i]));
     return s;
 }
 
@@ -99,8 +85,8 @@ __device__ __forceinline__ void sz_xw_afrag(const u32* tile, const SzXWLane<K>& 
 #pragma unroll
     for (int i = 0; i < 8; i++) x[i] = st[i] * 0x83DCD12Du;
     u32 c[8];
-    sz_bytesum4c(x, S.sel0, S.sel1, S.base, c);
-    sz_bytesum4c(x + 4, S.sel0, S.sel1, S.base, c + 4);
+#pragma unroll
+    for (int i = 0; i < 8; i++) c[i] = __dp4a(x[i], 0x01010101u, 0x6400u);
     u32 p[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) {
@@ -113,8 +99,7 @@ __device__ __forceinline__ void sz_xw_afrag(const u32* tile, const SzXWLane<K>& 
 
 // Decodes and multiplies one staged unit (8 tile rows x 8 NTC tile columns): warp w takes tile columns w NTC .. w NTC + NTC - 1.
 // c[tc] = outputs (w NTC + tc) 16 + {g, g + 8} for rows 2 q, 2 q + 1.
-// The decode loop is fully unrolled: rolled over the tile rows it ran 6% slower, and moving the byte-sum packing or the
-// word-crossing windows from the ALU pipe to multiply-adds on the FMA pipe another 2 - 4% slower (measured on the benchmark's shape).
+// The decode loop is fully unrolled: rolled over the tile rows it ran 6% slower.
 template <int K, int TW>
 __device__ __forceinline__ void sz_xw_compute(const u8* stage, const uint4* frag, int warp, int lane, const SzXWLane<K>& S, float (*c)[4]) {
 #pragma unroll
@@ -221,15 +206,9 @@ template <int K, int NTC, int TW, int OCC>
 __global__ void __launch_bounds__(SZ_XW_THREADS, OCC)
 sz_xw_gateup_kernel(const SzPlan* __restrict__ plan, const u8* __restrict__ gate, u64 gstride, const u8* __restrict__ up, u64 ustride,
                     const u8* __restrict__ sh_gate, const u8* __restrict__ sh_up, const float* __restrict__ x, int m, int H, int top_k,
-                    long long* __restrict__ acc, u32* __restrict__ ctrl, long long win_x, long long win_acc) {
+                    long long* __restrict__ acc, u32* __restrict__ ctrl) {
     using X = SzXW<K, TW, OCC>;
     constexpr int FF = 128 * NTC, S = X::STAGES, NCH = NTC / TW;
-    // grid.y > 1: block row w works on plan w of an array of plans, with its own inputs and sums (win_x, win_acc: elements from one
-    // window's to the next's); a window without groups is left at once
-    if (gridDim.y > 1) {
-        plan += blockIdx.y; x += blockIdx.y * win_x; acc += blockIdx.y * win_acc;
-        if (plan->n_groups == 0 && !sh_gate) return;
-    }
     static_assert(NTC % TW == 0, "column chunks tile the matrix");
     extern __shared__ __align__(128) u8 smem[];
     SzXWRing<K, TW, OCC> R;
@@ -342,13 +321,9 @@ __global__ void __launch_bounds__(SZ_XW_THREADS, OCC)
 sz_xw_down_kernel(const SzPlan* __restrict__ plan, const u8* __restrict__ gate, u64 gstride, const u8* __restrict__ up, u64 ustride,
                   const u8* __restrict__ down, u64 dstride, const u8* __restrict__ sh_gate, const u8* __restrict__ sh_up,
                   const u8* __restrict__ sh_down, int m, int H, int FF, int top_k, const long long* __restrict__ acc,
-                  long long* __restrict__ out, u32* __restrict__ ctrl, long long win_acc, long long win_out) {
+                  long long* __restrict__ out, u32* __restrict__ ctrl) {
     using X = SzXW<K, TW, OCC>;
     constexpr int S = X::STAGES;
-    if (gridDim.y > 1) {   // (as the gate / up kernel)
-        plan += blockIdx.y; acc += blockIdx.y * win_acc; out += blockIdx.y * win_out;
-        if (plan->n_groups == 0 && !sh_down) return;
-    }
     extern __shared__ __align__(128) u8 smem[];
     SzXWRing<K, TW, OCC> R;
     R.init(smem);

@@ -104,7 +104,7 @@ class MoeLayer:
         assert x.is_cuda and x.dtype == torch.float32 and x.is_contiguous() and x.shape[1] == self.shape["hidden"]
         st = (stream or torch.cuda.current_stream(self.device)).cuda_stream
         have = getattr(self, "_rows_scratch", None)
-        if have is None or have[0] < rows:
+        if have is None:   # one size and one layout whatever the rows of a call
             n = C.c_int64()
             szlib.check(self.lib.sz_moe_rows_scratch_bytes(C.byref(self.c), rows, C.byref(n)))
             buf = torch.empty(n.value + 256, dtype=torch.uint8, device=self.device)
@@ -119,14 +119,7 @@ class MoeLayer:
             a, b = ridx.data_ptr(), rw.data_ptr()
         else:
             a = b = 0
-        if have[0] != rows:   # the layout depends on the row count: a smaller batch gets a scratch of its own size class
-            n = C.c_int64()
-            szlib.check(self.lib.sz_moe_rows_scratch_bytes(C.byref(self.c), rows, C.byref(n)))
-            szlib.check(self.lib.sz_moe_rows_status(C.byref(self.c), rows, have[2], None, st))
-            nbytes = n.value
-        else:
-            nbytes = have[3]
-        szlib.check(self.lib.sz_moe_rows(C.byref(self.c), x.data_ptr(), rows, y.data_ptr(), a, b, have[2], nbytes, st))
+        szlib.check(self.lib.sz_moe_rows(C.byref(self.c), x.data_ptr(), rows, y.data_ptr(), a, b, have[2], have[3], st))
         return (y, ridx, rw) if want_routing else y
 
     def moe_rows_status(self, rows, stream=None):
