@@ -156,6 +156,19 @@ __device__ __forceinline__ double sz_rsqrt64(double v) {
 
 __device__ __forceinline__ float sz_silu(float x) { return x * sz_sigmoid(x); }
 
+// ---- thread-block clusters --------------------------------------------------------------------------------------------------
+__device__ __forceinline__ void sz_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// the f32 at `p` (an address in this block's shared memory) as block `rank` of the cluster has it
+__device__ __forceinline__ float sz_cluster_ld(const float* p, int rank) {
+    u32 a;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((u32)__cvta_generic_to_shared(p)), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
+}
+
 // ---- mbarrier + bulk async copy (TMA engine, untiled form) ---------------------------------------------------------------
 __device__ __forceinline__ u32 sz_smem_addr(const void* p) { return (u32)__cvta_generic_to_shared(p); }
 

@@ -1048,7 +1048,8 @@ static int sz_rows_experts(cudaStream_t st, const sz_moe_layer* L, int slots, co
 }
 
 // The rows of one call (cap: what the scratch was laid out for).
-static int sz_rows_run(const sz_moe_layer* L, uint64_t x, int rows, uint64_t y, uint64_t route_idx, uint64_t route_w, uint64_t scratch, int64_t scratch_bytes, int cap,
+// live: the rows that count (the others only pad the routing to whole block rows: they choose no experts and get no output)
+static int sz_rows_run(const sz_moe_layer* L, uint64_t x, int rows, int live, uint64_t y, uint64_t route_idx, uint64_t route_w, uint64_t scratch, int64_t scratch_bytes, int cap,
                        uint64_t stream) {
     int rc = sz_moe_check(L, 8);
     if (rc) return rc;
@@ -1086,9 +1087,9 @@ static int sz_rows_run(const sz_moe_layer* L, uint64_t x, int rows, uint64_t y, 
     const size_t pmem = (size_t)L->n_expert * (SZ_ROWS_CAP / 32) * 4;
     static bool set = false;
     if (!set) { SZ_CUDA(cudaFuncSetAttribute(sz_rows_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SZ_MAX_EXPERTS * (SZ_ROWS_CAP / 32) * 4)); set = true; }
-    SZ_CUDA(sz_launch("rows_plan", sz_rows_plan_kernel, dim3(1), dim3(1024), pmem, st, true, (const int32_t*)ridx, rows, (int)L->top_k, (int)L->n_expert,
+    SZ_CUDA(sz_launch("rows_plan", sz_rows_plan_kernel, dim3(1), dim3(1024), pmem, st, true, (const int32_t*)ridx, live, (int)L->top_k, (int)L->n_expert,
                       shared ? 1 : 0, 2 * (H / 128), H / 128, H / 512 * (L->expert_ff / 128), (int)L->expert_ff / 128, sz_rows_grid(), P));
-    const int slots = rows * (L->top_k + (shared ? 1 : 0));
+    const int slots = live * (L->top_k + (shared ? 1 : 0));
     rc = SZ_E_TYPE;
 #define SZ_ROWS_K(KK)                                                                                                                              \
     if (L->expert_type == 1020 + KK) rc = L->expert_ff % 256 == 0 ? sz_rows_experts<KK, 2>(st, L, slots, P, (const float*)x, base, S, err)      \
@@ -1096,9 +1097,9 @@ static int sz_rows_run(const sz_moe_layer* L, uint64_t x, int rows, uint64_t y, 
     SZ_ROWS_K(2) SZ_ROWS_K(3) SZ_ROWS_K(4)
 #undef SZ_ROWS_K
     if (rc) return rc;
-    SZ_CUDA(sz_launch("rows_combine", sz_rows_combine_kernel, dim3(rows * (H / 128)), dim3((L->top_k + 1) * 32), 0, st, true, (const float*)(base + S.dn),
+    SZ_CUDA(sz_launch("rows_combine", sz_rows_combine_kernel, dim3(live * (H / 128)), dim3((L->top_k + 1) * 32), 0, st, true, (const float*)(base + S.dn),
                       (const long long*)(base + S.parts), (const SzRowsPlan*)P, (const int32_t*)ridx, (const double*)rw, (const u8*)L->down, (u64)L->down_stride, (const u8*)L->sh_down,
-                      (const float*)logits, (int)L->n_expert, (int)L->top_k, rows, H, (int)L->expert_ff, (int)L->shared_ff, shared ? 1 : 0, (float*)y));
+                      (const float*)logits, (int)L->n_expert, (int)L->top_k, live, H, (int)L->expert_ff, (int)L->shared_ff, shared ? 1 : 0, (float*)y));
     return SZ_OK;
 }
 
@@ -1113,7 +1114,16 @@ extern "C" int sz_moe_rows_scratch_bytes(const sz_moe_layer* L, int rows, int64_
 // route_idx / route_w: as sz_moe_verify's, [rows][top_k], or 0.
 extern "C" int sz_moe_rows(const sz_moe_layer* L, uint64_t x, int rows, uint64_t y, uint64_t route_idx, uint64_t route_w, uint64_t scratch,
                            int64_t scratch_bytes, uint64_t stream) {
-    return sz_rows_run(L, x, rows, y, route_idx, route_w, scratch, scratch_bytes, SZ_ROWS_MAX, stream);
+    return sz_rows_run(L, x, rows, rows, y, route_idx, route_w, scratch, scratch_bytes, SZ_ROWS_MAX, stream);
+}
+
+// The form inside a session's step: `live` of the rows count; and whether a layer has it.
+int sz_moe_rows_live(const sz_moe_layer* L, uint64_t x, int rows, int live, uint64_t y, uint64_t scratch, int64_t scratch_bytes, uint64_t stream) {
+    return sz_rows_run(L, x, rows, live, y, 0, 0, scratch, scratch_bytes, SZ_ROWS_MAX, stream);
+}
+bool sz_moe_rows_takes(const sz_moe_layer* L) {
+    const SzFast f = sz_fast_path(L);
+    return f.exl3 && L->ep_count <= 0 && (L->shared_ff == 0 || f.shared_fused);
 }
 
 // Clears the scratch's counters (once after allocation, and after a failed call); code != null: reads the expert kernels'

@@ -7,6 +7,7 @@
 // recurrences for the kept rows from the pass's saved inputs - the reference's replay (session.rs:6245-6268) - into `cur ^ 1`,
 // then the buffers swap.  The KV cache is append-only: rejected positions are overwritten by the next pass.
 #include "sz_session_kernels.cuh"
+#include "sz_session_rows.cuh"
 #include "sz_indexer.cuh"
 #include "sz_ple.cuh"
 
@@ -32,6 +33,8 @@ int sz_ep_p2p_graph_refs(int delta);  // ... that hold the addresses of the atta
 int sz_ep_generation(void);           // changes whenever the exchange set-up does
 extern "C" int sz_ep_world(void);
 extern "C" int sz_ep_p2p_world(void);
+int sz_moe_rows_live(const sz_moe_layer* L, uint64_t x, int rows, int live, uint64_t y, uint64_t scratch, int64_t scratch_bytes, uint64_t stream);   // sz_moe.cu
+bool sz_moe_rows_takes(const sz_moe_layer* L);
 
 struct sz_session {
     sz_model model;
@@ -42,6 +45,9 @@ struct sz_session {
     int cur;          // which state buffer is current
     int last_m;       // rows of the last pass (0: none pending)
     int want_routes;
+    int ws_rows = 0;        // rows of a prompt's chunk the session has room for (0: prompts go in passes)
+    u8* ws = nullptr;
+    int64_t ws_bytes = 0;
     // device memory (all inside the caller's block)
     u8* base;
     int64_t bytes;
@@ -54,7 +60,7 @@ struct sz_session {
     int hc_n;             // reads launched so far in the pass being built (buffer parities are static per launch)
     float *d_xin, *d_z, *d_b, *d_a, *d_xc, *d_beta, *d_decay, *d_og;   // per-layer saved: xin, xc, beta, decay [n_delta][8][...]
     float *S[2], *conv[2];
-    float *a_qg, *a_k, *a_v, *a_q, *a_gate, *a_o, *a_part;
+    float *a_qg, *a_k, *a_v, *a_q, *a_o, *a_part;
     u8 *kc, *vc;
     float* logits;
     u64* tk_tmp;
@@ -105,13 +111,13 @@ struct sz_session {
 static int sz_is_attn(const sz_model_config& c, int l) { return l % c.attn_interval == c.attn_interval - 1; }
 
 struct SzSessLayout {
-    int64_t r, r2, hc_acc, rope, rn, hdown, mix, u, g, y, d_xin, d_z, d_b, d_a, d_xc, d_beta, d_decay, d_og, S0, S1, conv0, conv1, a_qg, a_k, a_v, a_q, a_gate,
+    int64_t rows_ws, rows_ws_bytes, r, r2, hc_acc, rope, rn, hdown, mix, u, g, y, d_xin, d_z, d_b, d_a, d_xc, d_beta, d_decay, d_og, S0, S1, conv0, conv1, a_qg, a_k, a_v, a_q,
         a_o, a_part, kc, vc, logits, tk_tmp, top, ids, res, state, routes, route_w, moe, head_q2, head_sc, head_work, fork, i_q, i_k, i_qn, i_raw, i_blocks, i_scores, i_sel, i_list, i_count, i_trace, p_e, p_key, p_val, p_gv, p_gvn, p_hist, p_tail, total;
     int64_t p_hist_bytes;
     int64_t i_raw_layer, i_blocks_layer;   // bytes of one attention layer's raw-key and pooled-key caches
     int i_ctx_blocks, i_words;
     int64_t moe_bytes, S_bytes, conv_bytes, kv_bytes, head_work_bytes;
-    int splits, splits2;
+    int splits, splits2, ws_rows;
 };
 
 // output.weight as an EXL3 blob: the head is sz_head_top's (dense, or screened by the 2-bit proxy with SZ_HEAD_PROXY).
@@ -133,6 +139,9 @@ static int sz_head_describe(const sz_model* m, int flags, sz_head* h) {
 
 static int64_t up256(int64_t v) { return (v + 255) & ~(int64_t)255; }
 
+struct SzBatchScratch;
+static int sz_rows_ws_plan(const sz_model* m, int ctx, int flags, int* rows, int64_t* bytes);
+
 static int sz_sess_layout(const sz_model* m, int ctx, int flags, SzSessLayout* L) {
     const sz_model_config& c = m->cfg;
     const int64_t M = SZ_MAX_VERIFY, H = c.hidden, C = c.streams, CH = C * H;
@@ -151,7 +160,7 @@ static int sz_sess_layout(const sz_model* m, int ctx, int flags, SzSessLayout* L
     L->conv_bytes = 4 * nd * (c.conv_k - 1) * ch;
     L->S0 = take(L->S_bytes); L->S1 = take(L->S_bytes); L->conv0 = take(L->conv_bytes); L->conv1 = take(L->conv_bytes);
     L->a_qg = take(4 * M * 2 * qd); L->a_k = take(4 * M * kvd); L->a_v = take(4 * M * kvd); L->a_q = take(4 * M * qd);
-    L->a_gate = take(4 * M * qd); L->a_o = take(4 * M * qd);
+    L->a_o = take(4 * M * qd);
     // enough (head, row, split) blocks to fill the GPU twice over, at least 256 positions a split
     int splits = 1;
     if (c.n_head > 0) {
@@ -228,6 +237,12 @@ static int sz_sess_layout(const sz_model* m, int ctx, int flags, SzSessLayout* L
             L->head_sc = take(sc);
         }
     }
+    // what a prompt's chunks need beside a pass's buffers
+    L->rows_ws = 0; L->rows_ws_bytes = 0;
+    int ws_rows = 0;
+    if ((hrc = sz_rows_ws_plan(m, ctx, flags, &ws_rows, &L->rows_ws_bytes))) return hrc;
+    L->ws_rows = ws_rows;
+    if (ws_rows > 0) L->rows_ws = take(L->rows_ws_bytes);
     L->total = o;
     return SZ_OK;
 }
@@ -424,7 +439,7 @@ extern "C" int sz_session_create(const sz_model* m, int ctx, int flags, uint64_t
     s->d_xc = (float*)(b + L.d_xc); s->d_beta = (float*)(b + L.d_beta); s->d_decay = (float*)(b + L.d_decay); s->d_og = (float*)(b + L.d_og);
     s->S[0] = (float*)(b + L.S0); s->S[1] = (float*)(b + L.S1); s->conv[0] = (float*)(b + L.conv0); s->conv[1] = (float*)(b + L.conv1);
     s->a_qg = (float*)(b + L.a_qg); s->a_k = (float*)(b + L.a_k); s->a_v = (float*)(b + L.a_v); s->a_q = (float*)(b + L.a_q);
-    s->a_gate = (float*)(b + L.a_gate); s->a_o = (float*)(b + L.a_o); s->a_part = (float*)(b + L.a_part);
+    s->a_o = (float*)(b + L.a_o); s->a_part = (float*)(b + L.a_part);
     s->kc = b + L.kc; s->vc = b + L.vc;
     s->logits = (float*)(b + L.logits); s->tk_tmp = (u64*)(b + L.tk_tmp); s->top = (u32*)(b + L.top);
     s->ids = (int32_t*)(b + L.ids); s->res = (int32_t*)(b + L.res); s->state = (int32_t*)(b + L.state); s->routes = (int32_t*)(b + L.routes); s->route_w = (double*)(b + L.route_w);
@@ -441,6 +456,8 @@ extern "C" int sz_session_create(const sz_model* m, int ctx, int flags, uint64_t
         s->i_raw_layer = L.i_raw_layer; s->i_blocks_layer = L.i_blocks_layer; s->i_ctx_blocks = L.i_ctx_blocks; s->i_words = L.i_words;
     }
     s->attn_splits = L.splits; s->attn_splits2 = L.splits2;
+    s->ws_rows = L.ws_rows; s->ws = b + L.rows_ws; s->ws_bytes = L.rows_ws_bytes;
+    if (s->ws_rows > 0 && (rc = sz_batch_scratch_init(&s->model, s->ws_rows, (uint64_t)s->ws, stream))) { delete s; return rc; }
     if ((rc = sz_head_describe(m, flags, &s->head))) { delete s; return rc; }
     if (s->head.rows > 0) {
         s->head.work = (uint64_t)(b + L.head_work); s->head.work_bytes = L.head_work_bytes;
@@ -799,32 +816,7 @@ static int sz_hc_read_rows(const sz_session* s, cudaStream_t st, const sz_hc& hc
     return SZ_OK;
 }
 
-// The DeltaNet scan: the pass of one layer (l >= 0: all m rows, with outputs) or the replay of a commit (l < 0: every layer in one
-// launch, the kept rows only, decided on the device).
-template <int D, int PARTS>
-static int sz_scan_launch(sz_session* s, cudaStream_t st, int l, int m, const SzDeltaPrep& pp) {
-    const sz_model_config& c = s->model.cfg;
-    const int64_t kd = (int64_t)c.ssm_k_heads * D, vd = (int64_t)c.ssm_v_heads * D, ch = 2 * kd + vd;
-    const int64_t Sl = (int64_t)c.ssm_v_heads * D * D;
-    const int di = l >= 0 ? s->lb[l].delta_index : 0;
-    const float* xc = s->d_xc + (int64_t)di * SZ_MAX_VERIFY * ch;
-    const float* beta = s->d_beta + (int64_t)di * SZ_MAX_VERIFY * c.ssm_v_heads;
-    const float* decay = s->d_decay + (int64_t)di * SZ_MAX_VERIFY * c.ssm_v_heads;
-    const float* nw = l >= 0 ? (const float*)s->layers[l].ssm_norm.data : nullptr;
-    SZ_CUDA(sz_launch(l >= 0 ? "delta_scan" : "delta_replay", sz_delta_scan_kernel<D, PARTS>, dim3(c.ssm_v_heads, l >= 0 ? 1 : s->n_delta),
-                      dim3(D * PARTS), 0, st, true, xc, beta, decay, (const float*)s->d_z, nw, (const float*)(s->S[0] + di * Sl),
-                      (const float*)(s->S[1] + di * Sl), s->S[0] + di * Sl, s->S[1] + di * Sl, (const int32_t*)s->state, (const int32_t*)s->res,
-                      (int)c.ssm_k_heads, (int)c.ssm_v_heads, m, c.eps, l >= 0 ? s->d_og : (float*)nullptr, pp,
-                      (const SzTree*)(s->tree_pass ? s->ids + 32 : nullptr), s->fork));
-    return SZ_OK;
-}
-
-static int sz_scan(sz_session* s, cudaStream_t st, int l, int m, const SzDeltaPrep& pp) {
-    if (s->model.cfg.ssm_head_dim == 128) return sz_scan_launch<128, 2>(s, st, l, m, pp);
-    return sz_scan_launch<64, 1>(s, st, l, m, pp);
-}
-
-// One sequence's entry of the table the many-sequence scan reads: what sz_delta_layer hands the scan of layer l, fused front end.
+// One sequence's scan of layer l as the scan kernels read it: the session's own buffers, fused front end.
 static void sz_scan_seq_entry(sz_session* s, int l, int m, SzScanSeq* e) {
     const sz_model_config& c = s->model.cfg;
     const sz_layer& L = s->layers[l];
@@ -852,16 +844,36 @@ static void sz_scan_seq_entry(sz_session* s, int l, int m, SzScanSeq* e) {
     e->pp.k = (int)c.conv_k;
     e->m = m;
 }
+// The DeltaNet scan: the pass of one layer (l >= 0: all m rows, with outputs) or the replay of a commit (l < 0: every layer in one
+// launch, the kept rows only, decided on the device).
+static int sz_scan(sz_session* s, cudaStream_t st, int l, int m, bool fused) {
+    const sz_model_config& c = s->model.cfg;
+    SzScanSeq e;
+    if (l >= 0) {
+        sz_scan_seq_entry(s, l, m, &e);
+        if (!fused) e.pp.xin = nullptr;
+    } else {
+        e = SzScanSeq{};
+        e.xc = s->d_xc; e.beta = s->d_beta; e.decay = s->d_decay;
+        e.S0 = e.O0 = s->S[0]; e.S1 = e.O1 = s->S[1];
+        e.state = s->state; e.res = s->res;
+        e.m = m;
+    }
+    const float* nw = l >= 0 ? (const float*)s->layers[l].ssm_norm.data : nullptr;
+    const SzTree* tr = s->tree_pass ? (const SzTree*)(s->ids + 32) : nullptr;
+    const int d = c.ssm_head_dim;
+    const dim3 grid(c.ssm_v_heads * (d / 32), l >= 0 ? 1 : s->n_delta), block(2 * d);
+    const char* name = l >= 0 ? "delta_scan" : "delta_replay";
+    SZ_CUDA(sz_launch(name, d == 128 ? sz_delta_scan_kernel<128> : sz_delta_scan_kernel<64>, grid, block, 0, st, true, e, nw, (int)c.ssm_k_heads, (int)c.ssm_v_heads,
+                      c.eps, tr, s->fork));
+    return SZ_OK;
+}
 // The scans of layer l of n sequences in one launch (tab: their entries on the device).
 static int sz_scan_seqs(sz_session* s0, cudaStream_t st, int l, int n, const SzScanSeq* tab, bool pdl) {
     const sz_model_config& c = s0->model.cfg;
-    const float* nw = (const float*)s0->layers[l].ssm_norm.data;
-    if (c.ssm_head_dim == 128)
-        SZ_CUDA(sz_launch("delta_scan_seqs", sz_delta_scan_seqs_kernel<128, 2>, dim3(c.ssm_v_heads, n), dim3(256), 0, st, pdl, tab, nw, (int)c.ssm_k_heads,
-                          (int)c.ssm_v_heads, c.eps));
-    else
-        SZ_CUDA(sz_launch("delta_scan_seqs", sz_delta_scan_seqs_kernel<64, 1>, dim3(c.ssm_v_heads, n), dim3(64), 0, st, pdl, tab, nw, (int)c.ssm_k_heads,
-                          (int)c.ssm_v_heads, c.eps));
+    const int d = c.ssm_head_dim;
+    SZ_CUDA(sz_launch("delta_scan_seqs", d == 128 ? sz_delta_scan_seqs_kernel<128> : sz_delta_scan_seqs_kernel<64>, dim3(c.ssm_v_heads * (d / 32), n), dim3(2 * d), 0, st,
+                      pdl, tab, (const float*)s0->layers[l].ssm_norm.data, (int)c.ssm_k_heads, (int)c.ssm_v_heads, c.eps));
     return SZ_OK;
 }
 
@@ -924,17 +936,12 @@ static int sz_delta_layer(sz_session* s, cudaStream_t st, int l, int m, int part
     if (!(parts & SZ_MIX_CORE)) return (parts & SZ_MIX_OUT) ? sz_dense_launch(b, st, "ssm_out") : SZ_OK;
     const int64_t cl = (int64_t)(c.conv_k - 1) * ch;
     static const bool split_prep = getenv("SZ_GENERIC_KERNELS") && atoi(getenv("SZ_GENERIC_KERNELS")) != 0;
-    SzDeltaPrep pp = {};
     if (split_prep) {  // the front end as a kernel of its own (the second implementation the fused one is checked against)
         SZ_CUDA(sz_launch("delta_prep", sz_delta_prep_kernel, dim3((unsigned)((ch + 255) / 256), m), dim3(256), 0, st, true, (const float*)xin, (const float*)(s->conv[0] + di * cl),
                           (const float*)(s->conv[1] + di * cl), (const int32_t*)s->state, (const float*)L.ssm_conv1d.data, (const float*)s->d_b,
                           (const float*)s->d_a, (const float*)L.ssm_a.data, (const float*)L.ssm_dt_bias.data, kh, vh, d, (int)c.conv_k, xc, beta, decay));
-    } else {
-        pp.xin = xin; pp.conv0 = s->conv[0] + di * cl; pp.conv1 = s->conv[1] + di * cl; pp.cw = (const float*)L.ssm_conv1d.data;
-        pp.b = s->d_b; pp.a = s->d_a; pp.a_log = (const float*)L.ssm_a.data; pp.dt = (const float*)L.ssm_dt_bias.data;
-        pp.xc = xc; pp.beta = beta; pp.decay = decay; pp.k = (int)c.conv_k;
     }
-    if ((rc = sz_scan(s, st, l, m, pp))) return rc;
+    if ((rc = sz_scan(s, st, l, m, !split_prep))) return rc;
     return (parts & SZ_MIX_OUT) ? sz_dense_launch(b, st, "ssm_out") : SZ_OK;
 }
 
@@ -947,16 +954,25 @@ static int sz_attn_launch(sz_session* s, cudaStream_t st, const u8* kc, const u8
     return SZ_OK;
 }
 
+// Splits of the cache a pass of m rows takes in the grouped kernel: about one block a multiprocessor, or, where two fit (few queries:
+// small fragments), twice as many, so that each block's chain of chunks is half as long and the two blocks hide each other's barriers.
+static int sz_attn2_splits(const sz_session* s, size_t smem) {
+    int splits = s->attn_splits2;
+    if (smem + 2048 <= 113 * 1024 && 2 * splits <= (s->ctx + 255) / 256) splits *= 2;
+    return splits;
+}
+static int sz_attn2_nqt(int queries) { return queries <= 16 ? 1 : (queries <= 32 ? 2 : 4); }
+static size_t sz_attn2_smem(int hd, int nqt) {
+    return (size_t)(hd == 64 ? SzAttn2<64>::smem_bytes(nqt) : (hd == 128 ? SzAttn2<128>::smem_bytes(nqt) : SzAttn2<256>::smem_bytes(nqt)));
+}
+
 template <int HD, int NQT>
 static int sz_attn2_go(sz_session* s, cudaStream_t st, const u8* kc, const u8* vc, int m, int* splits_used, int ratio) {
     const sz_model_config& c = s->model.cfg;
     static bool set = false;
     const size_t smem = (size_t)SzAttn2<HD>::smem_bytes(NQT);
     if (!set) { SZ_CUDA(cudaFuncSetAttribute(sz_attn2_kernel<HD, NQT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); set = true; }
-    // two blocks fit a multiprocessor when the query fragments are small: twice the splits then, so that each block's chain of
-    // chunks is half as long and the two blocks hide each other's barriers
-    int splits = s->attn_splits2;
-    if (smem + 2048 <= 113 * 1024 && 2 * splits <= (s->ctx + 255) / 256) splits *= 2;
+    int splits = sz_attn2_splits(s, smem);
     if (ratio) {   // the sparse form: a block a (kv head, split, row); a row's list holds about the budget's positions, 128 or more a split
         const int by_budget = (c.idx_budget + 127) / 128;
         if (splits > by_budget) splits = by_budget < 1 ? 1 : by_budget;
@@ -965,16 +981,16 @@ static int sz_attn2_go(sz_session* s, cudaStream_t st, const u8* kc, const u8* v
     SZ_CUDA(sz_launch("attention_grouped", sz_attn2_kernel<HD, NQT>, dim3(c.n_kv_head, splits, ratio ? m : 1), dim3(256), smem, st, true, (const float*)s->a_q,
                       kc, vc, (int)c.n_head, (int)c.n_kv_head, m, s->ctx, (const int32_t*)s->state, splits, s->a_part, (u32*)(s->state + 2),
                       (const SzTree*)(s->tree_pass ? s->ids + 32 : nullptr), (const int32_t*)(ratio ? s->i_list : nullptr), (const int32_t*)s->i_count,
-                      s->i_ctx_blocks, ratio));
+                      s->i_ctx_blocks, ratio, (const SzSeqDev*)nullptr, (const SzAttnGroup*)nullptr, 0));
     return SZ_OK;
 }
 
 template <int HD>
 static int sz_attn2_launch(sz_session* s, cudaStream_t st, const u8* kc, const u8* vc, int m, int* splits_used, int ratio) {
     const sz_model_config& c = s->model.cfg;
-    const int qv = c.n_head / c.n_kv_head * (ratio ? 1 : m);   // the sparse form serves one row a block
-    if (qv <= 16) return sz_attn2_go<HD, 1>(s, st, kc, vc, m, splits_used, ratio);
-    if (qv <= 32) return sz_attn2_go<HD, 2>(s, st, kc, vc, m, splits_used, ratio);
+    const int nqt = sz_attn2_nqt(c.n_head / c.n_kv_head * (ratio ? 1 : m));   // the sparse form serves one row a block
+    if (nqt == 1) return sz_attn2_go<HD, 1>(s, st, kc, vc, m, splits_used, ratio);
+    if (nqt == 2) return sz_attn2_go<HD, 2>(s, st, kc, vc, m, splits_used, ratio);
     return sz_attn2_go<HD, 4>(s, st, kc, vc, m, splits_used, ratio);
 }
 
@@ -1012,8 +1028,8 @@ static int sz_attn_layer(sz_session* s, cudaStream_t st, int l, int m, int parts
     }
     SZ_CUDA(sz_launch("attn_prep", sz_attn_prep_kernel, dim3(nh + 2 * nkv, m), dim3(128), 0, st, true, (const float*)s->a_qg, (const float*)s->a_k,
                       (const float*)s->a_v, (const float*)L.attn_q_norm.data, (const float*)L.attn_k_norm.data, nh, nkv, hd, s->ctx, c.eps,
-                      (const int32_t*)s->state, (int)c.rope_dims, (const double*)s->rope_den, q8, kc, vc, s->a_q, s->a_gate,
-                      (const SzTree*)(s->tree_pass ? s->ids + 32 : nullptr)));
+                      (const int32_t*)s->state, (int)c.rope_dims, (const double*)s->rope_den, q8, kc, vc, s->a_q,
+                      (const SzTree*)(s->tree_pass ? s->ids + 32 : nullptr), (const SzSeqDev*)nullptr, (const SzRowDev*)nullptr, 0));
     // the grouped tensor-core kernel serves the packed int8 cache with up to 64 queries a KV head; the simple kernel everything else
     static const bool generic_only = getenv("SZ_GENERIC_KERNELS") && atoi(getenv("SZ_GENERIC_KERNELS")) != 0;
     const bool grouped = q8 && (!generic_only || idx) && (nh / nkv) * m <= 64;
@@ -1028,8 +1044,8 @@ static int sz_attn_layer(sz_session* s, cudaStream_t st, int l, int m, int parts
         else rc = sz_attn_launch<8>(s, st, kc, vc, m);
     }
     if (rc) return rc;
-    SZ_CUDA(sz_launch("attn_merge", sz_attn_merge_kernel, dim3(nh, m), dim3(256), 0, st, true, (const float*)s->a_part, (const float*)s->a_gate, nh, hd,
-                      splits, s->a_o));
+    SZ_CUDA(sz_launch("attn_merge", sz_attn_merge_kernel, dim3(nh, m), dim3(256), 0, st, true, (const float*)s->a_part, (const float*)s->a_qg, nh, hd,
+                      splits, s->a_o, (const SzRowDev*)nullptr));
     return (parts & SZ_MIX_OUT) ? sz_dense_launch(b, st, "attn_output") : SZ_OK;
 }
 
@@ -1136,7 +1152,7 @@ static int sz_forward(sz_session* s, cudaStream_t st, int m, bool head) {
 static int sz_commit_device(sz_session* s, cudaStream_t st, int m) {
     const sz_model_config& c = s->model.cfg;
     if (s->n_delta > 0) {
-        const int rc = sz_scan(s, st, -1, m, SzDeltaPrep());
+        const int rc = sz_scan(s, st, -1, m, false);
         if (rc) return rc;
         const int64_t kd = (int64_t)c.ssm_k_heads * c.ssm_head_dim, vd = (int64_t)c.ssm_v_heads * c.ssm_head_dim, ch = 2 * kd + vd;
         SZ_CUDA(sz_launch("conv_commit", sz_conv_commit_kernel, dim3(c.conv_k - 1, s->n_delta), dim3(256), 0, st, true, (const float*)s->conv[0],
@@ -1414,11 +1430,14 @@ extern "C" int sz_session_commit_path(sz_session* s, const int32_t* path, int n,
     return SZ_OK;
 }
 
-// Feeds a prompt: passes of up to 8 rows, every row kept; the head runs for the last pass only.  Afterwards sz_session_result gives the
+// Feeds a prompt: chunks of many rows, then passes of up to 8, every row kept; the head runs for the last pass only.  Afterwards sz_session_result gives the
 // top-64 (and logits) of the last pass's rows; the last row's are the prompt's.
+static int sz_prefill_chunks(sz_session* s, const int32_t* ids, int body, uint64_t stream, int* done);
 extern "C" int sz_session_prefill(sz_session* s, const int32_t* ids, int n, uint64_t stream) {
     if (!s || !ids || n < 1) return sz_fail(SZ_E_ARG, "sz_session_prefill: nothing to feed");
     int done = 0;
+    const int crc = sz_prefill_chunks(s, ids, n - ((n - 1) % SZ_MAX_VERIFY + 1), stream, &done);   // all but the last pass, where the session has room for chunks
+    if (crc) return crc;
     while (done < n) {
         const int m = n - done < SZ_MAX_VERIFY ? n - done : SZ_MAX_VERIFY;
         const bool last = done + m == n;
@@ -1549,12 +1568,19 @@ sz_batch_move_kernel(const SzBatchTab* __restrict__ T, float* const* __restrict_
 }
 
 enum { SZ_BATCH_SLOTS = SZ_DENSE_MAX_JOBS + 1 };   // per layer: the outputs of the input projections, then the input of the output projection
-struct SzBatchScratch { int64_t tab, ptrs, ptrs_bytes, scan, scan_bytes, x, y, r, r2, rn, acc, in, in_row, core, core_row, partial, partial_floats, moe, moe_bytes, total; };
+struct SzBatchScratch { int64_t up, up_bytes, rtab, groups, rids, aq, xc, beta, decay, tab, ptrs, ptrs_bytes, scan, scan_bytes, x, y, r, r2, rn, acc, in, in_row, core, core_row, partial, partial_floats, moe, moe_bytes, total; };
 static int sz_batch_layout(const sz_model* m, int rows_max, SzBatchScratch* S) {
     if (!m || !m->layers) return sz_fail(SZ_E_ARG, "null model");
     if (rows_max < 8 || rows_max % 8) return sz_fail(SZ_E_ARG, "sz_batch: rows_max = %d (a multiple of 8)", rows_max);
     const sz_model_config& c = m->cfg;
     int64_t o = 0, mb = 0;
+    // the tables of a many-row step, uploaded together: sequences, rows, attention groups, tokens
+    S->up = o;
+    S->rtab = S->up + (int64_t)sizeof(SzSeqDev) * SZ_BATCH_MAX;
+    S->groups = S->rtab + (int64_t)sizeof(SzRowDev) * rows_max;
+    S->rids = S->groups + (int64_t)sizeof(SzAttnGroup) * rows_max;
+    S->up_bytes = S->rids + 4 * (int64_t)rows_max - S->up;
+    o = up256(o + S->up_bytes);
     S->tab = o; o = up256(o + (int64_t)sizeof(SzBatchTab));
     S->ptrs_bytes = (int64_t)c.n_layer * SZ_BATCH_SLOTS * SZ_BATCH_MAX * (int64_t)sizeof(float*);
     S->ptrs = o; o = up256(o + S->ptrs_bytes);
@@ -1578,6 +1604,10 @@ static int sz_batch_layout(const sz_model* m, int rows_max, SzBatchScratch* S) {
     S->core_row = vd > (int64_t)c.n_head * c.head_dim ? vd : (int64_t)c.n_head * c.head_dim;
     S->in = o; o = up256(o + 4 * rows_max * S->in_row);
     S->core = o; o = up256(o + 4 * rows_max * S->core_row);
+    S->aq = o; o = up256(o + 4 * rows_max * (int64_t)c.n_head * c.head_dim);
+    S->xc = o; o = up256(o + 4 * rows_max * (2 * kd + vd));
+    S->beta = o; o = up256(o + 4 * (int64_t)rows_max * c.ssm_v_heads);
+    S->decay = o; o = up256(o + 4 * (int64_t)rows_max * c.ssm_v_heads);
     // the many-row projection kernel's sums of the eight column parts, for the widest set of projections
     S->partial_floats = 8 * (int64_t)rows_max * (S->in_row > c.hidden ? S->in_row : c.hidden);
     S->partial = o; o = up256(o + 4 * S->partial_floats);
@@ -1607,6 +1637,234 @@ extern "C" int sz_batch_scratch_init(const sz_model* m, int rows_max, uint64_t s
     if (!scratch || (scratch & 255)) return sz_fail(SZ_E_ARG, "scratch must be 256-byte aligned");
     SZ_CUDA(cudaMemsetAsync((void*)(scratch + S.x), 0, (size_t)(S.moe - S.x), (cudaStream_t)stream));
     return sz_moe_rows_status(&m->layers[0].moe, rows_max, scratch + S.moe, nullptr, stream);
+}
+
+// ---- many rows through the layers ----------------------------------------------------------------------------------------------------------
+// What a step of sz_batch_verify and sz_batch_prefill and the chunks of sz_session_prefill run: every kernel of a layer once over the
+// rows of all sequences, from tables (sz_session_rows.cuh).  A sequence brings up to 8 rows of a pass, or, where every row is kept and
+// none needs logits (a prompt before its last pass), any number: the recurrences run through them in one launch and attention
+// takes them in groups of 8, so that the rows are bit for bit those of the passes they replace.
+static bool sz_rows_fits(const sz_session* s) {
+    const sz_model_config& c = s->model.cfg;
+    if (!s->hc_fast || s->p_hist || c.idx_heads > 0 || !(s->flags & SZ_KV_Q8) || c.n_head / c.n_kv_head * SZ_MAX_VERIFY > 64 || s->want_routes) return false;
+    for (const sz_layer& L : s->layers) if (!sz_moe_rows_takes(&L.moe)) return false;
+    return true;
+}
+
+struct SzAttnBatch { int row0, rows, g0[4], ng[3], splits[3]; };   // rows that attend in one go: their groups by size of the queries (16, 32, 64)
+
+template <int HD, int NQT>
+static int sz_rows_attn_go(cudaStream_t st, const sz_model_config& c, const float* aq, int splits, const SzSeqDev* seqs, const SzAttnGroup* groups, int ng, int ai, u32* err) {
+    static bool set = false;
+    const size_t smem = (size_t)SzAttn2<HD>::smem_bytes(NQT);
+    if (!set) { SZ_CUDA(cudaFuncSetAttribute(sz_attn2_kernel<HD, NQT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); set = true; }
+    SZ_CUDA(sz_launch("rows_attention", sz_attn2_kernel<HD, NQT>, dim3(c.n_kv_head, splits, ng), dim3(256), smem, st, true, aq, (const u8*)nullptr, (const u8*)nullptr,
+                      (int)c.n_head, (int)c.n_kv_head, 0, 0, (const int32_t*)nullptr, 0, (float*)nullptr, err, (const SzTree*)nullptr, (const int32_t*)nullptr,
+                      (const int32_t*)nullptr, 0, 0, seqs, groups, ai));
+    return SZ_OK;
+}
+template <int HD>
+static int sz_rows_attn(cudaStream_t st, const sz_model_config& c, const float* aq, const SzAttnBatch& B, const SzSeqDev* seqs, const SzAttnGroup* groups, int ai, u32* err) {
+    int rc = SZ_OK;
+    if (B.ng[0] && (rc = sz_rows_attn_go<HD, 1>(st, c, aq, B.splits[0], seqs, groups + B.g0[0], B.ng[0], ai, err))) return rc;
+    if (B.ng[1] && (rc = sz_rows_attn_go<HD, 2>(st, c, aq, B.splits[1], seqs, groups + B.g0[1], B.ng[1], ai, err))) return rc;
+    if (B.ng[2] && (rc = sz_rows_attn_go<HD, 4>(st, c, aq, B.splits[2], seqs, groups + B.g0[2], B.ng[2], ai, err))) return rc;
+    return SZ_OK;
+}
+
+// The layers for the rows of n sequences (all[b]: a prompt's chunk).  Leaves the rows' sublayer inputs of the output read in the
+// scratch's X when `read_out`, and commits the chunks on the device.
+static int sz_rows_layers(sz_session* const* ss, int n, const int32_t* ids, const int32_t* ms, const int* all, bool read_out, const SzBatchScratch& S, int rows_max,
+                          u8* base, cudaStream_t st) {
+    sz_session* s0 = ss[0];
+    const sz_model_config& c = s0->model.cfg;
+    const int nh = c.n_head, nkv = c.n_kv_head, hd = c.head_dim, G = nh / nkv;
+    int R = 0;
+    for (int b = 0; b < n; b++) R += ms[b];
+    const int Rp = (R + 7) & ~7;
+    // ---- the tables
+    static thread_local std::vector<u8> up;
+    static thread_local std::vector<SzAttnBatch> ab;
+    up.assign((size_t)S.up_bytes, 0);
+    ab.clear();
+    SzSeqDev* hs = (SzSeqDev*)up.data();
+    SzRowDev* hr = (SzRowDev*)(up.data() + (S.rtab - S.up));
+    SzAttnGroup* hg = (SzAttnGroup*)(up.data() + (S.groups - S.up));
+    int32_t* hi = (int32_t*)(up.data() + (S.rids - S.up));
+    memcpy(hi, ids, (size_t)R * 4);
+    const int64_t d2 = (int64_t)c.ssm_head_dim * c.ssm_head_dim;
+    (void)d2;
+    int row = 0;
+    for (int b = 0; b < n; b++) {
+        sz_session* s = ss[b];
+        SzSeqDev& q = hs[b];
+        q.state = s->state; q.res = s->res; q.ids = s->ids;
+        q.kc = s->kc; q.vc = s->vc;
+        q.S0 = s->S[0]; q.S1 = s->S[1]; q.conv0 = s->conv[0]; q.conv1 = s->conv[1];
+        q.xc = s->d_xc; q.beta = s->d_beta; q.decay = s->d_decay; q.xin = s->d_xin;
+        q.kv_layer = (long long)s->ctx * nkv * (hd + (((hd >> 5) * 2 + 15) & ~15));
+        q.ctx = s->ctx; q.off = row; q.m = ms[b]; q.all = all[b];
+        memcpy(q.staged, s->h_pin, 128);
+        memcpy(q.staged, ids + row, (size_t)(ms[b] < SZ_MAX_VERIFY ? ms[b] : SZ_MAX_VERIFY) * 4);
+        for (int j = 0; j < ms[b]; j++) { hr[row + j].seq = (int16_t)b; hr[row + j].j = (int16_t)j; }
+        row += ms[b];
+    }
+    // Attention in batches of consecutive rows whose partial results fit: a sequence's first group of a batch leaves them in its
+    // session's own buffer (8 rows of them), further ones in what the projections' partial sums use at other times.
+    float* PART = (float*)(base + S.partial);
+    int ng_all = 0;
+    {
+        std::vector<SzAttnGroup> cls[3];
+        int64_t used = 0;
+        int row0 = 0, last_own = -1;
+        auto close = [&](int end) {
+            SzAttnBatch B = {};
+            B.row0 = row0; B.rows = end - row0;
+            for (int k = 0; k < 3; k++) {
+                B.g0[k] = ng_all; B.ng[k] = (int)cls[k].size(); B.splits[k] = 0;
+                for (const SzAttnGroup& g : cls[k]) { if (g.splits > B.splits[k]) B.splits[k] = g.splits; hg[ng_all++] = g; }
+                cls[k].clear();
+            }
+            if (B.rows > 0) ab.push_back(B);
+            row0 = end; used = 0; last_own = -1;
+        };
+        for (int b = 0, at = 0; b < n; at += ms[b], b++)
+            for (int j = 0; j < ms[b]; j += SZ_MAX_VERIFY) {
+                SzAttnGroup g = {};
+                g.seq = b; g.row0 = at + j; g.j0 = j; g.m = ms[b] - j < SZ_MAX_VERIFY ? ms[b] - j : SZ_MAX_VERIFY;
+                const int nqt = sz_attn2_nqt(G * g.m), k = nqt == 1 ? 0 : (nqt == 2 ? 1 : 2);
+                g.splits = sz_attn2_splits(ss[b], sz_attn2_smem(hd, nqt));
+                const int64_t need = (int64_t)g.m * nh * g.splits * (hd + 2);
+                if (last_own == b && used + need > S.partial_floats) close(at + j);
+                if (last_own != b) { g.part = ss[b]->a_part; last_own = b; }
+                else { g.part = PART + used; used += (need + 63) & ~(int64_t)63; }
+                for (int i = 0; i < g.m; i++) { hr[g.row0 + i].part = g.part + (int64_t)i * nh * g.splits * (hd + 2); hr[g.row0 + i].splits = g.splits; }
+                cls[k].push_back(g);
+            }
+        close(R);
+    }
+    SZ_CUDA(cudaMemcpyAsync(base + S.up, up.data(), (size_t)S.up_bytes, cudaMemcpyHostToDevice, st));   // (pageable: staged before the call returns)
+    const SzSeqDev* seqs = (const SzSeqDev*)(base + S.up);
+    const SzRowDev* rws = (const SzRowDev*)(base + S.rtab);
+    const SzAttnGroup* groups = (const SzAttnGroup*)(base + S.groups);
+    float *X = (float*)(base + S.x), *Y = (float*)(base + S.y), *IN = (float*)(base + S.in), *CORE = (float*)(base + S.core), *AQ = (float*)(base + S.aq);
+    float *XC = (float*)(base + S.xc), *BETA = (float*)(base + S.beta), *DECAY = (float*)(base + S.decay);
+    SzBatchBufs BB = {(float*)(base + S.r), (float*)(base + S.r2), Y, X, (float*)(base + S.rn), (long long*)(base + S.acc), (int64_t)rows_max * SZ_HC_ACC_ROWS};
+    SZ_CUDA(cudaMemsetAsync(BB.acc, 0, sizeof(long long) * (size_t)Rp * SZ_HC_ACC_ROWS, st));   // read 0 adds into accumulator 0
+    SZ_CUDA(sz_launch("rows_embed", sz_rows_embed_kernel, dim3(R + n), dim3(256), 0, st, false, seqs, (const int32_t*)(base + S.rids), R,
+                      (const u8*)s0->model.token_embd.data, (int)s0->model.token_embd.type, (int)c.hidden, (int)c.streams, (int)c.vocab, BB.r));
+    const char* re = getenv("SZ_BATCH_DENSE_ROWS");   // 0: the projections 8 rows a launch (the second form; same bits)
+    const bool rows_form = !(re && atoi(re) == 0);
+    // a projection set over all rows: one launch where the many-row form of the kernel exists, else 8 rows a launch
+    auto dense = [&](const SzDenseArgs& a, const float* x, float* const* outs, const char* name) -> int {
+        SzDenseArgs ar = a;
+        ar.m = Rp; ar.x = x;
+        for (int k = 0; k < a.n_jobs; k++) ar.job[k].out = outs[k];
+        int taken = 0, r;
+        if (rows_form && (r = sz_dense_rows_launch(ar, PART, S.partial_floats, st, name, &taken))) return r;
+        for (int g = 0; g < Rp / 8 && !taken; g++) {
+            SzDenseArgs ag = a;
+            ag.m = 8; ag.x = x + (size_t)g * 8 * a.cols;
+            for (int k = 0; k < a.n_jobs; k++) ag.job[k].out = outs[k] + (size_t)g * 8 * a.job[k].ostride;
+            if ((r = sz_dense_launch(ag, st, name))) return r;
+        }
+        return SZ_OK;
+    };
+    u32* err = (u32*)(s0->state + 2);
+    int hn = 0, rc;
+    for (int l = 0; l < c.n_layer; l++) {
+        const sz_layer& L = s0->layers[l];
+        if ((rc = sz_hc_read_rows(s0, st, L.hc_attn, Rp, hn++, l > 0, true, BB, true))) return rc;
+        SzDenseArgs a, o;
+        sz_mixer_args(s0, l, 8, &a, &o);
+        float* outs[SZ_DENSE_MAX_JOBS];
+        int64_t at = 0;
+        for (int k = 0; k < a.n_jobs; k++) { outs[k] = IN + at; at += (int64_t)Rp * a.job[k].ostride; }
+        if ((rc = dense(a, X, outs, "rows_proj"))) return rc;
+        if (sz_is_attn(c, l)) {
+            const int ai = s0->lb[l].attn_index;
+            SZ_CUDA(sz_launch("rows_attn_prep", sz_attn_prep_kernel, dim3(nh + 2 * nkv, R), dim3(128), 0, st, true, (const float*)outs[0], (const float*)outs[1],
+                              (const float*)outs[2], (const float*)L.attn_q_norm.data, (const float*)L.attn_k_norm.data, nh, nkv, hd, 0, c.eps, (const int32_t*)nullptr,
+                              (int)c.rope_dims, (const double*)s0->rope_den, 1, (u8*)nullptr, (u8*)nullptr, AQ, (const SzTree*)nullptr, seqs, rws, ai));
+            for (const SzAttnBatch& B : ab) {
+                rc = hd == 64 ? sz_rows_attn<64>(st, c, AQ, B, seqs, groups, ai, err)
+                              : (hd == 128 ? sz_rows_attn<128>(st, c, AQ, B, seqs, groups, ai, err) : sz_rows_attn<256>(st, c, AQ, B, seqs, groups, ai, err));
+                if (rc) return rc;
+                SZ_CUDA(sz_launch("rows_attn_merge", sz_attn_merge_kernel, dim3(nh, B.rows), dim3(256), 0, st, true, (const float*)nullptr,
+                                  (const float*)(outs[0] + (int64_t)B.row0 * 2 * nh * hd), nh, hd, 0, CORE + (int64_t)B.row0 * nh * hd, rws + B.row0));
+            }
+        } else {
+            const int di = s0->lb[l].delta_index, vh = c.ssm_v_heads, kh = c.ssm_k_heads, d = c.ssm_head_dim, ch = (2 * kh + vh) * d;
+            SZ_CUDA(sz_launch("rows_delta_prep", sz_rows_delta_prep_kernel, dim3((ch + 255) / 256, R), dim3(256), 0, st, true, seqs, rws, di, (const float*)outs[0],
+                              (const float*)L.ssm_conv1d.data, (const float*)outs[2], (const float*)outs[3], (const float*)L.ssm_a.data, (const float*)L.ssm_dt_bias.data,
+                              kh, vh, d, (int)c.conv_k, XC, BETA, DECAY));
+            SZ_CUDA(sz_launch("rows_scan", d == 128 ? sz_rows_scan_kernel<128> : sz_rows_scan_kernel<64>, dim3(vh * (d / 32), n), dim3(2 * d), 0, st, true, seqs, di,
+                              (const float*)XC, (const float*)BETA, (const float*)DECAY, (const float*)outs[1], (const float*)L.ssm_norm.data, kh, vh, c.eps, CORE));
+        }
+        float* yo[1] = {Y};
+        if ((rc = dense(o, CORE, yo, "rows_out"))) return rc;
+        if ((rc = sz_hc_read_rows(s0, st, L.hc_ffn, Rp, hn++, true, true, BB, true))) return rc;
+        if ((rc = sz_moe_rows_live(&L.moe, (uint64_t)X, Rp, R, (uint64_t)Y, (uint64_t)(base + S.moe), S.moe_bytes, (uint64_t)st))) return rc;
+    }
+    if (read_out && (rc = sz_hc_read_rows(s0, st, s0->model.output_hc, Rp, hn++, true, false, BB, true))) return rc;
+    bool any_all = false;
+    for (int b = 0; b < n; b++) any_all = any_all || all[b];
+    if (any_all) SZ_CUDA(sz_launch("rows_commit", sz_rows_commit_kernel, dim3(1), dim3(SZ_BATCH_MAX), 0, st, true, seqs, n));
+    return SZ_OK;
+}
+
+// A stream a sequence (a pool owned by the calling thread, made at the first use) between two points of the caller's stream.
+struct SzBatchStreams {
+    cudaStream_t st = 0;
+    int n = 0;
+    bool multi = false;
+    cudaStream_t* pool = nullptr;
+    cudaEvent_t* ev = nullptr;
+    int begin(cudaStream_t stream, int count) {
+        static thread_local cudaStream_t tpool[SZ_BATCH_MAX] = {};
+        static thread_local cudaEvent_t tev[SZ_BATCH_MAX] = {};
+        static thread_local cudaEvent_t main_ev = nullptr;
+        static const bool off = getenv("SZ_BATCH_STREAMS") && atoi(getenv("SZ_BATCH_STREAMS")) == 0;
+        st = stream; n = count; pool = tpool; ev = tev;
+        multi = !off && n > 1;
+        if (!multi) return SZ_OK;
+        if (!main_ev) SZ_CUDA(cudaEventCreateWithFlags(&main_ev, cudaEventDisableTiming));
+        for (int b = 0; b < n; b++)
+            if (!pool[b]) {
+                SZ_CUDA(cudaStreamCreateWithFlags(&pool[b], cudaStreamNonBlocking));
+                SZ_CUDA(cudaEventCreateWithFlags(&ev[b], cudaEventDisableTiming));
+            }
+        SZ_CUDA(cudaEventRecord(main_ev, st));
+        for (int b = 0; b < n; b++) SZ_CUDA(cudaStreamWaitEvent(pool[b], main_ev, 0));
+        return SZ_OK;
+    }
+    int each(const std::function<int(int, cudaStream_t)>& fn) {
+        if (!multi) { for (int b = 0; b < n; b++) { const int r = fn(b, st); if (r) return r; } return SZ_OK; }
+        int dev = 0;
+        SZ_CUDA(cudaGetDevice(&dev));
+        std::atomic<int> worst{SZ_OK};   // (a failing launch: the first code is kept; its message is the last one written)
+        cudaStream_t* const pl = pool;
+        sz_issue_pool().each(n, dev, [&, pl](int b) { const int r = fn(b, pl[b]); if (r) { int z = SZ_OK; worst.compare_exchange_strong(z, r); } });
+        return worst.load();
+    }
+    int end() {
+        if (!multi) return SZ_OK;
+        for (int b = 0; b < n; b++) {
+            SZ_CUDA(cudaEventRecord(ev[b], pool[b]));
+            SZ_CUDA(cudaStreamWaitEvent(st, ev[b], 0));
+        }
+        return SZ_OK;
+    }
+};
+// Does a step of these sessions run through sz_rows_layers?  (SZ_BATCH_SHARED=0 or SZ_BATCH_SCAN_SEQS=0: the second forms, launches of
+// the sequences' own around what is shared; so do models with a per-layer embedding, the sparse indexer or an f32 cache.)
+static bool sz_rows_step_fits(sz_session* const* ss, int n) {
+    for (const char* v : {"SZ_BATCH_SHARED", "SZ_BATCH_SCAN_SEQS"}) {   // (read at every step: a test switches them inside one process)
+        const char* e = getenv(v);
+        if (e && atoi(e) == 0) return false;
+    }
+    for (int b = 0; b < n; b++) if (!sz_rows_fits(ss[b])) return false;
+    return true;
 }
 
 // One step of n sequences: sequence b reads ms[b] rows (ids: the rows of all sequences, one after the other).  accept_mode:
@@ -1639,7 +1897,7 @@ static int sz_batch_step(sz_session* const* ss, int n, const int32_t* ids, const
             return sz_fail(SZ_E_ARG, "sz_batch_verify: sequence %d is not a session of the same model", b);
         for (int q = 0; q < b; q++) if (ss[q] == s) return sz_fail(SZ_E_ARG, "sz_batch_verify: a session appears twice");
         const int m = ms[b];
-        if (m < 1 || m > SZ_MAX_VERIFY) return sz_fail(SZ_E_ARG, "a pass has 1..%d rows, got %d", SZ_MAX_VERIFY, m);
+        if (m < 1 || (m > SZ_MAX_VERIFY && heads[b])) return sz_fail(SZ_E_ARG, "a pass has 1..%d rows, got %d", SZ_MAX_VERIFY, m);
         if (s->last_m) return sz_fail(SZ_E_ARG, "sequence %d: the previous pass was not committed", b);
         if (s->len + m > s->ctx) return sz_fail(SZ_E_ARG, "sequence %d: %d positions + %d rows exceed the session's capacity %d", b, s->len, m, s->ctx);
         if (s->want_routes) return sz_fail(SZ_E_ARG, "sz_batch_verify: no routing trace in a batched step");
@@ -1649,6 +1907,39 @@ static int sz_batch_step(sz_session* const* ss, int n, const int32_t* ids, const
     tab.n = n;
     const int Rp = (R + 7) & ~7;
     if (Rp > rows_max) return sz_fail(SZ_E_ARG, "sz_batch_verify: %d rows in a scratch for %d", R, rows_max);
+    if (sz_rows_step_fits(ss, n)) {
+        int all[SZ_BATCH_MAX];
+        for (int b = 0; b < n; b++) {
+            all[b] = accept[b] == SZ_ACCEPT_ALL && !heads[b];
+            ss[b]->tree_pass = 0;
+        }
+        if ((rc = sz_rows_layers(ss, n, ids, ms, all, any_head, S, rows_max, (u8*)scratch, st))) return rc;
+        if (any_head) {
+            // the head, acceptance and commit stay launches of the sequence, each sequence's on a stream of its own
+            SzBatchStreams fan;
+            if ((rc = fan.begin(st, n))) return rc;
+            float* X = (float*)((u8*)scratch + S.x);
+            rc = fan.each([&](int b, cudaStream_t sb) -> int {
+                sz_session* s = ss[b];
+                if (all[b]) return SZ_OK;
+                float* const u = s->u;
+                s->u = X + (size_t)tab.off[b] * c.hidden;
+                int r = heads[b] ? sz_forward_head(s, sb, ms[b], true, false) : SZ_OK;
+                s->u = u;
+                return r ? r : sz_pass_tail(s, sb, ms[b], accept[b], eog_token, heads[b] != 0);
+            });
+            if (rc || (rc = fan.end())) return rc;
+        }
+        for (int b = 0; b < n; b++) {
+            sz_session* s = ss[b];
+            if (all[b]) { s->cur ^= 1; s->len += ms[b]; continue; }    // (committed on the device; nothing is pending)
+            s->last_m = ms[b];
+            s->pending_committed = accept[b] != SZ_ACCEPT_NONE;
+            s->device_keep = accept[b] == SZ_ACCEPT_ALL ? ms[b] : -1;
+        }
+        return SZ_OK;
+    }
+    for (int b = 0; b < n; b++) if (ms[b] > SZ_MAX_VERIFY) return sz_fail(SZ_E_ARG, "a pass has 1..%d rows, got %d", SZ_MAX_VERIFY, ms[b]);
     // the ids of every sequence into its session's staging block (pinned: the copy is asynchronous)
     int at = 0;
     for (int b = 0; b < n; b++) {
@@ -1872,6 +2163,40 @@ static int sz_batch_step(sz_session* const* ss, int n, const int32_t* ids, const
     return join();
 }
 
+// Rows of a prompt's chunk a session of this model keeps room for: SZ_ROWS_CHUNK, or what its capacity holds; 0 where sz_rows_layers
+// does not run the model, or the host said that prompts come through sz_batch_prefill (SZ_SESSION_LEAN).
+#define SZ_ROWS_CHUNK 256
+static int sz_rows_ws_plan(const sz_model* m, int ctx, int flags, int* rows, int64_t* bytes) {
+    const sz_model_config& c = m->cfg;
+    *rows = 0; *bytes = 0;
+    if ((flags & SZ_SESSION_LEAN) || !(flags & SZ_KV_Q8) || m->ple.ngram >= 2 || c.idx_heads > 0 || c.n_head / c.n_kv_head * SZ_MAX_VERIFY > 64) return SZ_OK;
+    for (int l = 0; l < c.n_layer; l++)
+        if (!sz_moe_rows_takes(&m->layers[l].moe)) return SZ_OK;
+    const int want = ctx < SZ_ROWS_CHUNK ? ctx / SZ_MAX_VERIFY * SZ_MAX_VERIFY : SZ_ROWS_CHUNK;
+    if (want < 2 * SZ_MAX_VERIFY) return SZ_OK;
+    SzBatchScratch S;
+    const int rc = sz_batch_layout(m, want, &S);
+    if (rc) return rc;
+    *rows = want; *bytes = S.total;
+    return SZ_OK;
+}
+// The first `body` tokens (whole passes' worth) of a prompt in chunks of equal size: *done of them, 0 when the session's prompts go in
+// passes.  A chunk costs little more for more rows (every expert's decode is the most of it), so chunks are as long as there is room.
+static int sz_prefill_chunks(sz_session* s, const int32_t* ids, int body, uint64_t stream, int* done) {
+    sz_session* const one[1] = {s};
+    if (s->ws_rows == 0 || body < 2 * SZ_MAX_VERIFY || s->last_m || s->len + body > s->ctx || !sz_rows_step_fits(one, 1)) return SZ_OK;
+    const int chunks = (body + s->ws_rows - 1) / s->ws_rows;
+    const int size = ((body + chunks - 1) / chunks + SZ_MAX_VERIFY - 1) / SZ_MAX_VERIFY * SZ_MAX_VERIFY;
+    while (*done < body) {
+        const int32_t m = body - *done < size ? body - *done : size;
+        const int accept = SZ_ACCEPT_ALL, head = 0;
+        const int rc = sz_batch_step(one, 1, ids + *done, &m, &accept, &head, -1, s->ws_rows, (uint64_t)s->ws, s->ws_bytes, stream);
+        if (rc) return rc;
+        *done += m;
+    }
+    return SZ_OK;
+}
+
 extern "C" int sz_batch_verify(sz_session* const* ss, int n, const int32_t* ids, const int32_t* ms, int accept_mode, int eog_token, int rows_max,
                                uint64_t scratch, int64_t scratch_bytes, uint64_t stream) {
     if (n < 1 || n > SZ_BATCH_MAX) return sz_fail(SZ_E_ARG, "sz_batch_verify: 1..%d sequences", SZ_BATCH_MAX);
@@ -1890,20 +2215,24 @@ extern "C" int sz_batch_prefill(sz_session* const* ss, int n, const int32_t* con
     std::vector<int> done((size_t)n, 0);
     for (int b = 0; b < n; b++)
         if (!ss[b] || !ids[b] || lens[b] < 1) return sz_fail(SZ_E_ARG, "sz_batch_prefill: sequence %d has nothing to feed", b);
+    const bool chunks = sz_rows_step_fits(ss, n);
     for (;;) {
         sz_session* step_s[SZ_BATCH_MAX];
         int32_t step_m[SZ_BATCH_MAX];
         int accept[SZ_BATCH_MAX], heads[SZ_BATCH_MAX], who[SZ_BATCH_MAX];
         std::vector<int32_t> rows;
-        int k = 0;
-        for (int b = 0; b < n && (k + 1) * SZ_MAX_VERIFY <= rows_max; b++) {
-            if (done[b] >= lens[b]) continue;
-            const int left = lens[b] - done[b];
-            const int m = left < SZ_MAX_VERIFY ? left : SZ_MAX_VERIFY;
-            const bool last = m == left;
+        int k = 0, room = rows_max;
+        for (int b = 0; b < n; b++) {
+            const int left = lens[b] - done[b], last_m = (lens[b] - 1) % SZ_MAX_VERIFY + 1, body = left - last_m;
+            if (left <= 0) continue;
+            // a prompt's last pass has the head; before it come passes of 8 rows, or as many of them at once as fit
+            int m = body > 0 ? SZ_MAX_VERIFY : last_m;
+            if (body > 0 && chunks) m = body < room / SZ_MAX_VERIFY * SZ_MAX_VERIFY ? body : room / SZ_MAX_VERIFY * SZ_MAX_VERIFY;
+            if (m < 1 || m > room) { if (chunks) continue; break; }
+            room -= chunks ? m : SZ_MAX_VERIFY;
             step_s[k] = ss[b]; step_m[k] = m; who[k] = b;
-            accept[k] = last ? SZ_ACCEPT_NONE : SZ_ACCEPT_ALL;
-            heads[k] = last ? 1 : 0;
+            heads[k] = body > 0 ? 0 : 1;
+            accept[k] = body > 0 ? SZ_ACCEPT_ALL : SZ_ACCEPT_NONE;
             rows.insert(rows.end(), ids[b] + done[b], ids[b] + done[b] + m);
             k++;
         }
@@ -1913,7 +2242,7 @@ extern "C" int sz_batch_prefill(sz_session* const* ss, int n, const int32_t* con
         for (int i = 0; i < k; i++) {
             const int b = who[i];
             done[b] += step_m[i];
-            if (done[b] < lens[b] && (rc = sz_session_commit(step_s[i], step_m[i], stream))) return rc;   // (a prompt's last pass stays pending)
+            if (done[b] < lens[b] && step_s[i]->last_m && (rc = sz_session_commit(step_s[i], step_m[i], stream))) return rc;   // (a prompt's last pass stays pending)
         }
     }
 }
@@ -2116,7 +2445,7 @@ struct SzKernelEntry {
     const char* name;
     const void* fn;
     int n;
-    int32_t types[20];
+    int32_t types[24];
 };
 const SzKernelEntry kKernels[] = {
     {"sz_embed_kernel", (const void*)sz_embed_kernel, 7, {SZ_P_CONST_PTR, SZ_P_CONST_PTR, SZ_P_I32, SZ_P_I32, SZ_P_I32, SZ_P_I32, SZ_P_PTR}},
@@ -2126,8 +2455,8 @@ const SzKernelEntry kKernels[] = {
     {"sz_delta_prep_kernel", (const void*)sz_delta_prep_kernel, 16, {SZ_P_CONST_PTR, SZ_P_CONST_PTR, SZ_P_CONST_PTR, SZ_P_CONST_PTR, SZ_P_CONST_PTR, SZ_P_CONST_PTR, SZ_P_CONST_PTR, SZ_P_CONST_PTR, SZ_P_CONST_PTR, SZ_P_I32, SZ_P_I32, SZ_P_I32, SZ_P_I32, SZ_P_PTR, SZ_P_PTR, SZ_P_PTR}},
     {"sz_conv_commit_kernel", (const void*)sz_conv_commit_kernel, 10, {SZ_P_CONST_PTR, SZ_P_CONST_PTR, SZ_P_CONST_PTR, SZ_P_CONST_PTR, SZ_P_CONST_PTR, SZ_P_I32, SZ_P_I32, SZ_P_PTR, SZ_P_PTR, SZ_P_I32}},
     {"sz_state_update_kernel", (const void*)sz_state_update_kernel, 2, {SZ_P_PTR, SZ_P_CONST_PTR}},
-    {"sz_attn_prep_kernel", (const void*)sz_attn_prep_kernel, 19, {SZ_P_CONST_PTR, SZ_P_CONST_PTR, SZ_P_CONST_PTR, SZ_P_CONST_PTR, SZ_P_CONST_PTR, SZ_P_I32, SZ_P_I32, SZ_P_I32, SZ_P_I32, SZ_P_F32, SZ_P_CONST_PTR, SZ_P_I32, SZ_P_CONST_PTR, SZ_P_I32, SZ_P_PTR, SZ_P_PTR, SZ_P_PTR, SZ_P_PTR, SZ_P_CONST_PTR}},
-    {"sz_attn_merge_kernel", (const void*)sz_attn_merge_kernel, 6, {SZ_P_CONST_PTR, SZ_P_CONST_PTR, SZ_P_I32, SZ_P_I32, SZ_P_I32, SZ_P_PTR}},
+    {"sz_attn_prep_kernel", (const void*)sz_attn_prep_kernel, 21, {SZ_P_CONST_PTR, SZ_P_CONST_PTR, SZ_P_CONST_PTR, SZ_P_CONST_PTR, SZ_P_CONST_PTR, SZ_P_I32, SZ_P_I32, SZ_P_I32, SZ_P_I32, SZ_P_F32, SZ_P_CONST_PTR, SZ_P_I32, SZ_P_CONST_PTR, SZ_P_I32, SZ_P_PTR, SZ_P_PTR, SZ_P_PTR, SZ_P_CONST_PTR, SZ_P_CONST_PTR, SZ_P_CONST_PTR, SZ_P_I32}},
+    {"sz_attn_merge_kernel", (const void*)sz_attn_merge_kernel, 7, {SZ_P_CONST_PTR, SZ_P_CONST_PTR, SZ_P_I32, SZ_P_I32, SZ_P_I32, SZ_P_PTR, SZ_P_CONST_PTR}},
     {"sz_accept_greedy_kernel", (const void*)sz_accept_greedy_kernel, 7, {SZ_P_CONST_PTR, SZ_P_CONST_PTR, SZ_P_I32, SZ_P_I32, SZ_P_I32, SZ_P_I32, SZ_P_PTR}},
     {"sz_accept_tree_kernel", (const void*)sz_accept_tree_kernel, 6, {SZ_P_CONST_PTR, SZ_P_CONST_PTR, SZ_P_CONST_PTR, SZ_P_I32, SZ_P_I32, SZ_P_PTR}},
     {"sz_kv_compact_kernel", (const void*)sz_kv_compact_kernel, 7, {SZ_P_PTR, SZ_P_PTR, SZ_P_CONST_PTR, SZ_P_CONST_PTR, SZ_P_I32, SZ_P_I32, SZ_P_I32}},
@@ -2168,7 +2497,7 @@ extern "C" int sz_kernel_launch(const char* name, const uint32_t grid[3], const 
     }
     if (!grid[0] || !grid[1] || !grid[2] || !block[0] || !block[1] || !block[2] || (uint64_t)block[0] * block[1] * block[2] > 1024)
         return sz_fail(SZ_E_ARG, "%s: a grid of %u x %u x %u blocks of %u x %u x %u threads does not fit", name, grid[0], grid[1], grid[2], block[0], block[1], block[2]);
-    uint64_t slots[20];
+    uint64_t slots[24];
     void* ptrs[20];
     for (int i = 0; i < nargs; i++) { slots[i] = args[i].bits; ptrs[i] = &slots[i]; }   // little-endian: a 4-byte parameter reads the low half of its slot
     SZ_CUDA(cudaLaunchKernel(e->fn, dim3(grid[0], grid[1], grid[2]), dim3(block[0], block[1], block[2]), ptrs, shared, (cudaStream_t)stream));

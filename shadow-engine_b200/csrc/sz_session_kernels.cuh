@@ -19,6 +19,31 @@ struct SzTree {
 };
 static_assert(sizeof(SzTree) == 128, "the tree tables are 32 words of the staging block");
 
+// ---- the tables of a many-row step (sz_session_rows.cuh)
+// One sequence of a step, as the kernels read it.
+struct SzSeqDev {
+    const int32_t *state, *res;
+    int32_t* ids;                                   // the session's staging block (the tokens, the stop ids)
+    u8 *kc, *vc;                                    // the caches of attention layer 0
+    float *S0, *S1, *conv0, *conv1;                 // recurrent states and carried conv rows of DeltaNet layer 0
+    float *xc, *beta, *decay, *xin;                 // what a replay reads, DeltaNet layer 0
+    long long kv_layer;                             // bytes from one attention layer's cache to the next
+    int ctx, off, m;                                // capacity; its first row in the step, and how many
+    int all;                                        // a prompt's chunk: every row is kept, nothing will be replayed
+    int staged[32];                                 // the staging block's first 32 words
+};
+// A row: its sequence, its place in it, where its attention splits' partial results lie.
+struct SzRowDev {
+    float* part;
+    int splits;
+    int16_t seq, j;
+};
+// Up to 8 consecutive rows of a sequence that attend together.
+struct SzAttnGroup {
+    float* part;
+    int row0, m, j0, splits, seq, pad;
+};
+
 #ifdef __CUDACC__
 
 // the row `dist` steps up the tree from row j; -1, -2, .. are the committed rows before the pass (most recent first)
@@ -656,15 +681,20 @@ __global__ void sz_state_update_kernel(int32_t* __restrict__ state, const int32_
     }
 }
 
-// ---- DeltaNet state scan (forward.rs:859-894): per value head, the d x d state column-resident in registers.
-// Thread (col = tid % D, part = tid / D) holds S[i][col] for the i of its part.  grid (vh, layers), block D * PARTS.
+// ---- DeltaNet state scan (forward.rs:859-894) ---------------------------------------------------------------------------------------
+// Per value head a D x D state whose columns are independent: a block takes 32 of them - lane = column - and its D / 16 warps 16 of the
+// D rows each, so a thread holds 16 values of the state in registers; the D / 32 blocks of a head are a cluster.  Sums over the rows run
+// in f32 over a warp's 16 and the warps' runs are added in f64 in a fixed order (the exact GPU scan's, kernels/forward.cu:991-1013):
+// one exchange through shared memory and one barrier a row of the pass is all that the recurrence waits for.  The outputs' sums are
+// left in shared memory and finished for up to 16 rows at once; the gated norm over a head's D outputs reads the neighbours' over the
+// cluster.  (One block of 256 threads a head, 64 values a thread and five barriers a row: 18 us a layer for 4 rows, some 1.5 us a row.)
 // Reads the state of the current buffer (state[1]) and writes the other one.  With `og` != null it applies all m rows and writes
-// the gated, normalised outputs (the pass itself, one layer: blockIdx.y = 0 and the pointers are that layer's).  With og == null it
-// is the replay of a commit: layer blockIdx.y of every per-layer array, only the res[0] kept rows, and nothing at all when every
-// row was kept (the pass already wrote that state) or none was.
-// In the pass itself (og != null) the block also does the front end for the channels it needs - q and k of its key head, v of its
-// own head: causal conv + SiLU, L2 norms, beta and decay (what sz_delta_prep_kernel does for a whole row) - so the layer needs no
-// launch between the projections and the scan.  It leaves the conv outputs, beta and decay where the replay of a commit reads them.
+// the gated, normalised outputs (the pass itself).  With og == null it is the replay of a commit: layer blockIdx.y of every per-layer
+// array, only the res[0] kept rows, and nothing at all when every row was kept (the pass already wrote that state) or none was.
+// With pp.xin the block also does the front end for the channels it needs - q and k of its key head, v of its own columns: causal conv
+// + SiLU, L2 norms, beta and decay (what sz_delta_prep_kernel does for whole rows) - and leaves the conv outputs, beta and decay (and,
+// with xsave, the raw projections) where the replay of a commit reads them: passes of up to SZ_MAX_VERIFY rows.  Without, the front
+// end ran as a kernel of its own and any number of rows follow one another.
 struct SzDeltaPrep {
     const float* xin;     // [m][ch] raw projections of this layer (null: the front end already ran as a kernel of its own)
     const float* conv0;   // (k - 1) x ch carried rows, two buffers
@@ -677,215 +707,10 @@ struct SzDeltaPrep {
     float* xc;            // [m][ch] out
     float* beta;          // [m][vh] out
     float* decay;         // [m][vh] out
+    float* xsave;         // [m][ch] out: a copy of xin, or null
     int k;
 };
-
-// (the kernel's body: block (hd, di) of the grid described above)
-template <int D, int PARTS>
-__device__ __forceinline__ void
-sz_delta_scan_body(const float* __restrict__ xc_all, const float* __restrict__ beta_all, const float* __restrict__ decay_all,
-                   const float* __restrict__ z, const float* __restrict__ norm_w, const float* __restrict__ S0, const float* __restrict__ S1,
-                   float* __restrict__ O0, float* __restrict__ O1, const int32_t* __restrict__ state, const int32_t* __restrict__ res, int kh,
-                   int vh, int m, float eps, float* __restrict__ og, const SzDeltaPrep& pp, const SzTree* __restrict__ tr,
-                   float* __restrict__ fork, const int hd, const int di) {
-    constexpr int NI = D / PARTS;
-    constexpr int RUN = NI < 16 ? NI : 16;  // sums run in f32 over 16 terms and the runs are added in f64, as the reference's exact
-                                            // GPU scan does (kernels/forward.cu:991-1013): a conversion to f64 per term would
-                                            // keep the conversion unit busy for longer than the state takes to arrive
-    __shared__ float sk[D], sq[D];
-    __shared__ double part[PARTS][D];
-    __shared__ float ofs[SZ_MAX_VERIFY][D];
-    __shared__ double rrs[SZ_MAX_VERIFY];
-    __shared__ float pbuf[SZ_MAX_VERIFY][3][D];   // the rows' q, k, v after the front end
-    __shared__ float sbeta[SZ_MAX_VERIFY], sdecay[SZ_MAX_VERIFY];
-    const int col = threadIdx.x % D, pt = threadIdx.x / D;
-    const int kx = hd % kh;  // value heads are tiled over the key heads (forward.rs:862-864)
-    const int kd = kh * D, ch = 2 * kd + vh * D;
-    const size_t Sl = (size_t)vh * D * D;
-    float S[NI];
-    // the state belongs to the previous pass (and the buffer index with it): in the pass itself it is fetched ahead of the wait
-    if (og) {
-        const int cur0 = state[1];
-        const float* Sg = (cur0 ? S1 : S0) + di * Sl + (size_t)hd * D * D;
-#pragma unroll
-        for (int i = 0; i < NI; i++) S[i] = sz_ld32_here(Sg + (size_t)(pt * NI + i) * D + col);
-    }
-    sz_pdl_wait();
-    sz_pdl_trigger();
-    // A tree pass (tr != null): a row continues from the state after its PARENT.  Rows come parents first, so the state after a row
-    // that a later row branches off (tr->save) is kept in `fork` ([value head][row][D * D]) and fetched when a row's parent is not the
-    // row just before it.  The state the pass leaves in the other buffer is then that of no one path: the commit of a tree pass
-    // always replays, along the kept path res[2 ..] (row indices), where a chain's kept rows are simply 0 .. res[0] - 1.
-    int rows = m;
-    if (!og) {
-        rows = res[0];
-        if (rows <= 0 || (!tr && rows >= m)) return;
-    }
-    const int cur = state[1];
-    const float* S_in = (cur ? S1 : S0) + di * Sl;
-    float* S_out = (cur ? O0 : O1) + di * Sl;
-    const float* xc = xc_all + (size_t)di * SZ_MAX_VERIFY * ch;
-    const float* beta = beta_all + (size_t)di * SZ_MAX_VERIFY * vh;
-    const float* decay = decay_all + (size_t)di * SZ_MAX_VERIFY * vh;
-    if (!og) {
-        const float* Sg = S_in + (size_t)hd * D * D;
-#pragma unroll
-        for (int i = 0; i < NI; i++) S[i] = Sg[(size_t)(pt * NI + i) * D + col];
-    }
-    const bool fused = og != nullptr && pp.xin != nullptr;
-    if (fused) {
-        // ---- front end for this block's channels (forward.rs:829-861)
-        const float* conv = cur ? pp.conv1 : pp.conv0;
-        const int k = pp.k;
-        for (int idx = threadIdx.x; idx < rows * 3 * D; idx += D * PARTS) {
-            const int j = idx / (3 * D), c = idx - j * 3 * D, part3 = c / D, i = c - part3 * D;
-            const int chn = part3 == 0 ? kx * D + i : (part3 == 1 ? kd + kx * D + i : 2 * kd + hd * D + i);
-            double acc = (double)pp.cw[chn * k + (k - 1)] * (double)pp.xin[(size_t)j * ch + chn];
-            for (int t = 0; t < k - 1; t++) {
-                const int tau = sz_tree_up(tr, j, (k - 1) - t);  // the row (k - 1) - t steps back: of this pass, or (negative) of the carried state
-                const float prev = tau >= 0 ? pp.xin[(size_t)tau * ch + chn] : conv[(size_t)((k - 1) + tau) * ch + chn];
-                acc += (double)pp.cw[chn * k + t] * (double)prev;
-            }
-            pbuf[j][part3][i] = sz_silu((float)acc);
-        }
-        if (threadIdx.x < rows) {
-            const int j = threadIdx.x;
-            const float bt = sz_sigmoid(pp.b[j * vh + hd]);
-            const float sp_in = pp.a[j * vh + hd] + pp.dt[hd];
-            const float sp = sp_in > 20.0f ? sp_in : log1pf(expf(sp_in));
-            const float dc = expf(pp.a_log[hd] * sp);
-            sbeta[j] = bt; sdecay[j] = dc;
-            pp.beta[j * vh + hd] = bt; pp.decay[j * vh + hd] = dc;
-        }
-        __syncthreads();
-        // L2 norm of q and k (q also / sqrt(d)): a warp an item (row, q or k)
-        {
-            const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-            for (int it = warp; it < rows * 2; it += (D * PARTS) / 32) {
-                const int j = it >> 1, part3 = it & 1;
-                double ss = 0.0;
-                for (int i = lane; i < D; i += 32) ss += (double)pbuf[j][part3][i] * (double)pbuf[j][part3][i];
-                ss = sz_warp_sum(ss);
-                const double nn = sz_rsqrt64(ss + 1e-6);
-                for (int i = lane; i < D; i += 32) {
-                    float t = (float)((double)pbuf[j][part3][i] * nn);
-                    if (part3 == 0) t = t / sqrtf((float)D);
-                    pbuf[j][part3][i] = t;
-                }
-            }
-        }
-        __syncthreads();
-        // what the replay of a commit reads: q and k once a key head (its first value head writes them), v by every head
-        for (int idx = threadIdx.x; idx < rows * 3 * D; idx += D * PARTS) {
-            const int j = idx / (3 * D), c = idx - j * 3 * D, part3 = c / D, i = c - part3 * D;
-            if (part3 == 2) pp.xc[(size_t)j * ch + 2 * kd + hd * D + i] = pbuf[j][2][i];
-            else if (hd < kh) pp.xc[(size_t)j * ch + part3 * kd + kx * D + i] = pbuf[j][part3][i];
-        }
-    }
-    float* fk = fork ? fork + ((size_t)di * vh + hd) * SZ_MAX_VERIFY * D * D : nullptr;
-    int prev_row = -1;
-    for (int jj = 0; jj < rows; jj++) {
-        const int j = (!og && tr) ? res[2 + jj] : jj;   // replay of a tree pass: the kept path
-        if (tr && og) {
-            const int par = tr->parents[j];
-            if (par != prev_row && par >= 0) {          // another branch: back to the state after the parent
-#pragma unroll
-                for (int i = 0; i < NI; i++) S[i] = fk[((size_t)par * D + pt * NI + i) * D + col];
-            }
-        }
-        prev_row = j;
-        const float* x = xc + (size_t)j * ch;
-        __syncthreads();
-        float vj, dc, bt;
-        if (fused) {
-            if (threadIdx.x < D) { sq[threadIdx.x] = pbuf[j][0][threadIdx.x]; sk[threadIdx.x] = pbuf[j][1][threadIdx.x]; }
-            vj = pbuf[j][2][col]; dc = sdecay[j]; bt = sbeta[j];
-        } else {
-            if (threadIdx.x < D) { sq[threadIdx.x] = x[kx * D + threadIdx.x]; sk[threadIdx.x] = x[kd + kx * D + threadIdx.x]; }
-            vj = x[2 * kd + hd * D + col];
-            dc = decay[j * vh + hd]; bt = beta[j * vh + hd];
-        }
-        __syncthreads();
-        double mem = 0.0;
-#pragma unroll
-        for (int i0 = 0; i0 < NI; i0 += RUN) {
-            float run = 0.f;
-#pragma unroll
-            for (int i = i0; i < i0 + RUN; i++) {
-                S[i] = S[i] * dc;
-                run = fmaf(S[i], sk[pt * NI + i], run);
-            }
-            mem += (double)run;
-        }
-        part[pt][col] = mem;
-        __syncthreads();
-        double tot = 0.0;
-#pragma unroll
-        for (int p = 0; p < PARTS; p++) tot += part[p][col];
-        const float dl = (float)(((double)vj - tot) * (double)bt);
-        double o = 0.0;
-#pragma unroll
-        for (int i0 = 0; i0 < NI; i0 += RUN) {
-            float run = 0.f;
-#pragma unroll
-            for (int i = i0; i < i0 + RUN; i++) {
-                S[i] = __fadd_rn(S[i], __fmul_rn(sk[pt * NI + i], dl));  // unfused, as the CPU reference
-                run = fmaf(S[i], sq[pt * NI + i], run);
-            }
-            o += (double)run;
-        }
-        if (og) {
-            __syncthreads();
-            part[pt][col] = o;
-            __syncthreads();
-            if (pt == 0) {
-                double ot = 0.0;
-#pragma unroll
-                for (int p = 0; p < PARTS; p++) ot += part[p][col];
-                ofs[j][col] = (float)ot;
-            }
-            if (tr && ((tr->save >> j) & 1u)) {
-#pragma unroll
-                for (int i = 0; i < NI; i++) fk[((size_t)j * D + pt * NI + i) * D + col] = S[i];
-            }
-        }
-    }
-    if (og) {
-        // gated RMS norm of every row's output at once: warp w sums the squares of row w, one thread a row takes the root, then
-        // every thread scales its share
-        __syncthreads();
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        for (int j = warp; j < rows; j += (D * PARTS) / 32) {
-            double ss = 0.0;
-            for (int i = lane; i < D; i += 32) ss += (double)ofs[j][i] * (double)ofs[j][i];
-            ss = sz_warp_sum(ss);
-            if (lane == 0) rrs[j] = sz_rsqrt64(ss / (double)D + (double)eps);
-        }
-        __syncthreads();
-        for (int idx = threadIdx.x; idx < rows * D; idx += D * PARTS) {
-            const int j = idx / D, c = idx - j * D;
-            const float normed = (float)((double)ofs[j][c] * rrs[j]) * norm_w[c];
-            og[(size_t)j * vh * D + hd * D + c] = normed * sz_sigmoid(z[(size_t)j * vh * D + hd * D + c]);
-        }
-    }
-    float* So = S_out + (size_t)hd * D * D;
-#pragma unroll
-    for (int i = 0; i < NI; i++) So[(size_t)(pt * NI + i) * D + col] = S[i];
-}
-
-template <int D, int PARTS>
-__global__ void __launch_bounds__(D * PARTS)
-sz_delta_scan_kernel(const float* __restrict__ xc_all, const float* __restrict__ beta_all, const float* __restrict__ decay_all,
-                     const float* __restrict__ z, const float* __restrict__ norm_w, const float* __restrict__ S0, const float* __restrict__ S1,
-                     float* __restrict__ O0, float* __restrict__ O1, const int32_t* __restrict__ state, const int32_t* __restrict__ res, int kh,
-                     int vh, int m, float eps, float* __restrict__ og, const SzDeltaPrep pp, const SzTree* __restrict__ tr,
-                     float* __restrict__ fork) {
-    sz_delta_scan_body<D, PARTS>(xc_all, beta_all, decay_all, z, norm_w, S0, S1, O0, O1, state, res, kh, vh, m, eps, og, pp, tr, fork,
-                                 (int)blockIdx.x, (int)blockIdx.y);
-}
-
-// The pass of one layer for SEVERAL sequences in one launch (a batched step): block row b is sequence b's scan, its pointers and
-// row count from a table.  grid (vh, sequences); the arithmetic is the kernel above's.
+// One sequence's scan of one layer.
 struct SzScanSeq {
     const float *xc, *beta, *decay, *z, *S0, *S1;
     float *O0, *O1;
@@ -894,18 +719,219 @@ struct SzScanSeq {
     SzDeltaPrep pp;
     int m, pad;
 };
-template <int D, int PARTS>
-__global__ void __launch_bounds__(D * PARTS, 512 / (D * PARTS))   // (128 registers a thread, as the kernel above happens to need)
-sz_delta_scan_seqs_kernel(const SzScanSeq* __restrict__ tab, const float* __restrict__ norm_w, int kh, int vh, float eps) {
-    __shared__ SzScanSeq q;   // (the entry in shared memory: two dozen pointers in registers would cost the kernel its second block)
-    static_assert(sizeof(SzScanSeq) % 8 == 0, "copied in 8-byte words");
-    if (threadIdx.x < sizeof(SzScanSeq) / 8) ((u64*)&q)[threadIdx.x] = ((const u64*)(tab + blockIdx.y))[threadIdx.x];
-    __syncthreads();
-    sz_delta_scan_body<D, PARTS>(q.xc, q.beta, q.decay, q.z, norm_w, q.S0, q.S1, q.O0, q.O1, q.state, q.res, kh, vh, q.m, eps, q.og, q.pp,
-                                 (const SzTree*)nullptr, (float*)nullptr, (int)blockIdx.x, 0);
+#define SZ_SCAN_RC 16     // rows between two exchanges of the outputs
+
+template <int D>
+struct SzScanShared {
+    float k[SZ_SCAN_RC][D], q[SZ_SCAN_RC][D], v[SZ_SCAN_RC][32];
+    float orun[SZ_SCAN_RC][D / 16][32];      // the outputs' runs
+    double mem[2][D / 16][32];                // a row's runs of S^T k
+    float ofs[2][SZ_SCAN_RC][32];            // finished outputs of the block's columns
+    float beta[SZ_SCAN_RC], decay[SZ_SCAN_RC];
+};
+// the runs of one column added as two halves of four each (D = 64: one half)
+template <int D, typename F>
+__device__ __forceinline__ double sz_scan_sum(F run) {
+    double tot = 0.0;
+#pragma unroll
+    for (int p = 0; p < D / 64; p++) {
+        double s = 0.0;
+#pragma unroll
+        for (int r = 0; r < 4; r++) s += run(4 * p + r);
+        tot += s;
+    }
+    return tot;
 }
 
-// ---- attention front end (forward.rs:908-927): per head RMSNorm + NeoX RoPE of q and k, the gate halves, K and V into the cache.
+template <int D>
+__device__ __forceinline__ void sz_delta_scan_body(const SzScanSeq& q, const float* __restrict__ norm_w, int kh, int vh, float eps,
+                                                   const SzTree* __restrict__ tr, float* __restrict__ fork, const int hd, const int cb, const int di) {
+    constexpr int RUNS = D / 16, NT = RUNS * 32;
+    __shared__ __align__(16) SzScanShared<D> sh;
+    const int run = threadIdx.x >> 5, lane = threadIdx.x & 31, col = cb * 32 + lane;
+    const int kx = hd % kh;  // value heads are tiled over the key heads (forward.rs:862-864)
+    const int kd = kh * D, ch = 2 * kd + vh * D;
+    const size_t Sl = (size_t)vh * D * D, Sat = (size_t)di * Sl + (size_t)hd * D * D + (size_t)(run * 16) * D + col;
+    float* og = q.og;
+    float S[16];
+    // the state belongs to the previous pass (and the buffer index with it): in the pass itself it is fetched ahead of the wait
+    if (og) {
+        const float* Sg = (q.state[1] ? q.S1 : q.S0) + Sat;
+#pragma unroll
+        for (int i = 0; i < 16; i++) S[i] = sz_ld32_here(Sg + (size_t)i * D);
+    }
+    sz_pdl_wait();
+    sz_pdl_trigger();
+    // A tree pass (tr != null): a row continues from the state after its PARENT.  Rows come parents first, so the state after a row
+    // that a later row branches off (tr->save) is kept in `fork` ([value head][row][D * D]) and fetched when a row's parent is not the
+    // row just before it.  The state the pass leaves in the other buffer is then that of no one path: the commit of a tree pass
+    // always replays, along the kept path res[2 ..] (row indices), where a chain's kept rows are simply 0 .. res[0] - 1.
+    int rows = q.m;
+    if (!og) {
+        rows = q.res[0];
+        if (rows <= 0 || (!tr && rows >= q.m)) return;
+    }
+    const int cur = q.state[1];
+    if (!og) {
+        const float* Sg = (cur ? q.S1 : q.S0) + Sat;
+#pragma unroll
+        for (int i = 0; i < 16; i++) S[i] = Sg[(size_t)i * D];
+    }
+    const float* xc = q.xc + (size_t)di * SZ_MAX_VERIFY * ch;          // (di > 0 in a replay only)
+    const float* beta = q.beta + (size_t)di * SZ_MAX_VERIFY * vh;
+    const float* decay = q.decay + (size_t)di * SZ_MAX_VERIFY * vh;
+    const bool fused = og != nullptr && q.pp.xin != nullptr;
+    float* fk = fork ? fork + ((size_t)di * vh + hd) * SZ_MAX_VERIFY * D * D : nullptr;
+    int prev_row = -1;
+    for (int c0 = 0; c0 < rows; c0 += SZ_SCAN_RC) {
+        const int nr = rows - c0 < SZ_SCAN_RC ? rows - c0 : SZ_SCAN_RC, par = (c0 / SZ_SCAN_RC) & 1;
+        if (fused) {
+            // ---- front end for this block's channels (forward.rs:829-861)
+            const SzDeltaPrep& pp = q.pp;
+            const float* conv = cur ? pp.conv1 : pp.conv0;
+            const int k = pp.k;
+            for (int idx = threadIdx.x; idx < nr * (2 * D + 32); idx += NT) {
+                const int j = idx / (2 * D + 32), c = idx - j * (2 * D + 32);
+                const int part3 = c < D ? 0 : (c < 2 * D ? 1 : 2), i = c - part3 * D;
+                const int chn = part3 == 0 ? kx * D + i : (part3 == 1 ? kd + kx * D + i : 2 * kd + hd * D + cb * 32 + i);
+                const float own = pp.xin[(size_t)j * ch + chn];
+                double acc = (double)pp.cw[chn * k + (k - 1)] * (double)own;
+                for (int t = 0; t < k - 1; t++) {
+                    const int tau = sz_tree_up(tr, j, (k - 1) - t);  // the row (k - 1) - t steps back: of this pass, or (negative) of the carried state
+                    const float prev = tau >= 0 ? pp.xin[(size_t)tau * ch + chn] : conv[(size_t)((k - 1) + tau) * ch + chn];
+                    acc += (double)pp.cw[chn * k + t] * (double)prev;
+                }
+                const float x = sz_silu((float)acc);
+                if (part3 == 0) sh.q[j][i] = x; else if (part3 == 1) sh.k[j][i] = x; else sh.v[j][i] = x;
+                // what a replay reads: v by every head, q and k once a key head (its first value head's blocks write 32 of them each)
+                const bool mine = part3 == 2 || (hd < kh && (i >> 5) == cb);
+                if (mine && pp.xsave) pp.xsave[(size_t)j * ch + chn] = own;
+                if (part3 == 2) pp.xc[(size_t)j * ch + chn] = x;
+            }
+            if (threadIdx.x < nr) {
+                const int j = threadIdx.x;
+                const float bt = sz_sigmoid(pp.b[j * vh + hd]);
+                const float sp_in = pp.a[j * vh + hd] + pp.dt[hd];
+                const float sp = sp_in > 20.0f ? sp_in : log1pf(expf(sp_in));
+                const float dc = expf(pp.a_log[hd] * sp);
+                sh.beta[j] = bt; sh.decay[j] = dc;
+                if (cb == 0) { pp.beta[j * vh + hd] = bt; pp.decay[j * vh + hd] = dc; }
+            }
+            __syncthreads();
+            // L2 norm of q and k (q also / sqrt(d)): a warp an item (row, q or k)
+            for (int it = run; it < nr * 2; it += RUNS) {
+                const int j = it >> 1, part3 = it & 1;
+                float* p = part3 ? sh.k[j] : sh.q[j];
+                double ss = 0.0;
+#pragma unroll
+                for (int i = 0; i < D / 32; i++) ss += (double)p[lane + 32 * i] * (double)p[lane + 32 * i];
+                ss = sz_warp_sum(ss);
+                const double nn = sz_rsqrt64(ss + 1e-6);
+#pragma unroll
+                for (int i = 0; i < D / 32; i++) {
+                    float t = (float)((double)p[lane + 32 * i] * nn);
+                    if (part3 == 0) t = t / sqrtf((float)D);
+                    p[lane + 32 * i] = t;
+                    if (hd < kh && i == cb) pp.xc[(size_t)j * ch + part3 * kd + kx * D + lane + 32 * i] = t;
+                }
+            }
+        } else {
+            for (int idx = threadIdx.x; idx < nr * (D / 2 + 8); idx += NT) {      // 16-byte pieces
+                const int jj = idx / (D / 2 + 8), c = idx - jj * (D / 2 + 8);
+                const int j = (!og && tr) ? q.res[2 + c0 + jj] : c0 + jj;           // replay of a tree pass: the kept path
+                const float* x = xc + (size_t)j * ch;
+                if (c < D / 4) ((float4*)sh.q[jj])[c] = __ldcg((const float4*)(x + kx * D) + c);
+                else if (c < D / 2) ((float4*)sh.k[jj])[c - D / 4] = __ldcg((const float4*)(x + kd + kx * D) + c - D / 4);
+                else ((float4*)sh.v[jj])[c - D / 2] = __ldcg((const float4*)(x + 2 * kd + hd * D + cb * 32) + c - D / 2);
+            }
+            if (threadIdx.x < nr) {
+                const int j = (!og && tr) ? q.res[2 + c0 + threadIdx.x] : c0 + (int)threadIdx.x;
+                sh.beta[threadIdx.x] = __ldcg(beta + (size_t)j * vh + hd); sh.decay[threadIdx.x] = __ldcg(decay + (size_t)j * vh + hd);
+            }
+        }
+        __syncthreads();
+        for (int jj = 0; jj < nr; jj++) {
+            const int j = (!og && tr) ? q.res[2 + c0 + jj] : c0 + jj;
+            if (tr && og) {
+                const int pr = tr->parents[j];
+                if (pr != prev_row && pr >= 0) {          // another branch: back to the state after the parent
+#pragma unroll
+                    for (int i = 0; i < 16; i++) S[i] = fk[((size_t)pr * D + run * 16 + i) * D + col];
+                }
+            }
+            prev_row = j;
+            const float dc = sh.decay[jj], bt = sh.beta[jj], vj = sh.v[jj][lane];
+            float kr[16], qr[16];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                *(float4*)(kr + 4 * i) = *(const float4*)(sh.k[jj] + run * 16 + 4 * i);
+                *(float4*)(qr + 4 * i) = *(const float4*)(sh.q[jj] + run * 16 + 4 * i);
+            }
+            float r = 0.f;
+#pragma unroll
+            for (int i = 0; i < 16; i++) { S[i] = S[i] * dc; r = fmaf(S[i], kr[i], r); }
+            sh.mem[jj & 1][run][lane] = (double)r;
+            __syncthreads();
+            const double tot = sz_scan_sum<D>([&](int w) { return sh.mem[jj & 1][w][lane]; });
+            const float dl = (float)(((double)vj - tot) * (double)bt);
+            r = 0.f;
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+                S[i] = __fadd_rn(S[i], __fmul_rn(kr[i], dl));  // unfused, as the CPU reference
+                r = fmaf(S[i], qr[i], r);
+            }
+            if (og) sh.orun[jj][run][lane] = r;
+            if (og && tr && ((tr->save >> j) & 1u)) {
+#pragma unroll
+                for (int i = 0; i < 16; i++) fk[((size_t)j * D + run * 16 + i) * D + col] = S[i];
+            }
+        }
+        __syncthreads();
+        if (og) {
+            for (int jj = run; jj < nr; jj += RUNS) sh.ofs[par][jj][lane] = (float)sz_scan_sum<D>([&](int w) { return (double)sh.orun[jj][w][lane]; });
+            sz_cluster_sync();       // (the other half of ofs is written next: a block that is one exchange ahead cannot reach this half)
+            // gated RMS norm of a row's D outputs: every block of the head sums them all and finishes its own
+            for (int jj = run; jj < nr; jj += RUNS) {
+                double ss = 0.0;
+#pragma unroll
+                for (int b = 0; b < D / 32; b++) {
+                    const float o = sz_cluster_ld(&sh.ofs[par][jj][lane], b);
+                    ss += (double)o * (double)o;
+                }
+                ss = sz_warp_sum(ss);
+                const double rr = sz_rsqrt64(ss / (double)D + (double)eps);
+                const size_t at = (size_t)(c0 + jj) * vh * D + hd * D + col;
+                const float normed = (float)((double)sh.ofs[par][jj][lane] * rr) * norm_w[col];
+                og[at] = normed * sz_sigmoid(q.z[at]);
+            }
+        }
+    }
+    float* So = (cur ? q.O0 : q.O1) + Sat;
+#pragma unroll
+    for (int i = 0; i < 16; i++) So[(size_t)i * D] = S[i];
+    if (og) sz_cluster_sync();       // no block leaves while another reads its outputs
+}
+
+// grid (vh * D / 32, layers), cluster D / 32
+template <int D>
+__global__ void __cluster_dims__(D / 32, 1, 1) __launch_bounds__(2 * D)
+sz_delta_scan_kernel(const SzScanSeq q, const float* __restrict__ norm_w, int kh, int vh, float eps, const SzTree* __restrict__ tr, float* __restrict__ fork) {
+    sz_delta_scan_body<D>(q, norm_w, kh, vh, eps, tr, fork, (int)blockIdx.x / (D / 32), (int)blockIdx.x % (D / 32), (int)blockIdx.y);
+}
+
+// The pass of one layer for SEVERAL sequences in one launch (a batched step, prompts): block row b is sequence b's scan, its pointers
+// and row count from a table.  grid (vh * D / 32, sequences); the arithmetic is the kernel above's.
+template <int D>
+__global__ void __cluster_dims__(D / 32, 1, 1) __launch_bounds__(2 * D)
+sz_delta_scan_seqs_kernel(const SzScanSeq* __restrict__ tab, const float* __restrict__ norm_w, int kh, int vh, float eps) {
+    __shared__ SzScanSeq q;   // (the entry in shared memory: two dozen pointers in registers would cost the kernel blocks)
+    static_assert(sizeof(SzScanSeq) % 8 == 0 && sizeof(SzScanSeq) / 8 <= 2 * 64, "copied in 8-byte words");
+    if (threadIdx.x < sizeof(SzScanSeq) / 8) ((u64*)&q)[threadIdx.x] = ((const u64*)(tab + blockIdx.y))[threadIdx.x];
+    __syncthreads();
+    sz_delta_scan_body<D>(q, norm_w, kh, vh, eps, (const SzTree*)nullptr, (float*)nullptr, (int)blockIdx.x / (D / 32), (int)blockIdx.x % (D / 32), 0);
+}
+
+// ---- attention front end (forward.rs:908-927): per head RMSNorm + NeoX RoPE of q and k, K and V into the cache.
 // grid (nh + 2 nkv, m), block 128.  Q8 cache: [kv head][pos][hd i8 | hd/32 f16 scales, zero-padded to 16 bytes] - the reference's packed
 // Q8_KV head (kernels/forward.cu:3652-3687), stored per head so that a range of positions of one head is contiguous; f32 cache:
 // [kv head][pos][hd].
@@ -938,15 +964,22 @@ __device__ __forceinline__ void sz_kv_store(const float* src, int hd, int q8, u8
 __global__ void __launch_bounds__(128)
 sz_attn_prep_kernel(const float* __restrict__ qg, const float* __restrict__ kk, const float* __restrict__ vv, const float* __restrict__ wq,
                     const float* __restrict__ wk, int nh, int nkv, int hd, int ctx, float eps, const int32_t* __restrict__ state, int rope_dims,
-                    const double* __restrict__ rope_den, int q8, u8* __restrict__ kc, u8* __restrict__ vc, float* __restrict__ q, float* __restrict__ gate,
-                    const SzTree* __restrict__ tr) {
+                    const double* __restrict__ rope_den, int q8, u8* __restrict__ kc, u8* __restrict__ vc, float* __restrict__ q,
+                    const SzTree* __restrict__ tr, const SzSeqDev* __restrict__ seqs, const SzRowDev* __restrict__ rws, int ai) {
     __shared__ float tmp[512];
     __shared__ double red[8];
+    const int b = blockIdx.x, j = blockIdx.y;
+    int jp = j;                                                // the row's place in its pass or chunk
+    if (rws) {                                                 // (a step of many rows: the row's sequence says where its cache is)
+        const SzSeqDev& sq = seqs[rws[j].seq];
+        jp = rws[j].j;
+        state = sq.state; ctx = sq.ctx;
+        kc = sq.kc + (size_t)ai * sq.kv_layer; vc = sq.vc + (size_t)ai * sq.kv_layer;
+    }
     sz_pdl_wait();
     sz_pdl_trigger();
-    const int b = blockIdx.x, j = blockIdx.y;
-    const int pos = state[0] + j;                              // the row's cache slot
-    const int rpos = state[0] + (tr ? tr->depth[j] : j);      // its position in the sequence (a tree: rows of one depth share it)
+    const int pos = state[0] + jp;                             // the row's cache slot
+    const int rpos = state[0] + (tr ? tr->depth[j] : jp);     // its position in the sequence (a tree: rows of one depth share it)
     const size_t hbytes = q8 ? (size_t)sz_kv_head_bytes(hd) : (size_t)hd * 4;  // the cache is [kv head][position][head bytes]
     if (b >= nh + nkv) {  // V head: raw into the cache
         const int h = b - nh - nkv;
@@ -979,10 +1012,7 @@ sz_attn_prep_kernel(const float* __restrict__ qg, const float* __restrict__ kk, 
     }
     __syncthreads();
     if (isq) {
-        for (int i = threadIdx.x; i < hd; i += 128) {
-            q[((size_t)j * nh + b) * hd + i] = tmp[i];
-            gate[((size_t)j * nh + b) * hd + i] = x[hd + i];
-        }
+        for (int i = threadIdx.x; i < hd; i += 128) q[((size_t)j * nh + b) * hd + i] = tmp[i];
     } else {
         const int h = b - nh;
         u8* dst = kc + ((size_t)h * ctx + pos) * hbytes;
@@ -1090,7 +1120,10 @@ template <int HD, int NQT>
 __global__ void __launch_bounds__(256)
 sz_attn2_kernel(const float* __restrict__ qin, const u8* __restrict__ kc, const u8* __restrict__ vc, int nh, int nkv, int m, int ctx,
                 const int32_t* __restrict__ state, int splits, float* __restrict__ part, u32* __restrict__ err, const SzTree* __restrict__ tr,
-                const int32_t* __restrict__ glist, const int32_t* __restrict__ gcount, int gstride, int ratio) {
+                const int32_t* __restrict__ glist, const int32_t* __restrict__ gcount, int gstride, int ratio, const SzSeqDev* __restrict__ seqs,
+                const SzAttnGroup* __restrict__ groups, int ai) {
+    // groups != null: a step of many rows, grid (kv heads, most splits, groups): up to 8 consecutive rows of one sequence, as a pass of
+    // that sequence at committed + j0 would carry them.
     // glist != null: the sparse form, grid (kv heads, splits, rows).  The block serves ONE row (blockIdx.z) and walks that row's list
     // of position groups (`ratio` positions each; row j's list at glist + j * gstride, gcount[j] long) instead of the positions
     // themselves.  A chunk of 64 list positions is then 64 / ratio copies of a group each for K and for V.
@@ -1108,6 +1141,18 @@ sz_attn2_kernel(const float* __restrict__ qin, const u8* __restrict__ kc, const 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g8 = lane >> 2, q4 = lane & 3;
     const int kvh = blockIdx.x, sp = blockIdx.y;
     const bool sparse = glist != nullptr;
+    int j0 = 0;
+    if (groups) {
+        const SzAttnGroup& gr = groups[blockIdx.z];
+        const SzSeqDev& sq = seqs[gr.seq];
+        splits = gr.splits;
+        if (sp >= splits) return;
+        j0 = gr.j0; m = gr.m;
+        state = sq.state; ctx = sq.ctx;
+        kc = sq.kc + (size_t)ai * sq.kv_layer; vc = sq.vc + (size_t)ai * sq.kv_layer;
+        qin += (size_t)gr.row0 * nh * HD;
+        part = gr.part;
+    }
     const int jz = sparse ? (int)blockIdx.z : 0;   // sparse: the one row of this block
     if (sparse) { glist += (size_t)jz * gstride; m = 1; }
     const int G = nh / nkv, QV = G * m;
@@ -1115,6 +1160,8 @@ sz_attn2_kernel(const float* __restrict__ qin, const u8* __restrict__ kc, const 
     // requested ahead of the dependency wait when it lies wholly there (the rows of this pass are written by the kernel before).
     int pos0;
     asm volatile("ld.global.s32 %0, [%1];" : "=r"(pos0) : "l"(state));
+    const int committed = pos0;
+    pos0 += j0;
     // (sparse: the list is written by the kernel before, so its length is read after the dependency wait, below)
     int nmax = pos0 + m;
     if (sparse) { sz_pdl_wait(); nmax = __ldcg(gcount + jz) * ratio; }
@@ -1123,7 +1170,7 @@ sz_attn2_kernel(const float* __restrict__ qin, const u8* __restrict__ kc, const 
     const int nchunk = t1 > t0 ? (t1 - t0 + SZ_AT_T - 1) / SZ_AT_T : 0;
     const u8* kbase = kc + (size_t)kvh * ctx * A::HB;
     const u8* vbase = vc + (size_t)kvh * ctx * A::HB;
-    const bool early = !sparse && nchunk > 0 && t0 + SZ_AT_T <= pos0;
+    const bool early = !sparse && nchunk > 0 && t0 + SZ_AT_T <= committed;
     if (threadIdx.x == 0) {
         sz_mbar_init(&bars[0], 1);
         sz_mbar_init(&bars[1], 1);
@@ -1370,15 +1417,18 @@ sz_attn2_kernel(const float* __restrict__ qin, const u8* __restrict__ kc, const 
 // thread each, the coefficients exp(max_s - max) go through shared memory, and the weighted sum over the splits runs in four
 // interleaved groups of threads so that many partial rows are in flight at once.
 __global__ void __launch_bounds__(256)
-sz_attn_merge_kernel(const float* __restrict__ part, const float* __restrict__ gate, int nh, int hd, int splits, float* __restrict__ o) {
+sz_attn_merge_kernel(const float* __restrict__ part, const float* __restrict__ qg, int nh, int hd, int splits, float* __restrict__ o,
+                     const SzRowDev* __restrict__ rws) {
+    // qg: the rows' query projections, [row][head][query, gate]; rws != null: a step of many rows, each with its own partial results
     __shared__ float coef[512];
     __shared__ float red[8];
     __shared__ float accs[4][256];
     sz_pdl_wait();
     sz_pdl_trigger();
     const int h = blockIdx.x, j = blockIdx.y, t = threadIdx.x, warp = t >> 5, lane = t & 31;
-    const float* p = part + ((size_t)j * nh + h) * splits * (hd + 2);
-    const float g = t < hd ? __ldcg(gate + ((size_t)j * nh + h) * hd + t) : 0.f;
+    if (rws) splits = rws[j].splits;
+    const float* p = (rws ? rws[j].part + (size_t)h * splits * (hd + 2) : part + ((size_t)j * nh + h) * splits * (hd + 2));
+    const float g = t < hd ? __ldcg(qg + (((size_t)j * nh + h) * 2 + 1) * hd + t) : 0.f;
     float mm[2], zz[2];
     float M = -INFINITY;
 #pragma unroll
