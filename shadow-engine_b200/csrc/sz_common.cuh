@@ -156,6 +156,17 @@ __device__ __forceinline__ double sz_rsqrt64(double v) {
 
 __device__ __forceinline__ float sz_silu(float x) { return x * sz_sigmoid(x); }
 
+// ---- small asynchronous copies, global -> shared --------------------------------------------------------------------------
+__device__ __forceinline__ void sz_cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((u32)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void sz_cp_async4(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((u32)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void sz_cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void sz_cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
 // ---- thread-block clusters --------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void sz_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");

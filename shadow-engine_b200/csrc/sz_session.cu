@@ -625,54 +625,30 @@ static bool sz_dense_q8_takes(const SzDenseArgs& a) {
     return false;
 }
 
-int sz_dense_rows_launch(SzDenseArgs& a, float* partial, int64_t partial_floats, cudaStream_t st, const char* name, int* taken) {
+int sz_dense_rows_launch(SzDenseArgs& a, void* xh, cudaStream_t st, const char* name, int* taken) {
     *taken = 0;
     if (a.m < 8 || a.m % 8 || !sz_dense_q8_takes(a)) return SZ_OK;
     int total = 0;
     for (int i = 0; i < a.n_jobs; i++) { a.job[i].row0 = total; total += a.job[i].rows; }
     a.total_rows = total;
-    if ((int64_t)8 * a.m * total > partial_floats) return SZ_OK;
     SzDenseRowsCfg c = {};
     int units = 0;
     for (int i = 0; i < a.n_jobs; i++) { c.units[i] = units; units += (a.job[i].rows + 15) / 16; }
     c.units[a.n_jobs] = units;
-    const int part = a.cols / 8;
-    c.sb = part / 32 * 34;
-    int rs = 0;
-    for (int p = 0; p < 8; p++) { const int need = ((((p * c.sb) & 15) + c.sb + 15) >> 4) << 4; rs = need > rs ? need : rs; }
-    while (((rs / 4) % 32) % 8 != 4) rs += 16;     // staged slices 4 (mod 8) words apart, rows of the pass 16 words, as the 8-row kernel
-    int xs = part;
-    while (((xs / 2) % 32) != 16) xs += 8;
-    c.rs = rs; c.xs = xs; c.rows = a.m; c.G = a.m / 8; c.partial = partial;
-    // row groups a block: what fits beside the two stages, two blocks a multiprocessor where four groups do
-    const size_t stages = 2 * (size_t)128 * rs, group = (size_t)8 * xs * 4;
-    int gb = 0;
-    if (stages + 4 * group <= 110 * 1024) gb = 4;
-    else if (c.G >= 8 && stages + 8 * group <= 216 * 1024) gb = 8;
-    else if (stages + 4 * group <= 216 * 1024) gb = 4;
-    else if (stages + 2 * group <= 216 * 1024) gb = 2;
-    else return SZ_OK;
-    if (c.G <= 2) gb = 2;
-    c.gb = gb;
-    c.nz = (c.G + gb - 1) / gb;
-    const size_t smem = stages + (size_t)gb * group;
-    const int target = sz_sm_count_session() * (smem <= 110 * 1024 ? 2 : 1);
-    int nc = target / (8 * c.nz);
-    if (nc < 1) nc = 1;
-    c.upc = ((units + nc - 1) / nc + 7) / 8 * 8;
-    nc = (units + c.upc - 1) / c.upc;
-    const dim3 grid(8, nc, c.nz);
-    cudaError_t e = cudaErrorInvalidValue;
-#define SZ_DR(GG)                                                                                                                            \
-    if (gb == GG) {                                                                                                                          \
-        static bool set = false;                                                                                                             \
-        if (!set) { SZ_CUDA(cudaFuncSetAttribute(sz_dense_rows_q8_kernel<GG>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)); set = true; } \
-        e = sz_launch(name, sz_dense_rows_q8_kernel<GG>, grid, dim3(256), smem, st, true, a, c);                                             \
+    c.rows = a.m;
+    c.xh = (const __half*)xh;
+    SZ_CUDA(sz_launch("dense_rows_pack", sz_dense_rows_pack_kernel, dim3((a.cols + 1023) / 1024, a.m), dim3(256), 0, st, true, a.x, a.xstride, a.cols, a.m, (__half*)xh));
+    const int tiles = (a.m + 31) / 32, sms = sz_sm_count_session();
+    // two units a warp (a row group's fragments loaded once for both) where that still leaves a thread block for every multiprocessor
+    const bool two = (units + 15) / 16 * tiles >= sms - sms / 8;
+    static bool set = false;
+    if (!set) {
+        SZ_CUDA(cudaFuncSetAttribute(sz_dense_rows_q8_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SzDenseRows<1>::SMEM));
+        SZ_CUDA(cudaFuncSetAttribute(sz_dense_rows_q8_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SzDenseRows<2>::SMEM));
+        set = true;
     }
-    SZ_DR(2) SZ_DR(4) SZ_DR(8)
-#undef SZ_DR
-    SZ_CUDA(e);
-    SZ_CUDA(sz_launch("dense_rows_reduce", sz_dense_rows_reduce_kernel, dim3((total + 255) / 256, a.m), dim3(256), 0, st, true, a, (const float*)partial, a.m));
+    if (two) SZ_CUDA(sz_launch(name, sz_dense_rows_q8_kernel<2>, dim3((units + 15) / 16, tiles), dim3(256), SzDenseRows<2>::SMEM, st, true, a, c));
+    else SZ_CUDA(sz_launch(name, sz_dense_rows_q8_kernel<1>, dim3((units + 7) / 8, tiles), dim3(256), SzDenseRows<1>::SMEM, st, true, a, c));
     *taken = 1;
     return SZ_OK;
 }
@@ -771,7 +747,7 @@ static int sz_hc_read(sz_session* s, cudaStream_t st, const sz_hc& hc, int m, bo
 
 // The fused read over the rows of a batch: buffers that hold the rows of all sequences one after the other (a multiple of 8 rows,
 // the sequences' own buffers pointing into them), eight rows a block row of the two kernels.  n: the read's number in the pass.
-struct SzBatchBufs { float *r, *r2, *y, *u, *rn; long long* acc; int64_t acc_stride; };
+struct SzBatchBufs { float *r, *r2, *y, *u, *rn; long long* acc; int64_t acc_stride; float* hd; };
 static int sz_hc_read_rows(const sz_session* s, cudaStream_t st, const sz_hc& hc, int rows, int n, bool pending, bool inject, const SzBatchBufs& B, bool pdl) {
     const sz_model_config& c = s->model.cfg;
     const int H = c.hidden, C = c.streams, CH = C * H;
@@ -790,6 +766,32 @@ static int sz_hc_read_rows(const sz_session* s, cudaStream_t st, const sz_hc& hc
     // kernel with a block row per `per` rows, where every block of a stream redoes the stream's norm; same bits).
     const char* sp = getenv("SZ_BATCH_HC_SPLIT");   // (read at every call: a test switches it inside one process)
     if (!(sp && atoi(sp) == 0)) {
+        // at the usual shape the two products in their own many-row form; elsewhere as block rows of the pass's kernels
+        const bool wide = B.hd && c.hc_rank == 256 && C == 4 && CH % (16 * SZ_HC_K) == 0;
+        if (wide) {
+            SZ_CUDA(sz_launch("hc_rows_norm", sz_hc_rows_norm_kernel, dim3(C, rows), dim3(nt), 0, st, pdl, (const float*)rin, rout,
+                              (const long long*)(pending ? acc_prev : nullptr), (const float*)B.y, (const float*)hc.norm.data, H, C, (int)c.hc_rank, c.eps,
+                              B.rn, acc_next));
+            static bool set = false;
+            if (!set) {
+                SZ_CUDA(cudaFuncSetAttribute(sz_hc_down_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024));
+                SZ_CUDA(cudaFuncSetAttribute(sz_hc_up_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SzHcUpRows::SMEM));
+                set = true;
+            }
+            // Few rows: a thread a matrix row and 8 rows of the step a block (28 us at 80 rows, where the tiled form has 40 blocks of the
+            // chip's 148 and takes 46); from 129 rows on the tiles (68 us at 256 against 82), the columns in 16 parts of 512.
+            if (rows <= 128) {
+                SZ_CUDA(sz_launch("hc_rows_down", sz_hc_rows_down_kernel<8>, dim3(CH / 64, rows / 8), dim3(nt), 0, st, true, (const float*)B.rn, (const u8*)hc.down.data,
+                                  (const u8*)(inject ? hc.inject.data : 0), H, C, (int)c.hc_rank, acc));
+                SZ_CUDA(sz_launch("hc_rows_act", sz_hc_rows_act_kernel, dim3(rows), dim3(256), 0, st, true, (const long long*)acc, C, B.hd));
+            } else {
+                SZ_CUDA(sz_launch("hc_down_rows", sz_hc_down_rows_kernel, dim3(16, (rows + SZ_HC_M - 1) / SZ_HC_M), dim3(288), sz_hc_down_rows_smem(CH / 16), st, true,
+                                  (const float*)B.rn, (const u8*)hc.down.data, (const u8*)(inject ? hc.inject.data : 0), H, rows, B.hd, acc));
+            }
+            SZ_CUDA(sz_launch("hc_up_rows", sz_hc_up_rows_kernel, dim3(H / 16, (rows + SZ_HC_UP_ROWS - 1) / SZ_HC_UP_ROWS), dim3(128), SzHcUpRows::SMEM, st, true,
+                              (const float*)B.hd, (const u8*)hc.up.data, (const float*)B.rn, H, rows, B.u));
+            return SZ_OK;
+        }
         SZ_CUDA(sz_launch("hc_rows_norm", sz_hc_rows_norm_kernel, dim3(C, rows), dim3(nt), 0, st, pdl, (const float*)rin, rout,
                           (const long long*)(pending ? acc_prev : nullptr), (const float*)B.y, (const float*)hc.norm.data, H, C, (int)c.hc_rank, c.eps,
                           B.rn, acc_next));
@@ -1568,7 +1570,7 @@ sz_batch_move_kernel(const SzBatchTab* __restrict__ T, float* const* __restrict_
 }
 
 enum { SZ_BATCH_SLOTS = SZ_DENSE_MAX_JOBS + 1 };   // per layer: the outputs of the input projections, then the input of the output projection
-struct SzBatchScratch { int64_t up, up_bytes, rtab, groups, rids, aq, xc, beta, decay, tab, ptrs, ptrs_bytes, scan, scan_bytes, x, y, r, r2, rn, acc, in, in_row, core, core_row, partial, partial_floats, moe, moe_bytes, total; };
+struct SzBatchScratch { int64_t up, up_bytes, rtab, groups, rids, hd, xh, aq, xc, beta, decay, tab, ptrs, ptrs_bytes, scan, scan_bytes, x, y, r, r2, rn, acc, in, in_row, core, core_row, partial, partial_floats, moe, moe_bytes, total; };
 static int sz_batch_layout(const sz_model* m, int rows_max, SzBatchScratch* S) {
     if (!m || !m->layers) return sz_fail(SZ_E_ARG, "null model");
     if (rows_max < 8 || rows_max % 8) return sz_fail(SZ_E_ARG, "sz_batch: rows_max = %d (a multiple of 8)", rows_max);
@@ -1604,12 +1606,15 @@ static int sz_batch_layout(const sz_model* m, int rows_max, SzBatchScratch* S) {
     S->core_row = vd > (int64_t)c.n_head * c.head_dim ? vd : (int64_t)c.n_head * c.head_dim;
     S->in = o; o = up256(o + 4 * rows_max * S->in_row);
     S->core = o; o = up256(o + 4 * rows_max * S->core_row);
+    S->hd = o; o = up256(o + 4 * rows_max * (int64_t)c.hc_rank);
     S->aq = o; o = up256(o + 4 * rows_max * (int64_t)c.n_head * c.head_dim);
     S->xc = o; o = up256(o + 4 * rows_max * (2 * kd + vd));
     S->beta = o; o = up256(o + 4 * (int64_t)rows_max * c.ssm_v_heads);
     S->decay = o; o = up256(o + 4 * (int64_t)rows_max * c.ssm_v_heads);
-    // the many-row projection kernel's sums of the eight column parts, for the widest set of projections
-    S->partial_floats = 8 * (int64_t)rows_max * (S->in_row > c.hidden ? S->in_row : c.hidden);
+    // the many-row projections' rows as f16 high and low parts; attention splits' partial results of a prompt's chunks (a bounded number
+    // of rows at once: the more splits a row has, the fewer rows)
+    S->xh = o; o = up256(o + 4 * rows_max * (S->core_row > c.hidden ? S->core_row : (int64_t)c.hidden));
+    S->partial_floats = 8 * (int64_t)rows_max * c.n_head * (c.head_dim + 2);
     S->partial = o; o = up256(o + 4 * S->partial_floats);
     for (int l = 0; l < c.n_layer; l++) {
         int64_t b = 0;
@@ -1710,7 +1715,7 @@ static int sz_rows_layers(sz_session* const* ss, int n, const int32_t* ids, cons
         row += ms[b];
     }
     // Attention in batches of consecutive rows whose partial results fit: a sequence's first group of a batch leaves them in its
-    // session's own buffer (8 rows of them), further ones in what the projections' partial sums use at other times.
+    // session's own buffer (8 rows of them), further ones in the step's.
     float* PART = (float*)(base + S.partial);
     int ng_all = 0;
     {
@@ -1749,7 +1754,8 @@ static int sz_rows_layers(sz_session* const* ss, int n, const int32_t* ids, cons
     const SzAttnGroup* groups = (const SzAttnGroup*)(base + S.groups);
     float *X = (float*)(base + S.x), *Y = (float*)(base + S.y), *IN = (float*)(base + S.in), *CORE = (float*)(base + S.core), *AQ = (float*)(base + S.aq);
     float *XC = (float*)(base + S.xc), *BETA = (float*)(base + S.beta), *DECAY = (float*)(base + S.decay);
-    SzBatchBufs BB = {(float*)(base + S.r), (float*)(base + S.r2), Y, X, (float*)(base + S.rn), (long long*)(base + S.acc), (int64_t)rows_max * SZ_HC_ACC_ROWS};
+    void* XH = base + S.xh;
+    SzBatchBufs BB = {(float*)(base + S.r), (float*)(base + S.r2), Y, X, (float*)(base + S.rn), (long long*)(base + S.acc), (int64_t)rows_max * SZ_HC_ACC_ROWS, (float*)(base + S.hd)};
     SZ_CUDA(cudaMemsetAsync(BB.acc, 0, sizeof(long long) * (size_t)Rp * SZ_HC_ACC_ROWS, st));   // read 0 adds into accumulator 0
     SZ_CUDA(sz_launch("rows_embed", sz_rows_embed_kernel, dim3(R + n), dim3(256), 0, st, false, seqs, (const int32_t*)(base + S.rids), R,
                       (const u8*)s0->model.token_embd.data, (int)s0->model.token_embd.type, (int)c.hidden, (int)c.streams, (int)c.vocab, BB.r));
@@ -1761,7 +1767,7 @@ static int sz_rows_layers(sz_session* const* ss, int n, const int32_t* ids, cons
         ar.m = Rp; ar.x = x;
         for (int k = 0; k < a.n_jobs; k++) ar.job[k].out = outs[k];
         int taken = 0, r;
-        if (rows_form && (r = sz_dense_rows_launch(ar, PART, S.partial_floats, st, name, &taken))) return r;
+        if (rows_form && (r = sz_dense_rows_launch(ar, XH, st, name, &taken))) return r;
         for (int g = 0; g < Rp / 8 && !taken; g++) {
             SzDenseArgs ag = a;
             ag.m = 8; ag.x = x + (size_t)g * 8 * a.cols;
@@ -1963,7 +1969,7 @@ static int sz_batch_step(sz_session* const* ss, int n, const int32_t* ids, const
     const bool shared_off = se && atoi(se) == 0;
     const bool shared = !shared_off && n > 1 && s0->hc_fast;
     const int64_t CH = (int64_t)c.streams * c.hidden;
-    SzBatchBufs BB = {(float*)(base + S.r), (float*)(base + S.r2), Y, X, (float*)(base + S.rn), (long long*)(base + S.acc), (int64_t)rows_max * SZ_HC_ACC_ROWS};
+    SzBatchBufs BB = {(float*)(base + S.r), (float*)(base + S.r2), Y, X, (float*)(base + S.rn), (long long*)(base + S.acc), (int64_t)rows_max * SZ_HC_ACC_ROWS, nullptr};
     struct Repoint {   // the sessions' buffers while they point into the batch's: put back however the step ends
         sz_session* const* ss = nullptr;
         int n = 0;
@@ -1976,7 +1982,7 @@ static int sz_batch_step(sz_session* const* ss, int n, const int32_t* ids, const
         }
     } repoint;
     float* const* ptrs = (float* const*)(base + S.ptrs);
-    float* PART = (float*)(base + S.partial);
+    void* XH = base + S.xh;
     const char* re = getenv("SZ_BATCH_DENSE_ROWS");   // 0: the projections 8 rows a launch (the second form; same bits)
     const bool rows_form = !(re && atoi(re) == 0);
     // the DeltaNet scans of a layer, all sequences in one launch from a table of their pointers (0, or the generic kernels: a launch
@@ -2096,7 +2102,7 @@ static int sz_batch_step(sz_session* const* ss, int n, const int32_t* ids, const
                 ar.m = Rp; ar.x = X;
                 for (int k = 0; k < a.n_jobs; k++) ar.job[k].out = IN + mi.off[k];
                 int taken = 0;
-                if (rows_form && (rc = sz_dense_rows_launch(ar, PART, S.partial_floats, st, "batch_proj", &taken))) return rc;
+                if (rows_form && (rc = sz_dense_rows_launch(ar, XH, st, "batch_proj", &taken))) return rc;
                 for (int g = 0; g < Rp / 8 && !taken; g++) {
                     SzDenseArgs ag = a;
                     ag.x = X + (size_t)g * 8 * c.hidden;
@@ -2121,7 +2127,7 @@ static int sz_batch_step(sz_session* const* ss, int n, const int32_t* ids, const
                 SzDenseArgs orr = o;
                 orr.m = Rp; orr.x = CORE; orr.job[0].out = Y;
                 int taken = 0;
-                if (rows_form && (rc = sz_dense_rows_launch(orr, PART, S.partial_floats, st, "batch_out", &taken))) return rc;
+                if (rows_form && (rc = sz_dense_rows_launch(orr, XH, st, "batch_out", &taken))) return rc;
                 for (int g = 0; g < Rp / 8 && !taken; g++) {
                     SzDenseArgs og = o;
                     og.x = CORE + (size_t)g * 8 * o.cols;
