@@ -171,6 +171,8 @@ __device__ __forceinline__ void sz_cp_async_wait() { asm volatile("cp.async.wait
 __device__ __forceinline__ void sz_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+__device__ __forceinline__ void sz_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void sz_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // the f32 at `p` (an address in this block's shared memory) as block `rank` of the cluster has it
 __device__ __forceinline__ float sz_cluster_ld(const float* p, int rank) {
     u32 a;

@@ -54,14 +54,16 @@ __device__ __forceinline__ void sz_warp_sum_many(double* v, int lane) {
 // wait) and of the M rows of the pass, so nothing is staged in shared memory and every product is formed and added in f64 with one
 // conversion a weight.  The 4 x M partial sums a thread ends with are summed over the warp (sz_warp_sum_many), then over the 8 warps
 // in warp order.  M: rows of the pass; MP: M rounded up to a power of two; NCH: float4 pieces a thread holds per row.
-template <int M, int MP, int NCH>
+// LOOP (many rows: sz_moe_rows): a block takes every gridDim.x-th group of 4 router rows, so that its rows of the pass are loaded and converted
+// to f64 once for all of them (a block a group had each of 129 blocks do it: 126 us at 256 rows, L2 traffic and conversions).
+template <int M, int MP, int NCH, bool LOOP>
 __global__ void __launch_bounds__(SZ_ROUTE_THREADS)
 sz_route_kernel(const float* __restrict__ x, int H, const float* __restrict__ router, const float* __restrict__ shared_router,
                 int ne, int k, float* __restrict__ logits, int32_t* __restrict__ ridx, double* __restrict__ rw, SzPlan* __restrict__ plan,
                 SzPlan* __restrict__ plan_sh, u32* __restrict__ ctrl, int32_t* __restrict__ out_idx, double* __restrict__ out_w,
                 uint4* __restrict__ zero, int zero_n, int ep_first, int ep_count) {
     constexpr int RB = SZ_ROUTE_RB, N = RB * MP;
-    __shared__ double part[SZ_ROUTE_THREADS / 32][N];
+    __shared__ double part[LOOP ? 2 : 1][SZ_ROUTE_THREADS / 32][N];
     __shared__ u32 rowmask[SZ_MAX_EXPERTS];     // which rows of the pass chose expert e
     __shared__ u32 bitmap[SZ_MAX_EXPERTS / 32]; // experts chosen at all (and held here)
     __shared__ int sel[SZ_MAX_VERIFY * SZ_MAX_TOPK];
@@ -87,19 +89,22 @@ sz_route_kernel(const float* __restrict__ x, int H, const float* __restrict__ ro
     SZ_PH();  // 0 start
     // the router rows do not depend on the previous kernel: fetched before waiting for it
     float4 w[RB][NCH];
+    auto fetch = [&](int r0) {
 #pragma unroll
-    for (int r = 0; r < RB; r++) {
-        const int row = row0 + r;
-        const float4* wrow = (const float4*)(row < ne ? router + (size_t)row * H : shared_router);
+        for (int r = 0; r < RB; r++) {
+            const int row = r0 + r;
+            const float4* wrow = (const float4*)(row < ne ? router + (size_t)row * H : shared_router);
 #pragma unroll
-        for (int u = 0; u < NCH; u++) {
-            w[r][u] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (row < nrows && t + 256 * u < H / 4) {
-                const uint4 q = sz_ldg16_here(wrow + t + 256 * u);
-                w[r][u] = make_float4(__uint_as_float(q.x), __uint_as_float(q.y), __uint_as_float(q.z), __uint_as_float(q.w));
+            for (int u = 0; u < NCH; u++) {
+                w[r][u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (row < nrows && t + 256 * u < H / 4) {
+                    const uint4 q = sz_ldg16_here(wrow + t + 256 * u);
+                    w[r][u] = make_float4(__uint_as_float(q.x), __uint_as_float(q.y), __uint_as_float(q.z), __uint_as_float(q.w));
+                }
             }
         }
-    }
+    };
+    fetch(row0);
     for (int i = t; i < SZ_MAX_EXPERTS; i += SZ_ROUTE_THREADS) rowmask[i] = 0u;
     if (t < SZ_MAX_EXPERTS / 32) bitmap[t] = 0u;
     sz_pdl_wait();
@@ -115,39 +120,76 @@ sz_route_kernel(const float* __restrict__ x, int H, const float* __restrict__ ro
     for (int i = blockIdx.x * blockDim.x + t; i < zero_n; i += gridDim.x * blockDim.x) zero[i] = make_uint4(0, 0, 0, 0);
 
     // ---- logits: f64 products, f64 sums
-    double acc[N];
+    constexpr int HB = N == 1 ? 0 : (N == 2 ? 1 : (N == 4 ? 2 : (N == 8 ? 3 : (N == 16 ? 4 : 5))));  // log2(N), N <= 32
+    auto finish = [&](int r0, const double (*p)[N]) {      // the warps' sums in warp order
+        if (t < N) {
+            double s = 0.0;
 #pragma unroll
-    for (int i = 0; i < N; i++) acc[i] = 0.0;
+            for (int q = 0; q < SZ_ROUTE_THREADS / 32; q++) s += p[q][t];
+            const int r = t / MP, j = t % MP;
+            if (j < M && r0 + r < nrows) logits[(size_t)j * ld + r0 + r] = (float)s;
+        }
+    };
+    if constexpr (LOOP) {
+        double xd[M][NCH][4];
 #pragma unroll
-    for (int u = 0; u < NCH; u++) {
-        double xd[M][4];
+        for (int j = 0; j < M; j++)
 #pragma unroll
-        for (int j = 0; j < M; j++) { xd[j][0] = (double)xv[j][u].x; xd[j][1] = (double)xv[j][u].y; xd[j][2] = (double)xv[j][u].z; xd[j][3] = (double)xv[j][u].w; }
+            for (int u = 0; u < NCH; u++) { xd[j][u][0] = (double)xv[j][u].x; xd[j][u][1] = (double)xv[j][u].y; xd[j][u][2] = (double)xv[j][u].z; xd[j][u][3] = (double)xv[j][u].w; }
+        int par = 0;
+        for (int r0 = row0; r0 < nrows; r0 += RB * gridDim.x, par ^= 1) {
+            double acc[N];
 #pragma unroll
-        for (int r = 0; r < RB; r++) {
-            const double w0 = (double)w[r][u].x, w1 = (double)w[r][u].y, w2 = (double)w[r][u].z, w3 = (double)w[r][u].w;
+            for (int i = 0; i < N; i++) acc[i] = 0.0;
 #pragma unroll
-            for (int j = 0; j < M; j++) {
-                double a = acc[r * MP + j];
-                a = fma(w0, xd[j][0], a);
-                a = fma(w1, xd[j][1], a);
-                a = fma(w2, xd[j][2], a);
-                a = fma(w3, xd[j][3], a);
-                acc[r * MP + j] = a;
+            for (int u = 0; u < NCH; u++)
+#pragma unroll
+                for (int r = 0; r < RB; r++) {
+                    const double w0 = (double)w[r][u].x, w1 = (double)w[r][u].y, w2 = (double)w[r][u].z, w3 = (double)w[r][u].w;
+#pragma unroll
+                    for (int j = 0; j < M; j++) {
+                        double a = acc[r * MP + j];
+                        a = fma(w0, xd[j][u][0], a);
+                        a = fma(w1, xd[j][u][1], a);
+                        a = fma(w2, xd[j][u][2], a);
+                        a = fma(w3, xd[j][u][3], a);
+                        acc[r * MP + j] = a;
+                    }
+                }
+            if (r0 + RB * (int)gridDim.x < nrows) fetch(r0 + RB * gridDim.x);
+            sz_warp_sum_many<N>(acc, lane);
+            if ((lane & ((32 >> HB) - 1)) == 0) part[par][warp][lane >> (5 - HB)] = acc[0];
+            __syncthreads();
+            finish(r0, part[par]);
+        }
+    } else {
+        double acc[N];
+#pragma unroll
+        for (int i = 0; i < N; i++) acc[i] = 0.0;
+#pragma unroll
+        for (int u = 0; u < NCH; u++) {
+            double xd[M][4];
+#pragma unroll
+            for (int j = 0; j < M; j++) { xd[j][0] = (double)xv[j][u].x; xd[j][1] = (double)xv[j][u].y; xd[j][2] = (double)xv[j][u].z; xd[j][3] = (double)xv[j][u].w; }
+#pragma unroll
+            for (int r = 0; r < RB; r++) {
+                const double w0 = (double)w[r][u].x, w1 = (double)w[r][u].y, w2 = (double)w[r][u].z, w3 = (double)w[r][u].w;
+#pragma unroll
+                for (int j = 0; j < M; j++) {
+                    double a = acc[r * MP + j];
+                    a = fma(w0, xd[j][0], a);
+                    a = fma(w1, xd[j][1], a);
+                    a = fma(w2, xd[j][2], a);
+                    a = fma(w3, xd[j][3], a);
+                    acc[r * MP + j] = a;
+                }
             }
         }
-    }
-    SZ_PH();  // 2 products
-    constexpr int HB = N == 1 ? 0 : (N == 2 ? 1 : (N == 4 ? 2 : (N == 8 ? 3 : (N == 16 ? 4 : 5))));  // log2(N), N <= 32
-    sz_warp_sum_many<N>(acc, lane);
-    if ((lane & ((32 >> HB) - 1)) == 0) part[warp][lane >> (5 - HB)] = acc[0];
-    __syncthreads();
-    if (t < N) {
-        double s = 0.0;
-#pragma unroll
-        for (int q = 0; q < SZ_ROUTE_THREADS / 32; q++) s += part[q][t];
-        const int r = t / MP, j = t % MP;
-        if (j < M && row0 + r < nrows) logits[(size_t)j * ld + row0 + r] = (float)s;
+        SZ_PH();  // 2 products
+        sz_warp_sum_many<N>(acc, lane);
+        if ((lane & ((32 >> HB) - 1)) == 0) part[0][warp][lane >> (5 - HB)] = acc[0];
+        __syncthreads();
+        finish(row0, part[0]);
     }
 
     // ---- the last block to arrive routes every row
@@ -889,7 +931,7 @@ static int sz_moe_run(const sz_moe_layer* L0, uint64_t x, int m, float* y, long 
         const int nch = (H / 4 + SZ_ROUTE_THREADS - 1) / SZ_ROUTE_THREADS;
         cudaError_t e = cudaErrorInvalidValue;
 #define SZ_ROUTE_GO(MM, MPP, NC)                                                                                                         \
-    e = sz_launch("route", sz_route_kernel<MM, MPP, NC>, grid, block, 0, st, true, xp, H, (const float*)L->router,                       \
+    e = sz_launch("route", sz_route_kernel<MM, MPP, NC, false>, grid, block, 0, st, true, xp, H, (const float*)L->router,                       \
                   (const float*)(shared ? L->shared_router : 0), (int)L->n_expert, (int)L->top_k, logits, ridx, rw, plan, plan_sh, ctrl, \
                   (int32_t*)route_idx, (double*)route_w, (uint4*)(base + S.acc_gu), fast.exl3 ? (int)(S.acc_bytes / 16) : 0,             \
                   (int)L->ep_first, (int)L->ep_count)
@@ -1073,14 +1115,18 @@ static int sz_rows_run(const sz_moe_layer* L, uint64_t x, int rows, int live, ui
     SzRowsPlan* P = (SzRowsPlan*)(base + S.plan);
     {   // routing: 8 rows a block row of the verify pass's router kernel (the chunks' own plans are written and not used)
         const int route_rows = L->n_expert + (shared ? 1 : 0);
-        const dim3 grid((route_rows + SZ_ROUTE_RB - 1) / SZ_ROUTE_RB, chunks), block(SZ_ROUTE_THREADS);
+        const int groups = (route_rows + SZ_ROUTE_RB - 1) / SZ_ROUTE_RB;
+        int gx = sz_sm_count() / chunks;                 // about one block a multiprocessor over all chunks of 8 rows
+        gx = gx < 1 ? 1 : (gx > groups ? groups : gx);
+        if (H > 2048) gx = groups;                       // (wider rows do not stay in registers as f64: a block a group)
+        const dim3 grid(gx, chunks), block(SZ_ROUTE_THREADS);
         const int nch = (H / 4 + SZ_ROUTE_THREADS - 1) / SZ_ROUTE_THREADS;
         cudaError_t e = cudaErrorInvalidValue;
-#define SZ_ROWS_ROUTE(NC)                                                                                                                  \
-    e = sz_launch("route_rows", sz_route_kernel<8, 8, NC>, grid, block, 0, st, true, (const float*)x, H, (const float*)L->router,           \
+#define SZ_ROWS_ROUTE(NC, LOOP)                                                                                                            \
+    e = sz_launch("route_rows", sz_route_kernel<8, 8, NC, LOOP>, grid, block, 0, st, true, (const float*)x, H, (const float*)L->router,           \
                   (const float*)(shared ? L->shared_router : 0), (int)L->n_expert, (int)L->top_k, logits, ridx, rw, (SzPlan*)(base + S.cplan), \
                   (SzPlan*)(base + S.cplan_sh), ctrl, (int32_t*)route_idx, (double*)route_w, (uint4*)nullptr, 0, 0, 0)
-        if (nch <= 1) SZ_ROWS_ROUTE(1); else if (nch == 2) SZ_ROWS_ROUTE(2); else SZ_ROWS_ROUTE(4);
+        if (nch <= 1) SZ_ROWS_ROUTE(1, true); else if (nch == 2) SZ_ROWS_ROUTE(2, true); else SZ_ROWS_ROUTE(4, false);
 #undef SZ_ROWS_ROUTE
         SZ_CUDA(e);
     }

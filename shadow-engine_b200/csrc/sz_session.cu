@@ -1804,7 +1804,7 @@ static int sz_rows_layers(sz_session* const* ss, int n, const int32_t* ids, cons
             SZ_CUDA(sz_launch("rows_delta_prep", sz_rows_delta_prep_kernel, dim3((ch + 255) / 256, R), dim3(256), 0, st, true, seqs, rws, di, (const float*)outs[0],
                               (const float*)L.ssm_conv1d.data, (const float*)outs[2], (const float*)outs[3], (const float*)L.ssm_a.data, (const float*)L.ssm_dt_bias.data,
                               kh, vh, d, (int)c.conv_k, XC, BETA, DECAY));
-            SZ_CUDA(sz_launch("rows_scan", d == 128 ? sz_rows_scan_kernel<128> : sz_rows_scan_kernel<64>, dim3(vh * (d / 32), n), dim3(2 * d), 0, st, true, seqs, di,
+            SZ_CUDA(sz_launch("rows_scan", d == 128 ? sz_rows_scan_kernel<128> : sz_rows_scan_kernel<64>, dim3(vh * (d / 32), n), dim3(d), 0, st, true, seqs, di,
                               (const float*)XC, (const float*)BETA, (const float*)DECAY, (const float*)outs[1], (const float*)L.ssm_norm.data, kh, vh, c.eps, CORE));
         }
         float* yo[1] = {Y};

@@ -682,18 +682,22 @@ __global__ void sz_state_update_kernel(int32_t* __restrict__ state, const int32_
 }
 
 // ---- DeltaNet state scan (forward.rs:859-894) ---------------------------------------------------------------------------------------
-// Per value head a D x D state whose columns are independent: a block takes 32 of them - lane = column - and its D / 16 warps 16 of the
-// D rows each, so a thread holds 16 values of the state in registers; the D / 32 blocks of a head are a cluster.  Sums over the rows run
-// in f32 over a warp's 16 and the warps' runs are added in f64 in a fixed order (the exact GPU scan's, kernels/forward.cu:991-1013):
-// one exchange through shared memory and one barrier a row of the pass is all that the recurrence waits for.  The outputs' sums are
-// left in shared memory and finished for up to 16 rows at once; the gated norm over a head's D outputs reads the neighbours' over the
-// cluster.  (One block of 256 threads a head, 64 values a thread and five barriers a row: 18 us a layer for 4 rows, some 1.5 us a row.)
+// Per value head a D x D state whose columns are independent: a block takes 32 of them - lane = column - and its D / RW warps RW of the
+// D rows each, so a thread holds RW values of the state in registers (16 in a pass: twice the threads for the front end and its loads;
+// 32 in a step of many rows: more blocks a multiprocessor, and k and q - which every thread must read - read half as often); the D / 32 blocks of a head are a cluster.  Sums over the rows run
+// in f32 over 16 of them and these runs are added in f64 in a fixed order (the exact GPU scan's, kernels/forward.cu:991-1013): one
+// exchange through shared memory and one barrier a row of the pass is what the recurrence waits for.  Everything else stays off its
+// path: the next row's operands are read before the barrier, the next 8 rows arrive by asynchronous copies, and the outputs of 8
+// rows - their runs left in shared memory - are finished 8 rows later, when the cluster's other blocks have theirs for the gated norm over
+// a head's D outputs.  (One block of 256 threads a head, 64 values a thread and five barriers a row was 18 us a layer for 4 rows; this
+// split with the outputs finished in line 0.65 us a row.  Shared-memory reads of k and q, 16 bytes a lane at 128 bytes a cycle, are what
+// the rows wait for now.)
 // Reads the state of the current buffer (state[1]) and writes the other one.  With `og` != null it applies all m rows and writes
 // the gated, normalised outputs (the pass itself).  With og == null it is the replay of a commit: layer blockIdx.y of every per-layer
 // array, only the res[0] kept rows, and nothing at all when every row was kept (the pass already wrote that state) or none was.
 // With pp.xin the block also does the front end for the channels it needs - q and k of its key head, v of its own columns: causal conv
-// + SiLU, L2 norms, beta and decay (what sz_delta_prep_kernel does for whole rows) - and leaves the conv outputs, beta and decay (and,
-// with xsave, the raw projections) where the replay of a commit reads them: passes of up to SZ_MAX_VERIFY rows.  Without, the front
+// + SiLU, L2 norms, beta and decay (what sz_delta_prep_kernel does for whole rows) - and leaves the conv outputs, beta and decay
+// where the replay of a commit reads them: passes of up to SZ_MAX_VERIFY rows.  Without, the front
 // end ran as a kernel of its own and any number of rows follow one another.
 struct SzDeltaPrep {
     const float* xin;     // [m][ch] raw projections of this layer (null: the front end already ran as a kernel of its own)
@@ -707,7 +711,6 @@ struct SzDeltaPrep {
     float* xc;            // [m][ch] out
     float* beta;          // [m][vh] out
     float* decay;         // [m][vh] out
-    float* xsave;         // [m][ch] out: a copy of xin, or null
     int k;
 };
 // One sequence's scan of one layer.
@@ -719,46 +722,52 @@ struct SzScanSeq {
     SzDeltaPrep pp;
     int m, pad;
 };
-#define SZ_SCAN_RC 16     // rows between two exchanges of the outputs
+#define SZ_SCAN_RC 8      // rows between two exchanges of the outputs
 
 template <int D>
 struct SzScanShared {
-    float k[SZ_SCAN_RC][D], q[SZ_SCAN_RC][D], v[SZ_SCAN_RC][32];
+    float k[2][SZ_SCAN_RC][D], q[2][SZ_SCAN_RC][D], v[2][SZ_SCAN_RC][32];   // two sets of rows: one at work, the next arriving
+    float beta[2][SZ_SCAN_RC], decay[2][SZ_SCAN_RC];
     float orun[SZ_SCAN_RC][D / 16][32];      // the outputs' runs
-    double mem[2][D / 16][32];                // a row's runs of S^T k
+    double mem[2][D / 64][4][32];             // a row's runs of S^T k, four a part (RW = 32: the first two added, the third, the fourth)
     float ofs[2][SZ_SCAN_RC][32];            // finished outputs of the block's columns
-    float beta[SZ_SCAN_RC], decay[SZ_SCAN_RC];
 };
-// the runs of one column added as two halves of four each (D = 64: one half)
-template <int D, typename F>
-__device__ __forceinline__ double sz_scan_sum(F run) {
-    double tot = 0.0;
-#pragma unroll
-    for (int p = 0; p < D / 64; p++) {
-        double s = 0.0;
-#pragma unroll
-        for (int r = 0; r < 4; r++) s += run(4 * p + r);
-        tot += s;
-    }
-    return tot;
-}
 
-template <int D>
+template <int D, int RW>
 __device__ __forceinline__ void sz_delta_scan_body(const SzScanSeq& q, const float* __restrict__ norm_w, int kh, int vh, float eps,
                                                    const SzTree* __restrict__ tr, float* __restrict__ fork, const int hd, const int cb, const int di) {
-    constexpr int RUNS = D / 16, NT = RUNS * 32;
+    constexpr int NW = D / RW, NT = NW * 32, RPW = SZ_SCAN_RC / NW;     // warps; rows of outputs a warp finishes
     __shared__ __align__(16) SzScanShared<D> sh;
-    const int run = threadIdx.x >> 5, lane = threadIdx.x & 31, col = cb * 32 + lane;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, col = cb * 32 + lane;
     const int kx = hd % kh;  // value heads are tiled over the key heads (forward.rs:862-864)
     const int kd = kh * D, ch = 2 * kd + vh * D;
-    const size_t Sl = (size_t)vh * D * D, Sat = (size_t)di * Sl + (size_t)hd * D * D + (size_t)(run * 16) * D + col;
+    const size_t Sl = (size_t)vh * D * D, Sat = (size_t)di * Sl + (size_t)hd * D * D + (size_t)(warp * RW) * D + col;
     float* og = q.og;
-    float S[16];
+    float S[RW];
     // the state belongs to the previous pass (and the buffer index with it): in the pass itself it is fetched ahead of the wait
     if (og) {
         const float* Sg = (q.state[1] ? q.S1 : q.S0) + Sat;
 #pragma unroll
-        for (int i = 0; i < 16; i++) S[i] = sz_ld32_here(Sg + (size_t)i * D);
+        for (int i = 0; i < RW; i++) S[i] = sz_ld32_here(Sg + (size_t)i * D);
+    }
+    // .. and so do the carried conv rows; with the usual 4 taps a thread takes its (one or two) channels for all rows of the pass, so that
+    // taps and carried values are there before the wait and the rows' projections are one round of loads after it
+    const bool quick = og != nullptr && q.pp.xin != nullptr && q.pp.k == 4 && !tr;
+    float taps[2][4], prev[2][3];
+    int chn[2];
+    if (quick) {
+        const float* conv = q.state[1] ? q.pp.conv1 : q.pp.conv0;
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const int c = threadIdx.x + e * NT;
+            chn[e] = c < D ? kx * D + c : (c < 2 * D ? kd + kx * D + c - D : 2 * kd + hd * D + cb * 32 + c - 2 * D);
+            if (c < 2 * D + 32) {
+#pragma unroll
+                for (int t = 0; t < 4; t++) taps[e][t] = sz_ld32_here(q.pp.cw + chn[e] * 4 + t);
+#pragma unroll
+                for (int t = 0; t < 3; t++) prev[e][t] = sz_ld32_here(conv + (size_t)t * ch + chn[e]);
+            }
+        }
     }
     sz_pdl_wait();
     sz_pdl_trigger();
@@ -775,123 +784,125 @@ __device__ __forceinline__ void sz_delta_scan_body(const SzScanSeq& q, const flo
     if (!og) {
         const float* Sg = (cur ? q.S1 : q.S0) + Sat;
 #pragma unroll
-        for (int i = 0; i < 16; i++) S[i] = Sg[(size_t)i * D];
+        for (int i = 0; i < RW; i++) S[i] = Sg[(size_t)i * D];
     }
     const float* xc = q.xc + (size_t)di * SZ_MAX_VERIFY * ch;          // (di > 0 in a replay only)
     const float* beta = q.beta + (size_t)di * SZ_MAX_VERIFY * vh;
     const float* decay = q.decay + (size_t)di * SZ_MAX_VERIFY * vh;
     const bool fused = og != nullptr && q.pp.xin != nullptr;
     float* fk = fork ? fork + ((size_t)di * vh + hd) * SZ_MAX_VERIFY * D * D : nullptr;
-    int prev_row = -1;
-    for (int c0 = 0; c0 < rows; c0 += SZ_SCAN_RC) {
-        const int nr = rows - c0 < SZ_SCAN_RC ? rows - c0 : SZ_SCAN_RC, par = (c0 / SZ_SCAN_RC) & 1;
-        if (fused) {
-            // ---- front end for this block's channels (forward.rs:829-861)
-            const SzDeltaPrep& pp = q.pp;
-            const float* conv = cur ? pp.conv1 : pp.conv0;
-            const int k = pp.k;
-            for (int idx = threadIdx.x; idx < nr * (2 * D + 32); idx += NT) {
-                const int j = idx / (2 * D + 32), c = idx - j * (2 * D + 32);
-                const int part3 = c < D ? 0 : (c < 2 * D ? 1 : 2), i = c - part3 * D;
-                const int chn = part3 == 0 ? kx * D + i : (part3 == 1 ? kd + kx * D + i : 2 * kd + hd * D + cb * 32 + i);
-                const float own = pp.xin[(size_t)j * ch + chn];
-                double acc = (double)pp.cw[chn * k + (k - 1)] * (double)own;
-                for (int t = 0; t < k - 1; t++) {
-                    const int tau = sz_tree_up(tr, j, (k - 1) - t);  // the row (k - 1) - t steps back: of this pass, or (negative) of the carried state
-                    const float prev = tau >= 0 ? pp.xin[(size_t)tau * ch + chn] : conv[(size_t)((k - 1) + tau) * ch + chn];
-                    acc += (double)pp.cw[chn * k + t] * (double)prev;
+    const bool pick = !og && tr;      // replay of a tree pass: the kept path's rows
+    // q, k, v, beta and decay of rows c0 .. into set `set`, asynchronously (one group of copies a call)
+    auto fetch = [&](int c0, int set) {
+        const int nr = rows - c0 < SZ_SCAN_RC ? rows - c0 : SZ_SCAN_RC;
+        for (int idx = threadIdx.x; idx < nr * (D / 2 + 8); idx += NT) {      // 16-byte pieces
+            const int jj = idx / (D / 2 + 8), c = idx - jj * (D / 2 + 8);
+            const float* x = xc + (size_t)(pick ? q.res[2 + c0 + jj] : c0 + jj) * ch;
+            if (c < D / 4) sz_cp_async16(sh.q[set][jj] + 4 * c, x + kx * D + 4 * c);
+            else if (c < D / 2) sz_cp_async16(sh.k[set][jj] + 4 * (c - D / 4), x + kd + kx * D + 4 * (c - D / 4));
+            else sz_cp_async16(sh.v[set][jj] + 4 * (c - D / 2), x + 2 * kd + hd * D + cb * 32 + 4 * (c - D / 2));
+        }
+        if (threadIdx.x < nr) {
+            const size_t j = (size_t)(pick ? q.res[2 + c0 + threadIdx.x] : c0 + (int)threadIdx.x);
+            sz_cp_async4(&sh.beta[set][threadIdx.x], beta + j * vh + hd);
+            sz_cp_async4(&sh.decay[set][threadIdx.x], decay + j * vh + hd);
+        }
+        sz_cp_async_commit();
+    };
+    if (fused) {
+        // ---- front end for this block's channels (forward.rs:829-861); at most SZ_SCAN_RC rows
+        const SzDeltaPrep& pp = q.pp;
+        const float* conv = cur ? pp.conv1 : pp.conv0;
+        const int k = pp.k;
+        if (quick) {
+            float x[2][SZ_SCAN_RC];
+#pragma unroll
+            for (int e = 0; e < 2; e++)
+                if (threadIdx.x + e * NT < 2 * D + 32) {
+#pragma unroll
+                    for (int j = 0; j < SZ_SCAN_RC; j++)
+                        if (j < rows) x[e][j] = __ldcg(pp.xin + (size_t)j * ch + chn[e]);
                 }
-                const float x = sz_silu((float)acc);
-                if (part3 == 0) sh.q[j][i] = x; else if (part3 == 1) sh.k[j][i] = x; else sh.v[j][i] = x;
-                // what a replay reads: v by every head, q and k once a key head (its first value head's blocks write 32 of them each)
-                const bool mine = part3 == 2 || (hd < kh && (i >> 5) == cb);
-                if (mine && pp.xsave) pp.xsave[(size_t)j * ch + chn] = own;
-                if (part3 == 2) pp.xc[(size_t)j * ch + chn] = x;
-            }
-            if (threadIdx.x < nr) {
-                const int j = threadIdx.x;
-                const float bt = sz_sigmoid(pp.b[j * vh + hd]);
-                const float sp_in = pp.a[j * vh + hd] + pp.dt[hd];
-                const float sp = sp_in > 20.0f ? sp_in : log1pf(expf(sp_in));
-                const float dc = expf(pp.a_log[hd] * sp);
-                sh.beta[j] = bt; sh.decay[j] = dc;
-                if (cb == 0) { pp.beta[j * vh + hd] = bt; pp.decay[j * vh + hd] = dc; }
-            }
-            __syncthreads();
-            // L2 norm of q and k (q also / sqrt(d)): a warp an item (row, q or k)
-            for (int it = run; it < nr * 2; it += RUNS) {
-                const int j = it >> 1, part3 = it & 1;
-                float* p = part3 ? sh.k[j] : sh.q[j];
-                double ss = 0.0;
 #pragma unroll
-                for (int i = 0; i < D / 32; i++) ss += (double)p[lane + 32 * i] * (double)p[lane + 32 * i];
-                ss = sz_warp_sum(ss);
-                const double nn = sz_rsqrt64(ss + 1e-6);
+            for (int e = 0; e < 2; e++) {
+                const int c = threadIdx.x + e * NT, i = c < D ? c : (c < 2 * D ? c - D : c - 2 * D);
+                if (c < 2 * D + 32) {
 #pragma unroll
-                for (int i = 0; i < D / 32; i++) {
-                    float t = (float)((double)p[lane + 32 * i] * nn);
-                    if (part3 == 0) t = t / sqrtf((float)D);
-                    p[lane + 32 * i] = t;
-                    if (hd < kh && i == cb) pp.xc[(size_t)j * ch + part3 * kd + kx * D + lane + 32 * i] = t;
+                    for (int j = 0; j < SZ_SCAN_RC; j++)
+                        if (j < rows) {
+                            double acc = (double)taps[e][3] * (double)x[e][j];
+#pragma unroll
+                            for (int t = 0; t < 3; t++) acc += (double)taps[e][t] * (double)(j - 3 + t >= 0 ? x[e][j - 3 + t >= 0 ? j - 3 + t : 0] : prev[e][j + t < 3 ? j + t : 0]);
+                            const float y = sz_silu((float)acc);
+                            if (c < D) sh.q[0][j][i] = y;
+                            else if (c < 2 * D) sh.k[0][j][i] = y;
+                            else { sh.v[0][j][i] = y; pp.xc[(size_t)j * ch + chn[e]] = y; }
+                        }
                 }
             }
-        } else {
-            for (int idx = threadIdx.x; idx < nr * (D / 2 + 8); idx += NT) {      // 16-byte pieces
-                const int jj = idx / (D / 2 + 8), c = idx - jj * (D / 2 + 8);
-                const int j = (!og && tr) ? q.res[2 + c0 + jj] : c0 + jj;           // replay of a tree pass: the kept path
-                const float* x = xc + (size_t)j * ch;
-                if (c < D / 4) ((float4*)sh.q[jj])[c] = __ldcg((const float4*)(x + kx * D) + c);
-                else if (c < D / 2) ((float4*)sh.k[jj])[c - D / 4] = __ldcg((const float4*)(x + kd + kx * D) + c - D / 4);
-                else ((float4*)sh.v[jj])[c - D / 2] = __ldcg((const float4*)(x + 2 * kd + hd * D + cb * 32) + c - D / 2);
+        } else for (int idx = threadIdx.x; idx < rows * (2 * D + 32); idx += NT) {
+            const int j = idx / (2 * D + 32), c = idx - j * (2 * D + 32);
+            const int part3 = c < D ? 0 : (c < 2 * D ? 1 : 2), i = c - part3 * D;
+            const int chn = part3 == 0 ? kx * D + i : (part3 == 1 ? kd + kx * D + i : 2 * kd + hd * D + cb * 32 + i);
+            double acc = (double)pp.cw[chn * k + (k - 1)] * (double)pp.xin[(size_t)j * ch + chn];
+            for (int t = 0; t < k - 1; t++) {
+                const int tau = sz_tree_up(tr, j, (k - 1) - t);  // the row (k - 1) - t steps back: of this pass, or (negative) of the carried state
+                const float prev = tau >= 0 ? pp.xin[(size_t)tau * ch + chn] : conv[(size_t)((k - 1) + tau) * ch + chn];
+                acc += (double)pp.cw[chn * k + t] * (double)prev;
             }
-            if (threadIdx.x < nr) {
-                const int j = (!og && tr) ? q.res[2 + c0 + threadIdx.x] : c0 + (int)threadIdx.x;
-                sh.beta[threadIdx.x] = __ldcg(beta + (size_t)j * vh + hd); sh.decay[threadIdx.x] = __ldcg(decay + (size_t)j * vh + hd);
-            }
+            const float x = sz_silu((float)acc);
+            // what a replay reads: v by every head, q and k once a key head (its first value head's blocks write 32 of them each)
+            if (part3 == 0) sh.q[0][j][i] = x;
+            else if (part3 == 1) sh.k[0][j][i] = x;
+            else { sh.v[0][j][i] = x; pp.xc[(size_t)j * ch + chn] = x; }
+        }
+        if (threadIdx.x < rows) {
+            const int j = threadIdx.x;
+            const float bt = sz_sigmoid(pp.b[j * vh + hd]);
+            const float sp_in = pp.a[j * vh + hd] + pp.dt[hd];
+            const float sp = sp_in > 20.0f ? sp_in : log1pf(expf(sp_in));
+            const float dc = expf(pp.a_log[hd] * sp);
+            sh.beta[0][j] = bt; sh.decay[0][j] = dc;
+            if (cb == 0) { pp.beta[j * vh + hd] = bt; pp.decay[j * vh + hd] = dc; }
         }
         __syncthreads();
-        for (int jj = 0; jj < nr; jj++) {
-            const int j = (!og && tr) ? q.res[2 + c0 + jj] : c0 + jj;
-            if (tr && og) {
-                const int pr = tr->parents[j];
-                if (pr != prev_row && pr >= 0) {          // another branch: back to the state after the parent
+        // L2 norm of q and k (q also / sqrt(d)): a warp an item (row, q or k)
+        for (int it = warp; it < rows * 2; it += NW) {
+            const int j = it >> 1, part3 = it & 1;
+            float* p = part3 ? sh.k[0][j] : sh.q[0][j];
+            double ss = 0.0;
 #pragma unroll
-                    for (int i = 0; i < 16; i++) S[i] = fk[((size_t)pr * D + run * 16 + i) * D + col];
-                }
-            }
-            prev_row = j;
-            const float dc = sh.decay[jj], bt = sh.beta[jj], vj = sh.v[jj][lane];
-            float kr[16], qr[16];
+            for (int i = 0; i < D / 32; i++) ss += (double)p[lane + 32 * i] * (double)p[lane + 32 * i];
+            ss = sz_warp_sum(ss);
+            const double nn = sz_rsqrt64(ss + 1e-6);
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                *(float4*)(kr + 4 * i) = *(const float4*)(sh.k[jj] + run * 16 + 4 * i);
-                *(float4*)(qr + 4 * i) = *(const float4*)(sh.q[jj] + run * 16 + 4 * i);
-            }
-            float r = 0.f;
-#pragma unroll
-            for (int i = 0; i < 16; i++) { S[i] = S[i] * dc; r = fmaf(S[i], kr[i], r); }
-            sh.mem[jj & 1][run][lane] = (double)r;
-            __syncthreads();
-            const double tot = sz_scan_sum<D>([&](int w) { return sh.mem[jj & 1][w][lane]; });
-            const float dl = (float)(((double)vj - tot) * (double)bt);
-            r = 0.f;
-#pragma unroll
-            for (int i = 0; i < 16; i++) {
-                S[i] = __fadd_rn(S[i], __fmul_rn(kr[i], dl));  // unfused, as the CPU reference
-                r = fmaf(S[i], qr[i], r);
-            }
-            if (og) sh.orun[jj][run][lane] = r;
-            if (og && tr && ((tr->save >> j) & 1u)) {
-#pragma unroll
-                for (int i = 0; i < 16; i++) fk[((size_t)j * D + run * 16 + i) * D + col] = S[i];
+            for (int i = 0; i < D / 32; i++) {
+                float t = (float)((double)p[lane + 32 * i] * nn);
+                if (part3 == 0) t = t / sqrtf((float)D);
+                p[lane + 32 * i] = t;
+                if (hd < kh && i == cb) pp.xc[(size_t)j * ch + part3 * kd + kx * D + lane + 32 * i] = t;
             }
         }
-        __syncthreads();
-        if (og) {
-            for (int jj = run; jj < nr; jj += RUNS) sh.ofs[par][jj][lane] = (float)sz_scan_sum<D>([&](int w) { return (double)sh.orun[jj][w][lane]; });
-            sz_cluster_sync();       // (the other half of ofs is written next: a block that is one exchange ahead cannot reach this half)
-            // gated RMS norm of a row's D outputs: every block of the head sums them all and finishes its own
-            for (int jj = run; jj < nr; jj += RUNS) {
+    } else {
+        fetch(0, 0);
+    }
+    // z of a warp's rows of outputs, requested when their 8 rows begin and used 8 rows later
+    float zn[RPW], zp[RPW];
+    const float nw = og ? __ldg(norm_w + col) : 0.f;
+    auto fetch_z = [&](int c0) {
+#pragma unroll
+        for (int e = 0; e < RPW; e++) {
+            const int row = c0 + warp + e * NW;
+            zn[e] = row < rows ? __ldcg(q.z + (size_t)row * vh * D + hd * D + col) : 0.f;
+        }
+    };
+    // gated RMS norm of the D outputs of the rows c0 .. left in half `par` of ofs: every block of the head sums them all and finishes
+    // its own
+    auto finish = [&](int c0, int par) {
+#pragma unroll
+        for (int e = 0; e < RPW; e++) {
+            const int jj = warp + e * NW;
+            if (c0 + jj < rows) {
                 double ss = 0.0;
 #pragma unroll
                 for (int b = 0; b < D / 32; b++) {
@@ -900,23 +911,124 @@ __device__ __forceinline__ void sz_delta_scan_body(const SzScanSeq& q, const flo
                 }
                 ss = sz_warp_sum(ss);
                 const double rr = sz_rsqrt64(ss / (double)D + (double)eps);
-                const size_t at = (size_t)(c0 + jj) * vh * D + hd * D + col;
-                const float normed = (float)((double)sh.ofs[par][jj][lane] * rr) * norm_w[col];
-                og[at] = normed * sz_sigmoid(q.z[at]);
+                const float normed = (float)((double)sh.ofs[par][jj][lane] * rr) * nw;
+                og[(size_t)(c0 + jj) * vh * D + hd * D + col] = normed * sz_sigmoid(zp[e]);
             }
+        }
+    };
+    int prev_row = -1;
+    for (int c0 = 0; c0 < rows; c0 += SZ_SCAN_RC) {
+        const int nr = rows - c0 < SZ_SCAN_RC ? rows - c0 : SZ_SCAN_RC, set = (c0 / SZ_SCAN_RC) & 1;
+        if (og) {
+#pragma unroll
+            for (int e = 0; e < RPW; e++) zp[e] = zn[e];
+            fetch_z(c0);
+        }
+        if (!fused) {
+            if (c0 + SZ_SCAN_RC < rows) { fetch(c0 + SZ_SCAN_RC, set ^ 1); sz_cp_async_wait<1>(); } else { sz_cp_async_wait<0>(); }
+        }
+        __syncthreads();
+        // a row's operands are read before the barrier of the row ahead of it
+        float kr[RW], dc, bt, vj;
+        auto operands = [&](int jj) {
+            dc = sh.decay[set][jj]; bt = sh.beta[set][jj]; vj = sh.v[set][jj][lane];
+#pragma unroll
+            for (int i = 0; i < RW / 4; i++) *(float4*)(kr + 4 * i) = *(const float4*)(sh.k[set][jj] + warp * RW + 4 * i);
+        };
+        operands(0);
+        for (int jj = 0; jj < nr; jj++) {
+            const int j = pick ? q.res[2 + c0 + jj] : c0 + jj;
+            if (tr && og) {
+                const int pr = tr->parents[j];
+                if (pr != prev_row && pr >= 0) {          // another branch: back to the state after the parent
+#pragma unroll
+                    for (int i = 0; i < RW; i++) S[i] = fk[((size_t)pr * D + warp * RW + i) * D + col];
+                }
+            }
+            prev_row = j;
+            float r0 = 0.f, r1 = 0.f;
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+                S[i] = S[i] * dc; r0 = fmaf(S[i], kr[i], r0);
+                if constexpr (RW == 32) { S[16 + i] = S[16 + i] * dc; r1 = fmaf(S[16 + i], kr[16 + i], r1); }
+            }
+            // four runs a part: of warps 4 p .. (RW = 16), or 2 p and 2 p + 1
+            if constexpr (RW == 16) {
+                sh.mem[jj & 1][warp >> 2][warp & 3][lane] = (double)r0;
+            } else {
+                double (*mp)[32] = sh.mem[jj & 1][warp >> 1];
+                if (warp & 1) { mp[1][lane] = (double)r0; mp[2][lane] = (double)r1; }
+                else mp[0][lane] = (0.0 + (double)r0) + (double)r1;
+            }
+            float qr[RW];
+            if (og) {
+#pragma unroll
+                for (int i = 0; i < RW / 4; i++) *(float4*)(qr + 4 * i) = *(const float4*)(sh.q[set][jj] + warp * RW + 4 * i);
+            }
+            const double vd = (double)vj, bd = (double)bt;
+            __syncthreads();
+            double tot = 0.0;
+#pragma unroll
+            for (int p = 0; p < D / 64; p++) {
+                const double s01 = RW == 32 ? sh.mem[jj & 1][p][0][lane] + sh.mem[jj & 1][p][1][lane]
+                                            : ((0.0 + sh.mem[jj & 1][p][0][lane]) + sh.mem[jj & 1][p][1][lane]) + sh.mem[jj & 1][p][2][lane];
+                tot += s01 + sh.mem[jj & 1][p][RW == 32 ? 2 : 3][lane];
+            }
+            const float dl = (float)((vd - tot) * bd);
+#pragma unroll
+            for (int i = 0; i < RW; i++) S[i] = __fadd_rn(S[i], __fmul_rn(kr[i], dl));  // unfused, as the CPU reference
+            if (jj + 1 < nr) operands(jj + 1);
+            if (og) {
+                r0 = 0.f; r1 = 0.f;
+#pragma unroll
+                for (int i = 0; i < 16; i++) {
+                    r0 = fmaf(S[i], qr[i], r0);
+                    if constexpr (RW == 32) r1 = fmaf(S[16 + i], qr[16 + i], r1);
+                }
+                sh.orun[jj][RW / 16 * warp][lane] = r0;
+                if constexpr (RW == 32) sh.orun[jj][2 * warp + 1][lane] = r1;
+                if (tr && ((tr->save >> j) & 1u)) {
+#pragma unroll
+                    for (int i = 0; i < RW; i++) fk[((size_t)j * D + warp * RW + i) * D + col] = S[i];
+                }
+            }
+        }
+        if (og) {
+            // the rows' outputs: those of the 8 rows before are finished, and these rows' runs added for the next time
+            if (c0 > 0) { sz_cluster_wait(); finish(c0 - SZ_SCAN_RC, set ^ 1); }
+            __syncthreads();
+            for (int jj = warp; jj < nr; jj += NW) {
+                double tot = 0.0;
+#pragma unroll
+                for (int p = 0; p < D / 64; p++) {
+                    double s = 0.0;
+#pragma unroll
+                    for (int r = 0; r < 4; r++) s += (double)sh.orun[jj][4 * p + r][lane];
+                    tot += s;
+                }
+                sh.ofs[set][jj][lane] = (float)tot;
+            }
+            sz_cluster_arrive();
         }
     }
     float* So = (cur ? q.O0 : q.O1) + Sat;
 #pragma unroll
-    for (int i = 0; i < 16; i++) So[(size_t)i * D] = S[i];
-    if (og) sz_cluster_sync();       // no block leaves while another reads its outputs
+    for (int i = 0; i < 32; i++) So[(size_t)i * D] = S[i];
+    if (og) {
+        const int c0 = (rows - 1) / SZ_SCAN_RC * SZ_SCAN_RC;
+#pragma unroll
+        for (int e = 0; e < RPW; e++) zp[e] = zn[e];
+        sz_cluster_wait();
+        finish(c0, (c0 / SZ_SCAN_RC) & 1);
+        sz_cluster_sync();       // no block leaves while another reads its outputs
+    }
 }
 
 // grid (vh * D / 32, layers), cluster D / 32
 template <int D>
 __global__ void __cluster_dims__(D / 32, 1, 1) __launch_bounds__(2 * D)
 sz_delta_scan_kernel(const SzScanSeq q, const float* __restrict__ norm_w, int kh, int vh, float eps, const SzTree* __restrict__ tr, float* __restrict__ fork) {
-    sz_delta_scan_body<D>(q, norm_w, kh, vh, eps, tr, fork, (int)blockIdx.x / (D / 32), (int)blockIdx.x % (D / 32), (int)blockIdx.y);
+    sz_delta_scan_body<D, 16>(q, norm_w, kh, vh, eps, tr, fork, (int)blockIdx.x / (D / 32), (int)blockIdx.x % (D / 32), (int)blockIdx.y);
 }
 
 // The pass of one layer for SEVERAL sequences in one launch (a batched step, prompts): block row b is sequence b's scan, its pointers
@@ -928,7 +1040,7 @@ sz_delta_scan_seqs_kernel(const SzScanSeq* __restrict__ tab, const float* __rest
     static_assert(sizeof(SzScanSeq) % 8 == 0 && sizeof(SzScanSeq) / 8 <= 2 * 64, "copied in 8-byte words");
     if (threadIdx.x < sizeof(SzScanSeq) / 8) ((u64*)&q)[threadIdx.x] = ((const u64*)(tab + blockIdx.y))[threadIdx.x];
     __syncthreads();
-    sz_delta_scan_body<D>(q, norm_w, kh, vh, eps, (const SzTree*)nullptr, (float*)nullptr, (int)blockIdx.x / (D / 32), (int)blockIdx.x % (D / 32), 0);
+    sz_delta_scan_body<D, 16>(q, norm_w, kh, vh, eps, (const SzTree*)nullptr, (float*)nullptr, (int)blockIdx.x / (D / 32), (int)blockIdx.x % (D / 32), 0);
 }
 
 // ---- attention front end (forward.rs:908-927): per head RMSNorm + NeoX RoPE of q and k, K and V into the cache.

@@ -339,7 +339,7 @@ sz_rows_delta_prep_kernel(const SzSeqDev* __restrict__ seqs, const SzRowDev* __r
 
 // The scans of a layer for the sequences of a step, after sz_rows_delta_prep_kernel.  grid (vh * D / 32, sequences)
 template <int D>
-__global__ void __cluster_dims__(D / 32, 1, 1) __launch_bounds__(2 * D)
+__global__ void __cluster_dims__(D / 32, 1, 1) __launch_bounds__(D)
 sz_rows_scan_kernel(const SzSeqDev* __restrict__ seqs, int di, const float* __restrict__ xc_all, const float* __restrict__ beta_all, const float* __restrict__ decay_all,
                     const float* __restrict__ z, const float* __restrict__ norm_w, int kh, int vh, float eps, float* __restrict__ og) {
     __shared__ SzScanSeq q;
@@ -358,7 +358,7 @@ sz_rows_scan_kernel(const SzSeqDev* __restrict__ seqs, int di, const float* __re
         q.m = s.m;
     }
     __syncthreads();
-    sz_delta_scan_body<D>(q, norm_w, kh, vh, eps, (const SzTree*)nullptr, (float*)nullptr, (int)blockIdx.x / (D / 32), (int)blockIdx.x % (D / 32), 0);
+    sz_delta_scan_body<D, 32>(q, norm_w, kh, vh, eps, (const SzTree*)nullptr, (float*)nullptr, (int)blockIdx.x / (D / 32), (int)blockIdx.x % (D / 32), 0);
 }
 
 // After a step: the sequences whose rows were all kept move on.  One block.
