@@ -698,12 +698,14 @@ extern "C" int sz_moe_scratch_init(uint64_t scratch, int64_t scratch_bytes, uint
     return SZ_OK;
 }
 
+static bool sz_blk_takes(const sz_moe_layer* L);
 extern "C" int sz_moe_launches(const sz_moe_layer* L) {
     if (!L) return 0;
     const SzFast f = sz_fast_path(L);
     const int ep = L->ep_count > 0 ? 1 : 0;  // the fixed-point finish (the all-reduce is NCCL's kernel, not counted)
     if (f.exl3) return 4 + (L->shared_ff > 0 && !f.shared_fused ? 2 : 0) + ep;
-    return (L->shared_ff > 0 ? 6 : 4) + ep;
+    const bool join = L->shared_ff > 0 && sz_blk_takes(L) && L->shared_type == L->expert_type;
+    return 4 + (L->shared_ff > 0 ? (join ? (L->shared_ff == L->expert_ff ? 0 : 1) : 2) : 0) + ep;
 }
 
 static int sz_sm_count() {
@@ -715,47 +717,67 @@ static int sz_sm_count() {
     return n;
 }
 
+// Bytes between the staged rows of a streaming block-format unit, and whether the kernel takes a matrix of this shape - decided for 8 rows
+// whatever the pass has: a row must not change kernels with the rows beside it.
+static int sz_blk_row_stride(int type, int n_in, bool* by_row) {
+    const size_t rb = type == SZ_TYPE_Q8_0 ? (size_t)(n_in / 32) * 34 : (size_t)(n_in / 256) * 110;
+    *by_row = rb % 16 == 0 && rb >= 1024;   // short rows go in one copy a unit: a copy a row would cost more to issue than the bank conflicts it avoids
+    int rbp = (int)rb;
+    if (*by_row) while (((rbp / 4) % 32) % 8 != 4) rbp += 16;   // consecutive rows 4 (mod 8) words apart in bank space
+    return rbp;
+}
+static size_t sz_blk_fixed(int n_in, bool down, int m, int* xsp_out) {
+    int xsp = n_in;
+    while (((xsp / 2) % 32) != 16) xsp += 8;
+    if (xsp_out) *xsp_out = xsp;
+    return 64 + 2048 + (size_t)(down ? 4 : 2) * 4096 + (size_t)2 * m * xsp * 2;
+}
+static bool sz_blk_fits(int type, int n_in, int n_out, bool down) {
+    if ((type != SZ_TYPE_Q8_0 && type != SZ_TYPE_IQ3_S) || n_in % 256 || n_out % (down ? 64 : 16)) return false;
+    bool by_row;
+    const size_t unit = (size_t)(down ? 64 : 32) * sz_blk_row_stride(type, n_in, &by_row);
+    return sz_blk_fixed(n_in, down, SZ_MAX_VERIFY, nullptr) + 2 * unit <= 222 * 1024;
+}
+
 // The streaming block-format kernels.  Returns SZ_E_TYPE (without setting an error text) when the shape is not one they take.
 template <int TYPE, bool DOWN>
 static int sz_launch_blk(cudaStream_t st, const SzPlan* plan, int groups, const u8* w0, u64 s0, const u8* w1, u64 s1, const float* in, int n_in,
-                         int n_out, float* out, u32* ctrl) {
+                         int n_out, float* out, int m, const SzBlkShared& shx, u32* ctrl) {
     constexpr int RT = DOWN ? 4 : 1;
-    if (n_in % 256 || n_out % (16 * RT) || groups < 1) return SZ_E_TYPE;
-    const size_t rb = TYPE == SZ_TYPE_Q8_0 ? (size_t)(n_in / 32) * 34 : (size_t)(n_in / 256) * 110;
+    if (groups < 1 || !sz_blk_fits(TYPE, n_in, n_out, DOWN)) return SZ_E_TYPE;
     SzBlkCfg c = {};
-    c.by_row = rb % 16 == 0 && rb >= 1024;   // short rows go in one copy a unit: a copy a row would cost more to issue than the bank conflicts it avoids
-    int rbp = (int)rb;
-    if (c.by_row) while (((rbp / 4) % 32) % 8 != 4) rbp += 16;   // consecutive rows 4 (mod 8) words apart in bank space
-    c.rbp = rbp;
-    c.unit_bytes = (DOWN ? 1 : 2) * 16 * RT * rbp;
-    int xsp = n_in;
-    while (((xsp / 2) % 32) != 16) xsp += 8;
-    c.xsp = xsp;
+    bool by_row;
+    c.rbp = sz_blk_row_stride(TYPE, n_in, &by_row);
+    c.by_row = by_row;
+    c.unit_bytes = (DOWN ? 1 : 2) * 16 * RT * c.rbp;
+    const size_t fixed = sz_blk_fixed(n_in, DOWN, m, &c.xsp);
     c.slices = n_out / (16 * RT);
-    const size_t fixed = 64 + 2048 + 4096 + (size_t)(DOWN ? 1 : 2) * RT * 4096 + (size_t)2 * SZ_MAX_VERIFY * xsp * 2;
-    const size_t budget = 222 * 1024;   // dynamic + the kernel's static shared memory stay under the 227 KB a block may have
-    if (fixed + 2 * (size_t)c.unit_bytes > budget) return SZ_E_TYPE;
+    c.xrows = m;
+    c.sh_slices = shx.w0 ? shx.n_out / (16 * RT) : 0;
+    // two blocks a multiprocessor where that leaves two stages (a block's barriers hide behind the other's work), else one with all of
+    // shared memory; dynamic + the kernel's static part stay under the 227 KB a block may have
+    const size_t half = 109 * 1024, budget = fixed + 2 * (size_t)c.unit_bytes <= half ? half : 222 * 1024;
     int NS = (int)((budget - fixed) / c.unit_bytes);
     c.NS = NS > 4 ? 4 : NS;
     const size_t smem = fixed + (size_t)c.NS * c.unit_bytes;
     static bool set = false;
     if (!set) { SZ_CUDA(cudaFuncSetAttribute(sz_blk_ffn_kernel<TYPE, DOWN, RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024)); set = true; }
-    const int per_sm = smem + 4096 <= 110 * 1024 ? 2 : 1;
+    const int per_sm = smem <= half ? 2 : 1;
     int blocks = sz_sm_count() * per_sm;
-    const long long units = (long long)groups * c.slices;
+    const long long units = (long long)groups * c.slices + c.sh_slices;
     if (blocks > units) blocks = (int)units;
     SZ_CUDA(sz_launch(DOWN ? "down_blk" : "gateup_blk", sz_blk_ffn_kernel<TYPE, DOWN, RT>, dim3(blocks), dim3(256), smem, st, true, plan, w0, s0, w1, s1,
-                      in, n_in, n_out, out, c, ctrl));
+                      in, n_in, n_out, out, c, shx, ctrl));
     return SZ_OK;
 }
 
 template <int TYPE>
 static int sz_launch_rows(cudaStream_t st, const SzPlan* plan, int groups, const u8* gate, u64 gs, const u8* up, u64 us, const u8* down,
-                          u64 ds, const float* x, int H, int FF, float* act, float* eo, bool down_pass, u32* ctrl) {
+                          u64 ds, const float* x, int H, int FF, float* act, float* eo, bool down_pass, int m, const SzBlkShared& shx, u32* ctrl) {
     static const bool generic_only = getenv("SZ_GENERIC_KERNELS") && atoi(getenv("SZ_GENERIC_KERNELS")) != 0;
     if (!generic_only) {  // the streaming tensor-pipe kernels, where the shapes fit them
-        int rc = down_pass ? sz_launch_blk<TYPE, true>(st, plan, groups, down, ds, nullptr, 0, act, FF, H, eo, ctrl)
-                           : sz_launch_blk<TYPE, false>(st, plan, groups, gate, gs, up, us, x, H, FF, act, ctrl);
+        int rc = down_pass ? sz_launch_blk<TYPE, true>(st, plan, groups, down, ds, nullptr, 0, act, FF, H, eo, m, shx, ctrl)
+                           : sz_launch_blk<TYPE, false>(st, plan, groups, gate, gs, up, us, x, H, FF, act, m, shx, ctrl);
         if (rc != SZ_E_TYPE) return rc;  // SZ_E_TYPE: not a shape for them
     }
     const size_t smem = 2048 + (size_t)SZ_MAX_VERIFY * (down_pass ? FF : H) * 4;
@@ -773,6 +795,13 @@ static int sz_launch_rows(cudaStream_t st, const SzPlan* plan, int groups, const
     return SZ_OK;
 }
 
+// Do the streaming block-format kernels take this layer's shapes (sz_launch_blk's conditions), so that the shared expert can join?
+static bool sz_blk_takes(const sz_moe_layer* L) {
+    static const bool generic_only = getenv("SZ_GENERIC_KERNELS") && atoi(getenv("SZ_GENERIC_KERNELS")) != 0;
+    return !generic_only && L->shared_ff > 0 && sz_blk_fits(L->expert_type, L->hidden, L->expert_ff, false) && sz_blk_fits(L->expert_type, L->hidden, L->shared_ff, false) &&
+           sz_blk_fits(L->expert_type, L->expert_ff, L->hidden, true);
+}
+
 template <int K>
 static int sz_launch_exl3(cudaStream_t st, const SzPlan* plan, int groups, const u8* w0, u64 s0, const u8* w1, u64 s1, const float* in0,
                           const float* in1, int by_pair, int n_in, int n_out, float* out0, float* out1) {
@@ -786,10 +815,10 @@ static int sz_launch_exl3(cudaStream_t st, const SzPlan* plan, int groups, const
 
 // One expert FFN pass (gate/up then down) for the groups of `plan`.
 static int sz_ffn(cudaStream_t st, int type, const SzPlan* plan, int groups, u64 gate, u64 gs, u64 up, u64 us, u64 down, u64 ds,
-                  const float* x, int H, int FF, float* g, float* u, float* eo, bool down_pass, u32* ctrl) {
+                  const float* x, int H, int FF, float* g, float* u, float* eo, bool down_pass, int m, const SzBlkShared& shx, u32* ctrl) {
     const u8 *pg = (const u8*)gate, *pu = (const u8*)up, *pd = (const u8*)down;
-    if (type == SZ_TYPE_Q8_0) return sz_launch_rows<SZ_TYPE_Q8_0>(st, plan, groups, pg, gs, pu, us, pd, ds, x, H, FF, g, eo, down_pass, ctrl);
-    if (type == SZ_TYPE_IQ3_S) return sz_launch_rows<SZ_TYPE_IQ3_S>(st, plan, groups, pg, gs, pu, us, pd, ds, x, H, FF, g, eo, down_pass, ctrl);
+    if (type == SZ_TYPE_Q8_0) return sz_launch_rows<SZ_TYPE_Q8_0>(st, plan, groups, pg, gs, pu, us, pd, ds, x, H, FF, g, eo, down_pass, m, shx, ctrl);
+    if (type == SZ_TYPE_IQ3_S) return sz_launch_rows<SZ_TYPE_IQ3_S>(st, plan, groups, pg, gs, pu, us, pd, ds, x, H, FF, g, eo, down_pass, m, shx, ctrl);
 #define SZ_EXL3_CASE(KK)                                                                                                        \
     case KK:                                                                                                                    \
         return down_pass ? sz_launch_exl3<KK>(st, plan, groups, pd, ds, nullptr, 0, g, u, 1, FF, H, eo, nullptr)               \
@@ -947,13 +976,14 @@ static int sz_moe_run(const sz_moe_layer* L0, uint64_t x, int m, float* y, long 
         SZ_CUDA(e);
     }
     const int groups = m * L->top_k;
+    const SzBlkShared none = {};
     if (fast.exl3) {
         // streaming EXL3 kernels for the routed experts (and the shared expert when it has the same type and width)
         long long *acc_gu = (long long*)(base + S.acc_gu), *acc_d = (long long*)(base + S.acc_d);
         const bool sh_fused = fast.shared_fused && shared;
         if (shared && !sh_fused) {
-            if ((rc = sz_ffn(st, L->shared_type, plan_sh, 1, L->sh_gate, 0, L->sh_up, 0, L->sh_down, 0, xp, H, SF, sg, su, so, false, ctrl))) return rc;
-            if ((rc = sz_ffn(st, L->shared_type, plan_sh, 1, L->sh_gate, 0, L->sh_up, 0, L->sh_down, 0, xp, H, SF, sg, su, so, true, ctrl))) return rc;
+            if ((rc = sz_ffn(st, L->shared_type, plan_sh, 1, L->sh_gate, 0, L->sh_up, 0, L->sh_down, 0, xp, H, SF, sg, su, so, false, m, none, ctrl))) return rc;
+            if ((rc = sz_ffn(st, L->shared_type, plan_sh, 1, L->sh_gate, 0, L->sh_up, 0, L->sh_down, 0, xp, H, SF, sg, su, so, true, m, none, ctrl))) return rc;
         }
         if ((rc = sz_x3_launch(st, L, m, plan, xp, acc_gu, acc_d, ctrl, sh_fused))) return rc;
         SZ_CUDA(sz_launch("combine_exl3", sz_x3_combine_kernel, dim3(m * (H / 128)), dim3((L->top_k + 1) * 32), 0, st, true, (const long long*)acc_d,
@@ -963,14 +993,19 @@ static int sz_moe_run(const sz_moe_layer* L0, uint64_t x, int m, float* y, long 
         if (combine_blocks) *combine_blocks = (unsigned long long)m * (H / 128);
         return SZ_OK;
     }
+    // the shared expert joins the routed ones' launches where its type, and for the down matrices its width, are theirs
+    const bool blk = sz_blk_takes(L);
+    const bool join_gu = shared && blk && L->shared_type == L->expert_type, join_d = join_gu && SF == FF;
+    const SzBlkShared sh_gu = join_gu ? SzBlkShared{(const u8*)L->sh_gate, (const u8*)L->sh_up, xp, sg, SF} : none;
+    const SzBlkShared sh_d = join_d ? SzBlkShared{(const u8*)L->sh_down, nullptr, sg, so, H} : none;
     if ((rc = sz_ffn(st, L->expert_type, plan, groups, L->gate, L->gate_stride, L->up, L->up_stride, L->down, L->down_stride, xp, H, FF, g, u,
-                     eo, false, ctrl)))
+                     eo, false, m, sh_gu, ctrl)))
         return rc;
-    if (shared && (rc = sz_ffn(st, L->shared_type, plan_sh, 1, L->sh_gate, 0, L->sh_up, 0, L->sh_down, 0, xp, H, SF, sg, su, so, false, ctrl))) return rc;
+    if (shared && !join_gu && (rc = sz_ffn(st, L->shared_type, plan_sh, 1, L->sh_gate, 0, L->sh_up, 0, L->sh_down, 0, xp, H, SF, sg, su, so, false, m, none, ctrl))) return rc;
     if ((rc = sz_ffn(st, L->expert_type, plan, groups, L->gate, L->gate_stride, L->up, L->up_stride, L->down, L->down_stride, xp, H, FF, g, u,
-                     eo, true, ctrl)))
+                     eo, true, m, sh_d, ctrl)))
         return rc;
-    if (shared && (rc = sz_ffn(st, L->shared_type, plan_sh, 1, L->sh_gate, 0, L->sh_up, 0, L->sh_down, 0, xp, H, SF, sg, su, so, true, ctrl))) return rc;
+    if (shared && !join_d && (rc = sz_ffn(st, L->shared_type, plan_sh, 1, L->sh_gate, 0, L->sh_up, 0, L->sh_down, 0, xp, H, SF, sg, su, so, true, m, none, ctrl))) return rc;
     SZ_CUDA(sz_launch("combine", sz_combine_kernel, dim3((H + 255) / 256, m), dim3(256), 0, st, true, (const float*)eo, (const int32_t*)ridx,
                       (const double*)rw, (const float*)so, (const float*)logits, (int)L->n_expert, (int)L->top_k, H, shared ? 1 : 0, y, y_fix, e_lo, e_hi, push));
     if (combine_blocks) *combine_blocks = (unsigned long long)((H + 255) / 256) * m;

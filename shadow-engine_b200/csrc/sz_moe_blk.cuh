@@ -20,11 +20,21 @@ struct SzBlkCfg {
     int unit_bytes;  // a stage: 16 rows (x 2 matrices for gate / up)
     int xsp;         // halves between the staged rows of the group
     int slices;      // units an expert's matrix has (16 * RT rows each)
+    int xrows;       // rows of the pass: what a group has at most
+    int sh_slices;   // units of the shared expert's matrix (0: it is not part of the launch)
+};
+// The shared expert as one more group, of all rows of the pass, after the routed ones (its launches of its own filled 32 of 148
+// multiprocessors and waited for the routed ones': 20 of 106 us of an IQ3_S layer): same type and columns, its own matrices and rows.
+struct SzBlkShared {
+    const u8 *w0, *w1;
+    const float* in;
+    float* out;
+    int n_out;
 };
 
 // the A fragments (two k-halves: columns 8q..8q+3 | 8q+4..8q+7 of the block) of rows r0, r1 for 32-column block `blk`, and the rows' scales
 template <int TYPE>
-__device__ __forceinline__ void sz_blk_frag(const u8* r0, const u8* r1, int blk, int q, const u32* grid, const uint4* slut, u32* a1, u32* a2,
+__device__ __forceinline__ void sz_blk_frag(const u8* r0, const u8* r1, int blk, int q, const u32* grid, u32* a1, u32* a2,
                                             float& d0, float& d1) {
     if (TYPE == SZ_TYPE_Q8_0) {
         const u8* p0 = r0 + (size_t)blk * 34;
@@ -47,13 +57,15 @@ __device__ __forceinline__ void sz_blk_frag(const u8* r0, const u8* r1, int blk,
             const u32 sc = (p[106 + (b32 >> 1)] >> (4 * (b32 & 1))) & 15u;
             const u32 m0 = grid[(qs2 & 0xffu) | ((qh & 1u) << 8)];
             const u32 m1 = grid[(qs2 >> 8) | ((qh & 2u) << 7)];
-            const uint4 sm = slut[sg];  // sign masks of the four f16 pairs
+            // the sign byte twice, 15 bits apart: bit 2k of it and bit 2k + 1 are then 16 apart, so one shift puts a pair's two signs on its
+            // halves' sign bits (a table of the masks, 16 bytes an entry, kept the shared-memory pipe busy for ten cycles a lookup)
+            const u32 sy = sg | (sg << 15);
             u32 t0 = __byte_perm(m0, 0x64646464u, 0x4140), t1 = __byte_perm(m0, 0x64646464u, 0x4342);
             u32 t2 = __byte_perm(m1, 0x64646464u, 0x4140), t3 = __byte_perm(m1, 0x64646464u, 0x4342);
             __half2 h0 = __hsub2(*(const __half2*)&t0, k1024), h1 = __hsub2(*(const __half2*)&t1, k1024);
             __half2 h2 = __hsub2(*(const __half2*)&t2, k1024), h3 = __hsub2(*(const __half2*)&t3, k1024);
-            a1[r] = *(const u32*)&h0 ^ sm.x; a1[2 + r] = *(const u32*)&h1 ^ sm.y;
-            a2[r] = *(const u32*)&h2 ^ sm.z; a2[2 + r] = *(const u32*)&h3 ^ sm.w;
+            a1[r] = *(const u32*)&h0 ^ ((sy << 15) & 0x80008000u); a1[2 + r] = *(const u32*)&h1 ^ ((sy << 13) & 0x80008000u);
+            a2[r] = *(const u32*)&h2 ^ ((sy << 11) & 0x80008000u); a2[2 + r] = *(const u32*)&h3 ^ ((sy << 9) & 0x80008000u);
             (r ? d1 : d0) = d * (float)(1u + 2u * sc);
         }
     }
@@ -62,22 +74,21 @@ __device__ __forceinline__ void sz_blk_frag(const u8* r0, const u8* r1, int blk,
 // grid: any; block 256.  DOWN = false: out[pair][r] = silu(gate_r . x_row) * (up_r . x_row) with x = in[rows of the group]; true:
 // out[pair][r] = down_r . in[pair].  n_in: columns (a multiple of 256); n_out: rows of the matrices (a multiple of 16).
 // RT: 16-row tiles of a unit (the down matrices have short rows - FF columns - so a unit takes several tiles to be worth its barriers).
-// dynamic shared memory: 64 (barriers) | 2048 (IQ3_S grid) | 4096 (sign masks) | NM * RT * 4096 (reduction) | 2 * 8 * xsp * 2 (B operand) | NS * unit_bytes
+// dynamic shared memory: 64 (barriers) | 2048 (IQ3_S grid) | NM * RT * 4096 (reduction) | 2 * xrows * xsp * 2 (B operand) | NS * unit_bytes
 template <int TYPE, bool DOWN, int RT>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 sz_blk_ffn_kernel(const SzPlan* __restrict__ plan, const u8* __restrict__ w0, u64 stride0, const u8* __restrict__ w1, u64 stride1,
-                  const float* __restrict__ in, int n_in, int n_out, float* __restrict__ out, const SzBlkCfg c, u32* __restrict__ ctrl) {
+                  const float* __restrict__ in, int n_in, int n_out, float* __restrict__ out, const SzBlkCfg c, const SzBlkShared shx, u32* __restrict__ ctrl) {
     extern __shared__ __align__(128) u8 smem[];
     constexpr int NM = DOWN ? 1 : 2;   // matrices staged per unit
     constexpr int UR = 16 * RT;        // rows of a unit (per matrix)
     static_assert(NM * RT <= 4, "the reduction buffer holds four 16-row tiles");
     u64* bars = (u64*)smem;
     u32* grid = (u32*)(smem + 64);
-    uint4* slut = (uint4*)(smem + 64 + 2048);
-    float* red = (float*)(smem + 64 + 2048 + 4096);           // [NM * RT][8 warps][16 rows][8 group rows]
-    __half* xhi = (__half*)(smem + 64 + 2048 + 4096 + NM * RT * 4096); // [8][xsp]
-    __half* xlo = xhi + (size_t)SZ_MAX_VERIFY * c.xsp;
-    u8* stages = (u8*)(xlo + (size_t)SZ_MAX_VERIFY * c.xsp);
+    float* red = (float*)(smem + 64 + 2048);                  // [NM * RT][8 warps][16 rows][8 group rows]
+    __half* xhi = (__half*)(smem + 64 + 2048 + NM * RT * 4096); // [xrows][xsp]
+    __half* xlo = xhi + (size_t)c.xrows * c.xsp;
+    u8* stages = (u8*)(xlo + (size_t)c.xrows * c.xsp);
     __shared__ __align__(16) SzPlan splan;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, q = lane & 3;
@@ -88,30 +99,25 @@ sz_blk_ffn_kernel(const SzPlan* __restrict__ plan, const u8* __restrict__ w0, u6
     }
     if (TYPE == SZ_TYPE_IQ3_S) {
         for (int i = threadIdx.x; i < 512; i += 256) grid[i] = c_iq3s_grid[i];
-        {   // sign byte -> the sign bits of the four f16 pairs (bit 2k of the byte: low half of pair k, bit 2k + 1: high half)
-            const u32 s = threadIdx.x;
-            slut[s] = make_uint4(((s & 1u) << 15) | ((s & 2u) << 30), ((s & 4u) << 13) | ((s & 8u) << 28), ((s & 16u) << 11) | ((s & 32u) << 26),
-                                 ((s & 64u) << 9) | ((s & 128u) << 24));
-        }
     }
     sz_pdl_wait();
     sz_pdl_trigger();
     plan = sz_plan_stage(plan, &splan);
     __syncthreads();
     const int NG = plan->n_groups;
-    const long long U = (long long)NG * c.slices;
+    const long long U = (long long)NG * c.slices + c.sh_slices;
     const int u0 = (int)(U * blockIdx.x / gridDim.x), u1 = (int)(U * (blockIdx.x + 1) / gridDim.x);
     const int count = u1 - u0;
     if (count <= 0) return;
     auto issue = [&](int i) {  // thread 0
-        const int u = u0 + i, gi = u / c.slices, sl = u - gi * c.slices;
-        const u64 e = (u64)plan->expert[gi];
+        const int u = u0 + i, gq = u / c.slices, gi = gq < NG ? gq : NG, sl = u - gi * c.slices;    // (group NG: the shared expert)
+        const u64 e = gi < NG ? (u64)plan->expert[gi] : 0;
         u64* bar = &bars[i % c.NS];
         u8* dst = stages + (size_t)(i % c.NS) * c.unit_bytes;
         sz_mbar_expect_tx(bar, (u32)(NM * UR * rb));
 #pragma unroll
         for (int mtx = 0; mtx < NM; mtx++) {
-            const u8* src = (mtx ? w1 + e * stride1 : w0 + e * stride0) + (size_t)sl * UR * rb;
+            const u8* src = (gi < NG ? (mtx ? w1 + e * stride1 : w0 + e * stride0) : (mtx ? shx.w1 : shx.w0)) + (size_t)sl * UR * rb;
             u8* d = dst + (size_t)mtx * UR * c.rbp;
             if (c.by_row) {
                 for (int r = 0; r < UR; r++) sz_bulk_g2s(d + (size_t)r * c.rbp, src + (size_t)r * rb, (u32)rb, bar);
@@ -127,15 +133,17 @@ sz_blk_ffn_kernel(const SzPlan* __restrict__ plan, const u8* __restrict__ w0, u6
     int failed = 0;
     for (int i = 0; i < count; i++) {
         if (threadIdx.x == 0 && i + c.NS - 1 < count) issue(i + c.NS - 1);
-        const int u = u0 + i, gi = u / c.slices, sl = u - gi * c.slices;
+        const int u = u0 + i, gq = u / c.slices, gi = gq < NG ? gq : NG, sl = u - gi * c.slices;
+        const bool sh = gi == NG;
         if (gi != cur_g) {  // a new group: its rows become the B operand (f16 high and low parts)
             __syncthreads();
             cur_g = gi;
-            n = plan->count[gi];
-            const u8* src_rows = DOWN ? plan->pairs[gi] : plan->rows[gi];
+            n = sh ? c.xrows : plan->count[gi];
+            const u8* src_rows = DOWN ? plan->pairs[sh ? 0 : gi] : plan->rows[sh ? 0 : gi];
+            const float* src = sh ? shx.in : in;
             for (int idx = threadIdx.x; idx < n * (n_in / 4); idx += 256) {
                 const int t = idx / (n_in / 4), c4 = idx - t * (n_in / 4);
-                const float4 v = __ldcg((const float4*)(in + (size_t)src_rows[t] * n_in) + c4);
+                const float4 v = __ldcg((const float4*)(src + (size_t)(sh ? t : src_rows[t]) * n_in) + c4);
                 const __half2 h0 = __floats2half2_rn(v.x, v.y), h1 = __floats2half2_rn(v.z, v.w);
                 const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
                 const __half2 l0 = __floats2half2_rn(v.x - f0.x, v.y - f0.y), l1 = __floats2half2_rn(v.z - f1.x, v.w - f1.y);
@@ -164,7 +172,7 @@ sz_blk_ffn_kernel(const SzPlan* __restrict__ plan, const u8* __restrict__ w0, u6
                     const u8* r1 = st + (size_t)(mtx * 16 + g + 8) * c.rbp;
                     u32 a1[4], a2[4];
                     float d0, d1;
-                    sz_blk_frag<TYPE>(r0, r1, blk, q, grid, slut, a1, a2, d0, d1);
+                    sz_blk_frag<TYPE>(r0, r1, blk, q, grid, a1, a2, d0, d1);
                     float t[4] = {0.f, 0.f, 0.f, 0.f};
                     sz_mma16816_z(t, a1, bh.x, bh.y);
                     sz_mma16816_z(t, a2, bh.z, bh.w);
@@ -195,8 +203,8 @@ sz_blk_ffn_kernel(const SzPlan* __restrict__ plan, const u8* __restrict__ w0, u6
                     v += red[tile * 1024 + (w * 16 + r16) * 8 + t];
                     if (!DOWN) v2 += red[(RT + tile) * 1024 + (w * 16 + r16) * 8 + t];
                 }
-                const int pair = plan->pairs[gi][t];
-                out[(size_t)pair * n_out + sl * UR + rr] = DOWN ? v : sz_silu(v) * v2;
+                float* o = sh ? shx.out + (size_t)t * shx.n_out : out + (size_t)plan->pairs[gi][t] * n_out;
+                o[sl * UR + rr] = DOWN ? v : sz_silu(v) * v2;
             }
         }
         __syncthreads();
