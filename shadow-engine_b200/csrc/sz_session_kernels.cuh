@@ -1541,6 +1541,22 @@ sz_attn_merge_kernel(const float* __restrict__ part, const float* __restrict__ q
     if (rws) splits = rws[j].splits;
     const float* p = (rws ? rws[j].part + (size_t)h * splits * (hd + 2) : part + ((size_t)j * nh + h) * splits * (hd + 2));
     const float g = t < hd ? __ldcg(qg + (((size_t)j * nh + h) * 2 + 1) * hd + t) : 0.f;
+    // group gq of threads takes splits gq, gq + 4, ...; a thread four consecutive dimensions.  The first 20 of a group (80 splits: all of
+    // them at the benchmark's context) are requested before anything waits for the maxima: read round by round behind the coefficients
+    // they were five trips to memory one after the other, 7.5 us a launch.
+    const int per = hd / 4;              // threads a partial row needs (64 at hd = 256)
+    const int ngrp = 256 / per > 4 ? 4 : 256 / per;
+    const int gq = t / per, i4 = (t % per) * 4;
+    constexpr int PRE = 20;
+    float2 pre[PRE][2];
+    if (gq < ngrp) {
+#pragma unroll
+        for (int i = 0; i < PRE; i++)
+            if (gq + ngrp * i < splits) {
+                const float2* row = (const float2*)(p + (size_t)(gq + ngrp * i) * (hd + 2) + i4);  // rows are 8-byte aligned (hd + 2 is even)
+                pre[i][0] = __ldcg(row); pre[i][1] = __ldcg(row + 1);
+            }
+    }
     float mm[2], zz[2];
     float M = -INFINITY;
 #pragma unroll
@@ -1570,16 +1586,17 @@ sz_attn_merge_kernel(const float* __restrict__ part, const float* __restrict__ q
     __syncthreads();
     z = 0.f;
     for (int q = 0; q < 8; q++) z += red[q];
-    // group gq of threads takes splits gq, gq + 4, ...; a thread four consecutive dimensions
-    const int per = hd / 4;              // threads a partial row needs (64 at hd = 256)
-    const int ngrp = 256 / per > 4 ? 4 : 256 / per;
-    const int gq = t / per, i4 = (t % per) * 4;
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
     if (gq < ngrp) {
-#pragma unroll 4
-        for (int s = gq; s < splits; s += ngrp) {
+#pragma unroll
+        for (int i = 0; i < PRE; i++)
+            if (gq + ngrp * i < splits) {
+                const float c = coef[gq + ngrp * i];
+                a.x = fmaf(pre[i][0].x, c, a.x); a.y = fmaf(pre[i][0].y, c, a.y); a.z = fmaf(pre[i][1].x, c, a.z); a.w = fmaf(pre[i][1].y, c, a.w);
+            }
+        for (int s = gq + ngrp * PRE; s < splits; s += ngrp) {
             const float c = coef[s];
-            const float2* row = (const float2*)(p + (size_t)s * (hd + 2) + i4);  // rows are 8-byte aligned (hd + 2 is even)
+            const float2* row = (const float2*)(p + (size_t)s * (hd + 2) + i4);
             const float2 v0 = __ldcg(row), v1 = __ldcg(row + 1);
             a.x = fmaf(v0.x, c, a.x); a.y = fmaf(v0.y, c, a.y); a.z = fmaf(v1.x, c, a.z); a.w = fmaf(v1.y, c, a.w);
         }
