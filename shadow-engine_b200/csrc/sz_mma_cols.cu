@@ -8,20 +8,30 @@
 // f16, products accumulate in f32; the order of the sum is the tensor core's.  The reference calls this mode inexact and uses it
 // for prompts only; so does this build (the verify step's projections stay on the bit-stable kernels).
 //
-// Shape of the kernel.  A block owns 128 weight rows (the M side of the instruction) and one tile of up to 256 tokens (the N side);
-// the accumulator D[128 rows][NT tokens] lives in tensor memory (NT columns of 128 lanes), so no register holds a partial sum until
-// the end.  K advances in steps of 64:
-//   warp 0      the copy warp.  Raw Q8_0 bytes of the block's 128 rows arrive 256 columns at a time (272 bytes a row: a multiple of
-//               16, which the 68 bytes of one 64-column step are not) as ONE tiled TMA copy (cp.async.bulk.tensor.2d over the
-//               matrix seen as [rows][row bytes / 2] 16-bit words, box 136 x 128; 128 separate 272-byte bulk copies a piece kept
-//               the copy engine, not the tensor core, as the bound), double-buffered; the token tile of a step, already in f16 and
-//               in the instruction's own shared-memory order (written once by sz_x16_pack_kernel), is one bulk copy.
-//   warps 1..8  decode: two threads a weight row turn a step's 2 blocks a row into f16 and store them in the canonical K-major
-//               no-swizzle order (8 rows x 16 bytes core matrices), then fence.proxy.async and arrive.
-//   warp 9      one thread issues the step's 4 tcgen05.mma (K = 16 each) from shared-memory descriptors and commits them to the
+// Shape of the kernel.  A block owns MT x 128 weight rows (the M side of the instruction), one tile of up to 256 tokens (the N side) and,
+// with a cluster of `ks` blocks, a part of K; the accumulators D[128 rows][NT tokens] live in tensor memory (MT x 256 columns of 128
+// lanes), so no register holds a partial sum until the end.  K advances in steps of 32 columns, one Q8_0 block a row, through a ring of
+// four stages:
+//   warp 18     raw Q8_0 bytes of the block's rows, 256 columns at a time (272 bytes a row: a multiple of 16, which the 34 bytes of a
+//               step are not) as MT tiled TMA copies (cp.async.bulk.tensor.2d over the matrix seen as [rows][row bytes / 2] 16-bit
+//               words, box 136 x 128; 128 separate 272-byte bulk copies a piece kept the copy engine, not the tensor core, as the bound).
+//   warp 0      the token tile of a step, already in f16 and in the instruction's own shared-memory order (written once by
+//               sz_x16_pack_kernel), one bulk copy.
+//   warps 1..16 decode, in groups of MT x 128 threads: a thread takes its group's blocks of a weight row's 272 bytes into registers -
+//               which frees the buffer for the next piece at once - and turns them block after block into f16 in the canonical K-major
+//               no-swizzle order (8 rows x 16 bytes core matrices), then fence.proxy.async and arrive.  The groups take the steps in turn.
+//   warp 17     one thread issues the step's 2 MT tcgen05.mma (K = 16 each) from shared-memory descriptors and commits them to the
 //               stage's "empty" barrier, which frees the stage for the decoders and the copy warp.
-// After the last step warps 1..8 read the accumulator with tcgen05.ld (lane = weight row, column = token) and write Y: for one
-// token, the 32 lanes of a warp write 32 consecutive rows.
+// After the last step the decode warps read the accumulators with tcgen05.ld (lane = weight row, column = token) and write Y: for one
+// token, the 32 lanes of a warp write 32 consecutive rows.  With ks > 1 a block of the cluster finishes its share of the columns: the
+// others store their parts of those into its shared memory (the stages' and the raw bytes', no longer needed), and it adds the parts in
+// the order of K.
+// What bounds it.  At many tokens L2 (10.8 TB/s): a step of 32 columns moves the token tile and the rows' bytes, so two row tiles share
+// a token tile (25 KB per 256 x 256 x 32) where one a block moved 41, and the tensor core, which needs 512 cycles of the step's 625; the
+// sums of a unit, which all blocks write at about the same time, are a fifth.  At few tokens latency: the chain decode, fence, barrier,
+// instruction.  The issuing thread took 390 cycles a step to make descriptors for 256 cycles of instructions; it makes them once.
+// 12,288 x 2,048: 4,093 tokens 281 -> 245 us (sustained, 1.4 GHz under the power cap), 256 tokens 28.8 -> 23.6;
+// 512 x 2,048, one token: 20 -> 12.4 (K in four parts).
 // Every wait is bounded; a wait that runs out records where in the error word, and the block still frees its tensor memory.
 #include <cuda.h>   // CUtensorMap and its enums; the encoder's entry point is asked of the runtime, nothing links against the driver
 #include "sz_common.cuh"
@@ -30,25 +40,37 @@
 namespace {
 
 constexpr int MC_BM = 128;        // weight rows a block
-constexpr int MC_KT = 64;         // columns a step
+constexpr int MC_KT = 32;         // columns a step
+constexpr int MC_PS = 64;         // columns of a unit of the packed tokens' order
 constexpr int MC_SS = 256;        // columns a raw copy
 constexpr int MC_RAW_ROW = 272;   // bytes of a row's 8 Q8_0 blocks
-constexpr int MC_STAGES = 3;
+constexpr int MC_STAGES = 4;
+constexpr int MC_STEPS = MC_SS / MC_KT;   // steps a raw piece: one a Q8_0 block of a row
+constexpr int MC_KS_MAX = 4;      // blocks along K at most
 constexpr int MC_NT_MAX = 256;    // tokens a tile
-constexpr int MC_THREADS = 320;   // copy warp + 8 decode warps + issue warp
+constexpr int MC_TILES_MORE = 3;  // token tiles more than the fewest, so that the units fill the chip's last turn
+constexpr int MC_DEC = 512;       // decode threads
+constexpr int MC_THREADS = MC_DEC + 96;   // copy warp, decode warps, issue warp, raw copy warp
 constexpr int MC_A_BYTES = MC_BM * MC_KT * 2;
 constexpr int MC_RAW_BYTES = MC_BM * MC_RAW_ROW;
+constexpr size_t MC_SMEM_MIN = 116 * 1024;   // one block a multiprocessor: blocks of clusters that wait for tensor memory another holds could wait for each other
 constexpr u32 MC_WAIT = 4000000u; // polls before a wait gives up
 
 struct McSmem {
-    u64 full[MC_STAGES], empty[MC_STAGES], raw_full[2], raw_empty[2], acc_full;
+    u64 full[MC_STAGES], empty[MC_STAGES], raw_full, raw_empty, acc_full, acc_empty;
     u32 tmem_base, failed;
 };
 
-__device__ __forceinline__ void mc_arrive(u64* bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sz_smem_addr(bar)) : "memory"); }
+// one arrival a warp: the arrivals of 32 lanes on one barrier are taken one after the other
+__device__ __forceinline__ void mc_arrive_warp(u64* bar) {
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sz_smem_addr(bar)) : "memory");
+}
 __device__ __forceinline__ void mc_fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void mc_tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void mc_tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+
+__device__ __forceinline__ void mc_cluster_sync() { asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory"); }
 
 // Shared-memory matrix descriptor, K-major, no swizzle: 8 rows x 16 bytes core matrices; `lbo` = bytes between the two core
 // matrices an instruction reads along K, `sbo` = bytes between 8-row groups.  Bits: address >> 4 at 0, lbo >> 4 at 16, sbo >> 4 at
@@ -70,19 +92,13 @@ __device__ __forceinline__ void mc_commit(u64* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(sz_smem_addr(bar)) : "memory");
 }
 
-// Block KB (0..7) of a row's 272 raw bytes -> 32 f16 weights, stored as the 4 chunks of 8 the block covers (chunk stride 16 * 128
-// bytes).  The block starts 34 * KB bytes into the row: not a multiple of 16, so three aligned 16-byte loads cover it and the
-// bytes are brought into place by funnel shifts whose amounts are known at compile time.  A weight is d * q rounded once to f16;
-// d is f16 and q an integer below 128, so the f16 product (one rounding of the exact product) is that same value.  q as f16: the
-// byte with its sign bit flipped is q + 128, placed under exponent 0x64 it reads 1024 + q + 128, and 1152 is subtracted.
-template <int KB>
-__device__ __forceinline__ void mc_decode_block(const u8* __restrict__ rowp, u8* __restrict__ dst) {
-    constexpr int OFF = KB * 34, BASE = OFF & ~15, SH = OFF & 15;
-    const uint4 v0 = *(const uint4*)(rowp + BASE), v1 = *(const uint4*)(rowp + BASE + 16), v2 = *(const uint4*)(rowp + BASE + 32);
-    const u32 W[12] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w, v2.x, v2.y, v2.z, v2.w};
-    constexpr int DW = SH / 4, DS = (SH % 4) * 8;
-    const u32 dbits = (W[DW] >> DS) & 0xffffu;
-    const u32 d2 = dbits | (dbits << 16);
+// A Q8_0 block that starts OFF bytes (even) into W -> 32 f16 weights, stored as the 4 chunks of 8 the block covers (chunk stride 16 * 128
+// bytes).  A pair of bytes is always one half of a word.  A weight is d * q rounded once to f16; d is f16 and q an integer below 128, so
+// the f16 product (one rounding of the exact product) is that same value.  q as f16: the byte with its sign bit flipped is q + 128, placed
+// under exponent 0x64 it reads 1024 + q + 128, and 1152 is subtracted.
+template <int OFF>
+__device__ __forceinline__ void mc_decode_block(const u32* W, u8* __restrict__ dst) {
+    const u32 d2 = __byte_perm(W[OFF / 4], 0, OFF % 4 ? 0x3232 : 0x1010);
     const __half2 dh = *(const __half2*)&d2;
     const u32 bias = 0x64806480u;   // 1152, twice
     const __half2 bh = *(const __half2*)&bias;
@@ -90,22 +106,38 @@ __device__ __forceinline__ void mc_decode_block(const u8* __restrict__ rowp, u8*
     for (int c = 0; c < 4; c++) {
         u32 o[4];
 #pragma unroll
-        for (int i = 0; i < 2; i++) {
-            const int b = SH + 2 + 4 * (2 * c + i);                       // first byte of this word of four q
-            const u32 q4 = (b % 4 ? __funnelshift_r(W[b / 4], W[b / 4 + 1], (b % 4) * 8) : W[b / 4]) ^ 0x80808080u;
-            const u32 lo = __byte_perm(q4, 0x64646464u, 0x4140), hi = __byte_perm(q4, 0x64646464u, 0x4342);   // {q0, q1}, {q2, q3} as 1024 + q + 128
-            const __half2 w0 = __hmul2(dh, __hsub2(*(const __half2*)&lo, bh)), w1 = __hmul2(dh, __hsub2(*(const __half2*)&hi, bh));
-            o[2 * i] = *(const u32*)&w0; o[2 * i + 1] = *(const u32*)&w1;
+        for (int i = 0; i < 4; i++) {
+            const int b = OFF + 2 + 2 * (4 * c + i);                      // first byte of the pair
+            const u32 v = __byte_perm(W[b / 4] ^ 0x80808080u, 0x64646464u, b % 4 ? 0x4342 : 0x4140);
+            const __half2 w = __hmul2(dh, __hsub2(*(const __half2*)&v, bh));
+            o[i] = *(const u32*)&w;
         }
         *(uint4*)(dst + c * 16 * 128) = make_uint4(o[0], o[1], o[2], o[3]);
     }
 }
+// The block of a piece that step j takes: the decode groups in turn, each the next of its blocks.
+template <int MT>
+__device__ __forceinline__ int mc_block(int j) { constexpr int G = MC_DEC / (MT * MC_BM); return j % G * (MC_STEPS / G) + j / G; }
+// Group g of G has blocks g * 8 / G on of a row's eight, from the 16 bytes on that its first one starts in: 8 / G blocks, their number I
+// known at compile time.
+template <int G>
+__device__ __forceinline__ int mc_group_start(int g) { return g * (MC_RAW_ROW / G) / 16 * 16; }
+template <int G, int I>
+__device__ __forceinline__ void mc_decode_of(int g, const u32* W, u8* __restrict__ dst) {
+    constexpr int S = MC_RAW_ROW / G;
+    if (g == 0) mc_decode_block<34 * I>(W, dst);
+    else if (g == 1) mc_decode_block<S % 16 + 34 * I>(W, dst);
+    else if (G == 4 && g == 2) mc_decode_block<2 * S % 16 + 34 * I>(W, dst);
+    else if (G == 4) mc_decode_block<3 * S % 16 + 34 * I>(W, dst);
+}
 
 // The token rows as f16 in the order the instruction reads them from shared memory, so that a step's tile is one contiguous copy:
 // out[tile][step][chunk c of 8 columns][token t][8 halves]; tokens past m are zero.  One thread a 16-byte unit.
-__global__ void __launch_bounds__(256) sz_x16_pack_kernel(const float* __restrict__ x, long long xs, int m, int cols, int nt, uint4* __restrict__ out) {
-    const int steps = cols / MC_KT;
-    const long long units = (long long)((m + nt - 1) / nt) * steps * 8 * nt;
+__global__ void __launch_bounds__(256) sz_x16_pack_kernel(const float* __restrict__ x, long long xs, int m, int cols, int nt, int tiles, uint4* __restrict__ out) {
+    const int steps = cols / MC_PS;
+    const long long units = (long long)tiles * steps * 8 * nt;
+    sz_pdl_wait();
+    sz_pdl_trigger();
     for (long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x; u < units; u += (long long)gridDim.x * blockDim.x) {
         const int t = (int)(u % nt);
         long long r = u / nt;
@@ -115,7 +147,7 @@ __global__ void __launch_bounds__(256) sz_x16_pack_kernel(const float* __restric
         const int tok = tile * nt + t;
         uint4 v = make_uint4(0, 0, 0, 0);
         if (tok < m) {
-            const float4* p = (const float4*)(x + (long long)tok * xs + ks * MC_KT + c * 8);
+            const float4* p = (const float4*)(x + (long long)tok * xs + ks * MC_PS + c * 8);
             const float4 a = __ldg(p), b = __ldg(p + 1);
             __half2 h0 = __floats2half2_rn(a.x, a.y), h1 = __floats2half2_rn(a.z, a.w), h2 = __floats2half2_rn(b.x, b.y), h3 = __floats2half2_rn(b.z, b.w);
             v = make_uint4(*(u32*)&h0, *(u32*)&h1, *(u32*)&h2, *(u32*)&h3);
@@ -124,29 +156,41 @@ __global__ void __launch_bounds__(256) sz_x16_pack_kernel(const float* __restric
     }
 }
 
+template <int I> struct McInt { static constexpr int value = I; };
+
+struct McArgs {
+    const uint4* x16;
+    float* y;
+    long long ys;
+    int rows, cols, m, nt, tiles, ks;   // nt: tokens a tile; ks: blocks of a cluster, the parts of K
+    u32* err;
+};
+
+// grid: ks == 1, up to 148 blocks that take (row tile, token tile) units in turn; else (units * ks), cluster (ks).
+template <int MT>
 __global__ void __launch_bounds__(MC_THREADS, 1)
-sz_mma_cols_q8_kernel(const __grid_constant__ CUtensorMap wmap, const uint4* __restrict__ x16, float* __restrict__ y, long long ys, int rows, int cols,
-                      int m, int nt, u32* __restrict__ err) {
+sz_mma_cols_q8_kernel(const __grid_constant__ CUtensorMap wmap, const McArgs a) {
     extern __shared__ __align__(128) u8 smem[];
-    u8* raw = smem;                                   // [2][128 rows][272]
-    u8* sa = raw + 2 * MC_RAW_BYTES;                  // [stages][16 chunks][16 row groups][128]
-    u8* sb = sa + MC_STAGES * MC_A_BYTES;             // [stages][8 chunks][nt / 8 token groups][128]
-    const int b_bytes = nt * MC_KT * 2;
+    const int nt = a.nt, b_bytes = nt * MC_KT * 2;
+    u8* raw = smem;                                   // [MT * 128 rows][272]
+    u8* sa = raw + MT * MC_RAW_BYTES;                 // [stages][MT][4 chunks][16 row groups][128]
+    u8* sb = sa + MC_STAGES * MT * MC_A_BYTES;        // [stages][4 chunks][nt / 8 token groups][128]
     McSmem* S = (McSmem*)(sb + MC_STAGES * b_bytes);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int row0 = blockIdx.x * MC_BM, tile = blockIdx.y;
-    const int valid = rows - row0 < MC_BM ? rows - row0 : MC_BM;
-    const int steps = cols / MC_KT;
+    const int rtiles = (a.rows + MT * MC_BM - 1) / (MT * MC_BM), units = rtiles * a.tiles;
+    const int kr = (int)blockIdx.x % a.ks, u0 = (int)blockIdx.x / a.ks, us = (int)gridDim.x / a.ks;
+    const int P = a.cols / MC_SS, p0 = P * kr / a.ks, pieces = P * (kr + 1) / a.ks - p0, steps = pieces * MC_STEPS;
+    constexpr int LAST = MC_DEC / 32;                 // the last decode warp
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < MC_STAGES; i++) { sz_mbar_init(&S->full[i], 256 + 1); sz_mbar_init(&S->empty[i], 1); }
-        for (int i = 0; i < 2; i++) { sz_mbar_init(&S->raw_full[i], 1); sz_mbar_init(&S->raw_empty[i], 256); }
-        sz_mbar_init(&S->acc_full, 1);
+        for (int i = 0; i < MC_STAGES; i++) { sz_mbar_init(&S->full[i], MT * MC_BM / 32 + 1); sz_mbar_init(&S->empty[i], 1); }
+        sz_mbar_init(&S->raw_full, 1); sz_mbar_init(&S->raw_empty, MC_DEC / 32);
+        sz_mbar_init(&S->acc_full, 1); sz_mbar_init(&S->acc_empty, MC_DEC / 32);
         S->failed = 0;
         sz_mbar_fence_init();
     }
-    if (warp == 0) {   // tensor memory for the accumulator: 256 columns (a power of two >= nt), the whole warp asks
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sz_smem_addr(&S->tmem_base)), "r"(256u) : "memory");
+    if (warp == 0) {   // tensor memory for the accumulators: MT x 256 columns, the whole warp asks
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sz_smem_addr(&S->tmem_base)), "r"((u32)MT * 256u) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     mc_tc_fence_before();
@@ -155,118 +199,213 @@ sz_mma_cols_q8_kernel(const __grid_constant__ CUtensorMap wmap, const uint4* __r
     const u32 tmem = S->tmem_base;
     int failed = 0;
 
+    // A step's stage is its number % MC_STAGES, a unit and a piece are whole rings; k counts the steps of all units, n the units.
     if (warp == 0) {
-        // ---- copies: raw weight bytes one 256-column piece ahead of the decoders, token tiles as stages come free
-        const int pieces = steps / 4;
-        auto issue_raw = [&](int ss) {   // x = 136 * ss words = 272 * ss bytes: a multiple of 16; rows past the matrix arrive as zeros
-            const int rb = ss & 1;
-            if (lane == 0) {
-                sz_mbar_expect_tx(&S->raw_full[rb], (u32)MC_RAW_BYTES);
-                asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-                                 sz_smem_addr(raw + rb * MC_RAW_BYTES)),
-                             "l"(&wmap), "r"(ss * (MC_RAW_ROW / 2)), "r"(row0), "r"(sz_smem_addr(&S->raw_full[rb]))
-                             : "memory");
+        // ---- token tiles as stages come free (what the pack kernel wrote: after the dependency wait)
+        sz_pdl_wait();
+        sz_pdl_trigger();
+        for (int u = u0, k = 0; u < units && !failed; u += us) {
+            const u8* src = (const u8*)a.x16 + ((size_t)(u / rtiles) * (a.cols / MC_KT) + p0 * MC_STEPS) * b_bytes;
+            for (int j = 0; j < steps; j++, k++) {
+                const int st = k % MC_STAGES;
+                if (k >= MC_STAGES && !sz_mbar_wait(&S->empty[st], ((k / MC_STAGES) - 1) & 1, MC_WAIT)) { failed = 1; break; }
+                if (lane == 0) {
+                    sz_mbar_expect_tx(&S->full[st], (u32)b_bytes);
+                    sz_bulk_g2s(sb + st * b_bytes, src + (size_t)(j / MC_STEPS * MC_STEPS + mc_block<MT>(j % MC_STEPS)) * b_bytes, (u32)b_bytes, &S->full[st]);
+                }
+            }
+        }
+    } else if (warp == LAST + 2) {
+        // ---- raw weight bytes, a piece as soon as the decoders have the one before it in registers
+        for (int u = u0, n = 0; u < units && !failed; u += us)
+            for (int p = 0; p < pieces; p++, n++) {
+                if (n > 0 && !sz_mbar_wait(&S->raw_empty, (n - 1) & 1, MC_WAIT)) { failed = 2; break; }
+                if (lane == 0) {   // x = 136 * piece words = 272 * piece bytes: a multiple of 16; rows past the matrix arrive as zeros
+                    sz_mbar_expect_tx(&S->raw_full, (u32)(MT * MC_RAW_BYTES));
+#pragma unroll
+                    for (int mt = 0; mt < MT; mt++)
+                        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+                                         sz_smem_addr(raw + mt * MC_RAW_BYTES)),
+                                     "l"(&wmap), "r"((p0 + p) * (MC_RAW_ROW / 2)), "r"((u % rtiles * MT + mt) * MC_BM), "r"(sz_smem_addr(&S->raw_full))
+                                     : "memory");
+                }
+            }
+    } else if (warp == LAST + 1) {
+        // ---- issue: one thread, descriptors of the ring's first stage made once (a step is 256 cycles of the tensor core
+        // at 256 tokens and MT = 1: what this thread does besides its instructions is on the path)
+        if (lane == 0) {
+            const u32 idesc = mc_idesc(nt);
+            const u64 ad = mc_desc(sz_smem_addr(sa), MC_BM * 16, 128), bd = mc_desc(sz_smem_addr(sb), (u32)nt * 16, 128);
+            u32 phase = 0;
+            for (int u = u0, n = 0; u < units && !failed; u += us, n++) {
+                if (n > 0 && !sz_mbar_wait(&S->acc_empty, (n - 1) & 1, MC_WAIT)) { failed = 7; break; }
+                for (int j = 0; j < steps; j += MC_STAGES, phase ^= 1) {
+#pragma unroll
+                    for (int st = 0; st < MC_STAGES; st++) {
+                        if (!sz_mbar_wait(&S->full[st], phase, MC_WAIT)) { failed = 5; break; }
+                        mc_tc_fence_after();
+#pragma unroll
+                        for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+                            for (int q = 0; q < MC_KT / 16; q++)      // (addresses are in 16-byte units, in the low bits)
+                                mc_mma(tmem + mt * 256, ad + (u32)((st * MT + mt) * (MC_A_BYTES / 16) + q * 2 * MC_BM), bd + (u32)(st * (nt * MC_KT / 8) + q * 2 * nt), idesc, (j | st | q) ? 1u : 0u);
+                        mc_commit(&S->empty[st]);
+                    }
+                    if (failed) break;
+                }
+                mc_commit(&S->acc_full);      // arrives when every instruction above has finished (also after a failure: nothing pending then)
+            }
+        }
+        __syncwarp();
+    } else {
+        // ---- decode: thread d has row d % (128 MT) and 8 / G blocks of it; then the accumulators to Y.  A warp reads the 32 lanes of
+        // its quadrant (warp % 4), the four warps of a quadrant take every fourth 16 columns.
+        constexpr int G = MC_DEC / (MT * MC_BM), NW = MC_RAW_ROW / 16 / G + 1;      // 16-byte words of a group's blocks
+        const int d = threadIdx.x - 32, g = d / (MT * MC_BM), r = d % (MT * MC_BM), mtd = r >> 7;
+        u8* const dst0 = sa + mtd * MC_A_BYTES + ((r & 127) >> 3) * 128 + (r & 7) * 16;
+        const int quad = warp & 3, part = (warp - 1) >> 2;
+        auto load16 = [&](int mt, int c, u32* v) {
+            asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                         : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+                           "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+                         : "r"(tmem + ((u32)(quad * 32) << 16) + (u32)(mt * 256 + c)));
+        };
+        auto loaded16 = [&](u32* v) {     // the registers go through the wait, so that nothing uses them before it
+            asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
+                         "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]) :: "memory");
+        };
+        auto store16 = [&](int u, int mt, int c, const u32* v) {
+            const int row = (u % rtiles * MT + mt) * MC_BM + quad * 32 + lane, tok = u / rtiles * nt + c;
+            if (row >= a.rows) return;
+            float* y = a.y + (long long)tok * a.ys + row;
+            if (tok + 16 <= a.m) {
+#pragma unroll
+                for (int i = 0; i < 16; i++, y += a.ys) *y = __uint_as_float(v[i]);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 16; i++, y += a.ys)
+                    if (tok + i < a.m) *y = __uint_as_float(v[i]);
             }
         };
-        issue_raw(0);
-        for (int ks = 0; ks < steps && !failed; ks++) {
-            const int st = ks % MC_STAGES;
-            if (ks % 4 == 0 && ks / 4 + 1 < pieces) {
-                const int ss = ks / 4 + 1;
-                if (ss >= 2 && !sz_mbar_wait(&S->raw_empty[ss & 1], ((ss / 2) - 1) & 1, MC_WAIT)) { failed = 2; break; }
-                issue_raw(ss);
-            }
-            if (ks >= MC_STAGES && !sz_mbar_wait(&S->empty[st], ((ks / MC_STAGES) - 1) & 1, MC_WAIT)) { failed = 1; break; }
-            if (lane == 0) {
-                sz_mbar_expect_tx(&S->full[st], (u32)b_bytes);
-                sz_bulk_g2s(sb + st * b_bytes, (const u8*)x16 + ((size_t)tile * steps + ks) * b_bytes, (u32)b_bytes, &S->full[st]);
-            }
-        }
-    } else if (warp <= 8) {
-        // ---- decode: thread d takes weight row d % 128 and block d / 128 of the step (a warp: 32 consecutive rows of one block
-        // index, so its 16-byte stores fill 512 consecutive bytes and its block index is known when the code is compiled)
-        const int d = threadIdx.x - 32, r = d & 127, half = d >> 7;
-        for (int ks0 = 0; ks0 < steps && !failed; ks0 += 4) {
-            const int ss = ks0 / 4, rb = ss & 1;
-            if (!sz_mbar_wait(&S->raw_full[rb], (ss / 2) & 1, MC_WAIT)) { failed = 4; break; }
-            const u8* rowp = raw + rb * MC_RAW_BYTES + r * MC_RAW_ROW;
+        int k0 = 0, n = 0, np = 0;
+        for (int u = u0; u < units && !failed; u += us, n++) {
+            for (int p = 0; p < pieces && !failed; p++, np++, k0 += MC_STEPS) {
+                if (!sz_mbar_wait(&S->raw_full, np & 1, MC_WAIT)) { failed = 4; break; }
+                u32 W[NW * 4];
+                const uint4* rp = (const uint4*)(raw + (size_t)r * MC_RAW_ROW + mc_group_start<G>(g));
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int ks = ks0 + j, st = ks % MC_STAGES;
-                if (ks >= MC_STAGES && !sz_mbar_wait(&S->empty[st], ((ks / MC_STAGES) - 1) & 1, MC_WAIT)) { failed = 3; break; }
-                u8* dst = sa + st * MC_A_BYTES + ((half * 4) * 16 + (r >> 3)) * 128 + (r & 7) * 16;
-                if (r < valid) {
-                    switch (2 * j + half) {   // j is an unrolled loop's counter and half is the same for a whole warp
-                        case 0: mc_decode_block<0>(rowp, dst); break;
-                        case 1: mc_decode_block<1>(rowp, dst); break;
-                        case 2: mc_decode_block<2>(rowp, dst); break;
-                        case 3: mc_decode_block<3>(rowp, dst); break;
-                        case 4: mc_decode_block<4>(rowp, dst); break;
-                        case 5: mc_decode_block<5>(rowp, dst); break;
-                        case 6: mc_decode_block<6>(rowp, dst); break;
-                        default: mc_decode_block<7>(rowp, dst); break;
-                    }
-                } else {
-#pragma unroll
-                    for (int c = 0; c < 4; c++) *(uint4*)(dst + c * 16 * 128) = make_uint4(0, 0, 0, 0);
-                }
-                mc_fence_async();                 // the tensor core reads shared memory through the async proxy
-                mc_arrive(&S->full[st]);
+                for (int i = 0; i < NW; i++) { const uint4 v = rp[i]; W[4 * i] = v.x; W[4 * i + 1] = v.y; W[4 * i + 2] = v.z; W[4 * i + 3] = v.w; }
+                mc_arrive_warp(&S->raw_empty);
+                auto step = [&](auto I) {
+                    constexpr int i = decltype(I)::value;
+                    const int k = k0 + i * G + g, st = k % MC_STAGES;
+                    if (failed) return;
+                    if (k >= MC_STAGES && !sz_mbar_wait(&S->empty[st], ((k / MC_STAGES) - 1) & 1, MC_WAIT)) { failed = 3; return; }
+                    mc_decode_of<G, i>(g, W, dst0 + st * MT * MC_A_BYTES);
+                    mc_fence_async();                 // the tensor core reads shared memory through the async proxy
+                    mc_arrive_warp(&S->full[st]);
+                };
+                step(McInt<0>()); step(McInt<1>());
+                if constexpr (G == 2) { step(McInt<2>()); step(McInt<3>()); }
             }
-            if (failed) break;
-            mc_arrive(&S->raw_empty[rb]);
-        }
-    } else {
-        // ---- issue
-        const u32 idesc = mc_idesc(nt);
-        for (int ks = 0; ks < steps && !failed; ks++) {
-            const int st = ks % MC_STAGES;
-            if (!sz_mbar_wait(&S->full[st], (ks / MC_STAGES) & 1, MC_WAIT)) { failed = 5; break; }
+            if (!failed && !sz_mbar_wait(&S->acc_full, n & 1, MC_WAIT)) failed = 6;
+            const int any = __any_sync(0xffffffffu, failed);
             mc_tc_fence_after();
-            if (lane == 0) {
-                const u32 a0 = sz_smem_addr(sa + st * MC_A_BYTES), b0 = sz_smem_addr(sb + st * b_bytes);
-#pragma unroll
-                for (int k = 0; k < MC_KT / 16; k++)
-                    mc_mma(tmem, mc_desc(a0 + k * 2 * (MC_BM * 16), MC_BM * 16, 128), mc_desc(b0 + k * 2 * (nt * 16), (u32)nt * 16, 128), idesc, (ks | k) ? 1u : 0u);
-                mc_commit(&S->empty[st]);
+            if (a.ks == 1) {
+                if (!any) {
+                    for (int t = part; t < MT * (nt / 16); t += 4) {
+                        u32 v[16];
+                        const int mt = MT == 2 && t >= nt / 16, c = (t - mt * (nt / 16)) * 16;
+                        load16(mt, c, v);
+                        loaded16(v);
+                        store16(u, mt, c, v);
+                    }
+                    mc_tc_fence_before();
+                    mc_arrive_warp(&S->acc_empty);
+                }
+                continue;
             }
-            __syncwarp();
+            // one unit: its sums are the cluster's
+            const int nu = nt / 16;
+            auto unit0 = [&](int rank) { return nu * rank / a.ks; };   // the 16-column units a block finishes
+            mc_cluster_sync();           // every block of the cluster is done with its stages: they take the other blocks' parts
+            if (!any)
+                for (int o = 0; o < a.ks; o++) {
+                    if (o == kr) continue;
+                    const int c0 = unit0(o), cn = unit0(o + 1) - c0, slot = kr < o ? kr : kr - 1;
+                    u32 base;
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(base) : "r"(sz_smem_addr(smem)), "r"(o));
+                    for (int t = part; t < MT * cn; t += 4) {
+                        u32 v[16];
+                        const int mt = t / cn, c = t - mt * cn;
+                        load16(mt, (c0 + c) * 16, v);
+                        loaded16(v);
+                        const u32 at = base + (u32)((((slot * MT + mt) * cn + c) * 16 * 128 + quad * 32 + lane) * 4);
+#pragma unroll
+                        for (int i = 0; i < 16; i++) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(at + (u32)i * 512u), "r"(v[i]) : "memory");
+                    }
+                }
+            mc_cluster_sync();           // .. which are here now
+            if (!any) {
+                const int c0 = unit0(kr), cn = unit0(kr + 1) - c0;
+                for (int t = part; t < MT * cn; t += 4) {
+                    u32 v[16];
+                    float s[16];
+                    const int mt = t / cn, c = t - mt * cn;
+                    load16(mt, (c0 + c) * 16, v);
+                    loaded16(v);
+                    for (int k = 0; k < a.ks; k++) {        // in the order of K, whoever has the part
+                        const float* part_k = (const float*)smem + (size_t)(((k < kr ? k : k - 1) * MT + mt) * cn + c) * 16 * 128 + quad * 32 + lane;
+#pragma unroll
+                        for (int i = 0; i < 16; i++) {
+                            const float x = k == kr ? __uint_as_float(v[i]) : part_k[i * 128];
+                            s[i] = k == 0 ? x : s[i] + x;
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < 16; i++) v[i] = __float_as_uint(s[i]);
+                    store16(u, mt, (c0 + c) * 16, v);
+                }
+            }
         }
-        if (lane == 0) mc_commit(&S->acc_full);   // arrives when every instruction above has finished (also after a failure: nothing pending then)
     }
     if (failed) atomicMax(&S->failed, (u32)failed);
-
-    // ---- the accumulator to Y: warps 1..8; a warp reads the 32 lanes of its quadrant (warp % 4), the two warps of a quadrant take
-    // half of the columns each
-    if (warp >= 1 && warp <= 8 && !failed) {
-        if (!sz_mbar_wait(&S->acc_full, 0, MC_WAIT)) {
-            atomicMax(&S->failed, 6u);
-        } else {
-            mc_tc_fence_after();
-            const int q = warp & 3, hcol = (warp - 1) >> 2;
-            const int c0 = hcol * (nt / 2), c1 = c0 + nt / 2;
-            const int row = row0 + q * 32 + lane;
-            for (int c = c0; c < c1; c += 8) {
-                u32 v[8];
-                asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                             : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-                             : "r"(tmem + ((u32)(q * 32) << 16) + (u32)c));
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    const int tok = tile * nt + c + i;
-                    if (tok < m && row < rows) y[(long long)tok * ys + row] = __uint_as_float(v[i]);
-                }
-            }
-        }
-    }
+    if (a.ks > 1 && (warp == 0 || warp > LAST)) { mc_cluster_sync(); mc_cluster_sync(); }    // the decoders' two
     mc_tc_fence_before();
     __syncthreads();
     if (warp == 0) {
         mc_tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((u32)MT * 256u) : "memory");
     }
-    if (threadIdx.x == 0 && S->failed) atomicMax(err, S->failed);
+    if (threadIdx.x == 0 && S->failed) atomicMax(a.err, S->failed);
+}
+
+// What a call takes: 128-row tiles a block (mt), blocks along K (ks), token tiles of nt tokens.  The least of an estimate in microseconds,
+// with what was measured put into it: a piece of 256 columns takes a block 1.85 us with one row tile and 3.2 with two at 256 tokens, of
+// which 0.35 and 1 go with the tokens (the rest is decoding); L2 gives the blocks that run together 10.8 TB/s; the sums go to memory at
+// 6.5 TB/s; a cluster's exchange costs a little for each block of it, and of clusters of 2, 3 and 4 blocks the chip holds 74, 45 and 33 at
+// once.  So two row tiles win where the units are many (the tokens cross L2 half as often), parts of K where they are few, and a token
+// tile more than the fewest where it fills the last turn.  With one token tile the estimate does not look at its width, so that a token's
+// sums are the same however many tokens come with it.
+struct McPlan { int mt, ks, nt, tiles; };
+McPlan mc_plan(int rows, int cols, int m) {
+    const int P = cols / MC_SS, t0 = (m + MC_NT_MAX - 1) / MC_NT_MAX;
+    McPlan best = {};
+    float least = -1.f;
+    for (int tiles = t0; tiles <= t0 + (t0 > 1 && t0 < 8 ? MC_TILES_MORE : 0); tiles++)
+        for (int mt = 1; mt <= 2; mt++)
+            for (int ks = 1; ks <= MC_KS_MAX && ks <= P; ks++) {
+                const int nt = (((m + tiles - 1) / tiles) + 15) & ~15, slots = ks == 1 ? 148 : ks == 2 ? 74 : ks == 3 ? 45 : 33;
+                const int units = (rows + mt * MC_BM - 1) / (mt * MC_BM) * tiles, pieces = (P + ks - 1) / ks;
+                const float w = tiles == 1 ? 1.f : nt / 256.f;
+                auto turn = [&](int n) {      // n units at once
+                    const float work = mt == 1 ? 1.5f + 0.35f * w : 2.2f + w, l2 = n * ks * (16.f * w + 4.35f * mt) * 7.6e-4f;
+                    return pieces * (work > l2 ? work : l2) + n * mt * w * 0.02f + (ks > 1 ? 1.7f * ks - 1.1f + 1.8f * (mt - 1) : 0.f) + 2.f * (mt - 1);
+                };
+                const float cost = units / slots * turn(slots) + (units % slots ? turn(units % slots) : 0.f);
+                if (least < 0.f || cost < 0.97f * least) { least = cost; best = {mt, ks, nt, tiles}; }
+            }
+    return best;
 }
 
 typedef CUresult (*McEncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
@@ -281,9 +420,35 @@ McEncodeTiled mc_encoder() {
     return fn;
 }
 
-int mc_nt(int m) {
-    const int r = (m + 15) & ~15;
-    return r < MC_NT_MAX ? r : MC_NT_MAX;
+
+template <int MT>
+int mc_launch(const CUtensorMap& wmap, const McArgs& a, cudaStream_t st) {
+    size_t smem = MT * MC_RAW_BYTES + MC_STAGES * (MT * MC_A_BYTES + (size_t)a.nt * MC_KT * 2) + sizeof(McSmem);
+    if (smem < MC_SMEM_MIN) smem = MC_SMEM_MIN;
+    static bool set = false;
+    if (!set) {
+        SZ_CUDA(cudaFuncSetAttribute(sz_mma_cols_q8_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     MT * MC_RAW_BYTES + MC_STAGES * (MT * MC_A_BYTES + MC_NT_MAX * MC_KT * 2) + (int)sizeof(McSmem)));
+        set = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    const int units = (a.rows + MT * MC_BM - 1) / (MT * MC_BM) * a.tiles;
+    cfg.gridDim = dim3(a.ks > 1 ? units * a.ks : units < 148 ? units : 148);
+    cfg.blockDim = dim3(MC_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)a.ks;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = a.ks > 1 ? 2 : 1;
+    SZ_CUDA(cudaLaunchKernelEx(&cfg, sz_mma_cols_q8_kernel<MT>, wmap, a));
+    sz_trace_mark("mma_cols_q8", st);
+    return SZ_OK;
 }
 
 }  // namespace
@@ -291,8 +456,7 @@ int mc_nt(int m) {
 // Bytes of scratch for up to m token rows of `cols` inputs: an error word and the f16 copy of the rows.
 extern "C" int sz_mma_cols_scratch_bytes(int cols, int m, int64_t* bytes) {
     if (!bytes || m < 1 || cols < MC_SS || cols % MC_SS) return sz_fail(SZ_E_ARG, "sz_mma_cols_scratch_bytes: m >= 1 and cols a multiple of %d", MC_SS);
-    const int nt = mc_nt(m);
-    *bytes = 256 + (int64_t)((m + nt - 1) / nt) * nt * cols * 2;
+    *bytes = 256 + ((int64_t)m + 16 * ((m + MC_NT_MAX - 1) / MC_NT_MAX + MC_TILES_MORE)) * cols * 2;     // whichever tiling a matrix takes
     return SZ_OK;
 }
 
@@ -308,15 +472,11 @@ extern "C" int sz_mma_cols(const sz_tensor* w, uint64_t x, int64_t xs, uint64_t 
     if ((x & 15) || (xs & 3) || (w->data & 15) || (scratch & 255)) return sz_fail(SZ_E_ARG, "sz_mma_cols: x rows and the weights 16-byte aligned, scratch 256-byte aligned");
     if (w->rows < 1) return sz_fail(SZ_E_ARG, "sz_mma_cols: no rows");
     cudaStream_t st = (cudaStream_t)stream;
-    const int nt = mc_nt(m), tiles = (m + nt - 1) / nt, cols = (int)w->cols, rows = (int)w->rows;
+    const int cols = (int)w->cols, rows = (int)w->rows;
+    const McPlan plan = mc_plan(rows, cols, m);
+    const int nt = plan.nt, tiles = plan.tiles;
     u32* err = (u32*)scratch;
     uint4* x16 = (uint4*)(scratch + 256);
-    const size_t smem = 2 * MC_RAW_BYTES + MC_STAGES * (MC_A_BYTES + (size_t)nt * MC_KT * 2) + sizeof(McSmem);
-    static bool set = false;
-    if (!set) {
-        SZ_CUDA(cudaFuncSetAttribute(sz_mma_cols_q8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * MC_RAW_BYTES + MC_STAGES * (MC_A_BYTES + MC_NT_MAX * MC_KT * 2) + (int)sizeof(McSmem)));
-        set = true;
-    }
     McEncodeTiled enc = mc_encoder();
     if (!enc) return sz_fail(SZ_E_CUDA, "sz_mma_cols: the driver has no cuTensorMapEncodeTiled");
     CUtensorMap wmap;
@@ -328,12 +488,12 @@ extern "C" int sz_mma_cols(const sz_tensor* w, uint64_t x, int64_t xs, uint64_t 
                                CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_SUCCESS) return sz_fail(SZ_E_CUDA, "sz_mma_cols: cuTensorMapEncodeTiled failed (%d)", (int)r);
     }
-    const long long units = (long long)tiles * (cols / MC_KT) * 8 * nt;
-    SZ_CUDA(sz_launch("x16_pack", sz_x16_pack_kernel, dim3((unsigned)((units + 255) / 256 < 1184 ? (units + 255) / 256 : 1184)), dim3(256), 0, st, false,
-                      (const float*)x, (long long)xs, m, cols, nt, x16));
-    SZ_CUDA(sz_launch("mma_cols_q8", sz_mma_cols_q8_kernel, dim3((rows + MC_BM - 1) / MC_BM, tiles), dim3(MC_THREADS), smem, st, false, wmap,
-                      (const uint4*)x16, (float*)y, (long long)ys, rows, cols, m, nt, err));
-    return SZ_OK;
+    const long long units = (long long)tiles * (cols / MC_PS) * 8 * nt;
+    SZ_CUDA(sz_launch("x16_pack", sz_x16_pack_kernel, dim3((unsigned)((units + 255) / 256 < 1184 ? (units + 255) / 256 : 1184)), dim3(256), 0, st, true,
+                      (const float*)x, (long long)xs, m, cols, nt, tiles, x16));
+    McArgs a;
+    a.x16 = x16; a.y = (float*)y; a.ys = (long long)ys; a.rows = rows; a.cols = cols; a.m = m; a.nt = nt; a.tiles = tiles; a.ks = plan.ks; a.err = err;
+    return plan.mt == 2 ? mc_launch<2>(wmap, a, st) : mc_launch<1>(wmap, a, st);
 }
 
 // Clears (init != 0) or reads the scratch's error word; reading synchronises the stream.  0: no wait of a kernel ran out.

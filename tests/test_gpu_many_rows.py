@@ -1,0 +1,77 @@
+"""The forms that take many rows at once, at the sizes where they could go wrong: one row more or less than a tile, a chunk, a block's
+group; the smallest and largest of their ranges.  A session's rows are bit for bit those of passes of up to 8 rows; a block-format expert
+layer and the tensor-core projections are held against the CPU restatement."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import binding as ob
+from tests.test_gpu_batch import CFG
+from tests.test_gpu_mma_cols import make
+from tests.test_gpu_moe import run_case
+from tests.util import pkg
+
+szlib, synth, md, moe = pkg.lib, pkg.synth, pkg.model, pkg.moe
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dm():
+    return md.DeviceModel(md.make_model(CFG, expert_type=szlib.TYPE_EXL3(3), seed=4, cycle_alpha=0.9, cycle_beta=0.5))
+
+
+# 16 rows: the fewest that go as a chunk; 128 / 136: where the reads change their form; 256 / 264: one chunk, two
+@pytest.mark.parametrize("n", [16, 17, 25, 129, 137, 145, 257, 265, 273])
+def test_a_prompt_in_chunks_equals_passes_of_eight_rows(dm, n):
+    prompt = md.make_prompt(n, CFG["vocab"], seed=60 + n)
+    a, b = md.Session(dm, 320, kv_q8=True), md.Session(dm, 320, kv_q8=True)
+    a.prefill(prompt)
+    for c in range(0, n, 8):
+        rows = prompt[c:c + 8]
+        b.verify(rows)
+        _, top2, lg2 = b.result(logits=True)
+        if c + 8 < n:
+            b.commit(len(rows))
+    _, top, lg = a.result(logits=True)
+    assert np.array_equal(lg.view(np.uint32), lg2.view(np.uint32)) and np.array_equal(top, top2)
+    for s in (a, b):
+        s.commit((n - 1) % 8 + 1)
+        s.verify([5, 6, 7])
+    assert np.array_equal(a.result(logits=True)[2].view(np.uint32), b.result(logits=True)[2].view(np.uint32))
+
+
+@pytest.mark.parametrize("n_expert,top_k,rows", [(16, 1, 8), (16, 16, 24), (16, 2, 256), (64, 4, 248), (512, 10, 136)])
+def test_groups_of_many_and_of_few_rows_an_expert(n_expert, top_k, rows):
+    """16 experts of 256 rows: more rows an expert than a group takes; 512 of 136: most experts have two or three; 16 of 16: all."""
+    ty = szlib.TYPE_EXL3(3)
+    ml = moe.MoeLayer(synth.make_moe_layer(512, n_expert, top_k, 256, 256, ty, ty, seed=7), "cuda:0")
+    x = synth.normal((rows, 512), 1.0, 9, "rows.edges").cuda()
+    y = ml.moe_rows(x)
+    assert ml.moe_rows_status(rows) == 0
+    for c in range(0, rows, 8):
+        yc = ml.moe_batch(x[c:c + 8].contiguous())
+        assert torch.equal(y[c:c + 8].view(torch.int32), yc.view(torch.int32)), "rows %d.." % c
+
+
+# the shared expert in both launches of the routed ones, in the first only (another width), in none (another type), absent
+@pytest.mark.parametrize("ff,sf,ety,sty,m", [(256, 256, "iq3", "iq3", 8), (256, 512, "iq3", "iq3", 3), (512, 512, "q8", "q8", 8), (256, 256, "iq3", "q8", 5),
+                                             (512, 0, "iq3", "iq3", 4), (1024, 1024, "iq3", "iq3", 8), (256, 256, "q8", "q8", 1)])
+def test_block_format_experts_with_and_without_the_shared_one_beside_them(ff, sf, ety, sty, m):
+    ty = {"iq3": szlib.TYPE_IQ3_S, "q8": szlib.TYPE_Q8_0}
+    run_case(512, 32, 4, ff, sf, ty[ety], ty[sty], m, seed=40)
+
+
+# K in 2, 3 and 4 parts (3 of unequal length), two row tiles a block with a ragged last one, several units a block, one token a tile
+@pytest.mark.parametrize("rows,cols,m", [(130, 1024, 1), (300, 1024, 70), (385, 3328, 40), (129, 2304, 257), (512, 2048, 17), (3000, 768, 2049), (2600, 512, 2000)])
+def test_projections_split_along_k_and_over_row_tiles(rows, cols, m):
+    wb = make(rows, cols, 21)
+    x = synth.normal((m, cols), 1.0, 23, "mma_cols.x")
+    op = pkg.mma_cols.MmaCols(wb, rows, cols, m)
+    y = torch.full((m + 1, rows + 5), -7.0, device="cuda")
+    op(x.cuda(), out=y[:m, :rows])
+    assert op.status() == 0 and bool((y[m] == -7.0).all()) and bool((y[:, rows:] == -7.0).all())
+    w16 = torch.from_numpy(ob.dequant(ob.Q8_0, wb.numpy()).reshape(rows, cols)).half().double()
+    x16 = x.half().double()
+    want, mag = x16 @ w16.T, x16.abs() @ w16.abs().T
+    assert float(((y[:m, :rows].cpu().double() - want).abs() / (cols * 2.0 ** -23 * mag + 1e-30)).max()) < 1.0
