@@ -1198,9 +1198,21 @@ extern "C" int sz_moe_rows(const sz_moe_layer* L, uint64_t x, int rows, uint64_t
     return sz_rows_run(L, x, rows, rows, y, route_idx, route_w, scratch, scratch_bytes, SZ_ROWS_MAX, stream);
 }
 
-// The form inside a session's step: `live` of the rows count; and whether a layer has it.
-int sz_moe_rows_live(const sz_moe_layer* L, uint64_t x, int rows, int live, uint64_t y, uint64_t scratch, int64_t scratch_bytes, uint64_t stream) {
-    return sz_rows_run(L, x, rows, live, y, 0, 0, scratch, scratch_bytes, SZ_ROWS_MAX, stream);
+// The form inside a session's step, where a prompt's chunk has up to SZ_ROWS_CAP rows: the scratch for room of `room` rows, cleared once,
+// and the pass, of which `live` rows count; and whether a layer has it.
+static int sz_rows_cap(int room) { return room <= SZ_ROWS_MAX ? SZ_ROWS_MAX : SZ_ROWS_CAP; }
+int sz_moe_rows_room(const sz_moe_layer* L, int room, int64_t* bytes) {
+    if (room < 8 || room > SZ_ROWS_CAP || room % 8) return sz_fail(SZ_E_ARG, "sz_moe_rows: rows = %d (a multiple of 8 up to %d)", room, SZ_ROWS_CAP);
+    *bytes = sz_rows_layout(L, sz_rows_cap(room)).total;
+    return SZ_OK;
+}
+int sz_moe_rows_clear(const sz_moe_layer* L, int room, uint64_t scratch, uint64_t stream) {
+    const SzRowsScratch S = sz_rows_layout(L, sz_rows_cap(room));
+    SZ_CUDA(cudaMemsetAsync((u8*)scratch + S.ctrl, 0, (size_t)(S.logits - S.ctrl), (cudaStream_t)stream));
+    return SZ_OK;
+}
+int sz_moe_rows_live(const sz_moe_layer* L, uint64_t x, int rows, int live, int room, uint64_t y, uint64_t scratch, int64_t scratch_bytes, uint64_t stream) {
+    return sz_rows_run(L, x, rows, live, y, 0, 0, scratch, scratch_bytes, sz_rows_cap(room), stream);
 }
 bool sz_moe_rows_takes(const sz_moe_layer* L) {
     const SzFast f = sz_fast_path(L);

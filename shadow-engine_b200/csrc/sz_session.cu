@@ -33,8 +33,11 @@ int sz_ep_p2p_graph_refs(int delta);  // ... that hold the addresses of the atta
 int sz_ep_generation(void);           // changes whenever the exchange set-up does
 extern "C" int sz_ep_world(void);
 extern "C" int sz_ep_p2p_world(void);
-int sz_moe_rows_live(const sz_moe_layer* L, uint64_t x, int rows, int live, uint64_t y, uint64_t scratch, int64_t scratch_bytes, uint64_t stream);   // sz_moe.cu
+int sz_moe_rows_room(const sz_moe_layer* L, int room, int64_t* bytes);
+int sz_moe_rows_clear(const sz_moe_layer* L, int room, uint64_t scratch, uint64_t stream);
+int sz_moe_rows_live(const sz_moe_layer* L, uint64_t x, int rows, int live, int room, uint64_t y, uint64_t scratch, int64_t scratch_bytes, uint64_t stream);   // sz_moe.cu
 bool sz_moe_rows_takes(const sz_moe_layer* L);
+static int sz_batch_scratch_clear(const sz_model* m, int rows_max, uint64_t scratch, uint64_t stream);
 
 struct sz_session {
     sz_model model;
@@ -457,7 +460,7 @@ extern "C" int sz_session_create(const sz_model* m, int ctx, int flags, uint64_t
     }
     s->attn_splits = L.splits; s->attn_splits2 = L.splits2;
     s->ws_rows = L.ws_rows; s->ws = b + L.rows_ws; s->ws_bytes = L.rows_ws_bytes;
-    if (s->ws_rows > 0 && (rc = sz_batch_scratch_init(&s->model, s->ws_rows, (uint64_t)s->ws, stream))) { delete s; return rc; }
+    if (s->ws_rows > 0 && (rc = sz_batch_scratch_clear(&s->model, s->ws_rows, (uint64_t)s->ws, stream))) { delete s; return rc; }
     if ((rc = sz_head_describe(m, flags, &s->head))) { delete s; return rc; }
     if (s->head.rows > 0) {
         s->head.work = (uint64_t)(b + L.head_work); s->head.work_bytes = L.head_work_bytes;
@@ -1618,7 +1621,7 @@ static int sz_batch_layout(const sz_model* m, int rows_max, SzBatchScratch* S) {
     S->partial = o; o = up256(o + 4 * S->partial_floats);
     for (int l = 0; l < c.n_layer; l++) {
         int64_t b = 0;
-        const int rc = sz_moe_rows_scratch_bytes(&m->layers[l].moe, rows_max, &b);
+        const int rc = sz_moe_rows_room(&m->layers[l].moe, rows_max, &b);
         if (rc) return rc;
         mb = b > mb ? b : mb;
     }
@@ -1626,8 +1629,14 @@ static int sz_batch_layout(const sz_model* m, int rows_max, SzBatchScratch* S) {
     S->total = o;
     return SZ_OK;
 }
+// What a caller's batch scratch may hold (a session's own, for its prompts' chunks, more: SZ_ROWS_CHUNK).
+#define SZ_BATCH_ROWS 256
+static int sz_batch_rows_check(int rows_max) {
+    return rows_max > SZ_BATCH_ROWS ? sz_fail(SZ_E_ARG, "sz_batch: rows_max = %d (a multiple of 8 up to %d)", rows_max, SZ_BATCH_ROWS) : SZ_OK;
+}
 extern "C" int sz_batch_scratch_bytes(const sz_model* m, int rows_max, int64_t* bytes) {
     SzBatchScratch S;
+    if (sz_batch_rows_check(rows_max)) return SZ_E_ARG;
     const int rc = sz_batch_layout(m, rows_max, &S);
     if (rc) return rc;
     if (!bytes) return sz_fail(SZ_E_ARG, "null bytes");
@@ -1635,13 +1644,16 @@ extern "C" int sz_batch_scratch_bytes(const sz_model* m, int rows_max, int64_t* 
     return SZ_OK;
 }
 // Once after the scratch is allocated (and after a failed step).
-extern "C" int sz_batch_scratch_init(const sz_model* m, int rows_max, uint64_t scratch, uint64_t stream) {
+static int sz_batch_scratch_clear(const sz_model* m, int rows_max, uint64_t scratch, uint64_t stream) {
     SzBatchScratch S;
     int rc = sz_batch_layout(m, rows_max, &S);
     if (rc) return rc;
     if (!scratch || (scratch & 255)) return sz_fail(SZ_E_ARG, "scratch must be 256-byte aligned");
     SZ_CUDA(cudaMemsetAsync((void*)(scratch + S.x), 0, (size_t)(S.moe - S.x), (cudaStream_t)stream));
-    return sz_moe_rows_status(&m->layers[0].moe, rows_max, scratch + S.moe, nullptr, stream);
+    return sz_moe_rows_clear(&m->layers[0].moe, rows_max, scratch + S.moe, stream);
+}
+extern "C" int sz_batch_scratch_init(const sz_model* m, int rows_max, uint64_t scratch, uint64_t stream) {
+    return sz_batch_rows_check(rows_max) ? SZ_E_ARG : sz_batch_scratch_clear(m, rows_max, scratch, stream);
 }
 
 // ---- many rows through the layers ----------------------------------------------------------------------------------------------------------
@@ -1810,7 +1822,7 @@ static int sz_rows_layers(sz_session* const* ss, int n, const int32_t* ids, cons
         float* yo[1] = {Y};
         if ((rc = dense(o, CORE, yo, "rows_out"))) return rc;
         if ((rc = sz_hc_read_rows(s0, st, L.hc_ffn, Rp, hn++, true, true, BB, true))) return rc;
-        if ((rc = sz_moe_rows_live(&L.moe, (uint64_t)X, Rp, R, (uint64_t)Y, (uint64_t)(base + S.moe), S.moe_bytes, (uint64_t)st))) return rc;
+        if ((rc = sz_moe_rows_live(&L.moe, (uint64_t)X, Rp, R, rows_max, (uint64_t)Y, (uint64_t)(base + S.moe), S.moe_bytes, (uint64_t)st))) return rc;
     }
     if (read_out && (rc = sz_hc_read_rows(s0, st, s0->model.output_hc, Rp, hn++, true, false, BB, true))) return rc;
     bool any_all = false;
@@ -2169,9 +2181,10 @@ static int sz_batch_step(sz_session* const* ss, int n, const int32_t* ids, const
     return join();
 }
 
-// Rows of a prompt's chunk a session of this model keeps room for: SZ_ROWS_CHUNK, or what its capacity holds; 0 where sz_rows_layers
+// Rows of a prompt's chunk a session of this model keeps room for: SZ_ROWS_CHUNK (the most the experts' plan holds: 507 tokens took 126.9 ms in
+// two chunks of up to 256 rows, 105.2 in one), or what its capacity holds; 0 where sz_rows_layers
 // does not run the model, or the host said that prompts come through sz_batch_prefill (SZ_SESSION_LEAN).
-#define SZ_ROWS_CHUNK 256
+#define SZ_ROWS_CHUNK 512
 static int sz_rows_ws_plan(const sz_model* m, int ctx, int flags, int* rows, int64_t* bytes) {
     const sz_model_config& c = m->cfg;
     *rows = 0; *bytes = 0;
@@ -2206,6 +2219,7 @@ static int sz_prefill_chunks(sz_session* s, const int32_t* ids, int body, uint64
 extern "C" int sz_batch_verify(sz_session* const* ss, int n, const int32_t* ids, const int32_t* ms, int accept_mode, int eog_token, int rows_max,
                                uint64_t scratch, int64_t scratch_bytes, uint64_t stream) {
     if (n < 1 || n > SZ_BATCH_MAX) return sz_fail(SZ_E_ARG, "sz_batch_verify: 1..%d sequences", SZ_BATCH_MAX);
+    if (sz_batch_rows_check(rows_max)) return SZ_E_ARG;
     int accept[SZ_BATCH_MAX], heads[SZ_BATCH_MAX];
     for (int b = 0; b < n; b++) { accept[b] = accept_mode; heads[b] = 1; }
     return sz_batch_step(ss, n, ids, ms, accept, heads, eog_token, rows_max, scratch, scratch_bytes, stream);
@@ -2218,6 +2232,7 @@ extern "C" int sz_batch_prefill(sz_session* const* ss, int n, const int32_t* con
                                 int64_t scratch_bytes, uint64_t stream) {
     if (!ss || !ids || !lens || n < 1 || n > SZ_BATCH_MAX) return sz_fail(SZ_E_ARG, "sz_batch_prefill: 1..%d sequences", SZ_BATCH_MAX);
     if (rows_max < SZ_MAX_VERIFY) return sz_fail(SZ_E_ARG, "sz_batch_prefill: a scratch for %d rows", rows_max);
+    if (sz_batch_rows_check(rows_max)) return SZ_E_ARG;
     std::vector<int> done((size_t)n, 0);
     for (int b = 0; b < n; b++)
         if (!ss[b] || !ids[b] || lens[b] < 1) return sz_fail(SZ_E_ARG, "sz_batch_prefill: sequence %d has nothing to feed", b);

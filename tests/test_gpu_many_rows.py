@@ -21,11 +21,11 @@ def dm():
     return md.DeviceModel(md.make_model(CFG, expert_type=szlib.TYPE_EXL3(3), seed=4, cycle_alpha=0.9, cycle_beta=0.5))
 
 
-# 16 rows: the fewest that go as a chunk; 128 / 136: where the reads change their form; 256 / 264: one chunk, two
-@pytest.mark.parametrize("n", [16, 17, 25, 129, 137, 145, 257, 265, 273])
+# 16 rows: the fewest that go as a chunk; 128 / 136: where the reads change their form; 512 / 520: one chunk, two
+@pytest.mark.parametrize("n", [16, 17, 25, 129, 137, 145, 265, 513, 521, 529])
 def test_a_prompt_in_chunks_equals_passes_of_eight_rows(dm, n):
     prompt = md.make_prompt(n, CFG["vocab"], seed=60 + n)
-    a, b = md.Session(dm, 320, kv_q8=True), md.Session(dm, 320, kv_q8=True)
+    a, b = md.Session(dm, 560, kv_q8=True), md.Session(dm, 560, kv_q8=True)
     a.prefill(prompt)
     for c in range(0, n, 8):
         rows = prompt[c:c + 8]
