@@ -429,9 +429,11 @@ static __global__ void __launch_bounds__(256, 2) sz_dense_q8_kernel(const SzDens
 // 8 of them.  There a warp owns an eighth of the columns and runs, block of 32 columns after block, four MMAs into a fresh accumulator and
 // one multiply-add with the block's scale into its part's running sum; the eight parts' sums are then added in order.  Here a warp runs
 // through all columns - the same chains, the parts one after the other, a part's sum added to the total when its last block is done - for
-// UPW units of 16 matrix rows and 32 rows of the step, so that nothing but the result leaves it.  A thread block's 8 warps stage the slices
+// a unit of 16 matrix rows and 32 rows of the step, so that nothing but the result leaves it.  A thread block's 8 warps stage the slices
 // of their units and of the rows (f16 high and low parts, made once by sz_dense_rows_pack_kernel) 128 columns at a time through a ring of
-// asynchronous copies; a block of 32 columns decoded into A fragments serves 4 row groups, a row group's fragments UPW units.
+// asynchronous copies; a block of 32 columns decoded into A fragments serves 4 row groups.  Two thread blocks a multiprocessor: with two
+// units a warp, which loads the rows' fragments half as often but needs 200 registers, one fitted, and its 8 warps kept the tensor pipe 40 %
+// busy (504 rows of 12,352 outputs: 251 -> 199 us; 80 rows 50.8 -> 45.0).
 // (The form before it gave a thread block one part and four or eight row groups: a fragment of the rows was loaded from shared memory for
 // every unit, and the parts' sums - 98 MB at 256 rows of 12,352 outputs - went through a scratch and a second kernel.  the four MMAs a
 // block and group alone are 44 us.)
@@ -444,11 +446,10 @@ struct SzDenseRowsCfg {
 #define SZ_DR_COLS 128      // columns a stage
 #define SZ_DR_RS 144        // bytes between the staged slices (136 and where they start)
 #define SZ_DR_XS 160        // halves between the staged rows (16 (mod 32) words: the eight rows a quarter of a warp reads at once)
-template <int UPW>
 struct SzDenseRows {
-    static constexpr int WROWS = 8 * 16 * UPW;                                   // matrix rows a thread block
+    static constexpr int WROWS = 8 * 16;                                         // matrix rows a thread block
     static constexpr int STAGE = WROWS * SZ_DR_RS + 2 * 32 * SZ_DR_XS * 2;
-    static constexpr int STAGES = UPW == 2 ? 3 : 2;                              // (one thread block a multiprocessor, or two)
+    static constexpr int STAGES = 2;
     static constexpr int SMEM = STAGES * STAGE + WROWS * 8;
 };
 
@@ -475,16 +476,15 @@ __device__ __forceinline__ void sz_q8_quad(u32 w, u32& lo, u32& hi) {
     lo = *(const u32*)&ha; hi = *(const u32*)&hb;
 }
 
-// grid (ceil(units / (8 UPW)), ceil(rows / 32)), block 256
-template <int UPW>
-static __global__ void __launch_bounds__(256, UPW == 2 ? 1 : 2) sz_dense_rows_q8_kernel(const SzDenseArgs a, const SzDenseRowsCfg c) {
-    using X = SzDenseRows<UPW>;
+// grid (ceil(units / 8), ceil(rows / 32)), block 256
+static __global__ void __launch_bounds__(256, 2) sz_dense_rows_q8_kernel(const SzDenseArgs a, const SzDenseRowsCfg c) {
+    using X = SzDenseRows;
     constexpr int S = X::STAGES;
     extern __shared__ __align__(128) u8 smem[];
     const u8** wrow = (const u8**)(smem + S * X::STAGE);       // where the thread block's matrix rows start
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, q = lane & 3;
-    const int total = c.units[a.n_jobs], u0 = blockIdx.x * 8 * UPW, j0 = blockIdx.y * 32;
+    const int total = c.units[a.n_jobs], u0 = blockIdx.x * 8, j0 = blockIdx.y * 32;
     const int ng = (c.rows - j0) / 8 < 4 ? (c.rows - j0) / 8 : 4;
     const size_t rb = (size_t)(a.cols / 32) * 34;
     const int nchunk = a.cols / SZ_DR_COLS, nblk = a.cols / 256;      // blocks a part
@@ -524,13 +524,11 @@ static __global__ void __launch_bounds__(256, UPW == 2 ? 1 : 2) sz_dense_rows_q8
     sz_pdl_wait();
     sz_pdl_trigger();
     for (int i = 0; i < S - 1; i++) { if (i < nchunk) stage_x(i); sz_cp_async_commit(); }
-    float tot[UPW][4][4], acc[UPW][4][4];
+    float tot[4][4], acc[4][4];
 #pragma unroll
-    for (int w = 0; w < UPW; w++)
+    for (int gi = 0; gi < 4; gi++)
 #pragma unroll
-        for (int gi = 0; gi < 4; gi++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) { tot[w][gi][e] = 0.f; acc[w][gi][e] = 0.f; }
+        for (int e = 0; e < 4; e++) { tot[gi][e] = 0.f; acc[gi][e] = 0.f; }
     int left = nblk;                       // blocks left of the part at hand
     for (int ci = 0; ci < nchunk; ci++) {
         sz_cp_async_wait<S - 2>();
@@ -538,77 +536,61 @@ static __global__ void __launch_bounds__(256, UPW == 2 ? 1 : 2) sz_dense_rows_q8
         if (ci + S - 1 < nchunk) { stage_w(ci + S - 1); stage_x(ci + S - 1); }
         sz_cp_async_commit();
         const u8* st = smem + (size_t)(ci % S) * X::STAGE;
-        const u8* wr = st + (size_t)(warp * 16 * UPW + g) * SZ_DR_RS + ((ci & 1) ? 8 : 0) + 8 * q;
+        const u8* wr = st + (size_t)(warp * 16 + g) * SZ_DR_RS + ((ci & 1) ? 8 : 0) + 8 * q;
         const __half* xr = (const __half*)(st + X::WROWS * SZ_DR_RS) + (size_t)g * SZ_DR_XS + 8 * q;
 #pragma unroll
         for (int b = 0; b < 4; b++) {
             // a block's 34 bytes: scale, 32 codes; the lane's 8 codes start at a multiple of 4 in odd blocks, 2 behind one in even ones
-            u32 a1[UPW][4], a2[UPW][4];
-            float d[UPW][2];
+            u32 a1[4], a2[4];
+            float d[2];
 #pragma unroll
-            for (int w = 0; w < UPW; w++)
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const u8* p = wr + (size_t)(w * 16 + 8 * h) * SZ_DR_RS + b * 34;
-                    u32 c01, c23;
-                    if (b & 1) {
-                        c01 = *(const u32*)(p + 2); c23 = *(const u32*)(p + 6);
-                    } else {
-                        const u32 w0 = *(const u32*)p, w1 = *(const u32*)(p + 4), w2 = *(const u32*)(p + 8);
-                        c01 = __funnelshift_r(w0, w1, 16); c23 = __funnelshift_r(w1, w2, 16);
-                    }
-                    d[w][h] = sz_f16_to_f32(*(const u16*)(p - 8 * q));
-                    sz_q8_quad(c01, a1[w][h], a1[w][2 + h]);
-                    sz_q8_quad(c23, a2[w][h], a2[w][2 + h]);
+            for (int h = 0; h < 2; h++) {
+                const u8* p = wr + (size_t)(8 * h) * SZ_DR_RS + b * 34;
+                u32 c01, c23;
+                if (b & 1) {
+                    c01 = *(const u32*)(p + 2); c23 = *(const u32*)(p + 6);
+                } else {
+                    const u32 w0 = *(const u32*)p, w1 = *(const u32*)(p + 4), w2 = *(const u32*)(p + 8);
+                    c01 = __funnelshift_r(w0, w1, 16); c23 = __funnelshift_r(w1, w2, 16);
                 }
+                d[h] = sz_f16_to_f32(*(const u16*)(p - 8 * q));
+                sz_q8_quad(c01, a1[h], a1[2 + h]);
+                sz_q8_quad(c23, a2[h], a2[2 + h]);
+            }
 #pragma unroll
             // (all four groups, whether the step has them or not: a branch around one would keep its MMAs - a chain of four - from running
             // between the others')
             for (int gi = 0; gi < 4; gi++) {
                 const uint4 bh = *(const uint4*)(xr + (size_t)gi * 8 * SZ_DR_XS + b * 32);
                 const uint4 bl = *(const uint4*)(xr + (size_t)(32 + gi * 8) * SZ_DR_XS + b * 32);
-                float t[UPW][4];
-#pragma unroll
-                for (int w = 0; w < UPW; w++) { t[w][0] = 0.f; t[w][1] = 0.f; t[w][2] = 0.f; t[w][3] = 0.f; }
-#pragma unroll
-                for (int w = 0; w < UPW; w++) sz_mma16816_zn(t[w], a1[w], bh.x, bh.y);
-#pragma unroll
-                for (int w = 0; w < UPW; w++) sz_mma16816_zn(t[w], a2[w], bh.z, bh.w);
-#pragma unroll
-                for (int w = 0; w < UPW; w++) sz_mma16816_zn(t[w], a1[w], bl.x, bl.y);
-#pragma unroll
-                for (int w = 0; w < UPW; w++) sz_mma16816_zn(t[w], a2[w], bl.z, bl.w);
-#pragma unroll
-                for (int w = 0; w < UPW; w++) {
-                    acc[w][gi][0] = fmaf(d[w][0], t[w][0], acc[w][gi][0]); acc[w][gi][1] = fmaf(d[w][0], t[w][1], acc[w][gi][1]);
-                    acc[w][gi][2] = fmaf(d[w][1], t[w][2], acc[w][gi][2]); acc[w][gi][3] = fmaf(d[w][1], t[w][3], acc[w][gi][3]);
-                }
+                float t[4] = {0.f, 0.f, 0.f, 0.f};
+                sz_mma16816_zn(t, a1, bh.x, bh.y);
+                sz_mma16816_zn(t, a2, bh.z, bh.w);
+                sz_mma16816_zn(t, a1, bl.x, bl.y);
+                sz_mma16816_zn(t, a2, bl.z, bl.w);
+                acc[gi][0] = fmaf(d[0], t[0], acc[gi][0]); acc[gi][1] = fmaf(d[0], t[1], acc[gi][1]);
+                acc[gi][2] = fmaf(d[1], t[2], acc[gi][2]); acc[gi][3] = fmaf(d[1], t[3], acc[gi][3]);
             }
             if (--left == 0) {             // the part's sum is complete
                 left = nblk;
 #pragma unroll
-                for (int w = 0; w < UPW; w++)
+                for (int gi = 0; gi < 4; gi++)
 #pragma unroll
-                    for (int gi = 0; gi < 4; gi++)
-#pragma unroll
-                        for (int e = 0; e < 4; e++) { tot[w][gi][e] += acc[w][gi][e]; acc[w][gi][e] = 0.f; }
+                    for (int e = 0; e < 4; e++) { tot[gi][e] += acc[gi][e]; acc[gi][e] = 0.f; }
             }
         }
     }
+    const int u = u0 + warp;
+    if (u < total) {
+        int ji, row0, nrows;
+        locate(u, ji, row0, nrows);
+        const SzDenseJob& jb = a.job[ji];
 #pragma unroll
-    for (int w = 0; w < UPW; w++) {
-        const int u = u0 + warp * UPW + w;
-        if (u < total) {
-            int ji, row0, nrows;
-            locate(u, ji, row0, nrows);
-            const SzDenseJob& jb = a.job[ji];
-#pragma unroll
-            for (int gi = 0; gi < 4; gi++) {
-                if (gi < ng) {
-                    float* o = jb.out + (size_t)(j0 + gi * 8 + 2 * q) * jb.ostride + row0 + g;
-                    if (g < nrows) { o[0] = sz_epilogue(jb.epi, tot[w][gi][0], jb.div); o[jb.ostride] = sz_epilogue(jb.epi, tot[w][gi][1], jb.div); }
-                    if (g + 8 < nrows) { o[8] = sz_epilogue(jb.epi, tot[w][gi][2], jb.div); o[jb.ostride + 8] = sz_epilogue(jb.epi, tot[w][gi][3], jb.div); }
-                }
+        for (int gi = 0; gi < 4; gi++) {
+            if (gi < ng) {
+                float* o = jb.out + (size_t)(j0 + gi * 8 + 2 * q) * jb.ostride + row0 + g;
+                if (g < nrows) { o[0] = sz_epilogue(jb.epi, tot[gi][0], jb.div); o[jb.ostride] = sz_epilogue(jb.epi, tot[gi][1], jb.div); }
+                if (g + 8 < nrows) { o[8] = sz_epilogue(jb.epi, tot[gi][2], jb.div); o[jb.ostride + 8] = sz_epilogue(jb.epi, tot[gi][3], jb.div); }
             }
         }
     }

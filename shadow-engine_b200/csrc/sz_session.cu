@@ -641,17 +641,9 @@ int sz_dense_rows_launch(SzDenseArgs& a, void* xh, cudaStream_t st, const char* 
     c.rows = a.m;
     c.xh = (const __half*)xh;
     SZ_CUDA(sz_launch("dense_rows_pack", sz_dense_rows_pack_kernel, dim3((a.cols + 1023) / 1024, a.m), dim3(256), 0, st, true, a.x, a.xstride, a.cols, a.m, (__half*)xh));
-    const int tiles = (a.m + 31) / 32, sms = sz_sm_count_session();
-    // two units a warp (a row group's fragments loaded once for both) where that still leaves a thread block for every multiprocessor
-    const bool two = (units + 15) / 16 * tiles >= sms - sms / 8;
     static bool set = false;
-    if (!set) {
-        SZ_CUDA(cudaFuncSetAttribute(sz_dense_rows_q8_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SzDenseRows<1>::SMEM));
-        SZ_CUDA(cudaFuncSetAttribute(sz_dense_rows_q8_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SzDenseRows<2>::SMEM));
-        set = true;
-    }
-    if (two) SZ_CUDA(sz_launch(name, sz_dense_rows_q8_kernel<2>, dim3((units + 15) / 16, tiles), dim3(256), SzDenseRows<2>::SMEM, st, true, a, c));
-    else SZ_CUDA(sz_launch(name, sz_dense_rows_q8_kernel<1>, dim3((units + 7) / 8, tiles), dim3(256), SzDenseRows<1>::SMEM, st, true, a, c));
+    if (!set) { SZ_CUDA(cudaFuncSetAttribute(sz_dense_rows_q8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SzDenseRows::SMEM)); set = true; }
+    SZ_CUDA(sz_launch(name, sz_dense_rows_q8_kernel, dim3((units + 7) / 8, (a.m + 31) / 32), dim3(256), SzDenseRows::SMEM, st, true, a, c));
     *taken = 1;
     return SZ_OK;
 }
