@@ -1013,7 +1013,7 @@ __device__ __forceinline__ void sz_delta_scan_body(const SzScanSeq& q, const flo
     }
     float* So = (cur ? q.O0 : q.O1) + Sat;
 #pragma unroll
-    for (int i = 0; i < 32; i++) So[(size_t)i * D] = S[i];
+    for (int i = 0; i < RW; i++) So[(size_t)i * D] = S[i];
     if (og) {
         const int c0 = (rows - 1) / SZ_SCAN_RC * SZ_SCAN_RC;
 #pragma unroll
