@@ -951,31 +951,29 @@ static int sz_attn_launch(sz_session* s, cudaStream_t st, const u8* kc, const u8
     return SZ_OK;
 }
 
-// Splits of the cache a pass of m rows takes in the grouped kernel: about one block a multiprocessor, or, where two fit (few queries:
-// small fragments), twice as many, so that each block's chain of chunks is half as long and the two blocks hide each other's barriers.
-static int sz_attn2_splits(const sz_session* s, size_t smem) {
+// Splits of the cache a pass takes in the grouped kernel (its queries in nqt tiles of 16): about one block a multiprocessor, or, where two
+// fit, twice as many, so that each block's chain of chunks is half as long and the two blocks hide each other's barriers.  (The splits are
+// part of the order in which a row's sums are made.)
+static int sz_attn2_splits(const sz_session* s, int nqt) {
     int splits = s->attn_splits2;
-    if (smem + 2048 <= 113 * 1024 && 2 * splits <= (s->ctx + 255) / 256) splits *= 2;
+    if ((s->model.cfg.head_dim < 256 || nqt == 1) && 2 * splits <= (s->ctx + 255) / 256) splits *= 2;
     return splits;
 }
 static int sz_attn2_nqt(int queries) { return queries <= 16 ? 1 : (queries <= 32 ? 2 : 4); }
-static size_t sz_attn2_smem(int hd, int nqt) {
-    return (size_t)(hd == 64 ? SzAttn2<64>::smem_bytes(nqt) : (hd == 128 ? SzAttn2<128>::smem_bytes(nqt) : SzAttn2<256>::smem_bytes(nqt)));
-}
 
 template <int HD, int NQT>
 static int sz_attn2_go(sz_session* s, cudaStream_t st, const u8* kc, const u8* vc, int m, int* splits_used, int ratio) {
     const sz_model_config& c = s->model.cfg;
     static bool set = false;
-    const size_t smem = (size_t)SzAttn2<HD>::smem_bytes(NQT);
+    const size_t smem = (size_t)SzAttn2<HD, NQT>::SMEM;
     if (!set) { SZ_CUDA(cudaFuncSetAttribute(sz_attn2_kernel<HD, NQT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); set = true; }
-    int splits = sz_attn2_splits(s, smem);
+    int splits = sz_attn2_splits(s, NQT);
     if (ratio) {   // the sparse form: a block a (kv head, split, row); a row's list holds about the budget's positions, 128 or more a split
         const int by_budget = (c.idx_budget + 127) / 128;
         if (splits > by_budget) splits = by_budget < 1 ? 1 : by_budget;
     }
     *splits_used = splits;
-    SZ_CUDA(sz_launch("attention_grouped", sz_attn2_kernel<HD, NQT>, dim3(c.n_kv_head, splits, ratio ? m : 1), dim3(256), smem, st, true, (const float*)s->a_q,
+    SZ_CUDA(sz_launch("attention_grouped", sz_attn2_kernel<HD, NQT>, dim3(c.n_kv_head, splits, ratio ? m : 1), dim3(32 * SzAttn2<HD, NQT>::NW), smem, st, true, (const float*)s->a_q,
                       kc, vc, (int)c.n_head, (int)c.n_kv_head, m, s->ctx, (const int32_t*)s->state, splits, s->a_part, (u32*)(s->state + 2),
                       (const SzTree*)(s->tree_pass ? s->ids + 32 : nullptr), (const int32_t*)(ratio ? s->i_list : nullptr), (const int32_t*)s->i_count,
                       s->i_ctx_blocks, ratio, (const SzSeqDev*)nullptr, (const SzAttnGroup*)nullptr, 0));
@@ -1665,9 +1663,9 @@ struct SzAttnBatch { int row0, rows, g0[4], ng[3], splits[3]; };   // rows that 
 template <int HD, int NQT>
 static int sz_rows_attn_go(cudaStream_t st, const sz_model_config& c, const float* aq, int splits, const SzSeqDev* seqs, const SzAttnGroup* groups, int ng, int ai, u32* err) {
     static bool set = false;
-    const size_t smem = (size_t)SzAttn2<HD>::smem_bytes(NQT);
+    const size_t smem = (size_t)SzAttn2<HD, NQT>::SMEM;
     if (!set) { SZ_CUDA(cudaFuncSetAttribute(sz_attn2_kernel<HD, NQT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); set = true; }
-    SZ_CUDA(sz_launch("rows_attention", sz_attn2_kernel<HD, NQT>, dim3(c.n_kv_head, splits, ng), dim3(256), smem, st, true, aq, (const u8*)nullptr, (const u8*)nullptr,
+    SZ_CUDA(sz_launch("rows_attention", sz_attn2_kernel<HD, NQT>, dim3(c.n_kv_head, splits, ng), dim3(32 * SzAttn2<HD, NQT>::NW), smem, st, true, aq, (const u8*)nullptr, (const u8*)nullptr,
                       (int)c.n_head, (int)c.n_kv_head, 0, 0, (const int32_t*)nullptr, 0, (float*)nullptr, err, (const SzTree*)nullptr, (const int32_t*)nullptr,
                       (const int32_t*)nullptr, 0, 0, seqs, groups, ai));
     return SZ_OK;
@@ -1742,7 +1740,7 @@ static int sz_rows_layers(sz_session* const* ss, int n, const int32_t* ids, cons
                 SzAttnGroup g = {};
                 g.seq = b; g.row0 = at + j; g.j0 = j; g.m = ms[b] - j < SZ_MAX_VERIFY ? ms[b] - j : SZ_MAX_VERIFY;
                 const int nqt = sz_attn2_nqt(G * g.m), k = nqt == 1 ? 0 : (nqt == 2 ? 1 : 2);
-                g.splits = sz_attn2_splits(ss[b], sz_attn2_smem(hd, nqt));
+                g.splits = sz_attn2_splits(ss[b], nqt);
                 const int64_t need = (int64_t)g.m * nh * g.splits * (hd + 2);
                 if (last_own == b && used + need > S.partial_floats) close(at + j);
                 if (last_own != b) { g.part = ss[b]->a_part; last_own = b; }
@@ -2174,8 +2172,9 @@ static int sz_batch_step(sz_session* const* ss, int n, const int32_t* ids, const
 }
 
 // Rows of a prompt's chunk a session of this model keeps room for: SZ_ROWS_CHUNK (the most the experts' plan holds: 507 tokens took 126.9 ms in
-// two chunks of up to 256 rows, 105.2 in one), or what its capacity holds; 0 where sz_rows_layers
-// does not run the model, or the host said that prompts come through sz_batch_prefill (SZ_SESSION_LEAN).
+// two chunks of up to 256 rows, 105.2 in one), or what its capacity holds where the room is not for a batch's prompts too
+// (SZ_SESSION_ROOM); 0 where sz_rows_layers does not run the model, or the host said that prompts come through sz_batch_prefill
+// (SZ_SESSION_LEAN).
 #define SZ_ROWS_CHUNK 512
 static int sz_rows_ws_plan(const sz_model* m, int ctx, int flags, int* rows, int64_t* bytes) {
     const sz_model_config& c = m->cfg;

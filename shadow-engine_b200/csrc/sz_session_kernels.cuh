@@ -1216,20 +1216,33 @@ sz_attn_kernel(const float* __restrict__ q, const u8* __restrict__ kc, const u8*
 // TMA engine (the cache is laid out per head, so a chunk is one contiguous copy), double-buffered.  Online softmax per query; the
 // partial (out, max, sum) of the block goes to the same merge kernel as the simple form.
 // Query vector qv = j * G + hh (row j of the pass, head hh of the group); row j attends to positions < pos0 + j + 1.
+// What bounds it is the chain scores - softmax - products of a chunk and the instructions of two warps a scheduler, not the 4 us that its
+// bytes take.  So a warp takes one tile of 16 queries and its share of a chunk's positions, with the queries' high parts in registers
+// (read from shared memory chunk after chunk by every warp, the fragments alone were 2,000 of a chunk's 6,000 cycles); a lane's four k
+// slots are four neighbouring dimensions, one word of a key; the next chunk's scores are made beside this one's products (two barriers a
+// chunk instead of four); the softmax spreads over all threads, and its sums, which only the end needs, are added up beside the products.
+// 24,576 positions, 16 heads on 2: 1 row 20.6 -> 16.5 us, 4 rows 37 -> 26.7, 8 rows 61.5 -> 41 (launched one after the other).
 #define SZ_AT_T 64
-template <int HD>
+template <int HD, int NQT>
 struct SzAttn2 {
     static constexpr int HB = HD + (((HD >> 5) * 2 + 15) & ~15);
-    static constexpr int KS = HD / 16;            // k-steps of the score contraction
-    static constexpr int DW = HD / 8;             // output dimensions of a warp
-    static constexpr int NT = DW / 8;             // its n-tiles
-    static constexpr int SST = SZ_AT_T + 2;       // row stride of the score / probability tile (floats)
-    static constexpr int STAGE = 2 * SZ_AT_T * HB;  // K chunk then V chunk
-    static int smem_bytes(int nqt) { return 64 + 2 * STAGE + nqt * KS * 32 * 16 * 2 + 64 * SST * 4 + 64 * 3 * 4; }
+    static constexpr int KS = HD / 16;              // k-steps of the score contraction
+    // 16 queries: 4 warps, two blocks a multiprocessor; the fragments of 256 dimensions take 128 registers a thread
+    static constexpr int NW = NQT == 1 ? 4 : 8;
+    static constexpr int OCC = HD == 256 && NQT > 1 ? 1 : 2;
+    static constexpr int NP = 64 * NQT / NW / 8;    // scores: tiles of 8 positions a warp
+    static constexpr int TPQ = 2 * NW / NQT;        // softmax: threads a query
+    static constexpr int PP = SZ_AT_T / TPQ;        // .. and positions a thread
+    static constexpr int DW = HD / NW;              // products: output dimensions of a warp
+    static constexpr int NT = DW / 8;               // .. its n-tiles
+    static constexpr int TG = NT < 4 ? NT : 4;      // .. n-tiles that share a scale group of the values
+    static constexpr int SST = SZ_AT_T + 8;         // row stride of the score / probability tile (floats)
+    static constexpr int STAGE = SZ_AT_T * HB;      // a chunk of K or of V
+    static constexpr int SMEM = 64 + 4 * STAGE + NQT * KS * 32 * 16 * 2 + 2 * NQT * 16 * SST * 4 + NQT * 16 * 4;
 };
 
 template <int HD, int NQT>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(32 * SzAttn2<HD, NQT>::NW, SzAttn2<HD, NQT>::OCC)
 sz_attn2_kernel(const float* __restrict__ qin, const u8* __restrict__ kc, const u8* __restrict__ vc, int nh, int nkv, int m, int ctx,
                 const int32_t* __restrict__ state, int splits, float* __restrict__ part, u32* __restrict__ err, const SzTree* __restrict__ tr,
                 const int32_t* __restrict__ glist, const int32_t* __restrict__ gcount, int gstride, int ratio, const SzSeqDev* __restrict__ seqs,
@@ -1239,18 +1252,18 @@ sz_attn2_kernel(const float* __restrict__ qin, const u8* __restrict__ kc, const 
     // glist != null: the sparse form, grid (kv heads, splits, rows).  The block serves ONE row (blockIdx.z) and walks that row's list
     // of position groups (`ratio` positions each; row j's list at glist + j * gstride, gcount[j] long) instead of the positions
     // themselves.  A chunk of 64 list positions is then 64 / ratio copies of a group each for K and for V.
-    using A = SzAttn2<HD>;
+    using A = SzAttn2<HD, NQT>;
+    constexpr int NTH = 32 * A::NW;
     extern __shared__ __align__(128) u8 smem[];
-    u64* bars = (u64*)smem;
-    u8* stage = smem + 64;
-    uint4* qhi = (uint4*)(smem + 64 + 2 * A::STAGE);
+    u64* bars = (u64*)smem;                                // K chunks in two stages, V chunks in two
+    u8* stage = smem + 64;                                 // [2] K, [2] V
+    uint4* qhi = (uint4*)(stage + 4 * A::STAGE);
     uint4* qlo = qhi + NQT * A::KS * 32;
-    float* S = (float*)(qlo + NQT * A::KS * 32);          // [64][SST]
-    float* rmax = S + 64 * A::SST;                           // running max, sum, and this chunk's rescale factor per query
-    float* rsum = rmax + 64;
-    float* ralpha = rsum + 64;
-    __shared__ int32_t cgrp[2][SZ_AT_T];     // sparse form: the groups of the chunk in each stage
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g8 = lane >> 2, q4 = lane & 3;
+    float* S = (float*)(qlo + NQT * A::KS * 32);           // [2][NQT * 16][SST]
+    float* ralpha = S + 2 * NQT * 16 * A::SST;             // this chunk's rescale factor per query
+    __shared__ int32_t qrow[16 * NQT];                     // query vector -> (row, head) of the pass
+    __shared__ int32_t cgrp[4][SZ_AT_T];                   // sparse form: the groups of the chunks under way
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g8 = lane >> 2, q4 = lane & 3;
     const int kvh = blockIdx.x, sp = blockIdx.y;
     const bool sparse = glist != nullptr;
     int j0 = 0;
@@ -1268,8 +1281,8 @@ sz_attn2_kernel(const float* __restrict__ qin, const u8* __restrict__ kc, const 
     const int jz = sparse ? (int)blockIdx.z : 0;   // sparse: the one row of this block
     if (sparse) { glist += (size_t)jz * gstride; m = 1; }
     const int G = nh / nkv, QV = G * m;
-    // The committed length belongs to the previous pass, and so does every cache position below it: the block's first chunk is
-    // requested ahead of the dependency wait when it lies wholly there (the rows of this pass are written by the kernel before).
+    // The committed length belongs to the previous pass, and so does every cache position below it: the block's first chunks are
+    // requested ahead of the dependency wait where they lie wholly there (the rows of this pass are written by the kernel before).
     int pos0;
     asm volatile("ld.global.s32 %0, [%1];" : "=r"(pos0) : "l"(state));
     const int committed = pos0;
@@ -1282,204 +1295,218 @@ sz_attn2_kernel(const float* __restrict__ qin, const u8* __restrict__ kc, const 
     const int nchunk = t1 > t0 ? (t1 - t0 + SZ_AT_T - 1) / SZ_AT_T : 0;
     const u8* kbase = kc + (size_t)kvh * ctx * A::HB;
     const u8* vbase = vc + (size_t)kvh * ctx * A::HB;
-    const bool early = !sparse && nchunk > 0 && t0 + SZ_AT_T <= committed;
-    if (threadIdx.x == 0) {
-        sz_mbar_init(&bars[0], 1);
-        sz_mbar_init(&bars[1], 1);
-        sz_mbar_fence_init();
-        if (early) {
-            const u32 bytes = (u32)(SZ_AT_T * A::HB);
-            sz_mbar_expect_tx(&bars[0], 2 * bytes);
-            sz_bulk_g2s(stage, kbase + (size_t)t0 * A::HB, bytes, &bars[0]);
-            sz_bulk_g2s(stage + SZ_AT_T * A::HB, vbase + (size_t)t0 * A::HB, bytes, &bars[0]);
+    // warp 0: chunk ci (if there is one) of K (which = 0) or V (1) into its stage ci & 1
+    auto issue = [&](int which, int ci) {
+        if (ci >= nchunk) return;
+        const int t = t0 + ci * SZ_AT_T, np = min(SZ_AT_T, t1 - t);
+        u64* bar = &bars[2 * which + (ci & 1)];
+        u8* dst = stage + (size_t)(2 * which + (ci & 1)) * A::STAGE;
+        const u8* base = which ? vbase : kbase;
+        if (lane == 0) sz_mbar_expect_tx(bar, (u32)(np * A::HB));
+        if (!sparse) {
+            if (lane == 0) sz_bulk_g2s(dst, base + (size_t)t * A::HB, (u32)(np * A::HB), bar);
+            return;
         }
+        __syncwarp();
+        for (int i = lane; i < np / ratio; i += 32) {      // lane i copies group i (list positions come in whole groups) and notes it for the masks
+            const int gi = __ldcg(glist + t / ratio + i);
+            if (!which) cgrp[ci & 3][i] = gi;
+            const u32 bytes = (u32)ratio * A::HB;
+            sz_bulk_g2s(dst + (size_t)i * bytes, base + (size_t)gi * bytes, bytes, bar);
+        }
+    };
+    if (tid < 16 * NQT) qrow[tid] = tid < QV ? (jz + tid / G) * nh + kvh * G + tid % G : -1;
+    int early = 0;
+    if (!sparse)
+        while (early < 2 && early < nchunk && t0 + (early + 1) * SZ_AT_T <= committed) early++;
+    if (warp == 0) {
+        if (lane == 0) {
+            for (int i = 0; i < 4; i++) sz_mbar_init(&bars[i], 1);
+            sz_mbar_fence_init();
+        }
+        __syncwarp();
+        for (int ci = 0; ci < early; ci++) { issue(0, ci); issue(1, ci); }
     }
     sz_pdl_wait();
     sz_pdl_trigger();
-    // the queries as A fragments (f16 high and low parts), scaled by 1 / sqrt(HD)
+    if (warp == 0)
+        for (int ci = early; ci < 2; ci++) { issue(0, ci); issue(1, ci); }
+    // the queries as A fragments (f16 high and low parts), scaled by 1 / sqrt(HD): made once by the block, then the warp's tile in registers.
+    // A lane's four k slots of a k-step (2 q, 2 q + 1, 2 q + 8, 2 q + 9) are the four dimensions 4 q .., here and in the keys: one word.
     const float scale = rsqrtf((float)HD);
-    for (int e = threadIdx.x; e < NQT * A::KS * 32; e += 256) {
-        const int ln = e & 31, ks = (e >> 5) % A::KS, qt = e / (32 * A::KS);
-        const int gg = ln >> 2, qq = ln & 3;
-        u32 hi[4], lo[4];
-#pragma unroll
-        for (int r = 0; r < 4; r++) {
-            const int qv = qt * 16 + gg + 8 * (r & 1);
-            const int dim = ks * 16 + 2 * qq + 8 * (r >> 1);
-            float v0 = 0.f, v1 = 0.f;
-            if (qv < QV) {
-                const int j = jz + qv / G, h = kvh * G + qv % G;
-                const float* src = qin + ((size_t)j * nh + h) * HD + dim;
-                v0 = src[0] * scale; v1 = src[1] * scale;
-            }
-            const __half h0 = __float2half_rn(v0), h1 = __float2half_rn(v1);
-            const __half l0 = __float2half_rn(v0 - __half2float(h0)), l1 = __float2half_rn(v1 - __half2float(h1));
-            hi[r] = (u32)__half_as_ushort(h0) | ((u32)__half_as_ushort(h1) << 16);
-            lo[r] = (u32)__half_as_ushort(l0) | ((u32)__half_as_ushort(l1) << 16);
-        }
-        qhi[e] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-        qlo[e] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-    }
-    if (threadIdx.x < 64) { rmax[threadIdx.x] = -INFINITY; rsum[threadIdx.x] = 0.f; }
-    auto issue = [&](int ci) {  // thread 0: chunk ci of this block into stage ci & 1
-        const int t = t0 + ci * SZ_AT_T;
-        const u32 bytes = (u32)(min(SZ_AT_T, t1 - t) * A::HB);
-        u64* bar = &bars[ci & 1];
-        u8* dst = stage + (size_t)(ci & 1) * A::STAGE;
-        sz_mbar_expect_tx(bar, 2 * bytes);
-        sz_bulk_g2s(dst, kbase + (size_t)t * A::HB, bytes, bar);
-        sz_bulk_g2s(dst + SZ_AT_T * A::HB, vbase + (size_t)t * A::HB, bytes, bar);
-    };
-    auto issue_sparse = [&](int ci) {  // warp 0: lane i copies group i of chunk ci (K and V) and notes the group for the masks
-        const int t = t0 + ci * SZ_AT_T;
-        const int np = min(SZ_AT_T, t1 - t), ng = np / ratio;        // list positions come in whole groups
-        u64* bar = &bars[ci & 1];
-        u8* dst = stage + (size_t)(ci & 1) * A::STAGE;
-        if (lane == 0) sz_mbar_expect_tx(bar, 2u * (u32)np * A::HB);
-        __syncwarp();
-        for (int i = lane; i < ng; i += 32) {
-            const int gi = __ldcg(glist + t / ratio + i);
-            cgrp[ci & 1][i] = gi;
-            const u32 bytes = (u32)ratio * A::HB;
-            sz_bulk_g2s(dst + (size_t)i * bytes, kbase + (size_t)gi * bytes, bytes, bar);
-            sz_bulk_g2s(dst + SZ_AT_T * A::HB + (size_t)i * bytes, vbase + (size_t)gi * bytes, bytes, bar);
-        }
-    };
-    if (sparse) { if (warp == 0 && nchunk > 0) issue_sparse(0); }
-    else if (threadIdx.x == 0 && nchunk > 0 && !early) issue(0);
     __syncthreads();
+    {
+        constexpr int EN = (NQT * A::KS * 32 + NTH - 1) / NTH;
+        float4 v[EN][2];      // (every value a thread needs is requested before the first is used)
+#pragma unroll
+        for (int i = 0; i < EN; i++) {
+            const int e = tid + NTH * i, ln = e & 31, ks = (e >> 5) % A::KS, qt = e / (32 * A::KS);
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                const int qr = e < NQT * A::KS * 32 ? qrow[qt * 16 + (ln >> 2) + 8 * r] : -1;
+                v[i][r] = qr >= 0 ? *(const float4*)(qin + (size_t)qr * HD + ks * 16 + 4 * (ln & 3)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < EN; i++) {
+            const int e = tid + NTH * i;
+            u32 hi[4], lo[4];
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                const float4 f = v[i][r & 1];
+                const float v0 = (r < 2 ? f.x : f.z) * scale, v1 = (r < 2 ? f.y : f.w) * scale;
+                const __half2 h = __floats2half2_rn(v0, v1), l = __floats2half2_rn(v0 - __low2float(h), v1 - __high2float(h));
+                hi[r] = *(const u32*)&h; lo[r] = *(const u32*)&l;
+            }
+            if (e < NQT * A::KS * 32) { qhi[e] = make_uint4(hi[0], hi[1], hi[2], hi[3]); qlo[e] = make_uint4(lo[0], lo[1], lo[2], lo[3]); }
+        }
+    }
+    __syncthreads();
+    const int qt = warp % NQT, pw = warp / NQT * 8 * A::NP;     // scores: the warp's query tile and first position
+    u32 qh[A::KS][4];
+#pragma unroll
+    for (int ks = 0; ks < A::KS; ks++) {
+        const uint4 h = qhi[(qt * A::KS + ks) * 32 + lane];
+        qh[ks][0] = h.x; qh[ks][1] = h.y; qh[ks][2] = h.z; qh[ks][3] = h.w;
+    }
+    // ---- scores of chunk ci into S[ci & 1]: the warp's queries and positions
+    auto scores = [&](int ci) {
+        const u8* kch = stage + (size_t)(ci & 1) * A::STAGE;
+        float* Sc = S + (size_t)(ci & 1) * NQT * 16 * A::SST;
+        constexpr int NB = A::NP < 4 ? A::NP : 4, GS = NB < 4 ? 2 : 1;     // position tiles and scale groups at once: four chains of MMAs
+#pragma unroll 1
+        for (int n0 = 0; n0 < A::NP; n0 += NB) {
+            float sacc[NB][4];
+#pragma unroll
+            for (int n = 0; n < NB; n++) { sacc[n][0] = 0.f; sacc[n][1] = 0.f; sacc[n][2] = 0.f; sacc[n][3] = 0.f; }
+            const u8* krow = kch + (size_t)(pw + 8 * n0 + g8) * A::HB + 4 * q4;          // the position this lane feeds as B
+            const u8* ksc = kch + (size_t)(pw + 8 * n0 + 2 * q4) * A::HB + HD;           // scales of the positions of its C columns
+#pragma unroll
+            for (int g0 = 0; g0 < HD / 32; g0 += GS) {
+                float t[GS][NB][4];
+#pragma unroll
+                for (int g = 0; g < GS; g++)
+#pragma unroll
+                    for (int n = 0; n < NB; n++) { t[g][n][0] = 0.f; t[g][n][1] = 0.f; t[g][n][2] = 0.f; t[g][n][3] = 0.f; }
+#pragma unroll
+                for (int kk = 0; kk < 2; kk++) {
+                    u32 b0[GS][NB], b1[GS][NB];
+                    uint4 l[GS];
+#pragma unroll
+                    for (int g = 0; g < GS; g++) {
+                        const int ks = (g0 + g) * 2 + kk;
+                        l[g] = qlo[(qt * A::KS + ks) * 32 + lane];
+#pragma unroll
+                        for (int n = 0; n < NB; n++) sz_q8_quad(*(const u32*)(krow + (size_t)n * 8 * A::HB + ks * 16), b0[g][n], b1[g][n]);
+                    }
+#pragma unroll
+                    for (int g = 0; g < GS; g++)
+#pragma unroll
+                        for (int n = 0; n < NB; n++) sz_mma16816_zn(t[g][n], qh[(g0 + g) * 2 + kk], b0[g][n], b1[g][n]);
+#pragma unroll
+                    for (int g = 0; g < GS; g++)
+#pragma unroll
+                        for (int n = 0; n < NB; n++) sz_mma16816_zn(t[g][n], (const u32*)&l[g], b0[g][n], b1[g][n]);
+                }
+#pragma unroll
+                for (int g = 0; g < GS; g++)
+#pragma unroll
+                    for (int n = 0; n < NB; n++) {
+                        const float s0 = sz_f16_to_f32(*(const u16*)(ksc + (size_t)n * 8 * A::HB + 2 * (g0 + g)));
+                        const float s1 = sz_f16_to_f32(*(const u16*)(ksc + (size_t)(n * 8 + 1) * A::HB + 2 * (g0 + g)));
+                        sacc[n][0] = fmaf(s0, t[g][n][0], sacc[n][0]); sacc[n][1] = fmaf(s1, t[g][n][1], sacc[n][1]);
+                        sacc[n][2] = fmaf(s0, t[g][n][2], sacc[n][2]); sacc[n][3] = fmaf(s1, t[g][n][3], sacc[n][3]);
+                    }
+            }
+#pragma unroll
+            for (int n = 0; n < NB; n++) {
+                float* r0 = Sc + (size_t)(qt * 16 + g8) * A::SST + pw + 8 * (n0 + n) + 2 * q4;
+                *(float2*)r0 = make_float2(sacc[n][0], sacc[n][1]);
+                *(float2*)(r0 + 8 * A::SST) = make_float2(sacc[n][2], sacc[n][3]);
+            }
+        }
+    };
+    // ---- softmax: TPQ threads a query, PP positions each; the query of a thread stays the same
+    const int sq = tid / A::TPQ, sub = tid % A::TPQ, sjr = sq / G;
+    const u32 smask = sq < QV ? (tr ? tr->mask[sjr] : (2u << sjr) - 1u) : 0u;
+    float mo = -INFINITY;                                       // the query's maximum so far
+    auto softmax = [&](int ci) {
+        // positions of the chunk this query may see: every committed one, and among the pass's own rows those of its mask
+        // (a chain: rows 0 .. j; a tree: its ancestors and itself).  vis: bit i = position sub * PP + i of the chunk.
+        const int tbase = t0 + ci * SZ_AT_T, c0 = tbase + sub * A::PP;
+        u32 vis = 0;
+        if (sq < QV && sparse) {
+            // position i of this thread: list position c0 + i, in group cgrp[(c0 - tbase + i) / ratio]; the row sees it up to its own
+            // position (the last group of a list may reach past it)
+            for (int i = 0; i < A::PP; i++) {
+                const int cl = sub * A::PP + i;
+                if (c0 + i >= t1) break;
+                const int ap = cgrp[ci & 3][cl / ratio] * ratio + cl % ratio;
+                vis |= ap <= pos0 + jz ? 1u << i : 0u;
+            }
+        } else if (sq < QV) {
+            constexpr u32 ALL = (1u << A::PP) - 1u;
+            const int ncom = min(max(min(pos0, t1) - c0, 0), A::PP);   // committed positions among them
+            vis = (1u << ncom) - 1u;
+            const int sh = c0 - pos0;                         // the pass's row that position c0 is, when >= 0
+            const u32 own = sh >= 0 ? (sh < 32 ? smask >> sh : 0u) : (sh > -32 ? smask << (-sh) : 0u);
+            vis |= own & ALL;
+            const int room = t1 - c0;                          // positions past the block's range are not there
+            vis &= room >= A::PP ? ALL : (room > 0 ? (1u << room) - 1u : 0u);
+        }
+        float* row = S + ((size_t)(ci & 1) * NQT * 16 + sq) * A::SST + sub * A::PP;
+        float p[A::PP], mx = -INFINITY;
+#pragma unroll
+        for (int i = 0; i < A::PP; i += 4) { const float4 f = *(const float4*)(row + i); p[i] = f.x; p[i + 1] = f.y; p[i + 2] = f.z; p[i + 3] = f.w; }
+#pragma unroll
+        for (int i = 0; i < A::PP; i++) { p[i] = ((vis >> i) & 1u) ? p[i] : -INFINITY; mx = fmaxf(mx, p[i]); }
+#pragma unroll
+        for (int o = 1; o < A::TPQ; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        const float mn = fmaxf(mo, mx);
+#pragma unroll
+        for (int i = 0; i < A::PP; i++) p[i] = ((vis >> i) & 1u) ? __expf(p[i] - mn) : 0.f;
+#pragma unroll
+        for (int i = 0; i < A::PP; i += 4) *(float4*)(row + i) = make_float4(p[i], p[i + 1], p[i + 2], p[i + 3]);
+        if (sub == 0) ralpha[sq] = mn == -INFINITY ? 1.f : __expf(mo - mn);
+        mo = mn;
+    };
+    // ---- out += P V: the warp's dimensions; column n = g8 of n-tile b is dimension d0 + 8 TG (b / TG) + TG g8 + b % TG, so that a lane's bytes
+    // of a position are one word (or half of one) for TG tiles
     float o[NQT][A::NT][4];
 #pragma unroll
     for (int a = 0; a < NQT; a++)
 #pragma unroll
         for (int b = 0; b < A::NT; b++) { o[a][b][0] = 0.f; o[a][b][1] = 0.f; o[a][b][2] = 0.f; o[a][b][3] = 0.f; }
-    int failed = 0;
-    for (int ci = 0; ci < nchunk; ci++) {
-        if (sparse) { if (warp == 0 && ci + 1 < nchunk) issue_sparse(ci + 1); }
-        else if (threadIdx.x == 0 && ci + 1 < nchunk) issue(ci + 1);
-        if (!sz_mbar_wait(&bars[ci & 1], (ci >> 1) & 1)) failed = 1;
-        if (__syncthreads_or(failed)) { failed = 1; break; }
-        const u8* kch = stage + (size_t)(ci & 1) * A::STAGE;
-        const u8* vch = kch + SZ_AT_T * A::HB;
-        const int tbase = t0 + ci * SZ_AT_T;
-        // ---- scores of the chunk: warp w takes positions 8 w .. 8 w + 7
-        {
-            float sacc[NQT][4];
+    const int d0 = warp * A::DW;
+    float rsum = 0.f;                                           // four threads a query: its sum so far
+    auto products = [&](int ci) {
+        const u8* vch = stage + (size_t)(2 + (ci & 1)) * A::STAGE;
+        const float* Sc = S + (size_t)(ci & 1) * NQT * 16 * A::SST;
 #pragma unroll
-            for (int a = 0; a < NQT; a++) { sacc[a][0] = 0.f; sacc[a][1] = 0.f; sacc[a][2] = 0.f; sacc[a][3] = 0.f; }
-            const u8* krow = kch + (size_t)(8 * warp + g8) * A::HB;                 // the position this lane feeds as B
-            const u16* ksc0 = (const u16*)(kch + (size_t)(8 * warp + 2 * q4) * A::HB + HD);  // scales of the positions of its C columns
-            const u16* ksc1 = (const u16*)(kch + (size_t)(8 * warp + 2 * q4 + 1) * A::HB + HD);
-#pragma unroll 2
-            for (int grp = 0; grp < HD / 32; grp++) {
-                float t[NQT][4];
+        for (int a = 0; a < NQT; a++) {
+            const float al0 = ralpha[a * 16 + g8], al1 = ralpha[a * 16 + g8 + 8];
 #pragma unroll
-                for (int a = 0; a < NQT; a++) { t[a][0] = 0.f; t[a][1] = 0.f; t[a][2] = 0.f; t[a][3] = 0.f; }
-#pragma unroll
-                for (int kk = 0; kk < 2; kk++) {
-                    const int ks = grp * 2 + kk;
-                    const u32 b0 = sz_q8_pair(*(const u16*)(krow + ks * 16 + 2 * q4));
-                    const u32 b1 = sz_q8_pair(*(const u16*)(krow + ks * 16 + 8 + 2 * q4));
-#pragma unroll
-                    for (int a = 0; a < NQT; a++) {
-                        const uint4 ah = qhi[(a * A::KS + ks) * 32 + lane], al = qlo[(a * A::KS + ks) * 32 + lane];
-                        sz_mma16816_z(t[a], (const u32*)&ah, b0, b1);
-                        sz_mma16816_z(t[a], (const u32*)&al, b0, b1);
-                    }
-                }
-                const float s0 = sz_f16_to_f32(ksc0[grp]), s1 = sz_f16_to_f32(ksc1[grp]);
-#pragma unroll
-                for (int a = 0; a < NQT; a++) {
-                    sacc[a][0] = fmaf(s0, t[a][0], sacc[a][0]); sacc[a][1] = fmaf(s1, t[a][1], sacc[a][1]);
-                    sacc[a][2] = fmaf(s0, t[a][2], sacc[a][2]); sacc[a][3] = fmaf(s1, t[a][3], sacc[a][3]);
-                }
-            }
-#pragma unroll
-            for (int a = 0; a < NQT; a++) {
-                float* r0 = S + (size_t)(a * 16 + g8) * A::SST + 8 * warp + 2 * q4;
-                float* r1 = S + (size_t)(a * 16 + g8 + 8) * A::SST + 8 * warp + 2 * q4;
-                r0[0] = sacc[a][0]; r0[1] = sacc[a][1]; r1[0] = sacc[a][2]; r1[1] = sacc[a][3];
-            }
+            for (int b = 0; b < A::NT; b++) { o[a][b][0] *= al0; o[a][b][1] *= al0; o[a][b][2] *= al1; o[a][b][3] *= al1; }
         }
-        __syncthreads();
-        // ---- online softmax: four threads a query, 16 positions each
-        {
-            const int qv = threadIdx.x >> 2, sub = threadIdx.x & 3;
-            if (qv < NQT * 16) {
-                // positions of the chunk this query may see: every committed one, and among the pass's own rows those of its mask
-                // (a chain: rows 0 .. j; a tree: its ancestors and itself).  vis: bit i = position sub * 16 + i of the chunk.
-                u32 vis = 0;
-                if (qv < QV && sparse) {
-                    // position i of this thread's 16: list position c0 + i, in group cgrp[(c0 - tbase + i) / ratio]; the row sees it
-                    // up to its own position (the last group of a list may reach past it)
-                    const int c0 = tbase + sub * 16;
-                    for (int i = 0; i < 16; i++) {
-                        const int cl = sub * 16 + i;
-                        if (c0 + i >= t1) break;
-                        const int ap = cgrp[ci & 1][cl / ratio] * ratio + cl % ratio;
-                        vis |= ap <= pos0 + jz ? 1u << i : 0u;
-                    }
-                } else if (qv < QV) {
-                    const int jr = qv / G;
-                    const u32 mk = tr ? tr->mask[jr] : (2u << jr) - 1u;
-                    const int c0 = tbase + sub * 16;                  // first position of this thread's 16
-                    const int ncom = min(max(min(pos0, t1) - c0, 0), 16);   // committed positions among them
-                    vis = ncom >= 16 ? 0xffffu : ((1u << ncom) - 1u);
-                    const int sh = c0 - pos0;                         // the pass's row that position c0 is, when >= 0
-                    const u32 own = sh >= 0 ? (sh < 32 ? mk >> sh : 0u) : (sh > -32 ? mk << (-sh) : 0u);
-                    vis |= own & 0xffffu;
-                    const int room = t1 - c0;                          // positions past the block's range are not there
-                    vis &= room >= 16 ? 0xffffu : (room > 0 ? (1u << room) - 1u : 0u);
-                }
-                float* row = S + (size_t)qv * A::SST + sub * 16;
-                float mx = -INFINITY;
 #pragma unroll
-                for (int i = 0; i < 16; i++) if ((vis >> i) & 1u) mx = fmaxf(mx, row[i]);
-                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-                const float mo = rmax[qv];
-                const float mn = fmaxf(mo, mx);
-                float sum = 0.f;
+        for (int kk = 0; kk < SZ_AT_T / 16; kk++) {
+            const int p0 = kk * 16 + 2 * q4;                    // positions p0, p0 + 1, p0 + 8, p0 + 9 are this lane's k slots
 #pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    const float p = ((vis >> i) & 1u) ? __expf(row[i] - mn) : 0.f;
-                    row[i] = p;
-                    sum += p;
-                }
-                sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-                sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-                if (sub == 0) {
-                    const float al = mn == -INFINITY ? 1.f : __expf(mo - mn);
-                    ralpha[qv] = al;
-                    rsum[qv] = rsum[qv] * al + sum;
-                    rmax[qv] = mn;
-                }
-            }
-        }
-        __syncthreads();
-        // ---- out += P V: warp w takes dimensions w DW .. w DW + DW - 1, whose values share one scale group
-        {
-            const int d0 = warp * A::DW, vgrp = d0 >> 5;
-#pragma unroll
-            for (int a = 0; a < NQT; a++) {
-                const float al0 = ralpha[a * 16 + g8], al1 = ralpha[a * 16 + g8 + 8];
-#pragma unroll
-                for (int b = 0; b < A::NT; b++) { o[a][b][0] *= al0; o[a][b][1] *= al0; o[a][b][2] *= al1; o[a][b][3] *= al1; }
-            }
-#pragma unroll
-            for (int kk = 0; kk < SZ_AT_T / 16; kk++) {
-                const int p0 = kk * 16 + 2 * q4;  // positions p0, p0 + 1, p0 + 8, p0 + 9 are this lane's k slots
+            for (int tg = 0; tg < A::NT / A::TG; tg++) {
+                const int dg = d0 + 8 * A::TG * tg, vgrp = dg >> 5;
                 float vs[4];
+                u32 v4[4], bf[A::TG][2];
 #pragma unroll
-                for (int r = 0; r < 4; r++) vs[r] = sz_f16_to_f32(*(const u16*)(vch + (size_t)(p0 + (r & 1) + 8 * (r >> 1)) * A::HB + HD + 2 * vgrp));
-                u32 bf[A::NT][2];
+                for (int r = 0; r < 4; r++) {
+                    const u8* vrow = vch + (size_t)(p0 + (r & 1) + 8 * (r >> 1)) * A::HB;
+                    vs[r] = sz_f16_to_f32(*(const u16*)(vrow + HD + 2 * vgrp));
+                    const u8* vp = vrow + dg + A::TG * g8;
+                    v4[r] = A::TG == 4 ? *(const u32*)vp : (A::TG == 2 ? (u32)*(const u16*)vp : (u32)*vp);
+                }
 #pragma unroll
-                for (int b = 0; b < A::NT; b++) {
-                    const int dim = d0 + 8 * b + g8;
-                    const u32 v00 = vch[(size_t)p0 * A::HB + dim], v01 = vch[(size_t)(p0 + 1) * A::HB + dim];
-                    const u32 v10 = vch[(size_t)(p0 + 8) * A::HB + dim], v11 = vch[(size_t)(p0 + 9) * A::HB + dim];
-                    bf[b][0] = sz_q8_pair(v00 | (v01 << 8));
-                    bf[b][1] = sz_q8_pair(v10 | (v11 << 8));
+                for (int b = 0; b < A::TG; b++) {
+                    bf[b][0] = sz_q8_pair(__byte_perm(v4[0], v4[1], b | ((4 + b) << 4) | 0x4400) & 0xffffu);
+                    bf[b][1] = sz_q8_pair(__byte_perm(v4[2], v4[3], b | ((4 + b) << 4) | 0x4400) & 0xffffu);
                 }
 #pragma unroll
                 for (int a = 0; a < NQT; a++) {
@@ -1487,19 +1514,42 @@ sz_attn2_kernel(const float* __restrict__ qin, const u8* __restrict__ kc, const 
 #pragma unroll
                     for (int r = 0; r < 4; r++) {
                         // a0: (query g, k p0..), a1: (query g + 8, k p0..), a2: (query g, k p0 + 8..), a3: (query g + 8, k p0 + 8..)
-                        const float* pr = S + (size_t)(a * 16 + g8 + 8 * (r & 1)) * A::SST + p0 + 8 * (r >> 1);
-                        const float pa = pr[0], pb = pr[1];
-                        const float wa = pa > 0.f ? pa * vs[2 * (r >> 1)] : 0.f, wb = pb > 0.f ? pb * vs[2 * (r >> 1) + 1] : 0.f;
-                        af[r] = (u32)__half_as_ushort(__float2half_rn(wa)) | ((u32)__half_as_ushort(__float2half_rn(wb)) << 16);
+                        const float2 pr = *(const float2*)(Sc + (size_t)(a * 16 + g8 + 8 * (r & 1)) * A::SST + p0 + 8 * (r >> 1));
+                        const float wa = pr.x > 0.f ? pr.x * vs[2 * (r >> 1)] : 0.f, wb = pr.y > 0.f ? pr.y * vs[2 * (r >> 1) + 1] : 0.f;
+                        const __half2 w2 = __floats2half2_rn(wa, wb);
+                        af[r] = *(const u32*)&w2;
                     }
 #pragma unroll
-                    for (int b = 0; b < A::NT; b++) sz_mma16816_z(o[a][b], af, bf[b][0], bf[b][1]);
+                    for (int b = 0; b < A::TG; b++) sz_mma16816_zn(o[a][tg * A::TG + b], af, bf[b][0], bf[b][1]);
                 }
             }
         }
+        if (tid < 64 * NQT) {                                   // the chunk's sum of a query: 16 positions a thread in order, then the four of it
+            const float* row = Sc + (size_t)(tid >> 2) * A::SST + (tid & 3) * 16;
+            float sum = 0.f;
+#pragma unroll
+            for (int i = 0; i < 16; i += 4) { const float4 f = *(const float4*)(row + i); sum += f.x; sum += f.y; sum += f.z; sum += f.w; }
+            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+            rsum = rsum * ralpha[tid >> 2] + sum;
+        }
+    };
+    int failed = 0;
+    for (int ci = -1; ci < nchunk && !failed; ci++) {           // (one copy of each body: a chunk runs through little more than them, once)
+        if (ci >= 0) softmax(ci);
         __syncthreads();
+        if (ci + 1 < nchunk) {
+            if (!__all_sync(0xffffffffu, sz_mbar_wait(&bars[(ci + 1) & 1], ((ci + 1) >> 1) & 1))) failed = 1;
+            else scores(ci + 1);
+        }
+        if (ci >= 0) {
+            if (!__all_sync(0xffffffffu, sz_mbar_wait(&bars[2 + (ci & 1)], (ci >> 1) & 1))) failed = 1;
+            else products(ci);
+        }
+        failed = __syncthreads_or(failed);
+        if (warp == 0 && !failed) { issue(0, ci + 3); if (ci >= 0) issue(1, ci + 2); }
     }
-    if (failed) { if (threadIdx.x == 0) atomicExch(err, 2u); return; }
+    if (failed) { if (tid == 0) atomicExch(err, 2u); return; }
     // ---- the block's partial result, in the merge kernel's layout: [row][head][split][HD + 2]
 #pragma unroll
     for (int a = 0; a < NQT; a++)
@@ -1507,22 +1557,20 @@ sz_attn2_kernel(const float* __restrict__ qin, const u8* __restrict__ kc, const 
         for (int r = 0; r < 2; r++) {
             const int qv = a * 16 + g8 + 8 * r;
             if (qv < QV) {
-                const int j = jz + qv / G, h = kvh * G + qv % G;
-                float* out = part + (((size_t)j * nh + h) * splits + sp) * (HD + 2);
+                float* out = part + ((size_t)qrow[qv] * splits + sp) * (HD + 2) + d0;      // (rows are 8-byte aligned)
 #pragma unroll
-                for (int b = 0; b < A::NT; b++) {
-                    const int dim = warp * A::DW + 8 * b + 2 * q4;
-                    out[dim] = o[a][b][2 * r];
-                    out[dim + 1] = o[a][b][2 * r + 1];
+                for (int tg = 0; tg < A::NT / A::TG; tg++) {
+                    float f[2 * A::TG];                          // the lane's 2 TG consecutive dimensions
+#pragma unroll
+                    for (int b = 0; b < A::TG; b++) { f[b] = o[a][tg * A::TG + b][2 * r]; f[A::TG + b] = o[a][tg * A::TG + b][2 * r + 1]; }
+#pragma unroll
+                    for (int e = 0; e < 2 * A::TG; e += 2) *(float2*)(out + 8 * A::TG * tg + 2 * A::TG * q4 + e) = make_float2(f[e], f[e + 1]);
                 }
             }
         }
-    if (threadIdx.x < QV) {
-        const int qv = threadIdx.x, j = jz + qv / G, h = kvh * G + qv % G;
-        float* out = part + (((size_t)j * nh + h) * splits + sp) * (HD + 2);
-        out[HD] = rmax[qv];
-        out[HD + 1] = rsum[qv];
-    }
+    auto place = [&](int qv) { return part + ((size_t)qrow[qv] * splits + sp) * (HD + 2) + HD; };
+    if (sub == 0 && sq < QV) place(sq)[0] = mo;
+    if (tid < 64 * NQT && (tid & 3) == 0 && (tid >> 2) < QV) place(tid >> 2)[1] = rsum;
 }
 
 // merge the splits and gate: o = (acc / z) * sigmoid(gate).  grid (nh, m), block 256.  The splits' (max, sum) pairs are read by one
