@@ -258,6 +258,8 @@ int sz_mma_cols_status(uint64_t scratch, int init, int* code, uint64_t stream);
                              * flag an EXL3 output.weight is evaluated in full.  Blocks kept a row: 128, or the environment's SZ_HEAD_KBLK */
 #define SZ_SESSION_LEAN 4   /* the session keeps no room for the chunks of a prompt (up to 512 rows through a layer at once: some 400 MB at
                              * the benchmark's shapes): its prompts come through sz_batch_prefill, with the batch's scratch, or in passes of 8 */
+#define SZ_SESSION_ROOM 8   /* the session's room for chunks is the full one whatever its capacity: sz_batch_prefill uses it for the prompts of
+                             * all sequences when one of them has it */
 #define SZ_ACCEPT_NONE 0    /* the caller decides: read the top-64 of every row, then sz_session_commit(keep) */
 #define SZ_ACCEPT_GREEDY 1  /* on the device: keep row i + 1 while row i's best token is the drafted ids[i + 1] (engine.rs:2377-2408) */
 #define SZ_ACCEPT_ALL 2     /* prompt rows: all kept */

@@ -2182,7 +2182,7 @@ static int sz_rows_ws_plan(const sz_model* m, int ctx, int flags, int* rows, int
     if ((flags & SZ_SESSION_LEAN) || !(flags & SZ_KV_Q8) || m->ple.ngram >= 2 || c.idx_heads > 0 || c.n_head / c.n_kv_head * SZ_MAX_VERIFY > 64) return SZ_OK;
     for (int l = 0; l < c.n_layer; l++)
         if (!sz_moe_rows_takes(&m->layers[l].moe)) return SZ_OK;
-    const int want = ctx < SZ_ROWS_CHUNK ? ctx / SZ_MAX_VERIFY * SZ_MAX_VERIFY : SZ_ROWS_CHUNK;
+    const int want = ctx < SZ_ROWS_CHUNK && !(flags & SZ_SESSION_ROOM) ? ctx / SZ_MAX_VERIFY * SZ_MAX_VERIFY : SZ_ROWS_CHUNK;
     if (want < 2 * SZ_MAX_VERIFY) return SZ_OK;
     SzBatchScratch S;
     const int rc = sz_batch_layout(m, want, &S);
@@ -2228,6 +2228,11 @@ extern "C" int sz_batch_prefill(sz_session* const* ss, int n, const int32_t* con
     for (int b = 0; b < n; b++)
         if (!ss[b] || !ids[b] || lens[b] < 1) return sz_fail(SZ_E_ARG, "sz_batch_prefill: sequence %d has nothing to feed", b);
     const bool chunks = sz_rows_step_fits(ss, n);
+    // a step of twice the rows costs half as much again (every expert's decode is the most of it): where one of the sessions has more room
+    // than the scratch, the steps take that (16 prompts of 75 tokens: 10 steps of 128 rows or 3 of up to 512)
+    if (chunks)
+        for (int b = 0; b < n; b++)
+            if (ss[b]->ws_rows > rows_max) { rows_max = ss[b]->ws_rows; scratch = (uint64_t)ss[b]->ws; scratch_bytes = ss[b]->ws_bytes; }
     for (;;) {
         sz_session* step_s[SZ_BATCH_MAX];
         int32_t step_m[SZ_BATCH_MAX];

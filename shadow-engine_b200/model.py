@@ -341,12 +341,12 @@ class DeviceModel(_Placed):
 class Session:
     """A verify session on the GPU (struct sz_session): owns the one device block the library asks for."""
 
-    def __init__(self, dm, ctx, kv_q8=True, stream=None, head_proxy=False, lean=False):
+    def __init__(self, dm, ctx, kv_q8=True, stream=None, head_proxy=False, lean=False, room=False):
         """head_proxy: screen an EXL3 output.weight with its 2-bit proxy (SZ_HEAD_PROXY); the proxy is built here.
-        lean: no room for a prompt's chunks (SZ_SESSION_LEAN)."""
+        lean: no room for a prompt's chunks (SZ_SESSION_LEAN); room: the full room, for a batch's prompts too (SZ_SESSION_ROOM)."""
         self.lib = szlib.load()
         self.dm = dm
-        self.flags = (1 if kv_q8 else 0) | (2 if head_proxy else 0) | (4 if lean else 0)
+        self.flags = (1 if kv_q8 else 0) | (2 if head_proxy else 0) | (4 if lean else 0) | (8 if room else 0)
         n = C.c_int64()
         szlib.check(self.lib.sz_session_bytes(C.byref(dm.model), ctx, self.flags, C.byref(n)))
         self.mem = torch.empty(n.value + 256, dtype=torch.uint8, device=dm.device)
@@ -536,7 +536,8 @@ class Batch:
         self.dm = dm
         self._stream = torch.cuda.Stream(dm.device)
         self.stream = self._stream.cuda_stream
-        self.sessions = [Session(dm, ctx, kv_q8=kv_q8, stream=self._stream, head_proxy=head_proxy, lean=n > 1) for _ in range(n)]
+        self.sessions = [Session(dm, ctx, kv_q8=kv_q8, stream=self._stream, head_proxy=head_proxy, lean=b > 0, room=b == 0 and n > 1)
+                         for b in range(n)]
         self.rows_max = rows_max or min(256, (n * szlib.MAX_VERIFY + 7) // 8 * 8)
         nb = C.c_int64()
         szlib.check(self.lib.sz_batch_scratch_bytes(C.byref(dm.model), self.rows_max, C.byref(nb)))

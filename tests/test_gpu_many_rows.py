@@ -75,3 +75,21 @@ def test_projections_split_along_k_and_over_row_tiles(rows, cols, m):
     x16 = x.half().double()
     want, mag = x16 @ w16.T, x16.abs() @ w16.abs().T
     assert float(((y[:m, :rows].cpu().double() - want).abs() / (cols * 2.0 ** -23 * mag + 1e-30)).max()) < 1.0
+
+
+@pytest.mark.parametrize("lens,which", [([75, 3, 80, 200, 8, 9], None), ([300, 290], None), ([25, 75, 16], [1, 2])])
+def test_prompts_of_a_batch_in_one_sessions_room_or_in_the_scratch(dm, lens, which):
+    """One session of a batch has room for steps of 512 rows; without it (the others alone) the steps are the scratch's."""
+    prompts = [md.make_prompt(n, CFG["vocab"], seed=80 + i) for i, n in enumerate(lens)]
+    which = which if which is not None else list(range(len(lens)))
+    batch = md.Batch(dm, len(lens), 320)
+    batch.prefill([prompts[b] for b in which], which=which)
+    for b in which:
+        alone = md.Session(dm, 320, kv_q8=True, lean=True)
+        alone.prefill(prompts[b])
+        for s in (alone, batch.sessions[b]):
+            s.top = s.result(logits=True)
+            s.commit((lens[b] - 1) % 8 + 1)
+            s.verify([5, 6, 7])
+        assert np.array_equal(batch.sessions[b].top[2].view(np.uint32), alone.top[2].view(np.uint32)), "prompt %d" % b
+        assert np.array_equal(batch.sessions[b].result(logits=True)[2].view(np.uint32), alone.result(logits=True)[2].view(np.uint32)), "after prompt %d" % b
