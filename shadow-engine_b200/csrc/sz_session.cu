@@ -1803,7 +1803,8 @@ static int sz_rows_layers(sz_session* const* ss, int n, const int32_t* ids, cons
             }
         } else {
             const int di = s0->lb[l].delta_index, vh = c.ssm_v_heads, kh = c.ssm_k_heads, d = c.ssm_head_dim, ch = (2 * kh + vh) * d;
-            SZ_CUDA(sz_launch("rows_delta_prep", sz_rows_delta_prep_kernel, dim3((ch + 255) / 256, R), dim3(256), 0, st, true, seqs, rws, di, (const float*)outs[0],
+            SZ_CUDA(sz_launch("rows_delta_prep", c.conv_k == 4 ? sz_rows_delta_prep_kernel<4> : sz_rows_delta_prep_kernel<0>,
+                              dim3((ch + 255) / 256, (R + SZ_PREP_ROWS - 1) / SZ_PREP_ROWS), dim3(256), 0, st, true, seqs, rws, R, di, (const float*)outs[0],
                               (const float*)L.ssm_conv1d.data, (const float*)outs[2], (const float*)outs[3], (const float*)L.ssm_a.data, (const float*)L.ssm_dt_bias.data,
                               kh, vh, d, (int)c.conv_k, XC, BETA, DECAY));
             SZ_CUDA(sz_launch("rows_scan", d == 128 ? sz_rows_scan_kernel<128> : sz_rows_scan_kernel<64>, dim3(vh * (d / 32), n), dim3(d), 0, st, true, seqs, di,

@@ -271,68 +271,106 @@ sz_hc_up_rows_kernel(const float* __restrict__ hd, const u8* __restrict__ up, co
     }
 }
 
-// The DeltaNet front end over the rows of a step (sz_delta_prep_kernel's arithmetic).  grid (ceil(ch / 256), rows).  What the scan
-// reads - and a replay, when the sequence's rows may be rejected - goes to the session's buffers, of a prompt's chunk to the step's
-// (xc_all, beta_all, decay_all), and a chunk's last row leaves the carried conv rows behind it in the other buffer.
+// The DeltaNet front end over the rows of a step (sz_delta_prep_kernel's arithmetic).  grid (ceil(ch / 256), ceil(rows / SZ_PREP_ROWS)).
+// What the scan reads - and a replay, when the sequence's rows may be rejected - goes to the session's buffers, of a prompt's chunk to
+// the step's (xc_all, beta_all, decay_all), and a chunk's last row leaves the carried conv rows behind it in the other buffer.
+// A thread takes its channel for 4 rows of the step: taps and their conversions once, a projection loaded for its own row serves the three
+// after it (a row a block: 504 rows 71 -> 45 us).  K: the taps where they are the usual 4, else 0.
+#define SZ_PREP_ROWS 4
+template <int K>
 __global__ void __launch_bounds__(256)
-sz_rows_delta_prep_kernel(const SzSeqDev* __restrict__ seqs, const SzRowDev* __restrict__ rws, int di, const float* __restrict__ xin, const float* __restrict__ cw,
+sz_rows_delta_prep_kernel(const SzSeqDev* __restrict__ seqs, const SzRowDev* __restrict__ rws, int rows, int di, const float* __restrict__ xin, const float* __restrict__ cw,
                           const float* __restrict__ b, const float* __restrict__ a, const float* __restrict__ a_log, const float* __restrict__ dt, int kh, int vh, int d,
-                          int k, float* __restrict__ xc_all, float* __restrict__ beta_all, float* __restrict__ decay_all) {
-    __shared__ double sred[8];
-    const int r = blockIdx.y, j = rws[r].j;
-    const SzSeqDev& q = seqs[rws[r].seq];
+                          int kr, float* __restrict__ xc_all, float* __restrict__ beta_all, float* __restrict__ decay_all) {
+    constexpr int RB = SZ_PREP_ROWS, KM = K ? K : 8;
+    __shared__ double sred[RB][8];
+    const int k = K ? K : kr;
+    const int r0 = blockIdx.y * RB, nr = min(RB, rows - r0), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int kd = kh * d, ch = 2 * kd + vh * d, i = blockIdx.x * 256 + threadIdx.x;
-    float taps[8];
-    for (int t = 0; t < k; t++) taps[t] = i < ch ? __ldg(cw + (size_t)i * k + t) : 0.f;
+    const bool norms = (int)blockIdx.x * 256 < 2 * kd;      // (d divides 256: a head of q or k is whole warps of one block)
+    double taps[KM];
+#pragma unroll
+    for (int t = 0; t < KM; t++) taps[t] = i < ch && t < k ? (double)__ldg(cw + (size_t)i * k + t) : 0.0;
     sz_pdl_wait();
     sz_pdl_trigger();
-    const int cur = q.state[1];
-    const size_t cl = (size_t)(k - 1) * ch;
-    const float* conv = (cur ? q.conv1 : q.conv0) + di * cl;
-    float* convw = (cur ? q.conv0 : q.conv1) + di * cl;
-    float* xc = q.all ? xc_all + (size_t)r * ch : q.xc + ((size_t)di * SZ_MAX_VERIFY + j) * ch;
-    const float* x = xin + (size_t)r * ch;          // (the rows before it in its sequence are the rows before it in the step)
-    float v = 0.f;
-    if (i < ch) {
-        const float own = x[i];
-        double acc = (double)taps[k - 1] * (double)own;
-        for (int t = 0; t < k - 1; t++) {
-            const int tau = j - (k - 1) + t;
-            const float prev = tau >= 0 ? x[(long long)(t - (k - 1)) * ch + i] : conv[(size_t)((k - 1) + tau) * ch + i];
-            acc += (double)taps[t] * (double)prev;
-        }
-        v = sz_silu((float)acc);
-        if (!q.all) q.xin[((size_t)di * SZ_MAX_VERIFY + j) * ch + i] = own;
-        else if (j == q.m - 1)
-            for (int t = 0; t < k - 1; t++) {
-                const int tau = q.m - (k - 1) + t;
-                convw[(size_t)t * ch + i] = tau >= 0 ? x[(long long)(t - (k - 2)) * ch + i] : conv[(size_t)((k - 1) + tau) * ch + i];
+    float xw[RB + KM - 1], v[RB];                            // rows r0 - (KM - 1) .. of the step; what is not of a row's sequence is not used
+#pragma unroll
+    for (int e = 0; e < RB + KM - 1; e++) {
+        const int r = r0 - (KM - 1) + e;
+        xw[e] = i < ch && r >= 0 && r < rows ? __ldcg(xin + (size_t)r * ch + i) : 0.f;
+    }
+#pragma unroll
+    for (int e = 0; e < RB; e++) {
+        v[e] = 0.f;
+        if (e < nr && i < ch) {
+            const SzSeqDev& q = seqs[rws[r0 + e].seq];
+            const int j = rws[r0 + e].j, cur = q.state[1];
+            const size_t cl = (size_t)(k - 1) * ch;
+            const float* conv = (cur ? q.conv1 : q.conv0) + di * cl;
+            const float own = xw[e + KM - 1];
+            double last = 0.0, acc;
+#pragma unroll
+            for (int t = 0; t < KM; t++) if (t == k - 1) last = taps[t];
+            acc = last * (double)own;
+#pragma unroll
+            for (int t = 0; t < KM - 1; t++)
+                if (t < k - 1) {
+                    const int tau = j - (k - 1) + t;
+                    float prev = 0.f;
+                    if (K) prev = xw[e + t];
+                    else {
+#pragma unroll
+                        for (int w = 0; w < KM - 1; w++) if (w == KM - k + t) prev = xw[e + w];
+                    }
+                    if (tau < 0) prev = conv[(size_t)((k - 1) + tau) * ch + i];
+                    acc += taps[t] * (double)prev;
+                }
+            v[e] = sz_silu((float)acc);
+            if (!q.all) q.xin[((size_t)di * SZ_MAX_VERIFY + j) * ch + i] = own;
+            else if (j == q.m - 1) {
+                float* convw = (cur ? q.conv0 : q.conv1) + di * cl;
+                const float* x = xin + (size_t)(r0 + e) * ch;
+                for (int t = 0; t < k - 1; t++) {
+                    const int tau = q.m - (k - 1) + t;
+                    convw[(size_t)t * ch + i] = tau >= 0 ? x[(long long)(t - (k - 2)) * ch + i] : conv[(size_t)((k - 1) + tau) * ch + i];
+                }
             }
-    }
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const double sq = sz_warp_sum((double)v * (double)v);
-    if (lane == 0) sred[warp] = sq;
-    __syncthreads();
-    if (i < ch) {
-        if (i < 2 * kd) {
-            const int w0 = (threadIdx.x / d) * (d / 32);
-            double ss = 0.0;
-            for (int t = 0; t < d / 32; t++) ss += sred[w0 + t];
-            const double n = sz_rsqrt64(ss + 1e-6);
-            float t = (float)((double)v * n);
-            if (i < kd) t = t / sqrtf((float)d);
-            v = t;
         }
-        xc[i] = v;
     }
-    if (blockIdx.x == 0) {
-        float* beta = q.all ? beta_all + (size_t)r * vh : q.beta + ((size_t)di * SZ_MAX_VERIFY + j) * vh;
-        float* decay = q.all ? decay_all + (size_t)r * vh : q.decay + ((size_t)di * SZ_MAX_VERIFY + j) * vh;
-        for (int h = threadIdx.x; h < vh; h += 256) {
-            beta[h] = sz_sigmoid(b[(size_t)r * vh + h]);
-            const float sp_in = a[(size_t)r * vh + h] + dt[h];
-            const float sp = sp_in > 20.0f ? sp_in : log1pf(expf(sp_in));
-            decay[h] = expf(a_log[h] * sp);
+    if (norms) {
+#pragma unroll
+        for (int e = 0; e < RB; e++) {
+            const double sq = sz_warp_sum((double)v[e] * (double)v[e]);
+            if (lane == 0) sred[e][warp] = sq;
+        }
+        __syncthreads();
+    }
+    for (int e = 0; e < nr; e++) {
+        const SzSeqDev& q = seqs[rws[r0 + e].seq];
+        const int j = rws[r0 + e].j;
+        float out = e == 0 ? v[0] : (e == 1 ? v[1] : (e == 2 ? v[2] : v[3]));
+        if (i < ch) {
+            if (i < 2 * kd) {
+                const int w0 = (threadIdx.x / d) * (d / 32);
+                double ss = 0.0;
+                for (int t = 0; t < d / 32; t++) ss += sred[e][w0 + t];
+                const double n = sz_rsqrt64(ss + 1e-6);
+                float t = (float)((double)out * n);
+                if (i < kd) t = t / sqrtf((float)d);
+                out = t;
+            }
+            (q.all ? xc_all + (size_t)(r0 + e) * ch : q.xc + ((size_t)di * SZ_MAX_VERIFY + j) * ch)[i] = out;
+        }
+        if (blockIdx.x == 0) {
+            const int r = r0 + e;
+            float* beta = q.all ? beta_all + (size_t)r * vh : q.beta + ((size_t)di * SZ_MAX_VERIFY + j) * vh;
+            float* decay = q.all ? decay_all + (size_t)r * vh : q.decay + ((size_t)di * SZ_MAX_VERIFY + j) * vh;
+            for (int h = threadIdx.x; h < vh; h += 256) {
+                beta[h] = sz_sigmoid(b[(size_t)r * vh + h]);
+                const float sp_in = a[(size_t)r * vh + h] + dt[h];
+                const float sp = sp_in > 20.0f ? sp_in : log1pf(expf(sp_in));
+                decay[h] = expf(a_log[h] * sp);
+            }
         }
     }
 }
