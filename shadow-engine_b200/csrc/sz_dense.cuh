@@ -437,6 +437,8 @@ static __global__ void __launch_bounds__(256, 2) sz_dense_q8_kernel(const SzDens
 // (The form before it gave a thread block one part and four or eight row groups: a fragment of the rows was loaded from shared memory for
 // every unit, and the parts' sums - 98 MB at 256 rows of 12,352 outputs - went through a scratch and a second kernel.  the four MMAs a
 // block and group alone are 44 us.)
+// Where thread blocks of 8 units and 32 rows would leave multiprocessors idle (80 rows of 2,048 outputs: 48 of them, 49 us, 3,000 cycles for
+// 128 columns in which the tensor pipe works 900), the blocks are of 4 units and 16 rows: 35 us.
 // A slice of a matrix row starts at a multiple of 8 bytes, not of 16: the copy starts at the 16-byte boundary below it.
 struct SzDenseRowsCfg {
     int units[SZ_DENSE_MAX_JOBS + 1];   // 16-row units before each job
@@ -446,10 +448,12 @@ struct SzDenseRowsCfg {
 #define SZ_DR_COLS 128      // columns a stage
 #define SZ_DR_RS 144        // bytes between the staged slices (136 and where they start)
 #define SZ_DR_XS 160        // halves between the staged rows (16 (mod 32) words: the eight rows a quarter of a warp reads at once)
+// NW: warps a thread block, a unit of 16 matrix rows each; NG: groups of 8 rows of the step
+template <int NW, int NG>
 struct SzDenseRows {
-    static constexpr int WROWS = 8 * 16;                                         // matrix rows a thread block
-    static constexpr int STAGE = WROWS * SZ_DR_RS + 2 * 32 * SZ_DR_XS * 2;
-    static constexpr int STAGES = 2;
+    static constexpr int WROWS = NW * 16;                                        // matrix rows a thread block
+    static constexpr int STAGE = WROWS * SZ_DR_RS + 2 * 8 * NG * SZ_DR_XS * 2;
+    static constexpr int STAGES = NW == 8 ? 2 : 4;
     static constexpr int SMEM = STAGES * STAGE + WROWS * 8;
 };
 
@@ -476,16 +480,18 @@ __device__ __forceinline__ void sz_q8_quad(u32 w, u32& lo, u32& hi) {
     lo = *(const u32*)&ha; hi = *(const u32*)&hb;
 }
 
-// grid (ceil(units / 8), ceil(rows / 32)), block 256
-static __global__ void __launch_bounds__(256, 2) sz_dense_rows_q8_kernel(const SzDenseArgs a, const SzDenseRowsCfg c) {
-    using X = SzDenseRows;
+// grid (ceil(units / NW), ceil(rows / (8 NG))), block 32 NW
+template <int NW, int NG>
+static __global__ void __launch_bounds__(32 * NW, 2) sz_dense_rows_q8_kernel(const SzDenseArgs a, const SzDenseRowsCfg c) {
+    using X = SzDenseRows<NW, NG>;
+    constexpr int NTH = 32 * NW;
     constexpr int S = X::STAGES;
     extern __shared__ __align__(128) u8 smem[];
     const u8** wrow = (const u8**)(smem + S * X::STAGE);       // where the thread block's matrix rows start
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, q = lane & 3;
-    const int total = c.units[a.n_jobs], u0 = blockIdx.x * 8, j0 = blockIdx.y * 32;
-    const int ng = (c.rows - j0) / 8 < 4 ? (c.rows - j0) / 8 : 4;
+    const int total = c.units[a.n_jobs], u0 = blockIdx.x * NW, j0 = blockIdx.y * 8 * NG;
+    const int ng = (c.rows - j0) / 8 < NG ? (c.rows - j0) / 8 : NG;
     const size_t rb = (size_t)(a.cols / 32) * 34;
     const int nchunk = a.cols / SZ_DR_COLS, nblk = a.cols / 256;      // blocks a part
     auto locate = [&](int u, int& ji, int& row0, int& nrows) {
@@ -496,7 +502,7 @@ static __global__ void __launch_bounds__(256, 2) sz_dense_rows_q8_kernel(const S
         row0 = (u - c.units[ji]) * 16;
         nrows = min(16, a.job[ji].rows - row0);
     };
-    for (int r = threadIdx.x; r < X::WROWS; r += 256) {
+    for (int r = threadIdx.x; r < X::WROWS; r += NTH) {
         const int u = min(u0 + (r >> 4), total - 1);          // (units past the last: its rows again; nothing of them is kept)
         int ji, row0, nrows;
         locate(u, ji, row0, nrows);
@@ -507,7 +513,7 @@ static __global__ void __launch_bounds__(256, 2) sz_dense_rows_q8_kernel(const S
         u8* st = smem + (size_t)(ci % S) * X::STAGE;
         const int at = ci * 136 & ~15;
 #pragma unroll
-        for (int i = threadIdx.x; i < X::WROWS * 9; i += 256) {
+        for (int i = threadIdx.x; i < X::WROWS * 9; i += NTH) {
             const int r = i / 9, ch = i - r * 9;
             sz_cp_async16(st + r * SZ_DR_RS + ch * 16, wrow[r] + at + ch * 16);
         }
@@ -515,18 +521,18 @@ static __global__ void __launch_bounds__(256, 2) sz_dense_rows_q8_kernel(const S
     auto stage_x = [&](int ci) {
         u8* st = smem + (size_t)(ci % S) * X::STAGE + X::WROWS * SZ_DR_RS;
 #pragma unroll
-        for (int i = threadIdx.x; i < 2 * 32 * 16; i += 256) {
-            const int part = i >> 9, j = (i >> 4) & 31, ch = i & 15;
-            if (j < ng * 8) sz_cp_async16(st + (size_t)(part * 32 + j) * SZ_DR_XS * 2 + ch * 16, c.xh + (size_t)(part * c.rows + j0 + j) * a.cols + ci * SZ_DR_COLS + ch * 8);
+        for (int i = threadIdx.x; i < 2 * 8 * NG * 16; i += NTH) {
+            const int part = i / (8 * NG * 16), j = (i >> 4) % (8 * NG), ch = i & 15;
+            if (j < ng * 8) sz_cp_async16(st + (size_t)(part * 8 * NG + j) * SZ_DR_XS * 2 + ch * 16, c.xh + (size_t)(part * c.rows + j0 + j) * a.cols + ci * SZ_DR_COLS + ch * 8);
         }
     };
     for (int i = 0; i < S - 1 && i < nchunk; i++) stage_w(i);      // (the matrices are constants: on their way before the wait)
     sz_pdl_wait();
     sz_pdl_trigger();
     for (int i = 0; i < S - 1; i++) { if (i < nchunk) stage_x(i); sz_cp_async_commit(); }
-    float tot[4][4], acc[4][4];
+    float tot[NG][4], acc[NG][4];
 #pragma unroll
-    for (int gi = 0; gi < 4; gi++)
+    for (int gi = 0; gi < NG; gi++)
 #pragma unroll
         for (int e = 0; e < 4; e++) { tot[gi][e] = 0.f; acc[gi][e] = 0.f; }
     int left = nblk;                       // blocks left of the part at hand
@@ -558,11 +564,11 @@ static __global__ void __launch_bounds__(256, 2) sz_dense_rows_q8_kernel(const S
                 sz_q8_quad(c23, a2[h], a2[2 + h]);
             }
 #pragma unroll
-            // (all four groups, whether the step has them or not: a branch around one would keep its MMAs - a chain of four - from running
+            // (all groups, whether the step has them or not: a branch around one would keep its MMAs - a chain of four - from running
             // between the others')
-            for (int gi = 0; gi < 4; gi++) {
+            for (int gi = 0; gi < NG; gi++) {
                 const uint4 bh = *(const uint4*)(xr + (size_t)gi * 8 * SZ_DR_XS + b * 32);
-                const uint4 bl = *(const uint4*)(xr + (size_t)(32 + gi * 8) * SZ_DR_XS + b * 32);
+                const uint4 bl = *(const uint4*)(xr + (size_t)(8 * NG + gi * 8) * SZ_DR_XS + b * 32);
                 float t[4] = {0.f, 0.f, 0.f, 0.f};
                 sz_mma16816_zn(t, a1, bh.x, bh.y);
                 sz_mma16816_zn(t, a2, bh.z, bh.w);
@@ -574,7 +580,7 @@ static __global__ void __launch_bounds__(256, 2) sz_dense_rows_q8_kernel(const S
             if (--left == 0) {             // the part's sum is complete
                 left = nblk;
 #pragma unroll
-                for (int gi = 0; gi < 4; gi++)
+                for (int gi = 0; gi < NG; gi++)
 #pragma unroll
                     for (int e = 0; e < 4; e++) { tot[gi][e] += acc[gi][e]; acc[gi][e] = 0.f; }
             }
@@ -586,7 +592,7 @@ static __global__ void __launch_bounds__(256, 2) sz_dense_rows_q8_kernel(const S
         locate(u, ji, row0, nrows);
         const SzDenseJob& jb = a.job[ji];
 #pragma unroll
-        for (int gi = 0; gi < 4; gi++) {
+        for (int gi = 0; gi < NG; gi++) {
             if (gi < ng) {
                 float* o = jb.out + (size_t)(j0 + gi * 8 + 2 * q) * jb.ostride + row0 + g;
                 if (g < nrows) { o[0] = sz_epilogue(jb.epi, tot[gi][0], jb.div); o[jb.ostride] = sz_epilogue(jb.epi, tot[gi][1], jb.div); }

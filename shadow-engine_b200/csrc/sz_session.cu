@@ -642,8 +642,15 @@ int sz_dense_rows_launch(SzDenseArgs& a, void* xh, cudaStream_t st, const char* 
     c.xh = (const __half*)xh;
     SZ_CUDA(sz_launch("dense_rows_pack", sz_dense_rows_pack_kernel, dim3((a.cols + 1023) / 1024, a.m), dim3(256), 0, st, true, a.x, a.xstride, a.cols, a.m, (__half*)xh));
     static bool set = false;
-    if (!set) { SZ_CUDA(cudaFuncSetAttribute(sz_dense_rows_q8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SzDenseRows::SMEM)); set = true; }
-    SZ_CUDA(sz_launch(name, sz_dense_rows_q8_kernel, dim3((units + 7) / 8, (a.m + 31) / 32), dim3(256), SzDenseRows::SMEM, st, true, a, c));
+    if (!set) {
+        SZ_CUDA(cudaFuncSetAttribute(sz_dense_rows_q8_kernel<8, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, SzDenseRows<8, 4>::SMEM));
+        SZ_CUDA(cudaFuncSetAttribute(sz_dense_rows_q8_kernel<4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SzDenseRows<4, 2>::SMEM));
+        set = true;
+    }
+    if ((units + 7) / 8 * ((a.m + 31) / 32) >= sz_sm_count_session())
+        SZ_CUDA(sz_launch(name, sz_dense_rows_q8_kernel<8, 4>, dim3((units + 7) / 8, (a.m + 31) / 32), dim3(256), SzDenseRows<8, 4>::SMEM, st, true, a, c));
+    else
+        SZ_CUDA(sz_launch(name, sz_dense_rows_q8_kernel<4, 2>, dim3((units + 3) / 4, (a.m + 15) / 16), dim3(128), SzDenseRows<4, 2>::SMEM, st, true, a, c));
     *taken = 1;
     return SZ_OK;
 }
