@@ -854,9 +854,11 @@ static int sz_x3_launch_k(cudaStream_t st, const sz_moe_layer* L, int m, const S
         // few rows mean few units (a 1-row pass of the benchmark's shape: 11 groups, 352 units 4 wide for 296 blocks): narrower units
         // and a third block a multiprocessor spread them better (4.30 -> 4.19 ms a 1-row pass of the 48-layer model); with 4 rows the
         // wide units win (6.18 against 6.35 ms)
-        const bool few = m * (int)L->top_k <= 24;
-        const int occ = eo && atoi(eo) == 2 ? 2 : (eo && atoi(eo) == 3 ? 3 : (few ? 3 : 2));
-        int tw = et ? atoi(et) : (few ? 2 : 4), twd = ed ? atoi(ed) : (few ? 2 : 4);
+        // (up to 48 groups, 40 at 4 rows of the benchmark's layer: three blocks and the down matrices in narrower units even out what is left
+        // over, 60.8 -> 59.3 us a layer; with 75 groups two blocks win, 10.30 against 10.37 ms a pass of 8 rows)
+        const bool few = m * (int)L->top_k <= 24, some = m * (int)L->top_k <= 48;
+        const int occ = eo && atoi(eo) == 2 ? 2 : (eo && atoi(eo) == 3 ? 3 : (few || some ? 3 : 2));
+        int tw = et ? atoi(et) : (few ? 2 : 4), twd = ed ? atoi(ed) : (few || some ? 2 : 4);
         if (!(tw == 1 || tw == 2 || tw == 4) || tw > NTC || NTC % tw) tw = NTC < 4 ? NTC : 4;
         if (tw == 3) tw = 1;
         if (!(twd == 1 || twd == 2 || twd == 4)) twd = 4;
