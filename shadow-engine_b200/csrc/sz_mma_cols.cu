@@ -18,7 +18,7 @@
 //   warp 0      the token tile of a step, already in f16 and in the instruction's own shared-memory order (written once by
 //               sz_x16_pack_kernel), one bulk copy.
 //   warps 1..16 decode, in groups of MT x 128 threads: a thread takes its group's blocks of a weight row's 272 bytes into registers -
-//               which frees the buffer for the next piece at once - and turns them block after block into f16 in the canonical K-major
+//               which frees the buffer for the next piece once the last word is there - and turns them block after block into f16 in the canonical K-major
 //               no-swizzle order (8 rows x 16 bytes core matrices), then fence.proxy.async and arrive.  The groups take the steps in turn.
 //   warp 17     one thread issues the step's 2 MT tcgen05.mma (K = 16 each) from shared-memory descriptors and commits them to the
 //               stage's "empty" barrier, which frees the stage for the decoders and the copy warp.
@@ -30,7 +30,7 @@
 // a token tile (25 KB per 256 x 256 x 32) where one a block moved 41, and the tensor core, which needs 512 cycles of the step's 625; the
 // sums of a unit, which all blocks write at about the same time, are a fifth.  At few tokens latency: the chain decode, fence, barrier,
 // instruction.  The issuing thread took 390 cycles a step to make descriptors for 256 cycles of instructions; it makes them once.
-// 12,288 x 2,048: 4,093 tokens 281 -> 245 us (sustained, 1.4 GHz under the power cap), 256 tokens 28.8 -> 23.6;
+// 12,288 x 2,048: 4,093 tokens 281 -> 243 us (sustained, 1.4 GHz under the power cap), 256 tokens 28.8 -> 24.7;
 // 512 x 2,048, one token: 20 -> 12.4 (K in four parts).
 // Every wait is bounded; a wait that runs out records where in the error word, and the block still frees its tensor memory.
 #include <cuda.h>   // CUtensorMap and its enums; the encoder's entry point is asked of the runtime, nothing links against the driver
@@ -61,10 +61,25 @@ struct McSmem {
     u32 tmem_base, failed;
 };
 
-// one arrival a warp: the arrivals of 32 lanes on one barrier are taken one after the other
+// One arrival a warp: the arrivals of 32 lanes on one barrier are taken one after the other.  What the other lanes did before it is
+// ordered by the __syncwarp (and by their own proxy fence, where the reader is a copy or the tensor core), then by the arrival's release.
 __device__ __forceinline__ void mc_arrive_warp(u64* bar) {
     __syncwarp();
     if ((threadIdx.x & 31) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sz_smem_addr(bar)) : "memory");
+}
+// The raw words a warp's lanes have loaded are in registers: the buffer may be refilled.  The refill is a write of the async proxy, and a
+// load that was only issued is ordered before it by nothing: released right after its loads, a buffer was at times overwritten under
+// one (16 bytes of one weight row wrong for all tokens, seen with four groups and a saturated shared memory).  So the arrival's
+// address depends on every word of every lane (`zero` is 0, which only the host knows), and every lane fences its reads.
+template <int N>
+__device__ __forceinline__ void mc_release_raw(u64* bar, const u32 (&W)[N], u32 zero) {
+    u32 any = 0;
+#pragma unroll
+    for (int i = 0; i < N; i++) any |= W[i];
+    any = __reduce_or_sync(0xffffffffu, any);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sz_smem_addr(bar) + (any & zero)) : "memory");
 }
 __device__ __forceinline__ void mc_fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void mc_tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -164,6 +179,7 @@ struct McArgs {
     long long ys;
     int rows, cols, m, nt, tiles, ks;   // nt: tokens a tile; ks: blocks of a cluster, the parts of K
     u32* err;
+    u32 zero;                             // 0 (mc_release_raw)
 };
 
 // grid: ks == 1, up to 148 blocks that take (row tile, token tile) units in turn; else (units * ks), cluster (ks).
@@ -204,6 +220,7 @@ sz_mma_cols_q8_kernel(const __grid_constant__ CUtensorMap wmap, const McArgs a) 
         // ---- token tiles as stages come free (what the pack kernel wrote: after the dependency wait)
         sz_pdl_wait();
         sz_pdl_trigger();
+        asm volatile("fence.proxy.async.global;" ::: "memory");   // the pack kernel's stores, visible since the wait, before the copies' reads
         for (int u = u0, k = 0; u < units && !failed; u += us) {
             const u8* src = (const u8*)a.x16 + ((size_t)(u / rtiles) * (a.cols / MC_KT) + p0 * MC_STEPS) * b_bytes;
             for (int j = 0; j < steps; j++, k++) {
@@ -216,7 +233,7 @@ sz_mma_cols_q8_kernel(const __grid_constant__ CUtensorMap wmap, const McArgs a) 
             }
         }
     } else if (warp == LAST + 2) {
-        // ---- raw weight bytes, a piece as soon as the decoders have the one before it in registers
+        // ---- raw weight bytes, a piece as soon as the decoders have the one before it in registers (mc_release_raw)
         for (int u = u0, n = 0; u < units && !failed; u += us)
             for (int p = 0; p < pieces; p++, n++) {
                 if (n > 0 && !sz_mbar_wait(&S->raw_empty, (n - 1) & 1, MC_WAIT)) { failed = 2; break; }
@@ -295,15 +312,15 @@ sz_mma_cols_q8_kernel(const __grid_constant__ CUtensorMap wmap, const McArgs a) 
                 const uint4* rp = (const uint4*)(raw + (size_t)r * MC_RAW_ROW + mc_group_start<G>(g));
 #pragma unroll
                 for (int i = 0; i < NW; i++) { const uint4 v = rp[i]; W[4 * i] = v.x; W[4 * i + 1] = v.y; W[4 * i + 2] = v.z; W[4 * i + 3] = v.w; }
-                mc_arrive_warp(&S->raw_empty);
+                mc_release_raw(&S->raw_empty, W, a.zero);
                 auto step = [&](auto I) {
                     constexpr int i = decltype(I)::value;
                     const int k = k0 + i * G + g, st = k % MC_STAGES;
                     if (failed) return;
                     if (k >= MC_STAGES && !sz_mbar_wait(&S->empty[st], ((k / MC_STAGES) - 1) & 1, MC_WAIT)) { failed = 3; return; }
                     mc_decode_of<G, i>(g, W, dst0 + st * MT * MC_A_BYTES);
-                    mc_fence_async();                 // the tensor core reads shared memory through the async proxy
-                    mc_arrive_warp(&S->full[st]);
+                    mc_fence_async();                 // every lane's stores, before the tensor core reads them through the async proxy:
+                    mc_arrive_warp(&S->full[st]);     // fence, warp, arrival; the issuing thread waits and goes through tcgen05.fence
                 };
                 step(McInt<0>()); step(McInt<1>());
                 if constexpr (G == 2) { step(McInt<2>()); step(McInt<3>()); }
@@ -492,7 +509,7 @@ extern "C" int sz_mma_cols(const sz_tensor* w, uint64_t x, int64_t xs, uint64_t 
     SZ_CUDA(sz_launch("x16_pack", sz_x16_pack_kernel, dim3((unsigned)((units + 255) / 256 < 1184 ? (units + 255) / 256 : 1184)), dim3(256), 0, st, true,
                       (const float*)x, (long long)xs, m, cols, nt, tiles, x16));
     McArgs a;
-    a.x16 = x16; a.y = (float*)y; a.ys = (long long)ys; a.rows = rows; a.cols = cols; a.m = m; a.nt = nt; a.tiles = tiles; a.ks = plan.ks; a.err = err;
+    a.x16 = x16; a.y = (float*)y; a.ys = (long long)ys; a.rows = rows; a.cols = cols; a.m = m; a.nt = nt; a.tiles = tiles; a.ks = plan.ks; a.err = err; a.zero = 0;
     return plan.mt == 2 ? mc_launch<2>(wmap, a, st) : mc_launch<1>(wmap, a, st);
 }
 

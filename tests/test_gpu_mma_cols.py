@@ -52,6 +52,37 @@ def test_strided_rows_and_a_second_call_reuse_the_scratch():
     assert float(np.max(np.abs(a.cpu().numpy() - want) / (cols * 2.0 ** -23 * mag))) < 1.0
 
 
+# Every form of the kernel: one row tile without parts of K (one and several units a block), two row tiles, K in 2, 3 and 4 parts (and
+# a tile narrower than 256 tokens); two calls in a burst write to buffers of their own, so that the second starts under the first.
+@pytest.mark.parametrize("rows,cols,m,calls", [(12288, 2048, 256, 2000), (2600, 512, 2000, 2000), (3000, 768, 2049, 2000), (12288, 2048, 4093, 400),
+                                               (8192, 2048, 256, 2000), (385, 3328, 40, 2000), (2048, 4096, 256, 2000), (512, 2048, 17, 2000)])
+def test_thousands_of_calls_give_the_same_bits(rows, cols, m, calls):
+    wb = make(rows, cols, 31)
+    x = synth.normal((m, cols), 1.0, 33, "mma_cols.x").cuda()
+    op = mc.MmaCols(wb, rows, cols, m)
+    first = op(x).clone()
+    w16 = torch.from_numpy(ob.dequant(ob.Q8_0, wb.numpy()).reshape(rows, cols)).cuda().half().double()
+    for t in range(0, m, 512):     # against the f64 product of the f16 operands, within f32 accumulation
+        x16 = x[t:t + 512].half().double()
+        bound = cols * 2.0 ** -23 * (x16.abs() @ w16.abs().T) + 1e-30
+        assert float(((first[t:t + 512].double() - x16 @ w16.T).abs() / bound).max()) < 1.0, "tokens %d.." % t
+    ys = [torch.empty_like(first) for _ in range(4 if first.numel() < 1 << 24 else 2)]
+    bad = torch.zeros((), dtype=torch.int64, device="cuda")
+    seen = torch.empty_like(first)
+    for _ in range(calls // len(ys)):
+        for y in ys:
+            op(x, out=y)
+        for y in ys:
+            off = torch.any(y.view(torch.int32) != first.view(torch.int32))
+            seen = torch.where(off, y, seen)
+            bad += off
+    assert op.status() == 0
+    if int(bad):
+        at = (seen.view(torch.int32) != first.view(torch.int32)).nonzero()
+        tok, row = at[:, 0].unique().tolist(), at[:, 1].unique().tolist()     # one row, all tokens: the weights' side; one token, 128 rows: the tokens'
+        pytest.fail("%d of %d calls differ; in the last of them %d tokens (%s ..) and %d rows (%s ..)" % (int(bad), calls, len(tok), tok[:8], len(row), row[:8]))
+
+
 def test_arguments_are_checked():
     wb = make(128, 256, 3)
     op = mc.MmaCols(wb, 128, 256, 16)
