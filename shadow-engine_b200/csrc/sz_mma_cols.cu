@@ -81,6 +81,9 @@ __device__ __forceinline__ void mc_release_raw(u64* bar, const u32 (&W)[N], u32 
     __syncwarp();
     if ((threadIdx.x & 31) == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sz_smem_addr(bar) + (any & zero)) : "memory");
 }
+// A decode warp's wait, all lanes with one outcome (those that gave up leave together, and nobody waits for them at the next __syncwarp).
+// The copy and issue warps wait in one lane: a lane that only waited could fall two phases behind and find its parity come round.
+__device__ __forceinline__ bool mc_wait_warp(u64* bar, u32 phase) { return __all_sync(0xffffffffu, sz_mbar_wait(bar, phase, MC_WAIT)); }
 __device__ __forceinline__ void mc_fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void mc_tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void mc_tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -221,32 +224,31 @@ sz_mma_cols_q8_kernel(const __grid_constant__ CUtensorMap wmap, const McArgs a) 
         sz_pdl_wait();
         sz_pdl_trigger();
         asm volatile("fence.proxy.async.global;" ::: "memory");   // the pack kernel's stores, visible since the wait, before the copies' reads
-        for (int u = u0, k = 0; u < units && !failed; u += us) {
+        for (int u = lane == 0 ? u0 : units, k = 0; u < units && !failed; u += us) {
             const u8* src = (const u8*)a.x16 + ((size_t)(u / rtiles) * (a.cols / MC_KT) + p0 * MC_STEPS) * b_bytes;
             for (int j = 0; j < steps; j++, k++) {
                 const int st = k % MC_STAGES;
                 if (k >= MC_STAGES && !sz_mbar_wait(&S->empty[st], ((k / MC_STAGES) - 1) & 1, MC_WAIT)) { failed = 1; break; }
-                if (lane == 0) {
-                    sz_mbar_expect_tx(&S->full[st], (u32)b_bytes);
-                    sz_bulk_g2s(sb + st * b_bytes, src + (size_t)(j / MC_STEPS * MC_STEPS + mc_block<MT>(j % MC_STEPS)) * b_bytes, (u32)b_bytes, &S->full[st]);
-                }
+                sz_mbar_expect_tx(&S->full[st], (u32)b_bytes);
+                sz_bulk_g2s(sb + st * b_bytes, src + (size_t)(j / MC_STEPS * MC_STEPS + mc_block<MT>(j % MC_STEPS)) * b_bytes, (u32)b_bytes, &S->full[st]);
             }
         }
+        __syncwarp();
     } else if (warp == LAST + 2) {
         // ---- raw weight bytes, a piece as soon as the decoders have the one before it in registers (mc_release_raw)
-        for (int u = u0, n = 0; u < units && !failed; u += us)
+        for (int u = lane == 0 ? u0 : units, n = 0; u < units && !failed; u += us)
             for (int p = 0; p < pieces; p++, n++) {
                 if (n > 0 && !sz_mbar_wait(&S->raw_empty, (n - 1) & 1, MC_WAIT)) { failed = 2; break; }
-                if (lane == 0) {   // x = 136 * piece words = 272 * piece bytes: a multiple of 16; rows past the matrix arrive as zeros
-                    sz_mbar_expect_tx(&S->raw_full, (u32)(MT * MC_RAW_BYTES));
+                // x = 136 * piece words = 272 * piece bytes: a multiple of 16; rows past the matrix arrive as zeros
+                sz_mbar_expect_tx(&S->raw_full, (u32)(MT * MC_RAW_BYTES));
 #pragma unroll
-                    for (int mt = 0; mt < MT; mt++)
-                        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-                                         sz_smem_addr(raw + mt * MC_RAW_BYTES)),
-                                     "l"(&wmap), "r"((p0 + p) * (MC_RAW_ROW / 2)), "r"((u % rtiles * MT + mt) * MC_BM), "r"(sz_smem_addr(&S->raw_full))
-                                     : "memory");
-                }
+                for (int mt = 0; mt < MT; mt++)
+                    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+                                     sz_smem_addr(raw + mt * MC_RAW_BYTES)),
+                                 "l"(&wmap), "r"((p0 + p) * (MC_RAW_ROW / 2)), "r"((u % rtiles * MT + mt) * MC_BM), "r"(sz_smem_addr(&S->raw_full))
+                                 : "memory");
             }
+        __syncwarp();
     } else if (warp == LAST + 1) {
         // ---- issue: one thread, descriptors of the ring's first stage made once (a step is 256 cycles of the tensor core
         // at 256 tokens and MT = 1: what this thread does besides its instructions is on the path)
@@ -307,7 +309,7 @@ sz_mma_cols_q8_kernel(const __grid_constant__ CUtensorMap wmap, const McArgs a) 
         int k0 = 0, n = 0, np = 0;
         for (int u = u0; u < units && !failed; u += us, n++) {
             for (int p = 0; p < pieces && !failed; p++, np++, k0 += MC_STEPS) {
-                if (!sz_mbar_wait(&S->raw_full, np & 1, MC_WAIT)) { failed = 4; break; }
+                if (!mc_wait_warp(&S->raw_full, np & 1)) { failed = 4; break; }
                 u32 W[NW * 4];
                 const uint4* rp = (const uint4*)(raw + (size_t)r * MC_RAW_ROW + mc_group_start<G>(g));
 #pragma unroll
@@ -317,7 +319,7 @@ sz_mma_cols_q8_kernel(const __grid_constant__ CUtensorMap wmap, const McArgs a) 
                     constexpr int i = decltype(I)::value;
                     const int k = k0 + i * G + g, st = k % MC_STAGES;
                     if (failed) return;
-                    if (k >= MC_STAGES && !sz_mbar_wait(&S->empty[st], ((k / MC_STAGES) - 1) & 1, MC_WAIT)) { failed = 3; return; }
+                    if (k >= MC_STAGES && !mc_wait_warp(&S->empty[st], ((k / MC_STAGES) - 1) & 1)) { failed = 3; return; }
                     mc_decode_of<G, i>(g, W, dst0 + st * MT * MC_A_BYTES);
                     mc_fence_async();                 // every lane's stores, before the tensor core reads them through the async proxy:
                     mc_arrive_warp(&S->full[st]);     // fence, warp, arrival; the issuing thread waits and goes through tcgen05.fence
@@ -325,11 +327,10 @@ sz_mma_cols_q8_kernel(const __grid_constant__ CUtensorMap wmap, const McArgs a) 
                 step(McInt<0>()); step(McInt<1>());
                 if constexpr (G == 2) { step(McInt<2>()); step(McInt<3>()); }
             }
-            if (!failed && !sz_mbar_wait(&S->acc_full, n & 1, MC_WAIT)) failed = 6;
-            const int any = __any_sync(0xffffffffu, failed);
+            if (!failed && !mc_wait_warp(&S->acc_full, n & 1)) failed = 6;
             mc_tc_fence_after();
             if (a.ks == 1) {
-                if (!any) {
+                if (!failed) {
                     for (int t = part; t < MT * (nt / 16); t += 4) {
                         u32 v[16];
                         const int mt = MT == 2 && t >= nt / 16, c = (t - mt * (nt / 16)) * 16;
@@ -346,7 +347,7 @@ sz_mma_cols_q8_kernel(const __grid_constant__ CUtensorMap wmap, const McArgs a) 
             const int nu = nt / 16;
             auto unit0 = [&](int rank) { return nu * rank / a.ks; };   // the 16-column units a block finishes
             mc_cluster_sync();           // every block of the cluster is done with its stages: they take the other blocks' parts
-            if (!any)
+            if (!failed)
                 for (int o = 0; o < a.ks; o++) {
                     if (o == kr) continue;
                     const int c0 = unit0(o), cn = unit0(o + 1) - c0, slot = kr < o ? kr : kr - 1;
@@ -363,7 +364,7 @@ sz_mma_cols_q8_kernel(const __grid_constant__ CUtensorMap wmap, const McArgs a) 
                     }
                 }
             mc_cluster_sync();           // .. which are here now
-            if (!any) {
+            if (!failed) {
                 const int c0 = unit0(kr), cn = unit0(kr + 1) - c0;
                 for (int t = part; t < MT * cn; t += 4) {
                     u32 v[16];
