@@ -1102,6 +1102,9 @@ static SzRowsScratch sz_rows_layout(const sz_moe_layer* L, int cap) {
     return s;
 }
 
+// The error word of the expert kernels (bit 0: a bounded wait ran out, bit 2: an expert id out of range), after the chunks' blocks.
+static u32* sz_rows_err(u8* ctrl, int cap) { return (u32*)ctrl + 16 * (cap / 8) + 1; }
+
 template <int K, int TW>
 static int sz_rows_experts(cudaStream_t st, const sz_moe_layer* L, int slots, const SzRowsPlan* P, const float* x, u8* base, const SzRowsScratch& S, u32* err) {
     using X = SzRowsX<K, TW>;
@@ -1145,7 +1148,7 @@ static int sz_rows_run(const sz_moe_layer* L, uint64_t x, int rows, int live, ui
     const int H = L->hidden, chunks = rows / 8;
     const bool shared = L->shared_ff > 0;
     u32* ctrl = (u32*)(base + S.ctrl);
-    u32* err = ctrl + 16 * (cap / 8) + 1;
+    u32* err = sz_rows_err(base + S.ctrl, cap);
     float* logits = (float*)(base + S.logits);
     int32_t* ridx = (int32_t*)(base + S.ridx);
     double* rw = (double*)(base + S.rw);
@@ -1171,7 +1174,7 @@ static int sz_rows_run(const sz_moe_layer* L, uint64_t x, int rows, int live, ui
     static bool set = false;
     if (!set) { SZ_CUDA(cudaFuncSetAttribute(sz_rows_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SZ_MAX_EXPERTS * (SZ_ROWS_CAP / 32) * 4)); set = true; }
     SZ_CUDA(sz_launch("rows_plan", sz_rows_plan_kernel, dim3(1), dim3(1024), pmem, st, true, (const int32_t*)ridx, live, (int)L->top_k, (int)L->n_expert,
-                      shared ? 1 : 0, 2 * (H / 128), H / 128, H / 512 * (L->expert_ff / 128), (int)L->expert_ff / 128, sz_rows_grid(), P));
+                      shared ? 1 : 0, 2 * (H / 128), H / 128, H / 512 * (L->expert_ff / 128), (int)L->expert_ff / 128, sz_rows_grid(), P, err));
     const int slots = live * (L->top_k + (shared ? 1 : 0));
     rc = SZ_E_TYPE;
 #define SZ_ROWS_K(KK)                                                                                                                              \
@@ -1213,6 +1216,7 @@ int sz_moe_rows_clear(const sz_moe_layer* L, int room, uint64_t scratch, uint64_
     SZ_CUDA(cudaMemsetAsync((u8*)scratch + S.ctrl, 0, (size_t)(S.logits - S.ctrl), (cudaStream_t)stream));
     return SZ_OK;
 }
+u32* sz_moe_rows_err(const sz_moe_layer* L, int room, uint64_t scratch) { return sz_rows_err((u8*)scratch + sz_rows_layout(L, sz_rows_cap(room)).ctrl, sz_rows_cap(room)); }
 int sz_moe_rows_live(const sz_moe_layer* L, uint64_t x, int rows, int live, int room, uint64_t y, uint64_t scratch, int64_t scratch_bytes, uint64_t stream) {
     return sz_rows_run(L, x, rows, live, y, 0, 0, scratch, scratch_bytes, sz_rows_cap(room), stream);
 }
@@ -1231,10 +1235,10 @@ extern "C" int sz_moe_rows_status(const sz_moe_layer* L, int rows, uint64_t scra
     if (!code) { SZ_CUDA(cudaMemsetAsync(base + S.ctrl, 0, (size_t)(S.logits - S.ctrl), st)); return SZ_OK; }
     u32 err = 0;
     int32_t over = 0;
-    SZ_CUDA(cudaMemcpyAsync(&err, base + S.ctrl + 64 * (SZ_ROWS_MAX / 8) + 4, 4, cudaMemcpyDeviceToHost, st));
+    SZ_CUDA(cudaMemcpyAsync(&err, sz_rows_err(base + S.ctrl, SZ_ROWS_MAX), 4, cudaMemcpyDeviceToHost, st));
     SZ_CUDA(cudaMemcpyAsync(&over, base + S.plan + offsetof(SzRowsPlan, overflow), 4, cudaMemcpyDeviceToHost, st));
     SZ_CUDA(cudaStreamSynchronize(st));
-    *code = (int)(err ? 1 : 0) | (over & 4);
+    *code = (int)(err & 1) | (over & 4);
     return SZ_OK;
 }
 

@@ -56,7 +56,7 @@ __device__ __forceinline__ int sz_rows_weight(int n) { return 64 + n + (n > 8 ? 
 // are prefix sums over the experts, one a thread.  Dynamic shared memory: the masks, [experts][SZ_ROWS_CAP / 32] words.
 __global__ void __launch_bounds__(1024)
 sz_rows_plan_kernel(const int32_t* __restrict__ ridx, int R, int k, int ne, int has_shared, int upg_gu, int ns, int upg_dn, int kb, int grid,
-                    SzRowsPlan* __restrict__ P) {
+                    SzRowsPlan* __restrict__ P, u32* __restrict__ err) {
     extern __shared__ u32 mask[];
     __shared__ int slot_of[SZ_MAX_EXPERTS], grp_of[SZ_MAX_EXPERTS];
     __shared__ int wsum[2][32];
@@ -132,7 +132,7 @@ sz_rows_plan_kernel(const int32_t* __restrict__ ridx, int R, int k, int ne, int 
     __syncthreads();
     for (int p = t; p < pairs; p += 1024) {
         const int e = __ldcg(ridx + p), row = p / k;
-        if ((unsigned)e >= (unsigned)ne) { P->pair_loc[p] = 0; P->overflow = 4; continue; }   // an expert id out of range: the call is reported as failed
+        if ((unsigned)e >= (unsigned)ne) { P->pair_loc[p] = 0; P->overflow = 4; atomicOr(err, 4u); continue; }   // an expert id out of range: the call is reported as failed (the flag is this call's, the word stays)
         int n = __popc(mask[e * MW + (row >> 5)] & ((1u << (row & 31)) - 1u));
         for (int q = 0; q < (row >> 5); q++) n += __popc(mask[e * MW + q]);
         const int slot = slot_of[e] + n;

@@ -36,6 +36,7 @@ extern "C" int sz_ep_p2p_world(void);
 int sz_moe_rows_room(const sz_moe_layer* L, int room, int64_t* bytes);
 int sz_moe_rows_clear(const sz_moe_layer* L, int room, uint64_t scratch, uint64_t stream);
 int sz_moe_rows_live(const sz_moe_layer* L, uint64_t x, int rows, int live, int room, uint64_t y, uint64_t scratch, int64_t scratch_bytes, uint64_t stream);   // sz_moe.cu
+u32* sz_moe_rows_err(const sz_moe_layer* L, int room, uint64_t scratch);
 bool sz_moe_rows_takes(const sz_moe_layer* L);
 static int sz_batch_scratch_clear(const sz_model* m, int rows_max, uint64_t scratch, uint64_t stream);
 
@@ -1362,7 +1363,8 @@ extern "C" int sz_session_result(sz_session* s, int32_t* keep_next, uint32_t* to
         if (hrc) return hrc;
         SZ_CUDA(cudaMemcpyAsync(s->h_pin + 12, (const void*)at, 4, cudaMemcpyDeviceToHost, st));
     }
-    // the error words the kernels raise when one of their bounded waits runs out: [10] the session's kernels, [11] the MoE kernels
+    // the error words the kernels raise when one of their bounded waits runs out: [10] the session's kernels (and what the kernels of a
+    // step over many rows raised, a prompt's chunks among them), [11] the MoE kernels of a pass
     SZ_CUDA(cudaMemcpyAsync(s->h_pin + 10, s->state + 2, 4, cudaMemcpyDeviceToHost, st));
     SZ_CUDA(cudaMemcpyAsync(s->h_pin + 11, s->moe_scratch + 4, 4, cudaMemcpyDeviceToHost, st));
     SZ_CUDA(cudaStreamSynchronize(st));
@@ -1526,9 +1528,17 @@ SzIssuePool& sz_issue_pool() {
 struct SzBatchTab {
     const float* u[SZ_BATCH_MAX];
     float* y[SZ_BATCH_MAX];
+    int32_t* state[SZ_BATCH_MAX];
     int32_t m[SZ_BATCH_MAX], off[SZ_BATCH_MAX];
     int32_t n, pad[3];
 };
+// What a kernel over all rows raised becomes every sequence's own (sz_rows_commit_kernel's part of it).  One block.
+static __global__ void sz_batch_errors_kernel(const SzBatchTab* __restrict__ T, u32* __restrict__ err) {
+    const u32 e = __ldcg(err);
+    if (e && (int)threadIdx.x < T->n) atomicOr((u32*)T->state[threadIdx.x] + 2, e);
+    __syncthreads();
+    if (e && threadIdx.x == 0) *err = 0u;
+}
 // grid (rows), block 256: dir 0: X[off_b + j] = u_b[j]; dir 1: y_b[j] = Y[off_b + j]
 static __global__ void __launch_bounds__(256)
 sz_batch_rows_kernel(const SzBatchTab* __restrict__ T, float* __restrict__ X, int H, int dir) {
@@ -1668,21 +1678,21 @@ static bool sz_rows_fits(const sz_session* s) {
 struct SzAttnBatch { int row0, rows, g0[4], ng[3], splits[3]; };   // rows that attend in one go: their groups by size of the queries (16, 32, 64)
 
 template <int HD, int NQT>
-static int sz_rows_attn_go(cudaStream_t st, const sz_model_config& c, const float* aq, int splits, const SzSeqDev* seqs, const SzAttnGroup* groups, int ng, int ai, u32* err) {
+static int sz_rows_attn_go(cudaStream_t st, const sz_model_config& c, const float* aq, int splits, const SzSeqDev* seqs, const SzAttnGroup* groups, int ng, int ai) {
     static bool set = false;
     const size_t smem = (size_t)SzAttn2<HD, NQT>::SMEM;
     if (!set) { SZ_CUDA(cudaFuncSetAttribute(sz_attn2_kernel<HD, NQT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); set = true; }
     SZ_CUDA(sz_launch("rows_attention", sz_attn2_kernel<HD, NQT>, dim3(c.n_kv_head, splits, ng), dim3(32 * SzAttn2<HD, NQT>::NW), smem, st, true, aq, (const u8*)nullptr, (const u8*)nullptr,
-                      (int)c.n_head, (int)c.n_kv_head, 0, 0, (const int32_t*)nullptr, 0, (float*)nullptr, err, (const SzTree*)nullptr, (const int32_t*)nullptr,
+                      (int)c.n_head, (int)c.n_kv_head, 0, 0, (const int32_t*)nullptr, 0, (float*)nullptr, (u32*)nullptr, (const SzTree*)nullptr, (const int32_t*)nullptr,
                       (const int32_t*)nullptr, 0, 0, seqs, groups, ai));
     return SZ_OK;
 }
 template <int HD>
-static int sz_rows_attn(cudaStream_t st, const sz_model_config& c, const float* aq, const SzAttnBatch& B, const SzSeqDev* seqs, const SzAttnGroup* groups, int ai, u32* err) {
+static int sz_rows_attn(cudaStream_t st, const sz_model_config& c, const float* aq, const SzAttnBatch& B, const SzSeqDev* seqs, const SzAttnGroup* groups, int ai) {
     int rc = SZ_OK;
-    if (B.ng[0] && (rc = sz_rows_attn_go<HD, 1>(st, c, aq, B.splits[0], seqs, groups + B.g0[0], B.ng[0], ai, err))) return rc;
-    if (B.ng[1] && (rc = sz_rows_attn_go<HD, 2>(st, c, aq, B.splits[1], seqs, groups + B.g0[1], B.ng[1], ai, err))) return rc;
-    if (B.ng[2] && (rc = sz_rows_attn_go<HD, 4>(st, c, aq, B.splits[2], seqs, groups + B.g0[2], B.ng[2], ai, err))) return rc;
+    if (B.ng[0] && (rc = sz_rows_attn_go<HD, 1>(st, c, aq, B.splits[0], seqs, groups + B.g0[0], B.ng[0], ai))) return rc;
+    if (B.ng[1] && (rc = sz_rows_attn_go<HD, 2>(st, c, aq, B.splits[1], seqs, groups + B.g0[1], B.ng[1], ai))) return rc;
+    if (B.ng[2] && (rc = sz_rows_attn_go<HD, 4>(st, c, aq, B.splits[2], seqs, groups + B.g0[2], B.ng[2], ai))) return rc;
     return SZ_OK;
 }
 
@@ -1706,8 +1716,6 @@ static int sz_rows_layers(sz_session* const* ss, int n, const int32_t* ids, cons
     SzAttnGroup* hg = (SzAttnGroup*)(up.data() + (S.groups - S.up));
     int32_t* hi = (int32_t*)(up.data() + (S.rids - S.up));
     memcpy(hi, ids, (size_t)R * 4);
-    const int64_t d2 = (int64_t)c.ssm_head_dim * c.ssm_head_dim;
-    (void)d2;
     int row = 0;
     for (int b = 0; b < n; b++) {
         sz_session* s = ss[b];
@@ -1785,13 +1793,15 @@ static int sz_rows_layers(sz_session* const* ss, int n, const int32_t* ids, cons
         }
         return SZ_OK;
     };
-    u32* err = (u32*)(s0->state + 2);
+    // the step's error word: what a kernel over the rows of all sequences raises (attention raises its sequence's own)
+    u32* err = sz_moe_rows_err(&s0->layers[0].moe, rows_max, (uint64_t)(base + S.moe));
     int hn = 0, rc;
     for (int l = 0; l < c.n_layer; l++) {
         const sz_layer& L = s0->layers[l];
         if ((rc = sz_hc_read_rows(s0, st, L.hc_attn, Rp, hn++, l > 0, true, BB, true))) return rc;
         SzDenseArgs a, o;
         sz_mixer_args(s0, l, 8, &a, &o);
+        a.err = o.err = err;
         float* outs[SZ_DENSE_MAX_JOBS];
         int64_t at = 0;
         for (int k = 0; k < a.n_jobs; k++) { outs[k] = IN + at; at += (int64_t)Rp * a.job[k].ostride; }
@@ -1802,8 +1812,8 @@ static int sz_rows_layers(sz_session* const* ss, int n, const int32_t* ids, cons
                               (const float*)outs[2], (const float*)L.attn_q_norm.data, (const float*)L.attn_k_norm.data, nh, nkv, hd, 0, c.eps, (const int32_t*)nullptr,
                               (int)c.rope_dims, (const double*)s0->rope_den, 1, (u8*)nullptr, (u8*)nullptr, AQ, (const SzTree*)nullptr, seqs, rws, ai));
             for (const SzAttnBatch& B : ab) {
-                rc = hd == 64 ? sz_rows_attn<64>(st, c, AQ, B, seqs, groups, ai, err)
-                              : (hd == 128 ? sz_rows_attn<128>(st, c, AQ, B, seqs, groups, ai, err) : sz_rows_attn<256>(st, c, AQ, B, seqs, groups, ai, err));
+                rc = hd == 64 ? sz_rows_attn<64>(st, c, AQ, B, seqs, groups, ai)
+                              : (hd == 128 ? sz_rows_attn<128>(st, c, AQ, B, seqs, groups, ai) : sz_rows_attn<256>(st, c, AQ, B, seqs, groups, ai));
                 if (rc) return rc;
                 SZ_CUDA(sz_launch("rows_attn_merge", sz_attn_merge_kernel, dim3(nh, B.rows), dim3(256), 0, st, true, (const float*)nullptr,
                                   (const float*)(outs[0] + (int64_t)B.row0 * 2 * nh * hd), nh, hd, 0, CORE + (int64_t)B.row0 * nh * hd, rws + B.row0));
@@ -1823,9 +1833,7 @@ static int sz_rows_layers(sz_session* const* ss, int n, const int32_t* ids, cons
         if ((rc = sz_moe_rows_live(&L.moe, (uint64_t)X, Rp, R, rows_max, (uint64_t)Y, (uint64_t)(base + S.moe), S.moe_bytes, (uint64_t)st))) return rc;
     }
     if (read_out && (rc = sz_hc_read_rows(s0, st, s0->model.output_hc, Rp, hn++, true, false, BB, true))) return rc;
-    bool any_all = false;
-    for (int b = 0; b < n; b++) any_all = any_all || all[b];
-    if (any_all) SZ_CUDA(sz_launch("rows_commit", sz_rows_commit_kernel, dim3(1), dim3(SZ_BATCH_MAX), 0, st, true, seqs, n));
+    SZ_CUDA(sz_launch("rows_commit", sz_rows_commit_kernel, dim3(1), dim3(SZ_BATCH_MAX), 0, st, true, seqs, n, err));
     return SZ_OK;
 }
 
@@ -1917,7 +1925,7 @@ static int sz_batch_step(sz_session* const* ss, int n, const int32_t* ids, const
         if (s->last_m) return sz_fail(SZ_E_ARG, "sequence %d: the previous pass was not committed", b);
         if (s->len + m > s->ctx) return sz_fail(SZ_E_ARG, "sequence %d: %d positions + %d rows exceed the session's capacity %d", b, s->len, m, s->ctx);
         if (s->want_routes) return sz_fail(SZ_E_ARG, "sz_batch_verify: no routing trace in a batched step");
-        tab.u[b] = s->u; tab.y[b] = s->y; tab.m[b] = m; tab.off[b] = R;
+        tab.u[b] = s->u; tab.y[b] = s->y; tab.state[b] = s->state; tab.m[b] = m; tab.off[b] = R;
         R += m;
     }
     tab.n = n;
@@ -2081,6 +2089,7 @@ static int sz_batch_step(sz_session* const* ss, int n, const int32_t* ids, const
     if ((rc = each([&](int b) { return sz_forward_begin(ss[b], sq(b), ms[b], !shared); }))) return rc;
     bool pending = false;
     const SzBatchTab* T = (const SzBatchTab*)(base + S.tab);
+    u32* err = sz_moe_rows_err(&s0->layers[0].moe, rows_max, scratch + S.moe);   // the step's, as in sz_rows_layers
     if (shared) {
         int hn = 0;   // hyper-connection reads so far (every session's count follows: the per-layer embedding looks at it)
         auto read_rows = [&](const sz_hc& hc, bool pend, bool inject, bool pdl) -> int {
@@ -2103,6 +2112,7 @@ static int sz_batch_step(sz_session* const* ss, int n, const int32_t* ids, const
             float* const* lp = ptrs + (size_t)l * SZ_BATCH_SLOTS * SZ_BATCH_MAX;
             SzDenseArgs a, o;
             sz_mixer_args(s0, l, 8, &a, &o);
+            a.err = o.err = err;
             SzBatchMove mi = {}, mo = {};
             long long at_in = 0;
             for (int k = 0; k < a.n_jobs; k++) { mi.off[k] = at_in; mi.width[k] = a.job[k].ostride; at_in += (long long)Rp * a.job[k].ostride; }
@@ -2162,6 +2172,7 @@ static int sz_batch_step(sz_session* const* ss, int n, const int32_t* ids, const
             pending = true;
         }
     }
+    SZ_CUDA(sz_launch("batch_errors", sz_batch_errors_kernel, dim3(1), dim3(SZ_BATCH_MAX), 0, st, false, T, err));
     if ((rc = each([&](int b) {
             sz_session* s = ss[b];
             int r = heads[b] ? sz_forward_head(s, sq(b), ms[b], pending, !shared) : SZ_OK;

@@ -1248,7 +1248,7 @@ sz_attn2_kernel(const float* __restrict__ qin, const u8* __restrict__ kc, const 
                 const int32_t* __restrict__ glist, const int32_t* __restrict__ gcount, int gstride, int ratio, const SzSeqDev* __restrict__ seqs,
                 const SzAttnGroup* __restrict__ groups, int ai) {
     // groups != null: a step of many rows, grid (kv heads, most splits, groups): up to 8 consecutive rows of one sequence, as a pass of
-    // that sequence at committed + j0 would carry them.
+    // that sequence at committed + j0 would carry them (and a wait that runs out is that sequence's).
     // glist != null: the sparse form, grid (kv heads, splits, rows).  The block serves ONE row (blockIdx.z) and walks that row's list
     // of position groups (`ratio` positions each; row j's list at glist + j * gstride, gcount[j] long) instead of the positions
     // themselves.  A chunk of 64 list positions is then 64 / ratio copies of a group each for K and for V.
@@ -1277,6 +1277,7 @@ sz_attn2_kernel(const float* __restrict__ qin, const u8* __restrict__ kc, const 
         kc = sq.kc + (size_t)ai * sq.kv_layer; vc = sq.vc + (size_t)ai * sq.kv_layer;
         qin += (size_t)gr.row0 * nh * HD;
         part = gr.part;
+        err = (u32*)const_cast<int32_t*>(sq.state) + 2;
     }
     const int jz = sparse ? (int)blockIdx.z : 0;   // sparse: the one row of this block
     if (sparse) { glist += (size_t)jz * gstride; m = 1; }

@@ -399,16 +399,23 @@ sz_rows_scan_kernel(const SzSeqDev* __restrict__ seqs, int di, const float* __re
     sz_delta_scan_body<D, 32>(q, norm_w, kh, vh, eps, (const SzTree*)nullptr, (float*)nullptr, (int)blockIdx.x / (D / 32), (int)blockIdx.x % (D / 32), 0);
 }
 
-// After a step: the sequences whose rows were all kept move on.  One block.
-__global__ void sz_rows_commit_kernel(const SzSeqDev* __restrict__ seqs, int n) {
+// After a step: the sequences whose rows were all kept move on, and what a kernel over all rows raised in the step's error word becomes
+// every sequence's own (it stays there until the session is reset; the step's word is ready for whoever has the room next).  One block.
+__global__ void sz_rows_commit_kernel(const SzSeqDev* __restrict__ seqs, int n, u32* __restrict__ err) {
     sz_pdl_wait();
     sz_pdl_trigger();
     const int b = threadIdx.x;
-    if (b < n && seqs[b].all) {
+    const u32 e = __ldcg(err);
+    if (b < n) {
         int32_t* state = const_cast<int32_t*>(seqs[b].state);
-        state[0] += seqs[b].m;
-        state[1] ^= 1;
+        if (e) atomicOr((u32*)state + 2, e);
+        if (seqs[b].all) {
+            state[0] += seqs[b].m;
+            state[1] ^= 1;
+        }
     }
+    __syncthreads();
+    if (b == 0 && e) *err = 0u;
 }
 
 #endif

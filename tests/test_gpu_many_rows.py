@@ -1,6 +1,8 @@
 """The forms that take many rows at once, at the sizes where they could go wrong: one row more or less than a tile, a chunk, a block's
 group; the smallest and largest of their ranges.  A session's rows are bit for bit those of passes of up to 8 rows; a block-format expert
 layer and the tensor-core projections are held against the CPU restatement."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -93,3 +95,48 @@ def test_prompts_of_a_batch_in_one_sessions_room_or_in_the_scratch(dm, lens, whi
             s.verify([5, 6, 7])
         assert np.array_equal(batch.sessions[b].top[2].view(np.uint32), alone.top[2].view(np.uint32)), "prompt %d" % b
         assert np.array_equal(batch.sessions[b].result(logits=True)[2].view(np.uint32), alone.result(logits=True)[2].view(np.uint32)), "after prompt %d" % b
+
+
+def raise_error(dm, mem, addr, size):
+    """Sets the error word of a room for up to 256 rows that ends `size` bytes after `addr` (its MoE scratch lies last: 64 bytes of
+    counters a block of 8 rows, then the word), as an expert kernel whose wait ran out would."""
+    n = C.c_int64()
+    szlib.check(szlib.load().sz_moe_rows_scratch_bytes(C.byref(dm.model.layers[0].moe), 256, C.byref(n)))
+    at = addr - mem.data_ptr() + size - n.value + 64 * (256 // 8) + 4
+    word = mem[at:at + 4].view(torch.int32)
+    assert int(word) == 0
+    word.fill_(1)
+    torch.cuda.synchronize()
+    return word
+
+
+def test_a_wait_that_ran_out_in_a_prompts_chunk_is_reported(dm):
+    s = md.Session(dm, 128, kv_q8=True)
+    n = C.c_int64()
+    szlib.check(s.lib.sz_session_bytes(C.byref(dm.model), 128, s.flags, C.byref(n)))
+    word = raise_error(dm, s.mem, s.mem.data_ptr() + (-s.mem.data_ptr()) % 256, n.value)
+    s.prefill(md.make_prompt(60, CFG["vocab"], seed=90))
+    with pytest.raises(szlib.SzError) as e:
+        s.result()
+    assert e.value.code == szlib.E_DEVICE
+    assert int(word) == 0            # the session's now, until it is reset
+    s.reset()
+    s.prefill(md.make_prompt(60, CFG["vocab"], seed=90))
+    s.result()
+
+
+@pytest.mark.parametrize("shared", ["1", "0"])
+def test_a_wait_that_ran_out_in_a_step_is_reported_by_every_sequence(dm, monkeypatch, shared):
+    monkeypatch.setenv("SZ_BATCH_SHARED", shared)
+    batch = md.Batch(dm, 3, 64)
+    word = raise_error(dm, batch.mem, batch.scratch, batch.scratch_bytes)
+    batch.verify([[1, 2], [3], [4, 5, 6]])
+    for s in batch.sessions:
+        with pytest.raises(szlib.SzError) as e:
+            s.result()
+        assert e.value.code == szlib.E_DEVICE
+        s.reset()
+    assert int(word) == 0
+    batch.verify([[1, 2], [3], [4, 5, 6]])
+    for s in batch.sessions:
+        s.result()
