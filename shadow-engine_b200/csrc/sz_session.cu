@@ -2500,6 +2500,7 @@ const SzKernelEntry kKernels[] = {
     {"sz_topk_slices_kernel", (const void*)sz_topk_slices_kernel, 6, {SZ_P_CONST_PTR, SZ_P_I32, SZ_P_I32, SZ_P_I32, SZ_P_PTR, SZ_P_CONST_PTR}},
     {"sz_topk_merge_kernel", (const void*)sz_topk_merge_kernel, 3, {SZ_P_CONST_PTR, SZ_P_I32, SZ_P_PTR}},
     {"sz_batch_rows_kernel", (const void*)sz_batch_rows_kernel, 4, {SZ_P_CONST_PTR, SZ_P_PTR, SZ_P_I32, SZ_P_I32}},
+    {"sz_batch_errors_kernel", (const void*)sz_batch_errors_kernel, 2, {SZ_P_CONST_PTR, SZ_P_PTR}},
     {"sz_fill_kv_kernel", (const void*)sz_fill_kv_kernel, 8, {SZ_P_PTR, SZ_P_I32, SZ_P_I32, SZ_P_I32, SZ_P_U64, SZ_P_I32, SZ_P_I32, SZ_P_U32}},
 };
 const int kKernelCount = (int)(sizeof(kKernels) / sizeof(kKernels[0]));
