@@ -256,10 +256,9 @@ int sz_mma_cols_status(uint64_t scratch, int init, int* code, uint64_t stream);
 #define SZ_KV_Q8 1
 #define SZ_HEAD_PROXY 2     /* output.weight is an EXL3 blob and the head is screened by its 2-bit proxy (see sz_head below); without the
                              * flag an EXL3 output.weight is evaluated in full.  Blocks kept a row: 128, or the environment's SZ_HEAD_KBLK */
-#define SZ_SESSION_LEAN 4   /* the session keeps no room for the chunks of a prompt (up to 512 rows through a layer at once: some 400 MB at
-                             * the benchmark's shapes): its prompts come through sz_batch_prefill, with the batch's scratch, or in passes of 8 */
-#define SZ_SESSION_ROOM 8   /* the session's room for chunks is the full one whatever its capacity: sz_batch_prefill uses it for the prompts of
-                             * all sequences when one of them has it */
+#define SZ_SESSION_LEAN 4   /* no room of the session's own, which is also what a session without flags has (and what holds where SZ_SESSION_ROOM
+                             * is given too) */
+#define SZ_SESSION_ROOM 8   /* the session's block holds a room of its own (below), for SZ_ROOM_ROWS rows */
 #define SZ_ACCEPT_NONE 0    /* the caller decides: read the top-64 of every row, then sz_session_commit(keep) */
 #define SZ_ACCEPT_GREEDY 1  /* on the device: keep row i + 1 while row i's best token is the drafted ids[i + 1] (engine.rs:2377-2408) */
 #define SZ_ACCEPT_ALL 2     /* prompt rows: all kept */
@@ -273,8 +272,23 @@ int sz_session_reset(sz_session* s, uint64_t stream);
 int sz_session_len(const sz_session* s);        /* committed positions: GpuSession::tokens().len() */
 int sz_session_capacity(const sz_session* s);   /* GpuSession::capacity() */
 int sz_session_pending(const sz_session* s);    /* rows of the pass that awaits sz_session_commit (0: none) */
-/* Feeds a prompt in passes of up to SZ_MAX_VERIFY rows.  The last pass is left pending: read it with sz_session_result (its last
- * row is the prompt's last token), then sz_session_commit(s, rows of that pass). */
+/* A room is where the chunks of a prompt go: up to SZ_ROOM_ROWS rows through a layer at once instead of passes of 8 (six times as fast
+ * for 507 tokens; some 400 MB at the benchmark's shapes).  One serves all sessions of a model: a host makes it once, in memory of its own
+ * (256-byte aligned, valid as long as a session uses it), and gives it to every session it makes; or a session has one of its own
+ * (SZ_SESSION_ROOM).  Any thread may use its session's room at any time: prompts in one room follow one another on the GPU, and the
+ * launches of each are issued under the room's lock.  rows: a multiple of 8 from 16 to SZ_ROOM_ROWS.  sz_room_bytes gives 0 where
+ * the model's prompts go in passes whatever room there is (block-format or sharded experts, per-layer embeddings, the sparse indexer);
+ * sz_room_create refuses those.  sz_session_use_room(s, NULL) gives the session its own again (or none).  sz_room_destroy may come
+ * before the sessions' end: they keep what they use, the memory is the host's. */
+#define SZ_ROOM_ROWS 512
+typedef struct sz_room sz_room;
+int sz_room_bytes(const sz_model* model, int rows, int64_t* bytes);
+int sz_room_create(const sz_model* model, int rows, uint64_t mem, int64_t bytes, uint64_t stream, sz_room** out);
+void sz_room_destroy(sz_room* room);
+int sz_session_use_room(sz_session* s, sz_room* room);
+/* Feeds a prompt: in chunks where the session has a room, then (or else) in passes of up to SZ_MAX_VERIFY rows; the results are the same
+ * bits.  The last pass is left pending: read it with sz_session_result (its last row is the prompt's last token), then
+ * sz_session_commit(s, rows of that pass). */
 int sz_session_prefill(sz_session* s, const int32_t* ids, int n, uint64_t stream);
 /* One pass over ids[0..m): row i's output is what follows ids[..=i] (step_batch_verify).  want_head = 0 skips the output
  * projection (prompt passes).  Asynchronous; the pass stays pending until sz_session_commit. */

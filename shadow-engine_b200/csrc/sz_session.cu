@@ -13,6 +13,7 @@
 
 #include <cmath>
 #include <map>
+#include <memory>
 #include <new>
 #include <stdlib.h>
 #include <string.h>
@@ -40,6 +41,33 @@ u32* sz_moe_rows_err(const sz_moe_layer* L, int room, uint64_t scratch);
 bool sz_moe_rows_takes(const sz_moe_layer* L);
 static int sz_batch_scratch_clear(const sz_model* m, int rows_max, uint64_t scratch, uint64_t stream);
 
+// Room for the chunks of a prompt (sz_batch_layout's buffers for `rows` rows), a session's own or shared by sessions of a model.  A chunk
+// is launches on the session's stream, and the next user's stream waits for them; `mu` is held while they are issued.
+struct SzRoom {
+    int rows = 0;
+    uint64_t mem = 0;
+    int64_t bytes = 0;
+    const void* model = nullptr;      // which model's it is: the first layer's expert weights (as sz_batch_step tells models apart)
+    int n_layer = 0;
+    std::mutex mu;
+    cudaEvent_t done = nullptr;       // after the last user's launches
+    ~SzRoom() { if (done) cudaEventDestroy(done); }
+};
+struct sz_room { std::shared_ptr<SzRoom> r; };
+// From begin to the end of the scope the room is the caller's, for launches on `st`.
+struct SzRoomUse {
+    SzRoom* r = nullptr;
+    cudaStream_t st = 0;
+    std::unique_lock<std::mutex> lock;
+    int begin(SzRoom& room, cudaStream_t stream) {
+        lock = std::unique_lock<std::mutex>(room.mu);
+        SZ_CUDA(cudaStreamWaitEvent(stream, room.done, 0));
+        r = &room; st = stream;
+        return SZ_OK;
+    }
+    ~SzRoomUse() { if (r) cudaEventRecord(r->done, st); }
+};
+
 struct sz_session {
     sz_model model;
     std::vector<sz_layer> layers;
@@ -49,9 +77,7 @@ struct sz_session {
     int cur;          // which state buffer is current
     int last_m;       // rows of the last pass (0: none pending)
     int want_routes;
-    int ws_rows = 0;        // rows of a prompt's chunk the session has room for (0: prompts go in passes)
-    u8* ws = nullptr;
-    int64_t ws_bytes = 0;
+    std::shared_ptr<SzRoom> own_room, room;   // where a prompt's chunks go: its own room, or the one it was given (none: prompts go in passes)
     // device memory (all inside the caller's block)
     u8* base;
     int64_t bytes;
@@ -121,7 +147,7 @@ struct SzSessLayout {
     int64_t i_raw_layer, i_blocks_layer;   // bytes of one attention layer's raw-key and pooled-key caches
     int i_ctx_blocks, i_words;
     int64_t moe_bytes, S_bytes, conv_bytes, kv_bytes, head_work_bytes;
-    int splits, splits2, ws_rows;
+    int splits, splits2;
 };
 
 // output.weight as an EXL3 blob: the head is sz_head_top's (dense, or screened by the 2-bit proxy with SZ_HEAD_PROXY).
@@ -144,7 +170,7 @@ static int sz_head_describe(const sz_model* m, int flags, sz_head* h) {
 static int64_t up256(int64_t v) { return (v + 255) & ~(int64_t)255; }
 
 struct SzBatchScratch;
-static int sz_rows_ws_plan(const sz_model* m, int ctx, int flags, int* rows, int64_t* bytes);
+static int sz_room_make(const sz_model* m, int rows, uint64_t mem, int64_t bytes, uint64_t stream, std::shared_ptr<SzRoom>* out);
 
 static int sz_sess_layout(const sz_model* m, int ctx, int flags, SzSessLayout* L) {
     const sz_model_config& c = m->cfg;
@@ -241,12 +267,12 @@ static int sz_sess_layout(const sz_model* m, int ctx, int flags, SzSessLayout* L
             L->head_sc = take(sc);
         }
     }
-    // what a prompt's chunks need beside a pass's buffers
+    // a room of the session's own for a prompt's chunks, where it was asked for
     L->rows_ws = 0; L->rows_ws_bytes = 0;
-    int ws_rows = 0;
-    if ((hrc = sz_rows_ws_plan(m, ctx, flags, &ws_rows, &L->rows_ws_bytes))) return hrc;
-    L->ws_rows = ws_rows;
-    if (ws_rows > 0) L->rows_ws = take(L->rows_ws_bytes);
+    if ((flags & SZ_SESSION_ROOM) && !(flags & SZ_SESSION_LEAN) && (flags & SZ_KV_Q8)) {
+        if ((hrc = sz_room_bytes(m, SZ_ROOM_ROWS, &L->rows_ws_bytes))) return hrc;
+        L->rows_ws = take(L->rows_ws_bytes);
+    }
     L->total = o;
     return SZ_OK;
 }
@@ -460,8 +486,8 @@ extern "C" int sz_session_create(const sz_model* m, int ctx, int flags, uint64_t
         s->i_raw_layer = L.i_raw_layer; s->i_blocks_layer = L.i_blocks_layer; s->i_ctx_blocks = L.i_ctx_blocks; s->i_words = L.i_words;
     }
     s->attn_splits = L.splits; s->attn_splits2 = L.splits2;
-    s->ws_rows = L.ws_rows; s->ws = b + L.rows_ws; s->ws_bytes = L.rows_ws_bytes;
-    if (s->ws_rows > 0 && (rc = sz_batch_scratch_clear(&s->model, s->ws_rows, (uint64_t)s->ws, stream))) { delete s; return rc; }
+    if (L.rows_ws_bytes > 0 && (rc = sz_room_make(&s->model, SZ_ROOM_ROWS, (uint64_t)(b + L.rows_ws), L.rows_ws_bytes, stream, &s->own_room))) { delete s; return rc; }
+    s->room = s->own_room;
     if ((rc = sz_head_describe(m, flags, &s->head))) { delete s; return rc; }
     if (s->head.rows > 0) {
         s->head.work = (uint64_t)(b + L.head_work); s->head.work_bytes = L.head_work_bytes;
@@ -1636,7 +1662,7 @@ static int sz_batch_layout(const sz_model* m, int rows_max, SzBatchScratch* S) {
     S->total = o;
     return SZ_OK;
 }
-// What a caller's batch scratch may hold (a session's own, for its prompts' chunks, more: SZ_ROWS_CHUNK).
+// What a caller's batch scratch may hold (a room for prompts' chunks more: SZ_ROOM_ROWS).
 #define SZ_BATCH_ROWS 256
 static int sz_batch_rows_check(int rows_max) {
     return rows_max > SZ_BATCH_ROWS ? sz_fail(SZ_E_ARG, "sz_batch: rows_max = %d (a multiple of 8 up to %d)", rows_max, SZ_BATCH_ROWS) : SZ_OK;
@@ -2190,37 +2216,77 @@ static int sz_batch_step(sz_session* const* ss, int n, const int32_t* ids, const
     return join();
 }
 
-// Rows of a prompt's chunk a session of this model keeps room for: SZ_ROWS_CHUNK (the most the experts' plan holds: 507 tokens took 126.9 ms in
-// two chunks of up to 256 rows, 105.2 in one), or what its capacity holds where the room is not for a batch's prompts too
-// (SZ_SESSION_ROOM); 0 where sz_rows_layers does not run the model, or the host said that prompts come through sz_batch_prefill
-// (SZ_SESSION_LEAN).
-#define SZ_ROWS_CHUNK 512
-static int sz_rows_ws_plan(const sz_model* m, int ctx, int flags, int* rows, int64_t* bytes) {
+// Room for prompts' chunks: of up to SZ_ROOM_ROWS rows, the most the experts' plan holds (507 tokens took 126.9 ms in two chunks of up to 256
+// rows, 105.2 in one), for models that sz_rows_layers runs.
+static_assert(SZ_ROOM_ROWS == 512, "the rows of the experts' plan");
+static bool sz_rows_takes_model(const sz_model* m) {
     const sz_model_config& c = m->cfg;
-    *rows = 0; *bytes = 0;
-    if ((flags & SZ_SESSION_LEAN) || !(flags & SZ_KV_Q8) || m->ple.ngram >= 2 || c.idx_heads > 0 || c.n_head / c.n_kv_head * SZ_MAX_VERIFY > 64) return SZ_OK;
+    if (m->ple.ngram >= 2 || c.idx_heads > 0 || c.n_kv_head < 1 || c.n_head / c.n_kv_head * SZ_MAX_VERIFY > 64) return false;
     for (int l = 0; l < c.n_layer; l++)
-        if (!sz_moe_rows_takes(&m->layers[l].moe)) return SZ_OK;
-    const int want = ctx < SZ_ROWS_CHUNK && !(flags & SZ_SESSION_ROOM) ? ctx / SZ_MAX_VERIFY * SZ_MAX_VERIFY : SZ_ROWS_CHUNK;
-    if (want < 2 * SZ_MAX_VERIFY) return SZ_OK;
+        if (!sz_moe_rows_takes(&m->layers[l].moe)) return false;
+    return true;
+}
+extern "C" int sz_room_bytes(const sz_model* m, int rows, int64_t* bytes) {
+    const int crc = sz_model_check(m);
+    if (crc) return crc;
+    if (!bytes) return sz_fail(SZ_E_ARG, "sz_room_bytes: null argument");
+    if (rows < 2 * SZ_MAX_VERIFY || rows > SZ_ROOM_ROWS || rows % SZ_MAX_VERIFY)
+        return sz_fail(SZ_E_ARG, "sz_room: rows = %d (a multiple of %d from %d to %d)", rows, SZ_MAX_VERIFY, 2 * SZ_MAX_VERIFY, SZ_ROOM_ROWS);
+    *bytes = 0;
+    if (!sz_rows_takes_model(m)) return SZ_OK;
     SzBatchScratch S;
-    const int rc = sz_batch_layout(m, want, &S);
+    const int rc = sz_batch_layout(m, rows, &S);
+    if (!rc) *bytes = S.total;
+    return rc;
+}
+static int sz_room_make(const sz_model* m, int rows, uint64_t mem, int64_t bytes, uint64_t stream, std::shared_ptr<SzRoom>* out) {
+    std::shared_ptr<SzRoom> r(new (std::nothrow) SzRoom());
+    if (!r) return sz_fail(SZ_E_ARG, "out of host memory");
+    r->rows = rows; r->mem = mem; r->bytes = bytes;
+    r->model = (const void*)m->layers[0].moe.gate; r->n_layer = m->cfg.n_layer;
+    SZ_CUDA(cudaEventCreateWithFlags(&r->done, cudaEventDisableTiming));
+    const int rc = sz_batch_scratch_clear(m, rows, mem, stream);
     if (rc) return rc;
-    *rows = want; *bytes = S.total;
+    SZ_CUDA(cudaEventRecord(r->done, (cudaStream_t)stream));
+    *out = r;
+    return SZ_OK;
+}
+extern "C" int sz_room_create(const sz_model* m, int rows, uint64_t mem, int64_t bytes, uint64_t stream, sz_room** out) {
+    int64_t need = 0;
+    int rc = sz_room_bytes(m, rows, &need);
+    if (rc) return rc;
+    if (need == 0) return sz_fail(SZ_E_TYPE, "sz_room_create: the prompts of this model go in passes, they need no room");
+    if (!out || !mem || (mem & 255)) return sz_fail(SZ_E_ARG, "sz_room_create: memory must be 256-byte aligned");
+    if (bytes < need) return sz_fail(SZ_E_SCRATCH, "sz_room_create: %lld bytes given, %lld needed", (long long)bytes, (long long)need);
+    sz_room* h = new (std::nothrow) sz_room();
+    if (!h) return sz_fail(SZ_E_ARG, "out of host memory");
+    if ((rc = sz_room_make(m, rows, mem, bytes, stream, &h->r))) { delete h; return rc; }
+    *out = h;
+    return SZ_OK;
+}
+extern "C" void sz_room_destroy(sz_room* r) { delete r; }
+extern "C" int sz_session_use_room(sz_session* s, sz_room* r) {
+    if (!s) return sz_fail(SZ_E_ARG, "null session");
+    if (r && (r->r->model != (const void*)s->layers[0].moe.gate || r->r->n_layer != s->model.cfg.n_layer))
+        return sz_fail(SZ_E_ARG, "sz_session_use_room: the room was made for another model");
+    s->room = r ? r->r : s->own_room;
     return SZ_OK;
 }
 // The first `body` tokens (whole passes' worth) of a prompt in chunks of equal size: *done of them, 0 when the session's prompts go in
 // passes.  A chunk costs little more for more rows (every expert's decode is the most of it), so chunks are as long as there is room.
 static int sz_prefill_chunks(sz_session* s, const int32_t* ids, int body, uint64_t stream, int* done) {
     sz_session* const one[1] = {s};
-    if (s->ws_rows == 0 || body < 2 * SZ_MAX_VERIFY || s->last_m || s->len + body > s->ctx || !sz_rows_step_fits(one, 1)) return SZ_OK;
-    const int chunks = (body + s->ws_rows - 1) / s->ws_rows;
+    if (!s->room || body < 2 * SZ_MAX_VERIFY || s->last_m || s->len + body > s->ctx || !sz_rows_step_fits(one, 1)) return SZ_OK;
+    const std::shared_ptr<SzRoom> room = s->room;
+    SzRoomUse use;
+    int rc = use.begin(*room, (cudaStream_t)stream);
+    if (rc) return rc;
+    const int chunks = (body + room->rows - 1) / room->rows;
     const int size = ((body + chunks - 1) / chunks + SZ_MAX_VERIFY - 1) / SZ_MAX_VERIFY * SZ_MAX_VERIFY;
     while (*done < body) {
         const int32_t m = body - *done < size ? body - *done : size;
         const int accept = SZ_ACCEPT_ALL, head = 0;
-        const int rc = sz_batch_step(one, 1, ids + *done, &m, &accept, &head, -1, s->ws_rows, (uint64_t)s->ws, s->ws_bytes, stream);
-        if (rc) return rc;
+        if ((rc = sz_batch_step(one, 1, ids + *done, &m, &accept, &head, -1, room->rows, room->mem, room->bytes, stream))) return rc;
         *done += m;
     }
     return SZ_OK;
@@ -2249,9 +2315,16 @@ extern "C" int sz_batch_prefill(sz_session* const* ss, int n, const int32_t* con
     const bool chunks = sz_rows_step_fits(ss, n);
     // a step of twice the rows costs half as much again (every expert's decode is the most of it): where one of the sessions has more room
     // than the scratch, the steps take that (16 prompts of 75 tokens: 10 steps of 128 rows or 3 of up to 512)
+    std::shared_ptr<SzRoom> room;
+    SzRoomUse use;
     if (chunks)
         for (int b = 0; b < n; b++)
-            if (ss[b]->ws_rows > rows_max) { rows_max = ss[b]->ws_rows; scratch = (uint64_t)ss[b]->ws; scratch_bytes = ss[b]->ws_bytes; }
+            if (ss[b]->room && ss[b]->room->rows > (room ? room->rows : rows_max)) room = ss[b]->room;
+    if (room) {
+        const int urc = use.begin(*room, (cudaStream_t)stream);
+        if (urc) return urc;
+        rows_max = room->rows; scratch = room->mem; scratch_bytes = room->bytes;
+    }
     for (;;) {
         sz_session* step_s[SZ_BATCH_MAX];
         int32_t step_m[SZ_BATCH_MAX];

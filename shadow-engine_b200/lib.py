@@ -82,6 +82,10 @@ SYMBOLS = {
     "sz_session_create": (C.c_int, [C.c_void_p, C.c_int, C.c_int, C.c_uint64, C.c_int64, C.c_uint64, C.POINTER(C.c_void_p)]),
     "sz_session_destroy": (None, [C.c_void_p]),
     "sz_session_reset": (C.c_int, [C.c_void_p, C.c_uint64]),
+    "sz_room_bytes": (C.c_int, [C.c_void_p, C.c_int, C.POINTER(C.c_int64)]),
+    "sz_room_create": (C.c_int, [C.c_void_p, C.c_int, C.c_uint64, C.c_int64, C.c_uint64, C.POINTER(C.c_void_p)]),
+    "sz_room_destroy": (None, [C.c_void_p]),
+    "sz_session_use_room": (C.c_int, [C.c_void_p, C.c_void_p]),
     "sz_session_len": (C.c_int, [C.c_void_p]),
     "sz_session_capacity": (C.c_int, [C.c_void_p]),
     "sz_session_pending": (C.c_int, [C.c_void_p]),

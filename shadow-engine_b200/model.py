@@ -2,6 +2,7 @@
 reference's tensor names (crates/shadowzero-model/src/exl3_model.rs:223-243), and the two placements of one model - host memory
 for the CPU oracle, HBM for the library."""
 import ctypes as C
+import threading
 
 import numpy as np
 import torch
@@ -336,6 +337,29 @@ class DeviceModel(_Placed):
             return ml.c
 
         self._build(M, put, put_moe)
+        self._room, self._room_mem, self._room_lock = None, None, threading.Lock()
+
+    def room(self, stream, rows=512):
+        """The room for prompts' chunks that the model's sessions share (`sz_room_create`), made for the first of them; None where
+        the model's prompts go in passes."""
+        lib = szlib.load()
+        with self._room_lock:
+            if self._room is None:
+                n = C.c_int64()
+                szlib.check(lib.sz_room_bytes(C.byref(self.model), rows, C.byref(n)))
+                if n.value:
+                    self._room_mem = torch.empty(n.value + 256, dtype=torch.uint8, device=self.device)
+                    torch.cuda.synchronize(self.device)      # (the memory may have been another stream's)
+                    h = C.c_void_p()
+                    szlib.check(lib.sz_room_create(C.byref(self.model), rows, self._room_mem.data_ptr() + (-self._room_mem.data_ptr()) % 256, n.value,
+                                                   stream, C.byref(h)))
+                    self._room = h
+        return self._room
+
+    def __del__(self):
+        if getattr(self, "_room", None):
+            szlib.load().sz_room_destroy(self._room)
+            self._room = None
 
 
 class Session:
@@ -343,7 +367,8 @@ class Session:
 
     def __init__(self, dm, ctx, kv_q8=True, stream=None, head_proxy=False, lean=False, room=False):
         """head_proxy: screen an EXL3 output.weight with its 2-bit proxy (SZ_HEAD_PROXY); the proxy is built here.
-        lean: no room for a prompt's chunks (SZ_SESSION_LEAN); room: the full room, for a batch's prompts too (SZ_SESSION_ROOM)."""
+        Prompts go in chunks through the model's room, shared by its sessions; room: through one of the session's own (SZ_SESSION_ROOM);
+        lean: in passes (SZ_SESSION_LEAN)."""
         self.lib = szlib.load()
         self.dm = dm
         self.flags = (1 if kv_q8 else 0) | (2 if head_proxy else 0) | (4 if lean else 0) | (8 if room else 0)
@@ -358,6 +383,10 @@ class Session:
         self.h = C.c_void_p()
         szlib.check(self.lib.sz_session_create(C.byref(dm.model), ctx, self.flags, addr, n.value, self.stream, C.byref(self.h)))
         self.vocab = dm.cfg["vocab"]
+        if kv_q8 and not lean and not room:
+            shared = dm.room(self.stream)
+            if shared:
+                szlib.check(self.lib.sz_session_use_room(self.h, shared))
 
     def __del__(self):
         if getattr(self, "h", None):
@@ -536,7 +565,7 @@ class Batch:
         self.dm = dm
         self._stream = torch.cuda.Stream(dm.device)
         self.stream = self._stream.cuda_stream
-        self.sessions = [Session(dm, ctx, kv_q8=kv_q8, stream=self._stream, head_proxy=head_proxy, lean=b > 0, room=b == 0 and n > 1)
+        self.sessions = [Session(dm, ctx, kv_q8=kv_q8, stream=self._stream, head_proxy=head_proxy, lean=b > 0)
                          for b in range(n)]
         self.rows_max = rows_max or min(256, (n * szlib.MAX_VERIFY + 7) // 8 * 8)
         nb = C.c_int64()

@@ -2,6 +2,7 @@
 group; the smallest and largest of their ranges.  A session's rows are bit for bit those of passes of up to 8 rows; a block-format expert
 layer and the tensor-core projections are held against the CPU restatement."""
 import ctypes as C
+import threading
 
 import numpy as np
 import pytest
@@ -110,11 +111,22 @@ def raise_error(dm, mem, addr, size):
     return word
 
 
+def make_room(dm, rows, stream):
+    lib, n, h = szlib.load(), C.c_int64(), C.c_void_p()
+    szlib.check(lib.sz_room_bytes(C.byref(dm.model), rows, C.byref(n)))
+    mem = torch.empty(n.value + 256, dtype=torch.uint8, device="cuda")
+    addr = mem.data_ptr() + (-mem.data_ptr()) % 256
+    torch.cuda.synchronize()
+    szlib.check(lib.sz_room_create(C.byref(dm.model), rows, addr, n.value, stream, C.byref(h)))
+    torch.cuda.synchronize()
+    return h, mem, addr, n.value
+
+
 def test_a_wait_that_ran_out_in_a_prompts_chunk_is_reported(dm):
-    s = md.Session(dm, 128, kv_q8=True)
-    n = C.c_int64()
-    szlib.check(s.lib.sz_session_bytes(C.byref(dm.model), 128, s.flags, C.byref(n)))
-    word = raise_error(dm, s.mem, s.mem.data_ptr() + (-s.mem.data_ptr()) % 256, n.value)
+    s = md.Session(dm, 128, kv_q8=True, lean=True)
+    room, mem, addr, size = make_room(dm, 64, s.stream)
+    szlib.check(s.lib.sz_session_use_room(s.h, room))
+    word = raise_error(dm, mem, addr, size)
     s.prefill(md.make_prompt(60, CFG["vocab"], seed=90))
     with pytest.raises(szlib.SzError) as e:
         s.result()
@@ -123,6 +135,7 @@ def test_a_wait_that_ran_out_in_a_prompts_chunk_is_reported(dm):
     s.reset()
     s.prefill(md.make_prompt(60, CFG["vocab"], seed=90))
     s.result()
+    s.lib.sz_room_destroy(room)
 
 
 @pytest.mark.parametrize("shared", ["1", "0"])
@@ -140,3 +153,78 @@ def test_a_wait_that_ran_out_in_a_step_is_reported_by_every_sequence(dm, monkeyp
     batch.verify([[1, 2], [3], [4, 5, 6]])
     for s in batch.sessions:
         s.result()
+
+
+@pytest.mark.parametrize("kind", ["shared", "own", "small"])
+def test_sessions_of_several_threads_feed_their_prompts_through_a_room(dm, kind):
+    """Four sessions, a thread and a stream each: the model's room, rooms of their own, one room of 16 rows (many chunks)."""
+    prompts = [[md.make_prompt(n, CFG["vocab"], seed=200 + 10 * t + i) for i, n in enumerate((70, 17, 150))] for t in range(4)]
+    room = None
+    sessions = []
+    for _ in prompts:
+        s = md.Session(dm, 320, kv_q8=True, room=kind == "own", lean=kind == "small")
+        if kind == "small":
+            room = room or make_room(dm, 16, s.stream)
+            szlib.check(s.lib.sz_session_use_room(s.h, room[0]))
+        sessions.append(s)
+    if room:
+        sessions[0].lib.sz_room_destroy(room[0])      # (the sessions keep it)
+    got = [[] for _ in prompts]
+
+    def feed(t):
+        s = sessions[t]
+        for p in prompts[t]:
+            s.reset()
+            s.prefill(p)
+            got[t].append(s.result(logits=True)[2])
+            s.commit((len(p) - 1) % 8 + 1)
+            s.verify([5, 6, 7])
+            got[t].append(s.result(logits=True)[2])
+
+    threads = [threading.Thread(target=feed, args=(t,)) for t in range(len(prompts))]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    alone = md.Session(dm, 320, kv_q8=True, lean=True)       # in passes of 8
+    for t, ps in enumerate(prompts):
+        for i, p in enumerate(ps):
+            alone.reset()
+            alone.prefill(p)
+            assert np.array_equal(alone.result(logits=True)[2].view(np.uint32), got[t][2 * i].view(np.uint32)), "thread %d, prompt %d" % (t, i)
+            alone.commit((len(p) - 1) % 8 + 1)
+            alone.verify([5, 6, 7])
+            assert np.array_equal(alone.result(logits=True)[2].view(np.uint32), got[t][2 * i + 1].view(np.uint32)), "after prompt %d of thread %d" % (i, t)
+
+
+def session_bytes(m, flags):
+    n = C.c_int64()
+    szlib.check(szlib.load().sz_session_bytes(C.byref(m.model), 320, flags, C.byref(n)))
+    return n.value
+
+
+def test_a_session_has_room_for_chunks_only_where_it_was_asked_for(dm):
+    lib = szlib.load()
+    n, small = C.c_int64(), C.c_int64()
+    szlib.check(lib.sz_room_bytes(C.byref(dm.model), 512, C.byref(n)))
+    szlib.check(lib.sz_room_bytes(C.byref(dm.model), 16, C.byref(small)))
+    assert n.value > small.value > 0
+    assert session_bytes(dm, 1) == session_bytes(dm, 1 | 4) == session_bytes(dm, 1 | 4 | 8)
+    assert session_bytes(dm, 1 | 8) == session_bytes(dm, 1) + n.value
+    assert session_bytes(dm, 8) == session_bytes(dm, 0)                                  # an f32 cache: prompts go in passes
+    for rows in (0, 8, 20, 520):
+        assert lib.sz_room_bytes(C.byref(dm.model), rows, C.byref(n)) == szlib.E_ARG
+    h = C.c_void_p()
+    assert lib.sz_room_create(C.byref(dm.model), 16, 4100, 1 << 40, 0, C.byref(h)) == szlib.E_ARG
+    assert lib.sz_room_create(C.byref(dm.model), 16, 4096, small.value - 1, 0, C.byref(h)) == szlib.E_SCRATCH
+    assert lib.sz_session_use_room(None, None) == szlib.E_ARG
+
+
+def test_a_model_whose_prompts_go_in_passes_needs_no_room():
+    lib = szlib.load()
+    q8 = md.DeviceModel(md.make_model(md.TINY, seed=1))                  # Q8_0 experts
+    n = C.c_int64(-1)
+    szlib.check(lib.sz_room_bytes(C.byref(q8.model), 512, C.byref(n)))
+    assert n.value == 0 and session_bytes(q8, 1 | 8) == session_bytes(q8, 1)
+    h = C.c_void_p()
+    assert lib.sz_room_create(C.byref(q8.model), 512, 4096, 1 << 40, 0, C.byref(h)) == szlib.E_TYPE
