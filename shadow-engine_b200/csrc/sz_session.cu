@@ -1494,12 +1494,10 @@ extern "C" int sz_session_prefill(sz_session* s, const int32_t* ids, int n, uint
 namespace {
 struct SzIssuePool {
     std::vector<std::thread> th;
-    std::mutex mu;
+    std::mutex callers, mu;       // one call of each() at a time; what follows
     std::condition_variable cv, cv_done;
     std::function<void(int)> job;
-    int n = 0, dev = 0;
-    std::atomic<int> next{0};
-    int done = 0;
+    int n = 0, dev = 0, next = 0, done = 0;
     unsigned long long gen = 0;
     bool stop = false;
     explicit SzIssuePool(int workers) {
@@ -1510,34 +1508,40 @@ struct SzIssuePool {
         cv.notify_all();
         for (auto& t : th) t.join();
     }
-    void work() {
-        for (;;) {
-            const int i = next.fetch_add(1);
-            if (i >= n) break;
+    // Items are taken under the lock: a worker late from one call then sees the next one's count with its index, never a mixture.  (The
+    // job is replaced only when every item taken is done.)
+    void work(int on = -1) {
+        std::unique_lock<std::mutex> lk(mu);
+        while (next < n) {
+            const int i = next++, d = dev;
+            lk.unlock();
+            if (on >= 0 && d != on) cudaSetDevice(on = d);
             job(i);
-            std::lock_guard<std::mutex> lk(mu);
+            lk.lock();
             if (++done == n) cv_done.notify_all();
         }
     }
     void run() {
         unsigned long long seen = 0;
         for (;;) {
+            int d;
             {
                 std::unique_lock<std::mutex> lk(mu);
                 cv.wait(lk, [&] { return stop || gen != seen; });
                 if (stop) return;
-                seen = gen;
+                seen = gen; d = dev;
             }
-            cudaSetDevice(dev);
-            work();
+            cudaSetDevice(d);
+            work(d);
         }
     }
-    // runs fn(0) .. fn(count - 1), the caller taking its share; returns when all are done
+    // runs fn(0) .. fn(count - 1), the caller taking its share; returns when all are done (steps of several threads take turns)
     void each(int count, int device, std::function<void(int)> fn) {
         if (th.empty() || count < 2) { for (int i = 0; i < count; i++) fn(i); return; }
+        std::lock_guard<std::mutex> turn(callers);
         {
             std::lock_guard<std::mutex> lk(mu);
-            job = std::move(fn); n = count; dev = device; done = 0; next.store(0); gen++;
+            job = std::move(fn); n = count; dev = device; done = 0; next = 0; gen++;
         }
         cv.notify_all();
         work();

@@ -1,5 +1,7 @@
 """Several sequences in one step (`sz_batch_verify`, `sz_batch_gen_run`): every sequence's logits, acceptance and tokens are bit for
 bit those of a session stepping alone - the sequences share the MoE sublayers' work, not their numbers."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -160,3 +162,33 @@ def test_the_shared_reads_and_projections_change_no_bit(dm, monkeypatch):
     for other in got[1:]:
         for a, b in zip(got[0], other):
             assert np.array_equal(a, b)
+
+
+def test_batches_of_several_threads_step_at_the_same_time(dm):
+    """Batches of 2, 3 and 5 sequences, a thread each: their launches share the process's issue threads, call by call."""
+    sizes, steps = (2, 3, 5), 12
+    batches = [md.Batch(dm, n, 128) for n in sizes]
+    rows = [[[[int(t) for t in np.random.default_rng(1000 * n + 100 * k + b).integers(0, CFG["vocab"], 1 + (b + k) % 4)] for b in range(n)]
+             for k in range(steps)] for n in sizes]
+    got = [[] for _ in sizes]
+
+    def run(t):
+        for r in rows[t]:
+            batches[t].verify(r)
+            for b, s in enumerate(batches[t].sessions):
+                got[t].append(s.result(logits=True)[2])
+                s.commit(len(r[b]))
+
+    threads = [threading.Thread(target=run, args=(t,)) for t in range(len(sizes))]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join(60)
+    assert not any(th.is_alive() for th in threads)
+    for t, n in enumerate(sizes):
+        for b in range(n):
+            alone = md.Session(dm, 128, kv_q8=True, lean=True)
+            for k in range(steps):
+                alone.verify(rows[t][k][b])
+                assert np.array_equal(alone.result(logits=True)[2].view(np.uint32), got[t][k * n + b].view(np.uint32)), "batch of %d, step %d" % (n, k)
+                alone.commit(len(rows[t][k][b]))
