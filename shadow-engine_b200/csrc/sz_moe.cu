@@ -831,6 +831,48 @@ static int sz_ffn(cudaStream_t st, int type, const SzPlan* plan, int groups, u64
 }
 
 
+// The shape of a pass's expert launches: OCC blocks a multiprocessor (2 or 3), units 8 TW (down: 8 TWD) tile columns wide (4, 2 or 1 a
+// consumer warp: 24, 12 or 6 KB of trellis at 3 bits).  Narrower units and a third block spread the work more evenly and cost more
+// hand-overs; which wins goes with what is left over when the units are shared out.  So the least of an estimate, in decoded tile columns
+// of a multiprocessor, over both kernels: between its even share of the units and what it has with blocks of the most units (a third of the way: the
+// others' share of its issue slots goes to a block that is late), at least 1.85 times a block's own (a block alone cannot use
+// all of them), each unit with 0.75 of a column's time for its hand-over.  Wide gate / up units of three blocks are left out where a block has
+// not two of them (the first one's copy, the longest there is, is overlapped with nothing).  The groups are what independent rows choose on average.
+// Measured over 1 .. 8 rows of three shapes at 3 bits, all 18 combinations (us a layer, best of them / this choice / the rule by pairs before it):
+// 2048 x 512, 512 experts, top 10: rows 3 50.8 / 51.6 / 52.7, 4 59.0 / 59.0 / 59.0, 5 73.8 / 73.8 / 75.6, 7 95.6 / 95.6 / 95.5, 8 106.4 / 107.0 / 110.1;
+// 1024 x 512, 64, top 6: rows 1 22.3 / 22.3 / 25.2, 8 45.8 / 45.8 / 48.8; 512 x 256, 32, top 4: rows 4 22.4 / 22.4 / 24.8.  Over 1 .. 8 rows of
+// ten shapes at 2, 3 and 4 bits, of which it was not made: 3.1 % faster than the rule before on average, 2.0 % slower at worst.
+struct SzXWShape { int occ, tw, twd; };
+static SzXWShape sz_xw_shape(const sz_moe_layer* L, int m, bool shared) {
+    const int sms = sz_sm_count(), NTC = L->expert_ff / 128, H = L->hidden;
+    double g = L->n_expert * (1. - pow(1. - (double)L->top_k / L->n_expert, m));
+    if (L->ep_count > 0) g *= (double)L->ep_count / L->n_expert;
+    g += shared ? 1 : 0;
+    auto estimate = [&](double per_group, int occ, int tw) {      // the expected value over a whole number of groups either side
+        double e = 0;
+        for (int side = 0; side < 2; side++) {
+            const double G = floor(g) + side, units = G * per_group, n = ceil(units / (occ * sms));
+            const double most = units < occ * sms ? ceil(units / sms) : (2 * units / sms + occ * n) / 3;
+            e += (side ? g - floor(g) : 1 - (g - floor(g))) * (most > 1.85 * n ? most : 1.85 * n) * (tw + 0.75);
+        }
+        return e;
+    };
+    SzXWShape best = {2, NTC % 4 == 0 ? 4 : (NTC % 2 == 0 ? 2 : 1), 4};
+    double least = -1;
+    for (int occ = 2; occ <= 3; occ++)
+        for (int tw = 4; tw >= 1; tw /= 2) {
+            if (NTC % tw) continue;
+            const double per_gu = 2. * (H / 128) * (NTC / tw);
+            if (occ == 3 && tw == 4 && g * per_gu < 2 * occ * sms) continue;
+            const double gu = estimate(per_gu, occ, tw);
+            for (int twd = 4; twd >= 1; twd /= 2) {
+                const double e = gu + estimate((double)NTC * (H / (128 * twd)), occ, twd);
+                if (least < 0 || e < least) { least = e; best = {occ, tw, twd}; }
+            }
+        }
+    return best;
+}
+
 template <int K, int NTC>
 static int sz_x3_launch_k(cudaStream_t st, const sz_moe_layer* L, int m, const SzPlan* plan, const float* x, long long* acc_gu, long long* acc_d,
                           u32* ctrl, bool sh) {
@@ -845,20 +887,12 @@ static int sz_x3_launch_k(cudaStream_t st, const sz_moe_layer* L, int m, const S
     const char* cl = getenv("SZ_X3_CLASSIC");   // (read at every call: a test switches it inside one process)
     const bool classic = cl && atoi(cl) != 0;
     if (!classic) {
-        // Shape of the launch: OCC blocks a multiprocessor (2 or 3), a unit 8 TW tile columns a consumer warp wide (TW = 4, 2 or 1: 24, 12
-        // or 6 KB of trellis at 3 bits).  Narrower units and a third block spread the units evenly: gate / up of 40 experts of the
-        // benchmark's shape are 1,280 units 4 wide - 4.3 a block at 296 blocks, so some take 5 - and the down matrices only 640.
-        // SZ_XW_OCC / SZ_XW_TW / SZ_XW_TWD override the choice (experiments).
+        // SZ_XW_OCC / SZ_XW_TW / SZ_XW_TWD override the choice (experiments)
         const dim3 block(SZ_XW_THREADS);
         const char *eo = getenv("SZ_XW_OCC"), *et = getenv("SZ_XW_TW"), *ed = getenv("SZ_XW_TWD");
-        // few rows mean few units (a 1-row pass of the benchmark's shape: 11 groups, 352 units 4 wide for 296 blocks): narrower units
-        // and a third block a multiprocessor spread them better (4.30 -> 4.19 ms a 1-row pass of the 48-layer model); with 4 rows the
-        // wide units win (6.18 against 6.35 ms)
-        // (up to 48 groups, 40 at 4 rows of the benchmark's layer: three blocks and the down matrices in narrower units even out what is left
-        // over, 60.8 -> 59.3 us a layer; with 75 groups two blocks win, 10.30 against 10.37 ms a pass of 8 rows)
-        const bool few = m * (int)L->top_k <= 24, some = m * (int)L->top_k <= 48;
-        const int occ = eo && atoi(eo) == 2 ? 2 : (eo && atoi(eo) == 3 ? 3 : (few || some ? 3 : 2));
-        int tw = et ? atoi(et) : (few ? 2 : 4), twd = ed ? atoi(ed) : (few || some ? 2 : 4);
+        const SzXWShape shape = sz_xw_shape(L, m, sh);
+        const int occ = eo && atoi(eo) == 2 ? 2 : (eo && atoi(eo) == 3 ? 3 : shape.occ);
+        int tw = et ? atoi(et) : shape.tw, twd = ed ? atoi(ed) : shape.twd;
         if (!(tw == 1 || tw == 2 || tw == 4) || tw > NTC || NTC % tw) tw = NTC < 4 ? NTC : 4;
         if (tw == 3) tw = 1;
         if (!(twd == 1 || twd == 2 || twd == 4)) twd = 4;
