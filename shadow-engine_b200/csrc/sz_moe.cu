@@ -837,11 +837,13 @@ static int sz_ffn(cudaStream_t st, int type, const SzPlan* plan, int groups, u64
 // of a multiprocessor, over both kernels: between its even share of the units and what it has with blocks of the most units (a third of the way: the
 // others' share of its issue slots goes to a block that is late), at least 1.85 times a block's own (a block alone cannot use
 // all of them), each unit with 0.75 of a column's time for its hand-over.  Wide gate / up units of three blocks are left out where a block has
-// not two of them (the first one's copy, the longest there is, is overlapped with nothing).  The groups are what independent rows choose on average.
+// not two of them (the first one's copy, the longest there is, is overlapped with nothing), wide down units, whose first copy is issued ahead
+// of the kernel's wait, where it has not one and a half (4 rows of the first shape, experts cold: 59.5 us a layer against 58.8).  The groups are what independent rows choose on average.
 // Measured over 1 .. 8 rows of three shapes at 3 bits, all 18 combinations (us a layer, best of them / this choice / the rule by pairs before it):
 // 2048 x 512, 512 experts, top 10: rows 3 50.8 / 51.6 / 52.7, 4 59.0 / 59.0 / 59.0, 5 73.8 / 73.8 / 75.6, 7 95.6 / 95.6 / 95.5, 8 106.4 / 107.0 / 110.1;
 // 1024 x 512, 64, top 6: rows 1 22.3 / 22.3 / 25.2, 8 45.8 / 45.8 / 48.8; 512 x 256, 32, top 4: rows 4 22.4 / 22.4 / 24.8.  Over 1 .. 8 rows of
-// ten shapes at 2, 3 and 4 bits, of which it was not made: 3.1 % faster than the rule before on average, 2.0 % slower at worst.
+// ten shapes at 2, 3 and 4 bits, eight of which it was not made from: 3.1 % faster than the rule before on average, 2.1 % slower at worst.  (Rows that
+// agree choose fewer: a tree of 8 rows of the 48-layer model 66 experts, not 75, and there the two rules are within 0.3 %.)
 struct SzXWShape { int occ, tw, twd; };
 static SzXWShape sz_xw_shape(const sz_moe_layer* L, int m, bool shared) {
     const int sms = sz_sm_count(), NTC = L->expert_ff / 128, H = L->hidden;
@@ -866,7 +868,9 @@ static SzXWShape sz_xw_shape(const sz_moe_layer* L, int m, bool shared) {
             if (occ == 3 && tw == 4 && g * per_gu < 2 * occ * sms) continue;
             const double gu = estimate(per_gu, occ, tw);
             for (int twd = 4; twd >= 1; twd /= 2) {
-                const double e = gu + estimate((double)NTC * (H / (128 * twd)), occ, twd);
+                const double per_dn = (double)NTC * (H / (128 * twd));
+                if (occ == 3 && twd == 4 && g * per_dn < 1.5 * occ * sms) continue;
+                const double e = gu + estimate(per_dn, occ, twd);
                 if (least < 0 || e < least) { least = e; best = {occ, tw, twd}; }
             }
         }
