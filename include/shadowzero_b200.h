@@ -115,8 +115,8 @@ int sz_moe_verify_host(const sz_moe_layer* layer, const float* x_host, int m, fl
  * experts of a long prompt (plan_scan_w / plan_fill_w, kernels/forward.cu:3234-3319; mma_grouped*, kernels/matvec.cu:1190-1260;
  * exl3_mma, kernels/exl3.cu:500-590), with the verify pass's exact kernels: a row's output is bit for bit sz_moe_verify's.  EXL3
  * experts, no expert sharding.  sz_moe_rows_status(layer, rows, scratch, NULL, stream) once after the scratch is allocated (and
- * after a failed call); with a code pointer it synchronises and reports (bit 0: a bounded wait ran out, bit 1: the routing needed
- * more windows than the scratch has, bit 2: an expert id out of range reached the plan).  The scratch has one size and one layout
+ * after a failed call); with a code pointer it synchronises and reports (bit 0: a bounded wait ran out, bit 2: an expert id out
+ * of range reached the plan).  The scratch has one size and one layout
  * whatever the rows of a call. */
 int sz_moe_rows_scratch_bytes(const sz_moe_layer* layer, int rows, int64_t* bytes);
 int sz_moe_rows(const sz_moe_layer* layer, uint64_t x, int rows, uint64_t y, uint64_t route_idx, uint64_t route_w, uint64_t scratch,
@@ -327,22 +327,24 @@ int sz_session_commit_path(sz_session* s, const int32_t* path, int n, uint64_t s
 int sz_session_result(sz_session* s, int32_t* keep_next, uint32_t* top, float* logits, uint64_t stream);
 /* Keeps the first `keep` rows of the pending pass and drops the rest (rollback(&snap, &batch[..keep])). */
 int sz_session_commit(sz_session* s, int keep, uint64_t stream);
-/* Several sequences in one step (the batch of config 5, from the pieces above): every sequence keeps its session and runs what
- * carries its own state (embedding, attention, head) in lockstep with the others; the hyper-connection reads, the mixers'
- * projections and the MoE sublayer of every layer take the rows of ALL sequences as one batch, so their weights are streamed once
- * a step and an expert several sequences chose is decoded once (sz_moe_rows); the DeltaNet scans of a layer are one launch.  While the call runs, the sessions' per-pass buffers
- * point into the batch's scratch: no other thread may use those sessions.  n <= 64 sessions of one model (EXL3 experts,
+/* Several sequences in one step (the batch of config 5, from the pieces above): every sequence keeps its session, and every kernel of
+ * a layer - reads, projections, DeltaNet scans, attention, MoE - runs once over the rows of ALL sequences, so weights are streamed
+ * once a step and an expert several sequences chose is decoded once (sz_moe_rows); head, acceptance and commit are launches of the
+ * sequence.  (Models with a per-layer embedding, the sparse indexer or an f32 cache: embedding, attention and head are the
+ * sequence's, reads, projections, scans and MoE shared.)  While the call runs no other thread may use those sessions; threads with
+ * batches of their own may step at the same time.  n <= 64 sessions of one model (EXL3 experts,
  * no expert sharding) on one stream; ms[b] rows of sequence b, ids = the rows of all sequences one after the other; the rows of
  * a step, padded to a multiple of 8, must fit rows_max (<= 256), the size the scratch was made for.  Afterwards every session
  * holds a pending pass: sz_session_result / sz_session_commit per session.  A sequence's results are bit for bit those of a pass
- * of its own.  sz_batch_scratch_init once after the scratch is allocated. */
+ * of its own.  sz_batch_scratch_init once after the scratch is allocated.  A bounded wait that ran out in a kernel over all rows is
+ * reported by the sz_session_result of every sequence of the step (SZ_E_DEVICE), as one in a prompt's chunk is by the session's. */
 int sz_batch_scratch_bytes(const sz_model* model, int rows_max, int64_t* bytes);
 int sz_batch_scratch_init(const sz_model* model, int rows_max, uint64_t scratch, uint64_t stream);
 int sz_batch_verify(sz_session* const* sessions, int n, const int32_t* ids, const int32_t* ms, int accept_mode, int eog_token, int rows_max,
                     uint64_t scratch, int64_t scratch_bytes, uint64_t stream);
-/* sz_session_prefill for n sequences in lockstep: every step takes up to 8 rows of every sequence that still has prompt left (as
- * many sequences a step as rows_max holds; the rest wait their turn), keeps them all, and runs the head only for a prompt's last
- * pass - which is left pending, as sz_session_prefill leaves it: sz_session_result, then sz_session_commit of its
+/* sz_session_prefill for n sequences in lockstep: every step takes as many rows of the prompts that are left as there is room for (the
+ * scratch's rows_max, or the rows of a session's room where one has more; up to 8 of a sequence on models whose steps are not
+ * many-row ones), keeps them all, and runs the head only for a prompt's last pass - which is left pending, as sz_session_prefill leaves it: sz_session_result, then sz_session_commit of its
  * (lens[b] - 1) % 8 + 1 rows.  Every sequence's state and results are bit for bit those of its own sz_session_prefill. */
 int sz_batch_prefill(sz_session* const* sessions, int n, const int32_t* const* ids, const int32_t* lens, int rows_max, uint64_t scratch,
                      int64_t scratch_bytes, uint64_t stream);

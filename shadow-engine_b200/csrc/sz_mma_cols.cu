@@ -30,8 +30,8 @@
 // a token tile (25 KB per 256 x 256 x 32) where one a block moved 41, and the tensor core, which needs 512 cycles of the step's 625; the
 // sums of a unit, which all blocks write at about the same time, are a fifth.  At few tokens latency: the chain decode, fence, barrier,
 // instruction.  The issuing thread took 390 cycles a step to make descriptors for 256 cycles of instructions; it makes them once.
-// 12,288 x 2,048: 4,093 tokens 281 -> 243 us (sustained, 1.4 GHz under the power cap), 256 tokens 28.8 -> 24.7;
-// 512 x 2,048, one token: 20 -> 12.4 (K in four parts).
+// 12,288 x 2,048: 4,093 tokens 281 -> 241 us (sustained, 1.4 GHz under the power cap), 256 tokens 28.8 -> 25.0;
+// 512 x 2,048, one token: 20 -> 11.9 (K in four parts).
 // Every wait is bounded; a wait that runs out records where in the error word, and the block still frees its tensor memory.
 #include <cuda.h>   // CUtensorMap and its enums; the encoder's entry point is asked of the runtime, nothing links against the driver
 #include "sz_common.cuh"

@@ -9,7 +9,7 @@
 //   gate/up   sz_rows_gateup_kernel: a persistent launch over all groups
 //   act       sz_rows_act_kernel: SwiGLU of every pair, left as the down product's operand fragments
 //   down      sz_rows_down_kernel: as gate/up, over those fragments
-//   combine   sz_rows_combine_kernel: per (row, 128 outputs) the ranks' terms in rank order, as sz_x3_combine_kernel adds them
+//   combine   sz_rows_combine_kernel: per (row, 512 outputs) the ranks' terms in rank order, as sz_x3_combine_kernel adds them
 // A pair's numbers do not depend on which rows share its group (every row of a group is a column of its own in the tensor-core
 // product, the sums over column blocks are integer): a row's output is bit for bit what sz_moe_verify gives for it.
 //

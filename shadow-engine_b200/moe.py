@@ -123,7 +123,7 @@ class MoeLayer:
         return (y, ridx, rw) if want_routing else y
 
     def moe_rows_status(self, rows, stream=None):
-        """Synchronises; 0 unless a bounded wait ran out (1) or the routing needed more windows than the scratch has (2)."""
+        """Synchronises; 0 unless a bounded wait ran out (1) or an expert id out of range reached the plan (4)."""
         st = (stream or torch.cuda.current_stream(self.device)).cuda_stream
         code = C.c_int()
         szlib.check(self.lib.sz_moe_rows_status(C.byref(self.c), rows, self._rows_scratch[2], C.byref(code), st))

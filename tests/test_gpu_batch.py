@@ -55,7 +55,7 @@ def test_a_step_of_several_sequences_equals_their_own_passes(dm):
 
 
 def test_a_step_of_forty_sequences_and_two_hundred_rows(dm):
-    """Many sequences: the reads, projections and experts then run over several row blocks and windows; every sequence still gets
+    """Many sequences: the reads, projections and experts then run over several row blocks and groups; every sequence still gets
     the bits of its own pass, step after step."""
     n = 40
     rng = np.random.default_rng(31)

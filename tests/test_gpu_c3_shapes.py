@@ -191,7 +191,7 @@ def test_a_batched_step_at_the_benchmark_shapes_equals_the_sequences_own_passes(
 
 
 def test_a_batched_step_of_a_hundred_rows_at_the_benchmark_shapes(c3):
-    """Twenty-four sequences of 3..6 rows: 512 experts over several windows, projections over three row blocks."""
+    """Twenty-four sequences of 3..6 rows: 512 experts in several hundred groups, projections over three row blocks."""
     M, hm, dm = c3
     n = 24
     rng = np.random.default_rng(23)
