@@ -273,7 +273,7 @@ int sz_session_len(const sz_session* s);        /* committed positions: GpuSessi
 int sz_session_capacity(const sz_session* s);   /* GpuSession::capacity() */
 int sz_session_pending(const sz_session* s);    /* rows of the pass that awaits sz_session_commit (0: none) */
 /* A room is where the chunks of a prompt go: up to SZ_ROOM_ROWS rows through a layer at once instead of passes of 8 (six times as fast
- * for 507 tokens; some 400 MB at the benchmark's shapes).  One serves all sessions of a model: a host makes it once, in memory of its own
+ * for 507 tokens; some 320 MB at the benchmark's shapes).  One serves all sessions of a model: a host makes it once, in memory of its own
  * (256-byte aligned, valid as long as a session uses it), and gives it to every session it makes; or a session has one of its own
  * (SZ_SESSION_ROOM).  Any thread may use its session's room at any time: prompts in one room follow one another on the GPU, and the
  * launches of each are issued under the room's lock.  rows: a multiple of 8 from 16 to SZ_ROOM_ROWS.  sz_room_bytes gives 0 where

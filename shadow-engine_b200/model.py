@@ -337,29 +337,37 @@ class DeviceModel(_Placed):
             return ml.c
 
         self._build(M, put, put_moe)
-        self._room, self._room_mem, self._room_lock = None, None, threading.Lock()
 
-    def room(self, stream, rows=512):
-        """The room for prompts' chunks that the model's sessions share (`sz_room_create`), made for the first of them; None where
-        the model's prompts go in passes."""
-        lib = szlib.load()
-        with self._room_lock:
-            if self._room is None:
-                n = C.c_int64()
-                szlib.check(lib.sz_room_bytes(C.byref(self.model), rows, C.byref(n)))
-                if n.value:
-                    self._room_mem = torch.empty(n.value + 256, dtype=torch.uint8, device=self.device)
-                    torch.cuda.synchronize(self.device)      # (the memory may have been another stream's)
-                    h = C.c_void_p()
-                    szlib.check(lib.sz_room_create(C.byref(self.model), rows, self._room_mem.data_ptr() + (-self._room_mem.data_ptr()) % 256, n.value,
-                                                   stream, C.byref(h)))
-                    self._room = h
-        return self._room
+
+class Room:
+    """Room for the chunks of prompts (`sz_room_create`), in memory of its own; `h` is None where the model's prompts go in passes."""
+
+    def __init__(self, dm, stream, rows=512):
+        self.lib = szlib.load()
+        self.h, n = None, C.c_int64()
+        szlib.check(self.lib.sz_room_bytes(C.byref(dm.model), rows, C.byref(n)))
+        if n.value:
+            self.mem = torch.empty(n.value + 256, dtype=torch.uint8, device=dm.device)
+            torch.cuda.synchronize(dm.device)      # (the memory may have been another stream's)
+            h = C.c_void_p()
+            szlib.check(self.lib.sz_room_create(C.byref(dm.model), rows, self.mem.data_ptr() + (-self.mem.data_ptr()) % 256, n.value, stream, C.byref(h)))
+            self.h = h
 
     def __del__(self):
-        if getattr(self, "_room", None):
-            szlib.load().sz_room_destroy(self._room)
-            self._room = None
+        if getattr(self, "h", None):
+            self.lib.sz_room_destroy(self.h)
+            self.h = None
+
+
+_room_lock = threading.Lock()
+
+
+def shared_room(dm, stream):
+    """The room that the sessions of a model share: made for the first of them, kept by the model."""
+    with _room_lock:
+        if getattr(dm, "_room", None) is None:
+            dm._room = Room(dm, stream)
+        return dm._room
 
 
 class Session:
@@ -384,9 +392,9 @@ class Session:
         szlib.check(self.lib.sz_session_create(C.byref(dm.model), ctx, self.flags, addr, n.value, self.stream, C.byref(self.h)))
         self.vocab = dm.cfg["vocab"]
         if kv_q8 and not lean and not room:
-            shared = dm.room(self.stream)
-            if shared:
-                szlib.check(self.lib.sz_session_use_room(self.h, shared))
+            self._room = shared_room(dm, self.stream)
+            if self._room.h:
+                szlib.check(self.lib.sz_session_use_room(self.h, self._room.h))
 
     def __del__(self):
         if getattr(self, "h", None):

@@ -218,6 +218,9 @@ def test_a_session_has_room_for_chunks_only_where_it_was_asked_for(dm):
     assert lib.sz_room_create(C.byref(dm.model), 16, 4100, 1 << 40, 0, C.byref(h)) == szlib.E_ARG
     assert lib.sz_room_create(C.byref(dm.model), 16, 4096, small.value - 1, 0, C.byref(h)) == szlib.E_SCRATCH
     assert lib.sz_session_use_room(None, None) == szlib.E_ARG
+    other = md.Session(md.DeviceModel(md.make_model(CFG, expert_type=szlib.TYPE_EXL3(3), seed=5)), 64, lean=True)
+    room = md.Room(dm, other.stream, rows=16)
+    assert lib.sz_session_use_room(other.h, room.h) == szlib.E_ARG       # another model's
 
 
 def test_a_model_whose_prompts_go_in_passes_needs_no_room():
