@@ -831,50 +831,23 @@ static int sz_ffn(cudaStream_t st, int type, const SzPlan* plan, int groups, u64
 }
 
 
-// The shape of a pass's expert launches: OCC blocks a multiprocessor (2 or 3), units 8 TW (down: 8 TWD) tile columns wide (4, 2 or 1 a
-// consumer warp: 24, 12 or 6 KB of trellis at 3 bits).  Narrower units and a third block spread the work more evenly and cost more
-// hand-overs; which wins goes with what is left over when the units are shared out.  So the least of an estimate, in decoded tile columns
-// of a multiprocessor, over both kernels: between its even share of the units and what it has with blocks of the most units (a third of the way: the
-// others' share of its issue slots goes to a block that is late), at least 1.85 times a block's own (a block alone cannot use
-// all of them), each unit with 0.75 of a column's time for its hand-over.  Wide gate / up units of three blocks are left out where a block has
-// not two of them (the first one's copy, the longest there is, is overlapped with nothing), wide down units, whose first copy is issued ahead
-// of the kernel's wait, where it has not one and a half (4 rows of the first shape, experts cold: 59.5 us a layer against 58.8).  The groups are what independent rows choose on average.
-// Measured over 1 .. 8 rows of three shapes at 3 bits, all 18 combinations (us a layer, best of them / this choice / the rule by pairs before it):
-// 2048 x 512, 512 experts, top 10: rows 3 50.8 / 51.6 / 52.7, 4 59.0 / 59.0 / 59.0, 5 73.8 / 73.8 / 75.6, 7 95.6 / 95.6 / 95.5, 8 106.4 / 107.0 / 110.1;
-// 1024 x 512, 64, top 6: rows 1 22.3 / 22.3 / 25.2, 8 45.8 / 45.8 / 48.8; 512 x 256, 32, top 4: rows 4 22.4 / 22.4 / 24.8.  Over 1 .. 8 rows of
-// ten shapes at 2, 3 and 4 bits, eight of which it was not made from: 3.1 % faster than the rule before on average, 2.1 % slower at worst.  (Rows that
-// agree choose fewer: a tree of 8 rows of the 48-layer model 66 experts, not 75, and there the two rules are within 0.3 %.)
-struct SzXWShape { int occ, tw, twd; };
+// The widths of a pass's expert units, in tile columns an item (TW of the gate / up launch, TWD of down's; 4, 2 or 1: 24, 12 or 6 KB of trellis a
+// unit at 3 bits).  Narrow units share the work out more evenly, wide ones have fewer hand-overs and fragments; which wins goes with the
+// units a multiprocessor has.  The groups are what independent rows choose on average.  Measured (us a layer, 2048 x 512, 512 experts, top
+// 10; TW TWD = 44 / 42 / 24 / 22 / 21 / 11): rows 1 33.4 / 31.8 / 33.1 / 31.3 / 31.1 / 31.2, 2 42.3 / 40.9 / 40.4 / 38.9 / 39.7 / 40.7, 3 50.6 /
+// 49.1 / 48.7 / 47.5 / 49.6 / 51.4, 4 56.8 / 56.6 / 56.4 / 56.1 / 59.5 / 62.0, 6 77.6 / 77.2 / 76.8 / 76.4 / 82.0 / 87.0, 8 89.9 / 91.0 / 90.1 / 91.0 /
+// 99.5 / 105.6 (three blocks a multiprocessor with eight decode warps each before: rows 1 31.8, 2 40.9, 3 53, 4 59.5, 6 86.5, 8 107).
+struct SzXWShape { int tw, twd; };
 static SzXWShape sz_xw_shape(const sz_moe_layer* L, int m, bool shared) {
-    const int sms = sz_sm_count(), NTC = L->expert_ff / 128, H = L->hidden;
+    const int NTC = L->expert_ff / 128, H = L->hidden;
     double g = L->n_expert * (1. - pow(1. - (double)L->top_k / L->n_expert, m));
     if (L->ep_count > 0) g *= (double)L->ep_count / L->n_expert;
-    g += shared ? 1 : 0;
-    auto estimate = [&](double per_group, int occ, int tw) {      // the expected value over a whole number of groups either side
-        double e = 0;
-        for (int side = 0; side < 2; side++) {
-            const double G = floor(g) + side, units = G * per_group, n = ceil(units / (occ * sms));
-            const double most = units < occ * sms ? ceil(units / sms) : (2 * units / sms + occ * n) / 3;
-            e += (side ? g - floor(g) : 1 - (g - floor(g))) * (most > 1.85 * n ? most : 1.85 * n) * (tw + 0.75);
-        }
-        return e;
-    };
-    SzXWShape best = {2, NTC % 4 == 0 ? 4 : (NTC % 2 == 0 ? 2 : 1), 4};
-    double least = -1;
-    for (int occ = 2; occ <= 3; occ++)
-        for (int tw = 4; tw >= 1; tw /= 2) {
-            if (NTC % tw) continue;
-            const double per_gu = 2. * (H / 128) * (NTC / tw);
-            if (occ == 3 && tw == 4 && g * per_gu < 2 * occ * sms) continue;
-            const double gu = estimate(per_gu, occ, tw);
-            for (int twd = 4; twd >= 1; twd /= 2) {
-                const double per_dn = (double)NTC * (H / (128 * twd));
-                if (occ == 3 && twd == 4 && g * per_dn < 1.5 * occ * sms) continue;
-                const double e = gu + estimate(per_dn, occ, twd);
-                if (least < 0 || e < least) { least = e; best = {occ, tw, twd}; }
-            }
-        }
-    return best;
+    g = (g + (shared ? 1 : 0)) / sz_sm_count();
+    const double gu = g * 2 * (H / 128) * NTC, dn = g * NTC * (H / 128);      // units a multiprocessor at width 1
+    SzXWShape s;
+    s.tw = NTC % 4 == 0 && gu / 4 >= 12 ? 4 : (NTC % 2 == 0 && gu / 2 >= 3 ? 2 : 1);
+    s.twd = dn / 4 >= 7 ? 4 : (dn / 2 >= 2.5 ? 2 : 1);
+    return s;
 }
 
 template <int K, int NTC>
@@ -891,42 +864,40 @@ static int sz_x3_launch_k(cudaStream_t st, const sz_moe_layer* L, int m, const S
     const char* cl = getenv("SZ_X3_CLASSIC");   // (read at every call: a test switches it inside one process)
     const bool classic = cl && atoi(cl) != 0;
     if (!classic) {
-        // SZ_XW_OCC / SZ_XW_TW / SZ_XW_TWD override the choice (experiments)
-        const dim3 block(SZ_XW_THREADS);
-        const char *eo = getenv("SZ_XW_OCC"), *et = getenv("SZ_XW_TW"), *ed = getenv("SZ_XW_TWD");
+        // SZ_XW_TW / SZ_XW_TWD override the choice (experiments)
+        const dim3 block(SZ_XW_THREADS), grid(sz_sm_count());
+        const char *et = getenv("SZ_XW_TW"), *ed = getenv("SZ_XW_TWD");
         const SzXWShape shape = sz_xw_shape(L, m, sh);
-        const int occ = eo && atoi(eo) == 2 ? 2 : (eo && atoi(eo) == 3 ? 3 : shape.occ);
         int tw = et ? atoi(et) : shape.tw, twd = ed ? atoi(ed) : shape.twd;
         if (!(tw == 1 || tw == 2 || tw == 4) || tw > NTC || NTC % tw) tw = NTC < 4 ? NTC : 4;
         if (tw == 3) tw = 1;
         if (!(twd == 1 || twd == 2 || twd == 4)) twd = 4;
-        const dim3 grid(occ * sz_sm_count());
         int rc = SZ_E_TYPE;
-#define SZ_XW_GU(TT, OO)                                                                                                                    \
-    if (tw == TT && occ == OO) {                                                                                                            \
+#define SZ_XW_GU(TT)                                                                                                                        \
+    if (tw == TT) {                                                                                                                         \
         static bool setv = false;                                                                                                           \
-        if (!setv) { SZ_CUDA(cudaFuncSetAttribute(sz_xw_gateup_kernel<K, NTC, TT, OO>, cudaFuncAttributeMaxDynamicSharedMemorySize, SzXW<K, TT, OO>::SMEM_BYTES)); setv = true; } \
-        SZ_CUDA(sz_launch("gateup_exl3s", sz_xw_gateup_kernel<K, NTC, TT, OO>, grid, block, SzXW<K, TT, OO>::SMEM_BYTES, st, true, plan, (const u8*)L->gate, \
+        if (!setv) { SZ_CUDA(cudaFuncSetAttribute(sz_xw_gateup_kernel<K, NTC, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SzXW<K, TT>::SMEM_BYTES)); setv = true; } \
+        SZ_CUDA(sz_launch("gateup_exl3s", sz_xw_gateup_kernel<K, NTC, TT>, grid, block, SzXW<K, TT>::SMEM_BYTES, st, true, plan, (const u8*)L->gate, \
                           (u64)L->gate_stride, (const u8*)L->up, (u64)L->up_stride, (const u8*)(sh ? L->sh_gate : 0), (const u8*)(sh ? L->sh_up : 0), x, m, \
                           (int)L->hidden, (int)L->top_k, acc_gu, ctrl));                                                                    \
         rc = SZ_OK;                                                                                                                         \
     }
-#define SZ_XW_DN(TT, OO)                                                                                                                    \
-    if (twd == TT && occ == OO) {                                                                                                           \
+#define SZ_XW_DN(TT)                                                                                                                        \
+    if (twd == TT) {                                                                                                                        \
         static bool setv = false;                                                                                                           \
-        if (!setv) { SZ_CUDA(cudaFuncSetAttribute(sz_xw_down_kernel<K, TT, OO>, cudaFuncAttributeMaxDynamicSharedMemorySize, SzXW<K, TT, OO>::SMEM_BYTES)); setv = true; } \
-        SZ_CUDA(sz_launch("down_exl3s", sz_xw_down_kernel<K, TT, OO>, grid, block, SzXW<K, TT, OO>::SMEM_BYTES, st, true, plan, (const u8*)L->gate, (u64)L->gate_stride, \
+        if (!setv) { SZ_CUDA(cudaFuncSetAttribute(sz_xw_down_kernel<K, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SzXW<K, TT>::SMEM_BYTES)); setv = true; } \
+        SZ_CUDA(sz_launch("down_exl3s", sz_xw_down_kernel<K, TT>, grid, block, SzXW<K, TT>::SMEM_BYTES, st, true, plan, (const u8*)L->gate, (u64)L->gate_stride, \
                           (const u8*)L->up, (u64)L->up_stride, (const u8*)L->down, (u64)L->down_stride, (const u8*)(sh ? L->sh_gate : 0),   \
                           (const u8*)(sh ? L->sh_up : 0), (const u8*)(sh ? L->sh_down : 0), m, (int)L->hidden, (int)L->expert_ff, (int)L->top_k, \
                           (const long long*)acc_gu, acc_d, ctrl));                                                                          \
         rc = SZ_OK;                                                                                                                         \
     }
-        if constexpr (NTC % 4 == 0) { SZ_XW_GU(4, 2) SZ_XW_GU(4, 3) }
-        if constexpr (NTC % 2 == 0) { SZ_XW_GU(2, 2) SZ_XW_GU(2, 3) }
-        SZ_XW_GU(1, 2) SZ_XW_GU(1, 3)
+        if constexpr (NTC % 4 == 0) { SZ_XW_GU(4) }
+        if constexpr (NTC % 2 == 0) { SZ_XW_GU(2) }
+        SZ_XW_GU(1)
         if (rc) return sz_fail(SZ_E_TYPE, "no gate/up kernel for this unit shape");
         rc = SZ_E_TYPE;
-        SZ_XW_DN(4, 2) SZ_XW_DN(4, 3) SZ_XW_DN(2, 2) SZ_XW_DN(2, 3) SZ_XW_DN(1, 2) SZ_XW_DN(1, 3)
+        SZ_XW_DN(4) SZ_XW_DN(2) SZ_XW_DN(1)
         if (rc) return sz_fail(SZ_E_TYPE, "no down kernel for this unit shape");
         return SZ_OK;
 #undef SZ_XW_GU

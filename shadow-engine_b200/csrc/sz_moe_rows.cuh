@@ -300,22 +300,6 @@ __device__ __forceinline__ void sz_rows_read(const float* done, const long long*
     for (int e = 0; e < 4; e++) v[e] = (float)((double)a[e] * SZ_FIX_INV);
 }
 
-// A row's 128 rotated values as the row's share of the B fragments: value k of the row at lane k & 31, register k >> 5.  In the
-// fragment order a row owns 32 whole 16-byte pieces - (tile row kr, quad q): values 16 kr + 2 q, + 1 and + 8, + 9 as f16 high parts,
-// then the low parts - so the values change lanes through `buf` (128 floats of the warp's own) and every lane makes one piece.
-__device__ __forceinline__ uint4 sz_rows_piece(float* v, float* buf, int lane) {
-    sz_wht128_warp(v, lane);
-    __syncwarp();
-#pragma unroll
-    for (int e = 0; e < 4; e++) buf[lane + 32 * e] = v[e] * SZ_RSQRT128;
-    __syncwarp();
-    const int at = 16 * (lane >> 2) + 2 * (lane & 3);
-    const float2 x0 = *(const float2*)(buf + at), x1 = *(const float2*)(buf + at + 8);
-    const __half2 h0 = __floats2half2_rn(x0.x, x0.y), h1 = __floats2half2_rn(x1.x, x1.y);
-    const __half2 l0 = __floats2half2_rn(x0.x - __low2float(h0), x0.y - __high2float(h0)), l1 = __floats2half2_rn(x1.x - __low2float(h1), x1.y - __high2float(h1));
-    return make_uint4(*(const u32*)&h0, *(const u32*)&h1, *(const u32*)&l0, *(const u32*)&l1);
-}
-
 #define SZ_ROWS_CW 16             // consumer warps
 #define SZ_ROWS_PW 4              // gate / up: warps that make the fragments (rows p, p + 4, .. of a group; warp 0 of them copies, too)
 template <int K, int TW>
@@ -403,7 +387,7 @@ sz_rows_gateup_kernel(const SzRowsPlan* __restrict__ P, const u8* __restrict__ g
                 if (t < n) {
 #pragma unroll
                     for (int e = 0; e < 4; e++) v[r][e] *= sc[e];
-                    frag[(t >> 3) * 256 + 4 * (t & 7)] = sz_rows_piece(v[r], buf[p], lane);
+                    frag[(t >> 3) * 256 + 4 * (t & 7)] = sz_xw_piece(v[r], buf[p], lane);
                 }
             }
             __syncwarp();
@@ -483,7 +467,7 @@ sz_rows_act_kernel(const SzRowsPlan* __restrict__ P, const u8* __restrict__ gate
         const float gv = (gg[e] * SZ_RSQRT128) * sc[e], uv = (uu[e] * SZ_RSQRT128) * sc[4 + e];
         v[e] = (sz_silu(gv) * uv) * sc[8 + e];
     }
-    frags[((size_t)g * KB + kb) * 512 + (t >> 3) * 256 + (lane >> 2) * 32 + 4 * (t & 7) + (lane & 3)] = sz_rows_piece(v, buf[warp], lane);
+    frags[((size_t)g * KB + kb) * 512 + (t >> 3) * 256 + (lane >> 2) * 32 + 4 * (t & 7) + (lane & 3)] = sz_xw_piece(v, buf[warp], lane);
 }
 
 // ---- down: dn[slot][H] = the pairs' sums -------------------------------------------------------------------------------------------------
