@@ -803,19 +803,20 @@ static int sz_hc_read_rows(const sz_session* s, cudaStream_t st, const sz_hc& hc
                               B.rn, acc_next));
             static bool set = false;
             if (!set) {
-                SZ_CUDA(cudaFuncSetAttribute(sz_hc_down_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024));
+                SZ_CUDA(cudaFuncSetAttribute(sz_hc_down_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SzHcDownRows::SMEM));
                 SZ_CUDA(cudaFuncSetAttribute(sz_hc_up_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SzHcUpRows::SMEM));
                 set = true;
             }
-            // Few rows: a thread a matrix row and 8 rows of the step a block (28 us at 80 rows, where the tiled form has 40 blocks of the
-            // chip's 148 and takes 46); from 129 rows on the tiles (68 us at 256 against 82), the columns in 16 parts of 512.
-            if (rows <= 128) {
+            // Few rows: a thread a matrix row and 8 rows of the step a block; from 56 rows on the tiles, the columns in as many parts as fill the
+            // chip (a prompt's whole chunk, 48 layers, both ways: 48 rows 31.6 / 31.7 ms, 56 33.8 / 33.4, 72 37.1 / 36.4, 264 67.9 / 63.7).
+            if (rows <= 48) {
                 SZ_CUDA(sz_launch("hc_rows_down", sz_hc_rows_down_kernel<8>, dim3(CH / 64, rows / 8), dim3(nt), 0, st, true, (const float*)B.rn, (const u8*)hc.down.data,
                                   (const u8*)(inject ? hc.inject.data : 0), H, C, (int)c.hc_rank, acc));
                 SZ_CUDA(sz_launch("hc_rows_act", sz_hc_rows_act_kernel, dim3(rows), dim3(256), 0, st, true, (const long long*)acc, C, B.hd));
             } else {
-                SZ_CUDA(sz_launch("hc_down_rows", sz_hc_down_rows_kernel, dim3(16, (rows + SZ_HC_M - 1) / SZ_HC_M), dim3(288), sz_hc_down_rows_smem(CH / 16), st, true,
-                                  (const float*)B.rn, (const u8*)hc.down.data, (const u8*)(inject ? hc.inject.data : 0), H, rows, B.hd, acc));
+                const int tiles = (rows + SZ_HC_M - 1) / SZ_HC_M * (256 / SZ_HC_N), parts = tiles < sz_sm_count_session() ? sz_sm_count_session() / tiles : 1;
+                SZ_CUDA(sz_launch("hc_down_rows", sz_hc_down_rows_kernel, dim3(tiles, parts), dim3(32 * SZ_HC_W), SzHcDownRows::SMEM, st, true, (const float*)B.rn,
+                                  (const u8*)hc.down.data, (const u8*)(inject ? hc.inject.data : 0), H, rows, B.hd, acc));
             }
             SZ_CUDA(sz_launch("hc_up_rows", sz_hc_up_rows_kernel, dim3(H / 16, (rows + SZ_HC_UP_ROWS - 1) / SZ_HC_UP_ROWS), dim3(128), SzHcUpRows::SMEM, st, true,
                               (const float*)B.hd, (const u8*)hc.up.data, (const float*)B.rn, H, rows, B.u));

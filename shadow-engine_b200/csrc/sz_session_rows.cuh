@@ -37,130 +37,205 @@ sz_rows_embed_kernel(const SzSeqDev* __restrict__ seqs, const int32_t* __restric
 
 // ---- the read over many rows at the usual shape (rank 256, 4 streams) -------------------------------------------------------------------
 // Both halves are matrix products on the FMA pipe whose additions keep the pass's order (sz_hc_down_body, sz_hc_up_body), so what is left
-// to choose is how often an operand is loaded.  Measured a launch at 256 rows (hidden 2048): first half 82 -> 68, second half 126 -> 55 us
-// (80 rows: 45 -> 25), where the multiply-adds alone take 15 and 14 us of the whole chip; loads from shared memory bound both.
+// to choose is how often an operand is loaded.
 //
-// First half.  A block takes 32 rows and 1 / gridDim.x of the C*H columns.  Its rows of rn and, 64 columns at a time in two buffers, the
-// matrix sit in shared memory; a thread sums 8 outputs of 4 rows, so that a loaded word feeds four multiply-adds (with a matrix row a
-// thread every input was loaded by every thread: the loads took twice the multiply-adds' time).  Per 64 columns the sums are rounded to
-// fixed point as the pass's kernel rounds them and added up as integers in shared memory, and the block adds them to the accumulator
-// once (128 atomics a value before, now 16).  The last block of a row tile finishes silu(down / C), so the second half reads plain
-// f32.  A ninth warp takes the inject rows.  (Clusters that added up over shared memory were tried: eight blocks that must share a GPC
-// left the chip in two waves, 127 us at 256 rows.)
+// First half.  A block takes 32 rows and 32 of the 256 outputs over 1 / gridDim.y of the C*H columns; its warps share the columns, 64 at a
+// time, each with two buffers of its own (32 columns by asynchronous copies) and no barrier between them: per 64 columns the sums are rounded to fixed
+// point as the pass's kernel rounds them, and integers may be added in any order - in registers, at the end over the warps, and over
+// gridDim.y blocks by atomics where a launch of few rows needs them to fill the chip.  A thread sums 8 outputs of 4 rows, two outputs an
+// instruction (fma.rn.f32x2: each half is the pass's multiply-add).  silu(down / C) is finished here, so the second half reads plain f32.  The
+// inject rows are dealt out: block j of a row tile's eight sums those of rows 4 j .. 4 j + 3, a chain a lane.
+// Measured (us a launch, events between the launches; 32 rows x all outputs a block over a sixteenth of the columns -> this): 504 rows 118 -> 86,
+// 264 68 -> 53; against a thread a matrix row, 8 rows a block and a launch for silu: 80 rows 34 + 6 -> 27.  The multiply-adds alone would take 30 us
+// at 504 rows; what bounds it is the loop over them (plain multiply-adds instead of pairs: 99; without rounding 82; with no copies after the
+// first the same; 8 warps instead of 12: 91).  More columns a block and atomics between more blocks were tried first: the atomics (2 M of
+// them at the end of a launch) cost what the fuller chip gave.
 #define SZ_HC_K 64        // columns between two roundings
-#define SZ_HC_WS 144      // bytes between two staged matrix rows
+#define SZ_HC_W 12        // warps a block
+#define SZ_HC_S 32        // columns a stage
+#define SZ_HC_WS (2 * SZ_HC_S + 16)      // bytes between two staged matrix rows
+#define SZ_HC_XS (4 * SZ_HC_S + 16)      // bytes between two staged rows of the step
 #define SZ_HC_M 32        // rows a block
-#define SZ_HC_TICKET 264  // the accumulator's word that counts a row tile's finished blocks (cleared with it)
-static inline size_t sz_hc_down_rows_smem(int part) { return (size_t)SZ_HC_M * (part + 4) * 4 + 2 * 260 * SZ_HC_WS + (size_t)SZ_HC_M * 260 * 8; }
-// a rounded to 2^-40 as __double2ll_rn((double)a * 2^40) rounds it: 1.5 * 2^12 puts the last place of the sum there
+#define SZ_HC_N 32        // outputs a block
+#define SZ_HC_TICKET 264  // the accumulator's words that count a tile's finished blocks, a word a tile of outputs (cleared with it)
+#define SZ_HC_STAGE (SZ_HC_M * SZ_HC_XS + (SZ_HC_N + 4) * SZ_HC_WS)
+struct SzHcDownRows { static constexpr int SMEM = SZ_HC_W * 2 * SZ_HC_STAGE; };
+__device__ __forceinline__ void sz_fma2(u64& a, u64 f, u64 x) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(a) : "l"(f), "l"(x)); }
+__device__ __forceinline__ u64 sz_pack2(u32 a, u32 b) { u64 d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(a), "r"(b)); return d; }
+// the halves rounded to 2^-40 as __double2ll_rn((double)a * 2^40) rounds them, + the bits of 6144 = 1.5 * 2^12 (which puts the last place there):
+// all is well while the exponents say so (and, or: of the results' upper words), else sz_hc_fix does it
+#define SZ_HC_MAGIC 0x40B8000000000000ll
 __device__ __forceinline__ long long sz_hc_fix(float a) {
-    if (fabsf(a) < 2048.0f) return __double_as_longlong((double)a + 6144.0) - __double_as_longlong(6144.0);
+    if (fabsf(a) < 2048.0f) return __double_as_longlong((double)a + 6144.0) - SZ_HC_MAGIC;
     return __double2ll_rn((double)a * SZ_HC_FIX);
 }
-// grid (column parts, ceil(rows / 32)), block 288; hd: f32 [rows][256]; acc: zero on entry
-__global__ void __launch_bounds__(288, 1)
+template <int N>
+__device__ __forceinline__ void sz_hc_round(const u64* a, long long* sum) {      // N pairs
+    u32 all = 0xffffffffu, any = 0u;
+#pragma unroll
+    for (int i = 0; i < 2 * N; i++) {
+        const u32 hi = (u32)__double2hiint((double)__uint_as_float((u32)(a[i >> 1] >> (32 * (i & 1)))) + 6144.0);
+        all &= hi; any |= hi;
+    }
+    if ((all >> 20) == 0x40Bu && (any >> 20) == 0x40Bu) {
+#pragma unroll
+        for (int i = 0; i < 2 * N; i++) sum[i] += __double_as_longlong((double)__uint_as_float((u32)(a[i >> 1] >> (32 * (i & 1)))) + 6144.0);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 2 * N; i++) sum[i] += sz_hc_fix(__uint_as_float((u32)(a[i >> 1] >> (32 * (i & 1))))) + SZ_HC_MAGIC;
+    }
+}
+// grid (8 row tiles, column parts), block 32 SZ_HC_W; hd: f32 [rows][256]; acc: zero on entry
+__global__ void __launch_bounds__(32 * SZ_HC_W, 1)
 sz_hc_down_rows_kernel(const float* __restrict__ rn, const u8* __restrict__ down, const u8* __restrict__ inject, int H, int rows, float* __restrict__ hd,
                        long long* __restrict__ acc) {
-    constexpr int C = 4, RANK = 256, OUTS = RANK + C, M = SZ_HC_M, OT = 8, OG = RANK / OT;
+    constexpr int C = 4, RANK = 256, NT = RANK / SZ_HC_N;
     extern __shared__ __align__(128) u8 smem[];
+    __shared__ long long isums[SZ_HC_W][16];
     __shared__ int s_last;
-    const int CH = C * H, part = CH / gridDim.x, xst = part + 4, k0 = blockIdx.x * part, row0 = blockIdx.y * M;
-    float* xs = (float*)smem;                                               // [M][part + 4]
-    u8* ws = smem + (size_t)M * xst * 4;                                    // [2][OUTS][SZ_HC_WS]
-    long long* sums = (long long*)(ws + 2 * OUTS * SZ_HC_WS);               // [M][OUTS]
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-    const int nout = inject != nullptr ? OUTS : RANK;
-    auto stage = [&](int s, int buf) {      // columns s .. s + 63 of every matrix row
-        for (int i = t; i < nout * 8; i += 288) {
-            const int o = i >> 3;
-            const u8* src = (o < RANK ? down + ((size_t)o * CH + k0 + s) * 2 : inject + ((size_t)(o - RANK) * CH + k0 + s) * 2) + 16 * (i & 7);
-            sz_cp_async16(ws + (size_t)(buf * OUTS + o) * SZ_HC_WS + 16 * (i & 7), src);
-        }
-        sz_cp_async_commit();
+    const int CH = C * H, NK = CH / SZ_HC_K, P = gridDim.y;
+    const int row0 = (int)blockIdx.x / NT * SZ_HC_M, nt = (int)blockIdx.x % NT, n0 = nt * SZ_HC_N;
+    const int k0 = NK * (int)blockIdx.y / P, k1 = NK * ((int)blockIdx.y + 1) / P;     // the block's pieces of 64 columns; a warp takes every SZ_HC_W-th
+    u8* mine = smem + (size_t)warp * 2 * SZ_HC_STAGE;
+    const bool injects = inject != nullptr;
+    // a warp's stages: number i is half i & 1 of its piece i >> 1, in buffer i & 1
+    const int NI = k0 + warp < k1 ? 2 * ((k1 - k0 - warp + SZ_HC_W - 1) / SZ_HC_W) : 0;
+    auto col = [&](int i) { return (k0 + warp + (i >> 1) * SZ_HC_W) * SZ_HC_K + (i & 1) * SZ_HC_S; };
+    auto stage_w = [&](int i) {
+        u8* d = mine + (i & 1) * SZ_HC_STAGE + SZ_HC_M * SZ_HC_XS;
+        const u8* src = down + ((size_t)(n0 + (lane >> 2)) * CH + col(i)) * 2 + 16 * (lane & 3);
+#pragma unroll
+        for (int q = 0; q < SZ_HC_N / 8; q++) sz_cp_async16(d + (8 * q + (lane >> 2)) * SZ_HC_WS + 16 * (lane & 3), src + (size_t)q * 16 * CH);
+        if (injects && lane < 16) sz_cp_async16(d + (SZ_HC_N + (lane >> 2)) * SZ_HC_WS + 16 * (lane & 3), inject + ((size_t)(lane >> 2) * CH + col(i)) * 2 + 16 * (lane & 3));
     };
-    stage(0, 0);                            // (constant data: ahead of the wait)
-    for (int i = t; i < M * OUTS; i += 288) sums[i] = 0;
+    auto stage_x = [&](int i) {                     // (rows past the last one repeat it; nobody keeps their sums)
+        u8* d = mine + (i & 1) * SZ_HC_STAGE + 16 * (lane & 7);
+        const float* src = rn + col(i) + 4 * (lane & 7);
+#pragma unroll
+        for (int q = 0; q < SZ_HC_M / 4; q++) {
+            const int r = 4 * q + (lane >> 3), row = row0 + r < rows ? row0 + r : rows - 1;
+            sz_cp_async16(d + r * SZ_HC_XS, src + (size_t)row * CH);
+        }
+    };
+    if (NI) stage_w(0);                             // (constant data: ahead of the wait)
     sz_pdl_wait();
     sz_pdl_trigger();
-    for (int i = t; i < M * part / 4; i += 288) {
-        const int j = i / (part / 4), c = i - j * (part / 4);
-        if (row0 + j < rows) sz_cp_async16(xs + (size_t)j * xst + 4 * c, rn + (size_t)(row0 + j) * CH + k0 + 4 * c);
-        else *(float4*)(xs + (size_t)j * xst + 4 * c) = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
+    if (NI) stage_x(0);
     sz_cp_async_commit();
-    // a thread's outputs og + 32 i and rows rg + 8 j
-    const int og = (warp & 3) * 8 + (lane & 7), rg = (warp >> 2) * 4 + (lane >> 3);
-    for (int s = 0, buf = 0; s < part; s += SZ_HC_K, buf ^= 1) {
-        sz_cp_async_wait<0>();
-        __syncthreads();                    // the buffer at hand has landed, and nobody reads the other any more
-        if (s + SZ_HC_K < part) stage(s + SZ_HC_K, buf ^ 1);
-        if (warp < 8) {
-            float a[OT][4];
+    // a thread's outputs og + 4 i and rows rg + 8 j; inject row lane & 3 of row 4 nt + (lane >> 2) (lanes 0 .. 15)
+    const int og = lane & 3, rg = lane >> 2;
+    long long sum[32], isum = 0, added = 0;         // [4 pairs of outputs][4 rows][2]
 #pragma unroll
-            for (int i = 0; i < OT; i++)
+    for (int i = 0; i < 32; i++) sum[i] = 0;
+    u64 a[4][4];
+    float b = 0.f;
+    for (int i = 0; i < NI; i++) {
+        if (i + 1 < NI) { stage_w(i + 1); stage_x(i + 1); }
+        sz_cp_async_commit();
+        sz_cp_async_wait<1>();
+        __syncwarp();
+        const u8* st = mine + (i & 1) * SZ_HC_STAGE;
+        const u8* x = st + rg * SZ_HC_XS;
+        const u8* w = st + SZ_HC_M * SZ_HC_XS + og * SZ_HC_WS;
+        if (!(i & 1)) {
 #pragma unroll
-                for (int j = 0; j < 4; j++) a[i][j] = 0.f;
-            const u8* w = ws + (size_t)(buf * OUTS + og) * SZ_HC_WS;
-            const float* x = xs + (size_t)rg * xst + s;
-#pragma unroll 4
-            for (int c = 0; c < SZ_HC_K; c += 4) {
-                float4 xv[4];
+            for (int p = 0; p < 4; p++)
 #pragma unroll
-                for (int j = 0; j < 4; j++) xv[j] = *(const float4*)(x + (size_t)j * 8 * xst + c);
-#pragma unroll
-                for (int i = 0; i < OT; i++) {
-                    const uint2 q = *(const uint2*)(w + (size_t)i * OG * SZ_HC_WS + 2 * c);
-                    const float f0 = __uint_as_float(q.x << 16), f1 = __uint_as_float(q.x & 0xffff0000u), f2 = __uint_as_float(q.y << 16), f3 = __uint_as_float(q.y & 0xffff0000u);
-#pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        a[i][j] = fmaf(f0, xv[j].x, a[i][j]);
-                        a[i][j] = fmaf(f1, xv[j].y, a[i][j]);
-                        a[i][j] = fmaf(f2, xv[j].z, a[i][j]);
-                        a[i][j] = fmaf(f3, xv[j].w, a[i][j]);
-                    }
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < OT; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) sums[(rg + 8 * j) * OUTS + og + i * OG] += sz_hc_fix(a[i][j]);
-        } else if (inject != nullptr) {     // lane: stream lane & 3, rows (lane >> 2) + 8 q
-            const int s4 = lane & 3;
-            float a[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
-            for (int c = 0; c < SZ_HC_K; c += 4) {
-                const uint2 p = *(const uint2*)(ws + (size_t)(buf * OUTS + RANK + s4) * SZ_HC_WS + 2 * c);
-                const float f0 = __uint_as_float(p.x << 16), f1 = __uint_as_float(p.x & 0xffff0000u), f2 = __uint_as_float(p.y << 16), f3 = __uint_as_float(p.y & 0xffff0000u);
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const float4 xv = *(const float4*)(xs + (size_t)((lane >> 2) + 8 * q) * xst + s + c);
-                    a[q] = fmaf(f0, xv.x, a[q]);
-                    a[q] = fmaf(f1, xv.y, a[q]);
-                    a[q] = fmaf(f2, xv.z, a[q]);
-                    a[q] = fmaf(f3, xv.w, a[q]);
-                }
-            }
-#pragma unroll
-            for (int q = 0; q < 4; q++) sums[((lane >> 2) + 8 * q) * OUTS + RANK + s4] += sz_hc_fix(a[q]);
+                for (int j = 0; j < 4; j++) a[p][j] = 0ull;
+            b = 0.f;
         }
+#pragma unroll 4
+        for (int c = 0; c < SZ_HC_S; c += 4) {
+            uint2 q[8];
+            uint4 xv[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) xv[j] = *(const uint4*)(x + j * 8 * SZ_HC_XS + 4 * c);
+#pragma unroll
+            for (int i = 0; i < 8; i++) q[i] = *(const uint2*)(w + i * 4 * SZ_HC_WS + 2 * c);
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                u64 f[4], xd[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const u32 lo = e < 2 ? q[2 * i].x : q[2 * i].y, hi = e < 2 ? q[2 * i + 1].x : q[2 * i + 1].y;
+                    f[i] = e & 1 ? sz_pack2(lo & 0xffff0000u, hi & 0xffff0000u) : sz_pack2(lo << 16, hi << 16);
+                }
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const u32 v = e == 0 ? xv[j].x : (e == 1 ? xv[j].y : (e == 2 ? xv[j].z : xv[j].w));
+                    xd[j] = sz_pack2(v, v);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+#pragma unroll
+                    for (int j = 0; j < 4; j++) sz_fma2(a[i][j], f[i], xd[j]);
+            }
+        }
+        if (injects && lane < 16) {
+            const u8* xi = st + (4 * nt + (lane >> 2)) * SZ_HC_XS;
+            const u8* wi = st + SZ_HC_M * SZ_HC_XS + (SZ_HC_N + og) * SZ_HC_WS;
+#pragma unroll
+            for (int c = 0; c < SZ_HC_S; c += 4) {
+                const uint2 q = *(const uint2*)(wi + 2 * c);
+                const float4 v = *(const float4*)(xi + 4 * c);
+                b = fmaf(__uint_as_float(q.x << 16), v.x, b);
+                b = fmaf(__uint_as_float(q.x & 0xffff0000u), v.y, b);
+                b = fmaf(__uint_as_float(q.y << 16), v.z, b);
+                b = fmaf(__uint_as_float(q.y & 0xffff0000u), v.w, b);
+            }
+        }
+        if (i & 1) {
+            sz_hc_round<16>(&a[0][0], sum);
+            added++;
+            isum += sz_hc_fix(b);
+        }
+        __syncwarp();                               // the buffer is read before the copies after the next ones fill it
     }
-    __syncthreads();
-    const int live = rows - row0 < M ? rows - row0 : M;
-    for (int i = t; i < live * OUTS; i += 288) {
-        const int j = i / OUTS, o = i - j * OUTS;
-        if (o < nout) atomicAdd((unsigned long long*)(acc + (size_t)(row0 + j) * SZ_HC_ACC_ROWS + o), (unsigned long long)sums[i]);
+    // ---- over the warps: [row][output] of a warp's sums where its buffers were
+    sz_cp_async_wait<0>();
+    __syncwarp();
+    long long* red = (long long*)mine;
+#pragma unroll
+    for (int i = 0; i < 32; i++) {
+        const int o = og + 4 * (2 * (i >> 3) + (i & 1)), r = rg + 8 * ((i >> 1) & 3);
+        red[r * (SZ_HC_N + 1) + o] = sum[i] - added * SZ_HC_MAGIC;
     }
-    __threadfence();
+    if (lane < 16) isums[warp][lane] = isum;
     __syncthreads();
-    if (t == 0) s_last = atomicAdd((unsigned long long*)(acc + (size_t)row0 * SZ_HC_ACC_ROWS + SZ_HC_TICKET), 1ull) == gridDim.x - 1;
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    for (int i = t; i < live * RANK; i += 288) {
-        const int j = i / RANK, o = i - j * RANK;
-        const float f = (float)((double)__ldcg(acc + (size_t)(row0 + j) * SZ_HC_ACC_ROWS + o) * SZ_HC_FIX_INV);
-        hd[(size_t)(row0 + j) * RANK + o] = sz_silu(f / (float)C);
+    if (injects && t < 16 && row0 + 4 * nt + (t >> 2) < rows) {
+        long long v = 0;
+#pragma unroll
+        for (int q = 0; q < SZ_HC_W; q++) v += isums[q][t];
+        atomicAdd((unsigned long long*)(acc + (size_t)(row0 + 4 * nt + (t >> 2)) * SZ_HC_ACC_ROWS + RANK + (t & 3)), (unsigned long long)v);
     }
+    const int live = warp < 8 ? rows - row0 : 0;
+    // thread: output lane of rows warp, warp + 8, ..
+    long long v[4] = {0, 0, 0, 0};
+    if (warp < 8) {
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+#pragma unroll
+            for (int q = 0; q < SZ_HC_W; q++) v[j] += *(const long long*)(smem + (size_t)q * 2 * SZ_HC_STAGE + ((warp + 8 * j) * (SZ_HC_N + 1) + lane) * 8);
+    }
+    long long* at = acc + (size_t)(row0 + warp) * SZ_HC_ACC_ROWS + n0 + lane;
+    if (P > 1) {
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (warp + 8 * j < live) atomicAdd((unsigned long long*)(at + (size_t)8 * j * SZ_HC_ACC_ROWS), (unsigned long long)v[j]);
+        __threadfence();
+        __syncthreads();
+        if (t == 0) s_last = atomicAdd((unsigned long long*)(acc + (size_t)row0 * SZ_HC_ACC_ROWS + SZ_HC_TICKET + nt), 1ull) == (unsigned long long)(P - 1);
+        __syncthreads();
+        if (!s_last) return;
+        __threadfence();
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (warp + 8 * j < live) v[j] = __ldcg(at + (size_t)8 * j * SZ_HC_ACC_ROWS);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+        if (warp + 8 * j < live) hd[(size_t)(row0 + warp + 8 * j) * RANK + n0 + lane] = sz_silu((float)((double)v[j] * SZ_HC_FIX_INV) / (float)C);
 }
 
 // silu(down / C) from the accumulator, for the first half's block-row form.  grid (rows), block 256

@@ -44,6 +44,27 @@ def test_a_prompt_in_chunks_equals_passes_of_eight_rows(dm, n):
     assert np.array_equal(a.result(logits=True)[2].view(np.uint32), b.result(logits=True)[2].view(np.uint32))
 
 
+# the reads' many-row kernels (rank 256): 48 rows are the last without tiles, 56 the first; tiles of 32 rows and what is over them.  scale: the
+# norm weights' - sums of 64 columns beyond 2^11 take the other way to fixed point, in both forms.
+@pytest.mark.parametrize("n,scale", [(49, 1.0), (57, 1.0), (65, 1.0), (73, 1.0), (137, 1.0), (513, 1.0), (65, 20000.0)])
+def test_the_reads_of_a_chunk_in_tiles_equal_the_passes(n, scale):
+    M = md.make_model(dict(CFG, hc_rank=256), expert_type=szlib.TYPE_EXL3(3), seed=6)
+    for k, t in M["tensors"].items():
+        if k.endswith("hc_attn_norm.weight") or k.endswith("hc_ffn_norm.weight"):
+            t[3].mul_(scale)
+    dm = md.DeviceModel(M)
+    prompt = md.make_prompt(n, CFG["vocab"], seed=n)
+    a, b = md.Session(dm, 560, kv_q8=True), md.Session(dm, 560, kv_q8=True)
+    a.prefill(prompt)
+    for c in range(0, n, 8):
+        b.verify(prompt[c:c + 8])
+        _, top2, lg2 = b.result(logits=True)
+        if c + 8 < n:
+            b.commit(8)
+    _, top, lg = a.result(logits=True)
+    assert np.isfinite(lg).all() and np.array_equal(lg.view(np.uint32), lg2.view(np.uint32)) and np.array_equal(top, top2)
+
+
 @pytest.mark.parametrize("n_expert,top_k,rows", [(16, 1, 8), (16, 16, 24), (16, 2, 256), (64, 4, 248), (512, 10, 136)])
 def test_groups_of_many_and_of_few_rows_an_expert(n_expert, top_k, rows):
     """16 experts of 256 rows: more rows an expert than a group takes; 512 of 136: most experts have two or three; 16 of 16: all."""
