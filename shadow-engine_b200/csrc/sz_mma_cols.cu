@@ -11,7 +11,7 @@
 // Shape of the kernel.  A block owns MT x 128 weight rows (the M side of the instruction), one tile of up to 256 tokens (the N side) and,
 // with a cluster of `ks` blocks, a part of K; the accumulators D[128 rows][NT tokens] live in tensor memory (MT x 256 columns of 128
 // lanes), so no register holds a partial sum until the end.  K advances in steps of 32 columns, one Q8_0 block a row, through a ring of
-// four stages:
+// four or eight stages:
 //   warp 18     raw Q8_0 bytes of the block's rows, 256 columns at a time (272 bytes a row: a multiple of 16, which the 34 bytes of a
 //               step are not) as MT tiled TMA copies (cp.async.bulk.tensor.2d over the matrix seen as [rows][row bytes / 2] 16-bit
 //               words, box 136 x 128; 128 separate 272-byte bulk copies a piece kept the copy engine, not the tensor core, as the bound).
@@ -20,8 +20,8 @@
 //   warps 1..16 decode, in groups of MT x 128 threads: a thread takes its group's blocks of a weight row's 272 bytes into registers -
 //               which frees the buffer for the next piece once the last word is there - and turns them block after block into f16 in the canonical K-major
 //               no-swizzle order (8 rows x 16 bytes core matrices), then fence.proxy.async and arrive.  The groups take the steps in turn.
-//   warp 17     one thread issues the step's 2 MT tcgen05.mma (K = 16 each) from shared-memory descriptors and commits them to the
-//               stage's "empty" barrier, which frees the stage for the decoders and the copy warp.
+//   warp 17     one thread issues a turn's (one or two steps') 2 MT tcgen05.mma a step (K = 16 each) from shared-memory descriptors and commits
+//               them to the turn's "empty" barrier, which frees its stages for the decoders and the copy warp.
 // After the last step the decode warps read the accumulators with tcgen05.ld (lane = weight row, column = token) and write Y: for one
 // token, the 32 lanes of a warp write 32 consecutive rows.  With ks > 1 a block of the cluster finishes its share of the columns: the
 // others store their parts of those into its shared memory (the stages' and the raw bytes', no longer needed), and it adds the parts in
@@ -30,7 +30,7 @@
 // a token tile (25 KB per 256 x 256 x 32) where one a block moved 41, and the tensor core, which needs 512 cycles of the step's 625; the
 // sums of a unit, which all blocks write at about the same time, are a fifth.  At few tokens latency: the chain decode, fence, barrier,
 // instruction.  The issuing thread took 390 cycles a step to make descriptors for 256 cycles of instructions; it makes them once.
-// 12,288 x 2,048: 4,093 tokens 281 -> 241 us (sustained, 1.4 GHz under the power cap), 256 tokens 28.8 -> 25.0;
+// 12,288 x 2,048: 4,093 tokens 281 -> 241 us (sustained, 1.4 GHz under the power cap), 256 tokens 28.8 -> 25.0 -> 22;
 // 512 x 2,048, one token: 20 -> 11.9 (K in four parts).
 // Every wait is bounded; a wait that runs out records where in the error word, and the block still frees its tensor memory.
 #include <cuda.h>   // CUtensorMap and its enums; the encoder's entry point is asked of the runtime, nothing links against the driver
@@ -44,7 +44,6 @@ constexpr int MC_KT = 32;         // columns a step
 constexpr int MC_PS = 64;         // columns of a unit of the packed tokens' order
 constexpr int MC_SS = 256;        // columns a raw copy
 constexpr int MC_RAW_ROW = 272;   // bytes of a row's 8 Q8_0 blocks
-constexpr int MC_STAGES = 4;
 constexpr int MC_STEPS = MC_SS / MC_KT;   // steps a raw piece: one a Q8_0 block of a row
 constexpr int MC_KS_MAX = 4;      // blocks along K at most
 constexpr int MC_NT_MAX = 256;    // tokens a tile
@@ -57,7 +56,7 @@ constexpr size_t MC_SMEM_MIN = 116 * 1024;   // one block a multiprocessor: bloc
 constexpr u32 MC_WAIT = 4000000u; // polls before a wait gives up
 
 struct McSmem {
-    u64 full[MC_STAGES], empty[MC_STAGES], raw_full, raw_empty, acc_full, acc_empty;
+    u64 full[8], empty[8], raw_full, raw_empty, acc_full, acc_empty;
     u32 tmem_base, failed;
 };
 
@@ -133,6 +132,15 @@ __device__ __forceinline__ void mc_decode_block(const u32* W, u8* __restrict__ d
         *(uint4*)(dst + c * 16 * 128) = make_uint4(o[0], o[1], o[2], o[3]);
     }
 }
+// G: decode groups, which take the steps in turn.  TS: the steps of a turn, which have one pair of barriers and one commit; SLOTS: turns in the ring.
+// What the issuing thread does per step besides its instructions (a wait, a commit) is on the path: with one row tile - where shared memory
+// has room for eight stages - two steps share it.  12,288 x 2,048, 256 tokens: 28 -> 24.6 us, 1 token 21.8 -> 18.8; 1,024 tokens 74 -> 63; four
+// steps a turn 22.1 where two give 21.9, eight stages of one step each 28.  Many token tiles whose units are split along K, all reading at
+// once, take the old ring (512 x 2,048, 4,093 tokens: 29.7 us, 32.7 with the deep one; 2,900 tokens 25.9 / 25.4).
+template <int MT, bool DEEP> struct McTurn {
+    static_assert(!DEEP || MT == 1, "two row tiles leave no room for the deep ring");
+    static constexpr int G = MC_DEC / (MT * MC_BM), TS = DEEP ? 2 : 1, STAGES = DEEP ? 8 : 4, SLOTS = STAGES / TS;
+};
 // The block of a piece that step j takes: the decode groups in turn, each the next of its blocks.
 template <int MT>
 __device__ __forceinline__ int mc_block(int j) { constexpr int G = MC_DEC / (MT * MC_BM); return j % G * (MC_STEPS / G) + j / G; }
@@ -186,15 +194,17 @@ struct McArgs {
 };
 
 // grid: ks == 1, up to 148 blocks that take (row tile, token tile) units in turn; else (units * ks), cluster (ks).
-template <int MT>
+template <int MT, bool DEEP>
 __global__ void __launch_bounds__(MC_THREADS, 1)
 sz_mma_cols_q8_kernel(const __grid_constant__ CUtensorMap wmap, const McArgs a) {
     extern __shared__ __align__(128) u8 smem[];
     const int nt = a.nt, b_bytes = nt * MC_KT * 2;
     u8* raw = smem;                                   // [MT * 128 rows][272]
     u8* sa = raw + MT * MC_RAW_BYTES;                 // [stages][MT][4 chunks][16 row groups][128]
-    u8* sb = sa + MC_STAGES * MT * MC_A_BYTES;        // [stages][4 chunks][nt / 8 token groups][128]
-    McSmem* S = (McSmem*)(sb + MC_STAGES * b_bytes);
+    using R = McTurn<MT, DEEP>;
+    constexpr int G = R::G, TS = R::TS, SLOTS = R::SLOTS, STAGES = R::STAGES;
+    u8* sb = sa + STAGES * MT * MC_A_BYTES;           // [stages][4 chunks][nt / 8 token groups][128]
+    McSmem* S = (McSmem*)(sb + STAGES * b_bytes);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rtiles = (a.rows + MT * MC_BM - 1) / (MT * MC_BM), units = rtiles * a.tiles;
     const int kr = (int)blockIdx.x % a.ks, u0 = (int)blockIdx.x / a.ks, us = (int)gridDim.x / a.ks;
@@ -202,7 +212,7 @@ sz_mma_cols_q8_kernel(const __grid_constant__ CUtensorMap wmap, const McArgs a) 
     constexpr int LAST = MC_DEC / 32;                 // the last decode warp
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < MC_STAGES; i++) { sz_mbar_init(&S->full[i], MT * MC_BM / 32 + 1); sz_mbar_init(&S->empty[i], 1); }
+        for (int i = 0; i < SLOTS; i++) { sz_mbar_init(&S->full[i], TS * MT * MC_BM / 32 + 1); sz_mbar_init(&S->empty[i], 1); }
         sz_mbar_init(&S->raw_full, 1); sz_mbar_init(&S->raw_empty, MC_DEC / 32);
         sz_mbar_init(&S->acc_full, 1); sz_mbar_init(&S->acc_empty, MC_DEC / 32);
         S->failed = 0;
@@ -218,19 +228,21 @@ sz_mma_cols_q8_kernel(const __grid_constant__ CUtensorMap wmap, const McArgs a) 
     const u32 tmem = S->tmem_base;
     int failed = 0;
 
-    // A step's stage is its number % MC_STAGES, a unit and a piece are whole rings; k counts the steps of all units, n the units.
+    // A turn's slot is its number % SLOTS; T counts the turns of all units (a piece is whole turns of the ring), n the units.
     if (warp == 0) {
         // ---- token tiles as stages come free (what the pack kernel wrote: after the dependency wait)
         sz_pdl_wait();
         sz_pdl_trigger();
         asm volatile("fence.proxy.async.global;" ::: "memory");   // the pack kernel's stores, visible since the wait, before the copies' reads
-        for (int u = lane == 0 ? u0 : units, k = 0; u < units && !failed; u += us) {
+        for (int u = lane == 0 ? u0 : units, T = 0; u < units && !failed; u += us) {
             const u8* src = (const u8*)a.x16 + ((size_t)(u / rtiles) * (a.cols / MC_KT) + p0 * MC_STEPS) * b_bytes;
-            for (int j = 0; j < steps; j++, k++) {
-                const int st = k % MC_STAGES;
-                if (k >= MC_STAGES && !sz_mbar_wait(&S->empty[st], ((k / MC_STAGES) - 1) & 1, MC_WAIT)) { failed = 1; break; }
-                sz_mbar_expect_tx(&S->full[st], (u32)b_bytes);
-                sz_bulk_g2s(sb + st * b_bytes, src + (size_t)(j / MC_STEPS * MC_STEPS + mc_block<MT>(j % MC_STEPS)) * b_bytes, (u32)b_bytes, &S->full[st]);
+            for (int j = 0; j < steps; j += TS, T++) {
+                const int sl = T % SLOTS;
+                if (T >= SLOTS && !sz_mbar_wait(&S->empty[sl], (T / SLOTS - 1) & 1, MC_WAIT)) { failed = 1; break; }
+                sz_mbar_expect_tx(&S->full[sl], (u32)(TS * b_bytes));
+#pragma unroll
+                for (int s = 0; s < TS; s++)
+                    sz_bulk_g2s(sb + (sl * TS + s) * b_bytes, src + (size_t)((j + s) / MC_STEPS * MC_STEPS + mc_block<MT>((j + s) % MC_STEPS)) * b_bytes, (u32)b_bytes, &S->full[sl]);
             }
         }
         __syncwarp();
@@ -258,17 +270,19 @@ sz_mma_cols_q8_kernel(const __grid_constant__ CUtensorMap wmap, const McArgs a) 
             u32 phase = 0;
             for (int u = u0, n = 0; u < units && !failed; u += us, n++) {
                 if (n > 0 && !sz_mbar_wait(&S->acc_empty, (n - 1) & 1, MC_WAIT)) { failed = 7; break; }
-                for (int j = 0; j < steps; j += MC_STAGES, phase ^= 1) {
+                for (int j = 0; j < steps; j += STAGES, phase ^= 1) {
 #pragma unroll
-                    for (int st = 0; st < MC_STAGES; st++) {
-                        if (!sz_mbar_wait(&S->full[st], phase, MC_WAIT)) { failed = 5; break; }
+                    for (int sl = 0; sl < SLOTS; sl++) {
+                        if (!sz_mbar_wait(&S->full[sl], phase, MC_WAIT)) { failed = 5; break; }
                         mc_tc_fence_after();
 #pragma unroll
-                        for (int mt = 0; mt < MT; mt++)
+                        for (int st = sl * TS; st < sl * TS + TS; st++)
 #pragma unroll
-                            for (int q = 0; q < MC_KT / 16; q++)      // (addresses are in 16-byte units, in the low bits)
-                                mc_mma(tmem + mt * 256, ad + (u32)((st * MT + mt) * (MC_A_BYTES / 16) + q * 2 * MC_BM), bd + (u32)(st * (nt * MC_KT / 8) + q * 2 * nt), idesc, (j | st | q) ? 1u : 0u);
-                        mc_commit(&S->empty[st]);
+                            for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+                                for (int q = 0; q < MC_KT / 16; q++)      // (addresses are in 16-byte units, in the low bits)
+                                    mc_mma(tmem + mt * 256, ad + (u32)((st * MT + mt) * (MC_A_BYTES / 16) + q * 2 * MC_BM), bd + (u32)(st * (nt * MC_KT / 8) + q * 2 * nt), idesc, (j | st | q) ? 1u : 0u);
+                        mc_commit(&S->empty[sl]);
                     }
                     if (failed) break;
                 }
@@ -279,7 +293,7 @@ sz_mma_cols_q8_kernel(const __grid_constant__ CUtensorMap wmap, const McArgs a) 
     } else {
         // ---- decode: thread d has row d % (128 MT) and 8 / G blocks of it; then the accumulators to Y.  A warp reads the 32 lanes of
         // its quadrant (warp % 4), the four warps of a quadrant take every fourth 16 columns.
-        constexpr int G = MC_DEC / (MT * MC_BM), NW = MC_RAW_ROW / 16 / G + 1;      // 16-byte words of a group's blocks
+        constexpr int NW = MC_RAW_ROW / 16 / G + 1;      // 16-byte words of a group's blocks
         const int d = threadIdx.x - 32, g = d / (MT * MC_BM), r = d % (MT * MC_BM), mtd = r >> 7;
         u8* const dst0 = sa + mtd * MC_A_BYTES + ((r & 127) >> 3) * 128 + (r & 7) * 16;
         const int quad = warp & 3, part = (warp - 1) >> 2;
@@ -317,12 +331,12 @@ sz_mma_cols_q8_kernel(const __grid_constant__ CUtensorMap wmap, const McArgs a) 
                 mc_release_raw(&S->raw_empty, W, a.zero);
                 auto step = [&](auto I) {
                     constexpr int i = decltype(I)::value;
-                    const int k = k0 + i * G + g, st = k % MC_STAGES;
+                    const int k = k0 + i * G + g, T = k / TS, sl = T % SLOTS;
                     if (failed) return;
-                    if (k >= MC_STAGES && !mc_wait_warp(&S->empty[st], ((k / MC_STAGES) - 1) & 1)) { failed = 3; return; }
-                    mc_decode_of<G, i>(g, W, dst0 + st * MT * MC_A_BYTES);
+                    if (T >= SLOTS && !mc_wait_warp(&S->empty[sl], (T / SLOTS - 1) & 1)) { failed = 3; return; }
+                    mc_decode_of<G, i>(g, W, dst0 + k % STAGES * MT * MC_A_BYTES);
                     mc_fence_async();                 // every lane's stores, before the tensor core reads them through the async proxy:
-                    mc_arrive_warp(&S->full[st]);     // fence, warp, arrival; the issuing thread waits and goes through tcgen05.fence
+                    mc_arrive_warp(&S->full[sl]);     // fence, warp, arrival; the issuing thread waits and goes through tcgen05.fence
                 };
                 step(McInt<0>()); step(McInt<1>());
                 if constexpr (G == 2) { step(McInt<2>()); step(McInt<3>()); }
@@ -439,14 +453,14 @@ McEncodeTiled mc_encoder() {
 }
 
 
-template <int MT>
+template <int MT, bool DEEP>
 int mc_launch(const CUtensorMap& wmap, const McArgs& a, cudaStream_t st) {
-    size_t smem = MT * MC_RAW_BYTES + MC_STAGES * (MT * MC_A_BYTES + (size_t)a.nt * MC_KT * 2) + sizeof(McSmem);
+    size_t smem = MT * MC_RAW_BYTES + McTurn<MT, DEEP>::STAGES * (MT * MC_A_BYTES + (size_t)a.nt * MC_KT * 2) + sizeof(McSmem);
     if (smem < MC_SMEM_MIN) smem = MC_SMEM_MIN;
     static bool set = false;
     if (!set) {
-        SZ_CUDA(cudaFuncSetAttribute(sz_mma_cols_q8_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     MT * MC_RAW_BYTES + MC_STAGES * (MT * MC_A_BYTES + MC_NT_MAX * MC_KT * 2) + (int)sizeof(McSmem)));
+        SZ_CUDA(cudaFuncSetAttribute(sz_mma_cols_q8_kernel<MT, DEEP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     MT * MC_RAW_BYTES + McTurn<MT, DEEP>::STAGES * (MT * MC_A_BYTES + MC_NT_MAX * MC_KT * 2) + (int)sizeof(McSmem)));
         set = true;
     }
     cudaLaunchConfig_t cfg = {};
@@ -464,7 +478,7 @@ int mc_launch(const CUtensorMap& wmap, const McArgs& a, cudaStream_t st) {
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = a.ks > 1 ? 2 : 1;
-    SZ_CUDA(cudaLaunchKernelEx(&cfg, sz_mma_cols_q8_kernel<MT>, wmap, a));
+    SZ_CUDA(cudaLaunchKernelEx(&cfg, sz_mma_cols_q8_kernel<MT, DEEP>, wmap, a));
     sz_trace_mark("mma_cols_q8", st);
     return SZ_OK;
 }
@@ -511,7 +525,8 @@ extern "C" int sz_mma_cols(const sz_tensor* w, uint64_t x, int64_t xs, uint64_t 
                       (const float*)x, (long long)xs, m, cols, nt, tiles, x16));
     McArgs a;
     a.x16 = x16; a.y = (float*)y; a.ys = (long long)ys; a.rows = rows; a.cols = cols; a.m = m; a.nt = nt; a.tiles = tiles; a.ks = plan.ks; a.err = err; a.zero = 0;
-    return plan.mt == 2 ? mc_launch<2>(wmap, a, st) : mc_launch<1>(wmap, a, st);
+    if (plan.mt == 2) return mc_launch<2, false>(wmap, a, st);
+    return plan.ks > 1 && tiles * plan.ks >= 32 ? mc_launch<1, false>(wmap, a, st) : mc_launch<1, true>(wmap, a, st);
 }
 
 // Clears (init != 0) or reads the scratch's error word; reading synchronises the stream.  0: no wait of a kernel ran out.

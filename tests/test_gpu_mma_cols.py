@@ -92,3 +92,18 @@ def test_arguments_are_checked():
     import ctypes as C
     rc = op.lib.sz_mma_cols(C.byref(bad), 256, 256, 256, 128, 1, op.scratch.data_ptr(), op.scratch.numel(), 0)
     assert rc == szlib.E_TYPE if hasattr(szlib, "E_TYPE") else rc != 0
+
+
+@pytest.mark.parametrize("rows,cols,m", [(200, 1024, 3830), (200, 1024, 3850), (130, 256, 513)])
+def test_token_tiles_either_side_of_the_deep_rings_rule(rows, cols, m):
+    # K in two parts: 15 token tiles take the deep ring, 16 the shallow one; 256 columns are one turn of the deep ring
+    wb = make(rows, cols, 31)
+    x = synth.normal((m, cols), 1.0, 33, "mma_cols.x")
+    op = mc.MmaCols(wb, rows, cols, m)
+    y = op(x.cuda())
+    assert op.status() == 0
+    w16 = torch.from_numpy(ob.dequant(ob.Q8_0, wb.numpy()).reshape(rows, cols)).half().double()
+    x16 = x.half().double()
+    want, mag = x16 @ w16.T, x16.abs() @ w16.abs().T
+    # (f32 accumulation of `cols` products: each partial sum is off by at most 2^-23 of the magnitudes summed so far)
+    assert float(((y.cpu().double() - want).abs() / (cols * 2.0 ** -23 * mag + 1e-30)).max()) < 1.0
