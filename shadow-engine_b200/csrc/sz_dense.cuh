@@ -298,11 +298,38 @@ __device__ __forceinline__ void sz_mma16816_zn(float* c, const u32* a, u32 b0, u
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+template <bool V> struct SzBool { static constexpr bool value = V; };
+
 // two int8 codes (the low 16 bits of p) as an f16 pair
 __device__ __forceinline__ u32 sz_q8_pair(u32 p) {
     const u32 t = __byte_perm(p ^ 0x8080u, 0x64646464u, 0x4140);  // 0x64 b1' 0x64 b0' with b' = b ^ 0x80
     const __half2 h = __hsub2(*(const __half2*)&t, __halves2half2(__ushort_as_half((u16)0x6480), __ushort_as_half((u16)0x6480)));  // - 1152
     return *(const u32*)&h;
+}
+
+// the four codes of a word as two f16 pairs
+__device__ __forceinline__ void sz_q8_quad(u32 w, u32& lo, u32& hi) {
+    const u32 x = w ^ 0x80808080u;
+    const __half2 k = __halves2half2(__ushort_as_half((u16)0x6480), __ushort_as_half((u16)0x6480));
+    const u32 a = __byte_perm(x, 0x64646464u, 0x4140), b = __byte_perm(x, 0x64646464u, 0x4342);
+    const __half2 ha = __hsub2(*(const __half2*)&a, k), hb = __hsub2(*(const __half2*)&b, k);
+    lo = *(const u32*)&ha; hi = *(const u32*)&hb;
+}
+
+// Codes 8 q .. 8 q + 7 of the Q8_0 block at p (of a row that starts at a multiple of 4 bytes; `odd`: the block's number) as the two A
+// fragments' registers of one row, and its scale.  In odd blocks the codes start at a multiple of 4, in even ones 2 behind one.
+template <bool ODD>
+__device__ __forceinline__ void sz_q8_row(const u8* p, int q, u32& a1l, u32& a1h, u32& a2l, u32& a2h, float& d) {
+    u32 c01, c23;
+    if (ODD) {
+        c01 = *(const u32*)(p + 2 + 8 * q); c23 = *(const u32*)(p + 6 + 8 * q);
+    } else {
+        const u32 w0 = *(const u32*)(p + 8 * q), w1 = *(const u32*)(p + 8 * q + 4), w2 = *(const u32*)(p + 8 * q + 8);   // (an odd block follows: no byte past the row)
+        c01 = __funnelshift_r(w0, w1, 16); c23 = __funnelshift_r(w1, w2, 16);
+    }
+    d = sz_f16_to_f32(*(const u16*)p);
+    sz_q8_quad(c01, a1l, a1h);
+    sz_q8_quad(c23, a2l, a2h);
 }
 
 struct SzDenseQ8Cfg {
@@ -342,34 +369,50 @@ static __global__ void __launch_bounds__(256, 2) sz_dense_q8_kernel(const SzDens
     };
     const int first = blockIdx.x, step = gridDim.x;
     const int count = first < total ? (total - first + step - 1) / step : 0;
-    auto issue = [&](int i) {
+    auto issue = [&](int i) {      // warp 0, a lane a row
         int ji, row0, nrows;
         locate(first + i * step, ji, row0, nrows);
         u64* bar = &bars[i % c.NS];
-        sz_mbar_expect_tx(bar, (u32)(nrows * rb));
+        if (lane == 0) sz_mbar_expect_tx(bar, (u32)(nrows * rb));
+        __syncwarp();
         u8* dst = stages + (size_t)(i % c.NS) * c.unit_bytes;
         const u8* src = a.job[ji].w + (size_t)row0 * rb;
-        for (int r = 0; r < nrows; r++) sz_bulk_g2s(dst + (size_t)r * c.rbp, src + (size_t)r * rb, (u32)rb, bar);
+        if (lane < nrows) sz_bulk_g2s(dst + (size_t)lane * c.rbp, src + (size_t)lane * rb, (u32)rb, bar);
     };
-    if (threadIdx.x == 0)
+    if (warp == 0)
         for (int i = 0; i < c.NS - 1 && i < count; i++) issue(i);
     sz_pdl_wait();
     sz_pdl_trigger();
-    for (int j = 0; j < a.m; j++)
-      for (int c4 = threadIdx.x; c4 < a.cols / 4; c4 += 256) {
-        const float4 v = __ldcg((const float4*)(a.x + (size_t)j * a.xstride) + c4);
-        const __half2 h0 = __floats2half2_rn(v.x, v.y), h1 = __floats2half2_rn(v.z, v.w);
-        const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
-        const __half2 l0 = __floats2half2_rn(v.x - f0.x, v.y - f0.y), l1 = __floats2half2_rn(v.z - f1.x, v.w - f1.y);
-        *(uint2*)(xhi + (size_t)j * c.xsp + 4 * c4) = make_uint2(*(const u32*)&h0, *(const u32*)&h1);
-        *(uint2*)(xlo + (size_t)j * c.xsp + 4 * c4) = make_uint2(*(const u32*)&l0, *(const u32*)&l1);
-    }
+    // the rows' pieces, of up to four rows and two places in flight (a piece after the other paid the way to L2 eight times at 4 rows)
+    const int pieces = a.cols / 4;
+    for (int c4 = threadIdx.x; c4 < pieces; c4 += 512)
+        for (int j0 = 0; j0 < a.m; j0 += 4) {
+            float4 v[4][2];
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+#pragma unroll
+                for (int e = 0; e < 2; e++)
+                    if (j0 + j < a.m && c4 + 256 * e < pieces) v[j][e] = __ldcg((const float4*)(a.x + (size_t)(j0 + j) * a.xstride) + c4 + 256 * e);
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+#pragma unroll
+                for (int e = 0; e < 2; e++)
+                    if (j0 + j < a.m && c4 + 256 * e < pieces) {
+                        const float4 f = v[j][e];
+                        const __half2 h0 = __floats2half2_rn(f.x, f.y), h1 = __floats2half2_rn(f.z, f.w);
+                        const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
+                        const __half2 l0 = __floats2half2_rn(f.x - f0.x, f.y - f0.y), l1 = __floats2half2_rn(f.z - f1.x, f.w - f1.y);
+                        const size_t at = (size_t)(j0 + j) * c.xsp + 4 * (c4 + 256 * e);
+                        *(uint2*)(xhi + at) = make_uint2(*(const u32*)&h0, *(const u32*)&h1);
+                        *(uint2*)(xlo + at) = make_uint2(*(const u32*)&l0, *(const u32*)&l1);
+                    }
+        }
     __syncthreads();
     const int part = a.cols / 8;          // columns of this warp: [warp * part, (warp + 1) * part), whole 32-column blocks
     const int nblk = part / 32;
     int failed = 0;
     for (int i = 0; i < count; i++) {
-        if (threadIdx.x == 0 && i + c.NS - 1 < count) issue(i + c.NS - 1);
+        if (warp == 0 && i + c.NS - 1 < count) issue(i + c.NS - 1);
         int ji, row0, nrows;
         locate(first + i * step, ji, row0, nrows);
         const SzDenseJob& jb = a.job[ji];
@@ -379,29 +422,32 @@ static __global__ void __launch_bounds__(256, 2) sz_dense_q8_kernel(const SzDens
         if (!failed) {
             const u8* r0 = st + (size_t)(g < nrows ? g : 0) * c.rbp;
             const u8* r1 = st + (size_t)(g + 8 < nrows ? g + 8 : 0) * c.rbp;
-            for (int b = 0; b < nblk; b++) {
-                const int blk = warp * nblk + b;
+            auto block = [&](int blk, auto odd) {
                 const int col = blk * 32 + 8 * q;
                 uint4 bh = make_uint4(0, 0, 0, 0), bl = make_uint4(0, 0, 0, 0);
                 if (g < a.m) {
                     bh = *(const uint4*)(xhi + (size_t)g * c.xsp + col);
                     bl = *(const uint4*)(xlo + (size_t)g * c.xsp + col);
                 }
-                const u8* p0 = r0 + (size_t)blk * 34;
-                const u8* p1 = r1 + (size_t)blk * 34;
-                const float d0 = sz_f16_to_f32(*(const u16*)p0), d1 = sz_f16_to_f32(*(const u16*)p1);
-                const u16* c0 = (const u16*)(p0 + 2 + 8 * q);
-                const u16* c1 = (const u16*)(p1 + 2 + 8 * q);
                 u32 a1[4], a2[4];
-                a1[0] = sz_q8_pair(c0[0]); a1[2] = sz_q8_pair(c0[1]); a2[0] = sz_q8_pair(c0[2]); a2[2] = sz_q8_pair(c0[3]);
-                a1[1] = sz_q8_pair(c1[0]); a1[3] = sz_q8_pair(c1[1]); a2[1] = sz_q8_pair(c1[2]); a2[3] = sz_q8_pair(c1[3]);
+                float d0, d1;
+                sz_q8_row<decltype(odd)::value>(r0 + (size_t)blk * 34, q, a1[0], a1[2], a2[0], a2[2], d0);
+                sz_q8_row<decltype(odd)::value>(r1 + (size_t)blk * 34, q, a1[1], a1[3], a2[1], a2[3], d1);
                 float t[4] = {0.f, 0.f, 0.f, 0.f};
-                sz_mma16816_z(t, a1, bh.x, bh.y);
-                sz_mma16816_z(t, a2, bh.z, bh.w);
-                sz_mma16816_z(t, a1, bl.x, bl.y);
-                sz_mma16816_z(t, a2, bl.z, bl.w);
+                sz_mma16816_zn(t, a1, bh.x, bh.y);
+                sz_mma16816_zn(t, a2, bh.z, bh.w);
+                sz_mma16816_zn(t, a1, bl.x, bl.y);
+                sz_mma16816_zn(t, a2, bl.z, bl.w);
                 acc[0] = fmaf(d0, t[0], acc[0]); acc[1] = fmaf(d0, t[1], acc[1]);
                 acc[2] = fmaf(d1, t[2], acc[2]); acc[3] = fmaf(d1, t[3], acc[3]);
+            };
+            // (the MMAs of a block are a chain of four: two blocks' run side by side; four's gain the tiny model's passes nothing but code)
+            if (!(nblk & 1)) {
+#pragma unroll 1
+                for (int blk = warp * nblk; blk < warp * nblk + nblk; blk += 2) { block(blk, SzBool<false>()); block(blk + 1, SzBool<true>()); }
+            } else {
+                for (int blk = warp * nblk; blk < warp * nblk + nblk; blk++)
+                    if (blk & 1) block(blk, SzBool<true>()); else block(blk, SzBool<false>());
             }
         }
         // the eight column parts of a row meet in shared memory
@@ -469,15 +515,6 @@ static __global__ void __launch_bounds__(256) sz_dense_rows_pack_kernel(const fl
     const __half2 l0 = __floats2half2_rn(v.x - f0.x, v.y - f0.y), l1 = __floats2half2_rn(v.z - f1.x, v.w - f1.y);
     *(uint2*)(xh + (size_t)j * cols + 4 * c4) = make_uint2(*(const u32*)&h0, *(const u32*)&h1);
     *(uint2*)(xh + (size_t)(rows + j) * cols + 4 * c4) = make_uint2(*(const u32*)&l0, *(const u32*)&l1);
-}
-
-// the four codes of a word as two f16 pairs
-__device__ __forceinline__ void sz_q8_quad(u32 w, u32& lo, u32& hi) {
-    const u32 x = w ^ 0x80808080u;
-    const __half2 k = __halves2half2(__ushort_as_half((u16)0x6480), __ushort_as_half((u16)0x6480));
-    const u32 a = __byte_perm(x, 0x64646464u, 0x4140), b = __byte_perm(x, 0x64646464u, 0x4342);
-    const __half2 ha = __hsub2(*(const __half2*)&a, k), hb = __hsub2(*(const __half2*)&b, k);
-    lo = *(const u32*)&ha; hi = *(const u32*)&hb;
 }
 
 // grid (ceil(units / NW), ceil(rows / (8 NG))), block 32 NW
