@@ -454,13 +454,22 @@ sz_hc_up_body(const long long* __restrict__ acc, const float* __restrict__ rn, i
     SZ_PH_DECL;
     SZ_PH();  // 1
     const bool on = t < 256;   // a wider block's extra warps only keep the barriers company
+    // everything the block reads from the kernel before it is in flight before the first of it is used: the accumulator, and rn of the (stream,
+    // position, row) triples the thread finishes below (16 C M of them, C at most 4: M / 4 a thread)
+    constexpr int NR = (64 * M + 255) / 256;
+    float rnv[NR];
     if (on) {
+        long long av[M];
 #pragma unroll
-        for (int j = 0; j < M; j++)
-            for (int q = t; q < rank; q += 256) {
-                const float v = (float)((double)__ldcg(acc + j * SZ_HC_ACC_ROWS + q) * SZ_HC_FIX_INV);
-                hd[j][q] = sz_silu(v / (float)C);
-            }
+        for (int j = 0; j < M; j++) av[j] = t < rank ? __ldcg(acc + j * SZ_HC_ACC_ROWS + t) : 0;    // (rank is at most 256)
+#pragma unroll
+        for (int k = 0; k < NR; k++) {
+            const int idx = t + 256 * k, lr = idx / M, j = idx - lr * M;
+            rnv[k] = idx < 16 * C * M ? __ldcg(rn + ((size_t)j * C + (lr >> 4)) * H + h0 + (lr & 15)) : 0.f;
+        }
+        if (t < rank)
+#pragma unroll
+            for (int j = 0; j < M; j++) hd[j][t] = sz_silu((float)((double)av[j] * SZ_HC_FIX_INV) / (float)C);
     }
     __syncthreads();
     SZ_PH();  // 2 hd
@@ -514,9 +523,10 @@ sz_hc_up_body(const long long* __restrict__ acc, const float* __restrict__ rn, i
     SZ_PH();  // 3 dots
     // mix * rn for each (stream, position, row), one a thread; then the mean over the streams
     if (on)
-        for (int idx = t; idx < 16 * C * M; idx += 256) {
-            const int lr = idx / M, j = idx - lr * M;
-            mixs[lr][j] = sz_sigmoid(mixs[lr][j]) * __ldcg(rn + ((size_t)j * C + (lr >> 4)) * H + h0 + (lr & 15));
+#pragma unroll
+        for (int k = 0; k < NR; k++) {
+            const int idx = t + 256 * k, lr = idx / M, j = idx - lr * M;
+            if (idx < 16 * C * M) mixs[lr][j] = sz_sigmoid(mixs[lr][j]) * rnv[k];
         }
     __syncthreads();
     if (on)
