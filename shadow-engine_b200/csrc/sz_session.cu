@@ -896,7 +896,8 @@ static int sz_scan(sz_session* s, cudaStream_t st, int l, int m, bool fused) {
     const int d = c.ssm_head_dim;
     const dim3 grid(c.ssm_v_heads * (d / 32), l >= 0 ? 1 : s->n_delta), block(2 * d);
     const char* name = l >= 0 ? "delta_scan" : "delta_replay";
-    SZ_CUDA(sz_launch(name, d == 128 ? sz_delta_scan_kernel<128> : sz_delta_scan_kernel<64>, grid, block, 0, st, true, e, nw, (int)c.ssm_k_heads, (int)c.ssm_v_heads,
+    const auto scan = tr ? (d == 128 ? sz_delta_scan_kernel<128, true> : sz_delta_scan_kernel<64, true>) : (d == 128 ? sz_delta_scan_kernel<128, false> : sz_delta_scan_kernel<64, false>);
+    SZ_CUDA(sz_launch(name, scan, grid, block, 0, st, true, e, nw, (int)c.ssm_k_heads, (int)c.ssm_v_heads,
                       c.eps, tr, s->fork));
     return SZ_OK;
 }

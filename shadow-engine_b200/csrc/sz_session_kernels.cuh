@@ -743,11 +743,13 @@ struct SzScanShared {
     float ofs[2][SZ_SCAN_RC][32];            // finished outputs of the block's columns
 };
 
-template <int D, int RW>
+// TREE: the pass or the commit of a draft tree (tr, fork); a chain's instance has neither the tables nor the state of another branch.
+template <int D, int RW, bool TREE>
 __device__ __forceinline__ void sz_delta_scan_body(const SzScanSeq& q, const float* __restrict__ norm_w, int kh, int vh, float eps,
-                                                   const SzTree* __restrict__ tr, float* __restrict__ fork, const int hd, const int cb, const int di) {
+                                                   const SzTree* __restrict__ tr_, float* __restrict__ fork, const int hd, const int cb, const int di) {
     constexpr int NW = D / RW, NT = NW * 32, RPW = SZ_SCAN_RC / NW;     // warps; rows of outputs a warp finishes
     __shared__ __align__(16) SzScanShared<D> sh;
+    const SzTree* __restrict__ tr = TREE ? tr_ : nullptr;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, col = cb * 32 + lane;
     const int kx = hd % kh;  // value heads are tiled over the key heads (forward.rs:862-864)
     const int kd = kh * D, ch = 2 * kd + vh * D;
@@ -762,8 +764,9 @@ __device__ __forceinline__ void sz_delta_scan_body(const SzScanSeq& q, const flo
     }
     // .. and so do the carried conv rows; with the usual 4 taps a thread takes its (one or two) channels for all rows of the pass, so that
     // taps and carried values are there before the wait and the rows' projections are one round of loads after it
-    const bool quick = og != nullptr && q.pp.xin != nullptr && q.pp.k == 4 && !tr;
-    float taps[2][4], prev[2][3];
+    const bool quick = og != nullptr && q.pp.xin != nullptr && q.pp.k == 4;
+    __shared__ int tpar[SZ_MAX_VERIFY + 1];     // a tree pass: the rows' parents, the rows whose state is kept
+    float taps[2][4], prev[2][3], dt = 0.f, al = 0.f;
     int chn[2];
     if (quick) {
         const float* conv = q.state[1] ? q.pp.conv1 : q.pp.conv0;
@@ -778,6 +781,7 @@ __device__ __forceinline__ void sz_delta_scan_body(const SzScanSeq& q, const flo
                 for (int t = 0; t < 3; t++) prev[e][t] = sz_ld32_here(conv + (size_t)t * ch + chn[e]);
             }
         }
+        dt = sz_ld32_here(q.pp.dt + hd); al = sz_ld32_here(q.pp.a_log + hd);
     }
     sz_pdl_wait();
     sz_pdl_trigger();
@@ -833,10 +837,44 @@ __device__ __forceinline__ void sz_delta_scan_body(const SzScanSeq& q, const flo
                     for (int j = 0; j < SZ_SCAN_RC; j++)
                         if (j < rows) x[e][j] = __ldcg(pp.xin + (size_t)j * ch + chn[e]);
                 }
+            const int bj = (int)threadIdx.x - (NT - 32);      // (the last warp has the fewest channels)
+            float bv = 0.f, av = 0.f;
+            if (bj >= 0 && bj < rows) { bv = __ldcg(pp.b + (size_t)bj * vh + hd); av = __ldcg(pp.a + (size_t)bj * vh + hd); }
+            if (tr) {      // a row's ancestors are not the rows before it: the tables beside the projections, which go through the set of rows that no pass uses
+                if (threadIdx.x < SZ_MAX_VERIFY) tpar[threadIdx.x] = tr->parents[threadIdx.x];
+                else if (threadIdx.x == SZ_MAX_VERIFY) tpar[SZ_MAX_VERIFY] = (int)tr->save;
+                __syncthreads();
+            }
 #pragma unroll
             for (int e = 0; e < 2; e++) {
                 const int c = threadIdx.x + e * NT, i = c < D ? c : (c < 2 * D ? c - D : c - 2 * D);
-                if (c < 2 * D + 32) {
+                if (c < 2 * D + 32 && tr) {
+                    float (*xr)[D] = c < D ? sh.q[1] : sh.k[1];
+                    float (*vr)[32] = sh.v[1];
+                    auto own = [&](int j) -> float& { return c < 2 * D ? xr[j][i] : vr[j][i]; };
+#pragma unroll
+                    for (int j = 0; j < SZ_SCAN_RC; j++)
+                        if (j < rows) own(j) = x[e][j];
+#pragma unroll
+                    for (int j = 0; j < SZ_SCAN_RC; j++)
+                        if (j < rows) {
+                            double acc = (double)taps[e][3] * (double)x[e][j];
+                            int up[4];
+                            up[3] = j;
+#pragma unroll
+                            for (int t = 2; t >= 0; t--) up[t] = up[t + 1] >= 0 ? tpar[up[t + 1]] : up[t + 1] - 1;     // (sz_tree_up, a step at a time)
+#pragma unroll
+                            for (int t = 0; t < 3; t++) {
+                                const int a = up[t];
+                                const float old = a == -1 ? prev[e][2] : (a == -2 ? prev[e][1] : prev[e][0]);
+                                acc += (double)taps[e][t] * (double)(a >= 0 ? own(a < 0 ? 0 : a) : old);
+                            }
+                            const float y = sz_silu((float)acc);
+                            if (c < D) sh.q[0][j][i] = y;
+                            else if (c < 2 * D) sh.k[0][j][i] = y;
+                            else { sh.v[0][j][i] = y; pp.xc[(size_t)j * ch + chn[e]] = y; }
+                        }
+                } else if (c < 2 * D + 32) {
 #pragma unroll
                     for (int j = 0; j < SZ_SCAN_RC; j++)
                         if (j < rows) {
@@ -849,6 +887,15 @@ __device__ __forceinline__ void sz_delta_scan_body(const SzScanSeq& q, const flo
                             else { sh.v[0][j][i] = y; pp.xc[(size_t)j * ch + chn[e]] = y; }
                         }
                 }
+            }
+            if (bj >= 0 && bj < rows) {
+                const int j = bj;
+                const float bt = sz_sigmoid(bv);
+                const float sp_in = av + dt;
+                const float sp = sp_in > 20.0f ? sp_in : log1pf(expf(sp_in));
+                const float dc = expf(al * sp);
+                sh.beta[0][j] = bt; sh.decay[0][j] = dc;
+                if (cb == 0) { pp.beta[j * vh + hd] = bt; pp.decay[j * vh + hd] = dc; }
             }
         } else for (int idx = threadIdx.x; idx < rows * (2 * D + 32); idx += NT) {
             const int j = idx / (2 * D + 32), c = idx - j * (2 * D + 32);
@@ -866,7 +913,7 @@ __device__ __forceinline__ void sz_delta_scan_body(const SzScanSeq& q, const flo
             else if (part3 == 1) sh.k[0][j][i] = x;
             else { sh.v[0][j][i] = x; pp.xc[(size_t)j * ch + chn] = x; }
         }
-        if (threadIdx.x < rows) {
+        if (!quick && threadIdx.x < rows) {
             const int j = threadIdx.x;
             const float bt = sz_sigmoid(pp.b[j * vh + hd]);
             const float sp_in = pp.a[j * vh + hd] + pp.dt[hd];
@@ -927,6 +974,7 @@ __device__ __forceinline__ void sz_delta_scan_body(const SzScanSeq& q, const flo
         }
     };
     int prev_row = -1;
+    float Sn[RW];           // (tree passes) the state a later branch goes on from
     for (int c0 = 0; c0 < rows; c0 += SZ_SCAN_RC) {
         const int nr = rows - c0 < SZ_SCAN_RC ? rows - c0 : SZ_SCAN_RC, set = (c0 / SZ_SCAN_RC) & 1;
         if (og) {
@@ -949,10 +997,16 @@ __device__ __forceinline__ void sz_delta_scan_body(const SzScanSeq& q, const flo
         for (int jj = 0; jj < nr; jj++) {
             const int j = pick ? q.res[2 + c0 + jj] : c0 + jj;
             if (tr && og) {
-                const int pr = tr->parents[j];
+                const int pr = quick ? tpar[j] : tr->parents[j];
                 if (pr != prev_row && pr >= 0) {          // another branch: back to the state after the parent
 #pragma unroll
-                    for (int i = 0; i < RW; i++) S[i] = fk[((size_t)pr * D + warp * RW + i) * D + col];
+                    for (int i = 0; i < RW; i++) S[i] = Sn[i];
+                }
+                // .. asked for a row ahead (a row's own parent is saved before it)
+                const int nx = j + 1 < rows ? (quick ? tpar[j + 1] : tr->parents[j + 1]) : -1;
+                if (nx >= 0 && nx != j) {
+#pragma unroll
+                    for (int i = 0; i < RW; i++) Sn[i] = fk[((size_t)nx * D + warp * RW + i) * D + col];
                 }
             }
             prev_row = j;
@@ -997,7 +1051,7 @@ __device__ __forceinline__ void sz_delta_scan_body(const SzScanSeq& q, const flo
                 }
                 sh.orun[jj][RW / 16 * warp][lane] = r0;
                 if constexpr (RW == 32) sh.orun[jj][2 * warp + 1][lane] = r1;
-                if (tr && ((tr->save >> j) & 1u)) {
+                if (tr && (((quick ? (u32)tpar[SZ_MAX_VERIFY] : tr->save) >> j) & 1u)) {
 #pragma unroll
                     for (int i = 0; i < RW; i++) fk[((size_t)j * D + warp * RW + i) * D + col] = S[i];
                 }
@@ -1035,10 +1089,10 @@ __device__ __forceinline__ void sz_delta_scan_body(const SzScanSeq& q, const flo
 }
 
 // grid (vh * D / 32, layers), cluster D / 32
-template <int D>
+template <int D, bool TREE>
 __global__ void __cluster_dims__(D / 32, 1, 1) __launch_bounds__(2 * D)
 sz_delta_scan_kernel(const SzScanSeq q, const float* __restrict__ norm_w, int kh, int vh, float eps, const SzTree* __restrict__ tr, float* __restrict__ fork) {
-    sz_delta_scan_body<D, 16>(q, norm_w, kh, vh, eps, tr, fork, (int)blockIdx.x / (D / 32), (int)blockIdx.x % (D / 32), (int)blockIdx.y);
+    sz_delta_scan_body<D, 16, TREE>(q, norm_w, kh, vh, eps, tr, fork, (int)blockIdx.x / (D / 32), (int)blockIdx.x % (D / 32), (int)blockIdx.y);
 }
 
 // The pass of one layer for SEVERAL sequences in one launch (a batched step, prompts): block row b is sequence b's scan, its pointers
@@ -1050,7 +1104,7 @@ sz_delta_scan_seqs_kernel(const SzScanSeq* __restrict__ tab, const float* __rest
     static_assert(sizeof(SzScanSeq) % 8 == 0 && sizeof(SzScanSeq) / 8 <= 2 * 64, "copied in 8-byte words");
     if (threadIdx.x < sizeof(SzScanSeq) / 8) ((u64*)&q)[threadIdx.x] = ((const u64*)(tab + blockIdx.y))[threadIdx.x];
     __syncthreads();
-    sz_delta_scan_body<D, 16>(q, norm_w, kh, vh, eps, (const SzTree*)nullptr, (float*)nullptr, (int)blockIdx.x / (D / 32), (int)blockIdx.x % (D / 32), 0);
+    sz_delta_scan_body<D, 16, false>(q, norm_w, kh, vh, eps, (const SzTree*)nullptr, (float*)nullptr, (int)blockIdx.x / (D / 32), (int)blockIdx.x % (D / 32), 0);
 }
 
 // ---- attention front end (forward.rs:908-927): per head RMSNorm + NeoX RoPE of q and k, K and V into the cache.

@@ -471,7 +471,7 @@ sz_rows_scan_kernel(const SzSeqDev* __restrict__ seqs, int di, const float* __re
         q.m = s.m;
     }
     __syncthreads();
-    sz_delta_scan_body<D, 32>(q, norm_w, kh, vh, eps, (const SzTree*)nullptr, (float*)nullptr, (int)blockIdx.x / (D / 32), (int)blockIdx.x % (D / 32), 0);
+    sz_delta_scan_body<D, 32, false>(q, norm_w, kh, vh, eps, (const SzTree*)nullptr, (float*)nullptr, (int)blockIdx.x / (D / 32), (int)blockIdx.x % (D / 32), 0);
 }
 
 // After a step: the sequences whose rows were all kept move on, and what a kernel over all rows raised in the step's error word becomes
