@@ -69,7 +69,7 @@ sz_route_kernel(const float* __restrict__ x, int H, const float* __restrict__ ro
     __shared__ int sel[SZ_MAX_VERIFY * SZ_MAX_TOPK];
     __shared__ int s_last;
     __shared__ float tk_red[SZ_ROUTE_THREADS / 32];
-    __shared__ u64 tk_max[SZ_ROUTE_THREADS];
+    __shared__ __align__(16) u64 tk_max[SZ_ROUTE_THREADS];
     __shared__ u64 tk_floor[SZ_MAX_VERIFY];
     __shared__ int tk_cnt[SZ_MAX_VERIFY];
     __shared__ u64 tk_cand[MP][SZ_MAX_TOPK * (SZ_MAX_EXPERTS / (SZ_ROUTE_THREADS / MP))];
@@ -238,8 +238,11 @@ sz_route_kernel(const float* __restrict__ x, int H, const float* __restrict__ ro
         if (g == 0) tk_cnt[j] = 0;
         __syncthreads();
         int rank = 0;
-#pragma unroll 4
-        for (int i = 0; i < G; i++) rank += tk_max[j * G + i] > best;
+#pragma unroll 8
+        for (int i = 0; i < G; i += 2) {      // (two keys a load: 256 of them a row are 2,048 loads of the block at one row)
+            const ulonglong2 m2 = *(const ulonglong2*)&tk_max[j * G + i];
+            rank += (m2.x > best) + (m2.y > best);
+        }
         if (live_row && rank == k - 1) tk_floor[j] = best;   // keys are distinct, so exactly one thread has this rank
         __syncthreads();
         const u64 fl = live_row ? tk_floor[j] : ~0ull;

@@ -479,7 +479,7 @@ sz_x3_down_kernel(const SzPlan* __restrict__ plan, const u8* __restrict__ gate, 
 
 // ---- combine ----------------------------------------------------------------------------------------------------------------------
 // y[j] = sum over ranks of w * (H eo * svh) + sigmoid(shared gate logit) * (H so * svh_shared).  A block a (row, 128-output block);
-// warp t finishes rank t's contribution (warp top_k: the shared expert's), then warp 0 adds them in rank order in f64.
+// warp t finishes rank t's contribution (warp top_k: the shared expert's), then a thread an output adds them in rank order in f64.
 // so_f32 != null: the shared expert's output comes finished (f32 [m][H]) from the generic kernels instead of the accumulators.
 static __global__ void __launch_bounds__((SZ_MAX_TOPK + 1) * 32)
 sz_x3_combine_kernel(const long long* __restrict__ out, const int32_t* __restrict__ ridx, const double* __restrict__ rw,
@@ -543,29 +543,31 @@ sz_x3_combine_kernel(const long long* __restrict__ out, const int32_t* __restric
         for (int q = 0; q < 4; q++) part[top_k][lane + 32 * q] = sg * v[q];
     }
     __syncthreads();
+    if (!y_fix) {      // an output a thread (four a lane of one warp took the terms' chain four times)
+        for (int i = threadIdx.x; i < 128; i += blockDim.x) {
+            double a = 0.0;
+            for (int t = 0; t < top_k; t++) a += rws[t] * (double)part[t][i];
+            if (has_shared) a += (double)part[top_k][i];
+            y[(size_t)j * H + b * 128 + i] = (float)a;
+        }
+        return;
+    }
     if (warp == 0) {
 #pragma unroll
-        for (int e = 0; e < 4; e++) {
+        for (int e = 0; e < 4; e++) {      // every term in 64-bit fixed point: the sum over ranks is then exact
             const int i = lane + 32 * e;
-            if (y_fix) {  // every term in 64-bit fixed point: the sum over ranks is then exact
-                long long f = 0;
-                for (int t = 0; t < top_k; t++)
-                    if (local[t]) f += __double2ll_rn(rws[t] * (double)part[t][i] * 1099511627776.0);
-                if (has_shared) f += __double2ll_rn((double)part[top_k][i] * 1099511627776.0);
-                if (push.world > 0) {
-                    for (int r = 0; r < push.world; r++)
-                        sz_ep_slot(push.buf[r], push.world, push.row_elems, slot, push.me)[(size_t)j * H + b * 128 + i] = f;
-                } else {
-                    y_fix[(size_t)j * H + b * 128 + i] = f;
-                }
+            long long f = 0;
+            for (int t = 0; t < top_k; t++)
+                if (local[t]) f += __double2ll_rn(rws[t] * (double)part[t][i] * 1099511627776.0);
+            if (has_shared) f += __double2ll_rn((double)part[top_k][i] * 1099511627776.0);
+            if (push.world > 0) {
+                for (int r = 0; r < push.world; r++)
+                    sz_ep_slot(push.buf[r], push.world, push.row_elems, slot, push.me)[(size_t)j * H + b * 128 + i] = f;
             } else {
-                double a = 0.0;
-                for (int t = 0; t < top_k; t++) a += rws[t] * (double)part[t][i];
-                if (has_shared) a += (double)part[top_k][i];
-                y[(size_t)j * H + b * 128 + i] = (float)a;
+                y_fix[(size_t)j * H + b * 128 + i] = f;
             }
         }
-        if (y_fix && push.world > 0) {  // the block's stores are out: make them visible system-wide, then announce them to every rank
+        if (push.world > 0) {  // the block's stores are out: make them visible system-wide, then announce them to every rank
             __threadfence_system();
             __syncwarp();
             if (lane < push.world) atomicAdd_system(sz_ep_arrive(push.buf[lane], push.me), 1ull);
