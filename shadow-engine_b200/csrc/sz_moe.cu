@@ -573,26 +573,38 @@ __global__ void __launch_bounds__(256)
 sz_combine_kernel(const float* __restrict__ eo, const int32_t* __restrict__ ridx, const double* __restrict__ rw, const float* __restrict__ so,
                   const float* __restrict__ logits, int ne, int k, int H, int has_shared, float* __restrict__ y, long long* __restrict__ y_fix,
                   int e_lo, int e_hi, const SzEpPush push) {
-    sz_pdl_wait();
-    sz_pdl_trigger();
     const int j = blockIdx.y;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool on = i < H;
+    // weights and the shared gate come from the router, three launches back or more: asked for ahead of the wait, the outputs all at once after it
+    // (rank after rank they were as many ways to L2: 10 us a launch at k = 10)
+    double wv[SZ_MAX_TOPK];
+    float ev[SZ_MAX_TOPK];
+    u32 local = 0xffffffffu;
+#pragma unroll
+    for (int t = 0; t < SZ_MAX_TOPK; t++)
+        if (t < k) {
+            wv[t] = sz_ldg64f_here(rw + j * k + t);
+            if (y_fix) { const int e = (int)sz_ldg32_here(ridx + j * k + t); if (e < e_lo || e >= e_hi) local &= ~(1u << t); }
+        }
+    const float sg = has_shared ? sz_sigmoid(__uint_as_float(sz_ldg32_here(logits + (size_t)j * (ne + 1) + ne))) : 0.f;
+    sz_pdl_wait();
+    sz_pdl_trigger();
     const int slot = y_fix && push.world > 0 ? (int)(__ldcg(&((const SzEpHeader*)push.buf[push.me])->epoch) & 1ull) : 0;
+#pragma unroll
+    for (int t = 0; t < SZ_MAX_TOPK; t++)
+        if (on && t < k && ((local >> t) & 1u)) ev[t] = __ldcg(eo + (size_t)(j * k + t) * H + i);
+    const float sv_ = on && has_shared ? __ldcg(so + (size_t)j * H + i) : 0.f;
     double acc = 0.0;
     long long fix = 0;
-    for (int t = 0; t < (on ? k : 0); t++) {
-        if (y_fix) {
-            const int e = __ldcg(ridx + j * k + t);
-            if (e < e_lo || e >= e_hi) continue;
-            fix += __double2ll_rn(__ldcg(rw + j * k + t) * (double)__ldcg(eo + (size_t)(j * k + t) * H + i) * SZ_YFIX_SCALE);
-        } else {
-            acc += __ldcg(rw + j * k + t) * (double)__ldcg(eo + (size_t)(j * k + t) * H + i);
+#pragma unroll
+    for (int t = 0; t < SZ_MAX_TOPK; t++)
+        if (on && t < k && ((local >> t) & 1u)) {
+            if (y_fix) fix += __double2ll_rn(wv[t] * (double)ev[t] * SZ_YFIX_SCALE);
+            else acc += wv[t] * (double)ev[t];
         }
-    }
     if (has_shared && on) {
-        const float sg = sz_sigmoid(__ldcg(logits + (size_t)j * (ne + 1) + ne));
-        const double sv = (double)(sg * __ldcg(so + (size_t)j * H + i));
+        const double sv = (double)(sg * sv_);
         if (y_fix) fix += __double2ll_rn(sv * SZ_YFIX_SCALE); else acc += sv;
     }
     if (!y_fix) { if (on) y[(size_t)j * H + i] = (float)acc; return; }
