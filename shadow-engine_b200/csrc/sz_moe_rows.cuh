@@ -46,9 +46,10 @@ struct SzRowsPlan {
     int32_t start[2][SZ_ROWS_MAXB + 1];
     u32 gu_blocks[SZ_ROWS_MAXG][2], dn_blocks[SZ_ROWS_MAXG][8];
 };
-// What a unit of a group of n rows costs, in about hundredths: the decode, the second eight rows' products, a row's fragments (a share
-// of equal unit counts left blocks with several full groups 15 % behind the others).
-__device__ __forceinline__ int sz_rows_weight(int n) { return 64 + n + (n > 8 ? 5 : 0); }
+// What a unit of a group of n rows costs, in 15 ns: the decode, a row's fragments, the second eight rows' products.  Least squares over the blocks
+// of gate / up launches of 48 .. 256 rows: 2,580 ns + 15.4 a row up to eight, 3,302 + 7.5 a row beyond (1.1 us rms a block of 311; down: 2,770 and
+// 3,230 + 6).  The weights before it (64 + n, 69 + n) charged a row two and a half times what it takes: at 256 rows blocks ended from 298 to 329 us.
+__device__ __forceinline__ int sz_rows_weight(int n) { return n <= 8 ? 172 + n : 218 + n / 2; }
 
 // ---- plan: one block of 1024 threads ---------------------------------------------------------------------------------------------------
 // Every (row, rank) pair marks its row in its expert's row mask; an expert's pairs in ascending row order are then the set bits of
