@@ -61,6 +61,8 @@ sz_rows_embed_kernel(const SzSeqDev* __restrict__ seqs, const int32_t* __restric
 #define SZ_HC_STAGE (SZ_HC_M * SZ_HC_XS + (SZ_HC_N + 4) * SZ_HC_WS)
 struct SzHcDownRows { static constexpr int SMEM = SZ_HC_W * 2 * SZ_HC_STAGE; };
 __device__ __forceinline__ void sz_fma2(u64& a, u64 f, u64 x) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(a) : "l"(f), "l"(x)); }
+__device__ __forceinline__ u64 sz_mul2(u64 a, u64 b) { u64 d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ u64 sz_add2(u64 a, u64 b) { u64 d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
 __device__ __forceinline__ u64 sz_pack2(u32 a, u32 b) { u64 d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(a), "r"(b)); return d; }
 // the halves rounded to 2^-40 as __double2ll_rn((double)a * 2^40) rounds them, + the bits of 6144 = 1.5 * 2^12 (which puts the last place there):
 // all is well while the exponents say so (and, or: of the results' upper words), else sz_hc_fix does it
@@ -248,7 +250,8 @@ sz_hc_rows_act_kernel(const long long* __restrict__ acc, int C, float* __restric
 }
 
 // Second half.  A block takes 16 hidden positions (the 64 rows of the up matrix that their 4 streams have) and 32 rows of the step; a thread
-// one position and 4 rows: 16 dot products, every operand in shared memory read for four of them.  A dot product is the pass's: 32 pieces
+// one position and 4 rows: 16 dot products, two streams an instruction, every operand in shared memory read for four of them (one stream an
+// instruction: 504 rows 92 us a launch, now 72; 264 57 -> 45, 80 24.7 -> 22.7; the multiply-adds alone would take 30 us at 504 rows).  A dot product is the pass's: 32 pieces
 // of 8 multiply-adds, added as the butterfly over a row's 32 lanes adds them - pieces 16 apart first, then 8, 4, 2, 1.
 #define SZ_HC_UP_ROWS 32
 #define SZ_HC_UP_WS 264       // halves between two rows of the staged up matrix (4 (mod 32) words: the 8 rows a warp reads at once)
@@ -256,39 +259,49 @@ sz_hc_rows_act_kernel(const long long* __restrict__ acc, int C, float* __restric
 struct SzHcUpRows { static constexpr int SMEM = 64 * SZ_HC_UP_WS * 2 + SZ_HC_UP_ROWS * SZ_HC_UP_XS * 4; };
 
 struct SzHcUpAt { const u8* w; const float* x; };
-// f(4, c) of the tree: pieces c, c + 4, .. c + 28; OFF: the first offset that is added
+// f(4, c) of the tree: pieces c, c + 4, .. c + 28; OFF: the first offset that is added.  v[p][j]: streams 2 p and 2 p + 1 of row j, two an instruction.
 template <int OFF>
-__device__ __forceinline__ void sz_hc_up_tree(const SzHcUpAt& at, int c, float (*v)[4]) {
+__device__ __forceinline__ void sz_hc_up_tree(const SzHcUpAt& at, int c, u64 (*v)[4]) {
     if constexpr (OFF == 32) {
-        float4 x[4][2];
+        uint4 x[4][2];
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            x[j][0] = *(const float4*)(at.x + (size_t)j * 8 * SZ_HC_UP_XS + 8 * c);
-            x[j][1] = *(const float4*)(at.x + (size_t)j * 8 * SZ_HC_UP_XS + 8 * c + 4);
+            x[j][0] = *(const uint4*)(at.x + (size_t)j * 8 * SZ_HC_UP_XS + 8 * c);
+            x[j][1] = *(const uint4*)(at.x + (size_t)j * 8 * SZ_HC_UP_XS + 8 * c + 4);
         }
+        uint4 w[4];
 #pragma unroll
-        for (int s = 0; s < 4; s++) {
-            const uint4 w = *(const uint4*)(at.w + (size_t)s * 16 * SZ_HC_UP_WS * 2 + 16 * c);
-            const u32 ww[4] = {w.x, w.y, w.z, w.w};
-            float f[8];
+        for (int s = 0; s < 4; s++) w[s] = *(const uint4*)(at.w + (size_t)s * 16 * SZ_HC_UP_WS * 2 + 16 * c);
 #pragma unroll
-            for (int q = 0; q < 4; q++) { f[2 * q] = __uint_as_float(ww[q] << 16); f[2 * q + 1] = __uint_as_float(ww[q] & 0xffff0000u); }
+        for (int e = 0; e < 8; e++) {
+            u64 f[2], xd[4];
+#pragma unroll
+            for (int p = 0; p < 2; p++) {
+                const u32* lo = (const u32*)&w[2 * p] + (e >> 1);
+                const u32* hi = (const u32*)&w[2 * p + 1] + (e >> 1);
+                f[p] = e & 1 ? sz_pack2(*lo & 0xffff0000u, *hi & 0xffff0000u) : sz_pack2(*lo << 16, *hi << 16);
+            }
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                float a = f[0] * x[j][0].x;
-                a = fmaf(f[1], x[j][0].y, a); a = fmaf(f[2], x[j][0].z, a); a = fmaf(f[3], x[j][0].w, a);
-                a = fmaf(f[4], x[j][1].x, a); a = fmaf(f[5], x[j][1].y, a); a = fmaf(f[6], x[j][1].z, a); a = fmaf(f[7], x[j][1].w, a);
-                v[s][j] = a;
+                const u32 q = *((const u32*)&x[j][e >> 2] + (e & 3));
+                xd[j] = sz_pack2(q, q);
             }
+#pragma unroll
+            for (int p = 0; p < 2; p++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    if (e == 0) v[p][j] = sz_mul2(f[p], xd[j]);
+                    else sz_fma2(v[p][j], f[p], xd[j]);
+                }
         }
     } else {
         sz_hc_up_tree<2 * OFF>(at, c, v);
-        float b[4][4];
+        u64 b[2][4];
         sz_hc_up_tree<2 * OFF>(at, c + OFF, b);
 #pragma unroll
-        for (int s = 0; s < 4; s++)
+        for (int p = 0; p < 2; p++)
 #pragma unroll
-            for (int j = 0; j < 4; j++) v[s][j] += b[s][j];
+            for (int j = 0; j < 4; j++) v[p][j] = sz_add2(v[p][j], b[p][j]);
     }
 }
 // grid (H / 16, ceil(rows / 32)), block 128
@@ -319,19 +332,19 @@ sz_hc_up_rows_kernel(const float* __restrict__ hd, const u8* __restrict__ up, co
     sz_cp_async_wait<0>();
     __syncthreads();
     const SzHcUpAt at = {smem + (size_t)hl * SZ_HC_UP_WS * 2, xs + (size_t)rg * SZ_HC_UP_XS};
-    float a[4][4] = {}, b[4][4] = {};
+    u64 a[2][4] = {}, b[2][4] = {};
 #pragma unroll 1
     for (int it = 0; it < 4; it++) {         // f(4, 0), f(4, 2), f(4, 1), f(4, 3)
-        float v[4][4];
+        u64 v[2][4];
         sz_hc_up_tree<4>(at, it == 0 ? 0 : (it == 1 ? 2 : (it == 2 ? 1 : 3)), v);
 #pragma unroll
-        for (int s = 0; s < 4; s++)
+        for (int p = 0; p < 2; p++)
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                if (it == 0) a[s][j] = v[s][j];
-                else if (it == 1) a[s][j] += v[s][j];
-                else if (it == 2) b[s][j] = v[s][j];
-                else a[s][j] += b[s][j] + v[s][j];
+                if (it == 0) a[p][j] = v[p][j];
+                else if (it == 1) a[p][j] = sz_add2(a[p][j], v[p][j]);
+                else if (it == 2) b[p][j] = v[p][j];
+                else a[p][j] = sz_add2(a[p][j], sz_add2(b[p][j], v[p][j]));
             }
     }
 #pragma unroll
@@ -340,7 +353,7 @@ sz_hc_up_rows_kernel(const float* __restrict__ hd, const u8* __restrict__ up, co
         if (row < rows) {
             float m = 0.f;
 #pragma unroll
-            for (int s = 0; s < 4; s++) m = __fadd_rn(m, __fmul_rn(sz_sigmoid(a[s][j]), rv[s][j]));    // (rounded one by one, as the pass's kernel does)
+            for (int s = 0; s < 4; s++) m = __fadd_rn(m, __fmul_rn(sz_sigmoid(__uint_as_float((u32)(a[s >> 1][j] >> (32 * (s & 1))))), rv[s][j]));    // (rounded one by one, as the pass's kernel does)
             u[(size_t)row * H + h0 + hl] = m / (float)C;
         }
     }
