@@ -32,8 +32,7 @@ struct SzXW {
     static constexpr int FRAG_BYTES = 8 * 32 * 16;                    // the unit's activation fragments: [8 tile rows][32 lanes] uint4
     static constexpr int FIT = 200 * 1024 / (STAGE_BYTES + FRAG_BYTES);
     static constexpr int STAGES = FIT > 8 ? 8 : FIT;
-    static_assert(STAGES > SZ_XW_DECODE / SZ_XW_ITEMS, "the decode warps hold three units at a time");
-    static constexpr int SMEM_BYTES = STAGES * (STAGE_BYTES + FRAG_BYTES) + 2 * STAGES * 8;
+    static constexpr int SMEM_BYTES = STAGES * (STAGE_BYTES + FRAG_BYTES) + STAGES * (2 * 8 + 4);
 };
 
 // Two-word form of SzExl3Tile<K>::states_pre: valid when the lane's span (16 + 7 K bits) starting at its bit offset inside the
@@ -147,22 +146,49 @@ __device__ __forceinline__ uint4 sz_xw_piece(float* v, float* buf, int lane) {
     return make_uint4(*(const u32*)&h0, *(const u32*)&h1, *(const u32*)&l0, *(const u32*)&l1);
 }
 
-// What the two sides of both kernels share: the stage ring, its barriers, the units in it and the counter of items.
+// What the two sides of both kernels share: the stage ring, its barriers and whose turn a stage is.  A wait for a phase looks at its parity, so
+// it is sound only where the barrier is at most one phase behind, and the ring alone does not see to that: gate / up's producers fill units
+// out of order (and with 5 or 7 stages a stage's next unit is another producer's), a decode warp takes an item of whatever unit comes
+// next, and one that is late with a stage does not keep the others from the units after it.  Without the turns a producer refilled
+// stages that were still being read (4 bits, 6 rows, five stages: the launch failed), and a decode warp could read a stage a fill early.
+// So a stage's word says which unit it was last given to, and from a stage's second fill on whoever needs it waits for that word before the
+// barrier (in the first fill no phase can be mistaken; asking there, too, cost 0.5 us a layer, all warps polling while the first units arrive).
+// Down's producers go through all units in order and each has arrived for a stage's unit before it waits for the next: theirs needs no word.
 template <int K, int TW>
 struct SzXWRing {
     using X = SzXW<K, TW>;
     u8* stages;
     uint4* frags;
     u64 *full, *empty;
+    int* turn;
     __device__ __forceinline__ void init(u8* smem, int arrivals) {
         stages = smem;
         frags = (uint4*)(smem + X::STAGES * X::STAGE_BYTES);
         full = (u64*)(smem + X::STAGES * (X::STAGE_BYTES + X::FRAG_BYTES));
         empty = full + X::STAGES;
+        turn = (int*)(empty + X::STAGES);
         if (threadIdx.x == 0) {
-            for (int i = 0; i < X::STAGES; i++) { sz_mbar_init(&full[i], arrivals); sz_mbar_init(&empty[i], SZ_XW_ITEMS); }
+            for (int i = 0; i < X::STAGES; i++) { sz_mbar_init(&full[i], arrivals); sz_mbar_init(&empty[i], SZ_XW_ITEMS); turn[i] = -1; }
             sz_mbar_fence_init();
         }
+    }
+    // one warp: unit i has its stage (bounded; the lanes leave together)
+    __device__ __forceinline__ bool given(int i, int lane) const {
+        bool ok = lane != 0;
+        if (lane == 0) {
+            for (u32 n = 0; n < 20000000u && !ok; n++) {
+                int v;
+                asm volatile("ld.acquire.cta.shared::cta.b32 %0, [%1];" : "=r"(v) : "r"(sz_smem_addr(turn + i % X::STAGES)) : "memory");
+                ok = v == i;
+            }
+        }
+        ok = __all_sync(0xffffffffu, ok);
+        __syncwarp();
+        return ok;
+    }
+    // .. is given it (by one lane, once the unit before it has been decoded)
+    __device__ __forceinline__ void give(int i) {
+        asm volatile("st.release.cta.shared::cta.b32 [%0], %1;" ::"r"(sz_smem_addr(turn + i % X::STAGES)), "r"(i) : "memory");
     }
     // one warp: the unit's 8 tile rows, `row_stride` bytes apart in the matrix, into stage st (a lane a row: one lane after the other took 60 ns each)
     __device__ __forceinline__ void issue(int st, const u8* src, u64 row_stride, int lane) {
@@ -191,7 +217,7 @@ __device__ __forceinline__ bool sz_xw_decode(const SzXWRing<K, TW>& R, const int
         item = __shfl_sync(0xffffffffu, item, 0);
         const int i = (int)(item / SZ_XW_ITEMS), part = (int)(item % SZ_XW_ITEMS), st = i % X::STAGES;
         if (i >= count) return true;
-        if (!sz_mbar_wait(&R.full[st], (i / X::STAGES) & 1)) return false;
+        if ((i >= X::STAGES && !R.given(i, lane)) || !sz_mbar_wait(&R.full[st], (i / X::STAGES) & 1)) return false;
         float c[TW][4];
         sz_xw_compute<K, TW>(R.stages + (size_t)st * X::STAGE_BYTES, R.frags + st * 256, part, lane, LS, c);
         const int4 d = unit[st];
@@ -256,8 +282,8 @@ sz_xw_gateup_kernel(const SzPlan* __restrict__ plan, const u8* __restrict__ gate
             u16 sc[4];
 #pragma unroll
             for (int q = 0; q < 4; q++) sc[q] = __ldg(suh + 32 * q);
-            if (i >= S && !sz_mbar_wait(&R.empty[st], ((i / S) - 1) & 1)) { ok = false; break; }
-            if (lane == 0) unit[st] = make_int4(g, mat, ch * SZ_XW_ITEMS * TW * 16, 0);
+            if (i >= S && ((i >= 2 * S && !R.given(i - S, lane)) || !sz_mbar_wait(&R.empty[st], ((i / S) - 1) & 1))) { ok = false; break; }
+            if (lane == 0) { unit[st] = make_int4(g, mat, ch * SZ_XW_ITEMS * TW * 16, 0); R.give(i); }
             R.issue(st, blob + hdr + (size_t)s * 8 * mrow + (size_t)ch * X::ROW_BYTES, mrow, lane);
             uint4* frag = R.frags + st * 256 + (lane >> 2) * 32 + (lane & 3);   // (unused rows hold whatever was there: a row is a column of its own in the products)
             for (int t0 = 0; t0 < n; t0 += 4) {
@@ -326,8 +352,9 @@ sz_xw_down_kernel(const SzPlan* __restrict__ plan, const u8* __restrict__ gate, 
         int g = u0 / (KB * NC), kb, c;
         { const int rem = u0 - g * KB * NC; kb = rem / NC; c = rem - kb * NC; }
         auto step = [&](int& g_, int& kb_, int& c_) { if (++c_ == NC) { c_ = 0; if (++kb_ == KB) { kb_ = 0; g_++; } } };
-        auto issue = [&](int st, int g_, int kb_, int c_) {
-            if (lane == 0) unit[st] = make_int4(g_, 0, c_ * SZ_XW_ITEMS * TW * 16, 0);
+        auto issue = [&](int i, int g_, int kb_, int c_) {
+            const int st = i % S;
+            if (lane == 0) { unit[st] = make_int4(g_, 0, c_ * SZ_XW_ITEMS * TW * 16, 0); R.give(i); }
             R.issue(st, (g_ < D ? down + (u64)plan->expert[g_] * dstride : sh_down) + hdr + (size_t)kb_ * 8 * drow + (size_t)c_ * X::ROW_BYTES, drow, lane);
         };
         const int pre = count < S ? count : S;
@@ -382,7 +409,7 @@ sz_xw_down_kernel(const SzPlan* __restrict__ plan, const u8* __restrict__ gate, 
             }
             if (i >= S) {
                 if (!sz_mbar_wait(&R.empty[st], ((i / S) - 1) & 1)) { ok = false; break; }
-                if (p == SZ_XW_PRODUCE - 1) issue(st, g, kb, c);
+                if (p == SZ_XW_PRODUCE - 1) issue(i, g, kb, c);
             }
             uint4* frag = R.frags + st * 256 + (lane >> 2) * 32 + (lane & 3);
             if (p < n) frag[4 * p] = piece[0];

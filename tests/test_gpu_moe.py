@@ -189,3 +189,23 @@ def test_every_launch_shape_of_the_warp_specialised_kernels_gives_the_same_bits(
                 assert torch.equal(layer.moe_batch(x).view(torch.int32), want), "rows %d, shape %s %s %s" % (m, occ, tw, twd)
         for v in ("SZ_XW_OCC", "SZ_XW_TW", "SZ_XW_TWD"):
             monkeypatch.delenv(v)
+
+
+# Rings of 5 (4 bits), 7 (3 bits) and 8 stages, whose next unit is another producer warp's in the first two: thousands of calls in a burst,
+# every stage filled several times in each, against the block-synchronous kernels' bits.  2,048 x 512 with rows 6 and 8 takes the wide units
+# by itself; the others are given them.
+@pytest.mark.parametrize("bits,m,tw", [(4, 6, None), (4, 8, None), (3, 8, None), (4, 4, ("4", "4")), (3, 4, ("4", "4")), (2, 8, ("4", "4")), (4, 8, ("1", "1"))])
+def test_bursts_of_calls_through_rings_of_five_seven_and_eight_stages(bits, m, tw, monkeypatch):
+    ety = szlib.TYPE_EXL3(bits)
+    layer = moe.MoeLayer(synth.make_moe_layer(2048, 512, 10, 512, 512, ety, ety, seed=29, device="cuda"), "cuda:0")
+    xs = [synth.normal((m, 2048), 1.0, 50 + i, "x", "cuda").contiguous() for i in range(4)]
+    monkeypatch.setenv("SZ_X3_CLASSIC", "1")
+    want = [layer.moe_batch(x).view(torch.int32).clone() for x in xs]
+    monkeypatch.setenv("SZ_X3_CLASSIC", "0")
+    if tw:
+        monkeypatch.setenv("SZ_XW_TW", tw[0])
+        monkeypatch.setenv("SZ_XW_TWD", tw[1])
+    bad = torch.zeros((), dtype=torch.int64, device="cuda")
+    for n in range(2000):
+        bad += (layer.moe_batch(xs[n % 4]).view(torch.int32) != want[n % 4]).sum()
+    assert int(bad) == 0
