@@ -30,7 +30,7 @@
 // a token tile (25 KB per 256 x 256 x 32) where one a block moved 41, and the tensor core, which needs 512 cycles of the step's 625; the
 // sums of a unit, which all blocks write at about the same time, are a fifth.  At few tokens latency: the chain decode, fence, barrier,
 // instruction.  The issuing thread took 390 cycles a step to make descriptors for 256 cycles of instructions; it makes them once.
-// 12,288 x 2,048: 4,093 tokens 281 -> 241 us (sustained, 1.4 GHz under the power cap), 256 tokens 28.8 -> 25.0 -> 22;
+// 12,288 x 2,048: 4,093 tokens 281 -> 241 us (sustained, 1.4 GHz under the power cap), 256 tokens 28.8 -> 25.0 -> 22.4;
 // 512 x 2,048, one token: 20 -> 11.9 (K in four parts).
 // Every wait is bounded; a wait that runs out records where in the error word, and the block still frees its tensor memory.
 #include <cuda.h>   // CUtensorMap and its enums; the encoder's entry point is asked of the runtime, nothing links against the driver
@@ -134,9 +134,8 @@ __device__ __forceinline__ void mc_decode_block(const u32* W, u8* __restrict__ d
 }
 // G: decode groups, which take the steps in turn.  TS: the steps of a turn, which have one pair of barriers and one commit; SLOTS: turns in the ring.
 // What the issuing thread does per step besides its instructions (a wait, a commit) is on the path: with one row tile - where shared memory
-// has room for eight stages - two steps share it.  12,288 x 2,048, 256 tokens: 28 -> 24.6 us, 1 token 21.8 -> 18.8; 1,024 tokens 74 -> 63; four
-// steps a turn 22.1 where two give 21.9, eight stages of one step each 28.  Many token tiles whose units are split along K, all reading at
-// once, take the old ring (512 x 2,048, 4,093 tokens: 29.7 us, 32.7 with the deep one; 2,900 tokens 25.9 / 25.4).
+// has room for eight stages - two steps share it (12,288 x 2,048, 256 tokens 25.0 -> 22.4 us, 1 token 21.8 -> 18.8, 1,024 tokens 74 -> 63; four
+// steps a turn 22.1 where two give 21.9 on the same day, eight stages of one step each 28).  mc_deep says where the ring of four stages is better.
 template <int MT, bool DEEP> struct McTurn {
     static_assert(!DEEP || MT == 1, "two row tiles leave no room for the deep ring");
     static constexpr int G = MC_DEC / (MT * MC_BM), TS = DEEP ? 2 : 1, STAGES = DEEP ? 8 : 4, SLOTS = STAGES / TS;
@@ -440,6 +439,17 @@ McPlan mc_plan(int rows, int cols, int m) {
     return best;
 }
 
+// Which ring a plan with one row tile a block takes.  The deep one asks for twice as much ahead, which stops paying when many blocks read
+// wide token tiles of a large packed matrix at the same time.  Both rings measured at 400 plans (128 .. 12,288 rows, 512 .. 8,192 columns, 1 .. 8,000
+// tokens; deep / ring of four): tiles of up to 192 tokens 0.80 .. 1.02, whatever the matrix; wider ones by the matrix and the blocks -
+// 512 x 2,048 (128 blocks) 0.98 at 2,900 tokens, 1.10 at 3,870; 128 x 2,048 (32 blocks) 0.96 at 3,870; 512 x 4,096 1.08 at 1,822, 1.14 at 3,102;
+// 256 x 8,192 1.05 at 1,822, 1.48 at 3,870; 1,024 x 3,072, K in one part, 0.98 at 2,846, 1.21 at 4,093.  The line below is never more than 2.5 % above the
+// better of the two at any of them (0.1 % on average); tiles x parts >= 32, before it, lost up to 21 % against the ring of four.
+bool mc_deep(const McPlan& p, int rows, int cols, int m) {
+    const long long blocks = (long long)((rows + MC_BM - 1) / MC_BM) * p.tiles * p.ks;
+    return p.nt <= 192 || (long long)m * cols + 30000 * (blocks < 148 ? blocks : 148) < 9500000;
+}
+
 typedef CUresult (*McEncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 McEncodeTiled mc_encoder() {
@@ -526,7 +536,7 @@ extern "C" int sz_mma_cols(const sz_tensor* w, uint64_t x, int64_t xs, uint64_t 
     McArgs a;
     a.x16 = x16; a.y = (float*)y; a.ys = (long long)ys; a.rows = rows; a.cols = cols; a.m = m; a.nt = nt; a.tiles = tiles; a.ks = plan.ks; a.err = err; a.zero = 0;
     if (plan.mt == 2) return mc_launch<2, false>(wmap, a, st);
-    return plan.ks > 1 && tiles * plan.ks >= 32 ? mc_launch<1, false>(wmap, a, st) : mc_launch<1, true>(wmap, a, st);
+    return mc_deep(plan, rows, cols, m) ? mc_launch<1, true>(wmap, a, st) : mc_launch<1, false>(wmap, a, st);
 }
 
 // Clears (init != 0) or reads the scratch's error word; reading synchronises the stream.  0: no wait of a kernel ran out.

@@ -86,8 +86,10 @@ def test_block_format_experts_with_and_without_the_shared_one_beside_them(ff, sf
     run_case(512, 32, 4, ff, sf, ty[ety], ty[sty], m, seed=40)
 
 
-# K in 2, 3 and 4 parts (3 of unequal length), two row tiles a block with a ragged last one, several units a block, one token a tile
-@pytest.mark.parametrize("rows,cols,m", [(130, 1024, 1), (300, 1024, 70), (385, 3328, 40), (129, 2304, 257), (512, 2048, 17), (3000, 768, 2049), (2600, 512, 2000)])
+# K in 2, 3 and 4 parts (3 of unequal length), two row tiles a block with a ragged last one, several units a block, one token a tile; either
+# side of the line between the two rings of stages with K in 1, 2 and 4 parts
+@pytest.mark.parametrize("rows,cols,m", [(130, 1024, 1), (300, 1024, 70), (385, 3328, 40), (129, 2304, 257), (512, 2048, 17), (3000, 768, 2049), (2600, 512, 2000),
+                                         (1024, 3072, 1676), (1024, 3072, 1870), (1024, 3072, 2840), (256, 8192, 1438), (256, 8192, 1870)])
 def test_projections_split_along_k_and_over_row_tiles(rows, cols, m):
     wb = make(rows, cols, 21)
     x = synth.normal((m, cols), 1.0, 23, "mma_cols.x")
