@@ -134,8 +134,7 @@ sz_hc_mix_kernel(const float* __restrict__ mix, const float* __restrict__ rn, in
 // accumulator rotates over three (this read's, the previous read's - it holds the inject gates the pending write needs - and the
 // next read's, which block 0 clears).
 #define SZ_HC_ACC_ROWS 272                    // rank + streams, padded
-#define SZ_HC_FIX 1099511627776.0             // 2^40
-#define SZ_HC_FIX_INV (1.0 / 1099511627776.0)
+#include "sz_hc_fix.cuh"
 
 // grid C*H / 64; block: a multiple of 32 threads, at least rank + C (one thread a matrix row) and at most 320
 // this thread's 64 weights of the down (or inject) matrix: constant data, requested before the dependency wait

@@ -64,36 +64,13 @@ __device__ __forceinline__ void sz_fma2(u64& a, u64 f, u64 x) { asm("fma.rn.f32x
 __device__ __forceinline__ u64 sz_mul2(u64 a, u64 b) { u64 d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
 __device__ __forceinline__ u64 sz_add2(u64 a, u64 b) { u64 d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
 __device__ __forceinline__ u64 sz_pack2(u32 a, u32 b) { u64 d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(a), "r"(b)); return d; }
-// the halves rounded to 2^-40 as __double2ll_rn((double)a * 2^40) rounds them, + the bits of 6144 = 1.5 * 2^12 (which puts the last place there):
-// all is well while the exponents say so (and, or: of the results' upper words), else sz_hc_fix does it
-#define SZ_HC_MAGIC 0x40B8000000000000ll
-__device__ __forceinline__ long long sz_hc_fix(float a) {
-    if (fabsf(a) < 2048.0f) return __double_as_longlong((double)a + 6144.0) - SZ_HC_MAGIC;
-    return __double2ll_rn((double)a * SZ_HC_FIX);
-}
-template <int N>
-__device__ __forceinline__ void sz_hc_round(const u64* a, long long* sum) {      // N pairs
-    u32 all = 0xffffffffu, any = 0u;
-#pragma unroll
-    for (int i = 0; i < 2 * N; i++) {
-        const u32 hi = (u32)__double2hiint((double)__uint_as_float((u32)(a[i >> 1] >> (32 * (i & 1)))) + 6144.0);
-        all &= hi; any |= hi;
-    }
-    if ((all >> 20) == 0x40Bu && (any >> 20) == 0x40Bu) {
-#pragma unroll
-        for (int i = 0; i < 2 * N; i++) sum[i] += __double_as_longlong((double)__uint_as_float((u32)(a[i >> 1] >> (32 * (i & 1)))) + 6144.0);
-    } else {
-#pragma unroll
-        for (int i = 0; i < 2 * N; i++) sum[i] += sz_hc_fix(__uint_as_float((u32)(a[i >> 1] >> (32 * (i & 1))))) + SZ_HC_MAGIC;
-    }
-}
 // grid (8 row tiles, column parts), block 32 SZ_HC_W; hd: f32 [rows][256]; acc: zero on entry
 __global__ void __launch_bounds__(32 * SZ_HC_W, 1)
 sz_hc_down_rows_kernel(const float* __restrict__ rn, const u8* __restrict__ down, const u8* __restrict__ inject, int H, int rows, float* __restrict__ hd,
                        long long* __restrict__ acc) {
     constexpr int C = 4, RANK = 256, NT = RANK / SZ_HC_N;
     extern __shared__ __align__(128) u8 smem[];
-    __shared__ long long isums[SZ_HC_W][16];
+    __shared__ u64 isums[SZ_HC_W][16];
     __shared__ int s_last;
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const int CH = C * H, NK = CH / SZ_HC_K, P = gridDim.y;
@@ -127,7 +104,7 @@ sz_hc_down_rows_kernel(const float* __restrict__ rn, const u8* __restrict__ down
     sz_cp_async_commit();
     // a thread's outputs og + 4 i and rows rg + 8 j; inject row lane & 3 of row 4 nt + (lane >> 2) (lanes 0 .. 15)
     const int og = lane & 3, rg = lane >> 2;
-    long long sum[32], isum = 0, added = 0;         // [4 pairs of outputs][4 rows][2]
+    u64 sum[32], isum = 0, added = 0;               // [4 pairs of outputs][4 rows][2]
 #pragma unroll
     for (int i = 0; i < 32; i++) sum[i] = 0;
     u64 a[4][4];
@@ -197,7 +174,7 @@ sz_hc_down_rows_kernel(const float* __restrict__ rn, const u8* __restrict__ down
     // ---- over the warps: [row][output] of a warp's sums where its buffers were
     sz_cp_async_wait<0>();
     __syncwarp();
-    long long* red = (long long*)mine;
+    u64* red = (u64*)mine;
 #pragma unroll
     for (int i = 0; i < 32; i++) {
         const int o = og + 4 * (2 * (i >> 3) + (i & 1)), r = rg + 8 * ((i >> 1) & 3);
@@ -206,19 +183,19 @@ sz_hc_down_rows_kernel(const float* __restrict__ rn, const u8* __restrict__ down
     if (lane < 16) isums[warp][lane] = isum;
     __syncthreads();
     if (injects && t < 16 && row0 + 4 * nt + (t >> 2) < rows) {
-        long long v = 0;
+        u64 v = 0;
 #pragma unroll
         for (int q = 0; q < SZ_HC_W; q++) v += isums[q][t];
         atomicAdd((unsigned long long*)(acc + (size_t)(row0 + 4 * nt + (t >> 2)) * SZ_HC_ACC_ROWS + RANK + (t & 3)), (unsigned long long)v);
     }
     const int live = warp < 8 ? rows - row0 : 0;
     // thread: output lane of rows warp, warp + 8, ..
-    long long v[4] = {0, 0, 0, 0};
+    u64 v[4] = {0, 0, 0, 0};
     if (warp < 8) {
 #pragma unroll
         for (int j = 0; j < 4; j++)
 #pragma unroll
-            for (int q = 0; q < SZ_HC_W; q++) v[j] += *(const long long*)(smem + (size_t)q * 2 * SZ_HC_STAGE + ((warp + 8 * j) * (SZ_HC_N + 1) + lane) * 8);
+            for (int q = 0; q < SZ_HC_W; q++) v[j] += *(const u64*)(smem + (size_t)q * 2 * SZ_HC_STAGE + ((warp + 8 * j) * (SZ_HC_N + 1) + lane) * 8);
     }
     long long* at = acc + (size_t)(row0 + warp) * SZ_HC_ACC_ROWS + n0 + lane;
     if (P > 1) {
@@ -233,11 +210,11 @@ sz_hc_down_rows_kernel(const float* __restrict__ rn, const u8* __restrict__ down
         __threadfence();
 #pragma unroll
         for (int j = 0; j < 4; j++)
-            if (warp + 8 * j < live) v[j] = __ldcg(at + (size_t)8 * j * SZ_HC_ACC_ROWS);
+            if (warp + 8 * j < live) v[j] = (u64)__ldcg(at + (size_t)8 * j * SZ_HC_ACC_ROWS);
     }
 #pragma unroll
     for (int j = 0; j < 4; j++)
-        if (warp + 8 * j < live) hd[(size_t)(row0 + warp + 8 * j) * RANK + n0 + lane] = sz_silu((float)((double)v[j] * SZ_HC_FIX_INV) / (float)C);
+        if (warp + 8 * j < live) hd[(size_t)(row0 + warp + 8 * j) * RANK + n0 + lane] = sz_silu((float)((double)(long long)v[j] * SZ_HC_FIX_INV) / (float)C);
 }
 
 // silu(down / C) from the accumulator, for the first half's block-row form.  grid (rows), block 256
