@@ -173,7 +173,7 @@ def test_warp_specialised_exl3_kernels_give_the_bits_of_the_block_synchronous_on
 
 @pytest.mark.parametrize("bits,H,ne,k,FF", [(3, 2048, 512, 10, 512), (4, 512, 16, 2, 128), (2, 1024, 64, 6, 256)])
 def test_every_launch_shape_of_the_warp_specialised_kernels_gives_the_same_bits(bits, H, ne, k, FF, monkeypatch):
-    # blocks a multiprocessor x widths of the units, forced and as chosen from the rows: the block-synchronous kernels' bits
+    # the widths of the units (gate / up's, down's), forced and as chosen from the rows: the block-synchronous kernels' bits
     ety = szlib.TYPE_EXL3(bits)
     layer = moe.MoeLayer(synth.make_moe_layer(H, ne, k, FF, FF, ety, ety, seed=23, device="cuda"), "cuda:0")
     for m in (1, 2, 3, 5, 8):
@@ -182,12 +182,12 @@ def test_every_launch_shape_of_the_warp_specialised_kernels_gives_the_same_bits(
         want = layer.moe_batch(x).view(torch.int32).clone()
         monkeypatch.setenv("SZ_X3_CLASSIC", "0")
         assert torch.equal(layer.moe_batch(x).view(torch.int32), want), "rows %d" % m
-        for occ in "23":
-            for tw, twd in (("4", "4"), ("4", "2"), ("2", "4"), ("2", "1"), ("1", "2"), ("1", "1")):
-                for v, s in (("SZ_XW_OCC", occ), ("SZ_XW_TW", tw), ("SZ_XW_TWD", twd)):
-                    monkeypatch.setenv(v, s)
-                assert torch.equal(layer.moe_batch(x).view(torch.int32), want), "rows %d, shape %s %s %s" % (m, occ, tw, twd)
-        for v in ("SZ_XW_OCC", "SZ_XW_TW", "SZ_XW_TWD"):
+        for tw in "421":
+            for twd in "421":
+                monkeypatch.setenv("SZ_XW_TW", tw)
+                monkeypatch.setenv("SZ_XW_TWD", twd)
+                assert torch.equal(layer.moe_batch(x).view(torch.int32), want), "rows %d, widths %s %s" % (m, tw, twd)
+        for v in ("SZ_XW_TW", "SZ_XW_TWD"):
             monkeypatch.delenv(v)
 
 
