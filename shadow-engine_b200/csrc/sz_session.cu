@@ -777,6 +777,22 @@ static int sz_hc_read(sz_session* s, cudaStream_t st, const sz_hc& hc, int m, bo
 // The fused read over the rows of a batch: buffers that hold the rows of all sequences one after the other (a multiple of 8 rows,
 // the sequences' own buffers pointing into them), eight rows a block row of the two kernels.  n: the read's number in the pass.
 struct SzBatchBufs { float *r, *r2, *y, *u, *rn; long long* acc; int64_t acc_stride; float* hd; };
+
+// In how many parts the tiles of the reads' first half take the columns (`pieces` of 64).  A block takes (turns + 1) x 6.5 us, turns: the pieces its
+// busiest warp gets; tiles x parts blocks run in waves of one a multiprocessor.  The parts with the least of waves x (turns + 1) - of equals those in fewer waves,
+// then the more.  Measured (us a launch, 8,192 columns, 1 / 2 / 3 / 4 / .. parts): 56 rows 84 / 51 / 39 / 33 / 31 / 27 / 25 / 23 / 23; 136 86 / 52 / 41 /
+// 58; 264 85 / 53 / 72 / 59; 296 - 384 86 / 95 / 73 / 84; 416 86 / 96 / 103 / 84; 504 86 / 96 / 105 / 109.  As many parts as fit one wave, the rule before,
+// gave 289 - 384 rows the time of 504.
+static int sz_hc_parts(int tiles, int pieces) {
+    int best = 1, best_cost = 1 << 30, best_waves = 1;
+    for (int p = 1; p <= 9; p++) {
+        const int waves = (tiles * p + sz_sm_count_session() - 1) / sz_sm_count_session(), share = (pieces + p - 1) / p;
+        const int cost = waves * ((share + SZ_HC_W - 1) / SZ_HC_W + 1);
+        if (cost < best_cost || (cost == best_cost && waves == best_waves)) { best = p; best_cost = cost; best_waves = waves; }
+    }
+    return best;
+}
+
 static int sz_hc_read_rows(const sz_session* s, cudaStream_t st, const sz_hc& hc, int rows, int n, bool pending, bool inject, const SzBatchBufs& B, bool pdl) {
     const sz_model_config& c = s->model.cfg;
     const int H = c.hidden, C = c.streams, CH = C * H;
@@ -807,14 +823,14 @@ static int sz_hc_read_rows(const sz_session* s, cudaStream_t st, const sz_hc& hc
                 SZ_CUDA(cudaFuncSetAttribute(sz_hc_up_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SzHcUpRows::SMEM));
                 set = true;
             }
-            // Few rows: a thread a matrix row and 8 rows of the step a block; from 56 rows on the tiles, the columns in as many parts as fill the
-            // chip (a prompt's whole chunk, 48 layers, both ways: 48 rows 31.6 / 31.7 ms, 56 33.8 / 33.4, 72 37.1 / 36.4, 264 67.9 / 63.7).
+            // Few rows: a thread a matrix row and 8 rows of the step a block; from 56 rows on the tiles (a prompt's whole chunk, 48 layers, both
+            // ways: 48 rows 31.6 / 31.7 ms, 56 33.8 / 33.4, 72 37.1 / 36.4, 264 67.9 / 63.7).
             if (rows <= 48) {
                 SZ_CUDA(sz_launch("hc_rows_down", sz_hc_rows_down_kernel<8>, dim3(CH / 64, rows / 8), dim3(nt), 0, st, true, (const float*)B.rn, (const u8*)hc.down.data,
                                   (const u8*)(inject ? hc.inject.data : 0), H, C, (int)c.hc_rank, acc));
                 SZ_CUDA(sz_launch("hc_rows_act", sz_hc_rows_act_kernel, dim3(rows), dim3(256), 0, st, true, (const long long*)acc, C, B.hd));
             } else {
-                const int tiles = (rows + SZ_HC_M - 1) / SZ_HC_M * (256 / SZ_HC_N), parts = tiles < sz_sm_count_session() ? sz_sm_count_session() / tiles : 1;
+                const int tiles = (rows + SZ_HC_M - 1) / SZ_HC_M * (256 / SZ_HC_N), parts = sz_hc_parts(tiles, (int)(CH / SZ_HC_K));
                 SZ_CUDA(sz_launch("hc_down_rows", sz_hc_down_rows_kernel, dim3(tiles, parts), dim3(32 * SZ_HC_W), SzHcDownRows::SMEM, st, true, (const float*)B.rn,
                                   (const u8*)hc.down.data, (const u8*)(inject ? hc.inject.data : 0), H, rows, B.hd, acc));
             }

@@ -45,10 +45,12 @@ def test_a_prompt_in_chunks_equals_passes_of_eight_rows(dm, n):
 
 
 # the reads' many-row kernels (rank 256): 48 rows are the last without tiles, 56 the first; tiles of 32 rows and what is over them.  scale: the
-# norm weights' - sums of 64 columns beyond 2^11 take the other way to fixed point, in both forms.
-@pytest.mark.parametrize("n,scale", [(49, 1.0), (57, 1.0), (65, 1.0), (73, 1.0), (137, 1.0), (513, 1.0), (65, 20000.0)])
-def test_the_reads_of_a_chunk_in_tiles_equal_the_passes(n, scale):
-    M = md.make_model(dict(CFG, hc_rank=256), expert_type=szlib.TYPE_EXL3(3), seed=6)
+# norm weights' - sums of 64 columns beyond 2^11 take the other way to fixed point, in both forms.  hidden 1,024: the columns in two parts (201 rows),
+# in one wave of blocks (289) and in three parts in two waves (297 and 385).
+@pytest.mark.parametrize("n,scale,hidden", [(49, 1.0, 0), (57, 1.0, 0), (65, 1.0, 0), (73, 1.0, 0), (137, 1.0, 0), (513, 1.0, 0), (65, 20000.0, 0),
+                                            (201, 1.0, 1024), (289, 1.0, 1024), (297, 1.0, 1024), (385, 1.0, 1024)])
+def test_the_reads_of_a_chunk_in_tiles_equal_the_passes(n, scale, hidden):
+    M = md.make_model(dict(CFG, hc_rank=256, hidden=hidden or CFG["hidden"]), expert_type=szlib.TYPE_EXL3(3), seed=6)
     for k, t in M["tensors"].items():
         if k.endswith("hc_attn_norm.weight") or k.endswith("hc_ffn_norm.weight"):
             t[3].mul_(scale)
