@@ -848,10 +848,12 @@ static int sz_ffn(cudaStream_t st, int type, const SzPlan* plan, int groups, u64
 
 // The widths of a pass's expert units, in tile columns an item (TW of the gate / up launch, TWD of down's; 4, 2 or 1: 24, 12 or 6 KB of trellis a
 // unit at 3 bits).  Narrow units share the work out more evenly, wide ones have fewer hand-overs and fragments; which wins goes with the
-// units a multiprocessor has.  The groups are what independent rows choose on average.  Measured (us a layer, 2048 x 512, 512 experts, top
-// 10; TW TWD = 44 / 42 / 24 / 22 / 21 / 11): rows 1 33.4 / 31.8 / 33.1 / 31.3 / 31.1 / 31.2, 2 42.3 / 40.9 / 40.4 / 38.9 / 39.7 / 40.7, 3 50.6 /
-// 49.1 / 48.7 / 47.5 / 49.6 / 51.4, 4 56.8 / 56.6 / 56.4 / 56.1 / 59.5 / 62.0, 6 77.6 / 77.2 / 76.8 / 76.4 / 82.0 / 87.0, 8 89.9 / 91.0 / 90.1 / 91.0 /
-// 99.5 / 105.6 (three blocks a multiprocessor with eight decode warps each before: rows 1 31.8, 2 40.9, 3 53, 4 59.5, 6 86.5, 8 107).
+// units a multiprocessor has, not with the bits.  The groups are what independent rows choose on average.  All widths measured at 1 .. 8 rows of 22
+// layers (2, 3 and 4 bits; 512 .. 4096 x 128 .. 512; 16 .. 512 experts, top 2 .. 10), us a layer, TW TWD = 44 / 42 / 22 / 21 / 11: 2048 x 512, 512
+// experts, top 10, 3 bits, rows 1 30.4 / 29.1 / 28.8 / 28.8 / 28.9, 4 54.5 / 54.5 / 54.4 / 58.3 / 61.5, 8 87.5 / 89.5 / 90.7 / 100.5 / 107.7; 1024 x 256, 64
+// experts, top 6, 4 bits (2 and 1 only), rows 1 18.6 / 17.8 / 17.5, 4 22.7 / 22.1 / 22.7, 8 29.0 / 30.4 / 31.1.  The lines below are 0.5 % above the best widths on average
+// and 6 % at most (2048 x 256, 64 experts, one row); the ones before - TW 2 from 3 on, TWD 4 from 7 and 2 from 2.5, found with 2048 x 512 at 3 bits alone - 1.2 and
+// 7, and nothing measured is over 1.1 % slower than with them.
 struct SzXWShape { int tw, twd; };
 static SzXWShape sz_xw_shape(const sz_moe_layer* L, int m, bool shared) {
     const int NTC = L->expert_ff / 128, H = L->hidden;
@@ -860,8 +862,8 @@ static SzXWShape sz_xw_shape(const sz_moe_layer* L, int m, bool shared) {
     g = (g + (shared ? 1 : 0)) / sz_sm_count();
     const double gu = g * 2 * (H / 128) * NTC, dn = g * NTC * (H / 128);      // units a multiprocessor at width 1
     SzXWShape s;
-    s.tw = NTC % 4 == 0 && gu / 4 >= 12 ? 4 : (NTC % 2 == 0 && gu / 2 >= 3 ? 2 : 1);
-    s.twd = dn / 4 >= 7 ? 4 : (dn / 2 >= 2.5 ? 2 : 1);
+    s.tw = NTC % 4 == 0 && gu / 4 >= 12 ? 4 : (NTC % 2 == 0 && gu / 2 >= 2 ? 2 : 1);
+    s.twd = dn / 4 >= 6 ? 4 : (dn / 2 >= 1.5 ? 2 : 1);
     return s;
 }
 
