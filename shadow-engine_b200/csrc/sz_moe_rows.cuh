@@ -46,9 +46,12 @@ struct SzRowsPlan {
     int32_t start[2][SZ_ROWS_MAXB + 1];
     u32 gu_blocks[SZ_ROWS_MAXG][2], dn_blocks[SZ_ROWS_MAXG][8];
 };
-// What a unit of a group of n rows costs, in 15 ns: the decode, a row's fragments, the second eight rows' products.  Least squares over the blocks
-// of gate / up launches of 48 .. 256 rows: 2,580 ns + 15.4 a row up to eight, 3,302 + 7.5 a row beyond (1.1 us rms a block of 311; down: 2,770 and
-// 3,230 + 6).  The weights before it (64 + n, 69 + n) charged a row two and a half times what it takes: at 256 rows blocks ended from 298 to 329 us.
+// What a unit of a group of n rows costs: the decode, a row's fragments, the second eight rows' products.  Least squares over the blocks of gate / up
+// launches of 8 .. 256 rows (cycles; 2,048 x 512, 512 experts): 2 bits 4,707 + 22.7 a row up to eight, 5,848 + 18.9 beyond; 3 bits 4,696 + 26.2 and
+// 5,901 + 15.2; 4 bits 4,679 + 25.7 and 5,902 + 17.8 (0.5 % rms of a block); 4,096 x 512, 64 experts, 3 bits: 4,774 + 23.0 and 5,853 + 18.6; 2,048 x 256, whose
+// units are half as large, 2,995 + 23.0 and 3,687 + 15.7 - the same proportions, which is all that counts.  Down's rows are copied, not made: 4,937 + 4.6 and 5,899 + 6.1
+// (3 bits), so a group beyond eight is 1.20 of a small one where the weights say 1.27: its blocks end within 96 - 98 % of the last one's time on average, gate /
+// up's within 98; weights of its own (1.17) changed down by -3 .. +2 %, none (no term a row) by under 1 %.
 __device__ __forceinline__ int sz_rows_weight(int n) { return n <= 8 ? 172 + n : 218 + n / 2; }
 
 // ---- plan: one block of 1024 threads ---------------------------------------------------------------------------------------------------
