@@ -205,6 +205,9 @@ __device__ __forceinline__ bool sz_mbar_wait(u64* bar, u32 phase, u32 limit = 20
     }
     return false;
 }
+__device__ __forceinline__ void sz_mbar_arrive(u64* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sz_smem_addr(bar)) : "memory");
+}
 // global -> shared bulk copy; src and dst 16-byte aligned, bytes a multiple of 16.
 __device__ __forceinline__ void sz_bulk_g2s(void* dst, const void* src, u32 bytes, u64* bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(sz_smem_addr(dst)),

@@ -645,6 +645,7 @@ static __global__ void __launch_bounds__(32 * NW, 2) sz_dense_rows_q8_kernel(con
 int sz_dense_launch(SzDenseArgs& a, cudaStream_t st, const char* name);
 // a.m rows, a multiple of 8 (any number of them), through the many-row form of the Q8_0 tensor-pipe kernel when sz_dense_launch would
 // take that kernel for 8 rows of these jobs: *taken = 1 and the rows are computed (bit for bit as 8 at a time); otherwise *taken = 0
-// and nothing is launched.  xh: a.m * a.cols * 2 halves of scratch.
-int sz_dense_rows_launch(SzDenseArgs& a, void* xh, cudaStream_t st, const char* name, int* taken);
+// and nothing is launched.  xh: a.m * a.cols * 2 halves of scratch; packed: they hold the rows already.
+bool sz_dense_rows_takes(const SzDenseArgs& a);
+int sz_dense_rows_launch(SzDenseArgs& a, void* xh, bool packed, cudaStream_t st, const char* name, int* taken);
 int sz_dense_check(const sz_tensor* t, const char* what, int64_t rows, int64_t cols);

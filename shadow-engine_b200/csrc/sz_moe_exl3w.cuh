@@ -126,10 +126,6 @@ __device__ __forceinline__ void sz_xw_compute(const u8* stage, const uint4* frag
     }
 }
 
-__device__ __forceinline__ void sz_mbar_arrive(u64* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sz_smem_addr(bar)) : "memory");
-}
-
 // A row's 128 values (k = lane + 32 e on entry), rotated, as its share of the B fragments.  In the fragment order a row owns 32 whole 16-byte
 // pieces - (tile row kr, quad q): values 16 kr + 2 q, + 1 and + 8, + 9 as f16 high parts, then the low parts - so the values change lanes
 // through `buf` (128 floats of the warp's own) and every lane makes the piece (lane / 4, lane % 4).

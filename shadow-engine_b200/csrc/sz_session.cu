@@ -655,9 +655,10 @@ static bool sz_dense_q8_takes(const SzDenseArgs& a) {
     return false;
 }
 
-int sz_dense_rows_launch(SzDenseArgs& a, void* xh, cudaStream_t st, const char* name, int* taken) {
+bool sz_dense_rows_takes(const SzDenseArgs& a) { return a.m >= 8 && a.m % 8 == 0 && sz_dense_q8_takes(a); }
+int sz_dense_rows_launch(SzDenseArgs& a, void* xh, bool packed, cudaStream_t st, const char* name, int* taken) {
     *taken = 0;
-    if (a.m < 8 || a.m % 8 || !sz_dense_q8_takes(a)) return SZ_OK;
+    if (!sz_dense_rows_takes(a)) return SZ_OK;
     int total = 0;
     for (int i = 0; i < a.n_jobs; i++) { a.job[i].row0 = total; total += a.job[i].rows; }
     a.total_rows = total;
@@ -667,7 +668,7 @@ int sz_dense_rows_launch(SzDenseArgs& a, void* xh, cudaStream_t st, const char* 
     c.units[a.n_jobs] = units;
     c.rows = a.m;
     c.xh = (const __half*)xh;
-    SZ_CUDA(sz_launch("dense_rows_pack", sz_dense_rows_pack_kernel, dim3((a.cols + 1023) / 1024, a.m), dim3(256), 0, st, true, a.x, a.xstride, a.cols, a.m, (__half*)xh));
+    if (!packed) SZ_CUDA(sz_launch("dense_rows_pack", sz_dense_rows_pack_kernel, dim3((a.cols + 1023) / 1024, a.m), dim3(256), 0, st, true, a.x, a.xstride, a.cols, a.m, (__half*)xh));
     static bool set = false;
     if (!set) {
         SZ_CUDA(cudaFuncSetAttribute(sz_dense_rows_q8_kernel<8, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, SzDenseRows<8, 4>::SMEM));
@@ -1826,13 +1827,15 @@ static int sz_rows_layers(sz_session* const* ss, int n, const int32_t* ids, cons
                       (const u8*)s0->model.token_embd.data, (int)s0->model.token_embd.type, (int)c.hidden, (int)c.streams, (int)c.vocab, BB.r));
     const char* re = getenv("SZ_BATCH_DENSE_ROWS");   // 0: the projections 8 rows a launch (the second form; same bits)
     const bool rows_form = !(re && atoi(re) == 0);
-    // a projection set over all rows: one launch where the many-row form of the kernel exists, else 8 rows a launch
-    auto dense = [&](const SzDenseArgs& a, const float* x, float* const* outs, const char* name) -> int {
+    // a projection set over all rows: one launch where the many-row form of the kernel exists (its rows made by it, or left in XH by the
+    // kernel before: `packed`), else 8 rows a launch
+    auto in_xh = [&](SzDenseArgs a) { a.m = Rp; return rows_form && sz_dense_rows_takes(a); };
+    auto dense = [&](const SzDenseArgs& a, const float* x, float* const* outs, const char* name, bool packed) -> int {
         SzDenseArgs ar = a;
         ar.m = Rp; ar.x = x;
         for (int k = 0; k < a.n_jobs; k++) ar.job[k].out = outs[k];
         int taken = 0, r;
-        if (rows_form && (r = sz_dense_rows_launch(ar, XH, st, name, &taken))) return r;
+        if (rows_form && (r = sz_dense_rows_launch(ar, XH, packed, st, name, &taken))) return r;
         for (int g = 0; g < Rp / 8 && !taken; g++) {
             SzDenseArgs ag = a;
             ag.m = 8; ag.x = x + (size_t)g * 8 * a.cols;
@@ -1853,7 +1856,8 @@ static int sz_rows_layers(sz_session* const* ss, int n, const int32_t* ids, cons
         float* outs[SZ_DENSE_MAX_JOBS];
         int64_t at = 0;
         for (int k = 0; k < a.n_jobs; k++) { outs[k] = IN + at; at += (int64_t)Rp * a.job[k].ostride; }
-        if ((rc = dense(a, X, outs, "rows_proj"))) return rc;
+        if ((rc = dense(a, X, outs, "rows_proj", false))) return rc;
+        bool packed = false;
         if (sz_is_attn(c, l)) {
             const int ai = s0->lb[l].attn_index;
             SZ_CUDA(sz_launch("rows_attn_prep", sz_attn_prep_kernel, dim3(nh + 2 * nkv, R), dim3(128), 0, st, true, (const float*)outs[0], (const float*)outs[1],
@@ -1872,11 +1876,14 @@ static int sz_rows_layers(sz_session* const* ss, int n, const int32_t* ids, cons
                               dim3((ch + 255) / 256, (R + SZ_PREP_ROWS - 1) / SZ_PREP_ROWS), dim3(256), 0, st, true, seqs, rws, R, di, (const float*)outs[0],
                               (const float*)L.ssm_conv1d.data, (const float*)outs[2], (const float*)outs[3], (const float*)L.ssm_a.data, (const float*)L.ssm_dt_bias.data,
                               kh, vh, d, (int)c.conv_k, XC, BETA, DECAY));
-            SZ_CUDA(sz_launch("rows_scan", d == 128 ? sz_rows_scan_kernel<128> : sz_rows_scan_kernel<64>, dim3(vh * (d / 32), n), dim3(d), 0, st, true, seqs, di,
-                              (const float*)XC, (const float*)BETA, (const float*)DECAY, (const float*)outs[1], (const float*)L.ssm_norm.data, kh, vh, c.eps, CORE));
+            SZ_CUDA(sz_launch("rows_scan", d == 128 ? sz_rows_scan_kernel<128> : sz_rows_scan_kernel<64>, dim3(vh * (d / 32), n), dim3(d + 32), 0, st, true, seqs, di,
+                              (const float*)XC, (const float*)BETA, (const float*)DECAY, kh, vh, CORE, err));
+            packed = in_xh(o);
+            SZ_CUDA(sz_launch("rows_gate", d == 128 ? sz_rows_gate_kernel<128> : sz_rows_gate_kernel<64>, dim3((R * vh + 7) / 8), dim3(256), 0, st, true, CORE,
+                              (const float*)outs[1], (const float*)L.ssm_norm.data, R, vh, c.eps, Rp, (__half*)(packed ? XH : nullptr)));
         }
         float* yo[1] = {Y};
-        if ((rc = dense(o, CORE, yo, "rows_out"))) return rc;
+        if ((rc = dense(o, CORE, yo, "rows_out", packed))) return rc;
         if ((rc = sz_hc_read_rows(s0, st, L.hc_ffn, Rp, hn++, true, true, BB, true))) return rc;
         if ((rc = sz_moe_rows_live(&L.moe, (uint64_t)X, Rp, R, rows_max, (uint64_t)Y, (uint64_t)(base + S.moe), S.moe_bytes, (uint64_t)st))) return rc;
     }
@@ -2170,7 +2177,7 @@ static int sz_batch_step(sz_session* const* ss, int n, const int32_t* ids, const
                 ar.m = Rp; ar.x = X;
                 for (int k = 0; k < a.n_jobs; k++) ar.job[k].out = IN + mi.off[k];
                 int taken = 0;
-                if (rows_form && (rc = sz_dense_rows_launch(ar, XH, st, "batch_proj", &taken))) return rc;
+                if (rows_form && (rc = sz_dense_rows_launch(ar, XH, false, st, "batch_proj", &taken))) return rc;
                 for (int g = 0; g < Rp / 8 && !taken; g++) {
                     SzDenseArgs ag = a;
                     ag.x = X + (size_t)g * 8 * c.hidden;
@@ -2195,7 +2202,7 @@ static int sz_batch_step(sz_session* const* ss, int n, const int32_t* ids, const
                 SzDenseArgs orr = o;
                 orr.m = Rp; orr.x = CORE; orr.job[0].out = Y;
                 int taken = 0;
-                if (rows_form && (rc = sz_dense_rows_launch(orr, XH, st, "batch_out", &taken))) return rc;
+                if (rows_form && (rc = sz_dense_rows_launch(orr, XH, false, st, "batch_out", &taken))) return rc;
                 for (int g = 0; g < Rp / 8 && !taken; g++) {
                     SzDenseArgs og = o;
                     og.x = CORE + (size_t)g * 8 * o.cols;

@@ -691,16 +691,16 @@ __global__ void sz_state_update_kernel(int32_t* __restrict__ state, const int32_
 }
 
 // ---- DeltaNet state scan (forward.rs:859-894) ---------------------------------------------------------------------------------------
-// Per value head a D x D state whose columns are independent: a block takes 32 of them - lane = column - and its D / RW warps RW of the
-// D rows each, so a thread holds RW values of the state in registers (16 in a pass: twice the threads for the front end and its loads;
-// 32 in a step of many rows: more blocks a multiprocessor, and k and q - which every thread must read - read half as often); the D / 32 blocks of a head are a cluster.  Sums over the rows run
+// Per value head a D x D state whose columns are independent: a block takes 32 of them - lane = column - and its D / 16 warps 16 of the
+// D rows each, so a thread holds 16 values of the state in registers; the D / 32 blocks of a head are a cluster.  (A step of many rows has
+// a kernel of its own, sz_rows_scan_kernel.)  Sums over the rows run
 // in f32 over 16 of them and these runs are added in f64 in a fixed order (the exact GPU scan's, kernels/forward.cu:991-1013): one
 // exchange through shared memory and one barrier a row of the pass is what the recurrence waits for.  Everything else stays off its
 // path: the next row's operands are read before the barrier, the next 8 rows arrive by asynchronous copies, and the outputs of 8
 // rows - their runs left in shared memory - are finished 8 rows later, when the cluster's other blocks have theirs for the gated norm over
 // a head's D outputs.  (One block of 256 threads a head, 64 values a thread and five barriers a row was 18 us a layer for 4 rows; this
-// split with the outputs finished in line 0.65 us a row.  Shared-memory reads of k and q, 16 bytes a lane at 128 bytes a cycle, are what
-// the rows wait for now.)
+// split with the outputs finished in line 0.65 us a row.  A column's threads in one warp, summed by shuffles without a barrier, were
+// slower for the few rows of a pass: the state then comes and goes in pieces of 16 bytes, 1 row +1.6 us a launch.)
 // Reads the state of the current buffer (state[1]) and writes the other one.  With `og` != null it applies all m rows and writes
 // the gated, normalised outputs (the pass itself).  With og == null it is the replay of a commit: layer blockIdx.y of every per-layer
 // array, only the res[0] kept rows, and nothing at all when every row was kept (the pass already wrote that state) or none was.
@@ -738,15 +738,15 @@ struct SzScanShared {
     float k[2][SZ_SCAN_RC][D], q[2][SZ_SCAN_RC][D], v[2][SZ_SCAN_RC][32];   // two sets of rows: one at work, the next arriving
     float beta[2][SZ_SCAN_RC], decay[2][SZ_SCAN_RC];
     float orun[SZ_SCAN_RC][D / 16][32];      // the outputs' runs
-    double mem[2][D / 64][4][32];             // a row's runs of S^T k, four a part (RW = 32: the first two added, the third, the fourth)
+    double mem[2][D / 64][4][32];             // a row's runs of S^T k, four a part
     float ofs[2][SZ_SCAN_RC][32];            // finished outputs of the block's columns
 };
 
 // TREE: the pass or the commit of a draft tree (tr, fork); a chain's instance has neither the tables nor the state of another branch.
-template <int D, int RW, bool TREE>
+template <int D, bool TREE>
 __device__ __forceinline__ void sz_delta_scan_body(const SzScanSeq& q, const float* __restrict__ norm_w, int kh, int vh, float eps,
                                                    const SzTree* __restrict__ tr_, float* __restrict__ fork, const int hd, const int cb, const int di) {
-    constexpr int NW = D / RW, NT = NW * 32, RPW = SZ_SCAN_RC / NW;     // warps; rows of outputs a warp finishes
+    constexpr int RW = 16, NW = D / RW, NT = NW * 32, RPW = SZ_SCAN_RC / NW;     // warps; rows of outputs a warp finishes
     __shared__ __align__(16) SzScanShared<D> sh;
     const SzTree* __restrict__ tr = TREE ? tr_ : nullptr;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, col = cb * 32 + lane;
@@ -1009,20 +1009,10 @@ __device__ __forceinline__ void sz_delta_scan_body(const SzScanSeq& q, const flo
                 }
             }
             prev_row = j;
-            float r0 = 0.f, r1 = 0.f;
+            float r0 = 0.f;
 #pragma unroll
-            for (int i = 0; i < 16; i++) {
-                S[i] = S[i] * dc; r0 = fmaf(S[i], kr[i], r0);
-                if constexpr (RW == 32) { S[16 + i] = S[16 + i] * dc; r1 = fmaf(S[16 + i], kr[16 + i], r1); }
-            }
-            // four runs a part: of warps 4 p .. (RW = 16), or 2 p and 2 p + 1
-            if constexpr (RW == 16) {
-                sh.mem[jj & 1][warp >> 2][warp & 3][lane] = (double)r0;
-            } else {
-                double (*mp)[32] = sh.mem[jj & 1][warp >> 1];
-                if (warp & 1) { mp[1][lane] = (double)r0; mp[2][lane] = (double)r1; }
-                else mp[0][lane] = (0.0 + (double)r0) + (double)r1;
-            }
+            for (int i = 0; i < RW; i++) { S[i] = S[i] * dc; r0 = fmaf(S[i], kr[i], r0); }
+            sh.mem[jj & 1][warp >> 2][warp & 3][lane] = (double)r0;      // four runs a part
             float qr[RW];
             if (og) {
 #pragma unroll
@@ -1033,23 +1023,18 @@ __device__ __forceinline__ void sz_delta_scan_body(const SzScanSeq& q, const flo
             double tot = 0.0;
 #pragma unroll
             for (int p = 0; p < D / 64; p++) {
-                const double s01 = RW == 32 ? sh.mem[jj & 1][p][0][lane] + sh.mem[jj & 1][p][1][lane]
-                                            : ((0.0 + sh.mem[jj & 1][p][0][lane]) + sh.mem[jj & 1][p][1][lane]) + sh.mem[jj & 1][p][2][lane];
-                tot += s01 + sh.mem[jj & 1][p][RW == 32 ? 2 : 3][lane];
+                const double (*mp)[32] = sh.mem[jj & 1][p];
+                tot += (((0.0 + mp[0][lane]) + mp[1][lane]) + mp[2][lane]) + mp[3][lane];
             }
             const float dl = (float)((vd - tot) * bd);
 #pragma unroll
             for (int i = 0; i < RW; i++) S[i] = __fadd_rn(S[i], __fmul_rn(kr[i], dl));  // unfused, as the CPU reference
             if (jj + 1 < nr) operands(jj + 1);
             if (og) {
-                r0 = 0.f; r1 = 0.f;
+                r0 = 0.f;
 #pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    r0 = fmaf(S[i], qr[i], r0);
-                    if constexpr (RW == 32) r1 = fmaf(S[16 + i], qr[16 + i], r1);
-                }
-                sh.orun[jj][RW / 16 * warp][lane] = r0;
-                if constexpr (RW == 32) sh.orun[jj][2 * warp + 1][lane] = r1;
+                for (int i = 0; i < RW; i++) r0 = fmaf(S[i], qr[i], r0);
+                sh.orun[jj][warp][lane] = r0;
                 if (tr && (((quick ? (u32)tpar[SZ_MAX_VERIFY] : tr->save) >> j) & 1u)) {
 #pragma unroll
                     for (int i = 0; i < RW; i++) fk[((size_t)j * D + warp * RW + i) * D + col] = S[i];
@@ -1091,7 +1076,7 @@ __device__ __forceinline__ void sz_delta_scan_body(const SzScanSeq& q, const flo
 template <int D, bool TREE>
 __global__ void __cluster_dims__(D / 32, 1, 1) __launch_bounds__(2 * D)
 sz_delta_scan_kernel(const SzScanSeq q, const float* __restrict__ norm_w, int kh, int vh, float eps, const SzTree* __restrict__ tr, float* __restrict__ fork) {
-    sz_delta_scan_body<D, 16, TREE>(q, norm_w, kh, vh, eps, tr, fork, (int)blockIdx.x / (D / 32), (int)blockIdx.x % (D / 32), (int)blockIdx.y);
+    sz_delta_scan_body<D, TREE>(q, norm_w, kh, vh, eps, tr, fork, (int)blockIdx.x / (D / 32), (int)blockIdx.x % (D / 32), (int)blockIdx.y);
 }
 
 // The pass of one layer for SEVERAL sequences in one launch (a batched step, prompts): block row b is sequence b's scan, its pointers
@@ -1103,7 +1088,7 @@ sz_delta_scan_seqs_kernel(const SzScanSeq* __restrict__ tab, const float* __rest
     static_assert(sizeof(SzScanSeq) % 8 == 0 && sizeof(SzScanSeq) / 8 <= 2 * 64, "copied in 8-byte words");
     if (threadIdx.x < sizeof(SzScanSeq) / 8) ((u64*)&q)[threadIdx.x] = ((const u64*)(tab + blockIdx.y))[threadIdx.x];
     __syncthreads();
-    sz_delta_scan_body<D, 16, false>(q, norm_w, kh, vh, eps, (const SzTree*)nullptr, (float*)nullptr, (int)blockIdx.x / (D / 32), (int)blockIdx.x % (D / 32), 0);
+    sz_delta_scan_body<D, false>(q, norm_w, kh, vh, eps, (const SzTree*)nullptr, (float*)nullptr, (int)blockIdx.x / (D / 32), (int)blockIdx.x % (D / 32), 0);
 }
 
 // ---- attention front end (forward.rs:908-927): per head RMSNorm + NeoX RoPE of q and k, K and V into the cache.

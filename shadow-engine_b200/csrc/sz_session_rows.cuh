@@ -440,28 +440,207 @@ sz_rows_delta_prep_kernel(const SzSeqDev* __restrict__ seqs, const SzRowDev* __r
     }
 }
 
-// The scans of a layer for the sequences of a step, after sz_rows_delta_prep_kernel.  grid (vh * D / 32, sequences)
+// The scans of a layer for the sequences of a step, after sz_rows_delta_prep_kernel: sz_delta_scan_body's recurrence, its sums in the same
+// order, for any number of rows one after the other.  What bounds a lone prompt's launch is the chain of a row (128 blocks, a warp a
+// scheduler), so everything that is not the chain is kept off it:
+//   - a column's D / 32 threads sit in one warp, 32 of the state's D rows in each, and add their runs by shuffles: no barrier, no trip through
+//     shared memory, and the warps of a block go at their own pace;
+//   - the two runs of a thread are the halves of packed instructions (mul, fma, add.rn.f32x2: each half rounded as the plain one), which take half
+//     the issue slots; the k and q of a row lie interleaved in shared memory, so that a 16-byte read is two operand pairs;
+//   - the output products of a row run beside the next row's k products; runs of 8 rows are added up at once, and left unnormed: the gated
+//     norm over a head's D outputs is sz_rows_gate_kernel's, not eight f64 chains a stage inside this one;
+//   - a fifth warp keeps SZ_RS_STAGES stages of 8 rows' operands on their way.
+// Measured (128 x 128 states, 32 heads; us a launch, events between the launches): 504 rows of one prompt 298 -> 186 and 10 for the gate, which
+// packs the rows as a launch of 7 did before; 80 rows of 32 sequences 63 -> 48 and 8.  A row takes some 800 cycles: 300 the products with
+// the reads of its operands, 270 the sum (two conversions of 27 cycles, ten f64 operations of 8, two shuffles), 105 the update, 115 a row's share of a
+// stage.  The next row's k in registers of its own or conversions by integer instructions: 179 for one prompt, but 57 - 60 for 32 sequences,
+// whose blocks then fit twice a multiprocessor instead of three times.
+// grid (vh * D / 32, sequences), block D + 32
+#define SZ_RS_STAGES 3
+#define SZ_RS_SEG 36          // floats between the 32 k (or q) of one thread of a column and the next one's (32, kept out of each other's banks)
 template <int D>
-__global__ void __cluster_dims__(D / 32, 1, 1) __launch_bounds__(D)
+struct SzRowsScan {
+    float k[SZ_RS_STAGES][SZ_SCAN_RC][D / 32 * SZ_RS_SEG], q[SZ_RS_STAGES][SZ_SCAN_RC][D / 32 * SZ_RS_SEG], v[SZ_RS_STAGES][SZ_SCAN_RC][32];
+    float beta[SZ_RS_STAGES][SZ_SCAN_RC], decay[SZ_RS_STAGES][SZ_SCAN_RC];
+    float orun[SZ_SCAN_RC][D / 16][36];          // the outputs' runs (36: a warp writes its columns' of D / 32 runs at once)
+    u64 full[SZ_RS_STAGES], empty[SZ_RS_STAGES];
+    u64 nz2;                                     // two floats, -0
+};
+template <int D>
+__global__ void __launch_bounds__(D + 32)
 sz_rows_scan_kernel(const SzSeqDev* __restrict__ seqs, int di, const float* __restrict__ xc_all, const float* __restrict__ beta_all, const float* __restrict__ decay_all,
-                    const float* __restrict__ z, const float* __restrict__ norm_w, int kh, int vh, float eps, float* __restrict__ og) {
-    __shared__ SzScanSeq q;
+                    int kh, int vh, float* __restrict__ og, u32* __restrict__ err) {
+    constexpr int NW = D / 32, CW = 32 / NW, RC = SZ_SCAN_RC, ST = SZ_RS_STAGES;     // warps that scan (and threads a column); columns a warp
+    __shared__ __align__(16) SzRowsScan<D> sh;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, hd = blockIdx.x / (D / 32), cb = blockIdx.x % (D / 32);
+    const int ch = (2 * kh + vh) * D, vd = vh * D, kx = hd % kh;      // value heads are tiled over the key heads
     if (threadIdx.x == 0) {
-        const SzSeqDev& s = seqs[blockIdx.y];
-        const int ch = (2 * kh + vh) * D, vd = vh * D;
-        const size_t Sl = (size_t)vh * D * D * di, at = (size_t)di * SZ_MAX_VERIFY;
-        q.xc = s.all ? xc_all + (size_t)s.off * ch : s.xc + at * ch;
-        q.beta = s.all ? beta_all + (size_t)s.off * vh : s.beta + at * vh;
-        q.decay = s.all ? decay_all + (size_t)s.off * vh : s.decay + at * vh;
-        q.z = z + (size_t)s.off * vd;
-        q.S0 = s.S0 + Sl; q.S1 = s.S1 + Sl; q.O0 = s.S0 + Sl; q.O1 = s.S1 + Sl;
-        q.state = s.state; q.res = s.res;
-        q.og = og + (size_t)s.off * vd;
-        q.pp.xin = nullptr;
-        q.m = s.m;
+        for (int i = 0; i < ST; i++) { sz_mbar_init(&sh.full[i], 1); sz_mbar_init(&sh.empty[i], NW); }
+        sz_mbar_fence_init();
+        *(volatile u64*)&sh.nz2 = 0x8000000080000000ull;
+    }
+    const SzSeqDev& sq = seqs[blockIdx.y];
+    const int rows = sq.m, off = sq.off, cur = sq.state[1];     // (the buffers change places at the end of a step only)
+    const int rq = lane / CW, cl = (warp % NW) * CW + lane % CW;       // the thread's rows 32 rq .. of the state, and its column of the block's 32
+    const size_t Sat = ((size_t)di * vh + hd) * D * D + (size_t)(rq * 32) * D + cb * 32 + cl;
+    u64 S[16];                   // rows i and 16 + i of the thread's
+    if (warp < NW) {
+        const float* Sg = (cur ? sq.S1 : sq.S0) + Sat;
+#pragma unroll
+        for (int i = 0; i < 16; i++) S[i] = sz_pack2(__float_as_uint(sz_ld32_here(Sg + (size_t)i * D)), __float_as_uint(sz_ld32_here(Sg + (size_t)(16 + i) * D)));
     }
     __syncthreads();
-    sz_delta_scan_body<D, 32, false>(q, norm_w, kh, vh, eps, (const SzTree*)nullptr, (float*)nullptr, (int)blockIdx.x / (D / 32), (int)blockIdx.x % (D / 32), 0);
+    sz_pdl_wait();
+    sz_pdl_trigger();
+    const int sets = (rows + RC - 1) / RC;
+    if (warp == NW) {
+        // ---- the operands' warp
+        const size_t at = (size_t)di * SZ_MAX_VERIFY;
+        const float* x = (sq.all ? xc_all + (size_t)off * ch : sq.xc + at * ch);
+        const float* be = (sq.all ? beta_all + (size_t)off * vh : sq.beta + at * vh) + hd;
+        const float* de = (sq.all ? decay_all + (size_t)off * vh : sq.decay + at * vh) + hd;
+        float4 qv[RC], kv[RC];
+        float vv[RC], bv = 0.f, dv = 0.f;
+        auto load = [&](int c0) {
+#pragma unroll
+            for (int j = 0; j < RC; j++)
+                if (c0 + j < rows) {
+                    const float* xr = x + (size_t)(c0 + j) * ch;
+                    if (lane < D / 4) { qv[j] = __ldcg((const float4*)(xr + kx * D) + lane); kv[j] = __ldcg((const float4*)(xr + (kh + kx) * D) + lane); }
+                    vv[j] = __ldcg(xr + 2 * kh * D + hd * D + cb * 32 + lane);
+                }
+            if (lane < RC && c0 + lane < rows) { bv = __ldcg(be + (size_t)(c0 + lane) * vh); dv = __ldcg(de + (size_t)(c0 + lane) * vh); }
+        };
+        // element e of piece `lane`: row 4 lane + e, so half (row / 16) & 1 of pair row & 15 of thread row / 32
+        const int to = (lane >> 3) * SZ_RS_SEG + 8 * (lane & 3) + ((lane >> 2) & 1);
+        load(0);
+        for (int c = 0; c < sets; c++) {
+            const int st = c % ST;
+            if (c >= ST && !sz_mbar_wait(&sh.empty[st], ((c / ST) - 1) & 1)) { if (lane == 0) atomicExch(err, 1u); return; }
+#pragma unroll
+            for (int j = 0; j < RC; j++)
+                if (c * RC + j < rows) {
+                    if (lane < D / 4) {
+                        const float qe[4] = {qv[j].x, qv[j].y, qv[j].z, qv[j].w}, ke[4] = {kv[j].x, kv[j].y, kv[j].z, kv[j].w};
+#pragma unroll
+                        for (int e = 0; e < 4; e++) { sh.q[st][j][to + 2 * e] = qe[e]; sh.k[st][j][to + 2 * e] = ke[e]; }
+                    }
+                    sh.v[st][j][lane] = vv[j];
+                }
+            if (lane < RC) { sh.beta[st][lane] = bv; sh.decay[st][lane] = dv; }
+            __syncwarp();
+            if (lane == 0) sz_mbar_arrive(&sh.full[st]);
+            if (c + 1 < sets) load((c + 1) * RC);
+        }
+        return;
+    }
+    float* o = og + (size_t)off * vd + hd * D + cb * 32;
+    u64 kr[16], qr[16], nz2;
+    nz2 = *(volatile u64*)&sh.nz2;
+    for (int c = 0; c < sets; c++) {
+        const int st = c % ST, nr = rows - c * RC < RC ? rows - c * RC : RC;
+        if (!sz_mbar_wait(&sh.full[st], (c / ST) & 1)) { if (lane == 0) atomicExch(err, 1u); return; }
+        const float (*ks)[D / 32 * SZ_RS_SEG] = sh.k[st], (*qs)[D / 32 * SZ_RS_SEG] = sh.q[st];
+        auto pairs = [&](const float* row, u64* to) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) { const ulonglong2 p = *(const ulonglong2*)(row + rq * SZ_RS_SEG + 4 * i); to[2 * i] = p.x; to[2 * i + 1] = p.y; }
+        };
+        pairs(ks[0], kr);
+        float dc = sh.decay[st][0], bt = sh.beta[st][0], vj = sh.v[st][0][cl];
+        auto keep_runs = [&](int jj, u64 r) {
+            sh.orun[jj][2 * rq][cl] = __uint_as_float((u32)r);
+            sh.orun[jj][2 * rq + 1][cl] = __uint_as_float((u32)(r >> 32));
+        };
+        for (int jj = 0; jj < nr; jj++) {
+            const u64 dc2 = sz_pack2(__float_as_uint(dc), __float_as_uint(dc));
+            u64 r = 0, out = 0;
+            if (jj > 0) {                          // with the output products of the row before
+#pragma unroll
+                for (int i = 0; i < 16; i++) { sz_fma2(out, S[i], qr[i]); S[i] = sz_mul2(S[i], dc2); sz_fma2(r, S[i], kr[i]); }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 16; i++) { S[i] = sz_mul2(S[i], dc2); sz_fma2(r, S[i], kr[i]); }
+            }
+            const float r0 = __uint_as_float((u32)r), r1 = __uint_as_float((u32)(r >> 32));
+            // the column's sum: parts of four runs, each ((0 + r) + r) + r) + r in f64 over two threads, the parts in order
+            const double a = (double)(0.f + r0) + (double)r1;      // (an f32 sum with zero is exact)
+            const double b = (__shfl_xor_sync(0xffffffffu, a, CW) + (double)r0) + (double)r1;      // the second thread of a part has it
+            double tot = 0.0;
+#pragma unroll
+            for (int p = 0; p < D / 64; p++) tot += __shfl_sync(0xffffffffu, b, (2 * p + 1) * CW + lane % CW);
+            if (jj > 0) keep_runs(jj - 1, out);
+            pairs(qs[jj], qr);
+            const float dl = (float)(((double)vj - tot) * (double)bt);
+            const u64 dl2 = sz_pack2(__float_as_uint(dl), __float_as_uint(dl));
+#pragma unroll
+            for (int i = 0; i < 16; i++) {      // rounded twice, as the CPU reference does (the compiler makes a packed mul and add one instruction, even with .rn; k dl + a -0 that it cannot see, not)
+                u64 kd = nz2;
+                sz_fma2(kd, kr[i], dl2);
+                S[i] = sz_add2(S[i], kd);
+            }
+            const int nx = jj + 1 < nr ? jj + 1 : jj;
+            pairs(ks[nx], kr);
+            dc = sh.decay[st][nx]; bt = sh.beta[st][nx]; vj = sh.v[st][nx][cl];
+        }
+        u64 out = 0;
+#pragma unroll
+        for (int i = 0; i < 16; i++) sz_fma2(out, S[i], qr[i]);
+        keep_runs(nr - 1, out);
+        __syncwarp();
+        if (lane == 0) sz_mbar_arrive(&sh.empty[st]);
+        // the outputs of the warp's columns: a thread adds the runs of every NW-th row
+#pragma unroll
+        for (int e = 0; e < RC / NW; e++) {
+            const int jj = rq + NW * e;
+            if (jj < nr) {
+                double tot = 0.0;
+#pragma unroll
+                for (int p = 0; p < D / 64; p++) {
+                    double s = 0.0;
+#pragma unroll
+                    for (int i = 0; i < 4; i++) s += (double)sh.orun[jj][4 * p + i][cl];
+                    tot += s;
+                }
+                o[(size_t)(c * RC + jj) * vd + cl] = (float)tot;
+            }
+        }
+        __syncwarp();            // (read before the next rows' runs are written)
+    }
+    float* So = (cur ? sq.S0 : sq.S1) + Sat;
+#pragma unroll
+    for (int i = 0; i < 16; i++) { So[(size_t)i * D] = __uint_as_float((u32)S[i]); So[(size_t)(16 + i) * D] = __uint_as_float((u32)(S[i] >> 32)); }
+}
+
+// The scan's outputs through the gated RMS norm of their head (sz_delta_scan_body's `finish`), a warp a (row, value head): into xh as the
+// output projection's f16 high and low parts (sz_dense_rows_pack_kernel's) or, where that takes another form, in place.
+// grid (rows * vh / 8), block 256
+template <int D>
+__global__ void __launch_bounds__(256)
+sz_rows_gate_kernel(float* __restrict__ og, const float* __restrict__ z, const float* __restrict__ norm_w, int rows, int vh, float eps, int padded, __half* __restrict__ xh) {
+    const int lane = threadIdx.x & 31, item = blockIdx.x * 8 + (threadIdx.x >> 5);
+    float nw[D / 32];
+#pragma unroll
+    for (int i = 0; i < D / 32; i++) nw[i] = __ldg(norm_w + lane + 32 * i);
+    sz_pdl_wait();
+    sz_pdl_trigger();
+    if (item >= rows * vh) return;
+    const size_t at = (size_t)item * D + lane;
+    float o[D / 32], zv[D / 32];
+#pragma unroll
+    for (int i = 0; i < D / 32; i++) { o[i] = __ldcg(og + at + 32 * i); zv[i] = __ldcg(z + at + 32 * i); }
+    double ss = 0.0;
+#pragma unroll
+    for (int i = 0; i < D / 32; i++) ss += (double)o[i] * (double)o[i];
+    ss = sz_warp_sum(ss);
+    const double rr = sz_rsqrt64(ss / (double)D + (double)eps);
+#pragma unroll
+    for (int i = 0; i < D / 32; i++) {
+        const float y = __fmul_rn((float)((double)o[i] * rr) * nw[i], sz_sigmoid(zv[i]));      // (rounded before the high part is taken from it)
+        if (xh == nullptr) { og[at + 32 * i] = y; continue; }
+        const __half h = __float2half_rn(y);
+        xh[at + 32 * i] = h;
+        xh[(size_t)padded * vh * D + at + 32 * i] = __float2half_rn(y - __half2float(h));
+    }
 }
 
 // After a step: the sequences whose rows were all kept move on, and what a kernel over all rows raised in the step's error word becomes

@@ -24,6 +24,25 @@ def dm():
     return md.DeviceModel(md.make_model(CFG, expert_type=szlib.TYPE_EXL3(3), seed=4, cycle_alpha=0.9, cycle_beta=0.5))
 
 
+# the scan's stages of 8 rows: two, three, more than its ring; states of 64 and of 128 rows; value heads that share a key head
+@pytest.mark.parametrize("n,d,kh,vh", [(17, 128, 4, 4), (25, 128, 2, 4), (66, 128, 1, 3), (41, 64, 2, 4)])
+def test_the_scan_of_a_chunk_equals_the_scans_of_passes(n, d, kh, vh):
+    cfg = dict(CFG, n_layer=2, ssm_head_dim=d, ssm_k_heads=kh, ssm_v_heads=vh)
+    dm = md.DeviceModel(md.make_model(cfg, expert_type=szlib.TYPE_EXL3(3), seed=14))
+    prompt = md.make_prompt(n, cfg["vocab"], seed=n)
+    a, b = md.Session(dm, 160, kv_q8=True), md.Session(dm, 160, kv_q8=True)
+    a.prefill(prompt)
+    for c in range(0, n, 8):
+        rows = prompt[c:c + 8]
+        b.verify(rows)
+        if c + 8 < n:
+            b.result()
+            b.commit(len(rows))
+    _, top, lg = a.result(logits=True)
+    _, top2, lg2 = b.result(logits=True)
+    assert np.array_equal(lg.view(np.uint32), lg2.view(np.uint32)) and np.array_equal(top, top2)
+
+
 # 16 rows: the fewest that go as a chunk; 128 / 136: where the reads change their form; 512 / 520: one chunk, two
 @pytest.mark.parametrize("n", [16, 17, 25, 129, 137, 145, 265, 513, 521, 529])
 def test_a_prompt_in_chunks_equals_passes_of_eight_rows(dm, n):
