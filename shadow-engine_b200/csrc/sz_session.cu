@@ -1481,11 +1481,11 @@ extern "C" int sz_session_commit_path(sz_session* s, const int32_t* path, int n,
 
 // Feeds a prompt: chunks of many rows, then passes of up to 8, every row kept; the head runs for the last pass only.  Afterwards sz_session_result gives the
 // top-64 (and logits) of the last pass's rows; the last row's are the prompt's.
-static int sz_prefill_chunks(sz_session* s, const int32_t* ids, int body, uint64_t stream, int* done);
+static int sz_prefill_chunks(sz_session* s, const int32_t* ids, int n, uint64_t stream, int* done);
 extern "C" int sz_session_prefill(sz_session* s, const int32_t* ids, int n, uint64_t stream) {
     if (!s || !ids || n < 1) return sz_fail(SZ_E_ARG, "sz_session_prefill: nothing to feed");
     int done = 0;
-    const int crc = sz_prefill_chunks(s, ids, n - ((n - 1) % SZ_MAX_VERIFY + 1), stream, &done);   // all but the last pass, where the session has room for chunks
+    const int crc = sz_prefill_chunks(s, ids, n, stream, &done);   // all of it, or all but the last pass, where the session has room for chunks
     if (crc) return crc;
     while (done < n) {
         const int m = n - done < SZ_MAX_VERIFY ? n - done : SZ_MAX_VERIFY;
@@ -1745,9 +1745,10 @@ static int sz_rows_attn(cudaStream_t st, const sz_model_config& c, const float* 
     return SZ_OK;
 }
 
-// The layers for the rows of n sequences (all[b]: a prompt's chunk).  Leaves the rows' sublayer inputs of the output read in the
-// scratch's X when `read_out`, and commits the chunks on the device.
-static int sz_rows_layers(sz_session* const* ss, int n, const int32_t* ids, const int32_t* ms, const int* all, bool read_out, const SzBatchScratch& S, int rows_max,
+// The layers for the rows of n sequences.  keep[b]: sequence b's first rows that are a prompt's chunk - kept, and committed on the device -, a
+// multiple of 8 or all of them; the rows after them are a pass that stands on them.  Leaves the rows' sublayer inputs of the output read in the
+// scratch's X when `read_out`.
+static int sz_rows_layers(sz_session* const* ss, int n, const int32_t* ids, const int32_t* ms, const int* keep, bool read_out, const SzBatchScratch& S, int rows_max,
                           u8* base, cudaStream_t st) {
     sz_session* s0 = ss[0];
     const sz_model_config& c = s0->model.cfg;
@@ -1774,9 +1775,9 @@ static int sz_rows_layers(sz_session* const* ss, int n, const int32_t* ids, cons
         q.S0 = s->S[0]; q.S1 = s->S[1]; q.conv0 = s->conv[0]; q.conv1 = s->conv[1];
         q.xc = s->d_xc; q.beta = s->d_beta; q.decay = s->d_decay; q.xin = s->d_xin;
         q.kv_layer = (long long)s->ctx * nkv * (hd + (((hd >> 5) * 2 + 15) & ~15));
-        q.ctx = s->ctx; q.off = row; q.m = ms[b]; q.all = all[b];
+        q.ctx = s->ctx; q.off = row; q.m = ms[b]; q.keep = keep[b];
         memcpy(q.staged, s->h_pin, 128);
-        memcpy(q.staged, ids + row, (size_t)(ms[b] < SZ_MAX_VERIFY ? ms[b] : SZ_MAX_VERIFY) * 4);
+        memcpy(q.staged, ids + row + keep[b], (size_t)(ms[b] - keep[b]) * 4);
         for (int j = 0; j < ms[b]; j++) { hr[row + j].seq = (int16_t)b; hr[row + j].j = (int16_t)j; }
         row += ms[b];
     }
@@ -1876,7 +1877,10 @@ static int sz_rows_layers(sz_session* const* ss, int n, const int32_t* ids, cons
                               dim3((ch + 255) / 256, (R + SZ_PREP_ROWS - 1) / SZ_PREP_ROWS), dim3(256), 0, st, true, seqs, rws, R, di, (const float*)outs[0],
                               (const float*)L.ssm_conv1d.data, (const float*)outs[2], (const float*)outs[3], (const float*)L.ssm_a.data, (const float*)L.ssm_dt_bias.data,
                               kh, vh, d, (int)c.conv_k, XC, BETA, DECAY));
-            SZ_CUDA(sz_launch("rows_scan", d == 128 ? sz_rows_scan_kernel<128> : sz_rows_scan_kernel<64>, dim3(vh * (d / 32), n), dim3(d + 32), 0, st, true, seqs, di,
+            // (up to two blocks a multiprocessor: as many registers as the row's chain can use; more of them: three fit)
+            const bool few = vh * (d / 32) * n <= 2 * sz_sm_count_session();
+            const auto scan = d == 128 ? (few ? sz_rows_scan_kernel<128, 2> : sz_rows_scan_kernel<128, 3>) : (few ? sz_rows_scan_kernel<64, 2> : sz_rows_scan_kernel<64, 5>);
+            SZ_CUDA(sz_launch("rows_scan", scan, dim3(vh * (d / 32), n), dim3(d + 32), 0, st, true, seqs, di,
                               (const float*)XC, (const float*)BETA, (const float*)DECAY, kh, vh, CORE, err));
             packed = in_xh(o);
             SZ_CUDA(sz_launch("rows_gate", d == 128 ? sz_rows_gate_kernel<128> : sz_rows_gate_kernel<64>, dim3((R * vh + 7) / 8), dim3(256), 0, st, true, CORE,
@@ -1887,7 +1891,18 @@ static int sz_rows_layers(sz_session* const* ss, int n, const int32_t* ids, cons
         if ((rc = sz_hc_read_rows(s0, st, L.hc_ffn, Rp, hn++, true, true, BB, true))) return rc;
         if ((rc = sz_moe_rows_live(&L.moe, (uint64_t)X, Rp, R, rows_max, (uint64_t)Y, (uint64_t)(base + S.moe), S.moe_bytes, (uint64_t)st))) return rc;
     }
-    if (read_out && (rc = sz_hc_read_rows(s0, st, s0->model.output_hc, Rp, hn++, true, false, BB, true))) return rc;
+    if (read_out) {     // (the chunks' rows ahead of the first pass's need none)
+        int first = 0;
+        for (int b = 0; b < n && keep[b] == ms[b]; b++) first += ms[b];
+        for (int b = 0; b < n; b++) if (keep[b] < ms[b]) { first += keep[b]; break; }
+        first &= ~7;
+        const int64_t CH = (int64_t)c.streams * c.hidden;
+        SzBatchBufs BT = BB;
+        BT.r += first * CH; BT.r2 += first * CH; BT.rn += first * CH;
+        BT.y += (int64_t)first * c.hidden; BT.u += (int64_t)first * c.hidden; BT.acc += (int64_t)first * SZ_HC_ACC_ROWS;
+        if (BT.hd) BT.hd += (int64_t)first * c.hc_rank;
+        if ((rc = sz_hc_read_rows(s0, st, s0->model.output_hc, Rp - first, hn++, true, false, BT, true))) return rc;
+    }
     SZ_CUDA(sz_launch("rows_commit", sz_rows_commit_kernel, dim3(1), dim3(SZ_BATCH_MAX), 0, st, true, seqs, n, err));
     return SZ_OK;
 }
@@ -1950,8 +1965,9 @@ static bool sz_rows_step_fits(sz_session* const* ss, int n) {
 // SZ_ACCEPT_NONE, _GREEDY or _ALL, as sz_session_verify.  Afterwards every session holds a pending pass: sz_session_result and
 // sz_session_commit per session, as after a pass of its own.
 // (accept[b], heads[b]: sequence b's acceptance mode and whether its rows go through the head - a prompt's passes before its last
-// keep all rows and need no logits)
-static int sz_batch_step(sz_session* const* ss, int n, const int32_t* ids, const int32_t* ms, const int* accept, const int* heads, int eog_token,
+// keep all rows and need no logits; keep[b], where sz_rows_step_fits: of the rows of a pass with a head, the first ones that are the chunk of a
+// prompt which the pass ends: a multiple of 8)
+static int sz_batch_step(sz_session* const* ss, int n, const int32_t* ids, const int32_t* ms, const int* accept, const int* heads, const int* keep, int eog_token,
                          int rows_max, uint64_t scratch, int64_t scratch_bytes, uint64_t stream) {
     if (!ss || !ids || !ms || n < 1 || n > SZ_BATCH_MAX) return sz_fail(SZ_E_ARG, "sz_batch_verify: 1..%d sequences", SZ_BATCH_MAX);
     bool any_head = false;
@@ -1976,7 +1992,7 @@ static int sz_batch_step(sz_session* const* ss, int n, const int32_t* ids, const
             return sz_fail(SZ_E_ARG, "sz_batch_verify: sequence %d is not a session of the same model", b);
         for (int q = 0; q < b; q++) if (ss[q] == s) return sz_fail(SZ_E_ARG, "sz_batch_verify: a session appears twice");
         const int m = ms[b];
-        if (m < 1 || (m > SZ_MAX_VERIFY && heads[b])) return sz_fail(SZ_E_ARG, "a pass has 1..%d rows, got %d", SZ_MAX_VERIFY, m);
+        if (m < 1 || (m - keep[b] > SZ_MAX_VERIFY && heads[b])) return sz_fail(SZ_E_ARG, "a pass has 1..%d rows, got %d", SZ_MAX_VERIFY, m);
         if (s->last_m) return sz_fail(SZ_E_ARG, "sequence %d: the previous pass was not committed", b);
         if (s->len + m > s->ctx) return sz_fail(SZ_E_ARG, "sequence %d: %d positions + %d rows exceed the session's capacity %d", b, s->len, m, s->ctx);
         if (s->want_routes) return sz_fail(SZ_E_ARG, "sz_batch_verify: no routing trace in a batched step");
@@ -1987,12 +2003,14 @@ static int sz_batch_step(sz_session* const* ss, int n, const int32_t* ids, const
     const int Rp = (R + 7) & ~7;
     if (Rp > rows_max) return sz_fail(SZ_E_ARG, "sz_batch_verify: %d rows in a scratch for %d", R, rows_max);
     if (sz_rows_step_fits(ss, n)) {
-        int all[SZ_BATCH_MAX];
+        int kept[SZ_BATCH_MAX];     // rows that the layers commit
         for (int b = 0; b < n; b++) {
-            all[b] = accept[b] == SZ_ACCEPT_ALL && !heads[b];
+            kept[b] = accept[b] == SZ_ACCEPT_ALL && !heads[b] ? ms[b] : keep[b];
             ss[b]->tree_pass = 0;
         }
-        if ((rc = sz_rows_layers(ss, n, ids, ms, all, any_head, S, rows_max, (u8*)scratch, st))) return rc;
+        if ((rc = sz_rows_layers(ss, n, ids, ms, kept, any_head, S, rows_max, (u8*)scratch, st))) return rc;
+        for (int b = 0; b < n; b++)
+            if (kept[b]) { ss[b]->cur ^= 1; ss[b]->len += kept[b]; }
         if (any_head) {
             // the head, acceptance and commit stay launches of the sequence, each sequence's on a stream of its own
             SzBatchStreams fan;
@@ -2000,21 +2018,22 @@ static int sz_batch_step(sz_session* const* ss, int n, const int32_t* ids, const
             float* X = (float*)((u8*)scratch + S.x);
             rc = fan.each([&](int b, cudaStream_t sb) -> int {
                 sz_session* s = ss[b];
-                if (all[b]) return SZ_OK;
+                const int m = ms[b] - kept[b];
+                if (!m) return SZ_OK;
                 float* const u = s->u;
-                s->u = X + (size_t)tab.off[b] * c.hidden;
-                int r = heads[b] ? sz_forward_head(s, sb, ms[b], true, false) : SZ_OK;
+                s->u = X + (size_t)(tab.off[b] + kept[b]) * c.hidden;
+                int r = heads[b] ? sz_forward_head(s, sb, m, true, false) : SZ_OK;
                 s->u = u;
-                return r ? r : sz_pass_tail(s, sb, ms[b], accept[b], eog_token, heads[b] != 0);
+                return r ? r : sz_pass_tail(s, sb, m, accept[b], eog_token, heads[b] != 0);
             });
             if (rc || (rc = fan.end())) return rc;
         }
         for (int b = 0; b < n; b++) {
             sz_session* s = ss[b];
-            if (all[b]) { s->cur ^= 1; s->len += ms[b]; continue; }    // (committed on the device; nothing is pending)
-            s->last_m = ms[b];
+            if (kept[b] == ms[b]) continue;    // (committed on the device; nothing is pending)
+            s->last_m = ms[b] - kept[b];
             s->pending_committed = accept[b] != SZ_ACCEPT_NONE;
-            s->device_keep = accept[b] == SZ_ACCEPT_ALL ? ms[b] : -1;
+            s->device_keep = accept[b] == SZ_ACCEPT_ALL ? s->last_m : -1;
         }
         return SZ_OK;
     }
@@ -2301,9 +2320,11 @@ extern "C" int sz_session_use_room(sz_session* s, sz_room* r) {
     s->room = r ? r->r : s->own_room;
     return SZ_OK;
 }
-// The first `body` tokens (whole passes' worth) of a prompt in chunks of equal size: *done of them, 0 when the session's prompts go in
-// passes.  A chunk costs little more for more rows (every expert's decode is the most of it), so chunks are as long as there is room.
-static int sz_prefill_chunks(sz_session* s, const int32_t* ids, int body, uint64_t stream, int* done) {
+// A prompt of n tokens in chunks of equal size: *done of them, 0 when the session's prompts go in passes.  A chunk costs little more for more
+// rows (every expert's decode is the most of it), so chunks are as long as there is room, and the last one carries the rows of the prompt's last
+// pass, too, where they fit beside it (a pass of its own would read every layer again: 5 ms of the 92 of 507 tokens); else all but them are done.
+static int sz_prefill_chunks(sz_session* s, const int32_t* ids, int n, uint64_t stream, int* done) {
+    const int last = (n - 1) % SZ_MAX_VERIFY + 1, body = n - last;
     sz_session* const one[1] = {s};
     if (!s->room || body < 2 * SZ_MAX_VERIFY || s->last_m || s->len + body > s->ctx || !sz_rows_step_fits(one, 1)) return SZ_OK;
     const std::shared_ptr<SzRoom> room = s->room;
@@ -2313,9 +2334,11 @@ static int sz_prefill_chunks(sz_session* s, const int32_t* ids, int body, uint64
     const int chunks = (body + room->rows - 1) / room->rows;
     const int size = ((body + chunks - 1) / chunks + SZ_MAX_VERIFY - 1) / SZ_MAX_VERIFY * SZ_MAX_VERIFY;
     while (*done < body) {
-        const int32_t m = body - *done < size ? body - *done : size;
-        const int accept = SZ_ACCEPT_ALL, head = 0;
-        if ((rc = sz_batch_step(one, 1, ids + *done, &m, &accept, &head, -1, room->rows, room->mem, room->bytes, stream))) return rc;
+        int32_t m = body - *done < size ? body - *done : size;
+        const bool ends = *done + m == body && m + SZ_MAX_VERIFY <= room->rows && s->len + m + last <= s->ctx;
+        const int accept = ends ? SZ_ACCEPT_NONE : SZ_ACCEPT_ALL, head = ends, keep = ends ? m : 0;
+        if (ends) m += last;
+        if ((rc = sz_batch_step(one, 1, ids + *done, &m, &accept, &head, &keep, -1, room->rows, room->mem, room->bytes, stream))) return rc;
         *done += m;
     }
     return SZ_OK;
@@ -2326,8 +2349,9 @@ extern "C" int sz_batch_verify(sz_session* const* ss, int n, const int32_t* ids,
     if (n < 1 || n > SZ_BATCH_MAX) return sz_fail(SZ_E_ARG, "sz_batch_verify: 1..%d sequences", SZ_BATCH_MAX);
     if (sz_batch_rows_check(rows_max)) return SZ_E_ARG;
     int accept[SZ_BATCH_MAX], heads[SZ_BATCH_MAX];
+    const int keep[SZ_BATCH_MAX] = {};
     for (int b = 0; b < n; b++) { accept[b] = accept_mode; heads[b] = 1; }
-    return sz_batch_step(ss, n, ids, ms, accept, heads, eog_token, rows_max, scratch, scratch_bytes, stream);
+    return sz_batch_step(ss, n, ids, ms, accept, heads, keep, eog_token, rows_max, scratch, scratch_bytes, stream);
 }
 
 // The prompts of n sequences fed in lockstep: every step takes up to 8 rows of every sequence that still has some (as many
@@ -2357,7 +2381,7 @@ extern "C" int sz_batch_prefill(sz_session* const* ss, int n, const int32_t* con
     for (;;) {
         sz_session* step_s[SZ_BATCH_MAX];
         int32_t step_m[SZ_BATCH_MAX];
-        int accept[SZ_BATCH_MAX], heads[SZ_BATCH_MAX], who[SZ_BATCH_MAX];
+        int accept[SZ_BATCH_MAX], heads[SZ_BATCH_MAX], keep[SZ_BATCH_MAX], who[SZ_BATCH_MAX];
         std::vector<int32_t> rows;
         int k = 0, room = rows_max;
         for (int b = 0; b < n; b++) {
@@ -2367,15 +2391,19 @@ extern "C" int sz_batch_prefill(sz_session* const* ss, int n, const int32_t* con
             int m = body > 0 ? SZ_MAX_VERIFY : last_m;
             if (body > 0 && chunks) m = body < room / SZ_MAX_VERIFY * SZ_MAX_VERIFY ? body : room / SZ_MAX_VERIFY * SZ_MAX_VERIFY;
             if (m < 1 || m > room) { if (chunks) continue; break; }
+            // the prompt's last pass along with its last chunk where that fits: a step less for its few rows
+            const bool ends = body <= 0 || (chunks && m == body && body + last_m <= room && ss[b]->len + body + last_m <= ss[b]->ctx);
+            keep[k] = ends && body > 0 ? body : 0;
+            if (keep[k]) m += last_m;
             room -= chunks ? m : SZ_MAX_VERIFY;
             step_s[k] = ss[b]; step_m[k] = m; who[k] = b;
-            heads[k] = body > 0 ? 0 : 1;
-            accept[k] = body > 0 ? SZ_ACCEPT_ALL : SZ_ACCEPT_NONE;
+            heads[k] = ends ? 1 : 0;
+            accept[k] = ends ? SZ_ACCEPT_NONE : SZ_ACCEPT_ALL;
             rows.insert(rows.end(), ids[b] + done[b], ids[b] + done[b] + m);
             k++;
         }
         if (k == 0) return SZ_OK;
-        int rc = sz_batch_step(step_s, k, rows.data(), step_m, accept, heads, -1, rows_max, scratch, scratch_bytes, stream);
+        int rc = sz_batch_step(step_s, k, rows.data(), step_m, accept, heads, keep, -1, rows_max, scratch, scratch_bytes, stream);
         if (rc) return rc;
         for (int i = 0; i < k; i++) {
             const int b = who[i];

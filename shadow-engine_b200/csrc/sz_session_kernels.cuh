@@ -29,7 +29,7 @@ struct SzSeqDev {
     float *xc, *beta, *decay, *xin;                 // what a replay reads, DeltaNet layer 0
     long long kv_layer;                             // bytes from one attention layer's cache to the next
     int ctx, off, m;                                // capacity; its first row in the step, and how many
-    int all;                                        // a prompt's chunk: every row is kept, nothing will be replayed
+    int keep;                                       // its first rows that are a prompt's chunk: kept, not replayed (a multiple of 8, or all of them)
     int staged[32];                                 // the staging block's first 32 words
 };
 // A row: its sequence, its place in it, where its attention splits' partial results lie.

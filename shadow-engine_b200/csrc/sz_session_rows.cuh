@@ -337,8 +337,8 @@ sz_hc_up_rows_kernel(const float* __restrict__ hd, const u8* __restrict__ up, co
 }
 
 // The DeltaNet front end over the rows of a step (sz_delta_prep_kernel's arithmetic).  grid (ceil(ch / 256), ceil(rows / SZ_PREP_ROWS)).
-// What the scan reads - and a replay, when the sequence's rows may be rejected - goes to the session's buffers, of a prompt's chunk to
-// the step's (xc_all, beta_all, decay_all), and a chunk's last row leaves the carried conv rows behind it in the other buffer.
+// What the scan reads goes to the step's buffers (xc_all, beta_all, decay_all), what a replay reads - of rows that may be rejected - to the
+// session's, too, and the last row of a prompt's chunk leaves the carried conv rows behind it in the other buffer.
 // A thread takes its channel for 4 rows of the step: taps and their conversions once, a projection loaded for its own row serves the three
 // after it (a row a block: 504 rows 71 -> 45 us).  K: the taps where they are the usual 4, else 0.
 #define SZ_PREP_ROWS 4
@@ -391,12 +391,12 @@ sz_rows_delta_prep_kernel(const SzSeqDev* __restrict__ seqs, const SzRowDev* __r
                     acc += taps[t] * (double)prev;
                 }
             v[e] = sz_silu((float)acc);
-            if (!q.all) q.xin[((size_t)di * SZ_MAX_VERIFY + j) * ch + i] = own;
-            else if (j == q.m - 1) {
+            if (j >= q.keep) q.xin[((size_t)di * SZ_MAX_VERIFY + j - q.keep) * ch + i] = own;
+            else if (j == q.keep - 1) {
                 float* convw = (cur ? q.conv0 : q.conv1) + di * cl;
                 const float* x = xin + (size_t)(r0 + e) * ch;
                 for (int t = 0; t < k - 1; t++) {
-                    const int tau = q.m - (k - 1) + t;
+                    const int tau = q.keep - (k - 1) + t;
                     convw[(size_t)t * ch + i] = tau >= 0 ? x[(long long)(t - (k - 2)) * ch + i] : conv[(size_t)((k - 1) + tau) * ch + i];
                 }
             }
@@ -424,17 +424,21 @@ sz_rows_delta_prep_kernel(const SzSeqDev* __restrict__ seqs, const SzRowDev* __r
                 if (i < kd) t = t / sqrtf((float)d);
                 out = t;
             }
-            (q.all ? xc_all + (size_t)(r0 + e) * ch : q.xc + ((size_t)di * SZ_MAX_VERIFY + j) * ch)[i] = out;
+            xc_all[(size_t)(r0 + e) * ch + i] = out;
+            if (j >= q.keep) q.xc[((size_t)di * SZ_MAX_VERIFY + j - q.keep) * ch + i] = out;
         }
         if (blockIdx.x == 0) {
             const int r = r0 + e;
-            float* beta = q.all ? beta_all + (size_t)r * vh : q.beta + ((size_t)di * SZ_MAX_VERIFY + j) * vh;
-            float* decay = q.all ? decay_all + (size_t)r * vh : q.decay + ((size_t)di * SZ_MAX_VERIFY + j) * vh;
             for (int h = threadIdx.x; h < vh; h += 256) {
-                beta[h] = sz_sigmoid(b[(size_t)r * vh + h]);
+                const float bt = sz_sigmoid(b[(size_t)r * vh + h]);
                 const float sp_in = a[(size_t)r * vh + h] + dt[h];
                 const float sp = sp_in > 20.0f ? sp_in : log1pf(expf(sp_in));
-                decay[h] = expf(a_log[h] * sp);
+                const float dc = expf(a_log[h] * sp);
+                beta_all[(size_t)r * vh + h] = bt; decay_all[(size_t)r * vh + h] = dc;
+                if (j >= q.keep) {
+                    const size_t at = ((size_t)di * SZ_MAX_VERIFY + j - q.keep) * vh + h;
+                    q.beta[at] = bt; q.decay[at] = dc;
+                }
             }
         }
     }
@@ -450,11 +454,11 @@ sz_rows_delta_prep_kernel(const SzSeqDev* __restrict__ seqs, const SzRowDev* __r
 //   - the output products of a row run beside the next row's k products; runs of 8 rows are added up at once, and left unnormed: the gated
 //     norm over a head's D outputs is sz_rows_gate_kernel's, not eight f64 chains a stage inside this one;
 //   - a fifth warp keeps SZ_RS_STAGES stages of 8 rows' operands on their way.
-// Measured (128 x 128 states, 32 heads; us a launch, events between the launches): 504 rows of one prompt 298 -> 186 and 10 for the gate, which
-// packs the rows as a launch of 7 did before; 80 rows of 32 sequences 63 -> 48 and 8.  A row takes some 800 cycles: 300 the products with
+// Measured (128 x 128 states, 32 heads; us a launch, events between the launches): 504 rows of one prompt 298 -> 169 and 10 for the gate, which
+// packs the rows as a launch of 7 did before; 80 rows of 32 sequences 63 -> 48 and 8.  MINB: blocks a multiprocessor that the registers leave room
+// for - 2 where no more come (three: 186 for one prompt), 3 for many sequences (two: 57 for the 32).  A row takes some 800 cycles: 300 the products with
 // the reads of its operands, 270 the sum (two conversions of 27 cycles, ten f64 operations of 8, two shuffles), 105 the update, 115 a row's share of a
-// stage.  The next row's k in registers of its own or conversions by integer instructions: 179 for one prompt, but 57 - 60 for 32 sequences,
-// whose blocks then fit twice a multiprocessor instead of three times.
+// stage.  The next row's k in registers of its own, its reads in a fixed order, or conversions by integer instructions: 179 - 190 for one prompt.
 // grid (vh * D / 32, sequences), block D + 32
 #define SZ_RS_STAGES 3
 #define SZ_RS_SEG 36          // floats between the 32 k (or q) of one thread of a column and the next one's (32, kept out of each other's banks)
@@ -466,8 +470,8 @@ struct SzRowsScan {
     u64 full[SZ_RS_STAGES], empty[SZ_RS_STAGES];
     u64 nz2;                                     // two floats, -0
 };
-template <int D>
-__global__ void __launch_bounds__(D + 32)
+template <int D, int MINB>
+__global__ void __launch_bounds__(D + 32, MINB)
 sz_rows_scan_kernel(const SzSeqDev* __restrict__ seqs, int di, const float* __restrict__ xc_all, const float* __restrict__ beta_all, const float* __restrict__ decay_all,
                     int kh, int vh, float* __restrict__ og, u32* __restrict__ err) {
     constexpr int NW = D / 32, CW = 32 / NW, RC = SZ_SCAN_RC, ST = SZ_RS_STAGES;     // warps that scan (and threads a column); columns a warp
@@ -495,10 +499,8 @@ sz_rows_scan_kernel(const SzSeqDev* __restrict__ seqs, int di, const float* __re
     const int sets = (rows + RC - 1) / RC;
     if (warp == NW) {
         // ---- the operands' warp
-        const size_t at = (size_t)di * SZ_MAX_VERIFY;
-        const float* x = (sq.all ? xc_all + (size_t)off * ch : sq.xc + at * ch);
-        const float* be = (sq.all ? beta_all + (size_t)off * vh : sq.beta + at * vh) + hd;
-        const float* de = (sq.all ? decay_all + (size_t)off * vh : sq.decay + at * vh) + hd;
+        const float* x = xc_all + (size_t)off * ch;
+        const float *be = beta_all + (size_t)off * vh + hd, *de = decay_all + (size_t)off * vh + hd;
         float4 qv[RC], kv[RC];
         float vv[RC], bv = 0.f, dv = 0.f;
         auto load = [&](int c0) {
@@ -534,6 +536,13 @@ sz_rows_scan_kernel(const SzSeqDev* __restrict__ seqs, int di, const float* __re
         }
         return;
     }
+    // the state goes to the other buffer; where a pass follows the chunk, the chunk's does - it is the pass's to start from - and the pass's to this one
+    auto leave = [&](bool other) {
+        float* So = ((cur != 0) == other ? sq.S0 : sq.S1) + Sat;
+#pragma unroll
+        for (int i = 0; i < 16; i++) { So[(size_t)i * D] = __uint_as_float((u32)S[i]); So[(size_t)(16 + i) * D] = __uint_as_float((u32)(S[i] >> 32)); }
+    };
+    const int chunk = sq.keep < rows ? sq.keep : 0;
     float* o = og + (size_t)off * vd + hd * D + cb * 32;
     u64 kr[16], qr[16], nz2;
     nz2 = *(volatile u64*)&sh.nz2;
@@ -605,10 +614,9 @@ sz_rows_scan_kernel(const SzSeqDev* __restrict__ seqs, int di, const float* __re
             }
         }
         __syncwarp();            // (read before the next rows' runs are written)
+        if ((c + 1) * RC == chunk) leave(true);
     }
-    float* So = (cur ? sq.S0 : sq.S1) + Sat;
-#pragma unroll
-    for (int i = 0; i < 16; i++) { So[(size_t)i * D] = __uint_as_float((u32)S[i]); So[(size_t)(16 + i) * D] = __uint_as_float((u32)(S[i] >> 32)); }
+    leave(chunk == 0);
 }
 
 // The scan's outputs through the gated RMS norm of their head (sz_delta_scan_body's `finish`), a warp a (row, value head): into xh as the
@@ -643,7 +651,7 @@ sz_rows_gate_kernel(float* __restrict__ og, const float* __restrict__ z, const f
     }
 }
 
-// After a step: the sequences whose rows were all kept move on, and what a kernel over all rows raised in the step's error word becomes
+// After a step: the sequences move on by the rows of their chunks, and what a kernel over all rows raised in the step's error word becomes
 // every sequence's own (it stays there until the session is reset; the step's word is ready for whoever has the room next).  One block.
 __global__ void sz_rows_commit_kernel(const SzSeqDev* __restrict__ seqs, int n, u32* __restrict__ err) {
     sz_pdl_wait();
@@ -653,8 +661,8 @@ __global__ void sz_rows_commit_kernel(const SzSeqDev* __restrict__ seqs, int n, 
     if (b < n) {
         int32_t* state = const_cast<int32_t*>(seqs[b].state);
         if (e) atomicOr((u32*)state + 2, e);
-        if (seqs[b].all) {
-            state[0] += seqs[b].m;
+        if (seqs[b].keep) {
+            state[0] += seqs[b].keep;
             state[1] ^= 1;
         }
     }

@@ -43,6 +43,32 @@ def test_the_scan_of_a_chunk_equals_the_scans_of_passes(n, d, kh, vh):
     assert np.array_equal(lg.view(np.uint32), lg2.view(np.uint32)) and np.array_equal(top, top2)
 
 
+# the rows of a prompt's last pass go with its last chunk: 1 and 8 of them; two chunks; a full room, where they do not fit; a session with
+# no position to spare.  Then some of them are kept, and the next pass stands on chunk and pass.
+@pytest.mark.parametrize("n,keep,ctx", [(17, 1, 64), (24, 3, 64), (31, 7, 64), (67, 0, 128), (48, 8, 48), (512, 5, 560), (520, 2, 560), (525, 4, 560)])
+def test_a_prompts_last_pass_beside_its_last_chunk(dm, n, keep, ctx):
+    prompt = md.make_prompt(n, CFG["vocab"], seed=90 + n)
+    a, b = md.Session(dm, ctx, kv_q8=True), md.Session(dm, ctx, kv_q8=True)
+    a.prefill(prompt)
+    for c in range(0, n, 8):
+        rows = prompt[c:c + 8]
+        b.verify(rows)
+        if c + 8 < n:
+            b.result()
+            b.commit(len(rows))
+    for s in (a, b):
+        s.first = s.result(logits=True)
+        s.commit(keep)
+    assert a.first[2].shape == b.first[2].shape and np.array_equal(a.first[2].view(np.uint32), b.first[2].view(np.uint32)) and np.array_equal(a.first[1], b.first[1])
+    assert len(a) == len(b) == (n - 1) // 8 * 8 + keep
+    if len(a) + 4 > ctx:
+        return
+    for s in (a, b):
+        s.verify([7, 8, 9, 10])
+        s.second = s.result(logits=True)
+    assert np.array_equal(a.second[2].view(np.uint32), b.second[2].view(np.uint32)) and np.array_equal(a.second[1], b.second[1])
+
+
 # 16 rows: the fewest that go as a chunk; 128 / 136: where the reads change their form; 512 / 520: one chunk, two
 @pytest.mark.parametrize("n", [16, 17, 25, 129, 137, 145, 265, 513, 521, 529])
 def test_a_prompt_in_chunks_equals_passes_of_eight_rows(dm, n):
