@@ -3,7 +3,7 @@
 // reference's grouped experts of a long prompt (device planner plan_scan_w / plan_fill_w, kernels/forward.cu:3234-3319; mma_grouped*,
 // kernels/matvec.cu:1190-1260; EXL3 exl3_mma, kernels/exl3.cu:500-590) with this library's exact arithmetic.
 //
-//   route     sz_route_kernel with a second grid dimension: 8 rows a block row, same arithmetic as a verify pass
+//   route     sz_route_kernel with a second grid dimension, 8 rows a block row, or sz_route_rows_kernel and sz_route_topk_kernel: a verify pass's logits and choice
 //   plan      sz_rows_plan_kernel: every expert's pairs in ascending row order side by side (a pair's place is its SLOT), cut into
 //             groups of up to 16; the shared expert's groups (16 consecutive rows each) are spread evenly among them
 //   gate/up   sz_rows_gateup_kernel: a persistent launch over all groups

@@ -73,3 +73,21 @@ def test_what_the_form_does_not_take_is_refused():
     ml2 = moe.MoeLayer(L2, "cuda:0")
     with pytest.raises(szlib.SzError):
         ml2.moe_rows(torch.zeros((12, 512), device="cuda"))     # a multiple of 8
+
+
+# either side of 128 rows, ragged tiles of rows and router rows, columns that end inside a tile's (512), three and four pieces a thread (3,072 and 4,096),
+# more experts than half a warp's registers hold (1,024), no shared expert's gate; equal experts - ties, chosen by index - and rows of zeros (all equal)
+@pytest.mark.parametrize("hidden,n_expert,top_k,shared,rows", [(512, 16, 4, True, 136), (1024, 60, 6, True, 152), (2048, 512, 10, True, 136), (2048, 1024, 16, False, 144),
+                                                                (3072, 33, 4, True, 168), (4096, 40, 3, False, 256), (2048, 300, 10, True, 200)])
+def test_routing_of_many_rows_is_the_verify_passes(hidden, n_expert, top_k, shared, rows):
+    L = synth.make_moe_layer(hidden, n_expert, top_k, 128, 128 if shared else 0, szlib.TYPE_EXL3(2), szlib.TYPE_EXL3(2), seed=27)
+    L["router"][1::3] = L["router"][0]
+    ml = moe.MoeLayer(L, "cuda:0")
+    x = synth.normal((rows, hidden), 1.0, 29, "rows.route").cuda()
+    x[5::17] = 0.0
+    y, ridx, rw = ml.moe_rows(x, want_routing=True)
+    assert ml.moe_rows_status(rows) == 0
+    for c in range(0, rows, 8):
+        yc, ic, wc = ml.moe_batch(x[c:c + 8].contiguous(), want_routing=True)
+        assert torch.equal(ridx[c:c + 8], ic) and torch.equal(rw[c:c + 8].view(torch.int64), wc.view(torch.int64)), "rows %d.." % c
+        assert torch.equal(y[c:c + 8].view(torch.int32), yc.view(torch.int32)), "rows %d.." % c
