@@ -1220,9 +1220,9 @@ static int sz_rows_run(const sz_moe_layer* L, uint64_t x, int rows, int live, ui
 #undef SZ_ROWS_ROUTE
         SZ_CUDA(e);
     }
-    const size_t pmem = (size_t)L->n_expert * (SZ_ROWS_CAP / 32) * 4;
+    const size_t pmem = sz_rows_plan_smem(L->n_expert);
     static bool set = false;
-    if (!set) { SZ_CUDA(cudaFuncSetAttribute(sz_rows_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SZ_MAX_EXPERTS * (SZ_ROWS_CAP / 32) * 4)); set = true; }
+    if (!set) { SZ_CUDA(cudaFuncSetAttribute(sz_rows_plan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sz_rows_plan_smem(SZ_MAX_EXPERTS))); set = true; }
     SZ_CUDA(sz_launch("rows_plan", sz_rows_plan_kernel, dim3(1), dim3(1024), pmem, st, true, (const int32_t*)ridx, live, (int)L->top_k, (int)L->n_expert,
                       shared ? 1 : 0, 2 * (H / 128), H / 128, H / 512 * (L->expert_ff / 128), (int)L->expert_ff / 128, sz_rows_grid(), P, err));
     const int slots = live * (L->top_k + (shared ? 1 : 0));
@@ -1233,7 +1233,7 @@ static int sz_rows_run(const sz_moe_layer* L, uint64_t x, int rows, int live, ui
     SZ_ROWS_K(2) SZ_ROWS_K(3) SZ_ROWS_K(4)
 #undef SZ_ROWS_K
     if (rc) return rc;
-    SZ_CUDA(sz_launch("rows_combine", sz_rows_combine_kernel, dim3(live * (H / 512)), dim3((L->top_k + 1) * 32), 0, st, true, (const float*)(base + S.dn),
+    SZ_CUDA(sz_launch("rows_combine", sz_rows_combine_kernel, dim3((live * (H / 128) + 7) / 8), dim3(256), 0, st, true, (const float*)(base + S.dn),
                       (const long long*)(base + S.parts), (const SzRowsPlan*)P, (const int32_t*)ridx, (const double*)rw, (const u8*)L->down, (u64)L->down_stride, (const u8*)L->sh_down,
                       (const float*)logits, (int)L->n_expert, (int)L->top_k, live, H, (int)L->expert_ff, (int)L->shared_ff, shared ? 1 : 0, (float*)y));
     return SZ_OK;

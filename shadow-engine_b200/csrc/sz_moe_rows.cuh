@@ -9,7 +9,7 @@
 //   gate/up   sz_rows_gateup_kernel: a persistent launch over all groups
 //   act       sz_rows_act_kernel: SwiGLU of every pair, left as the down product's operand fragments
 //   down      sz_rows_down_kernel: as gate/up, over those fragments
-//   combine   sz_rows_combine_kernel: per (row, 512 outputs) the ranks' terms in rank order, as sz_x3_combine_kernel adds them
+//   combine   sz_rows_combine_kernel: per (row, 128 outputs) the ranks' terms in rank order, as sz_x3_combine_kernel adds them
 // A pair's numbers do not depend on which rows share its group (every row of a group is a column of its own in the tensor-core
 // product, the sums over column blocks are integer): a row's output is bit for bit what sz_moe_verify gives for it.
 //
@@ -57,32 +57,44 @@ __device__ __forceinline__ int sz_rows_weight(int n) { return n <= 8 ? 172 + n :
 // ---- plan: one block of 1024 threads ---------------------------------------------------------------------------------------------------
 // Every (row, rank) pair marks its row in its expert's row mask; an expert's pairs in ascending row order are then the set bits of
 // its mask, and a pair's place among them the number of set bits below its row: no sorting, no order of arrival.  Slots and groups
-// are prefix sums over the experts, one a thread.  Dynamic shared memory: the masks, [experts][SZ_ROWS_CAP / 32] words.
+// are prefix sums over the experts, one a thread.  Dynamic shared memory: the masks, and the set bits before every word of them, a word an entry of
+// padding behind an expert's (sz_rows_plan_smem).
+// One block whose 32 warps wait for shared memory most of the time, so what counts is how often they go there one after the other: a pair's place
+// is one count and one word (counting its expert's words one by one, two banks for all experts, took 20,600 of 51,000 cycles at 504 rows), and the
+// block that an item falls to is guessed from its weight and put right (two binary searches an item: 16,400).  With the events around it: 504 rows 32 -> 25 us,
+// 256 25 -> 21, 80 18 -> 15.
+#define SZ_ROWS_MW (SZ_ROWS_CAP / 32 + 1)       // words of an expert's mask (odd: experts in different banks)
+static inline size_t sz_rows_plan_smem(int experts) { return (size_t)experts * SZ_ROWS_MW * 6; }
 __global__ void __launch_bounds__(1024)
 sz_rows_plan_kernel(const int32_t* __restrict__ ridx, int R, int k, int ne, int has_shared, int upg_gu, int ns, int upg_dn, int kb, int grid,
                     SzRowsPlan* __restrict__ P, u32* __restrict__ err) {
     extern __shared__ u32 mask[];
+    u16* pre = (u16*)(mask + (size_t)ne * SZ_ROWS_MW);
     __shared__ int slot_of[SZ_MAX_EXPERTS], grp_of[SZ_MAX_EXPERTS];
     __shared__ int wsum[2][32];
     __shared__ int before[SZ_ROWS_MAXG + 1];        // a group's weight, then the weights before it
     __shared__ int bs[2][SZ_ROWS_MAXB + 1];
-    constexpr int MW = SZ_ROWS_CAP / 32;
-    sz_pdl_wait();
-    sz_pdl_trigger();
+    constexpr int MW = SZ_ROWS_MW, NP = SZ_ROWS_CAP * SZ_MAX_TOPK / 1024;      // pairs a thread, at most
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31, pairs = R * k;
     const int words = (R + 31) / 32;
     for (int i = t; i < ne * MW; i += 1024) mask[i] = 0u;
+    sz_pdl_wait();
+    sz_pdl_trigger();
+    int pe[NP];                 // the pairs' experts, asked for at once
+#pragma unroll
+    for (int i = 0; i < NP; i++) pe[i] = t + 1024 * i < pairs ? __ldcg(ridx + t + 1024 * i) : -1;
     if (t == 0) P->overflow = 0;
     __syncthreads();
-    for (int p = t; p < pairs; p += 1024) {
-        const int e = __ldcg(ridx + p), row = p / k;
-        if ((unsigned)e >= (unsigned)ne) continue;     // (a routing that was never written: caught below, nothing is touched)
-        atomicOr(&mask[e * MW + (row >> 5)], 1u << (row & 31));
+#pragma unroll
+    for (int i = 0; i < NP; i++) {
+        const int row = (t + 1024 * i) / k;
+        if ((unsigned)pe[i] >= (unsigned)ne) continue;     // (a routing that was never written: caught below, nothing is touched)
+        atomicOr(&mask[pe[i] * MW + (row >> 5)], 1u << (row & 31));
     }
     __syncthreads();
     int c = 0;
     if (t < ne)
-        for (int q = 0; q < words; q++) c += __popc(mask[t * MW + q]);
+        for (int q = 0; q < words; q++) { pre[t * MW + q] = (u16)c; c += __popc(mask[t * MW + q]); }
     const int ng = (c + SZ_ROWS_G - 1) / SZ_ROWS_G;
     int sc = c, sg = ng;                                // inclusive sums over the warp, then over the warps
 #pragma unroll
@@ -134,11 +146,12 @@ sz_rows_plan_kernel(const int32_t* __restrict__ ridx, int R, int k, int ne, int 
         for (int r = t; r < R; r += 1024) { P->row[pairs + r] = (int16_t)r; P->group[pairs + r] = place_sh(r / SZ_ROWS_G); P->pair_loc[pairs + r] = pairs + r; }
     }
     __syncthreads();
-    for (int p = t; p < pairs; p += 1024) {
-        const int e = __ldcg(ridx + p), row = p / k;
+#pragma unroll
+    for (int i = 0; i < NP; i++) {
+        const int p = t + 1024 * i, e = pe[i], row = p / k;
+        if (p >= pairs) break;
         if ((unsigned)e >= (unsigned)ne) { P->pair_loc[p] = 0; P->overflow = 4; atomicOr(err, 4u); continue; }   // an expert id out of range: the call is reported as failed (the flag is this call's, the word stays)
-        int n = __popc(mask[e * MW + (row >> 5)] & ((1u << (row & 31)) - 1u));
-        for (int q = 0; q < (row >> 5); q++) n += __popc(mask[e * MW + q]);
+        const int n = pre[e * MW + (row >> 5)] + __popc(mask[e * MW + (row >> 5)] & ((1u << (row & 31)) - 1u));
         const int slot = slot_of[e] + n;
         P->row[slot] = (int16_t)row;
         P->group[slot] = place(grp_of[e] + n / SZ_ROWS_G);
@@ -175,16 +188,21 @@ sz_rows_plan_kernel(const int32_t* __restrict__ ridx, int R, int k, int ne, int 
         P->start[i & 1][b] = u;
     }
     __syncthreads();
-    auto block_of = [&](const int* st, int u) {      // the last block that starts at or before unit u
-        int lo = 0, hi = grid;
-        while (lo + 1 < hi) { const int mid = (lo + hi) >> 1; if (st[mid] <= u) lo = mid; else hi = mid; }
-        return lo;
+    // the last block that starts at or before unit u, the `r`-th of group g: about the share that the weight before it is of all
+    const float per = before[NG] > 0 ? (float)grid / (float)before[NG] : 0.f;
+    auto block_of = [&](const int* st, float inv, int g, int r, int u) {
+        int b = (int)(((float)before[g] + (float)(before[g + 1] - before[g]) * (float)r * inv) * per);
+        b = b < 0 ? 0 : (b > grid - 1 ? grid - 1 : b);
+        while (b > 0 && st[b] > u) b--;
+        while (b + 1 < grid && st[b + 1] <= u) b++;
+        return (u32)b;
     };
-    const int nc = upg_dn / kb;
-    for (int i = t; i < NG * (2 + nc); i += 1024) {
-        const int g = i / (2 + nc), q = i - g * (2 + nc);
-        if (q < 2) { const int u = g * upg_gu + q * ns; P->gu_blocks[g][q] = (u32)block_of(bs[0], u) | ((u32)block_of(bs[0], u + ns - 1) << 16); }
-        else { const int u = g * upg_dn + (q - 2) * kb; P->dn_blocks[g][q - 2] = (u32)block_of(bs[1], u) | ((u32)block_of(bs[1], u + kb - 1) << 16); }
+    const int nc = upg_dn / kb, per_g = 2 + nc;
+    const float inv_gu = 1.f / (float)upg_gu, inv_dn = 1.f / (float)upg_dn;
+    for (int i = t; i < NG * per_g; i += 1024) {
+        const int g = i / per_g, q = i - g * per_g;
+        if (q < 2) { const int r = q * ns, u = g * upg_gu + r; P->gu_blocks[g][q] = block_of(bs[0], inv_gu, g, r, u) | (block_of(bs[0], inv_gu, g, r + ns - 1, u + ns - 1) << 16); }
+        else { const int r = (q - 2) * kb, u = g * upg_dn + r; P->dn_blocks[g][q - 2] = block_of(bs[1], inv_dn, g, r, u) | (block_of(bs[1], inv_dn, g, r + kb - 1, u + kb - 1) << 16); }
     }
 }
 
@@ -583,67 +601,95 @@ sz_rows_down_kernel(const SzRowsPlan* __restrict__ P, const u8* __restrict__ dow
     if (failed && lane == 0) atomicExch(err, 1u);
 }
 
-// ---- combine: grid (rows * H / 512), block (top_k + 1) warps ---------------------------------------------------------------------------
-// y[j] = sum over ranks of w * (H eo * svh) + sigmoid(shared gate logit) * (H so * svh_shared), term by term as sz_x3_combine_kernel:
-// warp t finishes rank t's term (warp top_k: the shared expert's), then a thread adds an output's terms in rank order in f64.  dn, parts:
-// the down kernel's sums.  A block takes the 512 outputs of one of its items, so that the way to the sums - expert, slot, group, blocks:
-// four trips to memory one after the other - is gone once for 16 values a lane (a block per 128 outputs: 504 rows 55 -> 43 us).
-__global__ void __launch_bounds__((SZ_MAX_TOPK + 1) * 32)
+// ---- combine: a warp a (row, 128 outputs) ------------------------------------------------------------------------------------------------
+// y[j] = sum over ranks of w * (H eo * svh) + sigmoid(shared gate logit) * (H so * svh_shared), term by term as sz_x3_combine_kernel: the ranks'
+// terms are finished and added in rank order in f64.  dn, parts: the down kernel's sums.
+// What bounds it is the way to the sums - slot, group, blocks: three trips to memory one after the other - and then their 4 bytes an output and rank.
+// So the ranks go that way side by side, a lane each; the sums are asked for by their slots, without waiting for the blocks that say whether
+// they are finished there (of those that are not - one block's share ended inside - the parts are added instead), four ranks at a time; and one warp has all
+// ranks of its outputs, so nothing meets in shared memory.  (A block of a warp a rank for 512 outputs, its terms met in shared memory: 504 rows 42 us, this 38; 256
+// 27, 25; 80 the same 17.)  Shuffles and f64 conversions of eleven rotations an output are the most of it now.
+// grid (ceil(rows * H / 1024)), block 256
+__global__ void __launch_bounds__(256)
 sz_rows_combine_kernel(const float* __restrict__ dn, const long long* __restrict__ parts, const SzRowsPlan* __restrict__ P, const int32_t* __restrict__ ridx, const double* __restrict__ rw,
                        const u8* __restrict__ down, u64 dstride, const u8* __restrict__ sh_down, const float* __restrict__ logits, int ne, int top_k,
                        int rows, int H, int FF, int SF, int has_shared, float* __restrict__ y) {
-    __shared__ float part[SZ_MAX_TOPK + 1][512];
-    __shared__ double rws[SZ_MAX_TOPK];
+    constexpr int RB = 4;               // ranks at a time
     sz_pdl_wait();
     sz_pdl_trigger();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nb = H / 512;
-    const int j = blockIdx.x / nb, b = blockIdx.x % nb;
-    if (warp < top_k || has_shared) {
-        const bool routed = warp < top_k;
-        const int pair = routed ? j * top_k + warp : rows * top_k + j;
-        int e = routed ? __ldcg(ridx + pair) : 0;
-        const int loc = __ldcg(&P->pair_loc[pair]), g = __ldcg(&P->group[loc]);
-        e = (unsigned)e < (unsigned)ne ? e : 0;
-        const u16* svh = (const u16*)(routed ? down + (u64)e * dstride + 2 * (size_t)FF : sh_down + 2 * (size_t)SF) + b * 512 + lane;
-        u16 sv[16];
-#pragma unroll
-        for (int i = 0; i < 16; i++) sv[i] = __ldg(svh + 32 * i);
-        const float sg = routed ? 1.f : sz_sigmoid(__ldcg(logits + (size_t)j * (ne + 1) + ne));
-        const double wt = routed && lane == 0 ? __ldcg(rw + pair) : 0.0;
-        const u32 blocks = __ldcg(&P->dn_blocks[g][b]);
-        const int t = loc - __ldcg(&P->first[g]), b0 = (int)(blocks & 0xffffu), b1 = (int)(blocks >> 16);
-        float v[16];
-        if (b0 == b1) {
-#pragma unroll
-            for (int i = 0; i < 16; i++) v[i] = __ldcg(dn + (size_t)loc * H + b * 512 + lane + 32 * i);
-        } else {
-            long long a[16] = {};
-            for (int q = b0; q <= b1; q++) {
-                if (__ldcg(P->start[1] + q) == __ldcg(P->start[1] + q + 1)) continue;     // (fewer units than blocks: this one has none)
-                const long long* p = sz_rows_part(const_cast<long long*>(parts), q, q > b0) + t * 512 + lane;
-#pragma unroll
-                for (int i = 0; i < 16; i++) a[i] += __ldcg(p + 32 * i);
-            }
-#pragma unroll
-            for (int i = 0; i < 16; i++) v[i] = (float)((double)a[i] * SZ_FIX_INV);
-        }
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-            sz_wht128_warp(v + 4 * c, lane);
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const float x = (v[4 * c + q] * SZ_RSQRT128) * sz_f16_to_f32(sv[4 * c + q]);
-                part[warp][128 * c + lane + 32 * q] = routed ? x : sg * x;
-            }
-        }
-        if (routed && lane == 0) rws[warp] = wt;
+    const int lane = threadIdx.x & 31, nb = H / 128, item = blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int j = item / nb, b = item - j * nb, n = top_k + (has_shared ? 1 : 0);
+    if (j >= rows) return;
+    // lane t: rank t's expert, slot, weight (rank top_k: the shared expert's)
+    int e = 0, loc = 0;
+    double wt = 0.0;
+    float sg = 1.f;
+    if (lane < n) {
+        const bool routed = lane < top_k;
+        loc = __ldcg(&P->pair_loc[routed ? j * top_k + lane : rows * top_k + j]);
+        if (routed) {
+            e = __ldcg(ridx + j * top_k + lane);
+            e = (unsigned)e < (unsigned)ne ? e : 0;
+            wt = __ldcg(rw + j * top_k + lane);
+        } else sg = __ldcg(logits + (size_t)j * (ne + 1) + ne);
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < 512; i += blockDim.x) {
-        double a = 0.0;
-        for (int t = 0; t < top_k; t++) a += rws[t] * (double)part[t][i];
-        if (has_shared) a += (double)part[top_k][i];
-        y[(size_t)j * H + b * 512 + i] = (float)a;
+    float v[2][RB][4];
+    u16 sv[2][RB][4];
+    auto fetch = [&](int t0, float (*d)[4], u16 (*s)[4]) {
+#pragma unroll
+        for (int r = 0; r < RB; r++) {
+            const int t = t0 + r;
+            const int l = __shfl_sync(0xffffffffu, loc, t), ex = __shfl_sync(0xffffffffu, e, t);
+            if (t >= n) continue;
+            const u16* svh = (const u16*)(t < top_k ? down + (u64)ex * dstride + 2 * (size_t)FF : sh_down + 2 * (size_t)SF) + b * 128 + lane;
+#pragma unroll
+            for (int i = 0; i < 4; i++) { d[r][i] = __ldcg(dn + (size_t)l * H + b * 128 + lane + 32 * i); s[r][i] = __ldg(svh + 32 * i); }
+        }
+    };
+    fetch(0, v[0], sv[0]);
+    u32 blocks = 0;
+    int row = 0;                        // the pair's row of its group
+    if (lane < n) {
+        const int g = __ldcg(&P->group[loc]);
+        blocks = __ldcg(&P->dn_blocks[g][b >> 2]);
+        row = loc - __ldcg(&P->first[g]);
     }
+    if (has_shared) sg = sz_sigmoid(__shfl_sync(0xffffffffu, sg, top_k));
+    double a[4] = {0.0, 0.0, 0.0, 0.0};
+    auto add = [&](int t0, float (*d)[4], u16 (*s)[4]) {
+#pragma unroll
+        for (int r = 0; r < RB; r++) {
+            const int t = t0 + r;
+            const u32 bl = __shfl_sync(0xffffffffu, blocks, t);
+            const int tr = __shfl_sync(0xffffffffu, row, t), b0 = (int)(bl & 0xffffu), b1 = (int)(bl >> 16);
+            const double w = __shfl_sync(0xffffffffu, wt, t);
+            if (t >= n) continue;
+            if (b0 != b1) {
+                long long p[4] = {0, 0, 0, 0};
+                for (int q = b0; q <= b1; q++) {
+                    if (__ldcg(P->start[1] + q) == __ldcg(P->start[1] + q + 1)) continue;     // (fewer units than blocks: this one has none)
+                    const long long* at = sz_rows_part(const_cast<long long*>(parts), q, q > b0) + tr * 512 + (b & 3) * 128 + lane;
+#pragma unroll
+                    for (int i = 0; i < 4; i++) p[i] += __ldcg(at + 32 * i);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; i++) d[r][i] = (float)((double)p[i] * SZ_FIX_INV);
+            }
+            sz_wht128_warp(d[r], lane);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float x = (d[r][i] * SZ_RSQRT128) * sz_f16_to_f32(s[r][i]);
+                if (t < top_k) a[i] += w * (double)x;
+                else a[i] += (double)(sg * x);
+            }
+        }
+    };
+    for (int t0 = 0; t0 < n; t0 += 2 * RB) {
+        if (t0 + RB < n) fetch(t0 + RB, v[1], sv[1]);
+        add(t0, v[0], sv[0]);
+        if (t0 + 2 * RB < n) fetch(t0 + 2 * RB, v[0], sv[0]);
+        if (t0 + RB < n) add(t0 + RB, v[1], sv[1]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) y[(size_t)j * H + b * 128 + lane + 32 * i] = (float)a[i];
 }
