@@ -1019,14 +1019,14 @@ static int sz_attn2_go(sz_session* s, cudaStream_t st, const u8* kc, const u8* v
     const sz_model_config& c = s->model.cfg;
     static bool set = false;
     const size_t smem = (size_t)SzAttn2<HD, NQT>::SMEM;
-    if (!set) { SZ_CUDA(cudaFuncSetAttribute(sz_attn2_kernel<HD, NQT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); set = true; }
+    if (!set) { SZ_CUDA(cudaFuncSetAttribute(sz_attn2_kernel<HD, NQT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); set = true; }
     int splits = sz_attn2_splits(s, NQT);
     if (ratio) {   // the sparse form: a block a (kv head, split, row); a row's list holds about the budget's positions, 128 or more a split
         const int by_budget = (c.idx_budget + 127) / 128;
         if (splits > by_budget) splits = by_budget < 1 ? 1 : by_budget;
     }
     *splits_used = splits;
-    SZ_CUDA(sz_launch("attention_grouped", sz_attn2_kernel<HD, NQT>, dim3(c.n_kv_head, splits, ratio ? m : 1), dim3(32 * SzAttn2<HD, NQT>::NW), smem, st, true, (const float*)s->a_q,
+    SZ_CUDA(sz_launch("attention_grouped", sz_attn2_kernel<HD, NQT, false>, dim3(c.n_kv_head, splits, ratio ? m : 1), dim3(32 * SzAttn2<HD, NQT>::NW), smem, st, true, (const float*)s->a_q,
                       kc, vc, (int)c.n_head, (int)c.n_kv_head, m, s->ctx, (const int32_t*)s->state, splits, s->a_part, (u32*)(s->state + 2),
                       (const SzTree*)(s->tree_pass ? s->ids + 32 : nullptr), (const int32_t*)(ratio ? s->i_list : nullptr), (const int32_t*)s->i_count,
                       s->i_ctx_blocks, ratio, (const SzSeqDev*)nullptr, (const SzAttnGroup*)nullptr, 0));
@@ -1729,9 +1729,10 @@ struct SzAttnBatch { int row0, rows, g0[4], ng[3], splits[3]; };   // rows that 
 template <int HD, int NQT>
 static int sz_rows_attn_go(cudaStream_t st, const sz_model_config& c, const float* aq, int splits, const SzSeqDev* seqs, const SzAttnGroup* groups, int ng, int ai) {
     static bool set = false;
-    const size_t smem = (size_t)SzAttn2<HD, NQT>::SMEM;
-    if (!set) { SZ_CUDA(cudaFuncSetAttribute(sz_attn2_kernel<HD, NQT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); set = true; }
-    SZ_CUDA(sz_launch("rows_attention", sz_attn2_kernel<HD, NQT>, dim3(c.n_kv_head, splits, ng), dim3(32 * SzAttn2<HD, NQT>::NW), smem, st, true, aq, (const u8*)nullptr, (const u8*)nullptr,
+    constexpr bool FOUR = HD == 256 && NQT == 2;
+    const size_t smem = (size_t)SzAttn2<HD, NQT, FOUR>::SMEM;
+    if (!set) { SZ_CUDA(cudaFuncSetAttribute(sz_attn2_kernel<HD, NQT, FOUR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); set = true; }
+    SZ_CUDA(sz_launch("rows_attention", sz_attn2_kernel<HD, NQT, FOUR>, dim3(c.n_kv_head, splits, ng), dim3(32 * SzAttn2<HD, NQT, FOUR>::NW), smem, st, true, aq, (const u8*)nullptr, (const u8*)nullptr,
                       (int)c.n_head, (int)c.n_kv_head, 0, 0, (const int32_t*)nullptr, 0, (float*)nullptr, (u32*)nullptr, (const SzTree*)nullptr, (const int32_t*)nullptr,
                       (const int32_t*)nullptr, 0, 0, seqs, groups, ai));
     return SZ_OK;

@@ -1271,13 +1271,16 @@ sz_attn_kernel(const float* __restrict__ q, const u8* __restrict__ kc, const u8*
 // chunk instead of four); the softmax spreads over all threads, and its sums, which only the end needs, are added up beside the products.
 // 24,576 positions, 16 heads on 2: 1 row 20.6 -> 16.5 us, 4 rows 37 -> 26.7, 8 rows 61.5 -> 41 (launched one after the other).
 #define SZ_AT_T 64
-template <int HD, int NQT>
+// FOUR: two tiles of queries in blocks of 4 warps, two a multiprocessor, for a step of many sequences: its thousands of blocks have two or three
+// chunks each, and one alone on a multiprocessor waits for its queries, its first chunks and its barriers.  (A lone pass has a block a multiprocessor
+// anyway, and 8 warps do it sooner.)  16 sequences of 3 or 4 rows, contexts up to 15,000: 187 -> 142 us a launch.
+template <int HD, int NQT, bool FOUR = false>
 struct SzAttn2 {
     static constexpr int HB = HD + (((HD >> 5) * 2 + 15) & ~15);
     static constexpr int KS = HD / 16;              // k-steps of the score contraction
     // 16 queries: 4 warps, two blocks a multiprocessor; the fragments of 256 dimensions take 128 registers a thread
-    static constexpr int NW = NQT == 1 ? 4 : 8;
-    static constexpr int OCC = HD == 256 && NQT > 1 ? 1 : 2;
+    static constexpr int NW = NQT == 1 || FOUR ? 4 : 8;
+    static constexpr int OCC = HD == 256 && NW == 8 ? 1 : 2;
     static constexpr int NP = 64 * NQT / NW / 8;    // scores: tiles of 8 positions a warp
     static constexpr int TPQ = 2 * NW / NQT;        // softmax: threads a query
     static constexpr int PP = SZ_AT_T / TPQ;        // .. and positions a thread
@@ -1286,11 +1289,12 @@ struct SzAttn2 {
     static constexpr int TG = NT < 4 ? NT : 4;      // .. n-tiles that share a scale group of the values
     static constexpr int SST = SZ_AT_T + 8;         // row stride of the score / probability tile (floats)
     static constexpr int STAGE = SZ_AT_T * HB;      // a chunk of K or of V
-    static constexpr int SMEM = 64 + 4 * STAGE + NQT * KS * 32 * 16 * 2 + 2 * NQT * 16 * SST * 4 + NQT * 16 * 4;
+    static constexpr int SMEM = 64 + 4 * STAGE + NQT * KS * 32 * 16 + 2 * NQT * 16 * SST * 4 + NQT * 16 * 4;
+    static_assert(KS * 32 * 16 <= 2 * 16 * SST * 4, "the queries' high parts lie where the scores will");
 };
 
-template <int HD, int NQT>
-__global__ void __launch_bounds__(32 * SzAttn2<HD, NQT>::NW, SzAttn2<HD, NQT>::OCC)
+template <int HD, int NQT, bool FOUR>
+__global__ void __launch_bounds__(32 * SzAttn2<HD, NQT, FOUR>::NW, SzAttn2<HD, NQT, FOUR>::OCC)
 sz_attn2_kernel(const float* __restrict__ qin, const u8* __restrict__ kc, const u8* __restrict__ vc, int nh, int nkv, int m, int ctx,
                 const int32_t* __restrict__ state, int splits, float* __restrict__ part, u32* __restrict__ err, const SzTree* __restrict__ tr,
                 const int32_t* __restrict__ glist, const int32_t* __restrict__ gcount, int gstride, int ratio, const SzSeqDev* __restrict__ seqs,
@@ -1300,14 +1304,14 @@ sz_attn2_kernel(const float* __restrict__ qin, const u8* __restrict__ kc, const 
     // glist != null: the sparse form, grid (kv heads, splits, rows).  The block serves ONE row (blockIdx.z) and walks that row's list
     // of position groups (`ratio` positions each; row j's list at glist + j * gstride, gcount[j] long) instead of the positions
     // themselves.  A chunk of 64 list positions is then 64 / ratio copies of a group each for K and for V.
-    using A = SzAttn2<HD, NQT>;
+    using A = SzAttn2<HD, NQT, FOUR>;
     constexpr int NTH = 32 * A::NW;
     extern __shared__ __align__(128) u8 smem[];
     u64* bars = (u64*)smem;                                // K chunks in two stages, V chunks in two
     u8* stage = smem + 64;                                 // [2] K, [2] V
-    uint4* qhi = (uint4*)(stage + 4 * A::STAGE);
-    uint4* qlo = qhi + NQT * A::KS * 32;
+    uint4* qlo = (uint4*)(stage + 4 * A::STAGE);
     float* S = (float*)(qlo + NQT * A::KS * 32);           // [2][NQT * 16][SST]
+    uint4* qhi = (uint4*)S;                                // (in registers before the first score is written)
     float* ralpha = S + 2 * NQT * 16 * A::SST;             // this chunk's rescale factor per query
     __shared__ int32_t qrow[16 * NQT];                     // query vector -> (row, head) of the pass
     __shared__ int32_t cgrp[4][SZ_AT_T];                   // sparse form: the groups of the chunks under way
