@@ -484,7 +484,9 @@ static __global__ void __launch_bounds__(256, 2) sz_dense_q8_kernel(const SzDens
 // every unit, and the parts' sums - 98 MB at 256 rows of 12,352 outputs - went through a scratch and a second kernel.  the four MMAs a
 // block and group alone are 44 us.)
 // Where thread blocks of 8 units and 32 rows would leave multiprocessors idle (80 rows of 2,048 outputs: 48 of them, 49 us, 3,000 cycles for
-// 128 columns in which the tensor pipe works 900), the blocks are of 4 units and 16 rows: 35 us.
+// 128 columns in which the tensor pipe works 900), the blocks are of 4 units and 16 rows: 35 us; and of 8 rows where those, too, are fewer than the
+// multiprocessors - a step of few rows is a chain of stages, each as long as the groups a warp has in it (2,048 outputs of 4,096 columns: 24 rows 30.6 ->
+// 24.4 us, 40 rows 30.5 -> 29.1; 80 rows, 160 of the larger blocks, 37.1 both ways).
 // A slice of a matrix row starts at a multiple of 8 bytes, not of 16: the copy starts at the 16-byte boundary below it.
 struct SzDenseRowsCfg {
     int units[SZ_DENSE_MAX_JOBS + 1];   // 16-row units before each job

@@ -673,10 +673,13 @@ int sz_dense_rows_launch(SzDenseArgs& a, void* xh, bool packed, cudaStream_t st,
     if (!set) {
         SZ_CUDA(cudaFuncSetAttribute(sz_dense_rows_q8_kernel<8, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, SzDenseRows<8, 4>::SMEM));
         SZ_CUDA(cudaFuncSetAttribute(sz_dense_rows_q8_kernel<4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SzDenseRows<4, 2>::SMEM));
+        SZ_CUDA(cudaFuncSetAttribute(sz_dense_rows_q8_kernel<4, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SzDenseRows<4, 1>::SMEM));
         set = true;
     }
     if ((units + 7) / 8 * ((a.m + 31) / 32) >= sz_sm_count_session())
         SZ_CUDA(sz_launch(name, sz_dense_rows_q8_kernel<8, 4>, dim3((units + 7) / 8, (a.m + 31) / 32), dim3(256), SzDenseRows<8, 4>::SMEM, st, true, a, c));
+    else if ((units + 3) / 4 * ((a.m + 15) / 16) < sz_sm_count_session())
+        SZ_CUDA(sz_launch(name, sz_dense_rows_q8_kernel<4, 1>, dim3((units + 3) / 4, a.m / 8), dim3(128), SzDenseRows<4, 1>::SMEM, st, true, a, c));
     else
         SZ_CUDA(sz_launch(name, sz_dense_rows_q8_kernel<4, 2>, dim3((units + 3) / 4, (a.m + 15) / 16), dim3(128), SzDenseRows<4, 2>::SMEM, st, true, a, c));
     *taken = 1;
