@@ -484,9 +484,10 @@ static __global__ void __launch_bounds__(256, 2) sz_dense_q8_kernel(const SzDens
 // every unit, and the parts' sums - 98 MB at 256 rows of 12,352 outputs - went through a scratch and a second kernel.  the four MMAs a
 // block and group alone are 44 us.)
 // Where thread blocks of 8 units and 32 rows would leave multiprocessors idle (80 rows of 2,048 outputs: 48 of them, 49 us, 3,000 cycles for
-// 128 columns in which the tensor pipe works 900), the blocks are of 4 units and 16 rows: 35 us; and of 8 rows where those, too, are fewer than the
-// multiprocessors - a step of few rows is a chain of stages, each as long as the groups a warp has in it (2,048 outputs of 4,096 columns: 24 rows 30.6 ->
-// 24.4 us, 40 rows 30.5 -> 29.1; 80 rows, 160 of the larger blocks, 37.1 both ways).
+// 128 columns in which the tensor pipe works 900), the blocks are of 4 units and 16 rows: 35 us; of 8 rows where those, too, are fewer than the
+// multiprocessors (24 rows 30.6 -> 24.4).  What such a launch takes is then the chain of its stages, so up to three halves a multiprocessor two
+// thread blocks share the columns (2,048 outputs of 4,096 columns: 80 rows 37.1 -> 29.3 us, 24 rows 24.4 -> 21.4, 10 rows 24.2 -> 18.6; 12,352 of 2,048:
+// 10 rows 23.1 -> 20.6).
 // A slice of a matrix row starts at a multiple of 8 bytes, not of 16: the copy starts at the 16-byte boundary below it.
 struct SzDenseRowsCfg {
     int units[SZ_DENSE_MAX_JOBS + 1];   // 16-row units before each job
@@ -496,13 +497,16 @@ struct SzDenseRowsCfg {
 #define SZ_DR_COLS 128      // columns a stage
 #define SZ_DR_RS 144        // bytes between the staged slices (136 and where they start)
 #define SZ_DR_XS 160        // halves between the staged rows (16 (mod 32) words: the eight rows a quarter of a warp reads at once)
-// NW: warps a thread block, a unit of 16 matrix rows each; NG: groups of 8 rows of the step
-template <int NW, int NG>
+// NW: warps a thread block, a unit of 16 matrix rows each; NG: groups of 8 rows of the step; KS: thread blocks of a cluster that share the columns,
+// whole parts each.  A part's sums stay where they are made, in shared memory, and once all are there each block adds the parts of its groups in order.
+template <int NW, int NG, int KS = 1>
 struct SzDenseRows {
     static constexpr int WROWS = NW * 16;                                        // matrix rows a thread block
     static constexpr int STAGE = WROWS * SZ_DR_RS + 2 * 8 * NG * SZ_DR_XS * 2;
-    static constexpr int STAGES = NW == 8 ? 2 : 4;
-    static constexpr int SMEM = STAGES * STAGE + WROWS * 8;
+    static constexpr int STAGES = NW == 8 ? 2 : (KS > 1 ? 3 : 4);
+    static constexpr int PARTS = KS > 1 ? 8 / KS * NG * 4 * 32 * NW * 4 : 0;     // [part][group, value][thread]
+    static constexpr int OCC = KS > 1 ? 3 : 2;
+    static constexpr int SMEM = STAGES * STAGE + WROWS * 8 + PARTS;
 };
 
 // grid (ceil(cols / 1024), rows), block 256: the rows' f16 high and low parts
@@ -519,20 +523,21 @@ static __global__ void __launch_bounds__(256) sz_dense_rows_pack_kernel(const fl
     *(uint2*)(xh + (size_t)(rows + j) * cols + 4 * c4) = make_uint2(*(const u32*)&l0, *(const u32*)&l1);
 }
 
-// grid (ceil(units / NW), ceil(rows / (8 NG))), block 32 NW
-template <int NW, int NG>
-static __global__ void __launch_bounds__(32 * NW, 2) sz_dense_rows_q8_kernel(const SzDenseArgs a, const SzDenseRowsCfg c) {
-    using X = SzDenseRows<NW, NG>;
+// grid (ceil(units / NW) * KS, ceil(rows / (8 NG))), block 32 NW, cluster KS; KS > 1: cols a multiple of 128 KS
+template <int NW, int NG, int KS>
+static __global__ void __cluster_dims__(KS, 1, 1) __launch_bounds__(32 * NW, (SzDenseRows<NW, NG, KS>::OCC)) sz_dense_rows_q8_kernel(const SzDenseArgs a, const SzDenseRowsCfg c) {
+    using X = SzDenseRows<NW, NG, KS>;
     constexpr int NTH = 32 * NW;
     constexpr int S = X::STAGES;
     extern __shared__ __align__(128) u8 smem[];
     const u8** wrow = (const u8**)(smem + S * X::STAGE);       // where the thread block's matrix rows start
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, q = lane & 3;
-    const int total = c.units[a.n_jobs], u0 = blockIdx.x * NW, j0 = blockIdx.y * 8 * NG;
+    const int total = c.units[a.n_jobs], u0 = (int)blockIdx.x / KS * NW, j0 = blockIdx.y * 8 * NG, kr = (int)blockIdx.x % KS;
     const int ng = (c.rows - j0) / 8 < NG ? (c.rows - j0) / 8 : NG;
     const size_t rb = (size_t)(a.cols / 32) * 34;
-    const int nchunk = a.cols / SZ_DR_COLS, nblk = a.cols / 256;      // blocks a part
+    const int nchunk = a.cols / SZ_DR_COLS / KS, k0 = kr * nchunk, nblk = a.cols / 256;      // the block's stages, the first of them; blocks of 32 columns a part
+    float* const parts = (float*)(smem + S * X::STAGE + X::WROWS * 8);
     auto locate = [&](int u, int& ji, int& row0, int& nrows) {
         ji = 0;
 #pragma unroll
@@ -550,7 +555,7 @@ static __global__ void __launch_bounds__(32 * NW, 2) sz_dense_rows_q8_kernel(con
     __syncthreads();
     auto stage_w = [&](int ci) {
         u8* st = smem + (size_t)(ci % S) * X::STAGE;
-        const int at = ci * 136 & ~15;
+        const int at = (k0 + ci) * 136 & ~15;
 #pragma unroll
         for (int i = threadIdx.x; i < X::WROWS * 9; i += NTH) {
             const int r = i / 9, ch = i - r * 9;
@@ -562,7 +567,7 @@ static __global__ void __launch_bounds__(32 * NW, 2) sz_dense_rows_q8_kernel(con
 #pragma unroll
         for (int i = threadIdx.x; i < 2 * 8 * NG * 16; i += NTH) {
             const int part = i / (8 * NG * 16), j = (i >> 4) % (8 * NG), ch = i & 15;
-            if (j < ng * 8) sz_cp_async16(st + (size_t)(part * 8 * NG + j) * SZ_DR_XS * 2 + ch * 16, c.xh + (size_t)(part * c.rows + j0 + j) * a.cols + ci * SZ_DR_COLS + ch * 8);
+            if (j < ng * 8) sz_cp_async16(st + (size_t)(part * 8 * NG + j) * SZ_DR_XS * 2 + ch * 16, c.xh + (size_t)(part * c.rows + j0 + j) * a.cols + (k0 + ci) * SZ_DR_COLS + ch * 8);
         }
     };
     for (int i = 0; i < S - 1 && i < nchunk; i++) stage_w(i);      // (the matrices are constants: on their way before the wait)
@@ -574,14 +579,14 @@ static __global__ void __launch_bounds__(32 * NW, 2) sz_dense_rows_q8_kernel(con
     for (int gi = 0; gi < NG; gi++)
 #pragma unroll
         for (int e = 0; e < 4; e++) { tot[gi][e] = 0.f; acc[gi][e] = 0.f; }
-    int left = nblk;                       // blocks left of the part at hand
+    int left = nblk, part = 0;             // blocks left of the part at hand, and its number here
     for (int ci = 0; ci < nchunk; ci++) {
         sz_cp_async_wait<S - 2>();
         __syncthreads();                   // stage ci has landed, and everybody is done with the one that is filled next
         if (ci + S - 1 < nchunk) { stage_w(ci + S - 1); stage_x(ci + S - 1); }
         sz_cp_async_commit();
         const u8* st = smem + (size_t)(ci % S) * X::STAGE;
-        const u8* wr = st + (size_t)(warp * 16 + g) * SZ_DR_RS + ((ci & 1) ? 8 : 0) + 8 * q;
+        const u8* wr = st + (size_t)(warp * 16 + g) * SZ_DR_RS + (((k0 + ci) & 1) ? 8 : 0) + 8 * q;
         const __half* xr = (const __half*)(st + X::WROWS * SZ_DR_RS) + (size_t)g * SZ_DR_XS + 8 * q;
 #pragma unroll
         for (int b = 0; b < 4; b++) {
@@ -621,9 +626,25 @@ static __global__ void __launch_bounds__(32 * NW, 2) sz_dense_rows_q8_kernel(con
 #pragma unroll
                 for (int gi = 0; gi < NG; gi++)
 #pragma unroll
-                    for (int e = 0; e < 4; e++) { tot[gi][e] += acc[gi][e]; acc[gi][e] = 0.f; }
+                    for (int e = 0; e < 4; e++) {
+                        if constexpr (KS > 1) parts[((part * NG + gi) * 4 + e) * NTH + threadIdx.x] = acc[gi][e];
+                        else tot[gi][e] += acc[gi][e];
+                        acc[gi][e] = 0.f;
+                    }
+                part++;
             }
         }
+    }
+    if constexpr (KS > 1) {                // all parts of the block's groups, in order
+        sz_cluster_sync();
+#pragma unroll
+        for (int gi = 0; gi < NG; gi++)
+            if (gi % KS == kr)
+#pragma unroll
+                for (int k = 0; k < 8; k++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) tot[gi][e] += sz_cluster_ld(&parts[((k % (8 / KS) * NG + gi) * 4 + e) * NTH + threadIdx.x], k / (8 / KS));
+        sz_cluster_sync();                 // (no block leaves while another reads its parts)
     }
     const int u = u0 + warp;
     if (u < total) {
@@ -632,7 +653,7 @@ static __global__ void __launch_bounds__(32 * NW, 2) sz_dense_rows_q8_kernel(con
         const SzDenseJob& jb = a.job[ji];
 #pragma unroll
         for (int gi = 0; gi < NG; gi++) {
-            if (gi < ng) {
+            if (gi < ng && (KS == 1 || gi % KS == kr)) {
                 float* o = jb.out + (size_t)(j0 + gi * 8 + 2 * q) * jb.ostride + row0 + g;
                 if (g < nrows) { o[0] = sz_epilogue(jb.epi, tot[gi][0], jb.div); o[jb.ostride] = sz_epilogue(jb.epi, tot[gi][1], jb.div); }
                 if (g + 8 < nrows) { o[8] = sz_epilogue(jb.epi, tot[gi][2], jb.div); o[jb.ostride + 8] = sz_epilogue(jb.epi, tot[gi][3], jb.div); }

@@ -671,17 +671,22 @@ int sz_dense_rows_launch(SzDenseArgs& a, void* xh, bool packed, cudaStream_t st,
     if (!packed) SZ_CUDA(sz_launch("dense_rows_pack", sz_dense_rows_pack_kernel, dim3((a.cols + 1023) / 1024, a.m), dim3(256), 0, st, true, a.x, a.xstride, a.cols, a.m, (__half*)xh));
     static bool set = false;
     if (!set) {
-        SZ_CUDA(cudaFuncSetAttribute(sz_dense_rows_q8_kernel<8, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, SzDenseRows<8, 4>::SMEM));
-        SZ_CUDA(cudaFuncSetAttribute(sz_dense_rows_q8_kernel<4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SzDenseRows<4, 2>::SMEM));
-        SZ_CUDA(cudaFuncSetAttribute(sz_dense_rows_q8_kernel<4, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SzDenseRows<4, 1>::SMEM));
+#define SZ_DR_SET(NW, NG, KS) SZ_CUDA(cudaFuncSetAttribute(sz_dense_rows_q8_kernel<NW, NG, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SzDenseRows<NW, NG, KS>::SMEM))
+        SZ_DR_SET(8, 4, 1); SZ_DR_SET(4, 2, 1); SZ_DR_SET(4, 2, 2); SZ_DR_SET(4, 1, 2);
+#undef SZ_DR_SET
         set = true;
     }
-    if ((units + 7) / 8 * ((a.m + 31) / 32) >= sz_sm_count_session())
-        SZ_CUDA(sz_launch(name, sz_dense_rows_q8_kernel<8, 4>, dim3((units + 7) / 8, (a.m + 31) / 32), dim3(256), SzDenseRows<8, 4>::SMEM, st, true, a, c));
-    else if ((units + 3) / 4 * ((a.m + 15) / 16) < sz_sm_count_session())
-        SZ_CUDA(sz_launch(name, sz_dense_rows_q8_kernel<4, 1>, dim3((units + 3) / 4, a.m / 8), dim3(128), SzDenseRows<4, 1>::SMEM, st, true, a, c));
-    else
-        SZ_CUDA(sz_launch(name, sz_dense_rows_q8_kernel<4, 2>, dim3((units + 3) / 4, (a.m + 15) / 16), dim3(128), SzDenseRows<4, 2>::SMEM, st, true, a, c));
+#define SZ_DR_GO(NW, NG, KS)                                                                                                                     \
+    SZ_CUDA(sz_launch(name, sz_dense_rows_q8_kernel<NW, NG, KS>, dim3((units + NW - 1) / NW * KS, (a.m + 8 * NG - 1) / (8 * NG)), dim3(32 * NW), SzDenseRows<NW, NG, KS>::SMEM, \
+                      st, true, a, c))
+    const int sms = sz_sm_count_session();
+    auto blocks = [&](int nw, int ng) { return (units + nw - 1) / nw * ((a.m + 8 * ng - 1) / (8 * ng)); };
+    const bool halves = a.cols % 256 == 0;      // whole stages in each
+    if (blocks(8, 4) >= sms) SZ_DR_GO(8, 4, 1);
+    else if (!halves || blocks(4, 2) > 222) SZ_DR_GO(4, 2, 1);
+    else if (blocks(4, 2) >= sms) SZ_DR_GO(4, 2, 2);
+    else SZ_DR_GO(4, 1, 2);
+#undef SZ_DR_GO
     *taken = 1;
     return SZ_OK;
 }
