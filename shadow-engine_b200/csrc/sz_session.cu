@@ -672,7 +672,7 @@ int sz_dense_rows_launch(SzDenseArgs& a, void* xh, bool packed, cudaStream_t st,
     static bool set = false;
     if (!set) {
 #define SZ_DR_SET(NW, NG, KS) SZ_CUDA(cudaFuncSetAttribute(sz_dense_rows_q8_kernel<NW, NG, KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SzDenseRows<NW, NG, KS>::SMEM))
-        SZ_DR_SET(8, 4, 1); SZ_DR_SET(4, 2, 1); SZ_DR_SET(4, 2, 2); SZ_DR_SET(4, 1, 2);
+        SZ_DR_SET(8, 4, 1); SZ_DR_SET(4, 2, 1); SZ_DR_SET(4, 2, 2); SZ_DR_SET(4, 1, 2); SZ_DR_SET(4, 1, 4);
 #undef SZ_DR_SET
         set = true;
     }
@@ -681,11 +681,11 @@ int sz_dense_rows_launch(SzDenseArgs& a, void* xh, bool packed, cudaStream_t st,
                       st, true, a, c))
     const int sms = sz_sm_count_session();
     auto blocks = [&](int nw, int ng) { return (units + nw - 1) / nw * ((a.m + 8 * ng - 1) / (8 * ng)); };
-    const bool halves = a.cols % 256 == 0;      // whole stages in each
     if (blocks(8, 4) >= sms) SZ_DR_GO(8, 4, 1);
-    else if (!halves || blocks(4, 2) > 222) SZ_DR_GO(4, 2, 1);
-    else if (blocks(4, 2) >= sms) SZ_DR_GO(4, 2, 2);
-    else SZ_DR_GO(4, 1, 2);
+    else if (blocks(4, 2) > sms * 3 / 2) SZ_DR_GO(4, 2, 1);
+    else if (blocks(4, 2) >= sms) SZ_DR_GO(4, 2, 2);      // (a part of the columns has to be whole stages: cols is a multiple of 256)
+    else if (a.cols % 512 || blocks(4, 1) * 4 > sms * 3) SZ_DR_GO(4, 1, 2);
+    else SZ_DR_GO(4, 1, 4);
 #undef SZ_DR_GO
     *taken = 1;
     return SZ_OK;
