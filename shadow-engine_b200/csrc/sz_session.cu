@@ -1487,7 +1487,7 @@ extern "C" int sz_session_commit_path(sz_session* s, const int32_t* path, int n,
     return SZ_OK;
 }
 
-// Feeds a prompt: chunks of many rows, then passes of up to 8, every row kept; the head runs for the last pass only.  Afterwards sz_session_result gives the
+// Feeds a prompt: chunks of many rows - the last one with the last pass beside it, where both fit -, else passes of up to 8, every row kept; the head runs for the last pass only.  Afterwards sz_session_result gives the
 // top-64 (and logits) of the last pass's rows; the last row's are the prompt's.
 static int sz_prefill_chunks(sz_session* s, const int32_t* ids, int n, uint64_t stream, int* done);
 extern "C" int sz_session_prefill(sz_session* s, const int32_t* ids, int n, uint64_t stream) {
@@ -2376,7 +2376,7 @@ extern "C" int sz_batch_prefill(sz_session* const* ss, int n, const int32_t* con
         if (!ss[b] || !ids[b] || lens[b] < 1) return sz_fail(SZ_E_ARG, "sz_batch_prefill: sequence %d has nothing to feed", b);
     const bool chunks = sz_rows_step_fits(ss, n);
     // a step of twice the rows costs half as much again (every expert's decode is the most of it): where one of the sessions has more room
-    // than the scratch, the steps take that (16 prompts of 75 tokens: 10 steps of 128 rows or 3 of up to 512)
+    // than the scratch, the steps take that (16 prompts of 75 tokens: 10 steps of 128 rows or 2 of up to 512)
     std::shared_ptr<SzRoom> room;
     SzRoomUse use;
     if (chunks)
