@@ -205,6 +205,8 @@ __device__ __forceinline__ bool sz_mbar_wait(u64* bar, u32 phase, u32 limit = 20
     }
     return false;
 }
+// .. for a whole warp that leaves together: lanes count their polls each for itself, so one may give up where another has just seen the phase
+__device__ __forceinline__ bool sz_mbar_wait_warp(u64* bar, u32 phase) { return __all_sync(0xffffffffu, sz_mbar_wait(bar, phase)); }
 __device__ __forceinline__ void sz_mbar_arrive(u64* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sz_smem_addr(bar)) : "memory");
 }

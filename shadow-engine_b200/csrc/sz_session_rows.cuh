@@ -518,7 +518,7 @@ sz_rows_scan_kernel(const SzSeqDev* __restrict__ seqs, int di, const float* __re
         load(0);
         for (int c = 0; c < sets; c++) {
             const int st = c % ST;
-            if (c >= ST && !sz_mbar_wait(&sh.empty[st], ((c / ST) - 1) & 1)) { if (lane == 0) atomicExch(err, 1u); return; }
+            if (c >= ST && !sz_mbar_wait_warp(&sh.empty[st], ((c / ST) - 1) & 1)) { if (lane == 0) atomicExch(err, 1u); return; }
 #pragma unroll
             for (int j = 0; j < RC; j++)
                 if (c * RC + j < rows) {
@@ -548,7 +548,7 @@ sz_rows_scan_kernel(const SzSeqDev* __restrict__ seqs, int di, const float* __re
     nz2 = *(volatile u64*)&sh.nz2;
     for (int c = 0; c < sets; c++) {
         const int st = c % ST, nr = rows - c * RC < RC ? rows - c * RC : RC;
-        if (!sz_mbar_wait(&sh.full[st], (c / ST) & 1)) { if (lane == 0) atomicExch(err, 1u); return; }
+        if (!sz_mbar_wait_warp(&sh.full[st], (c / ST) & 1)) { if (lane == 0) atomicExch(err, 1u); return; }
         const float (*ks)[D / 32 * SZ_RS_SEG] = sh.k[st], (*qs)[D / 32 * SZ_RS_SEG] = sh.q[st];
         auto pairs = [&](const float* row, u64* to) {
 #pragma unroll
