@@ -5,6 +5,7 @@
 #include "sz_moe_exl3w.cuh"
 #include "sz_moe_blk.cuh"
 #include "sz_moe_rows.cuh"
+#include "sz_rows_rules.cuh"
 
 #include <float.h>
 #include <stdlib.h>
@@ -1233,7 +1234,9 @@ static int sz_rows_run(const sz_moe_layer* L, uint64_t x, int rows, int live, ui
     SZ_ROWS_K(2) SZ_ROWS_K(3) SZ_ROWS_K(4)
 #undef SZ_ROWS_K
     if (rc) return rc;
-    SZ_CUDA(sz_launch("rows_combine", sz_rows_combine_kernel, dim3((live * (H / 128) + 7) / 8), dim3(256), 0, st, true, (const float*)(base + S.dn),
+    const bool by_warp = sz_rows_combine_by_warp(live, H, (int)L->top_k, sz_sm_count());
+    SZ_CUDA(sz_launch("rows_combine", by_warp ? sz_rows_combine_kernel : sz_rows_combine_ranks_kernel, dim3(by_warp ? (live * (H / 128) + 7) / 8 : live * (H / 512)),
+                      dim3(by_warp ? 256 : (L->top_k + 1) * 32), 0, st, true, (const float*)(base + S.dn),
                       (const long long*)(base + S.parts), (const SzRowsPlan*)P, (const int32_t*)ridx, (const double*)rw, (const u8*)L->down, (u64)L->down_stride, (const u8*)L->sh_down,
                       (const float*)logits, (int)L->n_expert, (int)L->top_k, live, H, (int)L->expert_ff, (int)L->shared_ff, shared ? 1 : 0, (float*)y));
     return SZ_OK;

@@ -9,7 +9,7 @@
 //   gate/up   sz_rows_gateup_kernel: a persistent launch over all groups
 //   act       sz_rows_act_kernel: SwiGLU of every pair, left as the down product's operand fragments
 //   down      sz_rows_down_kernel: as gate/up, over those fragments
-//   combine   sz_rows_combine_kernel: per (row, 128 outputs) the ranks' terms in rank order, as sz_x3_combine_kernel adds them
+//   combine   sz_rows_combine_ranks_kernel, sz_rows_combine_kernel: an output's ranks' terms in rank order, as sz_x3_combine_kernel adds them
 // A pair's numbers do not depend on which rows share its group (every row of a group is a column of its own in the tensor-core
 // product, the sums over column blocks are integer): a row's output is bit for bit what sz_moe_verify gives for it.
 //
@@ -601,14 +601,79 @@ sz_rows_down_kernel(const SzRowsPlan* __restrict__ P, const u8* __restrict__ dow
     if (failed && lane == 0) atomicExch(err, 1u);
 }
 
-// ---- combine: a warp a (row, 128 outputs) ------------------------------------------------------------------------------------------------
+// ---- combine: two forms (which: sz_rows_combine_by_warp) ---------------------------------------------------------------------------------
 // y[j] = sum over ranks of w * (H eo * svh) + sigmoid(shared gate logit) * (H so * svh_shared), term by term as sz_x3_combine_kernel: the ranks'
 // terms are finished and added in rank order in f64.  dn, parts: the down kernel's sums.
+// A warp a rank for 512 outputs of a row: warp t finishes rank t's term (warp top_k: the shared expert's), then a thread adds an output's terms.
+// A block takes the 512 outputs of one of its items, so that the way to the sums - expert, slot, group, blocks: four trips to memory one after
+// the other - is gone once for 16 values a lane (a block per 128 outputs: 504 rows 55 -> 43 us), and the ranks go it side by side: few rows' sums, which
+// lie in many blocks' parts, are added by all warps at once (1 row of 10 experts 12 us, the form below 24).
+// grid (rows * H / 512), block (top_k + 1) warps
+__global__ void __launch_bounds__((SZ_MAX_TOPK + 1) * 32)
+sz_rows_combine_ranks_kernel(const float* __restrict__ dn, const long long* __restrict__ parts, const SzRowsPlan* __restrict__ P, const int32_t* __restrict__ ridx, const double* __restrict__ rw,
+                       const u8* __restrict__ down, u64 dstride, const u8* __restrict__ sh_down, const float* __restrict__ logits, int ne, int top_k,
+                       int rows, int H, int FF, int SF, int has_shared, float* __restrict__ y) {
+    __shared__ float part[SZ_MAX_TOPK + 1][512];
+    __shared__ double rws[SZ_MAX_TOPK];
+    sz_pdl_wait();
+    sz_pdl_trigger();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nb = H / 512;
+    const int j = blockIdx.x / nb, b = blockIdx.x % nb;
+    if (warp < top_k || has_shared) {
+        const bool routed = warp < top_k;
+        const int pair = routed ? j * top_k + warp : rows * top_k + j;
+        int e = routed ? __ldcg(ridx + pair) : 0;
+        const int loc = __ldcg(&P->pair_loc[pair]), g = __ldcg(&P->group[loc]);
+        e = (unsigned)e < (unsigned)ne ? e : 0;
+        const u16* svh = (const u16*)(routed ? down + (u64)e * dstride + 2 * (size_t)FF : sh_down + 2 * (size_t)SF) + b * 512 + lane;
+        u16 sv[16];
+#pragma unroll
+        for (int i = 0; i < 16; i++) sv[i] = __ldg(svh + 32 * i);
+        const float sg = routed ? 1.f : sz_sigmoid(__ldcg(logits + (size_t)j * (ne + 1) + ne));
+        const double wt = routed && lane == 0 ? __ldcg(rw + pair) : 0.0;
+        const u32 blocks = __ldcg(&P->dn_blocks[g][b]);
+        const int t = loc - __ldcg(&P->first[g]), b0 = (int)(blocks & 0xffffu), b1 = (int)(blocks >> 16);
+        float v[16];
+        if (b0 == b1) {
+#pragma unroll
+            for (int i = 0; i < 16; i++) v[i] = __ldcg(dn + (size_t)loc * H + b * 512 + lane + 32 * i);
+        } else {
+            long long a[16] = {};
+            for (int q = b0; q <= b1; q++) {
+                if (__ldcg(P->start[1] + q) == __ldcg(P->start[1] + q + 1)) continue;     // (fewer units than blocks: this one has none)
+                const long long* p = sz_rows_part(const_cast<long long*>(parts), q, q > b0) + t * 512 + lane;
+#pragma unroll
+                for (int i = 0; i < 16; i++) a[i] += __ldcg(p + 32 * i);
+            }
+#pragma unroll
+            for (int i = 0; i < 16; i++) v[i] = (float)((double)a[i] * SZ_FIX_INV);
+        }
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            sz_wht128_warp(v + 4 * c, lane);
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const float x = (v[4 * c + q] * SZ_RSQRT128) * sz_f16_to_f32(sv[4 * c + q]);
+                part[warp][128 * c + lane + 32 * q] = routed ? x : sg * x;
+            }
+        }
+        if (routed && lane == 0) rws[warp] = wt;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < 512; i += blockDim.x) {
+        double a = 0.0;
+        for (int t = 0; t < top_k; t++) a += rws[t] * (double)part[t][i];
+        if (has_shared) a += (double)part[top_k][i];
+        y[(size_t)j * H + b * 512 + i] = (float)a;
+    }
+}
+
+// .. and a warp a (row, 128 outputs), for many rows of many ranks.
 // What bounds it is the way to the sums - slot, group, blocks: three trips to memory one after the other - and then their 4 bytes an output and rank.
 // So the ranks go that way side by side, a lane each; the sums are asked for by their slots, without waiting for the blocks that say whether
 // they are finished there (of those that are not - one block's share ended inside - the parts are added instead), four ranks at a time; and one warp has all
-// ranks of its outputs, so nothing meets in shared memory.  (A block of a warp a rank for 512 outputs, its terms met in shared memory: 504 rows 42 us, this 38; 256
-// 27, 25; 80 the same 17.)  Shuffles and f64 conversions of eleven rotations an output are the most of it now.
+// ranks of its outputs, so nothing meets in shared memory.  (10 experts a row of 2,048: 504 rows 42 -> 37 us, 256 27 -> 25.)  Shuffles and f64 conversions of eleven rotations an output are the most of it now.
 // grid (ceil(rows * H / 1024)), block 256
 __global__ void __launch_bounds__(256)
 sz_rows_combine_kernel(const float* __restrict__ dn, const long long* __restrict__ parts, const SzRowsPlan* __restrict__ P, const int32_t* __restrict__ ridx, const double* __restrict__ rw,
