@@ -55,7 +55,7 @@ __device__ __forceinline__ void sz_warp_sum_many(double* v, int lane) {
 // wait) and of the M rows of the pass, so nothing is staged in shared memory and every product is formed and added in f64 with one
 // conversion a weight.  The 4 x M partial sums a thread ends with are summed over the warp (sz_warp_sum_many), then over the 8 warps
 // in warp order.  M: rows of the pass; MP: M rounded up to a power of two; NCH: float4 pieces a thread holds per row.
-// LOOP (sz_moe_rows, up to 128 rows; more: sz_route_rows_kernel): a block takes every gridDim.x-th group of 4 router rows, so that its rows of the pass are loaded and converted
+// LOOP (sz_moe_rows, where sz_route_rows_kernel does not take the rows): a block takes every gridDim.x-th group of 4 router rows, so that its rows of the pass are loaded and converted
 // to f64 once for all of them (a block a group had each of 129 blocks do it: 126 us at 256 rows, L2 traffic and conversions).
 template <int M, int MP, int NCH, bool LOOP>
 __global__ void __launch_bounds__(SZ_ROUTE_THREADS)
@@ -1183,10 +1183,9 @@ static int sz_rows_run(const sz_moe_layer* L, uint64_t x, int rows, int live, ui
     double* rw = (double*)(base + S.rw);
     SzRowsPlan* P = (SzRowsPlan*)(base + S.plan);
     const int route_rows = L->n_expert + (shared ? 1 : 0), nch = (H / 4 + SZ_ROUTE_THREADS - 1) / SZ_ROUTE_THREADS;
-    // routing.  Many rows: the logits as tiles on the f64 tensor instructions, then top-k; up to 128 the verify pass's kernel, 8 rows a block row, whose
-    // last blocks choose (us a layer with events between the launches, kernel + top-k against kernel: 80 rows 39 + 8 / 41, 128 41 + 8 / 51, 160 45 + 8 /
-    // 56, 256 54 + 8 / 72, 504 60 + 8 / 98)
-    if (live > 128) {
+    // routing (the forms and the lines between them: sz_route_rows_form)
+    const int form = sz_route_rows_form(route_rows, rows, live, H, sz_sm_count());
+    if (form != SZ_ROUTE_PASS) {
         cudaError_t e = cudaErrorInvalidValue;
 #define SZ_ROWS_ROUTE(NC, WE, WR, ME, NR)                                                                                                    \
     do {                                                                                                                                      \
@@ -1196,21 +1195,18 @@ static int sz_rows_run(const sz_moe_layer* L, uint64_t x, int rows, int live, ui
         e = sz_launch("route_rows", sz_route_rows_kernel<NC, WE, WR, ME, NR>, dim3((route_rows + X::E - 1) / X::E, (live + X::R - 1) / X::R), dim3(X::NT), X::SMEM, st, true, \
                       (const float*)x, H, (const float*)L->router, (const float*)(shared ? L->shared_router : 0), (int)L->n_expert, live, logits); \
     } while (0)
-        // 32 x 64, 32 x 32 or 16 x 16 outputs a block, by the waves of one block a multiprocessor (the smallest: two) and what a block takes
-        auto waves = [&](int e, int r) { return ((route_rows + e - 1) / e * ((live + r - 1) / r) + sz_sm_count() - 1) / sz_sm_count(); };
-        const int large = 86 * waves(32, 64), mid = 45 * waves(32, 32), small = 5 + 12 * waves(16, 16);
-        if (nch <= 1) { if (small <= mid && small <= large) SZ_ROWS_ROUTE(1, 2, 2, 1, 1); else if (mid <= large) SZ_ROWS_ROUTE(1, 2, 4, 2, 1); else SZ_ROWS_ROUTE(1, 2, 4, 2, 2); }
-        else if (nch == 2) { if (small <= mid && small <= large) SZ_ROWS_ROUTE(2, 2, 2, 1, 1); else if (mid <= large) SZ_ROWS_ROUTE(2, 2, 4, 2, 1); else SZ_ROWS_ROUTE(2, 2, 4, 2, 2); }
-        else SZ_ROWS_ROUTE(4, 2, 2, 1, 1);
+        if (nch <= 1) SZ_ROWS_ROUTE(1, 2, 2, 1, 1);
+        else if (nch > 2) SZ_ROWS_ROUTE(4, 2, 2, 1, 1);
+        else if (form == SZ_ROUTE_16x16) SZ_ROWS_ROUTE(2, 2, 2, 1, 1);
+        else if (form == SZ_ROUTE_32x32) SZ_ROWS_ROUTE(2, 2, 4, 2, 1);
+        else SZ_ROWS_ROUTE(2, 2, 4, 2, 2);
 #undef SZ_ROWS_ROUTE
         SZ_CUDA(e);
         SZ_CUDA(sz_launch("route_topk", L->n_expert <= 512 ? sz_route_topk_kernel<16> : sz_route_topk_kernel<SZ_MAX_EXPERTS / 32>, dim3((live + SZ_RR_TW - 1) / SZ_RR_TW),
                           dim3(32 * SZ_RR_TW), 0, st, true, (const float*)logits, (int)L->n_expert, (int)L->top_k, live, ridx, rw, (int32_t*)route_idx, (double*)route_w));
     } else {   // (the chunks' own plans are written and not used)
-        const int groups = (route_rows + SZ_ROUTE_RB - 1) / SZ_ROUTE_RB;
-        int gx = sz_sm_count() / chunks;                 // about one block a multiprocessor over all chunks of 8 rows
-        gx = gx < 1 ? 1 : (gx > groups ? groups : gx);
-        if (H > 2048) gx = groups;                       // (wider rows do not stay in registers as f64: a block a group)
+        const int gx = sz_route_pass_blocks((route_rows + SZ_ROUTE_RB - 1) / SZ_ROUTE_RB, chunks, H, sz_sm_count());
+        static_assert(SZ_ROUTE_RB == 4, "sz_route_rows_form counts groups of 4");
         const dim3 grid(gx, chunks), block(SZ_ROUTE_THREADS);
         cudaError_t e = cudaErrorInvalidValue;
 #define SZ_ROWS_ROUTE(NC, LOOP)                                                                                                            \

@@ -9,8 +9,8 @@
 // butterfly is a tree over the chains in registers (sz_rr_tree), and one warp goes through the 8 parts.
 // What bounds it is the f64 pipe, 64 multiply-adds a clock and multiprocessor: 29 us for 504 rows x 513 router rows x 2,048, an eighth more for the
 // tree's additions, and the conversions, which take it, too.  The f32 operands are staged 128 NCH columns at a time, two stages, and converted
-// behind shared memory.  Measured with the events around it: 504 rows 60 us, 256 54 (the pass's kernel with a block row for 8 rows, which adds
-// by shuffles and chooses, too: 98 and 72).  Conversions by integer instructions (504 rows: 76; of the rows alone 67), or once a block into
+// behind shared memory.  Measured with the events around it: 504 rows 59 us, 248 39 (the pass's kernel with a block row for 8 rows, which adds
+// by shuffles and chooses, too: 98 and 57; where it is the sooner one: sz_route_rows_form).  Conversions by integer instructions (504 rows: 76; of the rows alone 67), or once a block into
 // f64 stages (69, for want of a second stage): slower.
 // A block takes 8 ME WE router rows and 8 NR WR rows of the step: WE x WR warps, a warp 8 ME router rows and 8 NR rows.
 template <int NCH, int WE, int WR, int ME, int NR>

@@ -12,3 +12,32 @@ static inline bool sz_rows_combine_by_warp(int live, int hidden, int top_k, int 
     const int items = live * (hidden / 512);         // pieces of 512 outputs; two a block of the first form
     return top_k >= 10 && (items >= 832 || (items >= 480 && items / 2 <= 2 * sms));
 }
+
+// The router over more than 128 rows: the pass's kernel with a block row for 8 rows (its last blocks choose), or the logits as tiles on the f64 tensor
+// instructions and a kernel that chooses - in tiles of 16 x 16, for 1,025 .. 2,048 columns also 32 x 32 or 32 x 64 (router rows x rows; up
+// to 1,024 the larger ones were sooner nowhere: 513 router rows, 504 rows: 37 each; beyond 2,048 they do not fit shared memory).  Up to 128 rows the
+// pass's.  Each form's time in tenths of us, from runs of all of them at 17 .. 1,001 router rows x 136 .. 504 rows x 512 .. 4,096 columns; an estimate is
+// within a tenth of its measurement.
+//   pass  by how many groups of 4 router rows a block takes one after the other (wider than 2,048 columns, by its blocks: a group a block)
+//   tiles by waves of a block a multiprocessor, and 8 us of the kernel that chooses
+// (2,048 columns, 513 router rows, pass / best tiles: 136 rows 37 / 31 + 8, 200 47 / 32 + 8, 256 57 / 38 + 8, 504 98 / 59 + 8; 129 router rows: 136 20 / 20 + 8, 504 35 /
+// 27 + 8; 17: 504 17 / 21 + 8; 1,024 columns, 513: 136 31 / 18 + 8, 504 76 / 37 + 8; 4,096 columns, 17: 136 28 / 44 + 8, 256 36 / 45 + 8; 129: 256 80 / 46 + 8.)
+enum { SZ_ROUTE_PASS, SZ_ROUTE_16x16, SZ_ROUTE_32x32, SZ_ROUTE_32x64 };
+// blocks of the pass's kernel that share the router rows of 8 rows: about one a multiprocessor over all of them (wider rows do not stay in registers as f64: a block a group)
+static inline int sz_route_pass_blocks(int groups, int chunks, int hidden, int sms) {
+    const int gx = sms / chunks < 1 ? 1 : sms / chunks;
+    return hidden > 2048 || gx > groups ? groups : gx;
+}
+static inline int sz_route_rows_form(int route_rows, int rows, int live, int hidden, int sms) {
+    if (live <= 128) return SZ_ROUTE_PASS;
+    auto waves = [&](int e, int r) { return ((route_rows + e - 1) / e * ((live + r - 1) / r) + sms - 1) / sms; };
+    const int groups = (route_rows + 3) / 4, chunks = rows / 8, gx = sz_route_pass_blocks(groups, chunks, hidden, sms), in_turn = (groups + gx - 1) / gx;
+    const int w = waves(16, 16);
+    int pass, small, mid = 1 << 30, large = 1 << 30;
+    if (hidden <= 1024) { pass = 130 + 19 * in_turn / 2; small = 85 + 37 * w; }
+    else if (hidden <= 2048) {      // (three blocks of the smallest tiles a multiprocessor)
+        pass = 140 + 132 * in_turn / 10; small = 225 * ((w - 1) / 3) + (w % 3 == 1 ? 205 : w % 3 == 2 ? 265 : 315); mid = 60 + 320 * waves(32, 32); large = 50 + 540 * waves(32, 64);
+    } else { pass = 240 + (int)(groups * chunks * 148ll / sms / 2); small = 150 + 293 * w; }
+    const int best = small <= mid && small <= large ? small : mid <= large ? mid : large;
+    return best + 80 >= pass ? SZ_ROUTE_PASS : best == small ? SZ_ROUTE_16x16 : best == mid ? SZ_ROUTE_32x32 : SZ_ROUTE_32x64;
+}

@@ -5,6 +5,7 @@ import subprocess
 
 import pytest
 
+from tests.test_gpu_rows_forms import ROUTES
 from tests.util import ROOT
 
 CSRC = os.path.join(ROOT, "shadow-engine_b200", "csrc")
@@ -24,3 +25,17 @@ def ask(tmp_path, expr):
                                                        (504, 2048, 8, 0), (256, 4096, 8, 0), (256, 2048, 2, 0)])
 def test_combine(tmp_path, live, hidden, top_k, by_warp):
     assert ask(tmp_path, "sz_rows_combine_by_warp(%d, %d, %d, 148)" % (live, hidden, top_k)) == by_warp
+
+
+# (router rows, rows, columns) -> the form: where the router rows are few a verify pass's kernel, however many rows
+@pytest.mark.parametrize("route_rows,rows,hidden,form", [(513, 128, 2048, "PASS"), (513, 136, 2048, "PASS"), (513, 176, 2048, "16x16"), (513, 256, 2048, "32x32"), (513, 504, 2048, "32x64"),
+                                                         (17, 504, 2048, "PASS"), (65, 504, 2048, "PASS"), (129, 256, 2048, "PASS"), (257, 136, 2048, "PASS"), (257, 304, 2048, "16x16"),
+                                                         (1001, 400, 2048, "16x16"), (17, 256, 4096, "PASS"), (65, 256, 4096, "PASS"), (129, 256, 4096, "16x16"), (513, 136, 4096, "16x16"),
+                                                         (17, 504, 1024, "PASS"), (65, 256, 512, "PASS"), (513, 136, 1024, "16x16"), (513, 504, 512, "16x16")])
+def test_router(tmp_path, route_rows, rows, hidden, form):
+    assert ask(tmp_path, "sz_route_rows_form(%d, %d, %d, %d, 148) == SZ_ROUTE_%s" % (route_rows, rows, rows, hidden, form))
+
+
+@pytest.mark.parametrize("hidden,n_expert,top_k,shared,rows,form", ROUTES)
+def test_the_gpu_tests_reach_the_routers_forms(tmp_path, hidden, n_expert, top_k, shared, rows, form):
+    assert ask(tmp_path, "sz_route_rows_form(%d, %d, %d, %d, 148) == %s" % (n_expert + shared, rows, rows, hidden, form))
