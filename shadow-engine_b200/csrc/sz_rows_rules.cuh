@@ -41,3 +41,9 @@ static inline int sz_route_rows_form(int route_rows, int rows, int live, int hid
     const int best = small <= mid && small <= large ? small : mid <= large ? mid : large;
     return best + 80 >= pass ? SZ_ROUTE_PASS : best == small ? SZ_ROUTE_16x16 : best == mid ? SZ_ROUTE_32x32 : SZ_ROUTE_32x64;
 }
+
+// Attention of a step's groups of two query tiles, heads of 256 (sz_attn2_kernel), by the blocks that have positions: blocks of four warps, two a multiprocessor, or of eight, one a
+// multiprocessor.  Four win where blocks queue; where each has a multiprocessor of its own, eight do it sooner (eight / four: 1 sequence of 4 rows at 24,000
+// positions, 128 blocks, 30.8 / 36.8; 2, 256 blocks, 55 / 47; at 8,000 2 of them, 128 blocks, 24.4 / 28.6; 3, 192 blocks, 41 / 34; 32 at 200, 128 blocks,
+// 17.4 / 20.4) - a step of few sequences, and the last rows of a prompt.
+static inline bool sz_attn_four_warps(int blocks, int sms) { return blocks > sms; }

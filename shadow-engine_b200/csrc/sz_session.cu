@@ -8,6 +8,7 @@
 // then the buffers swap.  The KV cache is append-only: rejected positions are overwritten by the next pass.
 #include "sz_session_kernels.cuh"
 #include "sz_session_rows.cuh"
+#include "sz_rows_rules.cuh"
 #include "sz_indexer.cuh"
 #include "sz_ple.cuh"
 
@@ -1732,12 +1733,12 @@ static bool sz_rows_fits(const sz_session* s) {
     return true;
 }
 
-struct SzAttnBatch { int row0, rows, g0[4], ng[3], splits[3]; };   // rows that attend in one go: their groups by size of the queries (16, 32, 64)
+// rows that attend in one go: their groups by size of the queries (16, 32, 64); blocks: how many of a size's have positions to attend to
+struct SzAttnBatch { int row0, rows, g0[4], ng[3], splits[3], blocks[3]; };
 
-template <int HD, int NQT>
-static int sz_rows_attn_go(cudaStream_t st, const sz_model_config& c, const float* aq, int splits, const SzSeqDev* seqs, const SzAttnGroup* groups, int ng, int ai) {
+template <int HD, int NQT, bool FOUR>
+static int sz_rows_attn_launch(cudaStream_t st, const sz_model_config& c, const float* aq, int splits, const SzSeqDev* seqs, const SzAttnGroup* groups, int ng, int ai) {
     static bool set = false;
-    constexpr bool FOUR = HD == 256 && NQT == 2;
     const size_t smem = (size_t)SzAttn2<HD, NQT, FOUR>::SMEM;
     if (!set) { SZ_CUDA(cudaFuncSetAttribute(sz_attn2_kernel<HD, NQT, FOUR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); set = true; }
     SZ_CUDA(sz_launch("rows_attention", sz_attn2_kernel<HD, NQT, FOUR>, dim3(c.n_kv_head, splits, ng), dim3(32 * SzAttn2<HD, NQT, FOUR>::NW), smem, st, true, aq, (const u8*)nullptr, (const u8*)nullptr,
@@ -1745,12 +1746,18 @@ static int sz_rows_attn_go(cudaStream_t st, const sz_model_config& c, const floa
                       (const int32_t*)nullptr, 0, 0, seqs, groups, ai));
     return SZ_OK;
 }
+template <int HD, int NQT>
+static int sz_rows_attn_go(cudaStream_t st, const sz_model_config& c, const float* aq, int splits, const SzSeqDev* seqs, const SzAttnGroup* groups, int ng, int blocks, int ai) {
+    if constexpr (HD == 256 && NQT == 2)
+        if (sz_attn_four_warps(blocks, sz_sm_count_session())) return sz_rows_attn_launch<HD, NQT, true>(st, c, aq, splits, seqs, groups, ng, ai);
+    return sz_rows_attn_launch<HD, NQT, false>(st, c, aq, splits, seqs, groups, ng, ai);
+}
 template <int HD>
 static int sz_rows_attn(cudaStream_t st, const sz_model_config& c, const float* aq, const SzAttnBatch& B, const SzSeqDev* seqs, const SzAttnGroup* groups, int ai) {
     int rc = SZ_OK;
-    if (B.ng[0] && (rc = sz_rows_attn_go<HD, 1>(st, c, aq, B.splits[0], seqs, groups + B.g0[0], B.ng[0], ai))) return rc;
-    if (B.ng[1] && (rc = sz_rows_attn_go<HD, 2>(st, c, aq, B.splits[1], seqs, groups + B.g0[1], B.ng[1], ai))) return rc;
-    if (B.ng[2] && (rc = sz_rows_attn_go<HD, 4>(st, c, aq, B.splits[2], seqs, groups + B.g0[2], B.ng[2], ai))) return rc;
+    if (B.ng[0] && (rc = sz_rows_attn_go<HD, 1>(st, c, aq, B.splits[0], seqs, groups + B.g0[0], B.ng[0], B.blocks[0], ai))) return rc;
+    if (B.ng[1] && (rc = sz_rows_attn_go<HD, 2>(st, c, aq, B.splits[1], seqs, groups + B.g0[1], B.ng[1], B.blocks[1], ai))) return rc;
+    if (B.ng[2] && (rc = sz_rows_attn_go<HD, 4>(st, c, aq, B.splits[2], seqs, groups + B.g0[2], B.ng[2], B.blocks[2], ai))) return rc;
     return SZ_OK;
 }
 
@@ -1803,7 +1810,12 @@ static int sz_rows_layers(sz_session* const* ss, int n, const int32_t* ids, cons
             B.row0 = row0; B.rows = end - row0;
             for (int k = 0; k < 3; k++) {
                 B.g0[k] = ng_all; B.ng[k] = (int)cls[k].size(); B.splits[k] = 0;
-                for (const SzAttnGroup& g : cls[k]) { if (g.splits > B.splits[k]) B.splits[k] = g.splits; hg[ng_all++] = g; }
+                for (const SzAttnGroup& g : cls[k]) {
+                    if (g.splits > B.splits[k]) B.splits[k] = g.splits;
+                    const int np = ss[g.seq]->len + g.j0 + g.m, per = ((np + g.splits - 1) / g.splits + SZ_AT_T - 1) / SZ_AT_T * SZ_AT_T;   // as the kernel shares them
+                    B.blocks[k] += nkv * ((np + per - 1) / per);
+                    hg[ng_all++] = g;
+                }
                 cls[k].clear();
             }
             if (B.rows > 0) ab.push_back(B);

@@ -1272,8 +1272,8 @@ sz_attn_kernel(const float* __restrict__ q, const u8* __restrict__ kc, const u8*
 // 24,576 positions, 16 heads on 2: 1 row 20.6 -> 16.5 us, 4 rows 37 -> 26.7, 8 rows 61.5 -> 41 (launched one after the other).
 #define SZ_AT_T 64
 // FOUR: two tiles of queries in blocks of 4 warps, two a multiprocessor, for a step of many sequences: its thousands of blocks have two or three
-// chunks each, and one alone on a multiprocessor waits for its queries, its first chunks and its barriers.  (A lone pass has a block a multiprocessor
-// anyway, and 8 warps do it sooner.)  16 sequences of 3 or 4 rows, contexts up to 15,000: 187 -> 142 us a launch.
+// chunks each, and one alone on a multiprocessor waits for its queries, its first chunks and its barriers.  (Where there is a block a multiprocessor
+// anyway - a lone pass, a step of few sequences -, 8 warps do it sooner: sz_attn_four_warps.)  16 sequences of 3 or 4 rows, contexts up to 15,000: 187 -> 142 us a launch.
 template <int HD, int NQT, bool FOUR = false>
 struct SzAttn2 {
     static constexpr int HB = HD + (((HD >> 5) * 2 + 15) & ~15);

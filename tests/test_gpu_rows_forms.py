@@ -52,3 +52,35 @@ def test_rows_that_are_not_numbers_are_routed_as_in_the_passes(hidden, n_expert,
         assert torch.equal(ridx[c:c + 8], ic), "rows %d.." % c
         for a, b in ((rw[c:c + 8], wc), (y[c:c + 8], yc)):
             assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.nan_to_num(0.0, 1.0, -1.0), b.nan_to_num(0.0, 1.0, -1.0)), "rows %d.." % c
+
+
+SLICE = dict(n_layer=4, hidden=2048, streams=4, hc_rank=256, vocab=4096, n_head=16, n_kv_head=2, head_dim=256, rope_dims=64, n_expert=512, n_expert_used=10, expert_ff=512,
+             shared_ff=512, ssm_k_heads=16, ssm_v_heads=32, ssm_head_dim=128, conv_k=4, attn_interval=4, eps=1e-6, rope_theta=1e7)
+
+
+@pytest.fixture(scope="module")
+def slice4():
+    return md.DeviceModel(md.make_model(SLICE, dense_type=szlib.TYPE_Q8_0, expert_type=szlib.TYPE_EXL3(3), seed=5, device="cuda"))
+
+
+# histories of less than a chunk of 64 positions, of one, of many chunks a split and of many splits, at and beside their edges.  Five sequences in blocks of
+# four warps, two chunks and more each; one and two (at most 128 blocks with positions) in blocks of eight
+@pytest.mark.parametrize("lengths", [(70, 700, 1333, 3001, 5000), (2045, 4096, 8100, 61, 2048), (64, 7000), (6000,)])
+def test_attention_of_a_step_over_long_histories_is_the_passes(slice4, lengths):
+    n, ctx = len(lengths), 8192
+    rng = np.random.default_rng(41)
+    batch = md.Batch(slice4, n, ctx)
+    alone = [md.Session(slice4, ctx, kv_q8=True, lean=True) for _ in range(n)]
+    for b, length in enumerate(lengths):
+        batch.sessions[b].fill_synthetic(length, seed=50 + b)
+        alone[b].fill_synthetic(length, seed=50 + b)
+    for step in range(2):                # (the second one stands on the first one's rows)
+        rows = [[int(t) for t in rng.integers(0, SLICE["vocab"], 3 + (b + step) % 2)] for b in range(n)]
+        batch.verify(rows)
+        for b in range(n):
+            got = batch.sessions[b].result(logits=True)[2].view(np.uint32)
+            batch.sessions[b].commit(len(rows[b]))
+            alone[b].verify(rows[b])
+            want = alone[b].result(logits=True)[2].view(np.uint32)
+            alone[b].commit(len(rows[b]))
+            assert np.array_equal(got, want), "step %d, history %d" % (step, lengths[b])

@@ -39,3 +39,9 @@ def test_router(tmp_path, route_rows, rows, hidden, form):
 @pytest.mark.parametrize("hidden,n_expert,top_k,shared,rows,form", ROUTES)
 def test_the_gpu_tests_reach_the_routers_forms(tmp_path, hidden, n_expert, top_k, shared, rows, form):
     assert ask(tmp_path, "sz_route_rows_form(%d, %d, %d, %d, 148) == %s" % (n_expert + shared, rows, rows, hidden, form))
+
+
+# blocks with positions: one, two and three sequences at 8,000 (2 KV heads x 32 splits each), 32 at 200
+@pytest.mark.parametrize("blocks,four", [(64, 0), (128, 0), (148, 0), (192, 1), (256, 1), (4096, 1)])
+def test_attention_of_a_step(tmp_path, blocks, four):
+    assert ask(tmp_path, "sz_attn_four_warps(%d, 148)" % blocks) == four
