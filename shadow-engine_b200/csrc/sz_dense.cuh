@@ -484,10 +484,9 @@ static __global__ void __launch_bounds__(256, 2) sz_dense_q8_kernel(const SzDens
 // every unit, and the parts' sums - 98 MB at 256 rows of 12,352 outputs - went through a scratch and a second kernel.  the four MMAs a
 // block and group alone are 44 us.)
 // Where thread blocks of 8 units and 32 rows would leave multiprocessors idle (80 rows of 2,048 outputs: 48 of them, 49 us, 3,000 cycles for
-// 128 columns in which the tensor pipe works 900), the blocks are of 4 units and 16 rows: 35 us; of 8 rows where those, too, are fewer than the
-// multiprocessors (24 rows 30.6 -> 24.4).  What such a launch takes is then the chain of its stages, so as long as three of them fit
-// a multiprocessor two thread blocks share the columns, or four (2,048 outputs of 4,096 columns: 80 rows 37.1 -> 29.3 us in two, 24 rows 24.4 -> 21.4 and
-// 18.2 in four, 10 rows 24.2 -> 18.6 and 16.2; 12,352 of 2,048: 10 rows 23.1 -> 20.6 in two).
+// 128 columns in which the tensor pipe works 900), the blocks are of 4 units and 16 rows (35 us) or 8.  What such a launch takes is then the chain of its
+// stages, so two or four thread blocks share the columns as long as the multiprocessors have room for them: sz_dense_rows_form has the lines and what
+// the forms measured.
 // A slice of a matrix row starts at a multiple of 8 bytes, not of 16: the copy starts at the 16-byte boundary below it.
 struct SzDenseRowsCfg {
     int units[SZ_DENSE_MAX_JOBS + 1];   // 16-row units before each job

@@ -47,3 +47,19 @@ static inline int sz_route_rows_form(int route_rows, int rows, int live, int hid
 // positions, 128 blocks, 30.8 / 36.8; 2, 256 blocks, 55 / 47; at 8,000 2 of them, 128 blocks, 24.4 / 28.6; 3, 192 blocks, 41 / 34; 32 at 200, 128 blocks,
 // 17.4 / 20.4) - a step of few sequences, and the last rows of a prompt.
 static inline bool sz_attn_four_warps(int blocks, int sms) { return blocks > sms; }
+
+// The Q8_0 projections over many rows (sz_dense_rows_q8_kernel): units of 16 matrix rows -> warps a block (a unit each), groups of 8 rows a block, blocks
+// that share the columns.  Blocks of 8 units and 32 rows where they are as many as the multiprocessors; else of 4 and 16, or of 4 and 8 where those, too, are
+// fewer than the multiprocessors.  As long as three of them fit a multiprocessor two share the columns, or four (us a launch from memory, blocks of 16 rows alone / in
+// two, of 8 rows in two / in four: 2,048 x 4,096, 80 rows 37 / 29, 42 / 41; 24 rows 29 / 21, 21 / 17; 8 rows 29 / 21, 19 / 13).  Where blocks of 8 rows in two would be
+// more than that, those of 16 share (9,216 x 2,048, 16 rows: 18.9 / 16.9, 20.7 / 26.4; 4,096 x 1,024, 32 rows 12.7 / 12.8, 14.8 / 16.9).  Of 512 columns, four
+// stages, only blocks that are few do (1,024 rows, 32 rows: 10.7 / 9.5, 8.7 / 8.7; 8,192, 8 rows: 8.8 / 10.7, 10.7 / 10.7).
+struct SzDenseRowsForm { int warps, groups, share; };
+static inline SzDenseRowsForm sz_dense_rows_form(int units, int rows, int cols, int sms) {
+    auto blocks = [&](int nw, int ng) { return (units + nw - 1) / nw * ((rows + 8 * ng - 1) / (8 * ng)); };
+    if (blocks(8, 4) >= sms) return {8, 4, 1};
+    if (blocks(4, 2) > sms * 3 / 2 || (cols <= 512 && blocks(4, 1) * 4 > sms * 2)) return {4, 2, 1};
+    if (blocks(4, 2) >= sms || blocks(4, 1) * 2 > sms * 3) return {4, 2, 2};      // (a part of the columns has to be whole stages: cols is a multiple of 256)
+    if (cols % 512 || blocks(4, 1) * 4 > sms * 3) return {4, 1, 2};
+    return {4, 1, 4};
+}

@@ -680,12 +680,11 @@ int sz_dense_rows_launch(SzDenseArgs& a, void* xh, bool packed, cudaStream_t st,
 #define SZ_DR_GO(NW, NG, KS)                                                                                                                     \
     SZ_CUDA(sz_launch(name, sz_dense_rows_q8_kernel<NW, NG, KS>, dim3((units + NW - 1) / NW * KS, (a.m + 8 * NG - 1) / (8 * NG)), dim3(32 * NW), SzDenseRows<NW, NG, KS>::SMEM, \
                       st, true, a, c))
-    const int sms = sz_sm_count_session();
-    auto blocks = [&](int nw, int ng) { return (units + nw - 1) / nw * ((a.m + 8 * ng - 1) / (8 * ng)); };
-    if (blocks(8, 4) >= sms) SZ_DR_GO(8, 4, 1);
-    else if (blocks(4, 2) > sms * 3 / 2) SZ_DR_GO(4, 2, 1);
-    else if (blocks(4, 2) >= sms) SZ_DR_GO(4, 2, 2);      // (a part of the columns has to be whole stages: cols is a multiple of 256)
-    else if (a.cols % 512 || blocks(4, 1) * 4 > sms * 3) SZ_DR_GO(4, 1, 2);
+    const SzDenseRowsForm f = sz_dense_rows_form(units, a.m, a.cols, sz_sm_count_session());
+    if (f.warps == 8) SZ_DR_GO(8, 4, 1);
+    else if (f.share == 1) SZ_DR_GO(4, 2, 1);
+    else if (f.groups == 2) SZ_DR_GO(4, 2, 2);
+    else if (f.share == 2) SZ_DR_GO(4, 1, 2);
     else SZ_DR_GO(4, 1, 4);
 #undef SZ_DR_GO
     *taken = 1;

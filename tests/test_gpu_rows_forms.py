@@ -84,3 +84,16 @@ def test_attention_of_a_step_over_long_histories_is_the_passes(slice4, lengths):
             want = alone[b].result(logits=True)[2].view(np.uint32)
             alone[b].commit(len(rows[b]))
             assert np.array_equal(got, want), "step %d, history %d" % (step, lengths[b])
+
+
+# the projections of 9,216 and 12,352 outputs of 2,048 columns and of 2,048 of 4,096 at 8, 16, 24, 40, 64 and 80 rows: every form of their kernel
+@pytest.mark.parametrize("ms", [(5,), (8, 3), (8, 8, 2), (8,) * 4 + (3,), (8,) * 8, (8,) * 9 + (5,)])
+def test_projections_of_few_rows_are_the_passes(slice4, ms):
+    rng = np.random.default_rng(43)
+    batch = md.Batch(slice4, len(ms), 16)
+    rows = [[int(t) for t in rng.integers(0, SLICE["vocab"], m)] for m in ms]
+    batch.verify(rows)
+    for b, r in enumerate(rows):
+        s = md.Session(slice4, 16, kv_q8=True, lean=True)
+        s.verify(r)
+        assert np.array_equal(batch.sessions[b].result(logits=True)[2].view(np.uint32), s.result(logits=True)[2].view(np.uint32)), "sequence %d" % b

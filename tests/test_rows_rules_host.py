@@ -45,3 +45,12 @@ def test_the_gpu_tests_reach_the_routers_forms(tmp_path, hidden, n_expert, top_k
 @pytest.mark.parametrize("blocks,four", [(64, 0), (128, 0), (148, 0), (192, 1), (256, 1), (4096, 1)])
 def test_attention_of_a_step(tmp_path, blocks, four):
     assert ask(tmp_path, "sz_attn_four_warps(%d, 148)" % blocks) == four
+
+
+# (matrix rows, rows, columns) -> warps, groups of 8 rows, blocks that share the columns
+@pytest.mark.parametrize("out,rows,cols,form", [(12352, 80, 2048, (8, 4, 1)), (9216, 8, 2048, (4, 1, 2)), (9216, 16, 2048, (4, 2, 2)), (12352, 16, 2048, (4, 2, 2)),
+                                                (2048, 8, 4096, (4, 1, 4)), (2048, 24, 4096, (4, 1, 4)), (2048, 64, 4096, (4, 2, 2)), (2048, 80, 4096, (4, 2, 2)), (4096, 32, 1024, (4, 2, 2)),
+                                                (2048, 8, 768, (4, 1, 2)), (8192, 8, 512, (4, 2, 1)), (1024, 32, 512, (4, 1, 4)), (12352, 16, 512, (4, 2, 1)), (12352, 24, 2048, (4, 2, 1))])
+def test_projections(tmp_path, out, rows, cols, form):
+    f = "sz_dense_rows_form(%d, %d, %d, 148)" % (out // 16, rows, cols)
+    assert ask(tmp_path, "%s.warps * 100 + %s.groups * 10 + %s.share" % (f, f, f)) == form[0] * 100 + form[1] * 10 + form[2]
