@@ -61,8 +61,8 @@ __device__ __forceinline__ int sz_rows_weight(int n) { return n <= 8 ? 172 + n :
 // padding behind an expert's (sz_rows_plan_smem).
 // One block whose 32 warps wait for shared memory most of the time, so what counts is how often they go there one after the other: a pair's place
 // is one count and one word (counting its expert's words one by one, two banks for all experts, took 20,600 of 51,000 cycles at 504 rows), and the
-// block that an item falls to is guessed from its weight and put right (two binary searches an item: 16,400).  With the events around it: 504 rows 32 -> 25 us,
-// 256 25 -> 21, 80 18 -> 15.
+// block that an item falls to is guessed from its weight and put right (two binary searches an item: 16,400).  With the events around it, 512 experts: 504 rows 33 -> 25 us,
+// 256 25 -> 19, 96 18 -> 14, 8 12 -> 10.  (The loops over a thread's pairs end with the call's: all of them made a division each, 2 us where pairs are few.)
 #define SZ_ROWS_MW (SZ_ROWS_CAP / 32 + 1)       // words of an expert's mask (odd: experts in different banks)
 static inline size_t sz_rows_plan_smem(int experts) { return (size_t)experts * SZ_ROWS_MW * 6; }
 __global__ void __launch_bounds__(1024)
@@ -87,6 +87,7 @@ sz_rows_plan_kernel(const int32_t* __restrict__ ridx, int R, int k, int ne, int 
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < NP; i++) {
+        if (1024 * i >= pairs) break;
         const int row = (t + 1024 * i) / k;
         if ((unsigned)pe[i] >= (unsigned)ne) continue;     // (a routing that was never written: caught below, nothing is touched)
         atomicOr(&mask[pe[i] * MW + (row >> 5)], 1u << (row & 31));
@@ -148,8 +149,9 @@ sz_rows_plan_kernel(const int32_t* __restrict__ ridx, int R, int k, int ne, int 
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < NP; i++) {
-        const int p = t + 1024 * i, e = pe[i], row = p / k;
+        const int p = t + 1024 * i, e = pe[i];
         if (p >= pairs) break;
+        const int row = p / k;
         if ((unsigned)e >= (unsigned)ne) { P->pair_loc[p] = 0; P->overflow = 4; atomicOr(err, 4u); continue; }   // an expert id out of range: the call is reported as failed (the flag is this call's, the word stays)
         const int n = pre[e * MW + (row >> 5)] + __popc(mask[e * MW + (row >> 5)] & ((1u << (row & 31)) - 1u));
         const int slot = slot_of[e] + n;
