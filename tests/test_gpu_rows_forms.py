@@ -97,3 +97,49 @@ def test_projections_of_few_rows_are_the_passes(slice4, ms):
         s = md.Session(slice4, 16, kv_q8=True, lean=True)
         s.verify(r)
         assert np.array_equal(batch.sessions[b].result(logits=True)[2].view(np.uint32), s.result(logits=True)[2].view(np.uint32)), "sequence %d" % b
+
+
+def fed_alone(dm, ctx, prompt):
+    """A session that took the prompt in passes of up to 8 rows; the last one is pending."""
+    s = md.Session(dm, ctx, kv_q8=True, lean=True)
+    for c in range(0, len(prompt), 8):
+        s.verify(prompt[c:c + 8])
+        if c + 8 < len(prompt):
+            s.result()
+            s.commit(8)
+    return s
+
+
+# the scan's instances for more blocks than two a multiprocessor, with more stages of 8 rows than its ring has: prompts fed together, each one's last pass beside its
+# chunk.  Some of the last pass is kept, and the next pass stands on the chunk's state and the kept rows'.
+@pytest.mark.parametrize("d,lens", [(128, (75, 33, 41, 66)), (128, (17, 24, 57)), (64, (75, 40, 33, 64, 49, 9))])
+def test_the_scan_of_many_sequences_chunks_is_the_passes(d, lens):
+    cfg = dict(md.TINY, vocab=2048, n_expert=16, n_expert_used=4, shared_ff=256, n_layer=4, ssm_head_dim=d, ssm_k_heads=16, ssm_v_heads=32)
+    dm = md.DeviceModel(md.make_model(cfg, expert_type=szlib.TYPE_EXL3(3), seed=24))
+    prompts = [md.make_prompt(n, cfg["vocab"], seed=120 + n) for n in lens]
+    batch = md.Batch(dm, len(lens), 128)
+    batch.prefill(prompts)
+    for b, p in enumerate(prompts):
+        s, f = fed_alone(dm, 128, p), batch.sessions[b]
+        keep = ((len(p) - 1) % 8 + 1 + 1) // 2
+        for q in (s, f):
+            q.first = q.result(logits=True)[2].view(np.uint32)
+            q.commit(keep)
+            q.verify([7, 8, 9, 10])
+            q.second = q.result(logits=True)[2].view(np.uint32)
+        assert len(f) == len(s) and np.array_equal(f.first, s.first) and np.array_equal(f.second, s.second), "prompt %d" % b
+
+
+# a prompt's chunk at the shapes of the benchmark's layers: the router's 32 x 64 tiles, the combine a warp a row, the scan of one sequence, rows of two query tiles at its end
+@pytest.mark.parametrize("n", [507, 268])
+def test_a_long_chunk_at_the_benchmarks_layers_is_the_passes(slice4, n):
+    prompt = md.make_prompt(n, SLICE["vocab"], seed=n)
+    a, b = md.Session(slice4, 560, kv_q8=True), fed_alone(slice4, 560, prompt)
+    a.prefill(prompt)
+    for s in (a, b):
+        s.first = s.result(logits=True)
+        s.commit(2)
+        s.verify([5, 6, 7])
+        s.second = s.result(logits=True)
+    assert np.array_equal(a.first[2].view(np.uint32), b.first[2].view(np.uint32)) and np.array_equal(a.first[1], b.first[1])
+    assert np.array_equal(a.second[2].view(np.uint32), b.second[2].view(np.uint32)) and np.array_equal(a.second[1], b.second[1])
