@@ -1723,8 +1723,8 @@ extern "C" int sz_batch_scratch_init(const sz_model* m, int rows_max, uint64_t s
 // ---- many rows through the layers ----------------------------------------------------------------------------------------------------------
 // What a step of sz_batch_verify and sz_batch_prefill and the chunks of sz_session_prefill run: every kernel of a layer once over the
 // rows of all sequences, from tables (sz_session_rows.cuh).  A sequence brings up to 8 rows of a pass, or, where every row is kept and
-// none needs logits (a prompt before its last pass), any number: the recurrences run through them in one launch and attention
-// takes them in groups of 8, so that the rows are bit for bit those of the passes they replace.
+// none needs logits (a prompt before its last pass), any number, or such a chunk and behind it the rows of the pass that stands on it: the
+// recurrences run through them in one launch and attention takes them in groups of 8, so that the rows are bit for bit those of the passes they replace.
 static bool sz_rows_fits(const sz_session* s) {
     const sz_model_config& c = s->model.cfg;
     if (!s->hc_fast || s->p_hist || c.idx_heads > 0 || !(s->flags & SZ_KV_Q8) || c.n_head / c.n_kv_head * SZ_MAX_VERIFY > 64 || s->want_routes) return false;

@@ -454,8 +454,8 @@ sz_rows_delta_prep_kernel(const SzSeqDev* __restrict__ seqs, const SzRowDev* __r
 //   - the output products of a row run beside the next row's k products; runs of 8 rows are added up at once, and left unnormed: the gated
 //     norm over a head's D outputs is sz_rows_gate_kernel's, not eight f64 chains a stage inside this one;
 //   - a fifth warp keeps SZ_RS_STAGES stages of 8 rows' operands on their way.
-// Measured (128 x 128 states, 32 heads; us a launch, events between the launches): 504 rows of one prompt 298 -> 169 and 10 for the gate, which
-// packs the rows as a launch of 7 did before; 80 rows of 32 sequences 63 -> 48 and 8.  MINB: blocks a multiprocessor that the registers leave room
+// Measured (128 x 128 states, 32 heads; us a launch, events between the launches): 504 rows of one prompt 298 -> 164 and 10 for the gate, which
+// packs the rows as a launch of 7 did before; 80 rows of 32 sequences 63 -> 47 and 8.  MINB: blocks a multiprocessor that the registers leave room
 // for - 2 where no more come (three: 186 for one prompt), 3 for many sequences (two: 57 for the 32).  A row takes some 800 cycles: 300 the products with
 // the reads of its operands, 270 the sum (two conversions of 27 cycles, ten f64 operations of 8, two shuffles), 105 the update, 115 a row's share of a
 // stage.  The next row's k in registers of its own, its reads in a fixed order, or conversions by integer instructions: 179 - 190 for one prompt.
